@@ -90,10 +90,16 @@ class StackedGruQat:
         """Runs the two callables on the current and the side stream and joins them."""
         main = torch.cuda.current_stream(self.device)
         self.side.wait_stream(main)
-        self._lib.rxmet_set_concurrent_passes(2)   # the two directions share the SMs: their CTAs are resident together
-        fn_forward()
-        with torch.cuda.stream(self.side):
-            fn_reverse()
+        # The two directions share the SMs: their CTAs are resident together.  The setting is read where a launch is
+        # planned and holds for the whole process, so it goes back at once: left at 2, every later recurrence of the
+        # program plans for half of the SMs (a wide LSTM forward at batch 4096: 289 ms instead of 143 ms).
+        self._lib.rxmet_set_concurrent_passes(2)
+        try:
+            fn_forward()
+            with torch.cuda.stream(self.side):
+                fn_reverse()
+        finally:
+            self._lib.rxmet_set_concurrent_passes(1)
         main.wait_stream(self.side)
 
     def _layer_input(self, li: int, x: torch.Tensor) -> torch.Tensor:
