@@ -87,6 +87,34 @@ int residentPerSm(const void *kernel, int block, size_t smem) {
     return n;
 }
 
+int residentClusters(const void *kernel, int ctas, int block, size_t smem) {
+    static std::mutex guard;
+    static std::map<std::tuple<int, const void *, int, int, size_t>, int> known;
+    ensureDynamicSmem(kernel, smem);
+    const int device = currentDevice().device;
+    std::lock_guard<std::mutex> lock(guard);
+    const auto key = std::make_tuple(device, kernel, ctas, block, smem);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+    cfg.blockDim = dim3(static_cast<unsigned>(block));
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = static_cast<unsigned>(ctas);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    known[key] = n;
+    return n;
+}
+
 OverlapLane &overlapLane() {
     constexpr int kMaxDevices = 64;
     static thread_local OverlapLane lanes[kMaxDevices];

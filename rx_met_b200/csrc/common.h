@@ -127,6 +127,9 @@ void ensureDynamicSmem(const void *kernel, size_t bytes);
 // Resident CTAs per SM of `kernel` at this block size and dynamic shared memory, asked once per
 // device and configuration (at least 1).
 int residentPerSm(const void *kernel, int block, size_t smem);
+// Clusters of `ctas` CTAs of `kernel` that the device holds at the same time (0 when it holds none), asked once per
+// device and configuration.
+int residentClusters(const void *kernel, int ctas, int block, size_t smem);
 
 inline size_t alignUp(size_t v, size_t a) { return (v + a - 1) / a * a; }
 

@@ -179,6 +179,14 @@ def test_backward_quant(gl, cfg_name, shape):
         assert np.array_equal(a[k], b[k]), k
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 8, 96), (2, 5, 8, 128), (3, 9, 8, 160), (4, 17, 8, 192), (5, 3, 12, 224), (3, 300, 8, 256),
+                                   (2, 130, 8, 64), (2, 260, 8, 32)], ids=lambda s: "x".join(map(str, s)))
+def test_backward_quant_over_clusters(gl, shape):
+    """Every width the cluster recurrence is built for (32 and 64 units per CTA), 4, 8 and 16 rows per cluster with the
+    last cluster partly empty, and sequences shorter than its three-step operand ring."""
+    test_backward_quant(gl, "w8a8" if shape[3] <= 128 else "a16", shape)
+
+
 @pytest.mark.parametrize("shape", [(80, 256, 40, 128), (80, 256, 72, 64)], ids=lambda s: "x".join(map(str, s)))
 def test_backward_quant_row_ranges_of_several_tiles(gl, shape):
     """Enough rows (T*B = 20480) that every CTA of the tcgen05 input-gradient kernel walks two 128-row
