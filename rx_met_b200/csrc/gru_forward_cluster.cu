@@ -1,0 +1,350 @@
+// W8 / A16 QuantGRU recurrence over thread-block clusters: the integer cell on top of plane_recurrence_umma.cuh.
+//
+// The arithmetic is the integer carrier's, value for value (gru_device.cuh): 64-bit rounding rescales and 16-segment tables.
+// What differs from the generic cell is how much of it an element executes: shifts are known to lie in [1, 31] where the
+// operand is a grid difference, so a rescale is one widening multiply, one add and two funnel shifts; a table segment is found through a 256-bucket map (the segment of the
+// bucket's first code and the one behind its only threshold) instead of fifteen compare-and-selects; the scalar
+// constants come from the constant bank.
+// T = 100, B = 128, H = 256, one direction of two at a time: 490 -> 190 us per pass (recurrentPlanes, dp4a).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <climits>
+#include <cstdint>
+
+#include "common.h"
+#include "gru_device.cuh"
+#include "gru_forward_wide.h"
+#include "plane_recurrence_umma.cuh"
+
+namespace rxmet {
+namespace gru {
+namespace {
+
+constexpr int kBuckets = 256;
+
+struct FastLut {
+    int4 segment[kSegments];          // q_b, n_bx, term_c, threshold
+    uint16_t bucket[kBuckets];        // segment at the bucket's first code | segment behind its threshold << 8
+};
+
+// round_half_even(p / 2^n) for 1 <= n <= 31, low 32 bits: (p + 2^(n-1) - 1 + odd(floor(p / 2^n))) >> n on two words.
+__device__ __forceinline__ int32_t roundShift31(int64_t p, int n, uint32_t roundAdd) {
+    const uint32_t odd = __funnelshift_r(static_cast<uint32_t>(p), static_cast<uint32_t>(static_cast<uint64_t>(p) >> 32), n) & 1u;
+    const uint64_t sum = static_cast<uint64_t>(p) + (roundAdd + odd);
+    return static_cast<int32_t>(__funnelshift_r(static_cast<uint32_t>(sum), static_cast<uint32_t>(sum >> 32), n));
+}
+
+// Rounding rescale of a 32-bit operand, shift in [1, 31], and of a product of two, shift in [1, 62].
+struct ReadyRescale {
+    int32_t mult, shift;
+    uint32_t roundAdd;
+};
+struct ReadyWide {
+    int32_t mult, shift;
+    int64_t roundAdd;
+};
+__device__ __forceinline__ int32_t apply(int32_t x, const ReadyRescale &r) {
+    return roundShift31(static_cast<int64_t>(x) * r.mult, r.shift, r.roundAdd);
+}
+__device__ __forceinline__ int32_t apply(int64_t x, const ReadyWide &r) {
+    const int64_t p = x * r.mult;
+    if (r.shift <= 31) return roundShift31(p, r.shift, static_cast<uint32_t>(r.roundAdd));
+    return static_cast<int32_t>(rshiftRoundConst(p, r.shift, r.roundAdd));
+}
+
+// What the kernel needs of the tables, prepared on the host.
+struct CellScalars {
+    ReadyRescale ihTo[3], hhTo[2], newToH;
+    ReadyWide rhToNew, oldToH;
+    int32_t zpIh, zpHh, zpIn[3], loIn[3], hiIn[3], zpOut[3], loOut[3], hiOut[3], zpH, loH, hiH, loHh, hiHh, quantOne;
+    int32_t zpX[3], bucketShift[3];
+    float eff[3], effH, effHh;
+};
+
+// What a training forward saves of the clamp flags.
+enum class Flags { None, Bytes, Packed };
+
+template <int H, Flags FLAGS>
+struct GruPlaneCell {
+    static constexpr int kGates = 3;
+    CellScalars s;
+    FastLut luts[3];
+    size_t B;
+    const uint32_t *words;    // [kWords][3H]
+    const int64_t *addend;    // [3H]
+    const Rescale *rescale;   // [3H]
+    const int16_t *ih;        // [T][B][3H]
+    const int16_t *h0;        // [B][hPad] codes
+    int hPad;
+    float *h, *v;             // [T+1][B][H], [T][B][4H] dequantized
+    int32_t *hq, *vq;         // optional codes
+    uint8_t *maskHh, *maskGateIn, *maskGateOut, *maskH;
+    const uint8_t *maskIh;    // packed flags: those of the input projection, to be packed with the step's
+    uint16_t *stepBits;
+    const int *poison;        // status word of the tensor-core projection: non-zero turns the hidden outputs into NaN
+
+    struct Shared {
+        FastLut luts[3];
+    };
+    struct Lane {
+        int64_t addend, roundAdd;
+        int32_t mult, shift;
+        bool narrow;   // warp-uniform: the shifts of all lanes lie in [1, 31]
+    };
+    struct State {
+        int32_t h, code[3], hhn;
+        uint32_t keep;   // bits 0..2 gate output z, r, n; 3..5 gate input; 6..8 hh linear; 12 hidden state
+    };
+    struct Fetch {};
+    struct FetchB {
+        int32_t ih[3];
+        uint32_t keepIh[3];
+    };
+
+    __device__ __forceinline__ uint32_t weightWord(int gate, int unit, int kw) const {
+        return gate < 3 ? __ldg(words + static_cast<size_t>(kw) * 3 * H + gate * H + unit) : 0u;
+    }
+    __device__ __forceinline__ void init(Shared &sh, int tid, int threads) const {
+        for (int i = tid; i < static_cast<int>(sizeof(Shared) / 4); i += threads)
+            reinterpret_cast<uint32_t *>(&sh)[i] = reinterpret_cast<const uint32_t *>(luts)[i];
+    }
+    __device__ __forceinline__ Lane lane(const Shared &, int gate, int unit) const {
+        Lane l{0, 0, 0, 1, false};
+        if (gate < 3) {
+            const Rescale r = rescale[gate * H + unit];
+            l.addend = addend[gate * H + unit];
+            l.mult = r.mult;
+            l.shift = r.shift;
+        }
+        l.roundAdd = l.shift >= 1 ? (int64_t{1} << (l.shift - 1)) - 1 : 0;
+        l.narrow = __all_sync(0xffffffffu, l.shift >= 1 && l.shift <= 31);
+        return l;
+    }
+    __device__ __forceinline__ float scaleH(bool alive) const {
+        return (!alive || (poison && *poison)) ? __int_as_float(0x7fc00000) : s.effH;
+    }
+    __device__ __forceinline__ void begin(const Shared &, State &st, int row, int unit) const {
+        st.h = h0[static_cast<size_t>(row) * hPad + unit];
+        const size_t o = static_cast<size_t>(row) * H + unit;
+        h[o] = static_cast<float>(st.h - s.zpH) * scaleH(true);
+        if (hq) hq[o] = st.h;
+    }
+    __device__ __forceinline__ void fetch(Fetch &, size_t, uint32_t, int, int) const {}
+    __device__ __forceinline__ void fetchB(FetchB &f, size_t at, uint32_t row, int unit) const {
+        const int16_t *from = ih + at * (3 * H) + (row * (3 * H) + unit);
+#pragma unroll
+        for (int g = 0; g < 3; ++g) f.ih[g] = __ldg(from + g * H);
+        if (FLAGS == Flags::Packed) {
+            const uint8_t *keep = maskIh + at * (3 * H) + (row * (3 * H) + unit);
+#pragma unroll
+            for (int g = 0; g < 3; ++g) f.keepIh[g] = __ldg(keep + g * H);
+        }
+    }
+    // hh linear code, its keep flag in bit 0
+    template <int STRIDE>
+    __device__ __forceinline__ uint32_t linear(const Shared &, const Lane &l, const Fetch &, const uint32_t *acc, size_t, uint32_t, int, int, bool) const {
+        const int64_t total = (static_cast<int64_t>(static_cast<int32_t>(acc[0])) << 8) + static_cast<int32_t>(acc[STRIDE]) + l.addend;
+        const int64_t prod = total * l.mult;
+        int32_t res;
+        if (l.narrow) res = roundShift31(prod, l.shift, static_cast<uint32_t>(l.roundAdd));
+        else res = l.shift >= 1 ? static_cast<int32_t>(rshiftRoundConst(prod, l.shift, l.roundAdd)) : static_cast<int32_t>(prod << -l.shift);
+        uint8_t keep;
+        const int32_t code = clampCode(res + s.zpHh, s.loHh, s.hiHh, keep);
+        return static_cast<uint32_t>(code * 2 + keep);
+    }
+    __device__ __forceinline__ int32_t activation(const FastLut &lut, int g, int32_t qx, uint32_t &keepOut) const {
+        const uint32_t b = lut.bucket[static_cast<uint32_t>(qx - s.loIn[g]) >> s.bucketShift[g]];
+        const uint32_t before = b & 0xffu;
+        const uint32_t seg = qx < lut.segment[before].w ? before : b >> 8;
+        const int4 e = lut.segment[seg];
+        const int64_t bx = static_cast<int64_t>(e.x) * (qx - s.zpX[g]);
+        const int32_t y = roundShift31(bx, e.y, (1u << (e.y - 1)) - 1u) + e.z;
+        uint8_t keep;
+        const int32_t code = clampCode(y, s.loOut[g], s.hiOut[g], keep);
+        keepOut |= static_cast<uint32_t>(keep) << g;
+        return code;
+    }
+    __device__ __forceinline__ uint32_t cell(const Shared &sh, State &st, const FetchB &in, const uint32_t (&v)[4]) const {
+        uint32_t keep = 0;
+        int32_t hh[3];
+#pragma unroll
+        for (int g = 0; g < 3; ++g) {
+            hh[g] = static_cast<int32_t>(v[g]) >> 1;
+            keep |= (v[g] & 1u) << (6 + g);
+        }
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            uint8_t k;
+            const int32_t pre = clampCode(apply(in.ih[g] - s.zpIh, s.ihTo[g]) + apply(hh[g] - s.zpHh, s.hhTo[g]) + s.zpIn[g], s.loIn[g], s.hiIn[g], k);
+            keep |= static_cast<uint32_t>(k) << (3 + g);
+            st.code[g] = activation(sh.luts[g], g, pre, keep);
+        }
+        {
+            uint8_t k;
+            const int64_t prod = static_cast<int64_t>(st.code[1] - s.zpOut[1]) * (hh[2] - s.zpHh);
+            const int32_t pre = clampCode(apply(in.ih[2] - s.zpIh, s.ihTo[2]) + apply(prod, s.rhToNew) + s.zpIn[2], s.loIn[2], s.hiIn[2], k);
+            keep |= static_cast<uint32_t>(k) << 5;
+            st.code[2] = activation(sh.luts[2], 2, pre, keep);
+        }
+        {
+            uint8_t k;
+            const int32_t fresh = apply(st.code[2] - s.zpOut[2], s.newToH);
+            const int64_t sum = static_cast<int64_t>(st.code[0] - s.zpOut[0]) * (st.h - s.zpH) + static_cast<int64_t>(s.quantOne - st.code[0]) * fresh;
+            st.h = clampCode(apply(sum, s.oldToH) + s.zpH, s.loH, s.hiH, k);
+            keep |= static_cast<uint32_t>(k) << 12;
+        }
+        st.hhn = hh[2];
+        st.keep = keep;
+        return static_cast<uint32_t>(st.h - s.loH);
+    }
+    __device__ __forceinline__ void store(const Shared &, const State &st, const FetchB &in, size_t at, uint32_t row, int unit, bool good) const {
+        const uint32_t mine = row * H + unit, mine3 = row * (3 * H) + unit;
+        h[(at + B) * H + mine] = static_cast<float>(st.h - s.zpH) * scaleH(good);
+        float *vRow = v + at * (4 * H) + (row * (4 * H) + unit);
+#pragma unroll
+        for (int g = 0; g < 3; ++g) vRow[g * H] = static_cast<float>(st.code[g] - s.zpOut[g]) * s.eff[g];
+        vRow[3 * H] = static_cast<float>(st.hhn - s.zpHh) * s.effHh;
+        if (hq) hq[(at + B) * H + mine] = st.h;
+        if (vq) {
+            int32_t *to = vq + at * (4 * H) + (row * (4 * H) + unit);
+#pragma unroll
+            for (int g = 0; g < 3; ++g) to[g * H] = st.code[g];
+            to[3 * H] = st.hhn;
+        }
+        if (FLAGS == Flags::Packed)
+            stepBits[at * H + mine] = static_cast<uint16_t>(st.keep | (in.keepIh[0] << 9) | (in.keepIh[1] << 10) | (in.keepIh[2] << 11));
+        if (FLAGS == Flags::Bytes) {
+            if (maskHh) {
+                uint8_t *to = maskHh + at * (3 * H) + mine3;
+#pragma unroll
+                for (int g = 0; g < 3; ++g) to[g * H] = static_cast<uint8_t>((st.keep >> (6 + g)) & 1u);
+            }
+            if (maskGateIn) {
+                uint8_t *toIn = maskGateIn + at * (3 * H) + mine3, *toOut = maskGateOut + at * (3 * H) + mine3;
+#pragma unroll
+                for (int g = 0; g < 3; ++g) {
+                    toIn[g * H] = static_cast<uint8_t>((st.keep >> (3 + g)) & 1u);
+                    toOut[g * H] = static_cast<uint8_t>((st.keep >> g) & 1u);
+                }
+                maskH[at * H + mine] = static_cast<uint8_t>((st.keep >> 12) & 1u);
+            }
+        }
+    }
+    __device__ __forceinline__ void finish(const Shared &, const State &, int, int, bool) const {}
+};
+
+bool ready(const Rescale &r, ReadyRescale &out) {
+    if (r.shift < 1 || r.shift > 31) return false;
+    out = ReadyRescale{r.mult, r.shift, (1u << (r.shift - 1)) - 1u};
+    return true;
+}
+bool ready(const Rescale &r, ReadyWide &out) {
+    if (r.shift < 1 || r.shift > 62) return false;
+    out = ReadyWide{r.mult, r.shift, (int64_t{1} << (r.shift - 1)) - 1};
+    return true;
+}
+
+// Bucket map of one table over the gate-input grid; false when a shift leaves [1, 31] or a bucket holds two thresholds.
+bool ready(const Lut &lut, int32_t lo, int32_t hi, FastLut &out, int32_t &bucketShift) {
+    const int64_t span = static_cast<int64_t>(hi) - lo + 1;
+    bucketShift = 0;
+    while ((span - 1) >> bucketShift >= kBuckets) ++bucketShift;
+    auto segmentOf = [&](int64_t q) {
+        for (int i = 0; i < kSegments - 1; ++i)
+            if (q < lut.threshold[i]) return i;
+        return kSegments - 1;
+    };
+    for (int i = 0; i < kSegments; ++i) {
+        if (lut.n_bx[i] < 1 || lut.n_bx[i] > 31) return false;
+        out.segment[i] = make_int4(lut.q_b[i], lut.n_bx[i], lut.term_c[i], i < kSegments - 1 ? lut.threshold[i] : INT32_MAX);
+    }
+    for (int b = 0; b < kBuckets; ++b) {
+        const int64_t first = lo + (static_cast<int64_t>(b) << bucketShift), last = std::min<int64_t>(first + (int64_t{1} << bucketShift) - 1, hi);
+        if (first > hi) {
+            out.bucket[b] = 0;
+            continue;
+        }
+        const int s0 = segmentOf(first), s1 = segmentOf(last);
+        // only the threshold of s0 may lie in (first, last]
+        if (s1 != s0 && segmentOf(lut.threshold[s0]) != s1) return false;
+        out.bucket[b] = static_cast<uint16_t>(s0 | (s1 << 8));
+    }
+    return true;
+}
+
+// Everything of the cell that does not depend on the width or on what is saved.
+struct Prepared {
+    CellScalars s;
+    FastLut luts[3];
+};
+
+template <int H, Flags FLAGS>
+void launchFor(const WideRecurrence &r, const Prepared &prepared, cudaStream_t st) {
+    constexpr int U = H % 64 == 0 ? 64 : 32;
+    GruPlaneCell<H, FLAGS> cell{};
+    cell.s = prepared.s;
+    std::copy(prepared.luts, prepared.luts + 3, cell.luts);
+    cell.B = static_cast<size_t>(r.B);
+    cell.words = r.words; cell.addend = r.addend; cell.rescale = r.rescale; cell.ih = r.ih; cell.h0 = r.h0; cell.hPad = r.hPad;
+    cell.h = r.h; cell.v = r.v; cell.hq = r.hq; cell.vq = r.vq;
+    cell.maskHh = r.maskHh; cell.maskGateIn = r.maskGateIn; cell.maskGateOut = r.maskGateOut; cell.maskH = r.maskH;
+    cell.maskIh = r.maskIh; cell.stepBits = r.stepBits;
+    cell.poison = r.poison;
+    planerec::launchBest<GruPlaneCell<H, FLAGS>, H, U, 2, 8, 16>("recurrentForward", planerec::Problem{r.T, r.B, r.h0Planes}, cell, st);
+}
+template <int H>
+void launchFor(const WideRecurrence &r, const Prepared &prepared, cudaStream_t st) {
+    if (r.stepBits) launchFor<H, Flags::Packed>(r, prepared, st);
+    else if (r.maskHh || r.maskGateIn) launchFor<H, Flags::Bytes>(r, prepared, st);
+    else launchFor<H, Flags::None>(r, prepared, st);
+}
+
+bool prepare(const Exec &e, Prepared &cell) {
+    const GateExec &g = e.gate;
+    CellScalars &s = cell.s;
+    const int inOp[3] = {RXMET_GRU_UPDATE_GATE_INPUT, RXMET_GRU_RESET_GATE_INPUT, RXMET_GRU_NEW_GATE_INPUT};
+    const int outOp[3] = {RXMET_GRU_UPDATE_GATE_OUTPUT, RXMET_GRU_RESET_GATE_OUTPUT, RXMET_GRU_NEW_GATE_OUTPUT};
+    const Lut *luts[3] = {&g.lut_update, &g.lut_reset, &g.lut_new};
+    const Rescale ihTo[3] = {g.ih_to_update, g.ih_to_reset, g.ih_to_new}, hhTo[2] = {g.hh_to_update, g.hh_to_reset};
+    bool ok = ready(g.rh_to_new, s.rhToNew) && ready(g.new_to_h, s.newToH) && ready(g.update_old_to_h, s.oldToH);
+    for (int i = 0; i < 3 && ok; ++i) {
+        ok = ready(ihTo[i], s.ihTo[i]) && (i == 2 || ready(hhTo[i], s.hhTo[i])) &&
+             ready(*luts[i], g.qlo[inOp[i]], g.qhi[inOp[i]], cell.luts[i], s.bucketShift[i]);
+        s.zpIn[i] = g.zp[inOp[i]]; s.loIn[i] = g.qlo[inOp[i]]; s.hiIn[i] = g.qhi[inOp[i]];
+        s.zpOut[i] = g.zp[outOp[i]]; s.loOut[i] = g.qlo[outOp[i]]; s.hiOut[i] = g.qhi[outOp[i]];
+        s.zpX[i] = luts[i]->zp_x; s.eff[i] = g.eff[outOp[i]];
+    }
+    if (!ok) return false;
+    s.zpIh = g.zp[RXMET_GRU_WEIGHT_IH_LINEAR];
+    s.zpHh = g.zp[RXMET_GRU_WEIGHT_HH_LINEAR]; s.loHh = g.qlo[RXMET_GRU_WEIGHT_HH_LINEAR]; s.hiHh = g.qhi[RXMET_GRU_WEIGHT_HH_LINEAR];
+    s.effHh = g.eff[RXMET_GRU_WEIGHT_HH_LINEAR];
+    s.zpH = g.zp[RXMET_GRU_H]; s.loH = g.qlo[RXMET_GRU_H]; s.hiH = g.qhi[RXMET_GRU_H]; s.effH = g.eff[RXMET_GRU_H];
+    s.quantOne = g.quant_one;
+    return true;
+}
+
+}  // namespace
+
+bool forwardWideClusterTakes(const Exec &e, int H) {
+    Prepared prepared;
+    return H % 32 == 0 && H <= 256 && prepare(e, prepared);
+}
+
+void forwardWideCluster(const WideRecurrence &r, const Exec &e, cudaStream_t st) {
+    Prepared prepared;
+    prepare(e, prepared);
+    switch (r.H) {
+        case 32: launchFor<32>(r, prepared, st); break;
+        case 64: launchFor<64>(r, prepared, st); break;
+        case 96: launchFor<96>(r, prepared, st); break;
+        case 128: launchFor<128>(r, prepared, st); break;
+        case 160: launchFor<160>(r, prepared, st); break;
+        case 192: launchFor<192>(r, prepared, st); break;
+        case 224: launchFor<224>(r, prepared, st); break;
+        default: launchFor<256>(r, prepared, st); break;
+    }
+}
+
+}  // namespace gru
+}  // namespace rxmet

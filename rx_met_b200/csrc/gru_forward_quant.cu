@@ -1068,6 +1068,9 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
             wc.maskGateOut = mk.gate_output; wc.maskH = mk.h;
             if (mk.gate_input || mk.gate_output || mk.h)
                 RXMET_REQUIRE(mk.gate_input && mk.gate_output && mk.h, "gate_input, gate_output and h masks come together");
+            wc.stepBits = call.stepFlags;
+            if (call.stepFlags)
+                RXMET_REQUIRE(training && mk.weight_ih_linear, "packed step flags need a training forward with the weight_ih_linear mask");
             forwardWide(wc, e, ws, st);
             return;
         }
@@ -1554,7 +1557,7 @@ void forwardFpCarrier(const ForwardQuantCall &call, const Exec &e, Workspace &ws
 }
 
 bool packedFlagsSupported(const Exec &e, int B, int I, int H) {
-    (void)I;
+    if (forwardWideTakes(e, I, H)) return forwardWideClusterTakes(e, H);   // 16-bit activations: the cluster recurrence packs them
     if (e.weightClass != CodeClass::I8 || e.actClass != CodeClass::I8 || e.linearClass == CodeClass::I32) return false;
     if (std::getenv("RXMET_GRU_FWD_GENERIC") != nullptr || std::getenv("RXMET_GRU_FWD_BT") != nullptr) return false;
     const int sms = currentDevice().sms, C = 3 * H;
@@ -1567,7 +1570,7 @@ bool packedFlagsSupported(const Exec &e, int B, int I, int H) {
 void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, size_t workspaceBytes,
                   cudaStream_t st) {
     if (call.stepFlags && !packedFlagsSupported(e, call.B, call.I, call.H))
-        fail(RXMET_ERR_UNSUPPORTED, "packed step flags: these grids or sizes do not take the 8-bit register path");
+        fail(RXMET_ERR_UNSUPPORTED, "packed step flags: these grids or sizes take neither the 8-bit register path nor the cluster recurrence");
     Workspace ws(workspace, workspaceBytes);
     if (call.fpCarrier) {
         forwardFpCarrier(call, e, ws, st);

@@ -30,7 +30,7 @@ struct ForwardQuantCall {
     const rxmet_gru_quant_params *fpCarrier = nullptr;   // set: run the FP32 carrier with these (raw) scales
 };
 
-// Whether forwardQuant can write stepFlags for these parameters and sizes (the register-resident 8-bit path).
+// Whether forwardQuant can write stepFlags for these parameters and sizes (the register-resident 8-bit path, the cluster recurrence).
 bool packedFlagsSupported(const Exec &exec, int B, int I, int H);
 
 // Page-locked host copy of the per-channel block of `exec`, 12 arrays of 3H 32-bit words: effective

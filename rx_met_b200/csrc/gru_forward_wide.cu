@@ -194,21 +194,9 @@ __global__ void __launch_bounds__(kThreads) inputLinearPlanes(const __grid_const
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-struct RecurrentArgs {
-    int T, B, H, HP, kWords;
+struct RecurrentArgs : WideRecurrence {
+    int HP, kWords;
     int weightBytesInSmem;   // size of the shared-memory copy of `words` (WS variant), else 0
-    const uint32_t *words;   // [kWords][3H]
-    const int64_t *addend;   // [3H]
-    const Rescale *rescale;  // [3H]
-    const int16_t *ih;       // [T][B][3H]
-    const int16_t *h0;       // [B][hPad] codes
-    int hPad;
-    const uint32_t *h0Planes;  // [B][2][kWords]
-    float *h;                // [T+1][B][H] dequantized
-    float *v;                // [T][B][4H] dequantized
-    int32_t *hq, *vq;        // optional codes
-    uint8_t *maskHh, *maskGateIn, *maskGateOut, *maskH;
-    const int *poison;       // status word of the tensor-core projection: non-zero turns the hidden outputs into NaN
 };
 
 template <int RB, bool WS>
@@ -512,6 +500,12 @@ void forwardWide(const WideCall &call, const Exec &e, Workspace &ws, cudaStream_
         a.h = call.h; a.v = call.v; a.hq = call.hq; a.vq = call.vq;
         a.maskHh = call.maskHh; a.maskGateIn = call.maskGateIn; a.maskGateOut = call.maskGateOut; a.maskH = call.maskH;
         a.poison = tensorProjection ? l.projStatus : nullptr;
+        a.maskIh = call.maskIh; a.stepBits = call.stepBits;
+        if (forwardWideClusterTakes(e, H)) {
+            forwardWideCluster(a, e, st);
+            return;
+        }
+        RXMET_REQUIRE(call.stepBits == nullptr, "packed step flags need the cluster recurrence");
         const int groupsMax = std::max(1, kThreads / a.HP);
         const int want = std::max(1, (B + smsPerPass() - 1) / smsPerPass());
         int rb = 1;

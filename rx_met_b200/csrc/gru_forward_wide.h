@@ -24,12 +24,34 @@ struct WideCall {
     float *h, *v;
     int32_t *hq, *vq;                   // optional
     uint8_t *maskIh, *maskHh, *maskGateIn, *maskGateOut, *maskH;  // optional keep flags
+    uint16_t *stepBits;                 // optional packed flags
 };
 
 // Weight grids of at most 8 bits, x / h grids of 9..16 bits, linear grids of at most 16 bits, H <= 512.
 bool forwardWideTakes(const Exec &exec, int I, int H);
 size_t forwardWideExtraBytes(int T, int B, int I, int H);
 void forwardWide(const WideCall &call, const Exec &exec, Workspace &workspace, cudaStream_t stream);
+
+// Operands of the recurrence alone, after the input projection.
+struct WideRecurrence {
+    int T, B, H;
+    const uint32_t *words;     // [kWords][3H]: four recurrent weight bytes along K
+    const int64_t *addend;     // [3H]
+    const Rescale *rescale;    // [3H]
+    const int16_t *ih;         // [T][B][3H]
+    const int16_t *h0;         // [B][hPad] codes
+    int hPad;
+    const uint32_t *h0Planes;  // [B][2][kWords]
+    float *h, *v;              // [T+1][B][H], [T][B][4H] dequantized
+    int32_t *hq, *vq;          // optional codes
+    uint8_t *maskHh, *maskGateIn, *maskGateOut, *maskH;
+    const uint8_t *maskIh;     // with stepBits: the input projection's keep flags
+    uint16_t *stepBits;        // optional [T][B][H]: the 13 flags of an element packed (instead of the byte masks)
+    const int *poison;         // status word of the tensor-core projection: non-zero turns the hidden outputs into NaN
+};
+// The recurrence over thread-block clusters (gru_forward_cluster.cu), and whether it takes the shape and the parameters.
+bool forwardWideClusterTakes(const Exec &exec, int H);
+void forwardWideCluster(const WideRecurrence &r, const Exec &exec, cudaStream_t stream);
 
 }  // namespace gru
 }  // namespace rxmet

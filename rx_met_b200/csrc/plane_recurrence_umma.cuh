@@ -1,0 +1,309 @@
+// One step after another of a recurrence on byte-plane codes (QuantGRU W8 / A16, QuantLSTM W4 / W8 with 8- or 16-bit
+// activations) over a thread-block cluster, the product W_hh h on tcgen05 kind::i8.
+//
+// The H / U CTAs of a cluster advance ROWS batch rows together; a CTA owns U hidden units.  Their gate channels are the
+// accumulator lanes - tiles of 128 lanes = 4 quarters (gates; a GRU leaves the fourth empty) x 32 units - and their
+// weights stay in tensor memory for the whole sequence as the A operand (lane = channel, column = four bytes along K).
+// The hidden codes of the rows, split into unsigned byte planes, are the B operand: plane p of row r is accumulator column
+// p ROWS + r, so the weights are read once for both planes.  Per step:
+//   product -> phase A (warp = quarter, lane = unit: the operator's linear stage and, where it likes, its gate) -> exchange
+//   through shared memory inside the four warps of a tile -> phase B (lane = unit, a quarter of the rows per warp: the
+//   cell) -> the new codes of the CTA's units, staged in operand layout, travel as one bulk copy to every CTA.
+//
+// Bound: the chain of one step.  At H = 256 and 8 rows it is about 0.3 k cycles of tcgen05, 0.4 k of copy latency, 0.2 k of
+// barriers and the operator's epilogue; the operand in shared memory instead of tensor memory or an MMA issue loop
+// that is not warp-uniform double the first part.
+//
+// Synchronisation: operand and staging buffers by step parity; a CTA sends the codes of step t only after it has those of
+// step t - 1 of every peer, and a peer sends those only after its product of step t - 1 is complete: the operand
+// buffer of step t (= t - 2) and the staging buffer it came from are free by then.  Every wait is bounded; a thread whose
+// wait gave up waits no more and reports it to the operator, which turns its outputs into NaN.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+
+#include "cluster_device.cuh"
+#include "common.h"
+#include "plane_proj_umma.cuh"
+
+namespace rxmet {
+namespace planerec {
+
+using namespace umma;
+
+// D += A B with A (signed bytes) in tensor memory
+__device__ __forceinline__ void mmaI8TmemA(uint32_t tmemD, uint32_t tmemA, uint64_t descB, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t"
+        "}\n"
+        :
+        : "r"(tmemD), "r"(tmemA), "l"(descB), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+}
+__device__ __forceinline__ void tmemStore4(uint32_t addr, uint32_t v0, uint32_t v1, uint32_t v2, uint32_t v3) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "r"(v0), "r"(v1), "r"(v2), "r"(v3) : "memory");
+}
+__device__ __forceinline__ void tmemLoad4(uint32_t addr, uint32_t *r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+
+constexpr uint32_t powerOfTwoFrom(uint32_t n) {
+    uint32_t p = 32;
+    while (p < n) p *= 2;
+    return p;
+}
+
+template <int H, int U, int ROWS, int PLANES>
+struct Geometry {
+    static constexpr int kCtas = H / U, kTiles = U / 32;
+    static constexpr int kWarps = ROWS * kTiles >= 16 ? 16 : 8;   // of the epilogue; one more warp issues products and copies
+    static constexpr int kThreads = 32 * (kWarps + 1);
+    static constexpr int kRowGroups = kWarps / (4 * kTiles);   // warps that share the rows of a tile's quarter
+    static constexpr int kRowsA = ROWS / kRowGroups;            // rows of a lane in phase A
+    static constexpr int kRowsB = kRowsA / 4;                   // cells of a lane in phase B
+    static_assert(kRowsA % 4 == 0 && kRowsA * kRowGroups == ROWS, "rows divide into quads");
+    static constexpr int kPadK = (H + 31) / 32 * 32;
+    static constexpr int kCols = (PLANES * ROWS + 15) / 16 * 16;          // accumulator columns of a tile
+    static constexpr uint32_t kColsA = kPadK / 4;                          // tensor-memory columns of its weights
+    static constexpr uint32_t kTmemCols = powerOfTwoFrom(kTiles * (kCols + kColsA));
+    static_assert(kTmemCols <= 512, "tensor memory has 512 columns");
+    static constexpr uint32_t kGroupStride = kCols * 16;                   // next 16 bytes along K
+    static constexpr uint32_t kOperandBytes = kPadK / 16 * kGroupStride;
+    static constexpr uint32_t kSlabBytes = U / 16 * kGroupStride;          // this CTA's units
+    static constexpr uint32_t kExchangeBytes = kTiles * 4 * ROWS * 32 * 4;
+    static constexpr size_t kSharedBytes = 2 * kOperandBytes + 2 * kSlabBytes + kExchangeBytes;
+};
+
+struct Problem {
+    int T, B;
+    const uint32_t *h0;   // [B][PLANES][H padded to 16, / 4] words of four code bytes: the initial state
+};
+
+// Cell contract (device functions; `at` = first row of the step in the [T][B] arrays, `Shared` is placed in shared memory):
+//   kGates                                                  quarters in use
+//   uint32_t weightWord(gate, unit, kw)                     four weight bytes along K, 0 for an empty quarter
+//   void init(Shared &, tid, threads)                       fills Shared
+//   Lane lane(Shared, gate, unit)                           constants of phase A
+//   void begin(Shared, State &, row, unit)                  state of one cell of phase B from h0
+//   void fetch(Fetch &, at, row, gate, unit), fetchB(FetchB &, at, row, unit)     operands of a step, asked for before the product is awaited
+//   uint32_t linear<STRIDE>(Shared, Lane, Fetch, acc, at, row, gate, unit, live)    phase A; plane p of the sum at acc[p STRIDE]
+//   uint32_t cell(Shared, State &, FetchB, v[4])            phase B: new code - grid minimum
+//   void store(Shared, State, FetchB, at, row, unit, good)       outputs of the step; good = false: make them NaN
+//   void finish(Shared, State, row, unit, good)             after the last step
+template <class Cell, int H, int U, int ROWS, int PLANES>
+__global__ void __launch_bounds__(Geometry<H, U, ROWS, PLANES>::kThreads, 1)
+planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c) {
+    using G = Geometry<H, U, ROWS, PLANES>;
+    constexpr int MT = G::kTiles, NC = G::kCtas;
+    extern __shared__ __align__(128) uint8_t smemR[];
+    __shared__ __align__(8) uint64_t productBar, codeBar[2];
+    __shared__ uint32_t tmemSlot;
+    __shared__ volatile int failed;   // the control warp's wait gave up
+    __shared__ typename Cell::Shared shared;
+    uint8_t *operand = smemR;                                                // [2][K / 16][kCols][16]
+    uint8_t *staging = operand + 2 * G::kOperandBytes;                       // [2][U / 16][kCols][16]
+    uint32_t *exchange = reinterpret_cast<uint32_t *>(staging + 2 * G::kSlabBytes);   // [tile][row group][4 gates][rowsA][32 units]
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
+    const int quarter = warp & 3, tile = (warp >> 2) % MT, rowGroup = (warp >> 2) / MT;
+    const uint32_t rank = cluster::rank();
+    const int unit = static_cast<int>(rank) * U + tile * 32 + lane;
+    const int b0 = static_cast<int>(blockIdx.x) / NC * ROWS;
+    const int rowA = b0 + rowGroup * G::kRowsA, rowB = rowA + quarter * G::kRowsB;   // first rows of the two phases
+
+    if (tid == 0) {
+        failed = 0;
+        cluster::initBarrier(&productBar, 1);
+        for (int i = 0; i < 2; ++i) cluster::initBarrier(&codeBar[i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (int i = 0; i < 2; ++i) cluster::arriveExpect(smemAddr(&codeBar[i]), NC * G::kSlabBytes);
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(&tmemSlot)), "n"(G::kTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    c.init(shared, tid, G::kThreads);
+    for (uint32_t i = tid; i < (2 * G::kOperandBytes + 2 * G::kSlabBytes) / 16; i += G::kThreads)
+        reinterpret_cast<uint4 *>(operand)[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    constexpr int kWords = (H + 15) / 16 * 4;   // of a plane row
+    for (int i = tid; i < ROWS * PLANES * (kWords / 4); i += G::kThreads) {
+        const int kg = i % (kWords / 4), n = i / (kWords / 4), pl = n / ROWS, r = n - pl * ROWS;
+        if (b0 + r < p.B)
+            *reinterpret_cast<uint4 *>(operand + kg * G::kGroupStride + n * 16) =
+                *reinterpret_cast<const uint4 *>(p.h0 + (static_cast<size_t>(b0 + r) * PLANES + pl) * kWords + 4 * kg);
+    }
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmemSlot, 0), tmemWeights = tmem + MT * G::kCols;
+    const uint32_t quarterBase = static_cast<uint32_t>(32 * quarter) << 16;
+    if (rowGroup == 0 && warp < G::kWarps)
+        for (int kw = 0; kw < G::kPadK / 4; kw += 4) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) w[e] = kw + e < kWords ? c.weightWord(quarter, unit, kw + e) : 0u;
+            tmemStore4(tmemWeights + quarterBase + tile * G::kColsA + kw, w[0], w[1], w[2], w[3]);
+        }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    cluster::barrierAll();   // every CTA's barriers are armed before anyone sends
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+    constexpr uint32_t kIdesc = planeproj::instructionDescriptor(G::kCols);
+    bool alive = true;   // false once one of this thread's waits gave up
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+        if (alive) alive = waitPhase(bar, parity);
+    };
+    if (warp == G::kWarps) {
+        // ---- control warp: products and copies; lane d sends to CTA d
+        const uint32_t peer = static_cast<uint32_t>(lane) % NC;
+        const uint32_t sendTo = cluster::remote(smemAddr(operand), peer) + rank * G::kSlabBytes;
+        const uint32_t sendBar = cluster::remote(smemAddr(&codeBar[0]), peer);
+        const uint64_t descB0 = operandDescriptor(smemAddr(operand), G::kGroupStride, kCore);
+#pragma unroll 1
+        for (int t = 0; t < p.T; ++t) {
+            const uint32_t bar = smemAddr(&codeBar[0]) + (t & 1) * 8;
+            if (t > 0) wait(bar, ((t - 1) >> 1) & 1);
+            if (electOne()) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t descB = descB0 + static_cast<uint64_t>((t & 1) * (G::kOperandBytes >> 4));
+#pragma unroll
+                for (int m = 0; m < MT; ++m)
+#pragma unroll
+                    for (int ks = 0; ks < G::kPadK / 32; ++ks)
+                        mmaI8TmemA(tmem + m * G::kCols, tmemWeights + m * G::kColsA + ks * 8,
+                                   descB + static_cast<uint64_t>(ks * ((2 * G::kGroupStride) >> 4)), kIdesc, ks > 0 ? 1u : 0u);
+                commitTo(smemAddr(&productBar));
+                if (t > 0) cluster::arriveExpect(bar, NC * G::kSlabBytes);   // for step t + 2
+            }
+            __syncwarp();
+            if (!alive) failed = 1;
+            __syncthreads();   // the codes of step t are staged
+            if (t + 1 < p.T && lane < NC)
+                cluster::copyTo(sendTo + ((t + 1) & 1) * G::kOperandBytes, smemAddr(staging) + (t & 1) * G::kSlabBytes, G::kSlabBytes,
+                                sendBar + ((t + 1) & 1) * 8);
+        }
+    } else {
+        const typename Cell::Lane mine = c.lane(shared, quarter, unit);
+        typename Cell::State state[G::kRowsB];
+#pragma unroll
+        for (int i = 0; i < G::kRowsB; ++i)
+            if (rowB + i < p.B) c.begin(shared, state[i], rowB + i, unit);
+        const uint32_t column = tmem + quarterBase + tile * G::kCols + rowGroup * G::kRowsA;
+        uint32_t *exchangeTile = exchange + (tile * G::kRowGroups + rowGroup) * (4 * G::kRowsA * 32) + lane;
+        uint8_t *stageMine = staging + (tile * 2 + (lane >> 4)) * G::kGroupStride + (rowB - b0) * 16 + (lane & 15);
+#pragma unroll 1
+        for (int t = 0; t < p.T; ++t) {
+            const size_t at = static_cast<size_t>(t) * p.B;   // first row of the step in the [T][B] arrays
+            typename Cell::Fetch inA[G::kRowsA];
+            typename Cell::FetchB inB[G::kRowsB];
+#pragma unroll
+            for (int r = 0; r < G::kRowsA; ++r)
+                if (rowA + r < p.B) c.fetch(inA[r], at, rowA + r, quarter, unit);
+#pragma unroll
+            for (int i = 0; i < G::kRowsB; ++i)
+                if (rowB + i < p.B) c.fetchB(inB[i], at, rowB + i, unit);
+            wait(smemAddr(&productBar), t & 1);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            uint32_t acc[PLANES * G::kRowsA];
+#pragma unroll
+            for (int pl = 0; pl < PLANES; ++pl)
+#pragma unroll
+                for (int r = 0; r < G::kRowsA; r += 4) tmemLoad4(column + pl * ROWS + r, acc + pl * G::kRowsA + r);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (quarter < Cell::kGates) {
+#pragma unroll
+                for (int r = 0; r < G::kRowsA; ++r)
+                    exchangeTile[(quarter * G::kRowsA + r) * 32] =
+                        c.template linear<G::kRowsA>(shared, mine, inA[r], acc + r, at, rowA + r, quarter, unit, rowA + r < p.B);
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(1 + (warp >> 2)) : "memory");   // the four quarters of this tile and row group
+#pragma unroll
+            for (int i = 0; i < G::kRowsB; ++i) {
+                if (rowB + i >= p.B) continue;
+                uint32_t v[4];
+#pragma unroll
+                for (int g = 0; g < 4; ++g) v[g] = g < Cell::kGates ? exchangeTile[(g * G::kRowsA + quarter * G::kRowsB + i) * 32] : 0u;
+                const uint32_t u = c.cell(shared, state[i], inB[i], v);
+                uint8_t *dst = stageMine + (t & 1) * G::kSlabBytes + i * 16;
+                if (PLANES == 2) {
+                    dst[0] = static_cast<uint8_t>(u >> 8);
+                    dst[ROWS * 16] = static_cast<uint8_t>(u);
+                } else {
+                    dst[0] = static_cast<uint8_t>(u);
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncthreads();
+            // what nobody waits for leaves while the codes travel and the next product runs
+#pragma unroll
+            for (int i = 0; i < G::kRowsB; ++i)
+                if (rowB + i < p.B) c.store(shared, state[i], inB[i], at, rowB + i, unit, alive && !failed);
+        }
+#pragma unroll
+        for (int i = 0; i < G::kRowsB; ++i)
+            if (rowB + i < p.B) c.finish(shared, state[i], rowB + i, unit, alive && !failed);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(G::kTmemCols) : "memory");
+    cluster::barrierAll();   // nobody leaves while a peer may still copy into its shared memory
+}
+
+// Launches a variant with its clusters; false when the device holds none of them.
+template <class Cell, int H, int U, int ROWS, int PLANES>
+bool launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t st) {
+    using G = Geometry<H, U, ROWS, PLANES>;
+    const auto kernel = planeRecurrence<Cell, H, U, ROWS, PLANES>;
+    ensureDynamicSmem(reinterpret_cast<const void *>(kernel), G::kSharedBytes);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>((p.B + ROWS - 1) / ROWS * G::kCtas));
+    cfg.blockDim = dim3(G::kThreads);
+    cfg.dynamicSmemBytes = G::kSharedBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = G::kCtas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    {
+        KernelTimer timer__(name, st);
+        RXMET_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, cell));
+    }
+    afterLaunch(name);
+    return true;
+}
+
+// Rows of a cluster among `choices`: as few as let all clusters of the pass run at the same time (a step costs about
+// 1 + rows / 32 of the chain of a short step, a second wave costs the whole chain again).
+template <class Cell, int H, int U, int PLANES, int... ROWS>
+void launchBest(const char *name, const Problem &p, const Cell &cell, cudaStream_t st) {
+    double bestCost = 1e30;
+    int best = 0;
+    (
+        [&] {
+            using G = Geometry<H, U, ROWS, PLANES>;
+            const int resident = std::max(1, residentClusters(reinterpret_cast<const void *>(planeRecurrence<Cell, H, U, ROWS, PLANES>), G::kCtas,
+                                                              G::kThreads, G::kSharedBytes) / concurrentPasses());
+            const int clusters = (p.B + ROWS - 1) / ROWS, waves = (clusters + resident - 1) / resident;
+            const double cost = waves * (1.0 + ROWS / 32.0);
+            if (cost < bestCost) { bestCost = cost; best = ROWS; }
+        }(),
+        ...);
+    (
+        [&] {
+            if (best == ROWS) launch<Cell, H, U, ROWS, PLANES>(name, p, cell, st);
+        }(),
+        ...);
+}
+
+}  // namespace planerec
+}  // namespace rxmet
