@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstdint>
+#include <type_traits>
 
 #include "common.h"
 #include "gru_device.cuh"
@@ -24,9 +25,10 @@ namespace {
 constexpr int kBuckets = 256;
 
 struct FastLut {
-    int4 segment[kSegments];          // q_b, n_bx, term_c, threshold
-    uint16_t bucket[kBuckets];        // segment at the bucket's first code | segment behind its threshold << 8
+    int4 segment[kSegments];          // q_b, n_bx, term_c, 2^(n_bx - 1) - 1
+    uint2 bucket[kBuckets];           // the bucket's threshold; byte offset of the segment before it | of the one behind it << 16
 };
+static_assert(sizeof(int4) * kSegments == 256, "activation() addresses the buckets behind the segments");
 
 // round_half_even(p / 2^n) for 1 <= n <= 31, low 32 bits: (p + 2^(n-1) - 1 + odd(floor(p / 2^n))) >> n on two words.
 __device__ __forceinline__ int32_t roundShift31(int64_t p, int n, uint32_t roundAdd) {
@@ -65,12 +67,17 @@ struct CellScalars {
 // What a training forward saves of the clamp flags.
 enum class Flags { None, Bytes, Packed };
 
-template <int H, Flags FLAGS>
+// WIDTH: the hidden size where it is a compile-time constant (its multiples are address immediates then), else 0.
+template <Flags FLAGS, int WIDTH>
 struct GruPlaneCell {
     static constexpr int kGates = 3;
+    static constexpr bool kSaves = false, kFull = WIDTH != 0;
+    static constexpr int kChunk = 4;
     CellScalars s;
     FastLut luts[3];
+    int width;
     size_t B;
+    __device__ __forceinline__ int hidden() const { return WIDTH ? WIDTH : width; }
     const uint32_t *words;    // [kWords][3H]
     const int64_t *addend;    // [3H]
     const Rescale *rescale;   // [3H]
@@ -84,9 +91,7 @@ struct GruPlaneCell {
     uint16_t *stepBits;
     const int *poison;        // status word of the tensor-core projection: non-zero turns the hidden outputs into NaN
 
-    struct Shared {
-        FastLut luts[3];
-    };
+    size_t sharedBytes() const { return sizeof(luts); }
     struct Lane {
         int64_t addend, roundAdd;
         int32_t mult, shift;
@@ -97,21 +102,24 @@ struct GruPlaneCell {
         uint32_t keep;   // bits 0..2 gate output z, r, n; 3..5 gate input; 6..8 hh linear; 12 hidden state
     };
     struct Fetch {};
+    struct Saved {};
     struct FetchB {
         int32_t ih[3];
         uint32_t keepIh[3];
     };
 
     __device__ __forceinline__ uint32_t weightWord(int gate, int unit, int kw) const {
+        const int H = hidden();
         return gate < 3 ? __ldg(words + static_cast<size_t>(kw) * 3 * H + gate * H + unit) : 0u;
     }
-    __device__ __forceinline__ void init(Shared &sh, int tid, int threads) const {
-        for (int i = tid; i < static_cast<int>(sizeof(Shared) / 4); i += threads)
-            reinterpret_cast<uint32_t *>(&sh)[i] = reinterpret_cast<const uint32_t *>(luts)[i];
+    __device__ __forceinline__ void init(uint8_t *shared, int tid, int threads) const {
+        for (int i = tid; i < static_cast<int>(sizeof(luts) / 4); i += threads)
+            reinterpret_cast<uint32_t *>(shared)[i] = reinterpret_cast<const uint32_t *>(luts)[i];
     }
-    __device__ __forceinline__ Lane lane(const Shared &, int gate, int unit) const {
+    __device__ __forceinline__ Lane lane(uint32_t, int gate, int unit, bool real) const {
+        const int H = hidden();
         Lane l{0, 0, 0, 1, false};
-        if (gate < 3) {
+        if (gate < 3 && real) {
             const Rescale r = rescale[gate * H + unit];
             l.addend = addend[gate * H + unit];
             l.mult = r.mult;
@@ -124,7 +132,8 @@ struct GruPlaneCell {
     __device__ __forceinline__ float scaleH(bool alive) const {
         return (!alive || (poison && *poison)) ? __int_as_float(0x7fc00000) : s.effH;
     }
-    __device__ __forceinline__ void begin(const Shared &, State &st, int row, int unit) const {
+    __device__ __forceinline__ void begin(uint32_t, State &st, int row, int unit) const {
+        const int H = hidden();
         st.h = h0[static_cast<size_t>(row) * hPad + unit];
         const size_t o = static_cast<size_t>(row) * H + unit;
         h[o] = static_cast<float>(st.h - s.zpH) * scaleH(true);
@@ -132,6 +141,7 @@ struct GruPlaneCell {
     }
     __device__ __forceinline__ void fetch(Fetch &, size_t, uint32_t, int, int) const {}
     __device__ __forceinline__ void fetchB(FetchB &f, size_t at, uint32_t row, int unit) const {
+        const int H = hidden();
         const int16_t *from = ih + at * (3 * H) + (row * (3 * H) + unit);
 #pragma unroll
         for (int g = 0; g < 3; ++g) f.ih[g] = __ldg(from + g * H);
@@ -143,7 +153,7 @@ struct GruPlaneCell {
     }
     // hh linear code, its keep flag in bit 0
     template <int STRIDE>
-    __device__ __forceinline__ uint32_t linear(const Shared &, const Lane &l, const Fetch &, const uint32_t *acc, size_t, uint32_t, int, int, bool) const {
+    __device__ __forceinline__ uint32_t linear(uint32_t, const Lane &l, const Fetch &, const uint32_t *acc, Saved &) const {
         const int64_t total = (static_cast<int64_t>(static_cast<int32_t>(acc[0])) << 8) + static_cast<int32_t>(acc[STRIDE]) + l.addend;
         const int64_t prod = total * l.mult;
         int32_t res;
@@ -153,19 +163,25 @@ struct GruPlaneCell {
         const int32_t code = clampCode(res + s.zpHh, s.loHh, s.hiHh, keep);
         return static_cast<uint32_t>(code * 2 + keep);
     }
-    __device__ __forceinline__ int32_t activation(const FastLut &lut, int g, int32_t qx, uint32_t &keepOut) const {
-        const uint32_t b = lut.bucket[static_cast<uint32_t>(qx - s.loIn[g]) >> s.bucketShift[g]];
-        const uint32_t before = b & 0xffu;
-        const uint32_t seg = qx < lut.segment[before].w ? before : b >> 8;
-        const int4 e = lut.segment[seg];
+    __device__ __forceinline__ int32_t activation(uint32_t shared, int g, int32_t qx, uint32_t &keepOut) const {
+        const uint32_t lut = shared + g * static_cast<uint32_t>(sizeof(FastLut));
+        int32_t threshold;
+        uint32_t segments;
+        asm("ld.shared.v2.u32 {%0, %1}, [%2];"
+            : "=r"(threshold), "=r"(segments)
+            : "r"(lut + 256 + (static_cast<uint32_t>(qx - s.loIn[g]) >> s.bucketShift[g]) * 8));
+        int4 e;
+        asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+            : "=r"(e.x), "=r"(e.y), "=r"(e.z), "=r"(e.w)
+            : "r"(lut + (qx < threshold ? segments & 0xffffu : segments >> 16)));
         const int64_t bx = static_cast<int64_t>(e.x) * (qx - s.zpX[g]);
-        const int32_t y = roundShift31(bx, e.y, (1u << (e.y - 1)) - 1u) + e.z;
+        const int32_t y = roundShift31(bx, e.y, static_cast<uint32_t>(e.w)) + e.z;
         uint8_t keep;
         const int32_t code = clampCode(y, s.loOut[g], s.hiOut[g], keep);
         keepOut |= static_cast<uint32_t>(keep) << g;
         return code;
     }
-    __device__ __forceinline__ uint32_t cell(const Shared &sh, State &st, const FetchB &in, const uint32_t (&v)[4]) const {
+    __device__ __forceinline__ uint32_t cell(uint32_t shared, State &st, const FetchB &in, const uint32_t (&v)[4]) const {
         uint32_t keep = 0;
         int32_t hh[3];
 #pragma unroll
@@ -178,14 +194,14 @@ struct GruPlaneCell {
             uint8_t k;
             const int32_t pre = clampCode(apply(in.ih[g] - s.zpIh, s.ihTo[g]) + apply(hh[g] - s.zpHh, s.hhTo[g]) + s.zpIn[g], s.loIn[g], s.hiIn[g], k);
             keep |= static_cast<uint32_t>(k) << (3 + g);
-            st.code[g] = activation(sh.luts[g], g, pre, keep);
+            st.code[g] = activation(shared, g, pre, keep);
         }
         {
             uint8_t k;
             const int64_t prod = static_cast<int64_t>(st.code[1] - s.zpOut[1]) * (hh[2] - s.zpHh);
             const int32_t pre = clampCode(apply(in.ih[2] - s.zpIh, s.ihTo[2]) + apply(prod, s.rhToNew) + s.zpIn[2], s.loIn[2], s.hiIn[2], k);
             keep |= static_cast<uint32_t>(k) << 5;
-            st.code[2] = activation(sh.luts[2], 2, pre, keep);
+            st.code[2] = activation(shared, 2, pre, keep);
         }
         {
             uint8_t k;
@@ -198,7 +214,8 @@ struct GruPlaneCell {
         st.keep = keep;
         return static_cast<uint32_t>(st.h - s.loH);
     }
-    __device__ __forceinline__ void store(const Shared &, const State &st, const FetchB &in, size_t at, uint32_t row, int unit, bool good) const {
+    __device__ __forceinline__ void store(const State &st, const FetchB &in, size_t at, uint32_t row, int unit, bool good) const {
+        const int H = hidden();
         const uint32_t mine = row * H + unit, mine3 = row * (3 * H) + unit;
         h[(at + B) * H + mine] = static_cast<float>(st.h - s.zpH) * scaleH(good);
         float *vRow = v + at * (4 * H) + (row * (4 * H) + unit);
@@ -231,7 +248,8 @@ struct GruPlaneCell {
             }
         }
     }
-    __device__ __forceinline__ void finish(const Shared &, const State &, int, int, bool) const {}
+    __device__ __forceinline__ void storeLinear(const Saved &, size_t, uint32_t, int, int) const {}
+    __device__ __forceinline__ void finish(const State &, int, int, bool) const {}
 };
 
 bool ready(const Rescale &r, ReadyRescale &out) {
@@ -257,18 +275,19 @@ bool ready(const Lut &lut, int32_t lo, int32_t hi, FastLut &out, int32_t &bucket
     };
     for (int i = 0; i < kSegments; ++i) {
         if (lut.n_bx[i] < 1 || lut.n_bx[i] > 31) return false;
-        out.segment[i] = make_int4(lut.q_b[i], lut.n_bx[i], lut.term_c[i], i < kSegments - 1 ? lut.threshold[i] : INT32_MAX);
+        out.segment[i] = make_int4(lut.q_b[i], lut.n_bx[i], lut.term_c[i], (1 << (lut.n_bx[i] - 1)) - 1);
     }
     for (int b = 0; b < kBuckets; ++b) {
         const int64_t first = lo + (static_cast<int64_t>(b) << bucketShift), last = std::min<int64_t>(first + (int64_t{1} << bucketShift) - 1, hi);
         if (first > hi) {
-            out.bucket[b] = 0;
+            out.bucket[b] = make_uint2(0u, 0u);
             continue;
         }
         const int s0 = segmentOf(first), s1 = segmentOf(last);
         // only the threshold of s0 may lie in (first, last]
         if (s1 != s0 && segmentOf(lut.threshold[s0]) != s1) return false;
-        out.bucket[b] = static_cast<uint16_t>(s0 | (s1 << 8));
+        const int32_t threshold = s0 == s1 ? INT32_MAX : lut.threshold[s0];
+        out.bucket[b] = make_uint2(static_cast<uint32_t>(threshold), static_cast<uint32_t>(16 * s0) | (static_cast<uint32_t>(16 * s1) << 16));
     }
     return true;
 }
@@ -279,25 +298,31 @@ struct Prepared {
     FastLut luts[3];
 };
 
-template <int H, Flags FLAGS>
+template <int HP, Flags FLAGS, int WIDTH>
 void launchFor(const WideRecurrence &r, const Prepared &prepared, cudaStream_t st) {
-    constexpr int U = H % 64 == 0 ? 64 : 32;
-    GruPlaneCell<H, FLAGS> cell{};
+    using Cell = GruPlaneCell<FLAGS, WIDTH>;
+    Cell cell{};
     cell.s = prepared.s;
     std::copy(prepared.luts, prepared.luts + 3, cell.luts);
+    cell.width = r.H;
     cell.B = static_cast<size_t>(r.B);
     cell.words = r.words; cell.addend = r.addend; cell.rescale = r.rescale; cell.ih = r.ih; cell.h0 = r.h0; cell.hPad = r.hPad;
     cell.h = r.h; cell.v = r.v; cell.hq = r.hq; cell.vq = r.vq;
     cell.maskHh = r.maskHh; cell.maskGateIn = r.maskGateIn; cell.maskGateOut = r.maskGateOut; cell.maskH = r.maskH;
     cell.maskIh = r.maskIh; cell.stepBits = r.stepBits;
     cell.poison = r.poison;
-    planerec::launchBest<GruPlaneCell<H, FLAGS>, H, U, 2, 8, 16>("recurrentForward", planerec::Problem{r.T, r.B, r.h0Planes}, cell, st);
+    planerec::launchBest<Cell, HP, HP < 64 ? HP : 64, 2, 32, 8, 16>("recurrentForward", planerec::Problem{r.T, r.B, r.H, r.h0Planes}, cell, st);
 }
-template <int H>
+template <int HP>
 void launchFor(const WideRecurrence &r, const Prepared &prepared, cudaStream_t st) {
-    if (r.stepBits) launchFor<H, Flags::Packed>(r, prepared, st);
-    else if (r.maskHh || r.maskGateIn) launchFor<H, Flags::Bytes>(r, prepared, st);
-    else launchFor<H, Flags::None>(r, prepared, st);
+    auto run = [&](auto width) {
+        constexpr int kWidth = decltype(width)::value;
+        if (r.stepBits) launchFor<HP, Flags::Packed, kWidth>(r, prepared, st);
+        else if (r.maskHh || r.maskGateIn) launchFor<HP, Flags::Bytes, kWidth>(r, prepared, st);
+        else launchFor<HP, Flags::None, kWidth>(r, prepared, st);
+    };
+    if (r.H == HP) run(std::integral_constant<int, HP>{});
+    else run(std::integral_constant<int, 0>{});
 }
 
 bool prepare(const Exec &e, Prepared &cell) {
@@ -328,22 +353,17 @@ bool prepare(const Exec &e, Prepared &cell) {
 
 bool forwardWideClusterTakes(const Exec &e, int H) {
     Prepared prepared;
-    return H % 32 == 0 && H <= 256 && prepare(e, prepared);
+    return H <= 256 && prepare(e, prepared);
 }
 
 void forwardWideCluster(const WideRecurrence &r, const Exec &e, cudaStream_t st) {
     Prepared prepared;
     prepare(e, prepared);
-    switch (r.H) {
-        case 32: launchFor<32>(r, prepared, st); break;
-        case 64: launchFor<64>(r, prepared, st); break;
-        case 96: launchFor<96>(r, prepared, st); break;
-        case 128: launchFor<128>(r, prepared, st); break;
-        case 160: launchFor<160>(r, prepared, st); break;
-        case 192: launchFor<192>(r, prepared, st); break;
-        case 224: launchFor<224>(r, prepared, st); break;
-        default: launchFor<256>(r, prepared, st); break;
-    }
+    if (r.H <= 32) launchFor<32>(r, prepared, st);
+    else if (r.H <= 64) launchFor<64>(r, prepared, st);
+    else if (r.H <= 128) launchFor<128>(r, prepared, st);
+    else if (r.H <= 192) launchFor<192>(r, prepared, st);
+    else launchFor<256>(r, prepared, st);
 }
 
 }  // namespace gru

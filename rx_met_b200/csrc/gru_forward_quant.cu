@@ -1557,7 +1557,8 @@ void forwardFpCarrier(const ForwardQuantCall &call, const Exec &e, Workspace &ws
 }
 
 bool packedFlagsSupported(const Exec &e, int B, int I, int H) {
-    if (forwardWideTakes(e, I, H)) return forwardWideClusterTakes(e, H);   // 16-bit activations: the cluster recurrence packs them
+    // 16-bit activations: the cluster recurrence packs them, for widths whose backward reads them
+    if (forwardWideTakes(e, I, H)) return (H <= 128 || H % 32 == 0) && forwardWideClusterTakes(e, H);
     if (e.weightClass != CodeClass::I8 || e.actClass != CodeClass::I8 || e.linearClass == CodeClass::I32) return false;
     if (std::getenv("RXMET_GRU_FWD_GENERIC") != nullptr || std::getenv("RXMET_GRU_FWD_BT") != nullptr) return false;
     const int sms = currentDevice().sms, C = 3 * H;

@@ -1,0 +1,237 @@
+// Wide QuantLSTM recurrence (weights <= 8 bits, activations of 9 to 16 bits, H <= 512) over thread-block clusters: the float
+// q-carrier cell on top of plane_recurrence_umma.cuh.
+//
+// Every float rounding that decides a code is the reference's, value for value; what is cheaper than in the one-CTA kernels:
+//  - activations come from the compact tables (a line per segment and a bit per input) in shared memory: two shared loads and
+//    about fifteen instructions, where the full tables are gathers of one sector per lane from L2 - they bounded the large
+//    batches and put two L2 round trips into the chain of every step;
+//  - sums that provably fit 32 bits are combined in one multiply-add and converted once;
+//  - rounding to an integer that is clamped to a grid below 2^22 adds and subtracts 1.5 * 2^23 (clamp first: the limits are
+//    integers, so the order does not matter; a training forward clamps one step wider, which keeps the clamp flags).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#include "common.h"
+#include "lstm_device.cuh"
+#include "lstm_kernels.h"
+#include "plane_recurrence_umma.cuh"
+
+namespace rxmet {
+namespace lstm {
+
+constexpr float kRoundMagic = 12582912.0f;   // 1.5 * 2^23
+__device__ __forceinline__ float roundSmall(float x) { return __fadd_rn(__fadd_rn(x, kRoundMagic), -kRoundMagic); }
+__device__ __forceinline__ float clampF(float x, float lo, float hi) { return fminf(fmaxf(x, lo), hi); }
+
+// Addresses and constants of one compact table, ready for lookup().
+struct TableView {
+    uint32_t segments, bits;   // shared addresses, moved by the exponent bits that an index carries
+    float toIndex;             // x + toIndex = 2^23 + index
+    float outLo, outHi;
+};
+__device__ __forceinline__ float lookup(const TableView &v, int segShift, float x, uint32_t &index) {
+    index = __float_as_uint(__fadd_rn(x, v.toIndex));
+    float slope, intercept;
+    asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(slope), "=f"(intercept) : "r"(v.segments + ((index >> segShift) << 3)));
+    uint32_t word;
+    asm("ld.shared.u32 %0, [%1];" : "=r"(word) : "r"(v.bits + ((index >> 5) << 2)));
+    float y = roundSmall(__fmaf_rn(slope, x, intercept));
+    if ((word >> (index & 31u)) & 1u) y = __fadd_rn(y, 1.0f);
+    return clampF(y, v.outLo, v.outHi);
+}
+
+// WIDTH: the hidden size where it is a compile-time constant, else 0.
+template <bool TRAIN, int WIDTH = 0>
+struct LstmPlaneCell {
+    static constexpr int kGates = 4;
+    static constexpr bool kSaves = TRAIN, kFull = WIDTH != 0;
+    static constexpr int kChunk = TRAIN ? 4 : 16;
+    ScalarExec s;
+    int width, kWords;
+    __device__ __forceinline__ int hidden() const { return WIDTH ? WIDTH : width; }
+    size_t B;
+    int segShift, tableBytes;
+    int segOffset[kTables], bitOffset[kTables], flagBelow[kTables], flagFrom[kTables];
+    float inLo[kTables], outLo[kTables], outHi[kTables];
+    const uint8_t *tables;
+    const uint2 *words;        // [2 gate pairs][kWords][H]: (x, y) = gates (2 * pair, 2 * pair + 1)
+    const int64_t *addend;     // [4H]
+    const float *channel;
+    const float *lhs;          // [T][B][4H]
+    const float *c0;           // [B][H] centred cell codes
+    float *output, *finalHidden, *finalCell;
+    rxmet_lstm_trace ck;
+    const int *poison;         // status word of the tensor-core projection: non-zero turns the outputs into NaN
+
+    struct Lane {
+        int64_t addend;
+        float outMult, outPow2, gateMult, gatePow2, giLo, giHi;
+        TableView table;
+        bool narrow;   // warp-uniform: the sum fits 32 bits
+    };
+    struct State {
+        float cell, hidden, tanhC;
+        uint32_t flags;   // clamped: bit 0 cell state, 1 tanh, 2 hidden
+    };
+    struct Fetch {
+        float lhs;
+    };
+    struct FetchB {};
+    struct Saved {
+        float hh, gateIn, gateOut;
+        uint32_t index;   // of the gate input in its table
+        bool hhClamped, inClamped;
+    };
+
+    size_t sharedBytes() const { return static_cast<size_t>(tableBytes); }
+
+    __device__ __forceinline__ uint32_t weightWord(int gate, int unit, int kw) const {
+        const int H = hidden();
+        const uint2 pair = __ldg(words + (static_cast<size_t>(gate >> 1) * kWords + kw) * H + unit);
+        return (gate & 1) ? pair.y : pair.x;
+    }
+    __device__ __forceinline__ void init(uint8_t *shared, int tid, int threads) const {
+        for (int i = tid; i < tableBytes / 16; i += threads)
+            reinterpret_cast<uint4 *>(shared)[i] = __ldg(reinterpret_cast<const uint4 *>(tables) + i);
+    }
+    __device__ __forceinline__ TableView view(uint32_t shared, int t) const {
+        constexpr uint32_t kExponent = 0x4B000000u;   // of 2^23
+        return TableView{shared + segOffset[t] - ((kExponent >> segShift) << 3), shared + bitOffset[t] - ((kExponent >> 5) << 2),
+                         8388608.0f - inLo[t], outLo[t], outHi[t]};
+    }
+    __device__ __forceinline__ Lane lane(uint32_t shared, int gate, int unit, bool real) const {
+        const int H = hidden();
+        Lane l;
+        const int c = gate * H + unit, opIn = RXMET_LSTM_INPUT_GATE_INPUT + gate;
+        const size_t C = 4 * static_cast<size_t>(H);
+        l.addend = real ? addend[c] : 0;
+        l.outMult = real ? channel[kHhOutMult * C + c] : 0.0f;
+        l.outPow2 = real ? channel[kHhOutPow2 * C + c] : 0.0f;
+        l.gateMult = s.hhToGate[gate].mult;
+        l.gatePow2 = s.hhToGate[gate].pow2;
+        l.giLo = static_cast<float>(s.lo[opIn] - s.zp[opIn]);
+        l.giHi = static_cast<float>(s.hi[opIn] - s.zp[opIn]);
+        l.table = view(shared, gate);
+        const int64_t wMax = max(-static_cast<int64_t>(s.lo[RXMET_LSTM_WEIGHT_HH]), static_cast<int64_t>(s.hi[RXMET_LSTM_WEIGHT_HH]));
+        l.narrow = __all_sync(0xffffffffu, wMax * 65535 * H + llabs(l.addend) < (int64_t{1} << 31));
+        return l;
+    }
+    __device__ __forceinline__ float scaleH(bool good) const {
+        return (!good || (poison && *poison)) ? __int_as_float(0x7fc00000) : s.scale[RXMET_LSTM_OUTPUT];
+    }
+    // centred limits of an operator's grid
+    __device__ __forceinline__ float lowOf(int op) const { return static_cast<float>(s.lo[op] - s.zp[op]); }
+    __device__ __forceinline__ float highOf(int op) const { return static_cast<float>(s.hi[op] - s.zp[op]); }
+    // clamp(rint(x)) on a grid of integers below 2^22 and, where it is saved, whether it clamped
+    __device__ __forceinline__ float quantized(float x, float lo, float hi, bool &clamped) const {
+        if (TRAIN) {
+            const float r = roundSmall(clampF(x, lo - 1.0f, hi + 1.0f));
+            clamped = r < lo || r > hi;
+            return clampF(r, lo, hi);
+        }
+        clamped = false;
+        return roundSmall(clampF(x, lo, hi));
+    }
+
+    __device__ __forceinline__ void begin(uint32_t, State &st, int row, int unit) const {
+        const int H = hidden();
+        st.cell = c0[static_cast<size_t>(row) * H + unit];
+        st.hidden = st.tanhC = 0.0f;
+        st.flags = 0;
+    }
+    __device__ __forceinline__ void fetch(Fetch &f, size_t at, uint32_t row, int gate, int unit) const {
+        const int H = hidden();
+        f.lhs = __ldg(lhs + at * (4 * static_cast<size_t>(H)) + (row * (4 * H) + gate * H + unit));
+    }
+    __device__ __forceinline__ void fetchB(FetchB &, size_t, uint32_t, int) const {}
+    // gate output (centred code as a float)
+    template <int STRIDE>
+    __device__ __forceinline__ uint32_t linear(uint32_t, const Lane &l, const Fetch &in, const uint32_t *acc, Saved &saved) const {
+        const int32_t high = static_cast<int32_t>(acc[0]), low = static_cast<int32_t>(acc[STRIDE]);
+        float total;
+        if (l.narrow) total = __int2float_rn(static_cast<int32_t>(static_cast<uint32_t>(high) * 256u + static_cast<uint32_t>(low) + static_cast<uint32_t>(l.addend)));
+        else total = __ll2float_rn((static_cast<int64_t>(high) << 8) + low + l.addend);
+        bool hhClamped;
+        const float hh = quantized(__fmul_rn(__fmul_rn(total, l.outMult), l.outPow2), lowOf(RXMET_LSTM_WEIGHT_HH_LINEAR),
+                                   highOf(RXMET_LSTM_WEIGHT_HH_LINEAR), hhClamped);
+        const float sum = __fadd_rn(in.lhs, roundSmall(__fmul_rn(__fmul_rn(hh, l.gateMult), l.gatePow2)));
+        const float gateIn = clampF(sum, l.giLo, l.giHi);
+        uint32_t index;
+        const float gateOut = lookup(l.table, segShift, gateIn, index);
+        if (TRAIN) saved = Saved{hh, gateIn, gateOut, index, hhClamped, sum < l.giLo || sum > l.giHi};
+        return __float_as_uint(gateOut);
+    }
+    __device__ __forceinline__ uint32_t cell(uint32_t shared, State &st, const FetchB &, const uint32_t (&v)[4]) const {
+        const float gI = __uint_as_float(v[0]), gF = __uint_as_float(v[1]), gG = __uint_as_float(v[2]), gO = __uint_as_float(v[3]);
+        const float pf = __fmul_rn(gF, st.cell), pi = __fmul_rn(gI, gG);
+        const float sf = dev::scaleCell(pf, s.forgetRatio, s.forgetMantissa, s.forgetExponent, s.forgetUsesFp);
+        const float si = dev::scaleCell(pi, s.inputRatio, s.inputMantissa, s.inputExponent, s.inputUsesFp);
+        bool cellClamped, hiddenClamped;
+        st.cell = quantized(__fadd_rn(sf, si), lowOf(RXMET_LSTM_CELL_STATE), highOf(RXMET_LSTM_CELL_STATE), cellClamped);
+        uint32_t index;
+        st.tanhC = lookup(view(shared, 4), segShift, st.cell, index);
+        st.hidden = quantized(__fmul_rn(__fmul_rn(__fmul_rn(gO, st.tanhC), s.productToOutput.mult), s.productToOutput.pow2), lowOf(RXMET_LSTM_OUTPUT),
+                              highOf(RXMET_LSTM_OUTPUT), hiddenClamped);
+        if (TRAIN) st.flags = (cellClamped ? 1u : 0u) | (clampFlag(4, index) ? 2u : 0u) | (hiddenClamped ? 4u : 0u);
+        return __float_as_uint(__fadd_rn(st.hidden, 8388608.0f + static_cast<float>(s.zp[RXMET_LSTM_OUTPUT] - s.lo[RXMET_LSTM_OUTPUT]))) & 0xffffu;
+    }
+    __device__ __forceinline__ bool clampFlag(int t, uint32_t index) const {
+        const int i = static_cast<int>(index & 0x7fffffu);
+        return i < flagBelow[t] || i >= flagFrom[t];
+    }
+    __device__ __forceinline__ void store(const State &st, const FetchB &, size_t at, uint32_t row, int unit, bool good) const {
+        const int H = hidden();
+        const size_t o = at * H + (row * H + unit);
+        output[o] = __fmul_rn(st.hidden, scaleH(good));
+        if (TRAIN) {
+            if (ck.cell_states) ck.cell_states[o] = st.cell + s.zpF[RXMET_LSTM_CELL_STATE];
+            if (ck.cell_states_clamped) ck.cell_states_clamped[o] = static_cast<uint8_t>(st.flags & 1u);
+            if (ck.cell_tanh_outputs) ck.cell_tanh_outputs[o] = st.tanhC + s.zpF[RXMET_LSTM_CELL_TANH_OUTPUT];
+            if (ck.cell_tanh_outputs_clamped) ck.cell_tanh_outputs_clamped[o] = static_cast<uint8_t>((st.flags >> 1) & 1u);
+            if (ck.hidden_outputs) ck.hidden_outputs[o] = st.hidden + s.zpF[RXMET_LSTM_OUTPUT];
+            if (ck.hidden_outputs_clamped) ck.hidden_outputs_clamped[o] = static_cast<uint8_t>((st.flags >> 2) & 1u);
+        }
+    }
+    __device__ __forceinline__ void storeLinear(const Saved &v, size_t at, uint32_t row, int gate, int unit) const {
+        const int H = hidden();
+        const size_t o = at * (4 * static_cast<size_t>(H)) + (row * (4 * H) + gate * H + unit);
+        const int opIn = RXMET_LSTM_INPUT_GATE_INPUT + gate, opOut = RXMET_LSTM_INPUT_GATE_OUTPUT + gate;
+        if (ck.weight_hh_linear) ck.weight_hh_linear[o] = v.hh + s.zpF[RXMET_LSTM_WEIGHT_HH_LINEAR];
+        if (ck.weight_hh_linear_clamped) ck.weight_hh_linear_clamped[o] = v.hhClamped;
+        if (ck.gate_inputs) ck.gate_inputs[o] = v.gateIn + s.zpF[opIn];
+        if (ck.gate_inputs_clamped) ck.gate_inputs_clamped[o] = v.inClamped;
+        if (ck.gate_outputs) ck.gate_outputs[o] = v.gateOut + s.zpF[opOut];
+        if (ck.gate_outputs_clamped) ck.gate_outputs_clamped[o] = clampFlag(gate, v.index);
+    }
+    __device__ __forceinline__ void finish(const State &st, int row, int unit, bool good) const {
+        const int H = hidden();
+        const size_t o = static_cast<size_t>(row) * H + unit;
+        finalHidden[o] = __fmul_rn(st.hidden, scaleH(good));
+        finalCell[o] = __fmul_rn(st.cell, good ? s.scale[RXMET_LSTM_CELL_STATE] : __int_as_float(0x7fc00000));
+    }
+};
+
+// Rows: a step of n rows costs about 1 + n / 5 of the chain of a one-row step.
+template <bool TRAIN, int HP>
+void launchLstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &cell, cudaStream_t st) {
+    if (p.H == HP) {
+        LstmPlaneCell<TRAIN, HP> full;
+        static_assert(sizeof(full) == sizeof(cell), "the variants differ in the width only");
+        std::memcpy(&full, &cell, sizeof(full));
+        planerec::launchBest<LstmPlaneCell<TRAIN, HP>, HP, 64, 2, 5, 8, 16, 24, 32>("lstmRecurrentWide", p, full, st);
+    } else {
+        planerec::launchBest<LstmPlaneCell<TRAIN>, HP, 64, 2, 5, 8, 16, 24, 32>("lstmRecurrentWide", p, cell, st);
+    }
+}
+// One padded width each, built in separate files (lstm_forward_cluster_*.cu).
+template <bool TRAIN, int HP>
+void lstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &cell, cudaStream_t st);
+
+}  // namespace lstm
+}  // namespace rxmet

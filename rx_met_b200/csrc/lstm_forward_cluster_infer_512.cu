@@ -1,0 +1,13 @@
+// Instances of the cluster recurrence of lstm_forward_cluster.cuh.
+#include "lstm_forward_cluster.cuh"
+
+namespace rxmet {
+namespace lstm {
+
+template <>
+void lstmCluster<false, 512>(const planerec::Problem &p, const LstmPlaneCell<false> &cell, cudaStream_t st) {
+    launchLstmCluster<false, 512>(p, cell, st);
+}
+
+}  // namespace lstm
+}  // namespace rxmet

@@ -1,0 +1,17 @@
+// Instances of the cluster recurrence of lstm_forward_cluster.cuh.
+#include "lstm_forward_cluster.cuh"
+
+namespace rxmet {
+namespace lstm {
+
+template <>
+void lstmCluster<true, 64>(const planerec::Problem &p, const LstmPlaneCell<true> &cell, cudaStream_t st) {
+    launchLstmCluster<true, 64>(p, cell, st);
+}
+template <>
+void lstmCluster<true, 128>(const planerec::Problem &p, const LstmPlaneCell<true> &cell, cudaStream_t st) {
+    launchLstmCluster<true, 128>(p, cell, st);
+}
+
+}  // namespace lstm
+}  // namespace rxmet

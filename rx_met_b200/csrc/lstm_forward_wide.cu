@@ -35,6 +35,7 @@
 
 #include "common.h"
 #include "lstm_device.cuh"
+#include "lstm_forward_cluster.cuh"
 #include "plane_proj_umma.cuh"
 #include "lstm_kernels.h"
 
@@ -881,6 +882,23 @@ struct SizerAdapter {
     }
 };
 
+// The cluster kernel rounds by adding 1.5 * 2^23: grids and the linear code on the gate's grid stay below 2^22, and the compact
+// tables (60 kB at 128 inputs per line) leave room for the operands.
+bool clusterTakes(const Exec &e) {
+    static const bool off = std::getenv("RXMET_LSTM_REC_SIMT") != nullptr || std::getenv("RXMET_LSTM_REC_UMMA") != nullptr;
+    if (off || !e.compactTables().ok || e.compactTables().bytes.size() > 130 * 1024) return false;
+    const ScalarExec &s = e.scalar;
+    auto magnitude = [&](int op) {
+        return std::max(std::abs(static_cast<double>(s.lo[op]) - s.zp[op]), std::abs(static_cast<double>(s.hi[op]) - s.zp[op])) + 2.0;
+    };
+    const double limit = 1 << 22;
+    for (int op : {RXMET_LSTM_WEIGHT_HH_LINEAR, RXMET_LSTM_CELL_STATE, RXMET_LSTM_OUTPUT})
+        if (magnitude(op) >= limit) return false;
+    for (const DevRescale &r : s.hhToGate)
+        if (magnitude(RXMET_LSTM_WEIGHT_HH_LINEAR) * r.mult * r.pow2 >= limit) return false;
+    return true;
+}
+
 }  // namespace
 
 bool forwardQuantWideTakes(const Exec &e, int I, int H, const char **why) {
@@ -1017,6 +1035,34 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
         else RXMET_WIDE_IH(64);
 #undef RXMET_WIDE_IH
         afterLaunch("lstmInputLinearWide");
+    }
+    // Recurrence over clusters wherever the activation tables have a compact form and the grids are the usual ones.
+    if (planes == 2 && clusterTakes(e)) {
+        const planerec::Problem problem{T, B, H, l.h0};
+        const bool saves = ck.weight_hh_linear || ck.weight_hh_linear_clamped || ck.gate_inputs || ck.gate_inputs_clamped || ck.gate_outputs ||
+                           ck.gate_outputs_clamped || ck.cell_states || ck.cell_states_clamped || ck.cell_tanh_outputs ||
+                           ck.cell_tanh_outputs_clamped || ck.hidden_outputs || ck.hidden_outputs_clamped;
+        auto run = [&](auto cell) {
+            const CompactTables &t = e.compactTables();
+            cell.s = s; cell.width = H; cell.kWords = kHh; cell.B = static_cast<size_t>(B);
+            cell.segShift = t.segShift; cell.tableBytes = static_cast<int>(t.bytes.size()); cell.tables = e.compactTablesOnDevice();
+            for (int i = 0; i < kTables; ++i) {
+                cell.segOffset[i] = t.segOffset[i]; cell.bitOffset[i] = t.bitOffset[i]; cell.flagBelow[i] = t.flagBelow[i];
+                cell.flagFrom[i] = t.flagFrom[i]; cell.inLo[i] = t.inLo[i]; cell.outLo[i] = t.outLo[i]; cell.outHi[i] = t.outHi[i];
+            }
+            cell.words = reinterpret_cast<const uint2 *>(l.wHh); cell.addend = l.addHh; cell.channel = l.channel; cell.lhs = l.lhs;
+            cell.c0 = l.c0; cell.output = call.output; cell.finalHidden = call.finalHidden; cell.finalCell = call.finalCell; cell.ck = ck;
+            cell.poison = tensorProjection ? l.projStatus : nullptr;
+            constexpr bool kTrain = decltype(cell)::kSaves;
+            if (H <= 64) lstmCluster<kTrain, 64>(problem, cell, st);
+            else if (H <= 128) lstmCluster<kTrain, 128>(problem, cell, st);
+            else if (H <= 256) lstmCluster<kTrain, 256>(problem, cell, st);
+            else if (H <= 384) lstmCluster<kTrain, 384>(problem, cell, st);
+            else lstmCluster<kTrain, 512>(problem, cell, st);
+        };
+        if (saves) run(LstmPlaneCell<true>{});
+        else run(LstmPlaneCell<false>{});
+        return;
     }
     // Recurrence: per-step product on the tensor cores for hidden sizes whose weights fit no single SM
     // (RXMET_LSTM_REC_SIMT turns it off, RXMET_LSTM_REC_UMMA forces it for every eligible shape).

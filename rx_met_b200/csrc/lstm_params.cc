@@ -40,6 +40,11 @@ void checkConfig(const rxmet_lstm_quant_config &cfg) {
     }
 }
 
+constexpr int kTableIn[kTables] = {RXMET_LSTM_INPUT_GATE_INPUT, RXMET_LSTM_FORGET_GATE_INPUT, RXMET_LSTM_CELL_GATE_INPUT,
+                                   RXMET_LSTM_OUTPUT_GATE_INPUT, RXMET_LSTM_CELL_STATE};
+constexpr int kTableOut[kTables] = {RXMET_LSTM_INPUT_GATE_OUTPUT, RXMET_LSTM_FORGET_GATE_OUTPUT, RXMET_LSTM_CELL_GATE_OUTPUT,
+                                    RXMET_LSTM_OUTPUT_GATE_OUTPUT, RXMET_LSTM_CELL_TANH_OUTPUT};
+
 double roundEven(double v) { return std::nearbyint(v); }
 
 // ---- range -> scale / zero point ---------------------------------------------
@@ -520,28 +525,24 @@ std::shared_ptr<const Exec> deriveExec(const rxmet_lstm_quant_params &p, bool re
         field(kHhOutMult)[ch] = ho.mult;  field(kHhOutPow2)[ch] = ho.pow2;
     }
     bool tablesFit = true;
-    const int tableIn[kTables] = {RXMET_LSTM_INPUT_GATE_INPUT, RXMET_LSTM_FORGET_GATE_INPUT, RXMET_LSTM_CELL_GATE_INPUT,
-                                  RXMET_LSTM_OUTPUT_GATE_INPUT, RXMET_LSTM_CELL_STATE};
-    const int tableOut[kTables] = {RXMET_LSTM_INPUT_GATE_OUTPUT, RXMET_LSTM_FORGET_GATE_OUTPUT, RXMET_LSTM_CELL_GATE_OUTPUT,
-                                   RXMET_LSTM_OUTPUT_GATE_OUTPUT, RXMET_LSTM_CELL_TANH_OUTPUT};
-    for (int t = 0; t < kTables; ++t) tablesFit = tablesFit && p.config.bitwidth[tableIn[t]] <= 8;
+    for (int t = 0; t < kTables; ++t) tablesFit = tablesFit && p.config.bitwidth[kTableIn[t]] <= 8;
     if (tablesFit) {
         e->tables.assign(static_cast<size_t>(kTables) * kTableSize, 0);
         for (int t = 0; t < kTables; ++t)
-            buildTable(p, tableIn[t], tableOut[t], t == 2 || t == 4, e->tables.data() + static_cast<size_t>(t) * kTableSize);
+            buildTable(p, kTableIn[t], kTableOut[t], t == 2 || t == 4, e->tables.data() + static_cast<size_t>(t) * kTableSize);
     }
     bool wideFit = true;
     for (int t = 0; t < kTables; ++t)
-        wideFit = wideFit && p.config.bitwidth[tableIn[t]] <= 16 && p.config.bitwidth[tableOut[t]] <= 24;
+        wideFit = wideFit && p.config.bitwidth[kTableIn[t]] <= 16 && p.config.bitwidth[kTableOut[t]] <= 24;
     if (wideFit) {
         size_t total = 0;
         for (int t = 0; t < kTables; ++t) {
             e->wide.offset[t] = static_cast<int>(total);
-            total += size_t{1} << p.config.bitwidth[tableIn[t]];
+            total += size_t{1} << p.config.bitwidth[kTableIn[t]];
         }
         e->wide.entries.assign(total, 0);
         for (int t = 0; t < kTables; ++t)
-            buildTable(p, tableIn[t], tableOut[t], t == 2 || t == 4, e->wide.entries.data() + e->wide.offset[t]);
+            buildTable(p, kTableIn[t], kTableOut[t], t == 2 || t == 4, e->wide.entries.data() + e->wide.offset[t]);
     }
     e->weightsFitBytes = p.config.bitwidth[RXMET_LSTM_WEIGHT_IH] <= 8 && p.config.bitwidth[RXMET_LSTM_WEIGHT_HH] <= 8;
     const int actBits = std::max(p.config.bitwidth[RXMET_LSTM_INPUT], p.config.bitwidth[RXMET_LSTM_OUTPUT]);
@@ -552,21 +553,135 @@ std::shared_ptr<const Exec> deriveExec(const rxmet_lstm_quant_params &p, bool re
     return e;
 }
 
-const int32_t *Exec::wideTablesOnDevice() const {
+namespace {
+
+// Line of one segment: codes[i] (centred) for the inputs x0 + i.  Entries at a limit of the output grid bind on one side only
+// (the evaluation clamps).  Least squares for the slope, then the middle of the feasible intercepts.
+bool fitSegment(const int32_t *entries, int n, double x0, double outLo, double outHi, float *slope, float *intercept) {
+    double sx = 0, sy = 0, sxx = 0, sxy = 0;
+    int inner = 0;
+    auto code = [&](int i) { return static_cast<double>(entries[i] >> 1); };
+    for (int i = 0; i < n; ++i) {
+        const double c = code(i);
+        if (c <= outLo || c >= outHi) continue;
+        ++inner;
+        sx += i; sy += c; sxx += static_cast<double>(i) * i; sxy += i * c;
+    }
+    double b = 0;
+    if (inner >= 2) b = (inner * sxy - sx * sy) / (inner * sxx - sx * sx);
+    *slope = static_cast<float>(b);
+    double low = -1e30, high = 1e30;   // of the intercept: fmaf result in [code - 1.5, code + 0.5]
+    for (int i = 0; i < n; ++i) {
+        const double c = code(i), at = static_cast<double>(*slope) * (x0 + i);
+        if (c < outHi) high = std::min(high, c + 0.5 - at);
+        if (c > outLo) low = std::max(low, c - 1.5 - at);
+        if (c >= outHi) low = std::max(low, c - 1.5 - at);
+        if (c <= outLo) high = std::min(high, c + 0.5 - at);
+    }
+    if (!(low < high)) return false;
+    if (high - low > 1e6) *intercept = static_cast<float>(low > -1e29 ? low + 1.0 : high - 1.0);
+    else *intercept = static_cast<float>(0.5 * (low + high));
+    return true;
+}
+
+// base of the evaluation the kernels use: 1.5 * 2^23 added and taken away rounds to the nearest integer, ties to even
+float baseOf(float slope, float x, float intercept) {
+    const volatile float shifted = std::fmaf(slope, x, intercept) + 12582912.0f;
+    return shifted - 12582912.0f;
+}
+
+bool buildCompact(const Exec &e, int segShift, CompactTables &out) {
+    size_t at = 0;
+    out = CompactTables{};
+    out.segShift = segShift;
+    for (int t = 0; t < kTables; ++t) {
+        const int64_t entries = static_cast<int64_t>(e.scalar.hi[kTableIn[t]]) - e.scalar.lo[kTableIn[t]] + 1;
+        out.segOffset[t] = static_cast<int>(at);
+        at += static_cast<size_t>((entries + (int64_t{1} << segShift) - 1) >> segShift) * 8;
+        out.bitOffset[t] = static_cast<int>(at);
+        at += static_cast<size_t>((entries + 31) / 32) * 4;
+        at = (at + 15) & ~static_cast<size_t>(15);
+    }
+    out.bytes.assign(at, 0);
+    for (int t = 0; t < kTables; ++t) {
+        const ScalarExec &s = e.scalar;
+        const int in = kTableIn[t], to = kTableOut[t];
+        const int entries = s.hi[in] - s.lo[in] + 1;
+        if (static_cast<int64_t>(s.hi[to]) - s.lo[to] > 65535) return false;
+        const int32_t *table = e.wide.entries.data() + e.wide.offset[t];
+        const double x0 = static_cast<double>(s.lo[in]) - s.zp[in];
+        out.inLo[t] = static_cast<float>(x0);
+        out.outLo[t] = static_cast<float>(s.lo[to] - s.zp[to]);
+        out.outHi[t] = static_cast<float>(s.hi[to] - s.zp[to]);
+        float *segments = reinterpret_cast<float *>(out.bytes.data() + out.segOffset[t]);
+        uint32_t *bits = reinterpret_cast<uint32_t *>(out.bytes.data() + out.bitOffset[t]);
+        for (int first = 0, seg = 0; first < entries; first += 1 << segShift, ++seg) {
+            const int n = std::min(1 << segShift, entries - first);
+            float slope, intercept;
+            if (!fitSegment(table + first, n, x0 + first, out.outLo[t], out.outHi[t], &slope, &intercept)) return false;
+            segments[2 * seg] = slope;
+            segments[2 * seg + 1] = intercept;
+            for (int i = first; i < first + n; ++i) {
+                const float x = static_cast<float>(x0 + i), want = static_cast<float>(table[i] >> 1);
+                const float base = baseOf(slope, x, intercept);
+                auto clamped = [&](float v) { return std::fmin(std::fmax(v, out.outLo[t]), out.outHi[t]); };
+                if (clamped(base) == want) continue;
+                if (clamped(base + 1.0f) != want) return false;
+                bits[i >> 5] |= 1u << (i & 31);
+            }
+        }
+        int below = 0, from = entries;
+        while (below < entries && (table[below] & 1)) ++below;
+        while (from > below && (table[from - 1] & 1)) --from;
+        for (int i = below; i < from; ++i)
+            if (table[i] & 1) return false;
+        out.flagBelow[t] = below;
+        out.flagFrom[t] = from;
+    }
+    out.ok = true;
+    return true;
+}
+
+}  // namespace
+
+const CompactTables &Exec::compactTables() const {
+    std::call_once(compactOnce, [&] {
+        if (wide.entries.empty()) return;
+        for (int segShift = 7; segShift >= 5; --segShift)   // 8, 16, 32 kB of lines per 16-bit table beside 8 kB of bits
+            if (buildCompact(*this, segShift, compact)) return;
+        compact = CompactTables{};
+    });
+    return compact;
+}
+
+namespace {
+
+// Device copy of host bytes, one per device, kept with the Exec.
+template <class T>
+T *deviceCopy(std::mutex &mutex, std::vector<std::pair<int, std::shared_ptr<T>>> &copies, const void *host, size_t bytes) {
     int device = 0;
     RXMET_CUDA(cudaGetDevice(&device));
-    std::lock_guard<std::mutex> lock(deviceLock);
-    for (const auto &entry : deviceTables)
+    std::lock_guard<std::mutex> lock(mutex);
+    for (const auto &entry : copies)
         if (entry.first == device) return entry.second.get();
-    RXMET_REQUIRE(!wide.entries.empty(), "activation tables of this parameter set were not built");
-    int32_t *buffer = nullptr;
-    const size_t bytes = wide.entries.size() * sizeof(int32_t);
+    RXMET_REQUIRE(bytes > 0, "activation tables of this parameter set were not built");
+    T *buffer = nullptr;
     RXMET_CUDA(cudaMalloc(reinterpret_cast<void **>(&buffer), bytes));
-    std::shared_ptr<int32_t> owner(buffer, [](int32_t *ptr) { cudaFree(ptr); });
-    // synchronous on purpose: the entries are pageable host memory and the buffer is shared by every stream
-    RXMET_CUDA(cudaMemcpy(buffer, wide.entries.data(), bytes, cudaMemcpyHostToDevice));
-    deviceTables.emplace_back(device, owner);
+    std::shared_ptr<T> owner(buffer, [](T *ptr) { cudaFree(ptr); });
+    // synchronous on purpose: the bytes are pageable host memory and the buffer is shared by every stream
+    RXMET_CUDA(cudaMemcpy(buffer, host, bytes, cudaMemcpyHostToDevice));
+    copies.emplace_back(device, owner);
     return buffer;
+}
+
+}  // namespace
+
+const int32_t *Exec::wideTablesOnDevice() const {
+    return deviceCopy(deviceLock, deviceTables, wide.entries.data(), wide.entries.size() * sizeof(int32_t));
+}
+
+const uint8_t *Exec::compactTablesOnDevice() const {
+    return deviceCopy(deviceLock, deviceCompact, compactTables().bytes.data(), compactTables().bytes.size());
 }
 
 }  // namespace lstm

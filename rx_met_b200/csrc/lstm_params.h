@@ -85,6 +85,21 @@ struct WideTables {
     int offset[kTables] = {};
 };
 
+// The same tables in the form that fits shared memory: per segment of 2^segShift inputs a line, per input one correction
+// bit.  For the centred input code x (a float): t = fmaf(slope, x, intercept), base = round-half-even(t) and the centred
+// output code is clamp(base + bit, outLo, outHi), where (slope, intercept) sit at segOffset + 8 * (index >> segShift) and
+// the bit at bit (index & 31) of the word at bitOffset + 4 * (index >> 5), index = x - inLo.  The clamp flag of an
+// entry is index < flagBelow || index >= flagFrom.  Built from the full tables and checked entry by entry; `ok` is false
+// when some segment has no such line, an output grid is wider than 16 bits or the flags have another shape.
+struct CompactTables {
+    bool ok = false;
+    int segShift = 0;
+    std::vector<uint8_t> bytes;
+    int segOffset[kTables] = {}, bitOffset[kTables] = {};
+    float inLo[kTables] = {}, outLo[kTables] = {}, outHi[kTables] = {};
+    int flagBelow[kTables] = {}, flagFrom[kTables] = {};
+};
+
 struct Exec {
     int hidden = 0;
     ScalarExec scalar{};
@@ -96,6 +111,12 @@ struct Exec {
     int activationPlanes = 1;              // byte planes that hold an input / hidden code: 1 (<= 8 bit) or 2 (<= 16 bit); 0 = wider
     // Device copy of wide.entries on the current device (cudaMalloc on first use, freed with the Exec).
     const int32_t *wideTablesOnDevice() const;
+    // The compact form of the wide tables, built on first use, and its device copy.
+    const CompactTables &compactTables() const;
+    const uint8_t *compactTablesOnDevice() const;
+    mutable std::once_flag compactOnce;
+    mutable CompactTables compact;
+    mutable std::vector<std::pair<int, std::shared_ptr<uint8_t>>> deviceCompact;
     mutable std::mutex deviceLock;
     mutable std::vector<std::pair<int, std::shared_ptr<int32_t>>> deviceTables;  // (device ordinal, buffer)
 };

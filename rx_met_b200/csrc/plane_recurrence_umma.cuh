@@ -59,16 +59,16 @@ constexpr uint32_t powerOfTwoFrom(uint32_t n) {
     return p;
 }
 
-template <int H, int U, int ROWS, int PLANES>
+template <int HP, int U, int ROWS, int PLANES>
 struct Geometry {
-    static constexpr int kCtas = H / U, kTiles = U / 32;
+    static constexpr int kCtas = HP / U, kTiles = U / 32;
     static constexpr int kWarps = ROWS * kTiles >= 16 ? 16 : 8;   // of the epilogue; one more warp issues products and copies
     static constexpr int kThreads = 32 * (kWarps + 1);
     static constexpr int kRowGroups = kWarps / (4 * kTiles);   // warps that share the rows of a tile's quarter
     static constexpr int kRowsA = ROWS / kRowGroups;            // rows of a lane in phase A
     static constexpr int kRowsB = kRowsA / 4;                   // cells of a lane in phase B
     static_assert(kRowsA % 4 == 0 && kRowsA * kRowGroups == ROWS, "rows divide into quads");
-    static constexpr int kPadK = (H + 31) / 32 * 32;
+    static constexpr int kPadK = (HP + 31) / 32 * 32;
     static constexpr int kCols = (PLANES * ROWS + 15) / 16 * 16;          // accumulator columns of a tile
     static constexpr uint32_t kColsA = kPadK / 4;                          // tensor-memory columns of its weights
     static constexpr uint32_t kTmemCols = powerOfTwoFrom(kTiles * (kCols + kColsA));
@@ -81,34 +81,38 @@ struct Geometry {
 };
 
 struct Problem {
-    int T, B;
+    int T, B, H;
     const uint32_t *h0;   // [B][PLANES][H padded to 16, / 4] words of four code bytes: the initial state
 };
 
-// Cell contract (device functions; `at` = first row of the step in the [T][B] arrays, `Shared` is placed in shared memory):
-//   kGates                                                  quarters in use
+// Cell contract (device functions unless marked; `at` = first row of the step in the [T][B] arrays, `shared` = address of the
+// operator's part of shared memory):
+//   kGates, kSaves, kFull, kChunk                           quarters in use; whether storeLinear has anything to store; whether H is HP;
+//                                                           most rows of phase A at a time
+//   size_t sharedBytes()                                    host: size of that part
 //   uint32_t weightWord(gate, unit, kw)                     four weight bytes along K, 0 for an empty quarter
-//   void init(Shared &, tid, threads)                       fills Shared
-//   Lane lane(Shared, gate, unit)                           constants of phase A
-//   void begin(Shared, State &, row, unit)                  state of one cell of phase B from h0
+//   void init(uint8_t *, tid, threads)                      fills it
+//   Lane lane(shared, gate, unit, real)                     constants of phase A (all lanes of the warp call it)
+//   void begin(shared, State &, row, unit)                  state of one cell of phase B from h0
 //   void fetch(Fetch &, at, row, gate, unit), fetchB(FetchB &, at, row, unit)     operands of a step, asked for before the product is awaited
-//   uint32_t linear<STRIDE>(Shared, Lane, Fetch, acc, at, row, gate, unit, live)    phase A; plane p of the sum at acc[p STRIDE]
-//   uint32_t cell(Shared, State &, FetchB, v[4])            phase B: new code - grid minimum
-//   void store(Shared, State, FetchB, at, row, unit, good)       outputs of the step; good = false: make them NaN
-//   void finish(Shared, State, row, unit, good)             after the last step
-template <class Cell, int H, int U, int ROWS, int PLANES>
-__global__ void __launch_bounds__(Geometry<H, U, ROWS, PLANES>::kThreads, 1)
+//   uint32_t linear<STRIDE>(shared, Lane, Fetch, acc, Saved &)    phase A; plane p of the sum at acc[p STRIDE]
+//   uint32_t cell(shared, State &, FetchB, v[4])            phase B: new code - grid minimum
+//   void store(State, FetchB, at, row, unit, good)          outputs of the step; good = false: make them NaN
+//   void storeLinear(Saved, at, row, gate, unit)            what phase A saves
+//   void finish(State, row, unit, good)                     after the last step
+template <class Cell, int HP, int U, int ROWS, int PLANES>
+__global__ void __launch_bounds__(Geometry<HP, U, ROWS, PLANES>::kThreads, 1)
 planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c) {
-    using G = Geometry<H, U, ROWS, PLANES>;
+    using G = Geometry<HP, U, ROWS, PLANES>;
     constexpr int MT = G::kTiles, NC = G::kCtas;
     extern __shared__ __align__(128) uint8_t smemR[];
     __shared__ __align__(8) uint64_t productBar, codeBar[2];
     __shared__ uint32_t tmemSlot;
     __shared__ volatile int failed;   // the control warp's wait gave up
-    __shared__ typename Cell::Shared shared;
     uint8_t *operand = smemR;                                                // [2][K / 16][kCols][16]
     uint8_t *staging = operand + 2 * G::kOperandBytes;                       // [2][U / 16][kCols][16]
     uint32_t *exchange = reinterpret_cast<uint32_t *>(staging + 2 * G::kSlabBytes);   // [tile][row group][4 gates][rowsA][32 units]
+    const uint32_t shared = smemAddr(smemR) + static_cast<uint32_t>(G::kSharedBytes);                    // the operator's own part
 
     const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
     const int quarter = warp & 3, tile = (warp >> 2) % MT, rowGroup = (warp >> 2) / MT;
@@ -128,11 +132,11 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(&tmemSlot)), "n"(G::kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    c.init(shared, tid, G::kThreads);
+    c.init(smemR + G::kSharedBytes, tid, G::kThreads);
     for (uint32_t i = tid; i < (2 * G::kOperandBytes + 2 * G::kSlabBytes) / 16; i += G::kThreads)
         reinterpret_cast<uint4 *>(operand)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
-    constexpr int kWords = (H + 15) / 16 * 4;   // of a plane row
+    const int H = p.H, kWords = (H + 15) / 16 * 4;   // words of a plane row
     for (int i = tid; i < ROWS * PLANES * (kWords / 4); i += G::kThreads) {
         const int kg = i % (kWords / 4), n = i / (kWords / 4), pl = n / ROWS, r = n - pl * ROWS;
         if (b0 + r < p.B)
@@ -145,7 +149,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
         for (int kw = 0; kw < G::kPadK / 4; kw += 4) {
             uint32_t w[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) w[e] = kw + e < kWords ? c.weightWord(quarter, unit, kw + e) : 0u;
+            for (int e = 0; e < 4; ++e) w[e] = (kw + e < kWords && unit < H) ? c.weightWord(quarter, unit, kw + e) : 0u;
             tmemStore4(tmemWeights + quarterBase + tile * G::kColsA + kw, w[0], w[1], w[2], w[3]);
         }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -190,43 +194,68 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
                                 sendBar + ((t + 1) & 1) * 8);
         }
     } else {
-        const typename Cell::Lane mine = c.lane(shared, quarter, unit);
+        // units beyond the layer's width compute on zero weights and store nothing; their operand bytes stay zero
+        const bool real = Cell::kFull || unit < H;
+        // rows of phase A in one go: as many as the operator allows and the rows divide into
+        constexpr int kChunk = G::kRowsA <= Cell::kChunk ? G::kRowsA : (G::kRowsA % Cell::kChunk == 0 ? Cell::kChunk : 4);
+        constexpr bool kDefer = G::kRowsA == 4;   // more rows keep the epilogue busy by themselves; held back they would spill
+        const typename Cell::Lane mine = c.lane(shared, quarter, unit, real);
         typename Cell::State state[G::kRowsB];
 #pragma unroll
         for (int i = 0; i < G::kRowsB; ++i)
-            if (rowB + i < p.B) c.begin(shared, state[i], rowB + i, unit);
+            if (real && rowB + i < p.B) c.begin(shared, state[i], rowB + i, unit);
         const uint32_t column = tmem + quarterBase + tile * G::kCols + rowGroup * G::kRowsA;
         uint32_t *exchangeTile = exchange + (tile * G::kRowGroups + rowGroup) * (4 * G::kRowsA * 32) + lane;
         uint8_t *stageMine = staging + (tile * 2 + (lane >> 4)) * G::kGroupStride + (rowB - b0) * 16 + (lane & 15);
 #pragma unroll 1
         for (int t = 0; t < p.T; ++t) {
             const size_t at = static_cast<size_t>(t) * p.B;   // first row of the step in the [T][B] arrays
-            typename Cell::Fetch inA[G::kRowsA];
+            // Phase A walks its rows kChunk at a time in a rolled loop (the body of a step has to stay small for the instruction
+            // cache); the operands of the next chunk are asked for before the current ones are used.
+            typename Cell::Fetch in[kChunk];
             typename Cell::FetchB inB[G::kRowsB];
+            auto fetchA = [&](typename Cell::Fetch (&to)[kChunk], int first) {
 #pragma unroll
-            for (int r = 0; r < G::kRowsA; ++r)
-                if (rowA + r < p.B) c.fetch(inA[r], at, rowA + r, quarter, unit);
+                for (int r = 0; r < kChunk; ++r)
+                    if (real && rowA + first + r < p.B) c.fetch(to[r], at, rowA + first + r, quarter, unit);
+            };
+            fetchA(in, 0);
 #pragma unroll
             for (int i = 0; i < G::kRowsB; ++i)
-                if (rowB + i < p.B) c.fetchB(inB[i], at, rowB + i, unit);
+                if (real && rowB + i < p.B) c.fetchB(inB[i], at, rowB + i, unit);
             wait(smemAddr(&productBar), t & 1);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t acc[PLANES * G::kRowsA];
+            typename Cell::Saved saved[kChunk];
+#pragma unroll 1
+            for (int first = 0; first < G::kRowsA; first += kChunk) {
+                uint32_t acc[PLANES * kChunk];
 #pragma unroll
-            for (int pl = 0; pl < PLANES; ++pl)
+                for (int pl = 0; pl < PLANES; ++pl)
 #pragma unroll
-                for (int r = 0; r < G::kRowsA; r += 4) tmemLoad4(column + pl * ROWS + r, acc + pl * G::kRowsA + r);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (quarter < Cell::kGates) {
+                    for (int r = 0; r < kChunk; r += 4) tmemLoad4(column + pl * ROWS + first + r, acc + pl * kChunk + r);
+                typename Cell::Fetch later[kChunk];
+                if (first + kChunk < G::kRowsA) fetchA(later, first + kChunk);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (quarter < Cell::kGates) {
 #pragma unroll
-                for (int r = 0; r < G::kRowsA; ++r)
-                    exchangeTile[(quarter * G::kRowsA + r) * 32] =
-                        c.template linear<G::kRowsA>(shared, mine, inA[r], acc + r, at, rowA + r, quarter, unit, rowA + r < p.B);
+                    for (int r = 0; r < kChunk; ++r)
+                        if (rowA + first + r < p.B)
+                            exchangeTile[(quarter * G::kRowsA + first + r) * 32] = c.template linear<kChunk>(shared, mine, in[r], acc + r, saved[r]);
+                    if (Cell::kSaves && !kDefer) {
+#pragma unroll
+                        for (int r = 0; r < kChunk; ++r)
+                            if (real && rowA + first + r < p.B) c.storeLinear(saved[r], at, rowA + first + r, quarter, unit);
+                    }
+                }
+                if (G::kRowsA > kChunk) {
+#pragma unroll
+                    for (int r = 0; r < kChunk; ++r) in[r] = later[r];
+                }
             }
             asm volatile("bar.sync %0, 128;" ::"r"(1 + (warp >> 2)) : "memory");   // the four quarters of this tile and row group
 #pragma unroll
             for (int i = 0; i < G::kRowsB; ++i) {
-                if (rowB + i >= p.B) continue;
+                if (!real || rowB + i >= p.B) continue;
                 uint32_t v[4];
 #pragma unroll
                 for (int g = 0; g < 4; ++g) v[g] = g < Cell::kGates ? exchangeTile[(g * G::kRowsA + quarter * G::kRowsB + i) * 32] : 0u;
@@ -238,18 +267,25 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
                 } else {
                     dst[0] = static_cast<uint8_t>(u);
                 }
+                if (!kDefer) c.store(state[i], inB[i], at, rowB + i, unit, alive && !failed);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncthreads();
-            // what nobody waits for leaves while the codes travel and the next product runs
+            if (kDefer) {   // what nobody waits for leaves while the codes travel and the next product runs
 #pragma unroll
-            for (int i = 0; i < G::kRowsB; ++i)
-                if (rowB + i < p.B) c.store(shared, state[i], inB[i], at, rowB + i, unit, alive && !failed);
+                for (int i = 0; i < G::kRowsB; ++i)
+                    if (real && rowB + i < p.B) c.store(state[i], inB[i], at, rowB + i, unit, alive && !failed);
+                if (Cell::kSaves && quarter < Cell::kGates) {
+#pragma unroll
+                    for (int r = 0; r < kChunk; ++r)
+                        if (real && rowA + r < p.B) c.storeLinear(saved[r], at, rowA + r, quarter, unit);
+                }
+            }
         }
 #pragma unroll
         for (int i = 0; i < G::kRowsB; ++i)
-            if (rowB + i < p.B) c.finish(shared, state[i], rowB + i, unit, alive && !failed);
+            if (real && rowB + i < p.B) c.finish(state[i], rowB + i, unit, alive && !failed);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -257,16 +293,17 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
     cluster::barrierAll();   // nobody leaves while a peer may still copy into its shared memory
 }
 
-// Launches a variant with its clusters; false when the device holds none of them.
-template <class Cell, int H, int U, int ROWS, int PLANES>
-bool launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t st) {
-    using G = Geometry<H, U, ROWS, PLANES>;
-    const auto kernel = planeRecurrence<Cell, H, U, ROWS, PLANES>;
-    ensureDynamicSmem(reinterpret_cast<const void *>(kernel), G::kSharedBytes);
+// Launches a variant with its clusters.
+template <class Cell, int HP, int U, int ROWS, int PLANES>
+void launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t st) {
+    using G = Geometry<HP, U, ROWS, PLANES>;
+    const auto kernel = planeRecurrence<Cell, HP, U, ROWS, PLANES>;
+    const size_t smem = G::kSharedBytes + cell.sharedBytes();
+    ensureDynamicSmem(reinterpret_cast<const void *>(kernel), smem);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(static_cast<unsigned>((p.B + ROWS - 1) / ROWS * G::kCtas));
     cfg.blockDim = dim3(G::kThreads);
-    cfg.dynamicSmemBytes = G::kSharedBytes;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -279,28 +316,28 @@ bool launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t s
         RXMET_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, cell));
     }
     afterLaunch(name);
-    return true;
 }
 
-// Rows of a cluster among `choices`: as few as let all clusters of the pass run at the same time (a step costs about
-// 1 + rows / 32 of the chain of a short step, a second wave costs the whole chain again).
-template <class Cell, int H, int U, int PLANES, int... ROWS>
+// Rows of a cluster among ROWS...: the number of waves times the cost of a step, which is about 1 + rows / PER of the
+// chain of a short one - as few rows as let all clusters run at the same time, or many where they cannot.
+template <class Cell, int HP, int U, int PLANES, int PER, int... ROWS>
 void launchBest(const char *name, const Problem &p, const Cell &cell, cudaStream_t st) {
     double bestCost = 1e30;
     int best = 0;
     (
         [&] {
-            using G = Geometry<H, U, ROWS, PLANES>;
-            const int resident = std::max(1, residentClusters(reinterpret_cast<const void *>(planeRecurrence<Cell, H, U, ROWS, PLANES>), G::kCtas,
-                                                              G::kThreads, G::kSharedBytes) / concurrentPasses());
+            using G = Geometry<HP, U, ROWS, PLANES>;
+            if (G::kSharedBytes + cell.sharedBytes() > static_cast<size_t>(currentDevice().smemMax)) return;
+            const int resident = std::max(1, residentClusters(reinterpret_cast<const void *>(planeRecurrence<Cell, HP, U, ROWS, PLANES>), G::kCtas,
+                                                              G::kThreads, G::kSharedBytes + cell.sharedBytes()) / concurrentPasses());
             const int clusters = (p.B + ROWS - 1) / ROWS, waves = (clusters + resident - 1) / resident;
-            const double cost = waves * (1.0 + ROWS / 32.0);
+            const double cost = waves * (1.0 + ROWS / static_cast<double>(PER));
             if (cost < bestCost) { bestCost = cost; best = ROWS; }
         }(),
         ...);
     (
         [&] {
-            if (best == ROWS) launch<Cell, H, U, ROWS, PLANES>(name, p, cell, st);
+            if (best == ROWS) launch<Cell, HP, U, ROWS, PLANES>(name, p, cell, st);
         }(),
         ...);
 }

@@ -113,9 +113,9 @@ def test_forward_quant_saturating_inputs(gl):
 
 
 @pytest.mark.parametrize("shape", [(1, 1, 8, 32), (2, 3, 8, 64), (3, 9, 8, 96), (4, 17, 12, 160), (5, 6, 8, 224), (3, 300, 8, 256),
-                                   (2, 130, 8, 128), (2, 7, 8, 192)], ids=lambda s: "x".join(map(str, s)))
+                                   (2, 130, 8, 128), (2, 7, 8, 192), (3, 4, 5, 37), (4, 11, 9, 100), (3, 3, 8, 201)], ids=lambda s: "x".join(map(str, s)))
 def test_forward_quant_over_clusters(gl, shape):
-    """W8 / A16 at every width the cluster recurrence is built for, 8 and 16 rows per cluster with the last cluster partly
+    """W8 / A16 at every width the cluster recurrence is built for and widths below them, 8 and 16 rows per cluster with the last cluster partly
     empty, and one to five steps (operand and staging buffers alternate)."""
     test_forward_quant_matches_restatement(gl, "a16", shape)
 
