@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kThreads, 1) inputGradUmma(const Problem whole
     __shared__ uint32_t tmemSlot;
     __shared__ int failed;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
     const int rm = lane & 7, cq = lane >> 3;
     const int K = p.K, N = p.N, chunksPerTile = K / kChunkK;
     const uint32_t kBNStride = static_cast<uint32_t>(K / 8) * kCore;  // next 8 columns of the weight operand
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kThreads, 1) inputGradUmma(const Problem whole
         issueChunk(g + kRing, slot);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0 && electOne()) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t aBase = smemAddr(stage), bBase = smemAddr(weights) + kc * (kChunkK / 8) * kCore;
 #pragma unroll

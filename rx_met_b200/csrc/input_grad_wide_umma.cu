@@ -88,7 +88,7 @@ inputGradWideUmma(const Problem p, const WideShape shape, const __grid_constant_
     __shared__ uint32_t tmemSlot;
     __shared__ int failed;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
     const int K = p.K, N = p.N, NP = shape.NP, chunks = K / CH;
     const int ldN = p.ldN ? p.ldN : N;
     const uint32_t bBytes = static_cast<uint32_t>(NP) * CH * 2;
@@ -176,7 +176,7 @@ inputGradWideUmma(const Problem p, const WideShape shape, const __grid_constant_
         }
     } else if (warp == kConvWarps + 2) {
         // ---- MMA issue
-        if (lane == 0) {
+        if (electOne()) {
             const uint32_t idesc = instructionDescriptor(shape.NB, false, false);
             for (int c = 0; c < chunks; ++c) {
                 const int sa = c % kAStages, sb = c % kBRing;

@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
     __shared__ uint32_t tmemSlot;
     __shared__ int failed;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
     const int C = p.C, kWords = p.kWords, kPad = p.kPad;
     const uint32_t groupStride = static_cast<uint32_t>(kPad / 16) * kCore;  // next 8 channels / 8 rows
     uint8_t *weights = smem;                                               // [C / 8][kPad / 16][8][16]
@@ -187,14 +187,15 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
         loadRows(item, stage);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0 && electOne()) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int ct = item % channelTiles;
             const uint32_t aBase = smemAddr(weights) + static_cast<uint32_t>(ct * (kTileM / 8)) * groupStride;
             const uint32_t bBase = smemAddr(rowStages + stage * stageBytes);
+            const uint64_t descA = operandDescriptor(aBase, kCore, groupStride), descB = operandDescriptor(bBase, kCore, groupStride);
+            constexpr uint64_t kStep = (2 * kCore) >> 4;   // the start-address field counts 16-byte units
             for (int ks = 0; ks < kPad / 32; ++ks)
-                mmaI8(tmem + stage * kRows, operandDescriptor(aBase + ks * 2 * kCore, kCore, groupStride),
-                      operandDescriptor(bBase + ks * 2 * kCore, kCore, groupStride), kIdesc, ks > 0 ? 1u : 0u);
+                mmaI8(tmem + stage * kRows, descA + ks * kStep, descB + ks * kStep, kIdesc, ks > 0 ? 1u : 0u);
             commitTo(smemAddr(&bars[stage]));
         }
         if (previous >= 0) epilogue(previous, local - 1);

@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const Problem p, co
     __shared__ uint32_t tmemSlot;
     __shared__ int failed;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
     const int C = p.C, kWords = p.kWords, kPad = paddedK(kWords);
     const uint32_t groupStride = static_cast<uint32_t>(kPad / 16) * kCore;   // next 8 channels / 8 rows
     const uint32_t tileBytes = static_cast<uint32_t>(kChannelTile) * kPad;
@@ -191,15 +191,15 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const Problem p, co
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncthreads();
-            if (tid == 0) {
+            if (warp == 0 && electOne()) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t aBase = smemAddr(aTiles + buf * tileBytes);
+                const uint64_t descA = operandDescriptor(smemAddr(aTiles + buf * tileBytes), kCore, groupStride);
+                constexpr uint64_t kStep = (2 * kCore) >> 4;   // the start-address field counts 16-byte units
 #pragma unroll
                 for (int pl = 0; pl < PLANES; ++pl) {
-                    const uint32_t bBase = smemAddr(rowPlanes + pl * planeBytes);
+                    const uint64_t descB = operandDescriptor(smemAddr(rowPlanes + pl * planeBytes), kCore, groupStride);
                     for (int ks = 0; ks < kPad / 32; ++ks)
-                        mmaI8(tmem + buf * kBufCols + pl * NR, operandDescriptor(aBase + ks * 2 * kCore, kCore, groupStride),
-                              operandDescriptor(bBase + ks * 2 * kCore, kCore, groupStride), kIdesc, ks > 0 ? 1u : 0u);
+                        mmaI8(tmem + buf * kBufCols + pl * NR, descA + ks * kStep, descB + ks * kStep, kIdesc, ks > 0 ? 1u : 0u);
                 }
                 commitTo(smemAddr(&bars[buf]));
             }

@@ -75,7 +75,7 @@ weightGradStreamUmma(const __grid_constant__ StreamSet set, int K, int N, int ch
     __shared__ uint32_t tmemSlot;
     __shared__ int failed;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
     const int n0 = blockIdx.x * NT;
     const int kBegin = blockIdx.y * chunkK, kEnd = min(K, kBegin + chunkK);
     const int chunks = (kEnd - kBegin + kChunkRows - 1) / kChunkRows;
@@ -157,7 +157,7 @@ weightGradStreamUmma(const __grid_constant__ StreamSet set, int K, int N, int ch
         }
     } else if (warp == kConvWarps + 1) {
         // ---- MMA issue
-        if (lane == 0) {
+        if (electOne()) {
             for (int c = 0; c < chunks; ++c) {
                 const int s = c % kStages;
                 await(&stageFull[s], (c / kStages) & 1);
