@@ -190,6 +190,23 @@ def load_library() -> C.CDLL:
     return lib
 
 
+_binding = None
+
+
+def load_binding():
+    """The torch binding of the hot entry points (built beside the library, whose symbols it uses)."""
+    global _binding
+    if _binding is None:
+        load_library()
+        try:
+            import torch  # noqa: F401  its libraries have to be loaded first
+            from . import _binding as module
+        except ImportError as exc:
+            raise RuntimeError(f"the torch binding is not built or does not load ({exc}): make -C rx_met_b200/csrc") from exc
+        _binding = module
+    return _binding
+
+
 def check(status: int, what: str) -> None:
     """Turn a negative ``rxmet_status`` into the exception the reference raises."""
     if status == 0:

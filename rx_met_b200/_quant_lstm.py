@@ -164,7 +164,7 @@ def _mask_tensor(t: torch.Tensor, name: str, shape, device, allow_empty=False):
 
 
 def _backward(p: _Prepared, batch_first, trace4, grad_output, grad_final_hidden, grad_final_cell, master_masks,
-              checkpoint_masks, input_shape, params: Optional[L.ParamsBox]):
+              checkpoint_masks, input_shape):
     lib = _library()
     T, B, I, H = p.dims()
 
@@ -210,16 +210,10 @@ def _backward(p: _Prepared, batch_first, trace4, grad_output, grad_final_hidden,
         setattr(gs, n, t.data_ptr())
     ws, n = _workspace(2, T, B, I, H, p.device)
     with torch.cuda.device(p.device):
-        if params is None:
-            rc = lib.rxmet_lstm_backward_float(T, B, I, H, _ptr(p.w_ih), _ptr(p.w_hh), _ptr(p.x), _ptr(p.h0), _ptr(p.c0),
-                                               _ptr(gates), _ptr(cells), _ptr(ctanh), _ptr(hidden), _ptr(g_out), _ptr(g_hn),
-                                               _ptr(g_cn), C.byref(mk) if mk is not None else None, C.byref(gs), _ptr(ws),
-                                               C.c_size_t(n), _stream())
-        else:
-            rc = lib.rxmet_lstm_backward_qat(T, B, I, H, C.byref(params.struct), _ptr(p.w_ih), _ptr(p.w_hh), _ptr(p.x),
-                                             _ptr(p.h0), _ptr(p.c0), _ptr(gates), _ptr(cells), _ptr(ctanh), _ptr(hidden),
-                                             _ptr(g_out), _ptr(g_hn), _ptr(g_cn), C.byref(mk) if mk is not None else None,
-                                             C.byref(gs), _ptr(ws), C.c_size_t(n), _stream())
+        rc = lib.rxmet_lstm_backward_float(T, B, I, H, _ptr(p.w_ih), _ptr(p.w_hh), _ptr(p.x), _ptr(p.h0), _ptr(p.c0),
+                                           _ptr(gates), _ptr(cells), _ptr(ctanh), _ptr(hidden), _ptr(g_out), _ptr(g_hn),
+                                           _ptr(g_cn), C.byref(mk) if mk is not None else None, C.byref(gs), _ptr(ws),
+                                           C.c_size_t(n), _stream())
     _check(rc, RuntimeError)
     del keep
     if batch_first:
@@ -234,7 +228,7 @@ def lstm_backward_float(input, weight_ih, weight_hh, bias_ih, bias_hh, initial_h
     """Float backward through time: (d_input, d_weight_ih, d_weight_hh, d_bias_ih, d_bias_hh, d_h0, d_c0)."""
     p = _Prepared(input, weight_ih, weight_hh, bias_ih, bias_hh, initial_hidden, initial_cell, batch_first)
     return _backward(p, batch_first, (gate_outputs, cell_states, cell_tanh_outputs, hidden_outputs), grad_output,
-                     grad_final_hidden, grad_final_cell, list(master_masks), list(checkpoint_masks), input.shape, None)
+                     grad_final_hidden, grad_final_cell, list(master_masks), list(checkpoint_masks), input.shape)
 
 
 # --------------------------------------------------------------------------
@@ -253,16 +247,18 @@ def _shortest_float(v) -> str:
     return sci if len(sci) < len(fixed) else fixed
 
 
-def _parse_scale(text) -> np.float32:
-    if not isinstance(text, str):
+def _parse_scales(texts) -> np.ndarray:
+    """float32 values of decimal strings, each rounded through double as numpy parses them."""
+    if not all(isinstance(t, str) for t in texts):
         raise ValueError("scale must be a canonical float32 string")
     try:
-        v = np.float32(text)
+        with np.errstate(over="ignore"):   # out of range becomes infinite and is refused below
+            values = np.array([float(t) for t in texts], np.float64).astype(np.float32)
     except ValueError as e:
         raise ValueError("scale is not a float32 decimal string") from e
-    if not np.isfinite(v) or np.float32(_shortest_float(v)) != v:
+    if not np.isfinite(values).all():
         raise ValueError("scale is not a finite float32")
-    return v
+    return values
 
 
 _BUNDLE_CACHE: dict = {}
@@ -327,7 +323,7 @@ def _parse_bundle(bundle_json: str) -> L.ParamsBox:
         count = 4 * H if op in L.PARAMETER_OPS else 1
         if not isinstance(scales, list) or not isinstance(zps, list) or len(scales) != count or len(zps) != count:
             raise ValueError("quantization parameters must be given as the full 4H list or a single value")
-        values = [_parse_scale(v) for v in scales]
+        values = _parse_scales(scales)
         if op in L.PARAMETER_OPS:
             if any(z != 0 for z in zps):
                 raise ValueError("weight/bias zero points must all be 0")
@@ -445,57 +441,37 @@ def resolve_quant_config(defaults_json: str, override_json: str) -> str:
 # quantized forward / QAT backward
 # --------------------------------------------------------------------------
 
+_MASTER_NAMES = ("input", "weight_ih", "weight_hh", "bias_ih", "bias_hh", "h_0", "c_0")
+
+
 def lstm_forward_quantized(input, weight_ih, weight_hh, bias_ih=None, bias_hh=None, initial_hidden=None,
                            initial_cell=None, batch_first=False, bundle_json="", math_mode="pedantic",
                            require_exact_accumulation=False, save_checkpoints=False):
     """Quantized forward: (output, h_n, c_n, checkpoints, safety).  With save_checkpoints the fourth
     entry holds ``values`` / ``clamp_masks`` (7 per-step tensors each) and ``quantized_master`` /
     ``master_clamp_masks`` (the q-carrier copies of the inputs), as the QAT backward consumes them."""
-    p = _Prepared(input, weight_ih, weight_hh, bias_ih, bias_hh, initial_hidden, initial_cell, batch_first)
-    box = _bundle_to_params(bundle_json)
-    T, B, I, H = p.dims()
-    if box.struct.input_size != I or box.struct.hidden_size != H:
-        raise RuntimeError("quantization parameters do not match input_size / hidden_size of the module")
-    if bool(box.struct.bias_enabled) != (p.b_ih is not None):
-        raise RuntimeError("quantization parameters do not match the bias setting of the module")
-    if math_mode not in ("pedantic", "tf32"):
-        raise ValueError("cublas_math_mode must be pedantic or tf32")
-    ex = _execution(box, require_exact_accumulation)
-    out, hn, cn = p.empty(T, B, H), p.empty(1, B, H), p.empty(1, B, H)
+    try:
+        box = _bundle_to_params(bundle_json)
+        if math_mode not in ("pedantic", "tf32"):
+            raise ValueError("cublas_math_mode must be pedantic or tf32")
+        ex = _execution(box, require_exact_accumulation)
+    except ValueError:   # faults of the tensors are reported before those of the document
+        _Prepared(input, weight_ih, weight_hh, bias_ih, bias_hh, initial_hidden, initial_cell, batch_first)
+        raise
+    status, out, hn, cn, values, clamped, masters, master_clamped = _cabi.load_binding().lstm_forward_quant(
+        input, weight_ih, weight_hh, bias_ih, bias_hh, initial_hidden, initial_cell, batch_first, C.addressof(box.struct),
+        require_exact_accumulation, save_checkpoints)
+    if status != 0:
+        _check(status, RuntimeError)
     checkpoints: dict = {}
-    tr = ms = None
     if save_checkpoints:
-        values = {n: p.empty(T, B, 4 * H if i < 4 else H) for i, n in enumerate(L.TRACE_VALUES)}
-        masks = {n: p.empty(T, B, 4 * H if i < 4 else H, dtype=torch.uint8) for i, n in enumerate(L.TRACE_VALUES)}
-        tr = _trace_struct(values, masks)
-        mv = [torch.empty_like(p.x), torch.empty_like(p.w_ih), torch.empty_like(p.w_hh),
-              p.empty(4 * H) if p.b_ih is not None else p.empty(0), p.empty(4 * H) if p.b_ih is not None else p.empty(0),
-              p.empty(1, B, H), p.empty(1, B, H)]
-        # every flag is written by the library (0 or 1), so the buffers need no zero-fill
-        mm = [torch.empty(v.shape, dtype=torch.bool, device=p.device) for v in mv]
-        ms = L.Masters()
-        for n, v, m in zip(L.MASTER_VALUES, mv, mm):
-            setattr(ms, n, v.data_ptr() if v.numel() else None)
-            setattr(ms, n + "_clamped", m.data_ptr() if m.numel() else None)
-    ws, n = _workspace(1, T, B, I, H, p.device)
-    with torch.cuda.device(p.device):
-        rc = _library().rxmet_lstm_forward_quantized(
-            T, B, I, H, _ptr(p.w_ih), _ptr(p.w_hh), _ptr(p.b_ih), _ptr(p.b_hh), _ptr(p.x), _ptr(p.h0), _ptr(p.c0),
-            C.byref(box.struct), int(require_exact_accumulation), _ptr(out), _ptr(hn), _ptr(cn),
-            C.byref(tr) if tr is not None else None, C.byref(ms) if ms is not None else None, _ptr(ws), C.c_size_t(n),
-            _stream())
-    _check(rc, RuntimeError)
-    if save_checkpoints:
-        names = ("input", "weight_ih", "weight_hh", "bias_ih", "bias_hh", "h_0", "c_0")
-        qm, qk = {}, {}
-        for i, name in enumerate(names):
-            if p.b_ih is None and i in (3, 4):
-                continue
-            v, m = mv[i], mm[i]
-            if i == 0 and batch_first:
-                v, m = v.transpose(0, 1), m.transpose(0, 1)
-            qm[name], qk[name] = v, m
-        checkpoints = {"values": values, "clamp_masks": masks, "quantized_master": qm, "master_clamp_masks": qk}
+        if batch_first:
+            masters[0], master_clamped[0] = masters[0].transpose(0, 1), master_clamped[0].transpose(0, 1)
+        names = [n for i, n in enumerate(_MASTER_NAMES) if bias_ih is not None or i not in (3, 4)]
+        kept = [i for i in range(7) if bias_ih is not None or i not in (3, 4)]
+        checkpoints = {"values": dict(zip(L.TRACE_VALUES, values)), "clamp_masks": dict(zip(L.TRACE_VALUES, clamped)),
+                       "quantized_master": dict(zip(names, (masters[i] for i in kept))),
+                       "master_clamp_masks": dict(zip(names, (master_clamped[i] for i in kept)))}
     return (out.transpose(0, 1) if batch_first else out), hn, cn, checkpoints, _safety_summary(ex)
 
 
@@ -510,10 +486,12 @@ def lstm_backward_qat(master_values, batch_first, bundle_json, checkpoint_values
     bias = bool(box.struct.bias_enabled)
     if not bias and (master_values[3].numel() or master_values[4].numel()):
         raise RuntimeError("bias masters must be empty when bias is disabled")
-    p = _Prepared(master_values[0], master_values[1], master_values[2], master_values[3] if bias else None,
-                  master_values[4] if bias else None, master_values[5], master_values[6], batch_first)
-    return _backward(p, batch_first, checkpoint_values, grad_output, grad_final_hidden, grad_final_cell,
-                     list(master_masks), list(checkpoint_masks), master_values[0].shape, box)
+    status, grads = _cabi.load_binding().lstm_backward_qat(
+        list(master_values), batch_first, C.addressof(box.struct), list(checkpoint_values), grad_output, grad_final_hidden,
+        grad_final_cell, list(master_masks), list(checkpoint_masks))
+    if status != 0:
+        _check(status, RuntimeError)
+    return tuple(grads)
 
 
 # --------------------------------------------------------------------------

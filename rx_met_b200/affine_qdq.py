@@ -12,6 +12,7 @@ here).
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from typing import Optional, Tuple
 
 import torch
@@ -108,10 +109,15 @@ def _checked(tensor, scale, offset):
             offset.detach().to(torch.float32).contiguous())
 
 
-def _layout(x, scale, block_size):
+@functools.lru_cache(maxsize=1024)
+def _cached_layout(tensor_shape, scale_shape, block_size):
     if block_size is None:
-        return grid_layout(x.shape, scale.shape)
-    return grid_layout(*blocked_shapes(x.shape, scale.shape, block_size))
+        return grid_layout(tensor_shape, scale_shape)
+    return grid_layout(*blocked_shapes(tensor_shape, scale_shape, block_size))
+
+
+def _layout(x, scale, block_size):
+    return _cached_layout(x.shape, scale.shape, None if block_size is None else tuple(block_size))
 
 
 def forward(tensor, scale, offset, qmin: int, qmax: int, *, reciprocal: bool, want_keep: bool = False, block_size=None):
@@ -149,25 +155,23 @@ def backward(grad, tensor, scale, offset, qmin: int, qmax: int, *, reciprocal: b
     return (dx, ds.view(scale.shape) if ds is not None else None, do.view(offset.shape) if do is not None else None)
 
 
-class QuantDequantFunc(torch.autograd.Function):
-    """Differentiable quantize-dequantize; saves the input itself instead of a mask (the backward
-    recomputes the flags in the same pass that reads the input for the scale gradient)."""
+def _apply(tensor, scale, offset, qmin, qmax, reciprocal, block_size):
+    if not (tensor.is_cuda and scale.is_cuda and offset.is_cuda):
+        raise RuntimeError("affine_qdq runs on CUDA tensors only")
+    if tensor.dtype != torch.float32:
+        raise RuntimeError("affine_qdq: float32 tensors only")
+    if scale.numel() != offset.numel():
+        raise RuntimeError("affine_qdq: scale and offset differ in size")
+    return cabi.load_binding().quantize_dequantize(tensor, scale, offset, int(qmin), int(qmax), bool(reciprocal),
+                                                   *_cached_layout(tensor.shape, scale.shape, block_size))
+
+
+class QuantDequantFunc:
+    """Differentiable quantize-dequantize: the forward and its autograd node live in the binding."""
 
     @staticmethod
-    def forward(ctx, tensor, scale, offset, qmin: int, qmax: int, reciprocal: bool = False, block_size=None):
-        y, _ = forward(tensor, scale, offset, qmin, qmax, reciprocal=reciprocal, block_size=block_size)
-        ctx.qmin, ctx.qmax, ctx.reciprocal, ctx.block_size = qmin, qmax, reciprocal, block_size
-        ctx.save_for_backward(tensor, scale, offset)
-        return y
-
-    @staticmethod
-    def backward(ctx, grad):
-        tensor, scale, offset = ctx.saved_tensors
-        need = ctx.needs_input_grad
-        dx, ds, do = backward(grad, tensor, scale, offset, ctx.qmin, ctx.qmax, reciprocal=ctx.reciprocal,
-                              want_tensor_grad=need[0], want_scale_grad=need[1], want_offset_grad=need[2],
-                              block_size=ctx.block_size)
-        return dx, ds, do, None, None, None, None
+    def apply(tensor, scale, offset, qmin: int, qmax: int, reciprocal: bool = False, block_size=None):
+        return _apply(tensor, scale, offset, qmin, qmax, reciprocal, None if block_size is None else tuple(block_size))
 
 
 def quantize_dequantize(tensor: torch.Tensor, scale: torch.Tensor, offset: torch.Tensor, qmin: int, qmax: int,
@@ -179,5 +183,4 @@ def quantize_dequantize(tensor: torch.Tensor, scale: torch.Tensor, offset: torch
     trained = (scale.requires_grad or offset.requires_grad) and torch.is_grad_enabled()
     # blockwise grids always take the divide form: the reference's fast path does not handle them
     reciprocal = not trained and block_size is None
-    return QuantDequantFunc.apply(tensor, scale, offset, qmin, qmax, reciprocal,
-                                  None if block_size is None else tuple(block_size))
+    return _apply(tensor, scale, offset, qmin, qmax, reciprocal, None if block_size is None else tuple(block_size))

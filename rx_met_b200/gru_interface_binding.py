@@ -16,6 +16,7 @@ the dtype of the returned code caches, exactly as the reference's CPU build does
 from __future__ import annotations
 
 import ctypes as C
+from array import array
 from typing import List, Optional, Tuple
 
 import torch
@@ -138,6 +139,15 @@ def _range_stem(op: int) -> str:
     return _RANGE_STEM.get(op, cabi.OP_NAMES[op])
 
 
+_RANGE_ATTRS = tuple((op, f"min_{_range_stem(op)}_", f"max_{_range_stem(op)}_") for op in cabi.SCALAR_OPS)
+_CHANNEL_ATTRS = tuple(f"{kind}_{name}_" for name in _CHANNEL_NAMES for kind in ("min", "max"))
+
+
+def _float_pointer(values: array):
+    """ctypes view of an array of floats (the array has to outlive it)."""
+    return C.cast(values.buffer_info()[0], C.POINTER(C.c_float))
+
+
 class GRUQuantizationRanges:
     """min/max per quantization point (``min_x_`` ... ``max_mul_old_contribution_``) plus
     per-channel lists for W, R, bw, br; ``reset`` restores (FLT_MAX, -FLT_MAX)."""
@@ -149,41 +159,38 @@ class GRUQuantizationRanges:
     def reset(self, hidden: int = -1) -> None:
         if hidden > 0:
             self.hidden_ = int(hidden)
-        for op in cabi.SCALAR_OPS:
-            setattr(self, f"min_{_range_stem(op)}_", _FMAX)
-            setattr(self, f"max_{_range_stem(op)}_", -_FMAX)
+        for _, low, high in _RANGE_ATTRS:
+            setattr(self, low, _FMAX)
+            setattr(self, high, -_FMAX)
         n = 3 * self.hidden_
-        for name in _CHANNEL_NAMES:
-            setattr(self, f"min_{name}_", [_FMAX] * n)
-            setattr(self, f"max_{name}_", [-_FMAX] * n)
+        for attr in _CHANNEL_ATTRS:
+            setattr(self, attr, [_FMAX if attr.startswith("min") else -_FMAX] * n)
 
     # ---- C struct round trip
     def _to_c(self):
         n = 3 * self.hidden_
         c = cabi.Ranges()
         c.hidden = self.hidden_
-        for op in cabi.SCALAR_OPS:
-            c.min[op] = getattr(self, f"min_{_range_stem(op)}_")
-            c.max[op] = getattr(self, f"max_{_range_stem(op)}_")
+        lows, highs = c.min, c.max
+        for op, low, high in _RANGE_ATTRS:
+            lows[op] = getattr(self, low)
+            highs[op] = getattr(self, high)
         keep = []
-        for name in _CHANNEL_NAMES:
-            for kind in ("min", "max"):
-                values = list(getattr(self, f"{kind}_{name}_"))
-                if len(values) != n:
-                    raise ValueError(f"{kind}_{name}_ must hold 3*hidden = {n} values")
-                arr = (C.c_float * n)(*values)
-                keep.append(arr)
-                setattr(c, f"{kind}_{name}", C.cast(arr, C.POINTER(C.c_float)))
+        for attr in _CHANNEL_ATTRS:
+            values = array("f", getattr(self, attr))
+            if len(values) != n:
+                raise ValueError(f"{attr} must hold 3*hidden = {n} values")
+            keep.append(values)
+            setattr(c, attr[:-1], _float_pointer(values))
         return c, keep
 
     def _from_c(self, c, keep) -> None:
-        for op in cabi.SCALAR_OPS:
-            setattr(self, f"min_{_range_stem(op)}_", float(c.min[op]))
-            setattr(self, f"max_{_range_stem(op)}_", float(c.max[op]))
-        it = iter(keep)
-        for name in _CHANNEL_NAMES:
-            for kind in ("min", "max"):
-                setattr(self, f"{kind}_{name}_", list(next(it)))
+        lows, highs = list(c.min), list(c.max)
+        for op, low, high in _RANGE_ATTRS:
+            setattr(self, low, lows[op])
+            setattr(self, high, highs[op])
+        for attr, values in zip(_CHANNEL_ATTRS, keep):
+            setattr(self, attr, values.tolist())
 
 
 class GRUHistogramCollectors:
@@ -328,17 +335,9 @@ def calculate_gru_quantitative_parameters_from_histograms(hist_collectors, bitwi
 # device plumbing
 # --------------------------------------------------------------------------
 
-_workspaces = {}
-
-
 def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     """One growing scratch buffer per device and stream, reused across calls."""
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
-    return buf
+    return cabi.load_binding().workspace(device.index, nbytes)
 
 
 def _check_f32(t: torch.Tensor, name: str, shape: Optional[Tuple[int, ...]] = None) -> torch.Tensor:
@@ -424,36 +423,24 @@ def forward_calibrate(is_training, time_steps, batch_size, input_size, hidden_si
     dev = x.device
     h = torch.empty((T + 1, B, H), dtype=torch.float32, device=dev)
     v = torch.empty((T, B, 4 * H), dtype=torch.float32, device=dev)
-    ranges, keep = quant_ranges._to_c()
-    nbytes = lib.rxmet_gru_workspace_bytes(0, T, B, I, H)
-    ws = _workspace(dev, nbytes)
+    ws = _workspace(dev, lib.rxmet_gru_workspace_bytes(0, T, B, I, H))
+    stats = torch.empty(lib.rxmet_gru_stats_floats(H), dtype=torch.float32, device=dev)
+    with torch.cuda.device(dev):
+        cabi.check(lib.rxmet_gru_forward_calibrate_stats(
+            T, B, I, H, _ptr(W), _ptr(R), _ptr(bw), _ptr(br), _ptr(x), _ptr(h0v), _ptr(h), _ptr(v), _ptr(stats),
+            _ptr(ws), C.c_size_t(ws.numel()), _stream(dev)), "forward_calibrate")
     if _calibration_group is not None:
         # sharded batch: the packed extremes of this rank's shard are all-reduced before they are folded
         import torch.distributed as dist
-        stats = torch.empty(lib.rxmet_gru_stats_floats(H), dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
-            cabi.check(lib.rxmet_gru_forward_calibrate_stats(
-                T, B, I, H, _ptr(W), _ptr(R), _ptr(bw), _ptr(br), _ptr(x), _ptr(h0v), _ptr(h), _ptr(v), _ptr(stats),
-                _ptr(ws), C.c_size_t(ws.numel()), _stream(dev)), "forward_calibrate")
         half = stats.numel() // 2
         dist.all_reduce(stats[:half], op=dist.ReduceOp.MIN, group=_calibration_group)
         dist.all_reduce(stats[half:], op=dist.ReduceOp.MAX, group=_calibration_group)
-        host = stats.cpu().contiguous()
-        cabi.check(lib.rxmet_gru_ranges_fold_stats(C.byref(ranges), C.cast(host.data_ptr(), C.POINTER(C.c_float))),
-                   "ranges_fold_stats")
-    else:
-        with torch.cuda.device(dev):
-            cabi.check(lib.rxmet_gru_forward_calibrate_minmax(
-                T, B, I, H, _ptr(W), _ptr(R), _ptr(bw), _ptr(br), _ptr(x), _ptr(h0v), _ptr(h), _ptr(v),
-                C.byref(ranges), _ptr(ws), C.c_size_t(ws.numel()), _stream(dev)), "forward_calibrate")
+    ranges, keep = quant_ranges._to_c()   # while the kernels run
+    host = stats.cpu()
+    cabi.check(lib.rxmet_gru_ranges_fold_stats(C.byref(ranges), C.cast(host.data_ptr(), C.POINTER(C.c_float))),
+               "ranges_fold_stats")
     quant_ranges._from_c(ranges, keep)
     return h, v
-
-
-_MASK_SHAPES = lambda T, B, I, H: {  # noqa: E731
-    "x": (T, B, I), "h0": (B, H), "W": (I, 3 * H), "R": (H, 3 * H), "bw": (3 * H,), "br": (3 * H,),
-    "weight_ih_linear": (T, B, 3 * H), "weight_hh_linear": (T, B, 3 * H), "gate_input": (T, B, 3 * H),
-    "gate_output": (T, B, 3 * H), "h": (T, B, H)}
 
 
 def _carve(device, dtype, shapes):
@@ -495,42 +482,14 @@ def float_storage_carrier():
 
 
 def _forward_quant(is_training, T, B, I, H, W, R, bw, br, x, h0, quant_params, code_dtype, fp_carrier=False):
-    lib = cabi.load_library()
-    W, R, bw, br, x, h0v = _common_inputs(T, B, I, H, W, R, bw, br, x, h0)
-    dev = x.device
-    params, keep = quant_params._to_c()
-    h = torch.empty((T + 1, B, H), dtype=torch.float32, device=dev)
-    v = torch.empty((T, B, 4 * H), dtype=torch.float32, device=dev)
-    code_shapes = {"W_q": (I, 3 * H), "R_q": (H, 3 * H), "bw_q": (3 * H,), "br_q": (3 * H,), "x_q": (T, B, I)}
-    codes = dict(zip(code_shapes, _carve(dev, torch.int32, list(code_shapes.values()))))
-    mask_struct = cabi.Masks()
-    shapes = _MASK_SHAPES(T, B, I, H)
-    wanted = [name for name in shapes if is_training and not (name == "h0" and h0v is None)]
-    masks = dict(zip(wanted, _carve(dev, torch.uint8, [shapes[name] for name in wanted]))) if wanted else {}
-    empty = None
-    for name in shapes:
-        if name in masks:
-            setattr(mask_struct, name, masks[name].data_ptr())
-        else:
-            if empty is None:
-                empty = torch.empty((0,), dtype=torch.uint8, device=dev)
-            masks[name] = empty
-    ws = _workspace(dev, lib.rxmet_gru_workspace_bytes(1, T, B, I, H))
-    with torch.cuda.device(dev):
-        entry = lib.rxmet_gru_forward_quant_fp_carrier if fp_carrier else lib.rxmet_gru_forward_quant
-        cabi.check(entry(
-            int(bool(is_training)), T, B, I, H, _ptr(W), _ptr(R), _ptr(bw), _ptr(br), _ptr(x), _ptr(h0v),
-            C.byref(params), _ptr(h), _ptr(v), _ptr(codes["W_q"]), _ptr(codes["R_q"]), _ptr(codes["bw_q"]),
-            _ptr(codes["br_q"]), _ptr(codes["x_q"]), None, None,
-            C.byref(mask_struct) if is_training else None, _ptr(ws), C.c_size_t(ws.numel()), _stream(dev)),
-            "forward_quant")
-    del keep
+    params, _ = quant_params._to_c()
+    status, out = cabi.load_binding().gru_forward_quant(bool(is_training), T, B, I, H, W, R, bw, br, x, h0,
+                                                        C.addressof(params), fp_carrier)
+    if status != 0:
+        cabi.check(status, "forward_quant")
     if code_dtype != torch.int32:
-        codes = {k: t.to(code_dtype) for k, t in codes.items()}
-    return (h, v, codes["W_q"], codes["R_q"], codes["bw_q"], codes["br_q"], codes["x_q"],
-            masks["x"], masks["h0"], masks["W"], masks["R"], masks["bw"], masks["br"],
-            masks["weight_ih_linear"], masks["weight_hh_linear"], masks["gate_input"], masks["gate_output"],
-            masks["h"])
+        out[2:7] = [t.to(code_dtype) for t in out[2:7]]
+    return tuple(out)
 
 
 def forward_quant_int_storage(is_training, time_steps, batch_size, input_size, hidden_size, W, R, bw, br, x, h0,
@@ -577,36 +536,12 @@ def forward_quantized_int_io(time_steps, batch_size, input_size, hidden_size, W,
 
 
 def _backward_quant(T, B, I, H, W_q, R_q, bw_q, br_q, x_q, dh_new, h, v, quant_params, masks: List[torch.Tensor]):
-    lib = cabi.load_library()
-    dev = h.device
-    codes = []
-    for t, name, shape in ((W_q, "W_q", (I, 3 * H)), (R_q, "R_q", (H, 3 * H)), (bw_q, "bw_q", (3 * H,)),
-                           (br_q, "br_q", (3 * H,)), (x_q, "x_q", (T, B, I))):
-        if not t.is_cuda or tuple(t.shape) != shape:
-            raise RuntimeError(f"{name} must be a CUDA tensor of shape {list(shape)}")
-        codes.append(t.to(torch.int32).contiguous())
-    dh_new = _check_f32(dh_new, "dh_new", (T + 1, B, H))
-    h = _check_f32(h, "h", (T + 1, B, H))
-    v = _check_f32(v, "v", (T, B, 4 * H))
-    params, keep = quant_params._to_c()
-    mask_struct = cabi.Masks()
-    live = []
-    for name, m in zip(cabi.MASK_NAMES, masks):
-        if m is not None and m.numel() > 0:
-            m = m.contiguous()
-            live.append(m)
-            setattr(mask_struct, name, m.data_ptr())
-    dx, dW, dR, dbw, dbr, dh0 = _carve(dev, torch.float32,
-                                       [(T, B, I), (I, 3 * H), (H, 3 * H), (3 * H,), (3 * H,), (B, H)])
-    ws = _workspace(dev, lib.rxmet_gru_workspace_bytes(2, T, B, I, H))
-    with torch.cuda.device(dev):
-        cabi.check(lib.rxmet_gru_backward_quant(
-            T, B, I, H, _ptr(codes[0]), _ptr(codes[1]), _ptr(codes[2]), _ptr(codes[3]), _ptr(codes[4]),
-            _ptr(dh_new), _ptr(h), _ptr(v), C.byref(params), C.byref(mask_struct),
-            _ptr(dx), _ptr(dW), _ptr(dR), _ptr(dbw), _ptr(dbr), _ptr(dh0),
-            _ptr(ws), C.c_size_t(ws.numel()), _stream(dev)), "backward_quant")
-    del keep, live
-    return dx, dW, dR, dbw, dbr, dh0
+    params, _ = quant_params._to_c()
+    status, out = cabi.load_binding().gru_backward_quant(T, B, I, H, (W_q, R_q, bw_q, br_q, x_q), dh_new, h, v,
+                                                         C.addressof(params), masks)
+    if status != 0:
+        cabi.check(status, "backward_quant")
+    return tuple(out)
 
 
 def backward_quant_int_storage(time_steps, batch_size, input_size, hidden_size, W_q, R_q, bw_q, br_q, x_q, dh_new,
