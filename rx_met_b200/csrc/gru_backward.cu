@@ -1121,9 +1121,9 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         float *Wf = ws.take<float>(static_cast<size_t>(I) * C);
         float *Rf = ws.take<float>(static_cast<size_t>(H) * C);
         float *xf = ws.take<float>(rows * I);
-        float *chan = ws.take<float>(2 * static_cast<size_t>(C));
-        // effective scales of W then R: the first two arrays of the page-locked per-channel block
-        RXMET_CUDA(cudaMemcpyAsync(chan, pinnedChannelBlock(e, st), 2 * sizeof(float) * C, cudaMemcpyHostToDevice, st));
+        // effective scales of W then R: the first two arrays of the per-channel block
+        const size_t chanWords = 2 * static_cast<size_t>(C);
+        const float *chan = reinterpret_cast<const float *>(channelBlockOnDevice(e, ws.take<int32_t>(chanWords), chanWords, st));
         if (!tensorInputGrad) {
             KernelTimer timer__("dequantCodes", st);
             dequantCodes<<<gridFor(static_cast<size_t>(I) * C, 256), 256, 0, st>>>(call.W_q, static_cast<size_t>(I) * C, C, chan, 0.f, 0, Wf);

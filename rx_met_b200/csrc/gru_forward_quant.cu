@@ -28,10 +28,12 @@
 #include <vector>
 
 #include "common.h"
+#include "dependent_launch.cuh"
 #include "gru_device.cuh"
 #include "gru_forward_quant.h"
 #include "gru_forward_wide.h"
 #include "input_proj_umma.h"
+#include "plane_proj_umma.cuh"
 
 namespace rxmet {
 namespace gru {
@@ -40,25 +42,52 @@ namespace gru {
 // evicts old entries.  A copy recorded into a CUDA graph reads the block again at every replay, long
 // after the call returned, so a block handed out while the stream is being captured is kept for the
 // life of the process (one block per captured parameter set; a few tens of KB each).
-const int32_t *pinnedChannelBlock(const Exec &e, cudaStream_t st) {
-    std::call_once(e.pinnedOnce, [&] {
-        const size_t C = 3 * static_cast<size_t>(e.hidden);
-        int32_t *host = nullptr;
-        RXMET_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&host), 12 * C * sizeof(int32_t), cudaHostAllocDefault));
-        e.pinnedChannels = std::shared_ptr<int32_t>(host, [](int32_t *ptr) { cudaFreeHost(ptr); });
-        auto putF = [&](size_t slot, const std::vector<float> &v) { std::memcpy(host + slot * C, v.data(), C * 4); };
-        auto putR = [&](size_t slot, const std::vector<Rescale> &v) { std::memcpy(host + slot * C, v.data(), C * 8); };
-        putF(0, e.chan.eff_W); putF(1, e.chan.eff_R); putF(2, e.chan.eff_bw); putF(3, e.chan.eff_br);
-        putR(4, e.chan.gemm_x); putR(6, e.chan.bias_x); putR(8, e.chan.gemm_h); putR(10, e.chan.bias_h);
-    });
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone) {
-        static std::mutex mutex;
-        static std::vector<std::shared_ptr<int32_t>> captured;
-        std::lock_guard<std::mutex> lock(mutex);
-        if (std::find(captured.begin(), captured.end(), e.pinnedChannels) == captured.end()) captured.push_back(e.pinnedChannels);
+namespace {
+
+std::vector<int32_t> channelBlock(const Exec &e) {
+    const size_t C = 3 * static_cast<size_t>(e.hidden);
+    std::vector<int32_t> host(12 * C);
+    auto putF = [&](size_t slot, const std::vector<float> &v) { std::memcpy(host.data() + slot * C, v.data(), C * 4); };
+    auto putR = [&](size_t slot, const std::vector<Rescale> &v) { std::memcpy(host.data() + slot * C, v.data(), C * 8); };
+    putF(0, e.chan.eff_W); putF(1, e.chan.eff_R); putF(2, e.chan.eff_bw); putF(3, e.chan.eff_br);
+    putR(4, e.chan.gemm_x); putR(6, e.chan.bias_x); putR(8, e.chan.gemm_h); putR(10, e.chan.bias_h);
+    return host;
+}
+
+}  // namespace
+
+const int32_t *channelBlockOnDevice(const Exec &e, int32_t *scratch, size_t words, cudaStream_t st) {
+    const int device = currentDevice().device;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const bool capturing = cudaStreamIsCapturing(st, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
+    static std::mutex mutex;
+    static std::vector<std::shared_ptr<int32_t>> captured;   // blocks a graph refers to stay for good
+    auto keep = [&](const std::shared_ptr<int32_t> &block) {
+        if (capturing && std::find(captured.begin(), captured.end(), block) == captured.end()) captured.push_back(block);
+    };
+    std::lock_guard<std::mutex> lock(mutex);
+    for (const auto &entry : e.deviceChannels)
+        if (entry.first == device) {
+            keep(entry.second);
+            return entry.second.get();
+        }
+    const std::vector<int32_t> host = channelBlock(e);
+    const size_t bytes = host.size() * sizeof(int32_t);
+    int32_t *buffer = nullptr;
+    if (capturing) {   // nothing may be allocated on the device now: the graph copies from page-locked memory
+        RXMET_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&buffer), bytes, cudaHostAllocDefault));
+        const std::shared_ptr<int32_t> block(buffer, [](int32_t *ptr) { cudaFreeHost(ptr); });
+        std::memcpy(buffer, host.data(), bytes);
+        keep(block);
+        RXMET_CUDA(cudaMemcpyAsync(scratch, buffer, words * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+        return scratch;
     }
-    return e.pinnedChannels.get();
+    RXMET_CUDA(cudaMalloc(reinterpret_cast<void **>(&buffer), bytes));
+    const std::shared_ptr<int32_t> block(buffer, [](int32_t *ptr) { cudaFree(ptr); });
+    // synchronous: the source is pageable and the copy is shared by every stream
+    RXMET_CUDA(cudaMemcpy(buffer, host.data(), bytes, cudaMemcpyHostToDevice));
+    e.deviceChannels.emplace_back(device, block);
+    return buffer;
 }
 
 namespace {
@@ -190,11 +219,14 @@ struct WeightPrepArgs {
     int32_t *xCodes32;
     uint8_t *xMask;
     int prepBlocks;
+    int *clear;   // status word of a later kernel, set to 0 here
 };
 
 constexpr int kPrepLayers = 32;
 __global__ void __launch_bounds__(32 * kPrepLayers) prepareWeightsI8(const WeightPrepArgs a) {
     __shared__ int32_t sums[2][kPrepLayers][32];
+    letDependentsStart();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.clear = 0;
     if (static_cast<int>(blockIdx.x) >= a.prepBlocks) {  // the input tensor's blocks
         const size_t total = static_cast<size_t>(a.xRows) * a.xColsPadded;
         const size_t stride = static_cast<size_t>(gridDim.x - a.prepBlocks) * blockDim.x;
@@ -268,6 +300,120 @@ __global__ void __launch_bounds__(32 * kPrepLayers) prepareWeightsI8(const Weigh
     a.biasX[c] = applyRescale(static_cast<int64_t>(qBw), a.biasRescaleX[c]);
     a.compH[c] = totalR * a.zpH;
     a.biasH[c] = applyRescale(static_cast<int64_t>(qBr), a.biasRescaleH[c]);
+}
+
+// The same preparation for the byte-plane path (gru_forward_wide.cu) in ONE launch instead of fourteen: the parameter codes
+// as packed words (the input weights also as tensor-core tiles), both addends, and x and h0 as byte planes.  Blocks by job:
+// 32 channels, then words of x, then words of h0.  T = 98, B = 32, I = 40, H = 64: 64 -> 5 us of launches.
+struct WidePrepArgs {
+    const float *W, *R, *bw, *br;
+    int I, H, C, kI, kH, tileWords;                // tileWords: words of a channel's row in a tile, k padding included
+    const float *effW, *effR, *effBw, *effBr;
+    int32_t loW, hiW, loR, hiR, loBw, hiBw, loBr, hiBr;
+    uint32_t *wWords, *rWords, *tiles;
+    int32_t *W_q, *R_q, *bw_q, *br_q;              // optional 32-bit copies of the codes
+    uint8_t *mW, *mR, *mBw, *mBr;                  // optional clamp flags
+    int64_t zeroX, zeroH;                          // grid minimum - zero point of x and h
+    const Rescale *biasRescaleX, *biasRescaleH;
+    int64_t *addX, *addH;
+    struct Rows {                                  // a tensor that becomes byte planes [rows][2][kWords]
+        const float *src;                          // null: codes from `given`, and without these the zero point
+        const int32_t *given;
+        int rows, cols, kWords;
+        float scale;
+        int32_t zp, lo, hi;
+        uint32_t *planes;
+        int32_t *codes32;                          // optional
+        uint8_t *mask;                             // optional
+        int16_t *codes;                            // optional [rows][colsPadded]
+        int colsPadded;
+    } x, h0;
+    int prepBlocks, xBlocks, h0Blocks;
+    int *clear;                                    // status word of a later kernel, set to 0 here
+};
+__device__ __forceinline__ void planesOf(const WidePrepArgs::Rows &t, int block, int blocks) {
+    const size_t total = static_cast<size_t>(t.rows) * t.kWords, stride = static_cast<size_t>(blocks) * blockDim.x;
+    for (size_t i = static_cast<size_t>(block) * blockDim.x + threadIdx.x; i < total; i += stride) {
+        const size_t r = i / t.kWords;
+        const int kw = static_cast<int>(i - r * t.kWords);
+        uint32_t high = 0, low = 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int k = 4 * kw + e;
+            if (k >= t.cols) continue;
+            const size_t at = r * t.cols + k;
+            int32_t q = t.zp;
+            if (t.src != nullptr) {
+                uint8_t keep;
+                q = quantizeValue(t.src[at], t.scale, t.zp, t.lo, t.hi, keep);
+                if (t.mask) t.mask[at] = keep;
+            } else if (t.given != nullptr) {
+                q = t.given[at];
+            }
+            if (t.codes32) t.codes32[at] = q;
+            if (t.codes) t.codes[r * t.colsPadded + k] = static_cast<int16_t>(q);
+            const uint32_t u = static_cast<uint32_t>(q - t.lo);
+            low |= (u & 0xffu) << (8 * e);
+            high |= ((u >> 8) & 0xffu) << (8 * e);
+        }
+        t.planes[(2 * r) * t.kWords + kw] = high;
+        t.planes[(2 * r + 1) * t.kWords + kw] = low;
+    }
+}
+__global__ void __launch_bounds__(32 * kPrepLayers) prepareWide(const __grid_constant__ WidePrepArgs a) {
+    __shared__ int32_t sums[2][kPrepLayers][32];
+    letDependentsStart();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.clear = 0;
+    const int block = static_cast<int>(blockIdx.x) - a.prepBlocks;
+    if (block >= a.xBlocks) return planesOf(a.h0, block - a.xBlocks, a.h0Blocks);
+    if (block >= 0) return planesOf(a.x, block, a.xBlocks);
+    const int cl = threadIdx.x & 31, layer = threadIdx.x >> 5, c = blockIdx.x * 32 + cl;
+    const bool live = c < a.C;
+    auto pass = [&](const float *__restrict__ src, int rowsK, int words, int allWords, float scale, int32_t lo, int32_t hi,
+                    uint32_t *__restrict__ packed, uint32_t *__restrict__ tiles, int32_t *__restrict__ codes32, uint8_t *__restrict__ mask) {
+        int32_t sum = 0;
+        for (int kk = layer; kk < allWords; kk += kPrepLayers) {
+            float v[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) v[b] = live && 4 * kk + b < rowsK ? src[static_cast<size_t>(4 * kk + b) * a.C + c] : 0.0f;
+            uint32_t word = 0;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int k = 4 * kk + b;
+                if (!live || k >= rowsK) continue;
+                const size_t at = static_cast<size_t>(k) * a.C + c;
+                uint8_t keep;
+                const int32_t q = quantizeValue(v[b], scale, 0, lo, hi, keep);
+                if (codes32) codes32[at] = q;
+                if (mask) mask[at] = keep;
+                sum += q;
+                word |= static_cast<uint32_t>(q & 0xff) << (8 * b);
+            }
+            if (live && kk < words) packed[static_cast<size_t>(kk) * a.C + c] = word;
+            // canonical tile (packTiles in plane_proj_umma.cuh): 128 channels x tileWords, 16-byte rows of core matrices
+            if (tiles) tiles[static_cast<size_t>(c / 128) * (128 * a.tileWords) + (c % 128 / 8) * (8 * a.tileWords) + (kk / 4) * 32 + (c % 8) * 4 + kk % 4] = word;
+        }
+        return sum;
+    };
+    sums[0][layer][cl] = pass(a.W, a.I, a.kI, a.tiles ? a.tileWords : a.kI, live ? a.effW[c] : 1.0f, a.loW, a.hiW, a.wWords, a.tiles, a.W_q, a.mW);
+    sums[1][layer][cl] = pass(a.R, a.H, a.kH, a.kH, live ? a.effR[c] : 1.0f, a.loR, a.hiR, a.rWords, nullptr, a.R_q, a.mR);
+    __syncthreads();
+    if (layer != 0 || !live) return;
+    int64_t totalW = 0, totalR = 0;
+#pragma unroll
+    for (int l = 0; l < kPrepLayers; ++l) {
+        totalW += sums[0][l][cl];
+        totalR += sums[1][l][cl];
+    }
+    uint8_t keep;
+    const int32_t qBw = quantizeValue(a.bw[c], a.effBw[c], 0, a.loBw, a.hiBw, keep);
+    if (a.bw_q) a.bw_q[c] = qBw;
+    if (a.mBw) a.mBw[c] = keep;
+    const int32_t qBr = quantizeValue(a.br[c], a.effBr[c], 0, a.loBr, a.hiBr, keep);
+    if (a.br_q) a.br_q[c] = qBr;
+    if (a.mBr) a.mBr[c] = keep;
+    a.addX[c] = totalW * a.zeroX + applyRescale(static_cast<int64_t>(qBw), a.biasRescaleX[c]);
+    a.addH[c] = totalR * a.zeroH + applyRescale(static_cast<int64_t>(qBr), a.biasRescaleH[c]);
 }
 
 // Epilogue shared by both linear stages (gru_forward_gpu_quant.cu:163-178).
@@ -367,6 +513,8 @@ inputLinearI8(const int32_t *__restrict__ x, int rows, int kWords, int channels,
     __shared__ __align__(16) int32_t xs[2][kI8Rows][kRowWords];
     const int tid = threadIdx.x, c = tid;
     const bool live = c < channels;
+    waitForPredecessor();
+    letDependentsStart();
     int32_t wreg[kRowWords];
 #pragma unroll
     for (int kk = 0; kk < kRowWords; ++kk) wreg[kk] = (live && kk < kWords) ? w[static_cast<size_t>(kk) * channels + c] : 0;
@@ -849,6 +997,352 @@ recurrentForwardI8(const __grid_constant__ RecurrentArgs a, const __grid_constan
     }
 }
 
+// ---- 4c. the recurrence for small 8-bit grids and at most 128 hidden units: lanes of a warp share a unit ----------
+//
+// In recurrentForwardI8 (4b) a step crosses shared memory and a barrier twice (hidden codes -> linear codes -> cell),
+// waits for ih terms that were loaded one step ahead (about an L2 latency), leaves two thirds of the threads idle in
+// the cell and issues 400 instructions per thread.  Here LPU lanes own a hidden unit: each multiplies its part of K for
+// the three gates (weights in registers), shuffles add the parts so that a lane holds all three sums of its row, and the
+// cell follows in the same registers: ONE barrier per step.  With BT = LPU rows every lane computes a row of its own;
+// one row alone takes LPU = 4, which shortens the sums, and its four lanes compute the same element and share its stores.
+// Hidden codes alternate between two buffers, ih terms are loaded two steps ahead (two register sets, the loop unrolled
+// by two), outputs of step t are stored under the products of step t + 1.  What then bounds a step is the number of
+// instructions and their chain, so
+//   - all codes are kept as differences to their zero points, and the tables hold differences too,
+//   - the rescale of the candidate to the h grid is part of the candidate's table,
+//   - a rounding shift is an add of one half, a shift and, for the exact ties, a cleared lowest bit,
+//   - step offsets are added to uniform pointers, a lane keeps 32-bit offsets inside a step,
+//   - lanes beyond the last unit or row repeat the last one (same values to the same places) instead of branching.
+// T = 98, B = 1, I = 40, H = 64: 59.7 -> 29.6 us (0.30 us a step, 140 instructions per warp); T = 100, B = 256, H = 128 with
+// packed flags: 110 -> 64 us; T = 61, B = 45, H = 100 with byte flags: 50 -> 43 us.
+//
+// One rounding rescale, half to even, of a product that has half a unit added already: the floor is right except for an
+// exact tie, where it is the upper neighbour and an odd one must step down.  mask = 2^n - 1 (n = 0: half 0, mask all ones).
+__device__ __forceinline__ int32_t roundTies(int32_t floorOfSum, uint32_t low, uint32_t mask) {
+    return (low & mask) == 0 ? floorOfSum & ~1 : floorOfSum;
+}
+struct RoundingShift {
+    int32_t mult, shift, half;
+    uint32_t mask;
+};
+__device__ __forceinline__ RoundingShift roundingShift(Rescale r) {   // 0 <= shift <= 31
+    const int32_t half = r.shift ? static_cast<int32_t>(1u << (r.shift - 1)) : 0;
+    return {r.mult, r.shift, half, r.shift ? (1u << r.shift) - 1u : 0xffffffffu};
+}
+__device__ __forceinline__ int32_t rescaleSmallTies(int32_t x, const RoundingShift &r) {   // |x * mult| + half < 2^31
+    const int32_t v = x * r.mult + r.half;
+    return roundTies(v >> r.shift, static_cast<uint32_t>(v), r.mask);
+}
+__device__ __forceinline__ int32_t roundWideTies(int64_t sum, int32_t shift, uint32_t mask) {   // quotient fits 32 bits
+    const uint32_t low = static_cast<uint32_t>(sum), high = static_cast<uint32_t>(static_cast<uint64_t>(sum) >> 32);
+    return roundTies(static_cast<int32_t>(__funnelshift_r(low, high, shift)), low, mask);
+}
+
+enum class FlagForm { None, Bytes, Packed, Codes };   // Codes: byte flags and integer codes, whichever are asked for
+
+// KW: words of four codes that hold a row of hidden codes (H <= 4 KW)
+template <int KW, int LPU, int BT, FlagForm Flags>
+__global__ void __launch_bounds__(4 * KW * LPU)
+recurrentLanesI8(const __grid_constant__ RecurrentArgs a, const __grid_constant__ GateExec g) {
+    static_assert(BT == 1 || BT == LPU, "a lane has one row");
+    constexpr int kPadded = 4 * KW;      // hidden codes of a row
+    constexpr int KWQ = KW / LPU;        // words of a lane's part of K
+    constexpr int kLanes = LPU / BT;     // lanes that share an element
+    constexpr bool kFlags = Flags != FlagForm::None;
+    constexpr int kAhead = 2;            // steps that ih terms are loaded ahead (four measure the same)
+    __shared__ __align__(16) int8_t hS[2][BT][kPadded];
+    extern __shared__ __align__(16) unsigned char smemRaw[];
+
+    const int H = a.H, C = 3 * a.H;
+    const int tid = threadIdx.x, nthreads = blockDim.x;
+    const int b0 = blockIdx.x * BT, nb = min(BT, a.B - b0);
+    const int32_t zpZ = g.zp[RXMET_GRU_UPDATE_GATE_OUTPUT], zpR = g.zp[RXMET_GRU_RESET_GATE_OUTPUT];
+    const int32_t zpN = g.zp[RXMET_GRU_NEW_GATE_OUTPUT], zpH = g.zp[RXMET_GRU_H], zpHh = g.zp[RXMET_GRU_WEIGHT_HH_LINEAR];
+
+    // activation tables over the gate-input grids; an entry is (output code - zero point) << 16 | inside the grid << gate,
+    // that of the candidate followed by its value on the h grid
+    int2 *tabN = reinterpret_cast<int2 *>(smemRaw);
+    int32_t last[3], toIndex[3];   // highest index; zero point - grid minimum
+    int32_t *tabZ, *tabR;
+    {
+        const int inOp[3] = {RXMET_GRU_UPDATE_GATE_INPUT, RXMET_GRU_RESET_GATE_INPUT, RXMET_GRU_NEW_GATE_INPUT};
+        const int outOp[3] = {RXMET_GRU_UPDATE_GATE_OUTPUT, RXMET_GRU_RESET_GATE_OUTPUT, RXMET_GRU_NEW_GATE_OUTPUT};
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            last[l] = g.qhi[inOp[l]] - g.qlo[inOp[l]];
+            toIndex[l] = g.zp[inOp[l]] - g.qlo[inOp[l]];
+        }
+        tabZ = reinterpret_cast<int32_t *>(tabN + last[2] + 1);
+        tabR = tabZ + last[0] + 1;
+        auto entry = [&](int l, const Lut &lut, int i) {
+            uint8_t keep;
+            const int32_t code = clampCode(lutEval<true>(g.qlo[inOp[l]] + i, lut), g.qlo[outOp[l]], g.qhi[outOp[l]], keep);
+            return static_cast<int32_t>(static_cast<uint32_t>(code - g.zp[outOp[l]]) << 16) | (keep << l);
+        };
+        const PreparedRescale toH = prepareRescale(g.new_to_h);
+        for (int i = tid; i <= last[0]; i += nthreads) tabZ[i] = entry(0, g.lut_update, i);
+        for (int i = tid; i <= last[1]; i += nthreads) tabR[i] = entry(1, g.lut_reset, i);
+        for (int i = tid; i <= last[2]; i += nthreads) {
+            const int32_t e = entry(2, g.lut_new, i);
+            tabN[i] = make_int2(e, rescaleSmallPrepared(e >> 16, toH));
+        }
+    }
+
+    waitForPredecessor();
+    if (a.poison != nullptr && *reinterpret_cast<const volatile int *>(a.poison) != 0) {
+        // the producer of the ih codes gave up on a bounded wait: make that loud instead of computing on garbage
+        const float nan = __int_as_float(0x7fc00000);
+        for (int t = 0; t <= a.T; ++t)
+            for (int i = tid; i < nb * H; i += nthreads)
+                a.h[(static_cast<size_t>(t) * a.B + b0 + i / H) * H + i % H] = nan;
+        for (int t = 0; t < a.T; ++t)
+            for (int i = tid; i < nb * 4 * H; i += nthreads)
+                a.v[(static_cast<size_t>(t) * a.B + b0 + i / (4 * H)) * 4 * H + i % (4 * H)] = nan;
+        return;
+    }
+    const int j = min(tid / LPU, H - 1), lane = tid % LPU;
+    const int row = lane / kLanes, part = lane % kLanes;   // this lane's row of the tile, its share of the stores
+    const int batch = min(b0 + row, a.B - 1);
+
+    int32_t rw[3][KWQ];
+    int32_t mult[3], shift[3];
+    int64_t addend[3];
+    bool narrow = prepareRescale(g.rh_to_new).narrow && prepareRescale(g.update_old_to_h).narrow;
+#pragma unroll
+    for (int gate = 0; gate < 3; ++gate) {
+        const int c = gate * H + j;
+#pragma unroll
+        for (int i = 0; i < KWQ; ++i) {
+            const int word = lane * KWQ + i;
+            rw[gate][i] = word < a.kWords ? static_cast<const int32_t *>(a.R)[static_cast<size_t>(word) * C + c] : 0;
+        }
+        const Rescale rs = a.rescale[c];
+        const int64_t offset = a.biasAcc[c] - a.comp[c];
+        mult[gate] = rs.mult;
+        shift[gate] = rs.shift;
+        addend[gate] = offset * rs.mult;
+        // as in 4b: these products can be rounded with 32-bit pieces
+        narrow = narrow && rs.shift >= 1 && rs.shift <= 31 && rs.mult > 0 && static_cast<int64_t>(rs.mult) <= (1ll << rs.shift) &&
+                 offset > -(1ll << 30) && offset < (1ll << 30);
+    }
+
+    // initial codes (null: the zero point everywhere); h[0] is the initial state, dequantized like every other step
+    const int8_t *h0 = static_cast<const int8_t *>(a.h0);
+    const int srcPadded = a.kWords * 4;
+    const float scaleH = g.eff[RXMET_GRU_H];
+    for (int i = tid; i < BT * kPadded; i += nthreads) {
+        const int b = i / kPadded, k = i % kPadded, from = min(b0 + b, a.B - 1);
+        int32_t code = k < H ? zpH : 0;
+        if (k < H && h0 != nullptr) code = h0[static_cast<size_t>(from) * srcPadded + k];
+        hS[0][b][k] = static_cast<int8_t>(code);
+        hS[1][b][k] = 0;
+        if (b < nb && k < H) {
+            const size_t o = static_cast<size_t>(b0 + b) * H + k;
+            a.h[o] = static_cast<float>(code - zpH) * scaleH;
+            if (a.hq) a.hq[o] = code;
+        }
+    }
+    int32_t hDiff = h0 != nullptr ? h0[static_cast<size_t>(batch) * srcPadded + j] - zpH : 0;
+
+    const int32_t loHh = g.qlo[RXMET_GRU_WEIGHT_HH_LINEAR] - zpHh, hiHh = g.qhi[RXMET_GRU_WEIGHT_HH_LINEAR] - zpHh;
+    const int32_t loH = g.qlo[RXMET_GRU_H] - zpH, hiH = g.qhi[RXMET_GRU_H] - zpH;
+    const int32_t oneDiff = g.quant_one - zpZ;
+    const RoundingShift toUpdate = roundingShift(g.hh_to_update), toReset = roundingShift(g.hh_to_reset);
+    float vScale[4 / kLanes];   // of the quarters of v that this lane stores: part, part + kLanes, ... of z, r, n, hh
+#pragma unroll
+    for (int k = 0; k < 4 / kLanes; ++k) {
+        const int which = k * kLanes + part;
+        vScale[k] = which == 0 ? g.eff[RXMET_GRU_UPDATE_GATE_OUTPUT] : which == 1 ? g.eff[RXMET_GRU_RESET_GATE_OUTPUT] :
+                    which == 2 ? g.eff[RXMET_GRU_NEW_GATE_OUTPUT] : g.eff[RXMET_GRU_WEIGHT_HH_LINEAR];
+    }
+    // offsets of this element inside a step, in elements (the host checks that a step of v has less than 2^32 bytes)
+    const uint32_t offH = static_cast<uint32_t>(batch) * H + j, offC = static_cast<uint32_t>(batch) * C + j;
+    const uint32_t offV = static_cast<uint32_t>(batch) * 4 * H + part * H + j;
+    const size_t stepH = static_cast<size_t>(a.B) * H;
+
+    struct Terms {
+        int32_t ih[3];
+        uint32_t keep[3];
+    };
+    const int16_t *ihNext = static_cast<const int16_t *>(a.ih);   // of the step that is fetched next
+    const uint8_t *keepNext = a.maskIh;
+    auto fetch = [&](Terms &dst, bool more) {   // more: another step follows; the last one is fetched again otherwise
+#pragma unroll
+        for (int gate = 0; gate < 3; ++gate) dst.ih[gate] = (ihNext + gate * H)[offC];
+        if constexpr (Flags == FlagForm::Packed) {
+#pragma unroll
+            for (int gate = 0; gate < 3; ++gate) dst.keep[gate] = (keepNext + gate * H)[offC];
+        }
+        const size_t advance = more ? 3 * stepH : 0;
+        ihNext += advance;
+        if constexpr (Flags == FlagForm::Packed) keepNext += advance;
+    };
+
+    struct Outputs {
+        int32_t diff[4], h;   // z, r, n, hh of the new gate; h
+        uint32_t flags;       // bit 0..2 gate output, 3..5 gate input, 6..8 hh linear, 9..11 ih linear, 12 hidden state
+    };
+    size_t stored = 0;   // elements of h before the step that is stored next
+    auto store = [&](const Outputs &o) {
+        (a.h + stored + stepH)[offH] = static_cast<float>(o.h) * scaleH;
+#pragma unroll
+        for (int k = 0; k < 4 / kLanes; ++k) {
+            int32_t diff = o.diff[k * kLanes];
+#pragma unroll
+            for (int l = 1; l < kLanes; ++l) diff = part == l ? o.diff[k * kLanes + l] : diff;
+            (a.v + 4 * stored + k * kLanes * H)[offV] = static_cast<float>(diff) * vScale[k];
+        }
+        if constexpr (Flags == FlagForm::Packed) {
+            (a.stepBits + stored)[offH] = static_cast<uint16_t>(o.flags);
+        } else if constexpr (kFlags) {
+            constexpr bool kAlways = Flags == FlagForm::Bytes;   // all four flag tensors are there
+#pragma unroll
+            for (int k = 0; k < 4 / kLanes; ++k) {
+                const int which = k * kLanes + part;
+                const size_t at = 3 * stored + static_cast<size_t>(k * kLanes) * H;
+                const uint32_t off = offC + part * H;
+                if (which < 3) {
+                    if (kAlways || a.maskHh) (a.maskHh + at)[off] = (o.flags >> (6 + which)) & 1u;
+                    if (kAlways || a.maskGateIn) {
+                        (a.maskGateIn + at)[off] = (o.flags >> (3 + which)) & 1u;
+                        (a.maskGateOut + at)[off] = (o.flags >> which) & 1u;
+                    }
+                } else if (kAlways || a.maskGateIn) {
+                    (a.maskH + stored)[offH] = (o.flags >> 12) & 1u;
+                }
+            }
+            if constexpr (!kAlways) {
+                if (part == 0 && a.hq) (a.hq + stored + stepH)[offH] = o.h + zpH;
+                if (part == 0 && a.vq) {
+                    int32_t *vq = a.vq + 4 * stored + offV;
+                    vq[0] = o.diff[0] + zpZ;
+                    vq[H] = o.diff[1] + zpR;
+                    vq[2 * H] = o.diff[2] + zpN;
+                    vq[3 * H] = o.diff[3] + zpHh;
+                }
+            }
+        }
+        stored += stepH;
+    };
+
+    auto run = [&](auto narrowTag) {
+        constexpr bool kNarrow = decltype(narrowTag)::value;
+        const RoundingShift rhToNew = kNarrow ? roundingShift(g.rh_to_new) : RoundingShift{};
+        const RoundingShift toH = kNarrow ? roundingShift(g.update_old_to_h) : RoundingShift{};
+        uint32_t mask[3] = {};
+        if constexpr (kNarrow) {
+#pragma unroll
+            for (int gate = 0; gate < 3; ++gate) {
+                mask[gate] = (1u << shift[gate]) - 1u;
+                addend[gate] += 1ll << (shift[gate] - 1);
+            }
+        }
+        auto product = [&](int32_t x, const RoundingShift &r, const Rescale &general) {
+            if constexpr (kNarrow) return roundWideTies(static_cast<int64_t>(x) * r.mult + r.half, r.shift, r.mask);
+            else return rshiftRoundCalled(static_cast<int64_t>(x) * general.mult, general.shift);
+        };
+        Outputs out{};
+        auto step = [&](int t, auto first, Terms &terms) {
+            __syncthreads();   // hidden codes of step t
+            const int8_t *hNow = &hS[t & 1][0][lane * (4 * KWQ)];
+            int4 hv[BT][KWQ / 4];
+#pragma unroll
+            for (int b = 0; b < BT; ++b)
+#pragma unroll
+                for (int k4 = 0; k4 < KWQ / 4; ++k4) hv[b][k4] = *reinterpret_cast<const int4 *>(hNow + b * kPadded + k4 * 16);
+            if constexpr (!decltype(first)::value) store(out);
+            int32_t acc[BT][3];
+#pragma unroll
+            for (int b = 0; b < BT; ++b)
+#pragma unroll
+                for (int gate = 0; gate < 3; ++gate) {
+                    int32_t s = 0;
+#pragma unroll
+                    for (int k4 = 0; k4 < KWQ / 4; ++k4) {
+                        s = __dp4a(rw[gate][4 * k4 + 0], hv[b][k4].x, s);
+                        s = __dp4a(rw[gate][4 * k4 + 1], hv[b][k4].y, s);
+                        s = __dp4a(rw[gate][4 * k4 + 2], hv[b][k4].z, s);
+                        s = __dp4a(rw[gate][4 * k4 + 3], hv[b][k4].w, s);
+                    }
+                    acc[b][gate] = s;
+                }
+            // add the parts of K; rows are dealt to the lanes on the way
+            [[maybe_unused]] const bool upper = lane & 2, odd = lane & 1;
+            int32_t hh[3];
+            uint32_t flags = 0;
+#pragma unroll
+            for (int gate = 0; gate < 3; ++gate) {
+                int32_t sum;
+                if constexpr (BT == 1) {
+                    const int32_t s = acc[0][gate] + __shfl_xor_sync(0xffffffffu, acc[0][gate], 2);
+                    sum = s + __shfl_xor_sync(0xffffffffu, s, 1);
+                } else if constexpr (BT == 2) {
+                    sum = (odd ? acc[1][gate] : acc[0][gate]) +
+                          __shfl_xor_sync(0xffffffffu, odd ? acc[0][gate] : acc[1][gate], 1);
+                } else {
+                    int32_t s[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+                        s[i] = (upper ? acc[i + 2][gate] : acc[i][gate]) +
+                               __shfl_xor_sync(0xffffffffu, upper ? acc[i][gate] : acc[i + 2][gate], 2);
+                    sum = (odd ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, odd ? s[0] : s[1], 1);
+                }
+                const int64_t wide = static_cast<int64_t>(sum) * mult[gate] + addend[gate];
+                if constexpr (kNarrow) {
+                    const int32_t v = roundWideTies(wide, shift[gate], mask[gate]);
+                    hh[gate] = max(loHh, min(v, hiHh));
+                    if (kFlags && v == hh[gate]) flags += 64u << gate;
+                } else {
+                    uint8_t keep;
+                    hh[gate] = clampCode(rshiftRoundCalled(wide, shift[gate]) + zpHh, loHh + zpHh, hiHh + zpHh, keep) - zpHh;
+                    if (kFlags) flags += static_cast<uint32_t>(keep) << (6 + gate);
+                }
+            }
+            auto lookUp = [&](int32_t pre, int gate, auto *table) {
+                const int32_t index = max(0, min(pre, last[gate]));
+                if (kFlags && index == pre) flags += 8u << gate;
+                return table[index];
+            };
+            const int32_t z = lookUp(terms.ih[0] + rescaleSmallTies(hh[0], toUpdate) + toIndex[0], 0, tabZ);
+            const int32_t r = lookUp(terms.ih[1] + rescaleSmallTies(hh[1], toReset) + toIndex[1], 1, tabR);
+            const int2 n = lookUp(terms.ih[2] + product((r >> 16) * hh[2], rhToNew, g.rh_to_new) + toIndex[2], 2, tabN);
+            const int32_t zDiff = z >> 16;
+            const int32_t v = product(zDiff * hDiff + (oneDiff - zDiff) * n.y, toH, g.update_old_to_h);
+            hDiff = max(loH, min(v, hiH));
+            hS[(t + 1) & 1][row][j] = static_cast<int8_t>(hDiff + zpH);
+            out.diff[0] = zDiff; out.diff[1] = r >> 16; out.diff[2] = n.x >> 16; out.diff[3] = hh[2];
+            out.h = hDiff;
+            if constexpr (kFlags) {
+                if (v == hDiff) flags += 1u << 12;
+                flags += (z & 1) + (r & 2) + (n.x & 4);
+                if constexpr (Flags == FlagForm::Packed) flags += (terms.keep[0] << 9) + (terms.keep[1] << 10) + (terms.keep[2] << 11);
+                out.flags = flags;
+            }
+            fetch(terms, t + kAhead + 1 < a.T);
+        };
+        Terms terms[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) fetch(terms[i], i + 1 < a.T);
+        step(0, std::true_type{}, terms[0]);
+        int t = 1;
+        for (; t + kAhead <= a.T; t += kAhead)
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) step(t + i, std::false_type{}, terms[(1 + i) % kAhead]);
+#pragma unroll
+        for (int i = 0; i < kAhead - 1; ++i)
+            if (t + i < a.T) step(t + i, std::false_type{}, terms[(1 + i) % kAhead]);
+        store(out);
+    };
+    if (__syncthreads_and(narrow)) run(std::true_type{});
+    else run(std::false_type{});
+    if (a.hFinal != nullptr) {
+        __syncthreads();
+        int8_t *codes = static_cast<int8_t *>(a.hFinal);
+        for (int i = tid; i < nb * srcPadded; i += nthreads)
+            codes[static_cast<size_t>(b0) * srcPadded + i] = hS[a.T & 1][i / srcPadded][i % srcPadded];
+    }
+}
+
 size_t recurrentSmemBytes(int H, int kWords, int pack, size_t wordBytes, size_t actBytes, int BT, bool weights) {
     const int C = 3 * H;
     auto up = [](size_t v) { return (v + 15) & ~static_cast<size_t>(15); };
@@ -881,8 +1375,7 @@ struct ChannelDevice {
 
 ChannelDevice uploadChannels(const Exec &e, Workspace &ws, cudaStream_t st) {
     const size_t C = 3 * static_cast<size_t>(e.hidden);
-    auto *block = ws.take<int32_t>(12 * C);
-    RXMET_CUDA(cudaMemcpyAsync(block, pinnedChannelBlock(e, st), 12 * C * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+    const int32_t *block = channelBlockOnDevice(e, ws.take<int32_t>(12 * C), 12 * C, st);
     ChannelDevice d;
     d.effW = reinterpret_cast<const float *>(block);
     d.effR = d.effW + C; d.effBw = d.effW + 2 * C; d.effBr = d.effW + 3 * C;
@@ -935,6 +1428,69 @@ bool fastGateMath(const GateExec &g) {
     return true;
 }
 
+// Byte-plane path (gru_forward_wide.cu) on codes of at most 16 bits.
+void runWide(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaStream_t st) {
+    const int T = call.T, B = call.B, I = call.I, H = call.H, C = 3 * H;
+    const GateExec &g = e.gate;
+    const size_t rows = static_cast<size_t>(T) * B;
+    const rxmet_gru_masks none{};
+    const rxmet_gru_masks &mk = (call.isTraining && call.masks) ? *call.masks : none;
+    if (mk.gate_input || mk.gate_output || mk.h)
+        RXMET_REQUIRE(mk.gate_input && mk.gate_output && mk.h, "gate_input, gate_output and h masks come together");
+    if (call.stepFlags)
+        RXMET_REQUIRE(call.isTraining && mk.weight_ih_linear, "packed step flags need a training forward with the weight_ih_linear mask");
+    const ChannelDevice ch = uploadChannels(e, ws, st);
+    const WideOperands o = wideOperands(ws, T, B, I, H);
+
+    WidePrepArgs p{};
+    p.W = call.W; p.R = call.R; p.bw = call.bw; p.br = call.br;
+    p.I = I; p.H = H; p.C = C; p.kI = o.kI; p.kH = o.kH; p.tileWords = o.tileWords;
+    p.effW = ch.effW; p.effR = ch.effR; p.effBw = ch.effBw; p.effBr = ch.effBr;
+    p.loW = g.qlo[RXMET_GRU_W]; p.hiW = g.qhi[RXMET_GRU_W]; p.loR = g.qlo[RXMET_GRU_R]; p.hiR = g.qhi[RXMET_GRU_R];
+    p.loBw = g.qlo[RXMET_GRU_BW]; p.hiBw = g.qhi[RXMET_GRU_BW]; p.loBr = g.qlo[RXMET_GRU_BR]; p.hiBr = g.qhi[RXMET_GRU_BR];
+    p.wWords = o.wWords; p.rWords = o.rWords; p.tiles = reinterpret_cast<uint32_t *>(o.wTiles);
+    p.W_q = call.W_q; p.R_q = call.R_q; p.bw_q = call.bw_q; p.br_q = call.br_q;
+    p.mW = mk.W; p.mR = mk.R; p.mBw = mk.bw; p.mBr = mk.br;
+    p.zeroX = static_cast<int64_t>(g.qlo[RXMET_GRU_X]) - g.zp[RXMET_GRU_X];
+    p.zeroH = static_cast<int64_t>(g.qlo[RXMET_GRU_H]) - g.zp[RXMET_GRU_H];
+    p.biasRescaleX = ch.biasX; p.biasRescaleH = ch.biasH;
+    p.addX = o.addX; p.addH = o.addH;
+    auto tensor = [&](int op, const float *src, const int32_t *given, size_t nRows, int cols, int kWords, uint32_t *planes) {
+        WidePrepArgs::Rows r{};
+        r.src = given ? nullptr : src; r.given = given;
+        r.rows = static_cast<int>(nRows); r.cols = cols; r.kWords = kWords;
+        r.scale = g.eff[op]; r.zp = g.zp[op]; r.lo = g.qlo[op]; r.hi = g.qhi[op];
+        r.planes = planes;
+        return r;
+    };
+    p.x = tensor(RXMET_GRU_X, call.x, call.x_codes_in, rows, I, o.kI, o.xPlanes);
+    p.x.codes32 = call.x_codes_in ? nullptr : call.x_q; p.x.mask = mk.x;
+    p.h0 = tensor(RXMET_GRU_H, call.h0, call.h0_codes_in, static_cast<size_t>(B), H, o.kH, o.h0Planes);
+    p.h0.mask = mk.h0; p.h0.codes = o.h0Codes; p.h0.colsPadded = o.hPad;
+    constexpr int kBlock = 32 * kPrepLayers;
+    auto blocksFor = [&](const WidePrepArgs::Rows &r) {
+        return static_cast<int>(std::min<size_t>((static_cast<size_t>(r.rows) * r.kWords + kBlock - 1) / kBlock, 4 * 148));
+    };
+    p.prepBlocks = o.wTiles ? planeproj::paddedC(C) / 32 : (C + 31) / 32;
+    p.xBlocks = blocksFor(p.x); p.h0Blocks = blocksFor(p.h0);
+    p.clear = o.projStatus;
+    {
+        KernelTimer timer__("prepareWeights", st);
+        prepareWide<<<p.prepBlocks + p.xBlocks + p.h0Blocks, kBlock, 0, st>>>(p);
+    }
+    afterLaunch("prepareWeights");
+
+    WideCall wc{};
+    wc.T = T; wc.B = B; wc.I = I; wc.H = H;
+    wc.operands = o;
+    wc.gemmX = ch.gemmX; wc.gemmH = ch.gemmH;
+    wc.h = call.h; wc.v = call.v; wc.hq = call.h_q; wc.vq = call.v_q;
+    wc.maskIh = mk.weight_ih_linear; wc.maskHh = mk.weight_hh_linear; wc.maskGateIn = mk.gate_input;
+    wc.maskGateOut = mk.gate_output; wc.maskH = mk.h;
+    wc.stepBits = call.stepFlags;
+    forwardWide(wc, e, st);
+}
+
 template <class WT, class AT, class LT>
 void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaStream_t st) {
     using D = Dot<WT, AT>;
@@ -960,6 +1516,11 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
     auto *comp = ws.take<int64_t>(4 * static_cast<size_t>(C));
     int64_t *compX = comp, *biasX = comp + C, *compH = comp + 2 * C, *biasH = comp + 3 * C;
     int *projStatus = ws.take<int>(1);  // set by the tensor-core input projection when a bounded wait gave up
+    constexpr bool kI8 = std::is_same<WT, int8_t>::value && std::is_same<AT, int8_t>::value && std::is_same<LT, int16_t>::value;
+    // lanes of a warp share a hidden unit: beyond 128 units the weights leave no registers for the cell
+    const bool lanesPath = kI8 && H <= 128 && fastGateMath(g) && std::getenv("RXMET_GRU_FWD_GENERIC") == nullptr &&
+                          std::getenv("RXMET_GRU_FWD_MODE") == nullptr && std::getenv("RXMET_GRU_FWD_BT") == nullptr &&
+                          static_cast<size_t>(B) * H * 16 < (size_t{1} << 32);
 
     // 1. codes (8-bit weights: together with the per-channel terms of step 2)
     constexpr bool kPackedWeights = std::is_same<WT, int8_t>::value && std::is_same<AT, int8_t>::value;
@@ -980,6 +1541,7 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
         p.biasRescaleX = ch.biasX; p.biasRescaleH = ch.biasH;
         p.compX = compX; p.biasX = biasX; p.compH = compH; p.biasH = biasH;
         p.prepBlocks = (C + 31) / 32;
+        p.clear = projStatus;
         int xBlocks = 0;
         if constexpr (kPackedWeights) {
             if (!call.x_codes_in) {  // the input tensor rides in the same launch
@@ -1025,7 +1587,7 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
     } else if (call.h0) {
         launchQuantize<AT>(st, call.h0, B, H, B, hPad, nullptr, g.eff[RXMET_GRU_H], g.zp[RXMET_GRU_H],
                            g.qlo[RXMET_GRU_H], g.qhi[RXMET_GRU_H], 1, h0Codes, nullptr, mk.h0);
-    } else {
+    } else if (!lanesPath) {   // recurrentLanesI8 knows the zero point itself
         // padding columns hold the zero point too; they meet zero weights, so they do not matter
         if constexpr (sizeof(AT) == 1) {
             // one-byte codes: a memset node instead of a kernel
@@ -1052,34 +1614,8 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
         afterLaunch("channelPrep");
     }
 
-    // W8 / A16: byte-plane dp4a kernels instead of the 64-bit generic ones
-    if constexpr (std::is_same<WT, int8_t>::value && std::is_same<AT, int16_t>::value && std::is_same<LT, int16_t>::value) {
-        if (forwardWideTakes(e, I, H)) {
-            WideCall wc{};
-            wc.T = T; wc.B = B; wc.I = I; wc.H = H;
-            wc.wCodes = reinterpret_cast<const int8_t *>(wCodes); wc.rCodes = reinterpret_cast<const int8_t *>(rCodes);
-            wc.iPad = iPad; wc.hPad = hPad;
-            wc.xCodes = reinterpret_cast<const int16_t *>(xCodes); wc.h0Codes = reinterpret_cast<const int16_t *>(h0Codes);
-            wc.compX = compX; wc.biasX = biasX; wc.compH = compH; wc.biasH = biasH;
-            wc.gemmX = ch.gemmX; wc.gemmH = ch.gemmH;
-            wc.ihCodes = reinterpret_cast<int16_t *>(ihCodes);
-            wc.h = call.h; wc.v = call.v; wc.hq = call.h_q; wc.vq = call.v_q;
-            wc.maskIh = mk.weight_ih_linear; wc.maskHh = mk.weight_hh_linear; wc.maskGateIn = mk.gate_input;
-            wc.maskGateOut = mk.gate_output; wc.maskH = mk.h;
-            if (mk.gate_input || mk.gate_output || mk.h)
-                RXMET_REQUIRE(mk.gate_input && mk.gate_output && mk.h, "gate_input, gate_output and h masks come together");
-            wc.stepBits = call.stepFlags;
-            if (call.stepFlags)
-                RXMET_REQUIRE(training && mk.weight_ih_linear, "packed step flags need a training forward with the weight_ih_linear mask");
-            forwardWide(wc, e, ws, st);
-            return;
-        }
-    }
-
     // Which recurrence runs decides what the input projection stores.
     const int smemMax = currentDevice().smemMax, sms = currentDevice().sms;
-    constexpr bool kI8 = std::is_same<WT, int8_t>::value && std::is_same<AT, int8_t>::value &&
-                         std::is_same<LT, int16_t>::value;
     const int blockI8 = padTo(C, 32);
     int btI8 = (B > 2 * sms) ? 4 : ((B > sms) ? 2 : 1);
     if (const char *env = std::getenv("RXMET_GRU_FWD_BT")) btI8 = std::atoi(env);
@@ -1103,11 +1639,13 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
         const int kw4 = (iWords + 3) / 4;
         bool specialised = false;
         if constexpr (kI8) {
-            if (iproj::eligible(C, H, iWords, xCodes, ihCodes, mk.weight_ih_linear) && std::getenv("RXMET_GRU_FWD_GENERIC") == nullptr) {
+            // channel counts that leave the last tile partly empty: only where the register kernel below does not go
+            const bool registerProjection = C <= 512 && kw4 <= 4 && block >= kI8Rows * kw4 * 4;
+            if (iproj::eligible(C, H, iWords, xCodes, ihCodes, mk.weight_ih_linear) && (C % 128 == 0 || !registerProjection) &&
+                std::getenv("RXMET_GRU_FWD_GENERIC") == nullptr) {
                 // tcgen05 kind::i8 GEMM with the fused epilogue
                 specialised = true;
                 tensorProjection = true;
-                RXMET_CUDA(cudaMemsetAsync(projStatus, 0, sizeof(int), st));
                 // rows [r0, r0 + n) on stream `s`
                 auto projectRows = [&](size_t r0, size_t n, cudaStream_t s) {
                     iproj::Problem pj{};
@@ -1152,9 +1690,9 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
     case N: {                                                                                                              \
         const int perSm = residentPerSm(reinterpret_cast<const void *>(inputLinearI8<N>), block, 0);                       \
         const int grid = std::max(1, std::min(blocks, sms * std::max(1, perSm)));                                          \
-        inputLinearI8<N><<<grid, block, 0, st>>>(reinterpret_cast<const int32_t *>(xCodes), static_cast<int>(rows), iWords, C, \
-                                                 reinterpret_cast<const int32_t *>(wCodes), compX, biasX, ch.gemmX, zp, qlo, qhi, \
-                                                 reinterpret_cast<int16_t *>(ihCodes), mk.weight_ih_linear, pre);            \
+        launchDependent(inputLinearI8<N>, grid, block, 0, st, reinterpret_cast<const int32_t *>(xCodes), static_cast<int>(rows), \
+                        iWords, C, reinterpret_cast<const int32_t *>(wCodes), compX, biasX, ch.gemmX, zp, qlo, qhi,        \
+                        reinterpret_cast<int16_t *>(ihCodes), mk.weight_ih_linear, pre);                                    \
     } break;
                 switch (kw4) {
                     RXMET_IL_CASE(1) RXMET_IL_CASE(2) RXMET_IL_CASE(3) RXMET_IL_CASE(4)
@@ -1177,7 +1715,8 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
     // 4. recurrence
     RecurrentArgs a{};
     a.T = T; a.B = B; a.H = H; a.kWords = hWords;
-    a.R = rCodes; a.ih = ihCodes; a.h0 = h0Codes;
+    a.R = rCodes; a.ih = ihCodes;
+    a.h0 = lanesPath && !call.h0 && !call.h0_codes_in ? nullptr : h0Codes;
     a.comp = compH; a.biasAcc = biasH; a.rescale = ch.gemmH;
     a.h = call.h; a.v = call.v; a.hq = call.h_q; a.vq = call.v_q;
     a.maskHh = mk.weight_hh_linear; a.maskGateIn = mk.gate_input; a.maskGateOut = mk.gate_output; a.maskH = mk.h;
@@ -1211,6 +1750,7 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
         if (registerPath) {
             // register-resident variant: one thread per column, at most two gate elements per thread
             size_t smem = sizeof(int32_t) * btI8 * C;
+            if (lanesPath) smem = sizeof(int32_t) * (g.qhi[RXMET_GRU_NEW_GATE_INPUT] - g.qlo[RXMET_GRU_NEW_GATE_INPUT] + 1);
             if (mode == 2) {
                 for (int op : {RXMET_GRU_UPDATE_GATE_INPUT, RXMET_GRU_RESET_GATE_INPUT, RXMET_GRU_NEW_GATE_INPUT})
                     smem += sizeof(int32_t) * (g.qhi[op] - g.qlo[op] + 1);
@@ -1220,17 +1760,35 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
                 {
                     KernelTimer timer__("recurrentForward", st);
                     bool done = false;
+#define RXMET_LANES_CASE(KW, LPU, BT)                                                                                       \
+    if (!done && lanesPath && hWords <= KW && btI8 == BT) {                                                                \
+        auto kernel = ra.stepBits ? recurrentLanesI8<KW, LPU, BT, FlagForm::Packed>                                       \
+                      : ra.hq || ra.vq || (!ra.maskHh != !ra.maskGateIn) ? recurrentLanesI8<KW, LPU, BT, FlagForm::Codes> \
+                      : ra.maskHh ? recurrentLanesI8<KW, LPU, BT, FlagForm::Bytes>                                        \
+                                  : recurrentLanesI8<KW, LPU, BT, FlagForm::None>;                                        \
+        launchDependent(kernel, (B + BT - 1) / BT, padTo(LPU * H, 32), smem, st, ra, g);                                  \
+        done = true;                                                                                                      \
+    }
+                    RXMET_LANES_CASE(16, 4, 1) RXMET_LANES_CASE(16, 2, 2) RXMET_LANES_CASE(16, 4, 4)
+                    RXMET_LANES_CASE(32, 4, 1) RXMET_LANES_CASE(32, 2, 2) RXMET_LANES_CASE(32, 4, 4)
+#undef RXMET_LANES_CASE
 #define RXMET_I8_CASE(KW, BT)                                                 \
     if (!done && hWords <= KW && btI8 == BT) {                                 \
-        if (mode == 2 && ra.stepBits) launchI8(recurrentForwardI8<KW, BT, 2, true>); \
-        else if (mode == 2) launchI8(recurrentForwardI8<KW, BT, 2>);           \
-        else if (mode == 1) launchI8(recurrentForwardI8<KW, BT, 1>);           \
+        if (mode == 1) launchI8(recurrentForwardI8<KW, BT, 1>);                \
         else launchI8(recurrentForwardI8<KW, BT, 0>);                          \
         done = true;                                                           \
     }
+#define RXMET_I8_FAST_CASE(BT)                                                 \
+    if (!done && mode == 2 && btI8 == BT) {                                    \
+        if (ra.stepBits) launchI8(recurrentForwardI8<64, BT, 2, true>);        \
+        else launchI8(recurrentForwardI8<64, BT, 2>);                          \
+        done = true;                                                           \
+    }
+                    RXMET_I8_FAST_CASE(1) RXMET_I8_FAST_CASE(2) RXMET_I8_FAST_CASE(4)
                     RXMET_I8_CASE(16, 1) RXMET_I8_CASE(16, 2) RXMET_I8_CASE(16, 4)
                     RXMET_I8_CASE(32, 1) RXMET_I8_CASE(32, 2) RXMET_I8_CASE(32, 4)
                     RXMET_I8_CASE(64, 1) RXMET_I8_CASE(64, 2) RXMET_I8_CASE(64, 4)
+#undef RXMET_I8_FAST_CASE
 #undef RXMET_I8_CASE
                 }
                 afterLaunch("recurrentForwardI8");
@@ -1248,6 +1806,7 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
                 const size_t r0 = static_cast<size_t>(t0) * B;
                 RecurrentArgs ra = a;
                 ra.T = chunks[i];
+                if (i > 0) ra.h0 = h0Codes;
                 ra.hFinal = (i + 1 < chunks.size()) ? h0Codes : nullptr;
                 ra.ih = reinterpret_cast<const int16_t *>(ihCodes) + r0 * C;
                 ra.h = a.h + r0 * H; ra.v = a.v + r0 * 4 * H;
@@ -1558,7 +2117,7 @@ void forwardFpCarrier(const ForwardQuantCall &call, const Exec &e, Workspace &ws
 
 bool packedFlagsSupported(const Exec &e, int B, int I, int H) {
     // 16-bit activations: the cluster recurrence packs them, for widths whose backward reads them
-    if (forwardWideTakes(e, I, H)) return (H <= 128 || H % 32 == 0) && forwardWideClusterTakes(e, H);
+    if (e.actClass == CodeClass::I16 && forwardWideTakes(e, I, H)) return (H <= 128 || H % 32 == 0) && forwardWideClusterTakes(e, H);
     if (e.weightClass != CodeClass::I8 || e.actClass != CodeClass::I8 || e.linearClass == CodeClass::I32) return false;
     if (std::getenv("RXMET_GRU_FWD_GENERIC") != nullptr || std::getenv("RXMET_GRU_FWD_BT") != nullptr) return false;
     const int sms = currentDevice().sms, C = 3 * H;
@@ -1578,6 +2137,13 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, 
         return;
     }
     const CodeClass w = e.weightClass, a = e.actClass, l = e.linearClass;
+    // 16-bit codes, and 8-bit ones too wide for the lanes path: the register path below holds R of 256 units in spilled
+    // registers (H = 192, B = 500, T = 98: 666 us against 298 us over clusters)
+    if (forwardWideTakes(e, call.I, call.H) &&
+        (a == CodeClass::I16 || (call.H > 128 && !call.stepFlags && forwardWideClusterTakes(e, call.H)))) {
+        runWide(call, e, ws, st);
+        return;
+    }
     if (l == CodeClass::I32 || w == CodeClass::I32 || a == CodeClass::I32) {
         runTyped<int32_t, int32_t, int32_t>(call, e, ws, st);
     } else if (w == CodeClass::I8 && a == CodeClass::I8) {

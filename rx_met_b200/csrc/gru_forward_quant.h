@@ -33,10 +33,9 @@ struct ForwardQuantCall {
 // Whether forwardQuant can write stepFlags for these parameters and sizes (the register-resident 8-bit path, the cluster recurrence).
 bool packedFlagsSupported(const Exec &exec, int B, int I, int H);
 
-// Page-locked host copy of the per-channel block of `exec`, 12 arrays of 3H 32-bit words: effective
-// scales of W, R, bw, br (floats), then the Rescale pairs gemm_x, bias_x, gemm_h, bias_h.  Built on
-// first use and owned by `exec`.
-const int32_t *pinnedChannelBlock(const Exec &exec, cudaStream_t stream);
+// The per-channel block (four float arrays, four Rescale arrays of 3 * hidden entries each) on the current device: a copy
+// kept with the Exec, or, inside a stream capture that comes before the first call, `words` words of it copied to `scratch`.
+const int32_t *channelBlockOnDevice(const Exec &exec, int32_t *scratch, size_t words, cudaStream_t stream);
 
 size_t forwardQuantWorkspaceBytes(int T, int B, int I, int H);
 void forwardQuant(const ForwardQuantCall &call, const Exec &exec, void *workspace, size_t workspaceBytes,

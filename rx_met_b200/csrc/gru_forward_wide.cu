@@ -44,57 +44,7 @@ __device__ __forceinline__ void copyAsync16(void *dst, const void *src, bool val
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16u : 0u) : "memory");
 }
 
-int gridFor(size_t n, int block) { return static_cast<int>(std::min<size_t>((n + block - 1) / block, 148 * 8)); }
 int wordsFor(int k) { return (k + 15) / 16 * 4; }  // K padded to 16 bytes so that rows are read as 16-byte pieces
-
-// codes [K rows (padded to kPadRows)][C] int8 -> words [kWords][C], four consecutive k per word; one warp
-// per channel sums the codes: addend = (gridMin - zeroPoint) * sum + bias on the accumulator grid, where
-// comp = zeroPoint * sum was computed with the codes (so gridMin * sum - comp + bias).
-__global__ void packWeightWords(const int8_t *__restrict__ codes, int K, int C, int kWords, int32_t gridMin,
-                                const int64_t *__restrict__ comp, const int64_t *__restrict__ biasAcc,
-                                uint32_t *__restrict__ words, int64_t *__restrict__ addend) {
-    const int lane = threadIdx.x & 31;
-    const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (c >= C) return;
-    int32_t sum = 0;
-    for (int kw = lane; kw < kWords; kw += 32) {
-        uint32_t word = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int k = 4 * kw + i;
-            const int32_t q = k < K ? codes[static_cast<size_t>(k) * C + c] : 0;
-            sum += q;
-            word |= (static_cast<uint32_t>(q) & 0xffu) << (8 * i);
-        }
-        words[static_cast<size_t>(kw) * C + c] = word;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) addend[c] = static_cast<int64_t>(gridMin) * sum - comp[c] + biasAcc[c];
-}
-
-// int16 codes [rows][colsPadded] -> [rows][2][kWords] words of four bytes of u = code - gridMin (plane 0 = high
-// bytes); columns beyond `cols` are zero.
-__global__ void planesFromCodes(const int16_t *__restrict__ codes, size_t rows, int cols, int colsPadded, int kWords,
-                                int32_t gridMin, uint32_t *__restrict__ planes) {
-    const size_t total = rows * kWords;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const size_t r = i / kWords;
-        const int kw = static_cast<int>(i % kWords);
-        uint32_t high = 0, low = 0;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int k = 4 * kw + e;
-            if (k >= cols) continue;
-            const uint32_t u = static_cast<uint32_t>(static_cast<int32_t>(codes[r * colsPadded + k]) - gridMin);
-            low |= (u & 0xffu) << (8 * e);
-            high |= ((u >> 8) & 0xffu) << (8 * e);
-        }
-        planes[(2 * r) * kWords + kw] = high;
-        planes[(2 * r + 1) * kWords + kw] = low;
-    }
-}
 
 __device__ __forceinline__ int64_t combine(int32_t high, int32_t low, int64_t addend) {
     return (static_cast<int64_t>(high) << 8) + low + addend;
@@ -345,13 +295,6 @@ recurrentPlanes(const __grid_constant__ RecurrentArgs a, const __grid_constant__
     (void)stepC;
 }
 
-struct Layout {
-    uint32_t *xPlanes, *h0Planes, *wWords, *rWords;
-    int64_t *addX, *addH;
-    uint4 *wTiles;     // input weights as canonical tensor-core tiles (plane_proj_umma.cuh)
-    int *projStatus;
-};
-
 // Epilogue of the tensor-core input projection: exact 64-bit sum of the two planes and the addend, the
 // rounding rescale onto the linear-output grid, clamp, code and keep flag.
 struct PlaneEpilogue {
@@ -375,20 +318,35 @@ struct PlaneEpilogue {
     }
 };
 
+// Rows of a tile of the tensor-core projection, 0 where it does not run: operands beyond shared memory, or RXMET_IPROJ_SIMT.
+int projectionRows(int kI) {
+    const int kPad = planeproj::paddedK(kI);
+    if (std::getenv("RXMET_IPROJ_SIMT") != nullptr) return 0;
+    for (int rows : {128, 64})
+        if (planeproj::sharedBytes(kPad, 2, rows) <= 200 * 1024) return rows;
+    return 0;
+}
+
 template <class W>
-Layout layoutWide(W &ws, int T, int B, int I, int H) {
+WideOperands layoutWide(W &ws, int T, int B, int I, int H) {
     const size_t rows = static_cast<size_t>(T) * B, C = 3 * static_cast<size_t>(H);
-    const size_t kI = wordsFor(I), kH = wordsFor(H);
-    Layout l{};
-    l.xPlanes = ws.template take<uint32_t>(rows * 2 * kI);
-    l.h0Planes = ws.template take<uint32_t>(static_cast<size_t>(B) * 2 * kH);
-    l.wWords = ws.template take<uint32_t>(kI * C);
-    l.rWords = ws.template take<uint32_t>(kH * C);
-    l.addX = ws.template take<int64_t>(C);
-    l.addH = ws.template take<int64_t>(C);
-    l.wTiles = ws.template take<uint4>(C * planeproj::paddedK(static_cast<int>(kI)) / 16);
-    l.projStatus = ws.template take<int>(1);
-    return l;
+    WideOperands o{};
+    o.kI = wordsFor(I);
+    o.kH = wordsFor(H);
+    o.tileWords = planeproj::paddedK(o.kI) / 4;
+    o.hPad = H;
+    o.xPlanes = ws.template take<uint32_t>(rows * 2 * o.kI);
+    o.h0Planes = ws.template take<uint32_t>(static_cast<size_t>(B) * 2 * o.kH);
+    o.h0Codes = ws.template take<int16_t>(static_cast<size_t>(B) * o.hPad);
+    o.wWords = ws.template take<uint32_t>(o.kI * C);
+    o.rWords = ws.template take<uint32_t>(o.kH * C);
+    o.addX = ws.template take<int64_t>(C);
+    o.addH = ws.template take<int64_t>(C);
+    o.wTiles = ws.template take<uint4>(static_cast<size_t>(planeproj::paddedC(static_cast<int>(C))) * o.tileWords / 4);
+    o.projStatus = ws.template take<int>(1);
+    o.ihCodes = ws.template take<int16_t>(rows * C);
+    if (projectionRows(o.kI) == 0) o.wTiles = nullptr;
+    return o;
 }
 
 struct SizerAdapter {
@@ -408,57 +366,36 @@ size_t forwardWideExtraBytes(int T, int B, int I, int H) {
     return s.ws.used() + 2048;
 }
 
+WideOperands wideOperands(Workspace &ws, int T, int B, int I, int H) { return layoutWide(ws, T, B, I, H); }
+
 bool forwardWideTakes(const Exec &e, int I, int H) {
     static const bool disabled = std::getenv("RXMET_GRU_FWD_GENERIC") != nullptr;
-    if (disabled || e.weightClass != CodeClass::I8 || e.actClass != CodeClass::I16 || e.linearClass != CodeClass::I16) return false;
+    if (disabled || e.weightClass != CodeClass::I8 || e.actClass == CodeClass::I32 || e.linearClass != CodeClass::I16) return false;
     const GateExec &g = e.gate;
     for (int op : {RXMET_GRU_X, RXMET_GRU_H})
         if (static_cast<int64_t>(g.qhi[op]) - g.qlo[op] > 65535) return false;
     return H <= 512 && I <= 1024;
 }
 
-void forwardWide(const WideCall &call, const Exec &e, Workspace &ws, cudaStream_t st) {
-    const int T = call.T, B = call.B, I = call.I, H = call.H, C = 3 * H;
+void forwardWide(const WideCall &call, const Exec &e, cudaStream_t st) {
+    const int T = call.T, B = call.B, H = call.H, C = 3 * H;
     const GateExec &g = e.gate;
     const size_t rows = static_cast<size_t>(T) * B;
-    const int kI = wordsFor(I), kH = wordsFor(H);
-    const Layout l = layoutWide(ws, T, B, I, H);
+    const WideOperands &l = call.operands;
+    const int kI = l.kI, kH = l.kH;
     const int sms = currentDevice().sms;
 
-    {
-        KernelTimer timer__("packWeightWords", st);
-        packWeightWords<<<(C + 7) / 8, 256, 0, st>>>(call.wCodes, I, C, kI, g.qlo[RXMET_GRU_X], call.compX, call.biasX, l.wWords, l.addX);
-        afterLaunch("packWeightWords");
-        packWeightWords<<<(C + 7) / 8, 256, 0, st>>>(call.rCodes, H, C, kH, g.qlo[RXMET_GRU_H], call.compH, call.biasH, l.rWords, l.addH);
-        afterLaunch("packWeightWords");
-    }
-    {
-        KernelTimer timer__("planesFromCodes", st);
-        planesFromCodes<<<gridFor(rows * kI, 256), 256, 0, st>>>(call.xCodes, rows, I, call.iPad, kI, g.qlo[RXMET_GRU_X], l.xPlanes);
-        afterLaunch("planesFromCodes");
-        planesFromCodes<<<gridFor(static_cast<size_t>(B) * kH, 256), 256, 0, st>>>(call.h0Codes, static_cast<size_t>(B), H, call.hPad, kH,
-                                                                                   g.qlo[RXMET_GRU_H], l.h0Planes);
-        afterLaunch("planesFromCodes");
-    }
-    // Input projection: the tcgen05 kind::i8 kernel when the channel count tiles by 128 and the operands fit
-    // shared memory (RXMET_IPROJ_SIMT turns it off), else the dp4a kernel.
+    // Input projection: the tcgen05 kind::i8 kernel when the operands fit shared memory, else the dp4a kernel.
     const int kPadI = planeproj::paddedK(kI);
-    const int rowsPerTile = planeproj::sharedBytes(kPadI, 2, 128) <= 200 * 1024 ? 128 : 64;
-    const bool tensorProjection = C % planeproj::kChannelTile == 0 && planeproj::sharedBytes(kPadI, 2, rowsPerTile) <= 200 * 1024 &&
-                                  std::getenv("RXMET_IPROJ_SIMT") == nullptr;
+    const int rowsPerTile = projectionRows(kI);
+    const bool tensorProjection = l.wTiles != nullptr;
     if (tensorProjection) {
-        RXMET_CUDA(cudaMemsetAsync(l.projStatus, 0, sizeof(int), st));
-        {
-            KernelTimer timer__("packWeightWords", st);
-            planeproj::packTiles<<<gridFor(static_cast<size_t>(C) * kPadI / 16, 256), 256, 0, st>>>(l.wWords, kI, C, kPadI, l.wTiles);
-            afterLaunch("packTiles");
-        }
         planeproj::Problem pp{};
         pp.planes = l.xPlanes; pp.rows = static_cast<int>(rows); pp.kWords = kI; pp.tiles = l.wTiles; pp.C = C; pp.status = l.projStatus;
         PlaneEpilogue epi{};
         epi.addend = l.addX; epi.rescale = call.gemmX;
         epi.zpOut = g.zp[RXMET_GRU_WEIGHT_IH_LINEAR]; epi.lo = g.qlo[RXMET_GRU_WEIGHT_IH_LINEAR]; epi.hi = g.qhi[RXMET_GRU_WEIGHT_IH_LINEAR];
-        epi.out = call.ihCodes; epi.mask = call.maskIh; epi.C = C;
+        epi.out = l.ihCodes; epi.mask = call.maskIh; epi.C = C;
         const size_t smem = planeproj::sharedBytes(kPadI, 2, rowsPerTile);
         const int rowTiles = static_cast<int>((rows + rowsPerTile - 1) / rowsPerTile);
         const int grid = std::max(1, std::min(rowTiles, smsPerPass()));
@@ -475,7 +412,7 @@ void forwardWide(const WideCall &call, const Exec &e, Workspace &ws, cudaStream_
         a.rows = static_cast<int>(rows); a.C = C; a.kWords = kI;
         a.x = l.xPlanes; a.words = l.wWords; a.addend = l.addX; a.rescale = call.gemmX;
         a.zpOut = g.zp[RXMET_GRU_WEIGHT_IH_LINEAR]; a.lo = g.qlo[RXMET_GRU_WEIGHT_IH_LINEAR]; a.hi = g.qhi[RXMET_GRU_WEIGHT_IH_LINEAR];
-        a.out = call.ihCodes; a.mask = call.maskIh;
+        a.out = l.ihCodes; a.mask = call.maskIh;
         const int block = std::min(kThreads, (C + 31) / 32 * 32);
         const int slabs = (C + block - 1) / block;
         const int blocks = static_cast<int>((rows + kRowsPerBlock - 1) / kRowsPerBlock);
@@ -495,8 +432,8 @@ void forwardWide(const WideCall &call, const Exec &e, Workspace &ws, cudaStream_
     {
         RecurrentArgs a{};
         a.T = T; a.B = B; a.H = H; a.HP = (H + 31) / 32 * 32; a.kWords = kH;
-        a.words = l.rWords; a.addend = l.addH; a.rescale = call.gemmH; a.ih = call.ihCodes;
-        a.h0 = call.h0Codes; a.hPad = call.hPad; a.h0Planes = l.h0Planes;
+        a.words = l.rWords; a.addend = l.addH; a.rescale = call.gemmH; a.ih = l.ihCodes;
+        a.h0 = l.h0Codes; a.hPad = l.hPad; a.h0Planes = l.h0Planes;
         a.h = call.h; a.v = call.v; a.hq = call.hq; a.vq = call.vq;
         a.maskHh = call.maskHh; a.maskGateIn = call.maskGateIn; a.maskGateOut = call.maskGateOut; a.maskH = call.maskH;
         a.poison = tensorProjection ? l.projStatus : nullptr;

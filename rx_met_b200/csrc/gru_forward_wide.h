@@ -11,26 +11,33 @@
 namespace rxmet {
 namespace gru {
 
-// Everything the shared front of the forward has prepared: one code per element for the weights (int8,
-// [K padded][3H]), x and h0 (int16), the zero-point compensation and bias terms of both linear stages.
+// Operands in the workspace, filled by prepareWide (gru_forward_quant.cu).
+struct WideOperands {
+    int kI, kH, tileWords, hPad;        // words of a row of x / h (K padded to 16 bytes), of a channel's row in a tile; codes of a row of h0
+    uint32_t *xPlanes, *h0Planes;       // [T*B][2][kI], [B][2][kH] words of four bytes of code - grid minimum, high bytes first
+    int16_t *h0Codes;                   // [B][hPad]
+    uint32_t *wWords, *rWords;          // [kI][3H], [kH][3H]: four weight codes along K per word
+    int64_t *addX, *addH;               // [3H]: (grid minimum - zero point) * sum of the weight codes + bias on the accumulator grid
+    uint4 *wTiles;                      // input weights as tensor-core tiles (plane_proj_umma.cuh); null: the dp4a projection runs
+    int *projStatus;
+    int16_t *ihCodes;                   // [T*B][3H]
+};
+WideOperands wideOperands(Workspace &workspace, int T, int B, int I, int H);
+
 struct WideCall {
     int T, B, I, H;
-    const int8_t *wCodes, *rCodes;      // [iPad][3H], [hPad][3H]
-    int iPad, hPad;
-    const int16_t *xCodes, *h0Codes;    // [T*B][iPad], [B][hPad]
-    const int64_t *compX, *biasX, *compH, *biasH;
+    WideOperands operands;
     const Rescale *gemmX, *gemmH;
-    int16_t *ihCodes;                   // [T*B][3H] workspace
     float *h, *v;
     int32_t *hq, *vq;                   // optional
     uint8_t *maskIh, *maskHh, *maskGateIn, *maskGateOut, *maskH;  // optional keep flags
     uint16_t *stepBits;                 // optional packed flags
 };
 
-// Weight grids of at most 8 bits, x / h grids of 9..16 bits, linear grids of at most 16 bits, H <= 512.
+// Weight grids of at most 8 bits, x / h grids of at most 16 bits, linear grids of at most 16 bits, H <= 512.
 bool forwardWideTakes(const Exec &exec, int I, int H);
 size_t forwardWideExtraBytes(int T, int B, int I, int H);
-void forwardWide(const WideCall &call, const Exec &exec, Workspace &workspace, cudaStream_t stream);
+void forwardWide(const WideCall &call, const Exec &exec, cudaStream_t stream);
 
 // Operands of the recurrence alone, after the input projection.
 struct WideRecurrence {

@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "common.h"
+#include "dependent_launch.cuh"
 #include "gru_device.cuh"
 #include "input_proj_umma.h"
 #include "umma_device.cuh"
@@ -57,7 +58,8 @@ __device__ __forceinline__ void mmaI8(uint32_t tmemD, uint64_t descA, uint64_t d
 
 constexpr int kRows = 128;  // rows of the batch per work item = accumulator columns
 
-size_t sharedBytes(int C, int kPad) { return static_cast<size_t>(C) * kPad + 2 * static_cast<size_t>(kRows) * kPad; }
+__host__ __device__ inline int paddedC(int C) { return (C + kTileM - 1) / kTileM * kTileM; }
+size_t sharedBytes(int C, int kPad) { return static_cast<size_t>(paddedC(C)) * kPad + 2 * static_cast<size_t>(kRows) * kPad; }
 
 __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
     constexpr uint32_t kTmemCols = 2 * kRows;
@@ -68,10 +70,10 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
     __shared__ int failed;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
-    const int C = p.C, kWords = p.kWords, kPad = p.kPad;
+    const int C = p.C, padded = paddedC(C), kWords = p.kWords, kPad = p.kPad;
     const uint32_t groupStride = static_cast<uint32_t>(kPad / 16) * kCore;  // next 8 channels / 8 rows
-    uint8_t *weights = smem;                                               // [C / 8][kPad / 16][8][16]
-    uint8_t *rowStages = smem + static_cast<size_t>(C) * kPad;             // 2 x [kRows / 8][kPad / 16][8][16]
+    uint8_t *weights = smem;                                               // [padded / 8][kPad / 16][8][16]
+    uint8_t *rowStages = smem + static_cast<size_t>(padded) * kPad;             // 2 x [kRows / 8][kPad / 16][8][16]
     const size_t stageBytes = static_cast<size_t>(kRows) * kPad;
 
     if (tid == 0) {
@@ -84,17 +86,19 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // operands start as zeros: the k padding of both is never written again
-    for (size_t i = tid; i < (static_cast<size_t>(C) * kPad + 2 * stageBytes) / 16; i += kThreads)
+    // operands start as zeros: the k padding of both and the channels beyond C are never written again
+    for (size_t i = tid; i < (static_cast<size_t>(padded) * kPad + 2 * stageBytes) / 16; i += kThreads)
         reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
+    waitForPredecessor();
+    letDependentsStart();
     // weight word (kw, c) = codes k = 4 kw .. 4 kw + 3 of channel c -> four consecutive bytes of row c
     for (int i = tid; i < kWords * C; i += kThreads) {
         const int kw = i / C, c = i - kw * C;
         *reinterpret_cast<int32_t *>(weights + (c >> 3) * groupStride + (kw >> 2) * kCore + (c & 7) * 16 + (kw & 3) * 4) = p.w[i];
     }
 
-    const int channelTiles = C / kTileM;
+    const int channelTiles = padded / kTileM;
     const int rowTiles = (p.rows + kRows - 1) / kRows;
     const int items = rowTiles * channelTiles;
 
@@ -126,7 +130,8 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
         if (!waitPhase(smemAddr(&bars[buf]), (local >> 1) & 1)) failed = 1;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int tile = item / channelTiles, ct = item - tile * channelTiles;
-        const int c = ct * kTileM + 32 * q + lane;  // this thread's channel
+        const bool real = ct * kTileM + 32 * q + lane < C;
+        const int c = min(ct * kTileM + 32 * q + lane, C - 1);  // this thread's channel
         // per-channel constants in registers.  Narrow channels (|offset| < 2^30, a multiplier that shrinks,
         // shift in [1, 31]) round with 32-bit pieces of the product; the others take the 64-bit form.
         const Rescale rs = p.rescale[c];
@@ -168,7 +173,7 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
                         else code = gateNarrow ? gru::rshiftRoundNarrow(prodGate, gateRs.shift, gateMask, gateHalf)
                                                : gru::rshiftRoundCalled(prodGate, gateRs.shift);
                     }
-                    if (row0 + j < p.rows) {
+                    if (real && row0 + j < p.rows) {
                         p.out[o] = static_cast<int16_t>(code);
                         if (p.mask) p.mask[o] = keep;
                     }
@@ -216,7 +221,7 @@ int paddedK(int kWords) { return (kWords * 4 + 31) / 32 * 32; }
 bool eligible(int C, int H, int kWords, const void *x, const void *out, const void *mask) {
     static const bool disabled = std::getenv("RXMET_IPROJ_SIMT") != nullptr;
     (void)H; (void)out; (void)mask;
-    if (disabled || C % kTileM != 0 || kWords < 1 || !alignedTo(x, 4)) return false;
+    if (disabled || kWords < 1 || !alignedTo(x, 4)) return false;
     return sharedBytes(C, paddedK(kWords)) <= 200 * 1024;  // all weight codes and two row stages in one SM
 }
 
@@ -225,9 +230,9 @@ void launch(const Problem &problem, int sms, cudaStream_t st) {
     prob.kPad = paddedK(prob.kWords);
     const size_t smem = sharedBytes(prob.C, prob.kPad);
     ensureDynamicSmem(reinterpret_cast<const void *>(inputProjUmma), smem);
-    const int items = ((prob.rows + kRows - 1) / kRows) * (prob.C / kTileM);
+    const int items = ((prob.rows + kRows - 1) / kRows) * (paddedC(prob.C) / kTileM);
     KernelTimer timer__("inputLinear", st);
-    inputProjUmma<<<std::max(1, std::min(items, 2 * sms)), kThreads, smem, st>>>(prob);
+    launchDependent(inputProjUmma, std::max(1, std::min(items, 2 * sms)), kThreads, smem, st, prob);
 }
 
 }  // namespace iproj

@@ -865,7 +865,7 @@ WideLayout layoutWide(W &ws, int T, int B, int I, int H, int planes) {
     l.addHh = ws.template take<int64_t>(C);
     l.channel = ws.template take<float>(kChannelFields * C);
     l.lhs = ws.template take<float>(rows * C);
-    l.ihTiles = ws.template take<uint4>(C * planeproj::paddedK(static_cast<int>(kIh)) / 16);
+    l.ihTiles = ws.template take<uint4>(static_cast<size_t>(planeproj::paddedC(static_cast<int>(C))) * planeproj::paddedK(static_cast<int>(kIh)) / 16);
     l.projStatus = ws.template take<int>(1);
     l.hhTiles = ws.template take<uint4>(C * planeproj::paddedK(static_cast<int>(kHh)) / 16);
     l.exchange = ws.template take<uint32_t>(static_cast<size_t>(B) * planes * kHh);
@@ -979,17 +979,16 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
     const rxmet_lstm_trace noTrace{};
     const rxmet_lstm_trace &ck = call.checkpoints ? *call.checkpoints : noTrace;
     const int sms = currentDevice().sms;
-    // Input projection: the tcgen05 kind::i8 kernel when 4H tiles by 128 and the operands fit shared memory
+    // Input projection: the tcgen05 kind::i8 kernel when the operands fit shared memory
     // (RXMET_IPROJ_SIMT turns it off), else the dp4a kernel.
     const int kPadIh = planeproj::paddedK(kIh);
     const int rowsPerTile = planeproj::sharedBytes(kPadIh, planes, 128) <= 200 * 1024 ? 128 : 64;
-    const bool tensorProjection = C % planeproj::kChannelTile == 0 && planeproj::sharedBytes(kPadIh, planes, rowsPerTile) <= 200 * 1024 &&
-                                  std::getenv("RXMET_IPROJ_SIMT") == nullptr;
+    const bool tensorProjection = planeproj::sharedBytes(kPadIh, planes, rowsPerTile) <= 200 * 1024 && std::getenv("RXMET_IPROJ_SIMT") == nullptr;
     if (tensorProjection) {
         RXMET_CUDA(cudaMemsetAsync(l.projStatus, 0, sizeof(int), st));
         {
             KernelTimer timer__("lstmPrepChannelsWide", st);
-            planeproj::packTiles<<<gridFor(static_cast<size_t>(C) * kPadIh / 16, 256), 256, 0, st>>>(l.wIh, kIh, C, kPadIh, l.ihTiles);
+            planeproj::packTiles<<<gridFor(static_cast<size_t>(planeproj::paddedC(C)) * kPadIh / 16, 256), 256, 0, st>>>(l.wIh, kIh, C, kPadIh, l.ihTiles);
         }
         afterLaunch("packTiles");
         planeproj::Problem pp{};

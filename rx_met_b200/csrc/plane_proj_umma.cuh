@@ -54,29 +54,30 @@ struct Problem {
     const uint32_t *planes = nullptr;   // [rows][PLANES][kWords] words of four unsigned bytes, kWords a multiple of 4
     int rows = 0, kWords = 0;
     const uint4 *tiles = nullptr;       // [C / 128][kPad / 16][16 channel groups]... = packTiles' output, 128 * kPad bytes per tile
-    int C = 0;                          // a multiple of 128
+    int C = 0;                          // channels beyond C in the last tile are computed and dropped
     int *status = nullptr;              // device word, set to 1 when a bounded wait of the kernel gave up
 };
 
 __host__ __device__ inline int paddedK(int kWords) { return (kWords * 4 + 31) / 32 * 32; }
+__host__ __device__ inline int paddedC(int C) { return (C + kChannelTile - 1) / kChannelTile * kChannelTile; }
 inline size_t sharedBytes(int kPad, int planes, int rowsPerTile) {
     return 2 * static_cast<size_t>(kChannelTile) * kPad + static_cast<size_t>(planes) * rowsPerTile * kPad;
 }
 
 // words [kWords][C] (four signed codes along k per word) -> per channel tile of 128 the canonical K-major A
 // operand: byte (c, k) of tile c / 128 at ((c % 128) / 8) * (kPad / 16) * 128 + (k / 16) * 128 + (c % 8) * 16 + k % 16;
-// k beyond 4 kWords is zero.  One thread per 16-byte row of a core matrix.
+// k beyond 4 kWords and channels beyond C are zero.  One thread per 16-byte row of a core matrix.
 static __global__ void packTiles(const uint32_t *__restrict__ words, int kWords, int C, int kPad, uint4 *__restrict__ tiles) {
-    const int groups = kPad / 16;
-    const size_t total = static_cast<size_t>(C) * groups;
+    const int groups = kPad / 16, padded = paddedC(C);
+    const size_t total = static_cast<size_t>(padded) * groups;
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
         // consecutive threads -> consecutive channels of one k-group (coalesced reads of the word rows)
-        const int kg = static_cast<int>(i / C), c = static_cast<int>(i % C);
+        const int kg = static_cast<int>(i / padded), c = static_cast<int>(i % padded);
         uint32_t v[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int kw = 4 * kg + e;
-            v[e] = kw < kWords ? words[static_cast<size_t>(kw) * C + c] : 0u;
+            v[e] = kw < kWords && c < C ? words[static_cast<size_t>(kw) * C + c] : 0u;
         }
         const size_t tile = c / kChannelTile, within = c % kChannelTile;
         const size_t at = tile * (static_cast<size_t>(kChannelTile) * kPad / 16) + (within / 8) * (static_cast<size_t>(groups) * 8) +
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const Problem p, co
     const uint32_t tmem = tmemSlot;
     volatile int *failFlag = &failed;
 
-    const int channelTiles = C / kChannelTile;
+    const int channelTiles = paddedC(C) / kChannelTile;
     const int rowTiles = (p.rows + NR - 1) / NR;
     const int q = warp & 3, group = warp >> 2;   // tensor-memory lane quarter (32 channels) of this warp, row-chunk group
 
@@ -134,7 +135,8 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const Problem p, co
         if (!*failFlag && !waitPhase(smemAddr(&bars[buf]), (local >> 1) & 1)) *failFlag = 1;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int c = ct * kChannelTile + 32 * q + lane;
-        const typename Epilogue::Channel ch = epi.channel(c);
+        const bool real = c < C;
+        const typename Epilogue::Channel ch = epi.channel(min(c, C - 1));
         for (int chunk = group; chunk < NR / 16; chunk += kThreads / 128) {
             uint32_t acc[PLANES][16];
 #pragma unroll
@@ -155,7 +157,7 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const Problem p, co
                 int32_t a[PLANES];
 #pragma unroll
                 for (int pl = 0; pl < PLANES; ++pl) a[pl] = static_cast<int32_t>(acc[pl][j]);
-                epi.store(ch, static_cast<size_t>(row0 + j), c, a);
+                if (real) epi.store(ch, static_cast<size_t>(row0 + j), c, a);
             }
         }
         // the MMAs of the item after next overwrite this buffer: order them behind these loads

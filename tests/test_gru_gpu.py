@@ -651,3 +651,23 @@ def test_mse_loss_helper():
         losses.mse_loss_grad(h[1:], target[:, :, :-1])
     with pytest.raises(RuntimeError):
         losses.mse_loss_grad(h[1:].cpu(), target.cpu())
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 8, 1), (2, 149, 5, 65), (3, 4, 70, 64), (3, 299, 8, 127), (4, 298, 9, 128), (2, 2, 9, 129),
+                                   (3, 300, 130, 72)], ids=lambda s: "x".join(map(str, s)))
+def test_forward_quant_lanes_of_a_unit(gl, shape):
+    """8-bit grids at the edges of the recurrence whose lanes share a hidden unit (64 and 128 units, one, two and four rows
+    per CTA with a partly empty last CTA) and one unit beyond it: codes, then each form of its outputs."""
+    from rx_met_b200 import gru_interface_binding as m
+    test_forward_quant_matches_restatement(gl, "w8a8", shape)
+    T, B, I, H = shape
+    prob, params = calibrated(shape, seed=sum(shape), cfg=ol.make_config(**CONFIGS["w8a8"]), with_h0=True)
+    want = ol.forward_quant("orc", *prob, params, training=True)
+    p = m.GRUQuantParams._from_c(params.c, [params.chan["scale_" + n].tolist() for n in ("W", "R", "bw", "br")])
+    for training in (False, True):
+        out = [t.cpu().numpy() for t in m.forward_quant_int_storage(training, T, B, I, H, *[gl.dev(a) for a in prob], p)]
+        assert np.array_equal(out[0], want["h"]) and np.array_equal(out[1], want["v"])
+        for name, flags in zip(cabi.MASK_NAMES, out[7:]):
+            order = ("x", "h0", "W", "R", "bw", "br", "weight_ih_linear", "weight_hh_linear", "gate_input", "gate_output", "h")
+            assert cabi.MASK_NAMES == order
+            assert flags.size == 0 if not training else np.array_equal(flags, want["masks"].arr[name]), name
