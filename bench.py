@@ -466,7 +466,7 @@ def run_ours(args):
     if rank == 0:
         sampler.start()
     total_ms = timed(resident, args.steps, args.warmup)
-    launches = timed.launches if replays is None else args.steps * eng.captured_launches
+    launches = timed.launches if replays is None else args.steps * eng.library_launches
     resident_host_ms = timed.host_ms
     clocks = sampler.stop() if rank == 0 else None
     st_per_step = T * B * world
@@ -985,7 +985,7 @@ def run_kws_body(args, torch, dist, lib, device, group, rank, world, local_rank)
         # one captured graph per resident input set: a replay is one launch for the whole step
         replays = [eng.capture_step(xs[k], ys[k], lr)[0] for k in range(4)]
         total_ms = timed(lambda i: replays[i % 4](), args.steps, args.warmup)
-        launches = args.steps * eng.captured_launches
+        launches = args.steps * eng.library_launches
     else:
         total_ms = timed(lambda i: eng.step(xs[i % 4], ys[i % 4], lr), args.steps, args.warmup)
         launches = timed.launches
@@ -1114,7 +1114,7 @@ def lstm_secondary(lib, torch, device, flush, profile_steps=0, T_override=None):
     torch.cuda.synchronize()
     per = {}
     for n in ["lstmQuantizeCodes", "lstmPrepChannels", "lstmInputLinearQ", "lstmRecurrentQ", "lstmDequantWeights",
-              "lstmPackStepMasks", "lstmRecurrentBackward", "lstmRecurrentBackwardMma", "lstmGemmNN", "lstmInputGradNarrow", "inputGradUmma", "lstmGemmRowsTN", "lstmReduceSplits",
+              "lstmPackStepMasks", "lstmRecurrentBackward", "lstmRecurrentBackwardCluster", "lstmGemmNN", "lstmInputGradNarrow", "inputGradUmma", "lstmGemmRowsTN", "lstmReduceSplits",
               "lstmColumnSums", "weightGradMma", "weightGradUmma", "lstmReduceWeightGradT"]:
         ms, cnt = C.c_double(), C.c_longlong()
         lib.rxmet_get_kernel_timing(n.encode(), C.byref(ms), C.byref(cnt))
@@ -1127,7 +1127,7 @@ def lstm_secondary(lib, torch, device, flush, profile_steps=0, T_override=None):
     C4 = 4 * H
     algorithmic = {"lstmQuantizeCodes": 5 * I, "lstmInputLinearQ": I + C4 * 4 + C4 * 5,
                    "lstmRecurrentQ": C4 * 4 + H + (4 * C4 + 3 * H) * 5 - C4 * 5, "lstmPackStepMasks": (4 * C4 + 3 * H) + 4 * H,
-                   "lstmRecurrentBackwardMma": (C4 + 3 * H + H) * 4 + 4 * H + 2 * C4 * 4,
+                   "lstmRecurrentBackwardCluster": (C4 + 3 * H + H) * 4 + 4 * H + 2 * C4 * 4,
                    "lstmRecurrentBackward": (C4 + 3 * H + H) * 4 + 4 * H + 2 * C4 * 4,
                    "inputGradUmma": C4 * 4 + I * 5, "weightGradUmma": 2 * C4 * 4 + (I + H) * 4}
     peak, peak_kind = _peaks()

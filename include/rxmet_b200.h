@@ -50,6 +50,9 @@ RXMET_API uint64_t rxmet_kernel_launch_count(void);
  * it.  No counterpart in the reference. */
 RXMET_API int rxmet_set_concurrent_passes(int passes);
 
+/* Number of kernel nodes of a captured graph (a cudaGraph_t). */
+RXMET_API int rxmet_graph_kernel_nodes(void *graph, int *kernels);
+
 /* Per-kernel timing, off by default.  While enabled every kernel launch of the
  * library is bracketed by CUDA events on its stream;
  * rxmet_get_kernel_timing waits for the recorded events and returns the summed

@@ -236,6 +236,22 @@ const char *rxmet_last_error(void) { return lastError().c_str(); }
 const char *rxmet_version(void) { return "rxmet_b200 0.1.0 (sm_100a)"; }
 uint64_t rxmet_kernel_launch_count(void) { return launchCounter().load(); }
 
+int rxmet_graph_kernel_nodes(void *graph, int *kernels) {
+    return guarded([&] {
+        RXMET_PTR(graph); RXMET_PTR(kernels);
+        size_t n = 0;
+        RXMET_CUDA(cudaGraphGetNodes(static_cast<cudaGraph_t>(graph), nullptr, &n));
+        std::vector<cudaGraphNode_t> nodes(n);
+        RXMET_CUDA(cudaGraphGetNodes(static_cast<cudaGraph_t>(graph), nodes.data(), &n));
+        *kernels = 0;
+        for (cudaGraphNode_t node : nodes) {
+            cudaGraphNodeType type;
+            RXMET_CUDA(cudaGraphNodeGetType(node, &type));
+            *kernels += type == cudaGraphNodeTypeKernel;
+        }
+    });
+}
+
 int rxmet_set_concurrent_passes(int passes) {
     concurrentPassesSetting().store(passes < 1 ? 1 : passes);
     return RXMET_OK;

@@ -311,7 +311,9 @@ void launchFor(const WideRecurrence &r, const Prepared &prepared, cudaStream_t s
     cell.maskHh = r.maskHh; cell.maskGateIn = r.maskGateIn; cell.maskGateOut = r.maskGateOut; cell.maskH = r.maskH;
     cell.maskIh = r.maskIh; cell.stepBits = r.stepBits;
     cell.poison = r.poison;
-    planerec::launchBest<Cell, HP, HP < 64 ? HP : 64, 2, 32, 8, 16>("recurrentForward", planerec::Problem{r.T, r.B, r.H, r.h0Planes}, cell, st);
+    const planerec::Problem problem{r.T, r.B, r.H, r.h0Planes};
+    if constexpr (HP < 64) planerec::launchBest<Cell, HP, HP, 2, 32, 8, 16>("recurrentForward", problem, cell, st);
+    else planerec::launchBest<Cell, HP, 64, 2, 32, 4, 8, 16>("recurrentForward", problem, cell, st);
 }
 template <int HP>
 void launchFor(const WideRecurrence &r, const Prepared &prepared, cudaStream_t st) {

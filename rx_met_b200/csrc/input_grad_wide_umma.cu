@@ -375,7 +375,9 @@ size_t widePackedBytes(int K, int N) { return (N > kMaxColumns || K % kChunk != 
 bool wideTakes(int K, int N) {
     static const bool disabled = std::getenv("RXMET_IGRAD_SIMT") != nullptr || std::getenv("RXMET_IGRAD_NARROW") != nullptr;
     static const int least = std::getenv("RXMET_IGRAD_STREAM_ALL") != nullptr ? 1 : 65;
-    return !disabled && N >= least && N <= kMaxColumns && K >= kChunk && K % kChunk == 0 && encodeTiled() != nullptr;
+    // few columns stay with the resident-weight kernel for the channel counts it takes
+    const bool resident = K <= 768 && K % 64 == 0;
+    return !disabled && (N >= least || !resident) && N <= kMaxColumns && K >= kChunk && K % kChunk == 0 && encodeTiled() != nullptr;
 }
 
 bool wideEligible(const Problem &p) {

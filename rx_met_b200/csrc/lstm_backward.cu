@@ -20,6 +20,7 @@
 
 #include "common.h"
 #include "input_grad_umma.h"
+#include "lstm_backward_cluster.h"
 #include "lstm_kernels.h"
 #include "umma_device.cuh"
 #include "weight_grad_mma.h"
@@ -354,14 +355,6 @@ __global__ void __launch_bounds__(512, 1) recurrentBackwardWide(const __grid_con
     }
 }
 
-// ---- dh = G_hh W_hh on tensor cores (QAT with weight grids of at most 8 bits) ------------------
-//
-// Same data flow as recurrentBackward, but the per-step product runs as mma.sync m16n8k16 with
-// M = hidden column k, N = batch tile (padded to 8), K = the 4H channels.  Warp w owns two m16 tiles
-// (hidden columns 32*(w/4) .. +31) and the K range of gate w%4; its A fragments - the integer weight
-// codes, exact in bf16 - stay in registers for the whole sequence.  The gate gradient, multiplied by
-// the channel's weight scale, is split into three bf16 terms in shared memory so that every product
-// is exact and only the fp32 accumulation rounds.
 __device__ __forceinline__ uint32_t packBf16(float lo, float hi) {
     uint32_t r;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
@@ -369,155 +362,7 @@ __device__ __forceinline__ uint32_t packBf16(float lo, float hi) {
 }
 __device__ __forceinline__ float bf16Lo(uint32_t v) { return __uint_as_float(v << 16); }
 
-struct RecurrentMmaArgs {
-    RecurrentArgs base;
-    const float *weightCodes;   // q-carrier codes [4H][H]
-    const float *channelScale;  // [4H] scale of weight_hh per channel
-};
-
-template <int HT, int BT>  // H = 32*HT, blockDim = 128*HT
-__global__ void __launch_bounds__(128 * HT) recurrentBackwardMma(const __grid_constant__ RecurrentMmaArgs args) {
-    const RecurrentArgs &a = args.base;
-    constexpr int H = 32 * HT, C = 4 * H, KS = 2 * HT;  // k16 steps per warp
-    constexpr int CP = C + 8;                           // padded row of the bf16 gradient tiles
-    __shared__ __align__(16) uint16_t gB[3][8][CP];     // [split][batch row][channel]
-    __shared__ float partS[4][BT][H];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthreads = blockDim.x;
-    const int g8 = lane >> 2, t4 = lane & 3;
-    const int grp = warp % 4, mpair = warp / 4;
-    const int b0 = blockIdx.x * BT, nb = min(BT, a.B - b0);
-
-    // A fragments: element (m = hidden column, k = channel) = code[channel][hidden column]
-    uint32_t afrag[2][KS][4];
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int ks = 0; ks < KS; ++ks)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int row = mpair * 32 + mt * 16 + g8 + (q & 1) * 8;
-                const int col = grp * H + ks * 16 + 2 * t4 + (q >> 1) * 8;
-                const float w0 = args.weightCodes[static_cast<size_t>(col) * H + row];
-                const float w1 = args.weightCodes[static_cast<size_t>(col + 1) * H + row];
-                afrag[mt][ks][q] = (__float_as_uint(w0) >> 16) | (__float_as_uint(w1) & 0xffff0000u);
-            }
-    for (int i = tid; i < 3 * 8 * CP; i += nthreads) (&gB[0][0][0])[i] = 0;
-    for (int i = tid; i < 4 * BT * H; i += nthreads) (&partS[0][0][0])[i] = 0.0f;
-
-    const int elems = nb * H;
-    const bool hasElem = tid < elems;
-    const int eb = hasElem ? tid / H : 0, ej = hasElem ? tid % H : 0;
-    const size_t stateIdx = static_cast<size_t>(b0 + eb) * H + ej;
-    float dhCarry = hasElem ? a.gradFinalHidden[stateIdx] : 0.0f;
-    float dc = hasElem ? a.gradFinalCell[stateIdx] : 0.0f;
-    float scale[4];
-#pragma unroll
-    for (int g = 0; g < 4; ++g) scale[g] = args.channelScale[g * H + ej];
-
-    struct StepIn {
-        float gate[4], ct, cPrev, gradOut;
-        uint32_t bits;
-    };
-    auto fetch = [&](int t, StepIn &in) {
-        if (!hasElem) return;
-        const size_t row = static_cast<size_t>(t) * a.B + b0 + eb, so = row * H + ej, go = row * C + ej;
-#pragma unroll
-        for (int g = 0; g < 4; ++g) in.gate[g] = a.gateOutputs[go + static_cast<size_t>(g) * H];
-        in.ct = a.cellTanh[so];
-        in.cPrev = t > 0 ? a.cellStates[so - static_cast<size_t>(a.B) * H] : (a.c0 ? a.c0[stateIdx] : a.dqC.zeroPoint);
-        in.gradOut = a.gradOutput[so];
-        in.bits = a.stepMasks ? a.stepMasks[so] : 0u;
-    };
-    auto splitStore = [&](int b, int c, float v) {
-        const float hi = bf16Lo(packBf16(v, 0.0f));
-        const float r1 = v - hi;
-        const float mid = bf16Lo(packBf16(r1, 0.0f));
-        const float lo = r1 - mid;
-        gB[0][b][c] = static_cast<uint16_t>(__float_as_uint(hi) >> 16);
-        gB[1][b][c] = static_cast<uint16_t>(__float_as_uint(mid) >> 16);
-        gB[2][b][c] = static_cast<uint16_t>(packBf16(lo, 0.0f) & 0xffffu);
-    };
-    StepIn cur{}, nxt{};
-    fetch(a.T - 1, cur);
-    __syncthreads();
-
-    for (int t = a.T - 1; t >= 0; --t) {
-        const size_t rowBase = static_cast<size_t>(t) * a.B + b0;
-        if (t > 0) fetch(t - 1, nxt);
-        if (hasElem) {
-            const size_t row = rowBase + eb, go = row * C + ej;
-            auto keepBit = [&](int b) { return (cur.bits >> b) & 1u ? 0.0f : 1.0f; };
-            const float ig = realOf(cur.gate[0], a.dqGate[0]), fg = realOf(cur.gate[1], a.dqGate[1]);
-            const float cg = realOf(cur.gate[2], a.dqGate[2]), og = realOf(cur.gate[3], a.dqGate[3]);
-            const float ct = realOf(cur.ct, a.dqTanh);
-            const float cPrev = realOf(cur.cPrev, a.dqC);
-            const float incoming = dhCarry + partS[0][eb][ej] + partS[1][eb][ej] + partS[2][eb][ej] + partS[3][eb][ej];
-            const float dh = (incoming + cur.gradOut) * keepBit(0);
-            const float gOut = dh * ct;
-            const float gTanh = dh * og * keepBit(1);
-            const float dcAll = dc + gTanh * (1.0f - ct * ct);
-            const float mdc = dcAll * keepBit(2);
-            const float go4[4] = {mdc * cg * keepBit(3), mdc * cPrev * keepBit(4), mdc * ig * keepBit(5), gOut * keepBit(6)};
-            const float gi4[4] = {go4[0] * ig * (1.0f - ig), go4[1] * fg * (1.0f - fg), go4[2] * (1.0f - cg * cg),
-                                  go4[3] * og * (1.0f - og)};
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                const size_t o = go + static_cast<size_t>(g) * H;
-                const float grad = gi4[g] * keepBit(7 + g);
-                const float hh = grad * keepBit(15 + g);
-                a.gIh[o] = grad * keepBit(11 + g);
-                a.gHh[o] = hh;
-                splitStore(eb, g * H + ej, hh * scale[g]);
-            }
-            dc = mdc * fg;
-            dhCarry = 0.0f;
-        }
-        cur = nxt;
-        __syncthreads();
-        {
-            float acc[2][3][4];
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-                for (int sp = 0; sp < 3; ++sp) acc[mt][sp][0] = acc[mt][sp][1] = acc[mt][sp][2] = acc[mt][sp][3] = 0.0f;
-#pragma unroll
-            for (int ks = 0; ks < KS; ++ks) {
-                const int c0 = grp * H + ks * 16 + 2 * t4;
-#pragma unroll
-                for (int sp = 0; sp < 3; ++sp) {
-                    const uint32_t bf0 = *reinterpret_cast<const uint32_t *>(&gB[sp][g8][c0]);
-                    const uint32_t bf1 = *reinterpret_cast<const uint32_t *>(&gB[sp][g8][c0 + 8]);
-#pragma unroll
-                    for (int mt = 0; mt < 2; ++mt) {
-                        asm volatile(
-                            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-                            "{%0,%1,%2,%3};"
-                            : "+f"(acc[mt][sp][0]), "+f"(acc[mt][sp][1]), "+f"(acc[mt][sp][2]), "+f"(acc[mt][sp][3])
-                            : "r"(afrag[mt][ks][0]), "r"(afrag[mt][ks][1]), "r"(afrag[mt][ks][2]), "r"(afrag[mt][ks][3]),
-                              "r"(bf0), "r"(bf1));
-                    }
-                }
-            }
-            // D fragment: rows g8 / g8+8 are hidden columns, columns 2*t4 / 2*t4+1 are batch rows
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int n = 2 * t4 + (q & 1);
-                    const int k = mpair * 32 + mt * 16 + g8 + (q >> 1) * 8;
-                    if (n < BT) partS[grp][n][k] = (acc[mt][2][q] + acc[mt][1][q]) + acc[mt][0][q];
-                }
-        }
-        __syncthreads();
-    }
-    if (hasElem) {
-        const float dh0 = dhCarry + partS[0][eb][ej] + partS[1][eb][ej] + partS[2][eb][ej] + partS[3][eb][ej];
-        a.dh0[stateIdx] = dh0 * keepOf(a.mk.initial_hidden, stateIdx);
-        a.dc0[stateIdx] = dc * keepOf(a.mk.initial_cell, stateIdx);
-    }
-}
-
-// ---- hidden sizes above 128 on the tcgen05 tensor cores (QAT with weight grids of at most 8 bits) ---------
+// ---- hidden sizes above 256 on the tcgen05 tensor cores (QAT with weight grids of at most 8 bits) ---------
 //
 // dh[b][j] = sum_c G_hh[b][c] * code[c][j] * scale[c] needs every channel of a row for every hidden unit, and
 // weight_hh (4H x H) fits no single SM.  The contraction is therefore split over the CTAs of a row tile:
@@ -1074,7 +919,7 @@ constexpr int kMaxTensorSplits = 40;
 }  // namespace
 
 // The tcgen05 recurrence of wide layers takes hidden sizes whose accumulator quarters are whole 32-column pieces.
-bool wideTensorShape(int H) { return H > 128 && H <= 512 && H % 128 == 0; }
+bool wideTensorShape(int H) { return H > 256 && H <= 512 && H % 128 == 0; }
 // Row tiles (128 batch rows) one cooperative launch holds: every CTA must be resident, one per SM.
 int wideTensorRowTiles(int B, int H) {
     const int tilesPerRow = H / kBwdUnits;
@@ -1098,7 +943,6 @@ size_t backwardWorkspaceBytes(int T, int B, int I, int H) {
     ws.take<float>(static_cast<size_t>(splitsFor(static_cast<int>(rows), tilesOf(static_cast<int>(C), I))) * C * I);
     ws.take<float>(static_cast<size_t>(splitsFor(static_cast<int>(rows), tilesOf(static_cast<int>(C), H))) * C * H);
     ws.take<float>(2 * kBiasSplits * C);
-    ws.take<float>(2 * C);     // per-channel weight scales (QAT)
     ws.take<float>(rows * H);  // h_prev codes for the tensor-core weight gradient (QAT)
     ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, I, static_cast<int>(C))) * (I + 1) * C);
     ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, H, static_cast<int>(C))) * (H + 1) * C);
@@ -1128,7 +972,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
     float *partIh = ws.take<float>(static_cast<size_t>(splitIh) * C * I);
     float *partHh = ws.take<float>(static_cast<size_t>(splitHh) * C * H);
     float *partBias = ws.take<float>(2 * kBiasSplits * static_cast<size_t>(C));
-    float *channelScales = ws.take<float>(2 * static_cast<size_t>(C));
+    const float *channelScales = call.channelScales;   // weight_ih, weight_hh
     float *hPrev = ws.take<float>(rows * H);
     float *tensorIh = ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, I, C)) * (I + 1) * C);
     float *tensorHh = ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, H, C)) * (H + 1) * C);
@@ -1137,8 +981,22 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
 
     // Which kernels multiply by the saved integer weight codes directly (QAT on 8-bit grids); the
     // others read real-valued weights rebuilt here.
-    const bool tensorPath = !wide && call.quantized && call.weightCodesFitBf16 && H % 32 == 0 && H <= 128 &&
-                            std::getenv("RXMET_LSTM_BWD_SIMT") == nullptr;
+    const rxmet_lstm_backward_masks none{};
+    const rxmet_lstm_backward_masks &mk = call.masks ? *call.masks : none;
+    const bool anyStepMask = mk.hidden_outputs || mk.cell_tanh_outputs || mk.cell_states || mk.gate_outputs ||
+                             mk.gate_inputs || mk.weight_ih_linear || mk.weight_hh_linear;
+    const bool codes = call.quantized && call.weightCodesFitBf16 && std::getenv("RXMET_LSTM_BWD_SIMT") == nullptr;
+    BackwardClusterArgs cl{};
+    cl.T = T; cl.B = B; cl.H = H;
+    cl.stepMasks = anyStepMask ? stepMasks : nullptr;
+    cl.weightCodes = call.weightHh; cl.channelScale = channelScales ? channelScales + C : nullptr; cl.c0 = call.c0;
+    cl.gateOutputs = call.gateOutputs; cl.cellStates = call.cellStates; cl.cellTanh = call.cellTanhOutputs;
+    cl.gradOutput = call.gradOutput; cl.gradFinalHidden = call.gradFinalHidden; cl.gradFinalCell = call.gradFinalCell;
+    cl.dqC = call.dqC; cl.dqTanh = call.dqTanh;
+    std::copy(call.dqGate, call.dqGate + 4, cl.dqGate);
+    cl.maskH0 = static_cast<const uint8_t *>(mk.initial_hidden); cl.maskC0 = static_cast<const uint8_t *>(mk.initial_cell);
+    cl.gIh = gIh; cl.gHh = gHh; cl.dh0 = call.grads.initial_hidden; cl.dc0 = call.grads.initial_cell;
+    const bool clusterPath = codes && backwardClusterTakes(cl);
     // Wide layers: the tcgen05 recurrence (float4 loads of the saved tensors and of the incoming gradients)
     uint4 *wideTiles = nullptr;
     float *widePartial = nullptr;
@@ -1151,26 +1009,24 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
     const size_t wideSmem = static_cast<size_t>(H) * 256 + 3 * kBwdSplitBytes;
     int cooperative = 0;
     RXMET_CUDA(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, currentDevice().device));
-    const bool wideTensor = wide && wideTensorShape(H) && call.quantized && call.weightCodesFitBf16 && cooperative != 0 &&
+    const bool wideTensor = wide && wideTensorShape(H) && codes && cooperative != 0 &&
                             H / kBwdUnits <= smsPerPass() && wideSmem <= static_cast<size_t>(currentDevice().smemMax) &&
                             alignedTo(call.gateOutputs, 16) && alignedTo(call.cellStates, 16) && alignedTo(call.cellTanhOutputs, 16) &&
                             alignedTo(call.gradOutput, 16) && alignedTo(call.gradFinalHidden, 16) && alignedTo(call.gradFinalCell, 16) &&
-                            alignedTo(call.c0, 16) && std::getenv("RXMET_LSTM_BWD_SIMT") == nullptr;
+                            alignedTo(call.c0, 16);
     // 16-byte copies of the caller's weight codes, float4 stores of dx and 8-byte loads of the input mask
     const bool tensorInputGrad = call.quantized && call.weightIhCodesFitBf16 && igrad::eligible(C, I) &&
                                  alignedTo(call.grads.input, 16) && alignedTo(call.weightIh, 16) &&
                                  (call.masks == nullptr || alignedTo(call.masks->input, 8));
     const float *wIh = call.weightIh, *wHh = call.weightHh;
     if (call.quantized) {
-        RXMET_REQUIRE(call.weightIhScale && call.weightHhScale, "per-channel weight scales missing");
-        RXMET_CUDA(cudaMemcpyAsync(channelScales, call.weightIhScale, sizeof(float) * C, cudaMemcpyHostToDevice, st));
-        RXMET_CUDA(cudaMemcpyAsync(channelScales + C, call.weightHhScale, sizeof(float) * C, cudaMemcpyHostToDevice, st));
+        RXMET_REQUIRE(channelScales, "per-channel weight scales missing");
         if (!tensorInputGrad) {
             KernelTimer timer__("lstmDequantWeights", st);
             dequantWeights<<<gridFor(static_cast<size_t>(C) * I, 256), 256, 0, st>>>(call.weightIh, channelScales, C, I, wIhReal);
             afterLaunch("lstmDequantWeights");
         }
-        if (!tensorPath && !wideTensor) {
+        if (!clusterPath && !wideTensor) {
             KernelTimer timer__("lstmDequantWeights", st);
             dequantWeights<<<gridFor(static_cast<size_t>(C) * H, 256), 256, 0, st>>>(call.weightHh, channelScales + C, C, H, wHhReal);
             afterLaunch("lstmDequantWeights");
@@ -1178,10 +1034,6 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         wIh = wIhReal;
         wHh = wHhReal;
     }
-    const rxmet_lstm_backward_masks none{};
-    const rxmet_lstm_backward_masks &mk = call.masks ? *call.masks : none;
-    const bool anyStepMask = mk.hidden_outputs || mk.cell_tanh_outputs || mk.cell_states || mk.gate_outputs ||
-                             mk.gate_inputs || mk.weight_ih_linear || mk.weight_hh_linear;
     if (anyStepMask) {
         {
             KernelTimer timer__("lstmPackStepMasks", st);
@@ -1208,26 +1060,8 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         const int smemMax = currentDevice().smemMax, sms = currentDevice().sms;
         const int bt = (B >= 4 * sms) ? 4 : ((B > sms) ? 2 : 1);
         const int block = (C + 31) / 32 * 32;
-        if (tensorPath) {
-            RecurrentMmaArgs m{};
-            m.base = a;
-            m.weightCodes = call.weightHh;  // q-carrier codes as saved by the forward
-            m.channelScale = channelScales + C;
-            bool launched = false;
-#define RXMET_LSTM_MMA(HTV, BTV)                                                     \
-    if (!launched && H == 32 * HTV && bt == BTV) {                                    \
-        KernelTimer timer__("lstmRecurrentBackwardMma", st);                         \
-        recurrentBackwardMma<HTV, BTV><<<(B + BTV - 1) / BTV, 128 * HTV, 0, st>>>(m); \
-        launched = true;                                                              \
-    }
-            RXMET_LSTM_MMA(1, 1) RXMET_LSTM_MMA(1, 2) RXMET_LSTM_MMA(1, 4)
-            RXMET_LSTM_MMA(2, 1) RXMET_LSTM_MMA(2, 2) RXMET_LSTM_MMA(2, 4)
-            RXMET_LSTM_MMA(3, 1) RXMET_LSTM_MMA(3, 2) RXMET_LSTM_MMA(3, 4)
-            RXMET_LSTM_MMA(4, 1) RXMET_LSTM_MMA(4, 2) RXMET_LSTM_MMA(4, 4)
-#undef RXMET_LSTM_MMA
-            afterLaunch("lstmRecurrentBackwardMma");
-        }
-        if (wideTensor) {
+        if (clusterPath) backwardCluster(cl, st);
+        else if (wideTensor) {
             {
                 KernelTimer timer__("lstmPackBackwardTiles", st);
                 packBackwardTiles<<<gridFor(static_cast<size_t>(H / kBwdUnits) * 16 * H, 256), 256, 0, st>>>(call.weightHh, H, wideTiles);
@@ -1278,7 +1112,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
             afterLaunch("lstmRecurrentBackwardWide");
         }
         auto launch = [&](auto kernel, int BT) {
-            if (tensorPath || wide) return;
+            if (clusterPath || wide) return;
             const size_t base = sizeof(float) * (static_cast<size_t>(BT) * C + 4 * static_cast<size_t>(BT) * H);
             const size_t room = static_cast<size_t>(smemMax) > base + 1024 ? static_cast<size_t>(smemMax) - base - 1024 : 0;
             // rows per gate block in shared memory; the remaining rows of a block live in registers

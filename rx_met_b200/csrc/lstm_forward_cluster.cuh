@@ -224,9 +224,9 @@ void launchLstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &c
         LstmPlaneCell<TRAIN, HP> full;
         static_assert(sizeof(full) == sizeof(cell), "the variants differ in the width only");
         std::memcpy(&full, &cell, sizeof(full));
-        planerec::launchBest<LstmPlaneCell<TRAIN, HP>, HP, 64, 2, 5, 8, 16, 24, 32>("lstmRecurrentWide", p, full, st);
+        planerec::launchBest<LstmPlaneCell<TRAIN, HP>, HP, 64, 2, 5, 4, 8, 16, 24, 32>("lstmRecurrentWide", p, full, st);
     } else {
-        planerec::launchBest<LstmPlaneCell<TRAIN>, HP, 64, 2, 5, 8, 16, 24, 32>("lstmRecurrentWide", p, cell, st);
+        planerec::launchBest<LstmPlaneCell<TRAIN>, HP, 64, 2, 5, 4, 8, 16, 24, 32>("lstmRecurrentWide", p, cell, st);
     }
 }
 // One padded width each, built in separate files (lstm_forward_cluster_*.cu).

@@ -391,7 +391,7 @@ Plan planFor(int T, int B, int I, int H) {
 
 template <class W>
 void layout(W &ws, int T, int B, int I, int H, int8_t **x, int8_t **h0, float **c0, uint32_t **wIh, uint32_t **wHh,
-            int32_t **addIh, int32_t **addHh, float **channel, int32_t **tables, float **lhs) {
+            int32_t **addIh, int32_t **addHh, float **lhs) {
     const Plan p = planFor(T, B, I, H);
     const size_t C = 4 * static_cast<size_t>(H);
     auto set = [](auto **dst, auto *v) { if (dst) *dst = v; };
@@ -402,8 +402,6 @@ void layout(W &ws, int T, int B, int I, int H, int8_t **x, int8_t **h0, float **
     set(wHh, ws.template take<uint32_t>(p.kWordsHh * C));
     set(addIh, ws.template take<int32_t>(C));
     set(addHh, ws.template take<int32_t>(C));
-    set(channel, ws.template take<float>(kChannelFields * C));
-    set(tables, ws.template take<int32_t>(kTables * kTableSize));
     set(lhs, ws.template take<float>(p.rows * C));
 }
 
@@ -434,8 +432,7 @@ size_t forwardQuantWorkspaceBytes(int T, int B, int I, int H) {
     SizerAdapter s;
     layout(s, T, B, I, H, static_cast<int8_t **>(nullptr), static_cast<int8_t **>(nullptr), static_cast<float **>(nullptr),
            static_cast<uint32_t **>(nullptr), static_cast<uint32_t **>(nullptr), static_cast<int32_t **>(nullptr),
-           static_cast<int32_t **>(nullptr), static_cast<float **>(nullptr), static_cast<int32_t **>(nullptr),
-           static_cast<float **>(nullptr));
+           static_cast<int32_t **>(nullptr), static_cast<float **>(nullptr));
     return std::max(s.ws.used() + 1024, forwardQuantWideWorkspaceBytes(T, B, I, H));
 }
 
@@ -453,12 +450,12 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, 
     const Plan p = planFor(T, B, I, H);
     Workspace ws(workspace, workspaceBytes);
     int8_t *xq, *h0q;
-    float *c0c, *channel, *lhs;
+    float *c0c, *lhs;
     uint32_t *wIh, *wHh;
-    int32_t *addIh, *addHh, *tables;
-    layout(ws, T, B, I, H, &xq, &h0q, &c0c, &wIh, &wHh, &addIh, &addHh, &channel, &tables, &lhs);
-    RXMET_CUDA(cudaMemcpyAsync(channel, e.channel.data(), e.channel.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-    RXMET_CUDA(cudaMemcpyAsync(tables, e.tables.data(), e.tables.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+    int32_t *addIh, *addHh;
+    layout(ws, T, B, I, H, &xq, &h0q, &c0c, &wIh, &wHh, &addIh, &addHh, &lhs);
+    const float *channel = e.channelOnDevice();
+    const int32_t *tables = e.tablesOnDevice();
 
     const rxmet_lstm_masters none{};
     const rxmet_lstm_masters &m = call.masters ? *call.masters : none;

@@ -811,7 +811,8 @@ int wordsFor(int k) { return (k + 15) / 16 * 4; }
 
 struct WideLayout {
     uint32_t *x, *h0, *wIh, *wHh;
-    float *c0, *channel, *lhs;
+    float *c0, *lhs;
+    const float *channel;
     int64_t *addIh, *addHh;
     uint4 *ihTiles;    // weight_ih as canonical tensor-core tiles (plane_proj_umma.cuh)
     int *projStatus;
@@ -863,7 +864,6 @@ WideLayout layoutWide(W &ws, int T, int B, int I, int H, int planes) {
     l.wHh = ws.template take<uint32_t>(kHh * C);
     l.addIh = ws.template take<int64_t>(C);
     l.addHh = ws.template take<int64_t>(C);
-    l.channel = ws.template take<float>(kChannelFields * C);
     l.lhs = ws.template take<float>(rows * C);
     l.ihTiles = ws.template take<uint4>(static_cast<size_t>(planeproj::paddedC(static_cast<int>(C))) * planeproj::paddedK(static_cast<int>(kIh)) / 16);
     l.projStatus = ws.template take<int>(1);
@@ -932,9 +932,9 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
     const int kIh = wordsFor(I), kHh = wordsFor(H);
     const size_t rows = static_cast<size_t>(T) * B;
     Workspace ws(workspace, workspaceBytes);
-    const WideLayout l = layoutWide(ws, T, B, I, H, planes);
+    WideLayout l = layoutWide(ws, T, B, I, H, planes);
     const int32_t *tables = e.wideTablesOnDevice();
-    RXMET_CUDA(cudaMemcpyAsync(l.channel, e.channel.data(), e.channel.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+    l.channel = e.channelOnDevice();
 
     const rxmet_lstm_masters none{};
     const rxmet_lstm_masters &m = call.masters ? *call.masters : none;

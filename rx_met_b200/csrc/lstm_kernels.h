@@ -64,10 +64,10 @@ struct BackwardCall {
     const float *gradOutput, *gradFinalHidden, *gradFinalCell;
     const rxmet_lstm_backward_masks *masks;  // optional
     rxmet_lstm_gradients grads;
-    // QAT: grids of the saved tensors and per-channel weight scales (host, 4H each); null = float
+    // QAT: grids of the saved tensors and per-channel weight scales (4H each); null = float
     bool quantized = false;
     Dequant dqX, dqH, dqC, dqGate[4], dqTanh;
-    const float *weightIhScale = nullptr, *weightHhScale = nullptr;
+    const float *channelScales = nullptr;   // device: weight_ih, then weight_hh
     bool codesFitTensorPath = false;  // x and hidden grids span at most 256 codes around their zero points
     bool codesFitTwoTerms = false;    // x and hidden grids of at most 16 bits: a code is two exact bf16 terms
     bool weightCodesFitBf16 = false;  // weight_hh grid of at most 8 bits: codes are exact in bf16

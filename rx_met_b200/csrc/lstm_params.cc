@@ -664,7 +664,7 @@ T *deviceCopy(std::mutex &mutex, std::vector<std::pair<int, std::shared_ptr<T>>>
     std::lock_guard<std::mutex> lock(mutex);
     for (const auto &entry : copies)
         if (entry.first == device) return entry.second.get();
-    RXMET_REQUIRE(bytes > 0, "activation tables of this parameter set were not built");
+    RXMET_REQUIRE(bytes > 0, "the parameter set has no such table");
     T *buffer = nullptr;
     RXMET_CUDA(cudaMalloc(reinterpret_cast<void **>(&buffer), bytes));
     std::shared_ptr<T> owner(buffer, [](T *ptr) { cudaFree(ptr); });
@@ -678,6 +678,14 @@ T *deviceCopy(std::mutex &mutex, std::vector<std::pair<int, std::shared_ptr<T>>>
 
 const int32_t *Exec::wideTablesOnDevice() const {
     return deviceCopy(deviceLock, deviceTables, wide.entries.data(), wide.entries.size() * sizeof(int32_t));
+}
+
+const float *Exec::channelOnDevice() const {
+    return deviceCopy(deviceLock, deviceChannel, channel.data(), channel.size() * sizeof(float));
+}
+
+const int32_t *Exec::tablesOnDevice() const {
+    return deviceCopy(deviceLock, deviceSmallTables, tables.data(), tables.size() * sizeof(int32_t));
 }
 
 const uint8_t *Exec::compactTablesOnDevice() const {

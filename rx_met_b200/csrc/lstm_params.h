@@ -114,6 +114,11 @@ struct Exec {
     // The compact form of the wide tables, built on first use, and its device copy.
     const CompactTables &compactTables() const;
     const uint8_t *compactTablesOnDevice() const;
+    // Device copies of `channel` and of `tables`.
+    const float *channelOnDevice() const;
+    const int32_t *tablesOnDevice() const;
+    mutable std::vector<std::pair<int, std::shared_ptr<float>>> deviceChannel;
+    mutable std::vector<std::pair<int, std::shared_ptr<int32_t>>> deviceSmallTables;
     mutable std::once_flag compactOnce;
     mutable CompactTables compact;
     mutable std::vector<std::pair<int, std::shared_ptr<uint8_t>>> deviceCompact;

@@ -319,7 +319,8 @@ void launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t s
 }
 
 // Rows of a cluster among ROWS...: the number of waves times the cost of a step, which is about 1 + rows / PER of the
-// chain of a short one - as few rows as let all clusters run at the same time, or many where they cannot.
+// chain of a short one - as few rows as let all clusters run at the same time, or many where they cannot.  Four rows only
+// where they leave half of the GPU free: the other direction of a layer may run beside this pass.
 template <class Cell, int HP, int U, int PLANES, int PER, int... ROWS>
 void launchBest(const char *name, const Problem &p, const Cell &cell, cudaStream_t st) {
     double bestCost = 1e30;
@@ -331,6 +332,7 @@ void launchBest(const char *name, const Problem &p, const Cell &cell, cudaStream
             const int resident = std::max(1, residentClusters(reinterpret_cast<const void *>(planeRecurrence<Cell, HP, U, ROWS, PLANES>), G::kCtas,
                                                               G::kThreads, G::kSharedBytes + cell.sharedBytes()) / concurrentPasses());
             const int clusters = (p.B + ROWS - 1) / ROWS, waves = (clusters + resident - 1) / resident;
+            if (ROWS == 4 && 2 * clusters > resident) return;
             const double cost = waves * (1.0 + ROWS / static_cast<double>(PER));
             if (cost < bestCost) { bestCost = cost; best = ROWS; }
         }(),

@@ -23,6 +23,13 @@ def _p(t: Optional[torch.Tensor]):
     return C.c_void_p(t.data_ptr()) if t is not None else None
 
 
+def graph_kernels(graph: torch.cuda.CUDAGraph) -> int:
+    """Kernel nodes of a captured graph (kept with keep_graph=True)."""
+    count = C.c_int()
+    cabi.check(cabi.load_library().rxmet_graph_kernel_nodes(C.c_void_p(graph.raw_cuda_graph()), C.byref(count)), "graph_kernels")
+    return count.value
+
+
 class GruQatStep:
     def __init__(self, T: int, B: int, I: int, H: int, device: torch.device,
                  config: Optional[OperatorQuantConfig] = None, process_group=None, seed: int = 0,
@@ -232,11 +239,13 @@ class GruQatStep:
             for _ in range(max(warmup, 1)):
                 self.step(x, target, lr)
         torch.cuda.current_stream(self.device).wait_stream(side)
-        graph = torch.cuda.CUDAGraph()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
         before = self.lib.rxmet_kernel_launch_count()
         with torch.cuda.graph(graph, stream=side):
             loss = body()
-        self.captured_launches = int(self.lib.rxmet_kernel_launch_count() - before)  # library kernels per replay
+        self.library_launches = int(self.lib.rxmet_kernel_launch_count() - before)  # kernels of this library per replay
+        self.captured_launches = graph_kernels(graph)                               # all kernels per replay
+        graph.instantiate()
 
         def replay():
             graph.replay()

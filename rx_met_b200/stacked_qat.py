@@ -24,7 +24,7 @@ from typing import List, Optional
 import torch
 
 from .gru_interface_binding import OperatorQuantConfig
-from .qat import GruQatStep
+from .qat import GruQatStep, graph_kernels
 
 
 def a16_config(weight_bits: int = 8, activation_bits: int = 16) -> OperatorQuantConfig:
@@ -178,7 +178,7 @@ class StackedGruQat:
                 dy = self.dx[li]
 
     def capture_step(self, x: torch.Tensor, labels: torch.Tensor, lr: float, warmup: int = 2):
-        """Captures `step` on fixed buffers into ONE CUDA graph - about 600 kernel launches on two streams per
+        """Captures `step` on fixed buffers into ONE CUDA graph - about 100 kernel launches on two streams per
         step at three layers - and returns `(replay, loss)`: `replay()` launches the whole step and returns `loss`,
         the device scalar it refreshes.  `x` and `labels` are read at replay time, so the caller refills them in
         place.  With a process group the gradient all-reduce and the update follow the graph launch.  The
@@ -191,14 +191,16 @@ class StackedGruQat:
             for _ in range(max(warmup, 1)):
                 self.step(x, labels, lr)
         torch.cuda.current_stream(self.device).wait_stream(stream)
-        graph = torch.cuda.CUDAGraph()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
         before = self._lib.rxmet_kernel_launch_count()
         with torch.cuda.graph(graph, stream=stream):
             loss = self.head(self.forward(x), labels)
             self.backward()
             if local:
                 self.flat_w.add_(self.flat_g, alpha=-lr)
-        self.captured_launches = int(self._lib.rxmet_kernel_launch_count() - before)   # library kernels per replay
+        self.library_launches = int(self._lib.rxmet_kernel_launch_count() - before)   # kernels of this library per replay
+        self.captured_launches = graph_kernels(graph)                                 # all kernels per replay
+        graph.instantiate()
 
         def replay():
             graph.replay()
