@@ -22,6 +22,7 @@
 #include "common.h"
 #include "gru_backward.h"
 #include "gru_backward_cluster.h"
+#include "regroup.h"
 #include "gru_forward_quant.h"
 #include "input_grad_umma.h"
 #include "weight_grad_mma.h"
@@ -178,18 +179,22 @@ __global__ void packRecurrentBf16(const int32_t *__restrict__ Rq, int H, int CW,
 // needs: bits 0..2 gate_output (z,r,n), 3..5 gate_input, 6..8 weight_hh_linear, 9..11
 // weight_ih_linear, 12 h.  Packing them once, outside the serial time loop, replaces 13 byte loads
 // per element and step on the critical path by one.
+// `given` holds the words already; `width` >= H: words per row of out, the ones beyond H keep everything.
 __global__ void packStepMasks(const uint8_t *__restrict__ mIh, const uint8_t *__restrict__ mHh,
                               const uint8_t *__restrict__ mGateIn, const uint8_t *__restrict__ mGateOut,
-                              const uint8_t *__restrict__ mH, size_t rows, int H, uint16_t *__restrict__ out) {
-    const size_t total = rows * H;
+                              const uint8_t *__restrict__ mH, const uint16_t *__restrict__ given, size_t rows, int H, int width,
+                              uint16_t *__restrict__ out) {
+    const size_t total = rows * width;
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const size_t row = i / H, j = i % H, gi = row * 3 * H + j;
+        const size_t row = i / width, j = i - row * width, at = row * H + j, gi = row * 3 * H + j;
         auto bit = [](const uint8_t *m, size_t at, int pos) -> uint32_t { return (m ? (m[at] ? 1u : 0u) : 1u) << pos; };
-        out[i] = static_cast<uint16_t>(
+        if (j >= static_cast<size_t>(H)) out[i] = 0x1fff;
+        else if (given != nullptr) out[i] = given[at];
+        else out[i] = static_cast<uint16_t>(
             bit(mGateOut, gi, 0) | bit(mGateOut, gi + H, 1) | bit(mGateOut, gi + 2 * H, 2) | bit(mGateIn, gi, 3) |
             bit(mGateIn, gi + H, 4) | bit(mGateIn, gi + 2 * H, 5) | bit(mHh, gi, 6) | bit(mHh, gi + H, 7) |
-            bit(mHh, gi + 2 * H, 8) | bit(mIh, gi, 9) | bit(mIh, gi + H, 10) | bit(mIh, gi + 2 * H, 11) | bit(mH, i, 12));
+            bit(mHh, gi + 2 * H, 8) | bit(mIh, gi, 9) | bit(mIh, gi + H, 10) | bit(mIh, gi + 2 * H, 11) | bit(mH, at, 12));
     }
 }
 
@@ -1049,7 +1054,115 @@ void launchPair(const Problem &a, const Plan &planA, const Problem &b, const Pla
 
 namespace gru {
 
-size_t backwardWorkspaceBytes(int T, int B, int I, int H) {
+namespace {
+
+// Widths the tensor-core kernels tile: units in tiles of 64 make 3H a multiple of 192, inputs in groups of eight.
+int tiledHidden(int H) { return (H + 63) / 64 * 64; }
+int tiledInput(int I) { return I % 4 == 0 ? I : (I + 7) / 8 * 8; }
+
+struct PaddedOperands {
+    int32_t *W, *R, *x;
+    float *scales, *dh, *h, *v, *dW, *dR, *dbw, *dbr, *dh0;
+    uint16_t *bits;
+};
+template <class W>
+PaddedOperands layoutPadded(W &ws, int T, int B, int I, int H) {
+    const size_t rows = static_cast<size_t>(T) * B, Hp = tiledHidden(H), Ip = tiledInput(I), C = 3 * Hp;
+    PaddedOperands o{};
+    o.W = ws.template take<int32_t>(Ip * C);
+    o.R = ws.template take<int32_t>(Hp * C);
+    o.x = ws.template take<int32_t>(rows * Ip);
+    o.scales = ws.template take<float>(2 * C);
+    o.dh = ws.template take<float>((rows + B) * Hp);
+    o.h = ws.template take<float>((rows + B) * Hp);
+    o.v = ws.template take<float>(rows * 4 * Hp);
+    o.dW = ws.template take<float>(Ip * C);
+    o.dR = ws.template take<float>(Hp * C);
+    o.dbw = ws.template take<float>(C);
+    o.dbr = ws.template take<float>(C);
+    o.dh0 = ws.template take<float>(B * Hp);
+    o.bits = ws.template take<uint16_t>(rows * Hp);
+    return o;
+}
+struct PaddedSizer {
+    WorkspaceSizer ws;
+    template <class T>
+    T *take(size_t n) {
+        ws.take<T>(n);
+        return nullptr;
+    }
+};
+
+// Widths that no tile divides (H not a multiple of 64, I not of 4) used to fall back to SIMT kernels: T = 100, B = 300, H = 250,
+// 16 bits: 4.0 ms backward; T = 61, B = 45, I = 29, H = 100: 190 us.  Copied to padded arrays, whose extra units have zero
+// gradients by construction, the call takes the tensor-core kernels instead: 0.57 ms and 110 us.
+bool paddedTakes(const BackwardCall &call) {
+    static const bool disabled = std::getenv("RXMET_GRU_BWD_GENERIC") != nullptr || std::getenv("RXMET_GRU_GRAD_SIMT") != nullptr ||
+                                 std::getenv("RXMET_GRU_BWD_SIMT") != nullptr;
+    if (disabled || call.W_q == nullptr || call.exec == nullptr || call.H > 256 || call.I > 512) return false;
+    if (tiledHidden(call.H) == call.H && tiledInput(call.I) == call.I) return false;
+    return call.exec->weightClass == CodeClass::I8 && call.exec->actClass != CodeClass::I32 && alignedTo(call.dx, 16) &&
+           (call.masks == nullptr || alignedTo(call.masks->x, 8));
+}
+
+void backwardPadded(const BackwardCall &call, void *workspace, size_t workspaceBytes, cudaStream_t st) {
+    const int T = call.T, B = call.B, I = call.I, H = call.H, Hp = tiledHidden(H), Ip = tiledInput(I);
+    const size_t rows = static_cast<size_t>(T) * B;
+    const rxmet_gru_masks none{};
+    const rxmet_gru_masks &mk = call.masks ? *call.masks : none;
+    Workspace ws(workspace, workspaceBytes);
+    const PaddedOperands o = layoutPadded(ws, T, B, I, H);
+    int32_t *scratch = ws.take<int32_t>(6 * static_cast<size_t>(H));
+    const int32_t *scales = channelBlockOnDevice(*call.exec, scratch, 6 * static_cast<size_t>(H), st);
+    auto copy = [](const void *src, void *dst, int srcRows, int dstRows, int groups, int srcWidth, int dstWidth, uint32_t fill = 0) {
+        RegroupJob j;
+        j.src = src; j.dst = dst; j.srcRows = srcRows; j.dstRows = dstRows;
+        j.colGroups = groups; j.srcWidth = srcWidth; j.dstWidth = dstWidth; j.fill = fill;
+        return j;
+    };
+    const int steps = static_cast<int>(rows), zpX = call.exec->gate.zp[RXMET_GRU_X];
+    BackwardCall inner = call;
+    inner.H = Hp; inner.I = Ip; inner.dxColumns = I;
+    inner.W_q = o.W; inner.R_q = o.R; inner.channelScales = o.scales;
+    inner.dh_new = o.dh; inner.h = o.h; inner.v = o.v;
+    inner.dW = o.dW; inner.dR = o.dR; inner.dbw = o.dbw; inner.dbr = o.dbr; inner.dh0 = o.dh0;
+    const bool copyX = Ip != I || !alignedTo(call.x_q, 16);
+    if (copyX) inner.x_q = o.x;
+    const RegroupJob in[] = {
+        copy(call.v, o.v, steps, steps, 4, H, Hp),
+        copy(call.h, o.h, steps + B, steps + B, 1, H, Hp),
+        copy(call.dh_new, o.dh, steps + B, steps + B, 1, H, Hp),
+        copy(call.x_q, copyX ? o.x : nullptr, steps, steps, 1, I, Ip, static_cast<uint32_t>(zpX)),
+        copy(call.W_q, o.W, I, Ip, 3, H, Hp),
+        copy(call.R_q, o.R, H, Hp, 3, H, Hp),
+        copy(scales, o.scales, 2, 2, 3, H, Hp),
+    };
+    regroup("padBackward", in, 7, st);
+    rxmet_gru_masks innerMasks{};
+    innerMasks.x = mk.x;
+    inner.masks = &innerMasks;
+    inner.stepFlags = nullptr;
+    if (call.stepFlags || mk.weight_ih_linear || mk.weight_hh_linear || mk.gate_input || mk.gate_output || mk.h) {
+        {
+            KernelTimer timer__("packStepMasks", st);
+            packStepMasks<<<gridFor(rows * Hp, 256), 256, 0, st>>>(mk.weight_ih_linear, mk.weight_hh_linear, mk.gate_input, mk.gate_output,
+                                                                   mk.h, call.stepFlags, rows, H, Hp, o.bits);
+        }
+        afterLaunch("packStepMasks");
+        inner.stepFlags = o.bits;
+    }
+    const size_t used = alignUp(ws.used(), 256);
+    backward(inner, static_cast<char *>(workspace) + used, workspaceBytes - std::min(workspaceBytes, used), st);
+    RegroupJob out[] = {
+        copy(o.dW, call.dW, I, I, 3, Hp, H), copy(o.dR, call.dR, H, H, 3, Hp, H), copy(o.dbw, call.dbw, 1, 1, 3, Hp, H),
+        copy(o.dbr, call.dbr, 1, 1, 3, Hp, H), copy(o.dh0, call.dh0, B, B, 1, Hp, H),
+    };
+    const uint8_t *masks[] = {mk.W, mk.R, mk.bw, mk.br, mk.h0};
+    for (int k = 0; k < 5; ++k) out[k].mask = masks[k];
+    regroup("padBackward", out, 5, st);
+}
+
+size_t tiledWorkspaceBytes(int T, int B, int I, int H) {
     const size_t rows = static_cast<size_t>(T) * B, C = 3 * static_cast<size_t>(H);
     WorkspaceSizer ws;
     ws.take<float>(rows * C);          // dp
@@ -1078,7 +1191,21 @@ size_t backwardWorkspaceBytes(int T, int B, int I, int H) {
     return ws.used() + 4096;
 }
 
+}  // namespace
+
+size_t backwardWorkspaceBytes(int T, int B, int I, int H) {
+    size_t bytes = tiledWorkspaceBytes(T, B, I, H);
+    if (H <= 256 && (tiledHidden(H) != H || tiledInput(I) != I)) {
+        PaddedSizer sizer;
+        layoutPadded(sizer, T, B, I, H);
+        sizer.take<int32_t>(6 * static_cast<size_t>(H));
+        bytes = std::max(bytes, sizer.ws.used() + 512 + tiledWorkspaceBytes(T, B, tiledInput(I), tiledHidden(H)));
+    }
+    return bytes;
+}
+
 void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, cudaStream_t st) {
+    if (paddedTakes(call)) return backwardPadded(call, workspace, workspaceBytes, st);
     const int T = call.T, B = call.B, I = call.I, H = call.H, C = 3 * H;
     const size_t rows = static_cast<size_t>(T) * B;
     Workspace ws(workspace, workspaceBytes);
@@ -1123,7 +1250,9 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         float *xf = ws.take<float>(rows * I);
         // effective scales of W then R: the first two arrays of the per-channel block
         const size_t chanWords = 2 * static_cast<size_t>(C);
-        const float *chan = reinterpret_cast<const float *>(channelBlockOnDevice(e, ws.take<int32_t>(chanWords), chanWords, st));
+        int32_t *chanScratch = ws.take<int32_t>(chanWords);
+        const float *chan = call.channelScales ? call.channelScales
+                                               : reinterpret_cast<const float *>(channelBlockOnDevice(e, chanScratch, chanWords, st));
         if (!tensorInputGrad) {
             KernelTimer timer__("dequantCodes", st);
             dequantCodes<<<gridFor(static_cast<size_t>(I) * C, 256), 256, 0, st>>>(call.W_q, static_cast<size_t>(I) * C, C, chan, 0.f, 0, Wf);
@@ -1171,7 +1300,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
                                                                               reinterpret_cast<uint2 *>(bits));
                 else
                     packStepMasks<<<gridFor(rows * H, 256), 256, 0, st>>>(mk.weight_ih_linear, mk.weight_hh_linear,
-                                                                          mk.gate_input, mk.gate_output, mk.h, rows, H, bits);
+                                                                          mk.gate_input, mk.gate_output, mk.h, nullptr, rows, H, H, bits);
             }
             afterLaunch("packStepMasks");
             q.stepBits = bits;
@@ -1225,7 +1354,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
                                                                               reinterpret_cast<uint2 *>(bits));
                 else
                     packStepMasks<<<gridFor(rows * H, 256), 256, 0, st>>>(mk.weight_ih_linear, mk.weight_hh_linear,
-                                                                          mk.gate_input, mk.gate_output, mk.h, rows, H, bits);
+                                                                          mk.gate_input, mk.gate_output, mk.h, nullptr, rows, H, H, bits);
             }
             afterLaunch("packStepMasks");
             q.stepBits = bits;
@@ -1381,9 +1510,9 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
     if (tensorInputGrad) {
         // QAT: gradients times the integer weight codes on the tensor cores, scales folded into the gradients
         igrad::Problem pg{};
-        pg.G = dp; pg.kScale = chanScaleW; pg.codesNK = call.W_q; pg.rows = static_cast<int>(rows); pg.K = C; pg.N = I;
+        pg.G = dp; pg.kScale = chanScaleW; pg.codesNK = call.W_q; pg.rows = static_cast<int>(rows); pg.K = C; pg.N = call.dxColumns ? call.dxColumns : I;
         pg.mask = mk.x; pg.maskKeeps = 1; pg.out = call.dx; pg.status = status;
-        if (const size_t bytes = igrad::widePackedBytes(C, I)) pg.packed = ws.take<uint8_t>(bytes);
+        if (const size_t bytes = igrad::widePackedBytes(C, pg.N)) pg.packed = ws.take<uint8_t>(bytes);
         igrad::launch(pg, sms, st);
         afterLaunch("inputGradUmma");
     } else {

@@ -22,6 +22,9 @@ struct BackwardCall {
     const float *dh_new = nullptr, *h = nullptr, *v = nullptr;
     const rxmet_gru_masks *masks = nullptr;
     const uint16_t *stepFlags = nullptr;    // optional [T,B,H]: packed per-step keep flags as the forward wrote them
+    // a call on padded widths (backwardPadded): scales of W then R [2][3H] on the device, columns of dx
+    const float *channelScales = nullptr;
+    int dxColumns = 0;                      // 0 = I
     float *dx = nullptr, *dW = nullptr, *dR = nullptr, *dbw = nullptr, *dbr = nullptr, *dh0 = nullptr;
 };
 

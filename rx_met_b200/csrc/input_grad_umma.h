@@ -36,7 +36,7 @@ struct Problem {
 // Resident-weight kernel: K a multiple of 64 up to 768; any N: more than 64 columns (32 when K > 512, where the
 // weight operand of a wider slab no longer fits shared memory) run as column slabs that share one launch.
 // Streaming kernel (Problem::packed given, N <= 512): any K that is a multiple of 32; up to 64 columns only where the other does
-// not take K (H = 256, I = 40, 10,000 rows: inputGradNarrow 132 us, MEASURED_IGRAD here).
+// not take K (H = 256, I = 40, 10,000 rows: inputGradNarrow 132 us, this 26 us).
 // RXMET_IGRAD_SIMT in the environment turns both off, RXMET_IGRAD_NARROW the streaming kernel.
 bool eligible(int K, int N);
 size_t widePackedBytes(int K, int N);   // 0 when the streaming kernel does not take N

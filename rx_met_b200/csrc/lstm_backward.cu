@@ -17,11 +17,13 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
+#include <cstring>
 
 #include "common.h"
 #include "input_grad_umma.h"
 #include "lstm_backward_cluster.h"
 #include "lstm_kernels.h"
+#include "regroup.h"
 #include "umma_device.cuh"
 #include "weight_grad_mma.h"
 
@@ -44,13 +46,18 @@ __global__ void dequantWeights(const float *__restrict__ codes, const float *__r
 // One word of keep/drop flags per (t, b, j): bit 0 hidden, 1 tanh(cell), 2 cell, 3-6 gate outputs,
 // 7-10 gate inputs, 11-14 ih linear, 15-18 hh linear (a set bit = clamped = no gradient).  Packing them
 // once in a bandwidth-bound pass takes 19 byte loads per element off every step of the recurrence.
-__global__ void packStepMasks(const rxmet_lstm_backward_masks mk, size_t rows, int H, uint32_t *__restrict__ out) {
-    const size_t n = rows * H;
+// `width` >= H: words per row of out, the ones beyond H keep everything.
+__global__ void packStepMasks(const rxmet_lstm_backward_masks mk, size_t rows, int H, int width, uint32_t *__restrict__ out) {
+    const size_t n = rows * width;
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const size_t row = i / H, j = i % H, go = row * 4 * H + j;
+        const size_t row = i / width, j = i - row * width, at = row * H + j, go = row * 4 * H + j;
+        if (j >= static_cast<size_t>(H)) {
+            out[i] = 0u;
+            continue;
+        }
         auto bit = [](const uint8_t *m, size_t idx) -> uint32_t { return (m != nullptr && m[idx] != 0) ? 1u : 0u; };
-        uint32_t w = bit(mk.hidden_outputs, i) | (bit(mk.cell_tanh_outputs, i) << 1) | (bit(mk.cell_states, i) << 2);
+        uint32_t w = bit(mk.hidden_outputs, at) | (bit(mk.cell_tanh_outputs, at) << 1) | (bit(mk.cell_states, at) << 2);
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
             const size_t o = go + static_cast<size_t>(g) * H;
@@ -933,7 +940,121 @@ int tensorSplitBound(int rows, int I, int H, int M, int C) {
     return std::max(single, wgrad::slabPathTakes(I, H, C) ? wgrad::slabSplitBound(I, H, C) : 1);
 }
 
-size_t backwardWorkspaceBytes(int T, int B, int I, int H) {
+namespace {
+
+// Widths the tensor-core kernels tile: units in tiles of 32, inputs in groups of eight.
+int tiledHidden(int H) { return (H + 31) / 32 * 32; }
+int tiledInput(int I) { return I % 4 == 0 ? I : (I + 7) / 8 * 8; }
+
+struct PaddedOperands {
+    float *wIh, *wHh, *scales, *x, *h0, *c0, *gates, *cells, *tanhs, *hiddens, *gradOut, *gradHidden, *gradCell;
+    float *dWIh, *dWHh, *dBIh, *dBHh, *dh0, *dc0;
+    uint32_t *flags;
+};
+template <class W>
+PaddedOperands layoutPadded(W &ws, int T, int B, int I, int H) {
+    const size_t rows = static_cast<size_t>(T) * B, Hp = tiledHidden(H), Ip = tiledInput(I), C = 4 * Hp, state = static_cast<size_t>(B) * Hp;
+    PaddedOperands o{};
+    o.wIh = ws.template take<float>(C * I); o.wHh = ws.template take<float>(C * Hp); o.scales = ws.template take<float>(2 * C);
+    o.x = ws.template take<float>(rows * Ip);
+    o.h0 = ws.template take<float>(state); o.c0 = ws.template take<float>(state);
+    o.gates = ws.template take<float>(rows * C); o.cells = ws.template take<float>(rows * Hp); o.tanhs = ws.template take<float>(rows * Hp);
+    o.hiddens = ws.template take<float>(rows * Hp); o.gradOut = ws.template take<float>(rows * Hp);
+    o.gradHidden = ws.template take<float>(state); o.gradCell = ws.template take<float>(state);
+    o.dWIh = ws.template take<float>(C * Ip); o.dWHh = ws.template take<float>(C * Hp);
+    o.dBIh = ws.template take<float>(C); o.dBHh = ws.template take<float>(C);
+    o.dh0 = ws.template take<float>(state); o.dc0 = ws.template take<float>(state);
+    o.flags = ws.template take<uint32_t>(rows * Hp);
+    return o;
+}
+struct PaddedSizer {
+    WorkspaceSizer ws;
+    template <class T>
+    T *take(size_t n) {
+        ws.take<T>(n);
+        return nullptr;
+    }
+};
+
+// As backwardPadded of the GRU (gru_backward.cu): widths that no tile divides go through padded copies to the tensor-core
+// kernels; the extra units have zero gradients.  T = 100, B = 100, I = 37, H = 150, 16 bits: the step 1893 -> 630 us.
+bool paddedTakes(const BackwardCall &call) {
+    static const bool disabled = std::getenv("RXMET_LSTM_BWD_SIMT") != nullptr || std::getenv("RXMET_LSTM_WGRAD_SIMT") != nullptr;
+    if (disabled || !call.quantized || call.H > 256 || call.I > 512 || !call.weightCodesFitBf16 || !call.weightIhCodesFitBf16 ||
+        !call.codesFitTwoTerms || call.h0 == nullptr || call.c0 == nullptr)
+        return false;
+    if (tiledHidden(call.H) == call.H && tiledInput(call.I) == call.I) return false;
+    return alignedTo(call.grads.input, 16) && (call.masks == nullptr || alignedTo(call.masks->input, 8));
+}
+
+void backwardPadded(const BackwardCall &call, void *workspace, size_t workspaceBytes, cudaStream_t st) {
+    const int T = call.T, B = call.B, I = call.I, H = call.H, Hp = tiledHidden(H), Ip = tiledInput(I);
+    const size_t rows = static_cast<size_t>(T) * B;
+    const int steps = static_cast<int>(rows);
+    const rxmet_lstm_backward_masks none{};
+    const rxmet_lstm_backward_masks &mk = call.masks ? *call.masks : none;
+    Workspace ws(workspace, workspaceBytes);
+    const PaddedOperands o = layoutPadded(ws, T, B, I, H);
+    auto copy = [](const void *src, void *dst, int rowGroups, int srcRows, int dstRows, int colGroups, int srcWidth, int dstWidth, float fill = 0.0f) {
+        RegroupJob j;
+        j.src = src; j.dst = dst; j.rowGroups = rowGroups; j.srcRows = srcRows; j.dstRows = dstRows;
+        j.colGroups = colGroups; j.srcWidth = srcWidth; j.dstWidth = dstWidth;
+        std::memcpy(&j.fill, &fill, sizeof(fill));
+        return j;
+    };
+    BackwardCall inner = call;
+    inner.H = Hp; inner.I = Ip; inner.dxColumns = I;
+    inner.weightIh = o.wIh; inner.weightHh = o.wHh; inner.channelScales = o.scales; inner.x = o.x; inner.h0 = o.h0; inner.c0 = o.c0;
+    inner.gateOutputs = o.gates; inner.cellStates = o.cells; inner.cellTanhOutputs = o.tanhs; inner.hiddenOutputs = o.hiddens;
+    inner.gradOutput = o.gradOut; inner.gradFinalHidden = o.gradHidden; inner.gradFinalCell = o.gradCell;
+    inner.grads.weight_ih = o.dWIh; inner.grads.weight_hh = o.dWHh; inner.grads.bias_ih = o.dBIh; inner.grads.bias_hh = o.dBHh;
+    inner.grads.initial_hidden = o.dh0; inner.grads.initial_cell = o.dc0;
+    const float zeroH = call.dqH.zeroPoint;   // codes of padded inputs and units: real zero
+    const bool copyX = Ip != I || !alignedTo(call.x, 16);
+    if (!copyX) inner.x = call.x;
+    const RegroupJob in[] = {
+        copy(call.gateOutputs, o.gates, 1, steps, steps, 4, H, Hp),
+        copy(call.cellStates, o.cells, 1, steps, steps, 1, H, Hp),
+        copy(call.cellTanhOutputs, o.tanhs, 1, steps, steps, 1, H, Hp),
+        copy(call.hiddenOutputs, o.hiddens, 1, steps, steps, 1, H, Hp, zeroH),
+        copy(call.gradOutput, o.gradOut, 1, steps, steps, 1, H, Hp),
+        copy(call.x, copyX ? o.x : nullptr, 1, steps, steps, 1, I, Ip, call.dqX.zeroPoint),
+        copy(call.gradFinalHidden, o.gradHidden, 1, B, B, 1, H, Hp),
+        copy(call.gradFinalCell, o.gradCell, 1, B, B, 1, H, Hp),
+        copy(call.h0, o.h0, 1, B, B, 1, H, Hp, zeroH),
+        copy(call.c0, o.c0, 1, B, B, 1, H, Hp),
+        copy(call.weightIh, o.wIh, 4, H, Hp, 1, I, I),
+        copy(call.weightHh, o.wHh, 4, H, Hp, 1, H, Hp),
+        copy(call.channelScales, o.scales, 1, 2, 2, 4, H, Hp),
+    };
+    regroup("lstmPadBackward", in, 13, st);
+    rxmet_lstm_backward_masks innerMasks{};
+    innerMasks.input = mk.input;
+    inner.masks = &innerMasks;
+    if (mk.hidden_outputs || mk.cell_tanh_outputs || mk.cell_states || mk.gate_outputs || mk.gate_inputs || mk.weight_ih_linear || mk.weight_hh_linear) {
+        {
+            KernelTimer timer__("lstmPackStepMasks", st);
+            packStepMasks<<<gridFor(rows * Hp, 256), 256, 0, st>>>(mk, rows, H, Hp, o.flags);
+        }
+        afterLaunch("lstmPackStepMasks");
+        inner.stepMasks = o.flags;
+    }
+    const size_t used = alignUp(ws.used(), 256);
+    backward(inner, static_cast<char *>(workspace) + used, workspaceBytes - std::min(workspaceBytes, used), st);
+    RegroupJob out[] = {
+        copy(o.dWIh, call.grads.weight_ih, 4, Hp, H, 1, Ip, I), copy(o.dWHh, call.grads.weight_hh, 4, Hp, H, 1, Hp, H),
+        copy(o.dBIh, call.grads.bias_ih, 1, 1, 1, 4, Hp, H), copy(o.dBHh, call.grads.bias_hh, 1, 1, 1, 4, Hp, H),
+        copy(o.dh0, call.grads.initial_hidden, 1, B, B, 1, Hp, H), copy(o.dc0, call.grads.initial_cell, 1, B, B, 1, Hp, H),
+    };
+    const void *masks[] = {mk.weight_ih, mk.weight_hh, mk.bias_ih, mk.bias_hh, mk.initial_hidden, mk.initial_cell};
+    for (int k = 0; k < 6; ++k) {
+        out[k].mask = static_cast<const uint8_t *>(masks[k]);
+        out[k].maskKeeps = 0;
+    }
+    regroup("lstmPadBackward", out, 6, st);
+}
+
+size_t tiledWorkspaceBytes(int T, int B, int I, int H) {
     const size_t rows = static_cast<size_t>(T) * B, C = 4 * static_cast<size_t>(H);
     WorkspaceSizer ws;
     ws.take<float>(rows * C);  // G_ih
@@ -957,7 +1078,20 @@ size_t backwardWorkspaceBytes(int T, int B, int I, int H) {
     return ws.used() + 1024;
 }
 
+}  // namespace
+
+size_t backwardWorkspaceBytes(int T, int B, int I, int H) {
+    size_t bytes = tiledWorkspaceBytes(T, B, I, H);
+    if (H <= 256 && (tiledHidden(H) != H || tiledInput(I) != I)) {
+        PaddedSizer sizer;
+        layoutPadded(sizer, T, B, I, H);
+        bytes = std::max(bytes, sizer.ws.used() + 512 + tiledWorkspaceBytes(T, B, tiledInput(I), tiledHidden(H)));
+    }
+    return bytes;
+}
+
 void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, cudaStream_t st) {
+    if (paddedTakes(call)) return backwardPadded(call, workspace, workspaceBytes, st);
     const int T = call.T, B = call.B, I = call.I, H = call.H, C = 4 * H;
     if (H > 512) fail(RXMET_ERR_UNSUPPORTED, "hidden sizes up to 512 are built (got %d)", H);
     const bool wide = C > 512;
@@ -988,7 +1122,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
     const bool codes = call.quantized && call.weightCodesFitBf16 && std::getenv("RXMET_LSTM_BWD_SIMT") == nullptr;
     BackwardClusterArgs cl{};
     cl.T = T; cl.B = B; cl.H = H;
-    cl.stepMasks = anyStepMask ? stepMasks : nullptr;
+    cl.stepMasks = call.stepMasks ? call.stepMasks : anyStepMask ? stepMasks : nullptr;
     cl.weightCodes = call.weightHh; cl.channelScale = channelScales ? channelScales + C : nullptr; cl.c0 = call.c0;
     cl.gateOutputs = call.gateOutputs; cl.cellStates = call.cellStates; cl.cellTanh = call.cellTanhOutputs;
     cl.gradOutput = call.gradOutput; cl.gradFinalHidden = call.gradFinalHidden; cl.gradFinalCell = call.gradFinalCell;
@@ -1043,14 +1177,14 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
                 aligned4(mk.weight_hh_linear))
                 packStepMasks4<<<gridFor(rows * H / 4, 256), 256, 0, st>>>(mk, rows * H / 4, H, reinterpret_cast<uint4 *>(stepMasks));
             else
-                packStepMasks<<<gridFor(rows * H, 256), 256, 0, st>>>(mk, rows, H, stepMasks);
+                packStepMasks<<<gridFor(rows * H, 256), 256, 0, st>>>(mk, rows, H, H, stepMasks);
         }
         afterLaunch("lstmPackStepMasks");
     }
     {
         RecurrentArgs a{};
         a.T = T; a.B = B; a.H = H;
-        a.stepMasks = anyStepMask ? stepMasks : nullptr;
+        a.stepMasks = cl.stepMasks;
         a.weightHh = wHh; a.c0 = call.c0;
         a.gateOutputs = call.gateOutputs; a.cellStates = call.cellStates; a.cellTanh = call.cellTanhOutputs;
         a.gradOutput = call.gradOutput; a.gradFinalHidden = call.gradFinalHidden; a.gradFinalCell = call.gradFinalCell;
@@ -1147,9 +1281,9 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         // QAT: gradients times the integer weight codes on the tensor cores, scales folded into the gradients
         const int sms = currentDevice().sms;
         igrad::Problem pg{};
-        pg.G = gIh; pg.kScale = channelScales; pg.codesKN = call.weightIh; pg.rows = static_cast<int>(rows); pg.K = C; pg.N = I;
+        pg.G = gIh; pg.kScale = channelScales; pg.codesKN = call.weightIh; pg.rows = static_cast<int>(rows); pg.K = C; pg.N = call.dxColumns ? call.dxColumns : I;
         pg.mask = static_cast<const uint8_t *>(mk.input); pg.maskKeeps = 0; pg.out = call.grads.input; pg.status = tensorStatus;
-        if (const size_t bytes = igrad::widePackedBytes(C, I)) pg.packed = ws.take<uint8_t>(bytes);
+        if (const size_t bytes = igrad::widePackedBytes(C, pg.N)) pg.packed = ws.take<uint8_t>(bytes);
         igrad::launch(pg, sms, st);
         afterLaunch("inputGradUmma");
     } else if (I <= 128 && C % 4 == 0) {

@@ -68,6 +68,8 @@ struct BackwardCall {
     bool quantized = false;
     Dequant dqX, dqH, dqC, dqGate[4], dqTanh;
     const float *channelScales = nullptr;   // device: weight_ih, then weight_hh
+    int dxColumns = 0;                // a call on padded widths: columns of grads.input (0 = I)
+    const uint32_t *stepMasks = nullptr;   // ... and the clamp flags of its steps, packed already (else from `masks`)
     bool codesFitTensorPath = false;  // x and hidden grids span at most 256 codes around their zero points
     bool codesFitTwoTerms = false;    // x and hidden grids of at most 16 bits: a code is two exact bf16 terms
     bool weightCodesFitBf16 = false;  // weight_hh grid of at most 8 bits: codes are exact in bf16

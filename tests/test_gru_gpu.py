@@ -671,3 +671,11 @@ def test_forward_quant_lanes_of_a_unit(gl, shape):
             order = ("x", "h0", "W", "R", "bw", "br", "weight_ih_linear", "weight_hh_linear", "gate_input", "gate_output", "h")
             assert cabi.MASK_NAMES == order
             assert flags.size == 0 if not training else np.array_equal(flags, want["masks"].arr[name]), name
+
+
+@pytest.mark.parametrize("cfg_name", ["w8a8", "a16"])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 3, 5, 63), (3, 2, 29, 65), (2, 17, 40, 127), (3, 4, 6, 129), (2, 5, 33, 255)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_backward_quant_on_padded_widths(gl, cfg_name, shape):
+    """Widths one beside those the tensor-core kernels tile: the call goes through padded copies."""
+    test_backward_quant(gl, cfg_name, shape)
