@@ -16,6 +16,7 @@
 #include "common.h"
 #include "gru_device.cuh"
 #include "gru_forward_wide.h"
+#include "lane_recurrence.cuh"
 #include "plane_recurrence_umma.cuh"
 
 namespace rxmet {
@@ -25,33 +26,34 @@ namespace {
 constexpr int kBuckets = 256;
 
 struct FastLut {
-    int4 segment[kSegments];          // q_b, n_bx, term_c, 2^(n_bx - 1) - 1
+    int4 segment[kSegments];          // q_b, n_bx, term_c, 2^(n_bx - 1)
     uint2 bucket[kBuckets];           // the bucket's threshold; byte offset of the segment before it | of the one behind it << 16
 };
 static_assert(sizeof(int4) * kSegments == 256, "activation() addresses the buckets behind the segments");
 
-// round_half_even(p / 2^n) for 1 <= n <= 31, low 32 bits: (p + 2^(n-1) - 1 + odd(floor(p / 2^n))) >> n on two words.
-__device__ __forceinline__ int32_t roundShift31(int64_t p, int n, uint32_t roundAdd) {
-    const uint32_t odd = __funnelshift_r(static_cast<uint32_t>(p), static_cast<uint32_t>(static_cast<uint64_t>(p) >> 32), n) & 1u;
-    const uint64_t sum = static_cast<uint64_t>(p) + (roundAdd + odd);
-    return static_cast<int32_t>(__funnelshift_r(static_cast<uint32_t>(sum), static_cast<uint32_t>(sum >> 32), n));
+// round_half_even(p / 2^n) for 1 <= n <= 31, low 32 bits, of sum = p + 2^(n-1): the floor is right except for an exact tie,
+// where it is the upper neighbour and an odd one must step down.  mask = 2^n - 1.
+__device__ __forceinline__ int32_t roundShift31(int64_t sum, int n, uint32_t mask) {
+    const uint32_t low = static_cast<uint32_t>(sum), high = static_cast<uint32_t>(static_cast<uint64_t>(sum) >> 32);
+    const int32_t q = static_cast<int32_t>(__funnelshift_r(low, high, n));
+    return (low & mask) == 0 ? q & ~1 : q;
 }
 
 // Rounding rescale of a 32-bit operand, shift in [1, 31], and of a product of two, shift in [1, 62].
 struct ReadyRescale {
     int32_t mult, shift;
-    uint32_t roundAdd;
+    uint32_t half, mask;   // 2^(shift - 1), 2^shift - 1
 };
 struct ReadyWide {
     int32_t mult, shift;
-    int64_t roundAdd;
+    int64_t roundAdd;      // 2^(shift - 1) - 1
 };
 __device__ __forceinline__ int32_t apply(int32_t x, const ReadyRescale &r) {
-    return roundShift31(static_cast<int64_t>(x) * r.mult, r.shift, r.roundAdd);
+    return roundShift31(static_cast<int64_t>(x) * r.mult + r.half, r.shift, r.mask);
 }
 __device__ __forceinline__ int32_t apply(int64_t x, const ReadyWide &r) {
     const int64_t p = x * r.mult;
-    if (r.shift <= 31) return roundShift31(p, r.shift, static_cast<uint32_t>(r.roundAdd));
+    if (r.shift <= 31) return roundShift31(p + r.roundAdd + 1, r.shift, 2u * static_cast<uint32_t>(r.roundAdd) + 1u);
     return static_cast<int32_t>(rshiftRoundConst(p, r.shift, r.roundAdd));
 }
 
@@ -93,8 +95,9 @@ struct GruPlaneCell {
 
     size_t sharedBytes() const { return sizeof(luts); }
     struct Lane {
-        int64_t addend, roundAdd;
+        int64_t addend, roundAdd;   // narrow: (sum + addend) mult + 2^(shift - 1) = sum mult + addend
         int32_t mult, shift;
+        uint32_t mask;
         bool narrow;   // warp-uniform: the shifts of all lanes lie in [1, 31]
     };
     struct State {
@@ -118,7 +121,7 @@ struct GruPlaneCell {
     }
     __device__ __forceinline__ Lane lane(uint32_t, int gate, int unit, bool real) const {
         const int H = hidden();
-        Lane l{0, 0, 0, 1, false};
+        Lane l{0, 0, 0, 1, 1u, false};
         if (gate < 3 && real) {
             const Rescale r = rescale[gate * H + unit];
             l.addend = addend[gate * H + unit];
@@ -127,6 +130,10 @@ struct GruPlaneCell {
         }
         l.roundAdd = l.shift >= 1 ? (int64_t{1} << (l.shift - 1)) - 1 : 0;
         l.narrow = __all_sync(0xffffffffu, l.shift >= 1 && l.shift <= 31);
+        if (l.narrow) {
+            l.addend = l.addend * l.mult + (int64_t{1} << (l.shift - 1));
+            l.mask = (1u << l.shift) - 1u;
+        }
         return l;
     }
     __device__ __forceinline__ float scaleH(bool alive) const {
@@ -154,10 +161,10 @@ struct GruPlaneCell {
     // hh linear code, its keep flag in bit 0
     template <int STRIDE>
     __device__ __forceinline__ uint32_t linear(uint32_t, const Lane &l, const Fetch &, const uint32_t *acc, Saved &) const {
-        const int64_t total = (static_cast<int64_t>(static_cast<int32_t>(acc[0])) << 8) + static_cast<int32_t>(acc[STRIDE]) + l.addend;
-        const int64_t prod = total * l.mult;
+        const int64_t sum = (static_cast<int64_t>(static_cast<int32_t>(acc[0])) << 8) + static_cast<int32_t>(acc[STRIDE]);
+        const int64_t prod = (sum + l.addend) * l.mult;
         int32_t res;
-        if (l.narrow) res = roundShift31(prod, l.shift, static_cast<uint32_t>(l.roundAdd));
+        if (l.narrow) res = roundShift31(sum * l.mult + l.addend, l.shift, l.mask);
         else res = l.shift >= 1 ? static_cast<int32_t>(rshiftRoundConst(prod, l.shift, l.roundAdd)) : static_cast<int32_t>(prod << -l.shift);
         uint8_t keep;
         const int32_t code = clampCode(res + s.zpHh, s.loHh, s.hiHh, keep);
@@ -174,8 +181,8 @@ struct GruPlaneCell {
         asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
             : "=r"(e.x), "=r"(e.y), "=r"(e.z), "=r"(e.w)
             : "r"(lut + (qx < threshold ? segments & 0xffffu : segments >> 16)));
-        const int64_t bx = static_cast<int64_t>(e.x) * (qx - s.zpX[g]);
-        const int32_t y = roundShift31(bx, e.y, static_cast<uint32_t>(e.w)) + e.z;
+        const int64_t sum = static_cast<int64_t>(e.x) * (qx - s.zpX[g]) + static_cast<uint32_t>(e.w);
+        const int32_t y = roundShift31(sum, e.y, 2u * static_cast<uint32_t>(e.w) - 1u) + e.z;
         uint8_t keep;
         const int32_t code = clampCode(y, s.loOut[g], s.hiOut[g], keep);
         keepOut |= static_cast<uint32_t>(keep) << g;
@@ -254,7 +261,7 @@ struct GruPlaneCell {
 
 bool ready(const Rescale &r, ReadyRescale &out) {
     if (r.shift < 1 || r.shift > 31) return false;
-    out = ReadyRescale{r.mult, r.shift, (1u << (r.shift - 1)) - 1u};
+    out = ReadyRescale{r.mult, r.shift, 1u << (r.shift - 1), (1u << r.shift) - 1u};
     return true;
 }
 bool ready(const Rescale &r, ReadyWide &out) {
@@ -275,7 +282,7 @@ bool ready(const Lut &lut, int32_t lo, int32_t hi, FastLut &out, int32_t &bucket
     };
     for (int i = 0; i < kSegments; ++i) {
         if (lut.n_bx[i] < 1 || lut.n_bx[i] > 31) return false;
-        out.segment[i] = make_int4(lut.q_b[i], lut.n_bx[i], lut.term_c[i], (1 << (lut.n_bx[i] - 1)) - 1);
+        out.segment[i] = make_int4(lut.q_b[i], lut.n_bx[i], lut.term_c[i], static_cast<int>(1u << (lut.n_bx[i] - 1)));
     }
     for (int b = 0; b < kBuckets; ++b) {
         const int64_t first = lo + (static_cast<int64_t>(b) << bucketShift), last = std::min<int64_t>(first + (int64_t{1} << bucketShift) - 1, hi);
@@ -312,6 +319,8 @@ void launchFor(const WideRecurrence &r, const Prepared &prepared, cudaStream_t s
     cell.maskIh = r.maskIh; cell.stepBits = r.stepBits;
     cell.poison = r.poison;
     const planerec::Problem problem{r.T, r.B, r.H, r.h0Planes};
+    if constexpr (HP == 64 || HP == 128)
+        if (lanerec::launch<Cell, HP / 4>("recurrentForward", problem, cell, st)) return;
     if constexpr (HP < 64) planerec::launchBest<Cell, HP, HP, 2, 32, 8, 16>("recurrentForward", problem, cell, st);
     else planerec::launchBest<Cell, HP, 64, 2, 32, 4, 8, 16>("recurrentForward", problem, cell, st);
 }
@@ -361,7 +370,7 @@ bool forwardWideClusterTakes(const Exec &e, int H) {
 void forwardWideCluster(const WideRecurrence &r, const Exec &e, cudaStream_t st) {
     Prepared prepared;
     prepare(e, prepared);
-    if (r.H <= 32) launchFor<32>(r, prepared, st);
+    if (r.H <= 32 && lanerec::rowsFor<16>(r.B) == 0) launchFor<32>(r, prepared, st);
     else if (r.H <= 64) launchFor<64>(r, prepared, st);
     else if (r.H <= 128) launchFor<128>(r, prepared, st);
     else if (r.H <= 192) launchFor<192>(r, prepared, st);

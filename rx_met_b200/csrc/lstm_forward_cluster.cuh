@@ -20,6 +20,7 @@
 #include "common.h"
 #include "lstm_device.cuh"
 #include "lstm_kernels.h"
+#include "lane_recurrence.cuh"
 #include "plane_recurrence_umma.cuh"
 
 namespace rxmet {
@@ -220,6 +221,8 @@ struct LstmPlaneCell {
 // Rows: a step of n rows costs about 1 + n / 5 of the chain of a one-row step.
 template <bool TRAIN, int HP>
 void launchLstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &cell, cudaStream_t st) {
+    if constexpr (HP <= 128)
+        if (lanerec::launch<LstmPlaneCell<TRAIN>, HP / 4>("lstmRecurrentWide", p, cell, st)) return;
     if (p.H == HP) {
         LstmPlaneCell<TRAIN, HP> full;
         static_assert(sizeof(full) == sizeof(cell), "the variants differ in the width only");

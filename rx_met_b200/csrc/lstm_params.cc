@@ -7,8 +7,10 @@
 #include "lstm_params.h"
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
+#include <future>
 #include <limits>
 #include <map>
 #include <mutex>
@@ -338,6 +340,16 @@ void buildTable(const rxmet_lstm_quant_params &p, int inOp, int outOp, bool isTa
     }
 }
 
+// job(table) for all tables, on threads of their own where that pays; whether all returned true.
+template <class Job>
+bool forEachTable(bool threads, Job &&job) {
+    std::array<std::future<bool>, kTables> running;
+    for (int t = 1; t < kTables; ++t) running[t] = std::async(threads ? std::launch::async : std::launch::deferred, job, t);
+    bool good = job(0);
+    for (int t = 1; t < kTables; ++t) good = running[t].get() && good;
+    return good;
+}
+
 DevRescale device(const rxmet_lstm_rescale &r) {
     return {r.is_m_shift ? static_cast<float>(r.multiplier) : 1.0f, std::ldexp(1.0f, -r.shift)};
 }
@@ -541,8 +553,11 @@ std::shared_ptr<const Exec> deriveExec(const rxmet_lstm_quant_params &p, bool re
             total += size_t{1} << p.config.bitwidth[kTableIn[t]];
         }
         e->wide.entries.assign(total, 0);
-        for (int t = 0; t < kTables; ++t)
+        // 16-bit grids: 65,536 function values a table, a thread each (five tables: 20 -> 6 ms of a new parameter set's first call)
+        forEachTable(total > 4096, [&](int t) {
             buildTable(p, kTableIn[t], kTableOut[t], t == 2 || t == 4, e->wide.entries.data() + e->wide.offset[t]);
+            return true;
+        });
     }
     e->weightsFitBytes = p.config.bitwidth[RXMET_LSTM_WEIGHT_IH] <= 8 && p.config.bitwidth[RXMET_LSTM_WEIGHT_HH] <= 8;
     const int actBits = std::max(p.config.bitwidth[RXMET_LSTM_INPUT], p.config.bitwidth[RXMET_LSTM_OUTPUT]);
@@ -603,7 +618,7 @@ bool buildCompact(const Exec &e, int segShift, CompactTables &out) {
         at = (at + 15) & ~static_cast<size_t>(15);
     }
     out.bytes.assign(at, 0);
-    for (int t = 0; t < kTables; ++t) {
+    out.ok = forEachTable(at > 4096, [&](int t) {
         const ScalarExec &s = e.scalar;
         const int in = kTableIn[t], to = kTableOut[t];
         const int entries = s.hi[in] - s.lo[in] + 1;
@@ -637,9 +652,9 @@ bool buildCompact(const Exec &e, int segShift, CompactTables &out) {
             if (table[i] & 1) return false;
         out.flagBelow[t] = below;
         out.flagFrom[t] = from;
-    }
-    out.ok = true;
-    return true;
+        return true;
+    });
+    return out.ok;
 }
 
 }  // namespace

@@ -679,3 +679,10 @@ def test_forward_quant_lanes_of_a_unit(gl, shape):
 def test_backward_quant_on_padded_widths(gl, cfg_name, shape):
     """Widths one beside those the tensor-core kernels tile: the call goes through padded copies."""
     test_backward_quant(gl, cfg_name, shape)
+
+
+@pytest.mark.parametrize("shape", [(3, 75, 8, 64), (2, 149, 5, 63), (2, 290, 8, 33), (2, 148, 9, 128), (1, 1, 3, 65)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_forward_quant_planes_in_lanes(gl, shape):
+    """16-bit grids of at most 128 units: one, two and four rows per CTA with a partly empty last CTA, odd and even step counts."""
+    test_forward_quant_matches_restatement(gl, "a16", shape)
