@@ -50,6 +50,22 @@ RXMET_API uint64_t rxmet_kernel_launch_count(void);
  * it.  No counterpart in the reference. */
 RXMET_API int rxmet_set_concurrent_passes(int passes);
 
+/* Which part of a quantized GRU forward the calls of this thread run: 0 everything, 1 all but the
+ * recurrence, 2 only the recurrence (the same arguments and workspace as the call with 1 before it).
+ * A caller with two passes side by side can let both projections finish before either recurrence
+ * takes its SMs.  Paths that are not split run everything under 0 and 1 and nothing under 2. */
+RXMET_API int rxmet_set_forward_phase(int phase);
+
+/* Outputs of the two directions of a layer -> its output and, optionally, that output in reversed time:
+ * y[t] = (forward[t], reverse[T-1-t]), y_reversed[t] = y[T-1-t].  forward, reverse: [T,B,H]; y: [T,B,2H]. */
+RXMET_API int rxmet_join_directions(int T, int B, int H, const float *forward_dev, const float *reverse_dev, float *y_dev,
+                                    float *y_reversed_dev, void *stream);
+/* Gradient of a layer's output -> gradients of its two directions: g = a + b reversed in time (b may be
+ * null), forward[t] = g[t][:H], reverse[T-1-t] = g[t][H:]; sum (optional) receives g.  a, b, sum: [T,B,2H];
+ * forward, reverse: [T,B,H]. */
+RXMET_API int rxmet_split_directions(int T, int B, int H, const float *a_dev, const float *b_dev, float *sum_dev,
+                                     float *forward_dev, float *reverse_dev, void *stream);
+
 /* Number of kernel nodes of a captured graph (a cudaGraph_t). */
 RXMET_API int rxmet_graph_kernel_nodes(void *graph, int *kernels);
 

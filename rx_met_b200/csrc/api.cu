@@ -226,6 +226,11 @@ std::atomic<int> &concurrentPassesSetting() {
     return passes;
 }
 int concurrentPasses() { return concurrentPassesSetting().load(); }
+ForwardPhase &forwardPhaseSetting() {
+    static thread_local ForwardPhase phase = ForwardPhase::All;
+    return phase;
+}
+ForwardPhase forwardPhase() { return forwardPhaseSetting(); }
 }  // namespace rxmet
 
 using namespace rxmet;
@@ -235,6 +240,13 @@ extern "C" {
 const char *rxmet_last_error(void) { return lastError().c_str(); }
 const char *rxmet_version(void) { return "rxmet_b200 0.1.0 (sm_100a)"; }
 uint64_t rxmet_kernel_launch_count(void) { return launchCounter().load(); }
+
+int rxmet_set_forward_phase(int phase) {
+    return guarded([&] {
+        RXMET_REQUIRE(phase >= 0 && phase <= 2, "forward phase %d", phase);
+        forwardPhaseSetting() = static_cast<ForwardPhase>(phase);
+    });
+}
 
 int rxmet_graph_kernel_nodes(void *graph, int *kernels) {
     return guarded([&] {

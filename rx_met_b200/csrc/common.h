@@ -101,6 +101,9 @@ struct DeviceInfo {
 const DeviceInfo &currentDevice();
 // Recurrent passes the caller runs side by side on one GPU (rxmet_set_concurrent_passes); at least 1.
 int concurrentPasses();
+// Which part of a GRU forward a call of this thread runs (rxmet_set_forward_phase).
+enum class ForwardPhase { All = 0, Projection = 1, Recurrence = 2 };
+ForwardPhase forwardPhase();
 // SMs one of those passes can count on.
 inline int smsPerPass() { return std::max(1, currentDevice().sms / concurrentPasses()); }
 // A second stream of this thread on the current device, for work the library runs beside a recurrence that

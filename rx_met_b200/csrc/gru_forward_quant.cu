@@ -327,6 +327,7 @@ struct WidePrepArgs {
         uint8_t *mask;                             // optional
         int16_t *codes;                            // optional [rows][colsPadded]
         int colsPadded;
+        int vectors;                               // src, codes32 and mask take 16- and 4-byte accesses of four columns, no codes
     } x, h0;
     int prepBlocks, xBlocks, h0Blocks;
     int *clear;                                    // status word of a later kernel, set to 0 here
@@ -337,6 +338,27 @@ __device__ __forceinline__ void planesOf(const WidePrepArgs::Rows &t, int block,
         const size_t r = i / t.kWords;
         const int kw = static_cast<int>(i - r * t.kWords);
         uint32_t high = 0, low = 0;
+        if (t.vectors && 4 * kw < t.cols) {   // whole words: one 16-byte load, one 16-byte and one 4-byte store
+            const size_t at = r * t.cols + 4 * kw;
+            const float4 v = *reinterpret_cast<const float4 *>(t.src + at);
+            const float in[4] = {v.x, v.y, v.z, v.w};
+            int32_t q[4];
+            uint32_t keeps = 0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                uint8_t keep;
+                q[e] = quantizeValue(in[e], t.scale, t.zp, t.lo, t.hi, keep);
+                keeps |= static_cast<uint32_t>(keep) << (8 * e);
+                const uint32_t u = static_cast<uint32_t>(q[e] - t.lo);
+                low |= (u & 0xffu) << (8 * e);
+                high |= ((u >> 8) & 0xffu) << (8 * e);
+            }
+            if (t.codes32) *reinterpret_cast<int4 *>(t.codes32 + at) = make_int4(q[0], q[1], q[2], q[3]);
+            if (t.mask) *reinterpret_cast<uint32_t *>(t.mask + at) = keeps;
+            t.planes[(2 * r) * t.kWords + kw] = high;
+            t.planes[(2 * r + 1) * t.kWords + kw] = low;
+            continue;
+        }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int k = 4 * kw + e;
@@ -1465,6 +1487,7 @@ void runWide(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaStr
     };
     p.x = tensor(RXMET_GRU_X, call.x, call.x_codes_in, rows, I, o.kI, o.xPlanes);
     p.x.codes32 = call.x_codes_in ? nullptr : call.x_q; p.x.mask = mk.x;
+    p.x.vectors = I % 4 == 0 && p.x.src && alignedTo(p.x.src, 16) && alignedTo(p.x.codes32, 16) && alignedTo(p.x.mask, 4);
     p.h0 = tensor(RXMET_GRU_H, call.h0, call.h0_codes_in, static_cast<size_t>(B), H, o.kH, o.h0Planes);
     p.h0.mask = mk.h0; p.h0.codes = o.h0Codes; p.h0.colsPadded = o.hPad;
     constexpr int kBlock = 32 * kPrepLayers;
@@ -1474,11 +1497,13 @@ void runWide(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaStr
     p.prepBlocks = o.wTiles ? planeproj::paddedC(C) / 32 : (C + 31) / 32;
     p.xBlocks = blocksFor(p.x); p.h0Blocks = blocksFor(p.h0);
     p.clear = o.projStatus;
-    {
-        KernelTimer timer__("prepareWeights", st);
-        prepareWide<<<p.prepBlocks + p.xBlocks + p.h0Blocks, kBlock, 0, st>>>(p);
+    if (forwardPhase() != ForwardPhase::Recurrence) {
+        {
+            KernelTimer timer__("prepareWeights", st);
+            prepareWide<<<p.prepBlocks + p.xBlocks + p.h0Blocks, kBlock, 0, st>>>(p);
+        }
+        afterLaunch("prepareWeights");
     }
-    afterLaunch("prepareWeights");
 
     WideCall wc{};
     wc.T = T; wc.B = B; wc.I = I; wc.H = H;
@@ -2144,6 +2169,7 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, 
         runWide(call, e, ws, st);
         return;
     }
+    if (forwardPhase() == ForwardPhase::Recurrence) return;   // not split: done by the call before
     if (l == CodeClass::I32 || w == CodeClass::I32 || a == CodeClass::I32) {
         runTyped<int32_t, int32_t, int32_t>(call, e, ws, st);
     } else if (w == CodeClass::I8 && a == CodeClass::I8) {

@@ -389,7 +389,9 @@ void forwardWide(const WideCall &call, const Exec &e, cudaStream_t st) {
     const int kPadI = planeproj::paddedK(kI);
     const int rowsPerTile = projectionRows(kI);
     const bool tensorProjection = l.wTiles != nullptr;
-    if (tensorProjection) {
+    if (forwardPhase() == ForwardPhase::Recurrence) {
+        // the call before has projected
+    } else if (tensorProjection) {
         planeproj::Problem pp{};
         pp.planes = l.xPlanes; pp.rows = static_cast<int>(rows); pp.kWords = kI; pp.tiles = l.wTiles; pp.C = C; pp.status = l.projStatus;
         PlaneEpilogue epi{};
@@ -429,7 +431,7 @@ void forwardWide(const WideCall &call, const Exec &e, cudaStream_t st) {
         else launch(inputLinearPlanes<32, true>);
         afterLaunch("inputLinear");
     }
-    {
+    if (forwardPhase() != ForwardPhase::Projection) {
         RecurrentArgs a{};
         a.T = T; a.B = B; a.H = H; a.HP = (H + 31) / 32 * 32; a.kWords = kH;
         a.words = l.rWords; a.addend = l.addH; a.rescale = call.gemmH; a.ih = l.ihCodes;

@@ -19,18 +19,19 @@ layers run in the library.
 """
 from __future__ import annotations
 
+import ctypes as C
 from typing import List, Optional
 
 import torch
 
+from . import _cabi as cabi
 from .gru_interface_binding import OperatorQuantConfig
-from .qat import GruQatStep, graph_kernels
+from .qat import GruQatStep, _p, graph_kernels
 
 
 def a16_config(weight_bits: int = 8, activation_bits: int = 16) -> OperatorQuantConfig:
     """W8 per-channel weights and biases, every activation point on `activation_bits`."""
     cfg = OperatorQuantConfig()
-    from . import _cabi as cabi
     for name in cabi.OP_NAMES:
         setattr(cfg, f"{name}_", weight_bits if name in ("W", "R", "bw", "br") else activation_bits)
     return cfg
@@ -44,7 +45,6 @@ class StackedGruQat:
         self.group = process_group
         self.world = torch.distributed.get_world_size(process_group) if process_group is not None else 1
         self.config = config or a16_config()
-        from . import _cabi as cabi
         self._lib = cabi.load_library()
         f32 = dict(dtype=torch.float32, device=self.device)
         inputs = [I] + [2 * H] * (layers - 1)
@@ -81,25 +81,31 @@ class StackedGruQat:
         self.y = [torch.empty((T, B, 2 * H), **f32) for _ in range(layers)]
         self.dy = torch.empty((T, B, 2 * H), **f32)
         self.x_rev = [torch.empty((T, B, i), **f32) for i in inputs]
-        self.dx = [torch.empty((T, B, i), **f32) for i in inputs]
+        self.dx = [torch.empty((T, B, i), **f32) for i in inputs]   # gradients between the layers; dx[0] is not written
         self.side = torch.cuda.Stream(self.device)
         self.loss = torch.zeros((), **f32)
 
     # ---- helpers -----------------------------------------------------------
-    def _both(self, fn_forward, fn_reverse):
-        """Runs the two callables on the current and the side stream and joins them."""
+    def _stream(self):
+        return C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+
+    def _both(self, fn_forward, fn_reverse, phase=0):
+        """Runs the two callables on the current and the side stream and joins them; `phase` is the part of a forward
+        they run (rxmet_set_forward_phase)."""
         main = torch.cuda.current_stream(self.device)
         self.side.wait_stream(main)
         # The two directions share the SMs: their CTAs are resident together.  The setting is read where a launch is
         # planned and holds for the whole process, so it goes back at once: left at 2, every later recurrence of the
         # program plans for half of the SMs (a wide LSTM forward at batch 4096: 289 ms instead of 143 ms).
         self._lib.rxmet_set_concurrent_passes(2)
+        self._lib.rxmet_set_forward_phase(phase)
         try:
             fn_forward()
             with torch.cuda.stream(self.side):
                 fn_reverse()
         finally:
             self._lib.rxmet_set_concurrent_passes(1)
+            self._lib.rxmet_set_forward_phase(0)
         main.wait_stream(self.side)
 
     def _layer_input(self, li: int, x: torch.Tensor) -> torch.Tensor:
@@ -126,19 +132,17 @@ class StackedGruQat:
     # ---- one training step ------------------------------------------------------
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """Quantized training forward of all layers; returns the top layer's output [T,B,2H]."""
-        H = self.H
         for li, (fw, bw) in enumerate(self.dirs):
-            xin = self._layer_input(li, x)
-            y = self.y[li]
-
-            def run_forward():
-                y[..., :H].copy_(fw.forward(xin))
-
-            def run_reverse():
-                self.x_rev[li].copy_(xin.flip(0))
-                y[..., H:].copy_(bw.forward(self.x_rev[li]).flip(0))
-
-            self._both(run_forward, run_reverse)
+            xin, x_rev = self._layer_input(li, x), self.x_rev[li]
+            if li == 0:
+                x_rev.copy_(xin.flip(0))   # the layers above get theirs from the join below
+            # Both projections before either recurrence: the clusters of a recurrence need whole groups of free SMs, and one
+            # that starts beside the other direction's projection gets the last of them when the other recurrence is over.
+            self._both(lambda: fw.forward(xin), lambda: bw.forward(x_rev), phase=1)
+            self._both(lambda: fw.forward(xin), lambda: bw.forward(x_rev), phase=2)
+            above = self.x_rev[li + 1] if li + 1 < self.layers else None
+            cabi.check(self._lib.rxmet_join_directions(
+                self.T, self.B, self.H, _p(fw.h[1:]), _p(bw.h[1:]), _p(self.y[li]), _p(above), self._stream()), "join_directions")
         return self.y[-1]
 
     def head(self, y: torch.Tensor, labels: torch.Tensor) -> torch.Tensor:
@@ -159,23 +163,14 @@ class StackedGruQat:
 
     def backward(self) -> None:
         """BPTT of all layers from self.dy down to the input; gradients land in the flat gradient buffer."""
-        H = self.H
-        dy = self.dy
+        grads = (self.dy, None)   # of the layer's output; the second one in reversed time
         for li in range(self.layers - 1, -1, -1):
             fw, bw = self.dirs[li]
-
-            def run_forward():
-                fw.dh_new[1:].copy_(dy[..., :H])
-                fw.backward()
-
-            def run_reverse():
-                bw.dh_new[1:].copy_(dy[..., H:].flip(0))
-                bw.backward()
-
-            self._both(run_forward, run_reverse)
-            if li > 0:  # gradient of the layer below: both directions read the same input
-                torch.add(fw.dx, bw.dx.flip(0), out=self.dx[li])
-                dy = self.dx[li]
+            cabi.check(self._lib.rxmet_split_directions(
+                self.T, self.B, self.H, _p(grads[0]), _p(grads[1]), _p(self.dx[li + 1]) if li + 1 < self.layers else None,
+                _p(fw.dh_new[1:]), _p(bw.dh_new[1:]), self._stream()), "split_directions")
+            self._both(fw.backward, bw.backward)
+            grads = (fw.dx, bw.dx)   # both directions of this layer read the output of the one below
 
     def capture_step(self, x: torch.Tensor, labels: torch.Tensor, lr: float, warmup: int = 2):
         """Captures `step` on fixed buffers into ONE CUDA graph - about 100 kernel launches on two streams per
