@@ -136,9 +136,9 @@ struct GruPlaneCell {
         }
         return l;
     }
-    __device__ __forceinline__ float scaleH(bool alive) const {
-        return (!alive || (poison && *poison)) ? __int_as_float(0x7fc00000) : s.effH;
-    }
+    // whether the projection before it went through; asked once, before the first step
+    __device__ __forceinline__ bool valid() const { return poison == nullptr || *poison == 0; }
+    __device__ __forceinline__ float scaleH(bool good) const { return good ? s.effH : __int_as_float(0x7fc00000); }
     __device__ __forceinline__ void begin(uint32_t, State &st, int row, int unit) const {
         const int H = hidden();
         st.h = h0[static_cast<size_t>(row) * hPad + unit];
@@ -221,7 +221,9 @@ struct GruPlaneCell {
         st.keep = keep;
         return static_cast<uint32_t>(st.h - s.loH);
     }
-    __device__ __forceinline__ void store(const State &st, const FetchB &in, size_t at, uint32_t row, int unit, bool good) const {
+    // All lanes of a cell store all of it: picking a lane's share costs more than the stores (H = 64: 93 against 77 us).
+    template <int LANES = 1>
+    __device__ __forceinline__ void store(const State &st, const FetchB &in, size_t at, uint32_t row, int unit, bool good, int = 0) const {
         const int H = hidden();
         const uint32_t mine = row * H + unit, mine3 = row * (3 * H) + unit;
         h[(at + B) * H + mine] = static_cast<float>(st.h - s.zpH) * scaleH(good);

@@ -47,7 +47,9 @@ laneRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c
     const int H = p.H, tid = threadIdx.x, threads = blockDim.x, lane = tid & 3, first = tid & 28;
     const int unit = min(tid >> 2, H - 1), b0 = static_cast<int>(blockIdx.x) * BT;
     const int rowOf = BT == 1 ? 0 : BT == 2 ? lane >> 1 : lane;   // this lane's row in the cell
-    const int row = min(b0 + rowOf, p.B - 1);
+    constexpr int kLanes = 4 / BT;                                // lanes that hold the same cell
+    const int row = min(b0 + rowOf, p.B - 1), part = lane % kLanes;
+    const bool good = c.valid();
     const int kWords = (H + 15) / 16 * 4;
 
     c.init(smemL + codeBytes(KW, BT), tid, threads);
@@ -82,7 +84,7 @@ laneRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c
     };
     auto store = [&](int t, const Operands &of) {
         const size_t at = static_cast<size_t>(t) * p.B;
-        c.store(state, of.b, at, row, unit, true);
+        c.template store<kLanes>(state, of.b, at, row, unit, good, part);
         if (Cell::kSaves && lane < kGates) {
 #pragma unroll
             for (int r = 0; r < BT; ++r) c.storeLinear(saved[r], at, min(b0 + r, p.B - 1), lane, unit);
@@ -175,7 +177,7 @@ laneRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c
     } else {
         store(t - 1, odd);
     }
-    c.finish(state, row, unit, true);
+    c.finish(state, row, unit, good);
 }
 
 // Rows of a CTA for a batch: as few as leave half of the GPU to the other direction of a layer; 0 where the cluster kernel is

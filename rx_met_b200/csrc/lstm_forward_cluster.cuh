@@ -123,9 +123,9 @@ struct LstmPlaneCell {
         l.narrow = __all_sync(0xffffffffu, wMax * 65535 * H + llabs(l.addend) < (int64_t{1} << 31));
         return l;
     }
-    __device__ __forceinline__ float scaleH(bool good) const {
-        return (!good || (poison && *poison)) ? __int_as_float(0x7fc00000) : s.scale[RXMET_LSTM_OUTPUT];
-    }
+    // whether the projection before it went through; asked once, before the first step
+    __device__ __forceinline__ bool valid() const { return poison == nullptr || *poison == 0; }
+    __device__ __forceinline__ float scaleH(bool good) const { return good ? s.scale[RXMET_LSTM_OUTPUT] : __int_as_float(0x7fc00000); }
     // centred limits of an operator's grid
     __device__ __forceinline__ float lowOf(int op) const { return static_cast<float>(s.lo[op] - s.zp[op]); }
     __device__ __forceinline__ float highOf(int op) const { return static_cast<float>(s.hi[op] - s.zp[op]); }
@@ -186,10 +186,15 @@ struct LstmPlaneCell {
         const int i = static_cast<int>(index & 0x7fffffu);
         return i < flagBelow[t] || i >= flagFrom[t];
     }
-    __device__ __forceinline__ void store(const State &st, const FetchB &, size_t at, uint32_t row, int unit, bool good) const {
+    // LANES lanes hold the same cell and share its stores, `part` of them is this one's
+    template <int LANES = 1>
+    __device__ __forceinline__ void store(const State &st, const FetchB &, size_t at, uint32_t row, int unit, bool good, int part = 0) const {
         const int H = hidden();
         const size_t o = at * H + (row * H + unit);
-        output[o] = __fmul_rn(st.hidden, scaleH(good));
+        if (LANES == 1 || part == 0) output[o] = __fmul_rn(st.hidden, scaleH(good));
+        if (TRAIN && LANES > 1) {
+            if (part != LANES - 1) return;
+        }
         if (TRAIN) {
             if (ck.cell_states) ck.cell_states[o] = st.cell + s.zpF[RXMET_LSTM_CELL_STATE];
             if (ck.cell_states_clamped) ck.cell_states_clamped[o] = static_cast<uint8_t>(st.flags & 1u);
@@ -222,11 +227,13 @@ struct LstmPlaneCell {
 template <bool TRAIN, int HP>
 void launchLstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &cell, cudaStream_t st) {
     if constexpr (HP <= 128)
-        if (lanerec::launch<LstmPlaneCell<TRAIN>, HP / 4>("lstmRecurrentWide", p, cell, st)) return;
+        if (p.H != HP && lanerec::launch<LstmPlaneCell<TRAIN>, HP / 4>("lstmRecurrentWide", p, cell, st)) return;
     if (p.H == HP) {
         LstmPlaneCell<TRAIN, HP> full;
         static_assert(sizeof(full) == sizeof(cell), "the variants differ in the width only");
         std::memcpy(&full, &cell, sizeof(full));
+        if constexpr (HP <= 128)
+            if (lanerec::launch<LstmPlaneCell<TRAIN, HP>, HP / 4>("lstmRecurrentWide", p, full, st)) return;
         planerec::launchBest<LstmPlaneCell<TRAIN, HP>, HP, 64, 2, 5, 4, 8, 16, 24, 32>("lstmRecurrentWide", p, full, st);
     } else {
         planerec::launchBest<LstmPlaneCell<TRAIN>, HP, 64, 2, 5, 4, 8, 16, 24, 32>("lstmRecurrentWide", p, cell, st);

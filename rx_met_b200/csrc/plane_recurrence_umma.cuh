@@ -92,12 +92,13 @@ struct Problem {
 //   size_t sharedBytes()                                    host: size of that part
 //   uint32_t weightWord(gate, unit, kw)                     four weight bytes along K, 0 for an empty quarter
 //   void init(uint8_t *, tid, threads)                      fills it
+//   bool valid()                                            false: the inputs are not good, outputs become NaN
 //   Lane lane(shared, gate, unit, real)                     constants of phase A (all lanes of the warp call it)
 //   void begin(shared, State &, row, unit)                  state of one cell of phase B from h0
 //   void fetch(Fetch &, at, row, gate, unit), fetchB(FetchB &, at, row, unit)     operands of a step, asked for before the product is awaited
 //   uint32_t linear<STRIDE>(shared, Lane, Fetch, acc, Saved &)    phase A; plane p of the sum at acc[p STRIDE]
 //   uint32_t cell(shared, State &, FetchB, v[4])            phase B: new code - grid minimum
-//   void store(State, FetchB, at, row, unit, good)          outputs of the step; good = false: make them NaN
+//   void store<LANES>(State, FetchB, at, row, unit, good, part)   outputs of the step; good = false: make them NaN
 //   void storeLinear(Saved, at, row, gate, unit)            what phase A saves
 //   void finish(State, row, unit, good)                     after the last step
 template <class Cell, int HP, int U, int ROWS, int PLANES>
@@ -196,6 +197,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
     } else {
         // units beyond the layer's width compute on zero weights and store nothing; their operand bytes stay zero
         const bool real = Cell::kFull || unit < H;
+        const bool valid = c.valid();
         // rows of phase A in one go: as many as the operator allows and the rows divide into
         constexpr int kChunk = G::kRowsA <= Cell::kChunk ? G::kRowsA : (G::kRowsA % Cell::kChunk == 0 ? Cell::kChunk : 4);
         constexpr bool kDefer = G::kRowsA == 4;   // more rows keep the epilogue busy by themselves; held back they would spill
@@ -267,7 +269,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
                 } else {
                     dst[0] = static_cast<uint8_t>(u);
                 }
-                if (!kDefer) c.store(state[i], inB[i], at, rowB + i, unit, alive && !failed);
+                if (!kDefer) c.store(state[i], inB[i], at, rowB + i, unit, valid && alive && !failed);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -275,7 +277,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
             if (kDefer) {   // what nobody waits for leaves while the codes travel and the next product runs
 #pragma unroll
                 for (int i = 0; i < G::kRowsB; ++i)
-                    if (real && rowB + i < p.B) c.store(state[i], inB[i], at, rowB + i, unit, alive && !failed);
+                    if (real && rowB + i < p.B) c.store(state[i], inB[i], at, rowB + i, unit, valid && alive && !failed);
                 if (Cell::kSaves && quarter < Cell::kGates) {
 #pragma unroll
                     for (int r = 0; r < kChunk; ++r)
@@ -285,7 +287,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
         }
 #pragma unroll
         for (int i = 0; i < G::kRowsB; ++i)
-            if (real && rowB + i < p.B) c.finish(state[i], rowB + i, unit, alive && !failed);
+            if (real && rowB + i < p.B) c.finish(state[i], rowB + i, unit, valid && alive && !failed);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
