@@ -257,7 +257,7 @@ struct GruPlaneCell {
             }
         }
     }
-    __device__ __forceinline__ void storeLinear(const Saved &, size_t, uint32_t, int, int) const {}
+    __device__ __forceinline__ void storeLinear(const Lane &, const Saved &, size_t, uint32_t, int, int) const {}
     __device__ __forceinline__ void finish(const State &, int, int, bool) const {}
 };
 
@@ -322,7 +322,7 @@ void launchFor(const WideRecurrence &r, const Prepared &prepared, cudaStream_t s
     cell.poison = r.poison;
     const planerec::Problem problem{r.T, r.B, r.H, r.h0Planes};
     if constexpr (HP == 64 || HP == 128)
-        if (lanerec::launch<Cell, HP / 4>("recurrentForward", problem, cell, st)) return;
+        if (lanerec::launch<Cell, HP / 4, 2>("recurrentForward", problem, cell, st)) return;
     if constexpr (HP < 64) planerec::launchBest<Cell, HP, HP, 2, 32, 8, 16>("recurrentForward", problem, cell, st);
     else planerec::launchBest<Cell, HP, 64, 2, 32, 4, 8, 16>("recurrentForward", problem, cell, st);
 }
@@ -372,7 +372,7 @@ bool forwardWideClusterTakes(const Exec &e, int H) {
 void forwardWideCluster(const WideRecurrence &r, const Exec &e, cudaStream_t st) {
     Prepared prepared;
     prepare(e, prepared);
-    if (r.H <= 32 && lanerec::rowsFor<16>(r.B) == 0) launchFor<32>(r, prepared, st);
+    if (r.H <= 32 && lanerec::rowsFor<16, 2>(r.B) == 0) launchFor<32>(r, prepared, st);
     else if (r.H <= 64) launchFor<64>(r, prepared, st);
     else if (r.H <= 128) launchFor<128>(r, prepared, st);
     else if (r.H <= 192) launchFor<192>(r, prepared, st);

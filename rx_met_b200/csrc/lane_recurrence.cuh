@@ -32,17 +32,17 @@ __device__ __forceinline__ int32_t dotSignedUnsigned(uint32_t signedBytes, uint3
     return d;
 }
 
-__host__ __device__ constexpr size_t codeBytes(int KW, int BT) { return 2 * static_cast<size_t>(BT) * 2 * KW * 4; }
+__host__ __device__ constexpr size_t codeBytes(int KW, int BT, int planes) { return 2 * static_cast<size_t>(BT) * planes * KW * 4; }
 
-// KW: words of a plane row (H <= 4 KW); BT: rows of a CTA.  Two planes.
-template <class Cell, int KW, int BT>
+// KW: words of a plane row (H <= 4 KW); BT: rows of a CTA.  One plane (8-bit codes) or two.
+template <class Cell, int KW, int BT, int PLANES>
 __global__ void __launch_bounds__(16 * KW)
 laneRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c) {
     constexpr int KL = KW / 4, kGates = Cell::kGates;   // words of a lane's quarter of K
     static_assert(KL % 4 == 0, "a quarter is read in 16-byte pieces");
     extern __shared__ __align__(16) uint8_t smemL[];
-    uint32_t *codes = reinterpret_cast<uint32_t *>(smemL);   // [2][BT][2 planes][KW]
-    const uint32_t shared = static_cast<uint32_t>(__cvta_generic_to_shared(smemL)) + static_cast<uint32_t>(codeBytes(KW, BT));
+    uint32_t *codes = reinterpret_cast<uint32_t *>(smemL);   // [2][BT][PLANES][KW]
+    const uint32_t shared = static_cast<uint32_t>(__cvta_generic_to_shared(smemL)) + static_cast<uint32_t>(codeBytes(KW, BT, PLANES));
 
     const int H = p.H, tid = threadIdx.x, threads = blockDim.x, lane = tid & 3, first = tid & 28;
     const int unit = min(tid >> 2, H - 1), b0 = static_cast<int>(blockIdx.x) * BT;
@@ -52,10 +52,10 @@ laneRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c
     const bool good = c.valid();
     const int kWords = (H + 15) / 16 * 4;
 
-    c.init(smemL + codeBytes(KW, BT), tid, threads);
-    for (int i = tid; i < 2 * BT * 2 * KW; i += threads) {
-        const int kw = i % KW, plane = i / KW % 2, r = i / (2 * KW) % BT, buffer = i / (2 * KW * BT);
-        codes[i] = buffer == 0 && kw < kWords ? p.h0[(static_cast<size_t>(min(b0 + r, p.B - 1)) * 2 + plane) * kWords + kw] : 0u;
+    c.init(smemL + codeBytes(KW, BT, PLANES), tid, threads);
+    for (int i = tid; i < 2 * BT * PLANES * KW; i += threads) {
+        const int kw = i % KW, plane = i / KW % PLANES, r = i / (PLANES * KW) % BT, buffer = i / (PLANES * KW * BT);
+        codes[i] = buffer == 0 && kw < kWords ? p.h0[(static_cast<size_t>(min(b0 + r, p.B - 1)) * PLANES + plane) * kWords + kw] : 0u;
     }
     uint32_t w[kGates][KL];
 #pragma unroll
@@ -87,12 +87,12 @@ laneRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c
         c.template store<kLanes>(state, of.b, at, row, unit, good, part);
         if (Cell::kSaves && lane < kGates) {
 #pragma unroll
-            for (int r = 0; r < BT; ++r) c.storeLinear(saved[r], at, min(b0 + r, p.B - 1), lane, unit);
+            for (int r = 0; r < BT; ++r) c.storeLinear(mine, saved[r], at, min(b0 + r, p.B - 1), lane, unit);
         }
     };
     auto step = [&](int t, Operands &now, Operands &other) {
         __syncthreads();   // the codes of step t
-        const uint32_t *from = codes + (t & 1) * (BT * 2 * KW) + lane * KL;
+        const uint32_t *from = codes + (t & 1) * (BT * PLANES * KW) + lane * KL;
         int32_t sum[BT];
         if (t > 0) store(t - 1, other);
         if (t + 1 < p.T) fetch(t + 1, other);
@@ -100,13 +100,13 @@ laneRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c
         for (int r = 0; r < BT; ++r) {
             int32_t part[4] = {0, 0, 0, 0};
 #pragma unroll
-            for (int plane = 0; plane < 2; ++plane) {
+            for (int plane = 0; plane < PLANES; ++plane) {
                 int32_t acc[kGates];
 #pragma unroll
                 for (int g = 0; g < kGates; ++g) acc[g] = 0;
 #pragma unroll
                 for (int i = 0; i < KL; i += 4) {
-                    const uint4 h = *reinterpret_cast<const uint4 *>(from + (r * 2 + plane) * KW + i);
+                    const uint4 h = *reinterpret_cast<const uint4 *>(from + (r * PLANES + plane) * KW + i);
 #pragma unroll
                     for (int g = 0; g < kGates; ++g) {
                         acc[g] = dotSignedUnsigned(w[g][i], h.x, acc[g]);
@@ -159,9 +159,9 @@ laneRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c
             }
         }
         const uint32_t code = c.cell(shared, state, now.b, v);
-        uint8_t *to = reinterpret_cast<uint8_t *>(codes + ((t + 1) & 1) * (BT * 2 * KW) + rowOf * 2 * KW) + unit;
-        to[0] = static_cast<uint8_t>(code >> 8);
-        to[4 * KW] = static_cast<uint8_t>(code);
+        uint8_t *to = reinterpret_cast<uint8_t *>(codes + ((t + 1) & 1) * (BT * PLANES * KW) + rowOf * PLANES * KW) + unit;
+        if (PLANES == 2) to[0] = static_cast<uint8_t>(code >> 8);
+        to[(PLANES - 1) * 4 * KW] = static_cast<uint8_t>(code);
     };
     Operands even, odd;
     fetch(0, even);
@@ -180,21 +180,22 @@ laneRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c
     c.finish(state, row, unit, good);
 }
 
-// Rows of a CTA for a batch: as few as leave half of the GPU to the other direction of a layer; 0 where the cluster kernel is
-// the better one (more rows, or four rows of 128 units, whose products then take as long as its chain).
-template <int KW>
+// Rows of a CTA for a batch; 0 where other kernels are the better ones.  Two planes: as few as leave half of the GPU to the
+// other direction of a layer, and not four rows of 128 units, whose products take as long as the chain of a cluster.  One
+// plane: as few as one wave of CTAs holds, and not four rows of 64 units.
+template <int KW, int PLANES>
 int rowsFor(int B) {
-    const int half = std::max(1, currentDevice().sms / 2);
+    const int ctas = std::max(1, PLANES == 2 ? currentDevice().sms / 2 : currentDevice().sms);
     for (int rows : {1, 2, 4})
-        if ((B + rows - 1) / rows <= half) return KW == 32 && rows == 4 ? 0 : rows;
+        if ((B + rows - 1) / rows <= ctas) return rows == 4 && KW == (PLANES == 2 ? 32 : 16) ? 0 : rows;
     return 0;
 }
 
-template <class Cell, int KW>
+template <class Cell, int KW, int PLANES>
 bool launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t st) {
-    const int rows = rowsFor<KW>(p.B);
+    const int rows = rowsFor<KW, PLANES>(p.B);
     auto run = [&](auto kernel, int BT) {
-        const size_t smem = codeBytes(KW, BT) + cell.sharedBytes();
+        const size_t smem = codeBytes(KW, BT, PLANES) + cell.sharedBytes();
         if (smem > static_cast<size_t>(currentDevice().smemMax)) return false;
         ensureDynamicSmem(reinterpret_cast<const void *>(kernel), smem);
         {
@@ -204,10 +205,10 @@ bool launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t s
         afterLaunch(name);
         return true;
     };
-    if (rows == 1) return run(laneRecurrence<Cell, KW, 1>, 1);
-    if (rows == 2) return run(laneRecurrence<Cell, KW, 2>, 2);
-    if constexpr (KW < 32)
-        if (rows == 4) return run(laneRecurrence<Cell, KW, 4>, 4);
+    if (rows == 1) return run(laneRecurrence<Cell, KW, 1, PLANES>, 1);
+    if (rows == 2) return run(laneRecurrence<Cell, KW, 2, PLANES>, 2);
+    if constexpr (KW != (PLANES == 2 ? 32 : 16))
+        if (rows == 4) return run(laneRecurrence<Cell, KW, 4, PLANES>, 4);
     return false;
 }
 

@@ -74,6 +74,8 @@ struct LstmPlaneCell {
         int64_t addend;
         float outMult, outPow2, gateMult, gatePow2, giLo, giHi;
         TableView table;
+        float zpIn, zpOut;               // zero points and clamp limits that storeLinear needs
+        int flagBelow, flagFrom;
         bool narrow;   // warp-uniform: the sum fits 32 bits
     };
     struct State {
@@ -119,6 +121,10 @@ struct LstmPlaneCell {
         l.giLo = static_cast<float>(s.lo[opIn] - s.zp[opIn]);
         l.giHi = static_cast<float>(s.hi[opIn] - s.zp[opIn]);
         l.table = view(shared, gate);
+        l.zpIn = s.zpF[opIn];
+        l.zpOut = s.zpF[RXMET_LSTM_INPUT_GATE_OUTPUT + gate];
+        l.flagBelow = flagBelow[gate];
+        l.flagFrom = flagFrom[gate];
         const int64_t wMax = max(-static_cast<int64_t>(s.lo[RXMET_LSTM_WEIGHT_HH]), static_cast<int64_t>(s.hi[RXMET_LSTM_WEIGHT_HH]));
         l.narrow = __all_sync(0xffffffffu, wMax * 65535 * H + llabs(l.addend) < (int64_t{1} << 31));
         return l;
@@ -204,16 +210,16 @@ struct LstmPlaneCell {
             if (ck.hidden_outputs_clamped) ck.hidden_outputs_clamped[o] = static_cast<uint8_t>((st.flags >> 2) & 1u);
         }
     }
-    __device__ __forceinline__ void storeLinear(const Saved &v, size_t at, uint32_t row, int gate, int unit) const {
+    __device__ __forceinline__ void storeLinear(const Lane &l, const Saved &v, size_t at, uint32_t row, int gate, int unit) const {
         const int H = hidden();
         const size_t o = at * (4 * static_cast<size_t>(H)) + (row * (4 * H) + gate * H + unit);
-        const int opIn = RXMET_LSTM_INPUT_GATE_INPUT + gate, opOut = RXMET_LSTM_INPUT_GATE_OUTPUT + gate;
+        const int index = static_cast<int>(v.index & 0x7fffffu);
         if (ck.weight_hh_linear) ck.weight_hh_linear[o] = v.hh + s.zpF[RXMET_LSTM_WEIGHT_HH_LINEAR];
         if (ck.weight_hh_linear_clamped) ck.weight_hh_linear_clamped[o] = v.hhClamped;
-        if (ck.gate_inputs) ck.gate_inputs[o] = v.gateIn + s.zpF[opIn];
+        if (ck.gate_inputs) ck.gate_inputs[o] = v.gateIn + l.zpIn;
         if (ck.gate_inputs_clamped) ck.gate_inputs_clamped[o] = v.inClamped;
-        if (ck.gate_outputs) ck.gate_outputs[o] = v.gateOut + s.zpF[opOut];
-        if (ck.gate_outputs_clamped) ck.gate_outputs_clamped[o] = clampFlag(gate, v.index);
+        if (ck.gate_outputs) ck.gate_outputs[o] = v.gateOut + l.zpOut;
+        if (ck.gate_outputs_clamped) ck.gate_outputs_clamped[o] = index < l.flagBelow || index >= l.flagFrom;
     }
     __device__ __forceinline__ void finish(const State &st, int row, int unit, bool good) const {
         const int H = hidden();
@@ -227,21 +233,36 @@ struct LstmPlaneCell {
 template <bool TRAIN, int HP>
 void launchLstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &cell, cudaStream_t st) {
     if constexpr (HP <= 128)
-        if (p.H != HP && lanerec::launch<LstmPlaneCell<TRAIN>, HP / 4>("lstmRecurrentWide", p, cell, st)) return;
+        if (p.H != HP && lanerec::launch<LstmPlaneCell<TRAIN>, HP / 4, 2>("lstmRecurrentWide", p, cell, st)) return;
     if (p.H == HP) {
         LstmPlaneCell<TRAIN, HP> full;
         static_assert(sizeof(full) == sizeof(cell), "the variants differ in the width only");
         std::memcpy(&full, &cell, sizeof(full));
         if constexpr (HP <= 128)
-            if (lanerec::launch<LstmPlaneCell<TRAIN, HP>, HP / 4>("lstmRecurrentWide", p, full, st)) return;
+            if (lanerec::launch<LstmPlaneCell<TRAIN, HP>, HP / 4, 2>("lstmRecurrentWide", p, full, st)) return;
         planerec::launchBest<LstmPlaneCell<TRAIN, HP>, HP, 64, 2, 5, 4, 8, 16, 24, 32>("lstmRecurrentWide", p, full, st);
     } else {
         planerec::launchBest<LstmPlaneCell<TRAIN>, HP, 64, 2, 5, 4, 8, 16, 24, 32>("lstmRecurrentWide", p, cell, st);
     }
 }
+// 8-bit inference, at most 128 units, rows that one wave of CTAs holds (lanerec::rowsFor): the same cell on one byte plane.
+template <int HP>
+void launchLstmBytes(const planerec::Problem &p, const LstmPlaneCell<false> &cell, cudaStream_t st) {
+    bool done;
+    if (p.H == HP) {
+        LstmPlaneCell<false, HP> full;
+        std::memcpy(&full, &cell, sizeof(full));
+        done = lanerec::launch<LstmPlaneCell<false, HP>, HP / 4, 1>("lstmRecurrent", p, full, st);
+    } else {
+        done = lanerec::launch<LstmPlaneCell<false>, HP / 4, 1>("lstmRecurrent", p, cell, st);
+    }
+    RXMET_REQUIRE(done, "8-bit LSTM recurrence: %d rows", p.B);
+}
 // One padded width each, built in separate files (lstm_forward_cluster_*.cu).
 template <bool TRAIN, int HP>
 void lstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &cell, cudaStream_t st);
+template <int HP>
+void lstmBytes(const planerec::Problem &p, const LstmPlaneCell<false> &cell, cudaStream_t st);
 
 }  // namespace lstm
 }  // namespace rxmet

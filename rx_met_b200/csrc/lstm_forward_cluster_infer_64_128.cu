@@ -12,6 +12,14 @@ template <>
 void lstmCluster<false, 128>(const planerec::Problem &p, const LstmPlaneCell<false> &cell, cudaStream_t st) {
     launchLstmCluster<false, 128>(p, cell, st);
 }
+template <>
+void lstmBytes<64>(const planerec::Problem &p, const LstmPlaneCell<false> &cell, cudaStream_t st) {
+    launchLstmBytes<64>(p, cell, st);
+}
+template <>
+void lstmBytes<128>(const planerec::Problem &p, const LstmPlaneCell<false> &cell, cudaStream_t st) {
+    launchLstmBytes<128>(p, cell, st);
+}
 
 }  // namespace lstm
 }  // namespace rxmet

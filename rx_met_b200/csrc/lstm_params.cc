@@ -618,7 +618,7 @@ bool buildCompact(const Exec &e, int segShift, CompactTables &out) {
         at = (at + 15) & ~static_cast<size_t>(15);
     }
     out.bytes.assign(at, 0);
-    out.ok = forEachTable(at > 4096, [&](int t) {
+    out.ok = forEachTable(at > 65536, [&](int t) {
         const ScalarExec &s = e.scalar;
         const int in = kTableIn[t], to = kTableOut[t];
         const int entries = s.hi[in] - s.lo[in] + 1;
@@ -662,7 +662,8 @@ bool buildCompact(const Exec &e, int segShift, CompactTables &out) {
 const CompactTables &Exec::compactTables() const {
     std::call_once(compactOnce, [&] {
         if (wide.entries.empty()) return;
-        for (int segShift = 7; segShift >= 5; --segShift)   // 8, 16, 32 kB of lines per 16-bit table beside 8 kB of bits
+        // 8, 16, 32 kB of lines per 16-bit table beside 8 kB of bits; small tables take as many lines as they need
+        for (int segShift = 7; segShift >= (wide.entries.size() > 8192 ? 5 : 0); --segShift)
             if (buildCompact(*this, segShift, compact)) return;
         compact = CompactTables{};
     });

@@ -99,7 +99,7 @@ struct Problem {
 //   uint32_t linear<STRIDE>(shared, Lane, Fetch, acc, Saved &)    phase A; plane p of the sum at acc[p STRIDE]
 //   uint32_t cell(shared, State &, FetchB, v[4])            phase B: new code - grid minimum
 //   void store<LANES>(State, FetchB, at, row, unit, good, part)   outputs of the step; good = false: make them NaN
-//   void storeLinear(Saved, at, row, gate, unit)            what phase A saves
+//   void storeLinear(Lane, Saved, at, row, gate, unit)      what phase A saves
 //   void finish(State, row, unit, good)                     after the last step
 template <class Cell, int HP, int U, int ROWS, int PLANES>
 __global__ void __launch_bounds__(Geometry<HP, U, ROWS, PLANES>::kThreads, 1)
@@ -246,7 +246,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
                     if (Cell::kSaves && !kDefer) {
 #pragma unroll
                         for (int r = 0; r < kChunk; ++r)
-                            if (real && rowA + first + r < p.B) c.storeLinear(saved[r], at, rowA + first + r, quarter, unit);
+                            if (real && rowA + first + r < p.B) c.storeLinear(mine, saved[r], at, rowA + first + r, quarter, unit);
                     }
                 }
                 if (G::kRowsA > kChunk) {
@@ -281,7 +281,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
                 if (Cell::kSaves && quarter < Cell::kGates) {
 #pragma unroll
                     for (int r = 0; r < kChunk; ++r)
-                        if (real && rowA + r < p.B) c.storeLinear(saved[r], at, rowA + r, quarter, unit);
+                        if (real && rowA + r < p.B) c.storeLinear(mine, saved[r], at, rowA + r, quarter, unit);
                 }
             }
         }

@@ -285,3 +285,19 @@ def test_histogram_calibration_session_matches_reference(method, state):
             close([got_p.struct.scale[op]], [want_p.struct.scale[op]], 0.03, L.OP_NAMES[op])
     out = m.lstm_forward_quantized(*torch_args(p), False, final["bundle_json"])
     assert torch.isfinite(out[0]).all()
+
+
+@pytest.mark.parametrize("T,B,I,H", [(1, 1, 8, 1), (3, 149, 5, 65), (4, 297, 12, 128), (2, 150, 40, 64), (5, 3, 9, 63)])
+def test_inference_in_lanes_equals_the_training_forward(T, B, I, H):
+    """8-bit inference runs another recurrence than the forward with checkpoints: the same outputs bit for bit, one, two and
+    four rows per CTA with a partly empty last CTA, widths at the edges of its tiles."""
+    import torch
+    from rx_met_b200 import _quant_lstm as m
+    cfg = L.default_config()
+    p = ll.problem(T, B, I, H, seed=T + H, wscale=float(1.0 / np.sqrt(H)))
+    _, box = ll.calibrate("orc", cfg, p, np.stack([p["x"] * 0.8]))
+    args = [torch.from_numpy(p[k]).cuda() for k in ("x", "w_ih", "w_hh", "b_ih", "b_hh", "h0", "c0")]
+    args[5:] = [a[None] for a in args[5:]]
+    runs = [m.lstm_forward_quantized(*args, False, m._params_to_bundle(box), "pedantic", False, save) for save in (False, True)]
+    for a, b in zip(runs[0][:3], runs[1][:3]):
+        assert torch.equal(a, b)
