@@ -784,9 +784,9 @@ def _kernel_ms(lib, names, per=1):
 
 _LSTM_WIDE_KERNELS = ["lstmQuantizePlanes", "lstmQuantizeCodes", "lstmPrepChannelsWide", "lstmInputLinearWide", "lstmRecurrentWide",
                       "lstmRecurrentFloatWide", "lstmRecurrentFloat", "lstmInputLinearFloat", "lstmJobMinMax", "lstmJobHistogram",
-                      "lstmRecurrentBackwardWide", "lstmRecurrentBackward", "lstmGemmNN", "lstmGemmRowsTN", "lstmReduceSplits",
-                      "lstmColumnSums", "lstmDequantWeights", "lstmPackStepMasks", "inputGradUmma", "weightGradUmma",
-                      "lstmReduceWeightGradT", "lstmInputGradNarrow", "lstmPackBackwardTiles"]
+                      "lstmRecurrentBackwardCluster", "lstmRecurrentBackwardWide", "lstmRecurrentBackward", "lstmGemmNN", "lstmGemmRowsTN",
+                      "lstmReduceSplits", "lstmColumnSums", "lstmDequantWeights", "lstmPackStepMasks", "inputGradUmma", "weightGradUmma",
+                      "lstmReduceWeightGradT", "lstmInputGradNarrow"]
 
 
 def lstm_bidirectional_a16(lib, torch, device, flush, peak_gbs, args):

@@ -106,6 +106,7 @@ int residentClusters(const void *kernel, int ctas, int block, size_t smem) {
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
+    if (ctas > 8) RXMET_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
         cudaGetLastError();

@@ -24,7 +24,7 @@ struct BackwardClusterArgs {
     float *dh0, *dc0;             // [B][H]
 };
 
-// True when the kernel takes the call: hidden units in tiles of 32, at most 256 of them, pointers aligned for its paired accesses.
+// True when the kernel takes the call: hidden units in tiles of 32, at most 512 of them, pointers aligned for its paired accesses.
 bool backwardClusterTakes(const BackwardClusterArgs &args);
 void backwardCluster(const BackwardClusterArgs &args, cudaStream_t stream);
 
