@@ -229,7 +229,13 @@ struct LstmPlaneCell {
     }
 };
 
-// Rows: a step of n rows costs about 1 + n / 5 of the chain of a one-row step.
+// Rows: a step of n rows costs about 1 + n / 5 of the chain of a one-row step.  48 only without a training forward's stores, whose
+// sixteen warps do not divide them.
+template <class Cell, int HP>
+void launchRows(const planerec::Problem &p, const Cell &cell, cudaStream_t st) {
+    if constexpr (Cell::kSaves) planerec::launchBest<Cell, HP, 64, 2, 5, 4, 8, 12, 16, 24, 32>("lstmRecurrentWide", p, cell, st);
+    else planerec::launchBest<Cell, HP, 64, 2, 5, 4, 8, 12, 16, 24, 32, 48>("lstmRecurrentWide", p, cell, st);
+}
 template <bool TRAIN, int HP>
 void launchLstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &cell, cudaStream_t st) {
     if constexpr (HP <= 128)
@@ -240,9 +246,9 @@ void launchLstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &c
         std::memcpy(&full, &cell, sizeof(full));
         if constexpr (HP <= 128)
             if (lanerec::launch<LstmPlaneCell<TRAIN, HP>, HP / 4, 2>("lstmRecurrentWide", p, full, st)) return;
-        planerec::launchBest<LstmPlaneCell<TRAIN, HP>, HP, 64, 2, 5, 4, 8, 16, 24, 32>("lstmRecurrentWide", p, full, st);
+        launchRows<LstmPlaneCell<TRAIN, HP>, HP>(p, full, st);
     } else {
-        planerec::launchBest<LstmPlaneCell<TRAIN>, HP, 64, 2, 5, 4, 8, 16, 24, 32>("lstmRecurrentWide", p, cell, st);
+        launchRows<LstmPlaneCell<TRAIN>, HP>(p, cell, st);
     }
 }
 // 8-bit inference, at most 128 units, rows that one wave of CTAs holds (lanerec::rowsFor): the same cell on one byte plane.

@@ -59,10 +59,13 @@ constexpr uint32_t powerOfTwoFrom(uint32_t n) {
     return p;
 }
 
-template <int HP, int U, int ROWS, int PLANES>
+template <int HP, int U, int ROWS, int PLANES, bool SAVES>
 struct Geometry {
     static constexpr int kCtas = HP / U, kTiles = U / 32;
-    static constexpr int kWarps = ROWS * kTiles >= 16 ? 16 : 8;   // of the epilogue; one more warp issues products and copies
+    // Warps of the epilogue; one more issues products and copies.  Three row groups instead of two hide more of the table
+    // look-ups (LSTM, H = 512, 24 rows: 4.5 -> 4.1 us per step); with a training forward's stores they lose (7.6 -> 9.5 us), except
+    // that twelve rows need them.
+    static constexpr int kWarps = ROWS * kTiles < 16 ? 8 : kTiles == 2 && (ROWS == 12 || (ROWS % 24 == 0 && !SAVES)) ? 24 : 16;
     static constexpr int kThreads = 32 * (kWarps + 1);
     static constexpr int kRowGroups = kWarps / (4 * kTiles);   // warps that share the rows of a tile's quarter
     static constexpr int kRowsA = ROWS / kRowGroups;            // rows of a lane in phase A
@@ -102,9 +105,9 @@ struct Problem {
 //   void storeLinear(Lane, Saved, at, row, gate, unit)      what phase A saves
 //   void finish(State, row, unit, good)                     after the last step
 template <class Cell, int HP, int U, int ROWS, int PLANES>
-__global__ void __launch_bounds__(Geometry<HP, U, ROWS, PLANES>::kThreads, 1)
+__global__ void __launch_bounds__(Geometry<HP, U, ROWS, PLANES, Cell::kSaves>::kThreads, 1)
 planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c) {
-    using G = Geometry<HP, U, ROWS, PLANES>;
+    using G = Geometry<HP, U, ROWS, PLANES, Cell::kSaves>;
     constexpr int MT = G::kTiles, NC = G::kCtas;
     extern __shared__ __align__(128) uint8_t smemR[];
     __shared__ __align__(8) uint64_t productBar, codeBar[2];
@@ -298,7 +301,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
 // Launches a variant with its clusters.
 template <class Cell, int HP, int U, int ROWS, int PLANES>
 void launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t st) {
-    using G = Geometry<HP, U, ROWS, PLANES>;
+    using G = Geometry<HP, U, ROWS, PLANES, Cell::kSaves>;
     const auto kernel = planeRecurrence<Cell, HP, U, ROWS, PLANES>;
     const size_t smem = G::kSharedBytes + cell.sharedBytes();
     ensureDynamicSmem(reinterpret_cast<const void *>(kernel), smem);
@@ -329,7 +332,7 @@ void launchBest(const char *name, const Problem &p, const Cell &cell, cudaStream
     int best = 0;
     (
         [&] {
-            using G = Geometry<HP, U, ROWS, PLANES>;
+            using G = Geometry<HP, U, ROWS, PLANES, Cell::kSaves>;
             if (G::kSharedBytes + cell.sharedBytes() > static_cast<size_t>(currentDevice().smemMax)) return;
             const int resident = std::max(1, residentClusters(reinterpret_cast<const void *>(planeRecurrence<Cell, HP, U, ROWS, PLANES>), G::kCtas,
                                                               G::kThreads, G::kSharedBytes + cell.sharedBytes()) / concurrentPasses());

@@ -162,3 +162,9 @@ def test_wide_qat_backward_over_clusters_and_padded_widths(T, B, I, H, wb, ab):
     """The cluster recurrence at its widths of 32 and 64 units per CTA, one to sixteen CTAs and 4, 8 and 16 rows, and widths beside those that
     the tensor-core kernels tile, which go through padded copies."""
     test_wide_qat_backward(T, B, I, H, wb, ab)
+
+
+@pytest.mark.parametrize("B", [170, 250, 350, 700])
+def test_wide_forward_at_the_row_counts_of_a_cluster(B):
+    """Twelve, sixteen or 24, 24 and 48 rows of a cluster, two or three groups of warps over them, a partial last tile of units."""
+    test_wide_forward_is_bit_exact(2, B, 8, 500, 4, 16, L.PER_CHANNEL, True, True)
