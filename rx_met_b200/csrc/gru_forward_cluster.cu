@@ -73,7 +73,7 @@ enum class Flags { None, Bytes, Packed };
 template <Flags FLAGS, int WIDTH>
 struct GruPlaneCell {
     static constexpr int kGates = 3;
-    static constexpr bool kSaves = false, kFull = WIDTH != 0;
+    static constexpr bool kSaves = false, kFull = WIDTH != 0, kTotal = false;
     static constexpr int kChunk = 4;
     CellScalars s;
     FastLut luts[3];

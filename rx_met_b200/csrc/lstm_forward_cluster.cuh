@@ -51,7 +51,7 @@ __device__ __forceinline__ float lookup(const TableView &v, int segShift, float 
 template <bool TRAIN, int WIDTH = 0>
 struct LstmPlaneCell {
     static constexpr int kGates = 4;
-    static constexpr bool kSaves = TRAIN, kFull = WIDTH != 0;
+    static constexpr bool kSaves = TRAIN, kFull = WIDTH != 0, kTotal = true;
     static constexpr int kChunk = TRAIN ? 4 : 16;
     ScalarExec s;
     int width, kWords;
@@ -72,7 +72,7 @@ struct LstmPlaneCell {
 
     struct Lane {
         int64_t addend;
-        float outMult, outPow2, gateMult, gatePow2, giLo, giHi;
+        float outScale, gateScale, giLo, giHi;   // multiplier times power of two: as exact as one after the other
         TableView table;
         float zpIn, zpOut;               // zero points and clamp limits that storeLinear needs
         int flagBelow, flagFrom;
@@ -114,10 +114,8 @@ struct LstmPlaneCell {
         const int c = gate * H + unit, opIn = RXMET_LSTM_INPUT_GATE_INPUT + gate;
         const size_t C = 4 * static_cast<size_t>(H);
         l.addend = real ? addend[c] : 0;
-        l.outMult = real ? channel[kHhOutMult * C + c] : 0.0f;
-        l.outPow2 = real ? channel[kHhOutPow2 * C + c] : 0.0f;
-        l.gateMult = s.hhToGate[gate].mult;
-        l.gatePow2 = s.hhToGate[gate].pow2;
+        l.outScale = real ? __fmul_rn(channel[kHhOutMult * C + c], channel[kHhOutPow2 * C + c]) : 0.0f;
+        l.gateScale = __fmul_rn(s.hhToGate[gate].mult, s.hhToGate[gate].pow2);
         l.giLo = static_cast<float>(s.lo[opIn] - s.zp[opIn]);
         l.giHi = static_cast<float>(s.hi[opIn] - s.zp[opIn]);
         l.table = view(shared, gate);
@@ -152,22 +150,38 @@ struct LstmPlaneCell {
         st.hidden = st.tanhC = 0.0f;
         st.flags = 0;
     }
-    __device__ __forceinline__ void fetch(Fetch &f, size_t at, uint32_t row, int gate, int unit) const {
+    __device__ __forceinline__ void fetch(Fetch &f, size_t at, int row, int gate, int unit) const {
         const int H = hidden();
-        f.lhs = __ldg(lhs + at * (4 * static_cast<size_t>(H)) + (row * (4 * H) + gate * H + unit));
+        f.lhs = __ldg(lhs + (at + static_cast<size_t>(row)) * (4 * static_cast<size_t>(H)) + (gate * H + unit));
     }
     __device__ __forceinline__ void fetchB(FetchB &, size_t, uint32_t, int) const {}
+    // the sums of ROWS rows as floats, in place of the plane sums; one branch for all of them
+    template <int STRIDE, int ROWS>
+    __device__ __forceinline__ void totals(const Lane &l, uint32_t *acc) const {
+        if (l.narrow) {
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+                acc[r] = __float_as_uint(__int2float_rn(static_cast<int32_t>(acc[r] * 256u + acc[r + STRIDE] + static_cast<uint32_t>(l.addend))));
+        } else {
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+                acc[r] = __float_as_uint(__ll2float_rn((static_cast<int64_t>(static_cast<int32_t>(acc[r])) << 8) + static_cast<int32_t>(acc[r + STRIDE]) + l.addend));
+        }
+    }
     // gate output (centred code as a float)
     template <int STRIDE>
-    __device__ __forceinline__ uint32_t linear(uint32_t, const Lane &l, const Fetch &in, const uint32_t *acc, Saved &saved) const {
-        const int32_t high = static_cast<int32_t>(acc[0]), low = static_cast<int32_t>(acc[STRIDE]);
-        float total;
-        if (l.narrow) total = __int2float_rn(static_cast<int32_t>(static_cast<uint32_t>(high) * 256u + static_cast<uint32_t>(low) + static_cast<uint32_t>(l.addend)));
-        else total = __ll2float_rn((static_cast<int64_t>(high) << 8) + low + l.addend);
+    __device__ __forceinline__ uint32_t linear(uint32_t shared, const Lane &l, const Fetch &in, const uint32_t *acc, Saved &saved) const {
+        uint32_t sums[STRIDE + 1] = {acc[0]};
+        sums[STRIDE] = acc[STRIDE];
+        totals<STRIDE, 1>(l, sums);
+        return linearOfTotal(shared, l, in, sums[0], saved);
+    }
+    __device__ __forceinline__ uint32_t linearOfTotal(uint32_t, const Lane &l, const Fetch &in, uint32_t sum32, Saved &saved) const {
+        const float total = __uint_as_float(sum32);
         bool hhClamped;
-        const float hh = quantized(__fmul_rn(__fmul_rn(total, l.outMult), l.outPow2), lowOf(RXMET_LSTM_WEIGHT_HH_LINEAR),
+        const float hh = quantized(__fmul_rn(total, l.outScale), lowOf(RXMET_LSTM_WEIGHT_HH_LINEAR),
                                    highOf(RXMET_LSTM_WEIGHT_HH_LINEAR), hhClamped);
-        const float sum = __fadd_rn(in.lhs, roundSmall(__fmul_rn(__fmul_rn(hh, l.gateMult), l.gatePow2)));
+        const float sum = __fadd_rn(in.lhs, roundSmall(__fmul_rn(hh, l.gateScale)));
         const float gateIn = clampF(sum, l.giLo, l.giHi);
         uint32_t index;
         const float gateOut = lookup(l.table, segShift, gateIn, index);
@@ -183,7 +197,7 @@ struct LstmPlaneCell {
         st.cell = quantized(__fadd_rn(sf, si), lowOf(RXMET_LSTM_CELL_STATE), highOf(RXMET_LSTM_CELL_STATE), cellClamped);
         uint32_t index;
         st.tanhC = lookup(view(shared, 4), segShift, st.cell, index);
-        st.hidden = quantized(__fmul_rn(__fmul_rn(__fmul_rn(gO, st.tanhC), s.productToOutput.mult), s.productToOutput.pow2), lowOf(RXMET_LSTM_OUTPUT),
+        st.hidden = quantized(__fmul_rn(__fmul_rn(gO, st.tanhC), __fmul_rn(s.productToOutput.mult, s.productToOutput.pow2)), lowOf(RXMET_LSTM_OUTPUT),
                               highOf(RXMET_LSTM_OUTPUT), hiddenClamped);
         if (TRAIN) st.flags = (cellClamped ? 1u : 0u) | (clampFlag(4, index) ? 2u : 0u) | (hiddenClamped ? 4u : 0u);
         return __float_as_uint(__fadd_rn(st.hidden, 8388608.0f + static_cast<float>(s.zp[RXMET_LSTM_OUTPUT] - s.lo[RXMET_LSTM_OUTPUT]))) & 0xffffu;
@@ -209,6 +223,51 @@ struct LstmPlaneCell {
             if (ck.hidden_outputs) ck.hidden_outputs[o] = st.hidden + s.zpF[RXMET_LSTM_OUTPUT];
             if (ck.hidden_outputs_clamped) ck.hidden_outputs_clamped[o] = static_cast<uint8_t>((st.flags >> 2) & 1u);
         }
+    }
+    // The same for `count` of N consecutive rows: one address and one test per array.
+    template <int N>
+    __device__ __forceinline__ void storeRows(const State (&st)[N], size_t at, int row, int unit, bool good, int count) const {
+        const int H = hidden();
+        const size_t o = (at + static_cast<size_t>(row)) * H + unit;
+        auto put = [&](auto *to, auto value) {
+            if (to == nullptr) return;
+            to += o;
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+                if (i < count) to[static_cast<size_t>(i) * H] = value(st[i]);
+        };
+        const float scale = scaleH(good);
+        put(output, [&](const State &v) { return __fmul_rn(v.hidden, scale); });
+        if (!TRAIN) return;
+        const float zpCell = s.zpF[RXMET_LSTM_CELL_STATE], zpTanh = s.zpF[RXMET_LSTM_CELL_TANH_OUTPUT], zpHidden = s.zpF[RXMET_LSTM_OUTPUT];
+        put(ck.cell_states, [&](const State &v) { return v.cell + zpCell; });
+        put(ck.cell_states_clamped, [&](const State &v) { return static_cast<uint8_t>(v.flags & 1u); });
+        put(ck.cell_tanh_outputs, [&](const State &v) { return v.tanhC + zpTanh; });
+        put(ck.cell_tanh_outputs_clamped, [&](const State &v) { return static_cast<uint8_t>((v.flags >> 1) & 1u); });
+        put(ck.hidden_outputs, [&](const State &v) { return v.hidden + zpHidden; });
+        put(ck.hidden_outputs_clamped, [&](const State &v) { return static_cast<uint8_t>((v.flags >> 2) & 1u); });
+    }
+    template <int N>
+    __device__ __forceinline__ void storeLinearRows(const Lane &l, const Saved (&saved)[N], size_t at, int row, int gate, int unit, int count) const {
+        const int H = hidden();
+        const size_t o = (at + static_cast<size_t>(row)) * (4 * static_cast<size_t>(H)) + (gate * H + unit);
+        auto put = [&](auto *to, auto value) {
+            if (to == nullptr) return;
+            to += o;
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+                if (i < count) to[static_cast<size_t>(i) * (4 * H)] = value(saved[i]);
+        };
+        const float zpLinear = s.zpF[RXMET_LSTM_WEIGHT_HH_LINEAR];
+        put(ck.weight_hh_linear, [&](const Saved &v) { return v.hh + zpLinear; });
+        put(ck.weight_hh_linear_clamped, [&](const Saved &v) { return static_cast<uint8_t>(v.hhClamped); });
+        put(ck.gate_inputs, [&](const Saved &v) { return v.gateIn + l.zpIn; });
+        put(ck.gate_inputs_clamped, [&](const Saved &v) { return static_cast<uint8_t>(v.inClamped); });
+        put(ck.gate_outputs, [&](const Saved &v) { return v.gateOut + l.zpOut; });
+        put(ck.gate_outputs_clamped, [&](const Saved &v) {
+            const int index = static_cast<int>(v.index & 0x7fffffu);
+            return static_cast<uint8_t>(index < l.flagBelow || index >= l.flagFrom);
+        });
     }
     __device__ __forceinline__ void storeLinear(const Lane &l, const Saved &v, size_t at, uint32_t row, int gate, int unit) const {
         const int H = hidden();

@@ -864,7 +864,7 @@ WideLayout layoutWide(W &ws, int T, int B, int I, int H, int planes) {
     l.wHh = ws.template take<uint32_t>(kHh * C);
     l.addIh = ws.template take<int64_t>(C);
     l.addHh = ws.template take<int64_t>(C);
-    l.lhs = ws.template take<float>(rows * C);
+    l.lhs = ws.template take<float>((rows + 64) * C);   // the cluster recurrence reads on behind the last row
     l.ihTiles = ws.template take<uint4>(static_cast<size_t>(planeproj::paddedC(static_cast<int>(C))) * planeproj::paddedK(static_cast<int>(kIh)) / 16);
     l.projStatus = ws.template take<int>(1);
     l.hhTiles = ws.template take<uint4>(C * planeproj::paddedK(static_cast<int>(kHh)) / 16);

@@ -100,6 +100,12 @@ struct Problem {
 //   void begin(shared, State &, row, unit)                  state of one cell of phase B from h0
 //   void fetch(Fetch &, at, row, gate, unit), fetchB(FetchB &, at, row, unit)     operands of a step, asked for before the product is awaited
 //   uint32_t linear<STRIDE>(shared, Lane, Fetch, acc, Saved &)    phase A; plane p of the sum at acc[p STRIDE]
+//   kTotal                                                  whether it comes in two halves, totals<STRIDE, ROWS>(Lane, acc) and linearOfTotal, and
+//                                                           any operand is safe, also what lies up to 64 rows behind the last row: then
+//                                                           rows and units that do not exist are computed on like the others (no branch per
+//                                                           row keeps the rows of a thread interleaved) and only their stores are left out, by
+//                                                           storeRows(State[], at, row, unit, good, count) and storeLinearRows(Lane, Saved[], at, row, gate,
+//                                                           unit, count): the first `count` rows of the array
 //   uint32_t cell(shared, State &, FetchB, v[4])            phase B: new code - grid minimum
 //   void store<LANES>(State, FetchB, at, row, unit, good, part)   outputs of the step; good = false: make them NaN
 //   void storeLinear(Lane, Saved, at, row, gate, unit)      what phase A saves
@@ -204,8 +210,9 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
         // rows of phase A in one go: as many as the operator allows and the rows divide into
         constexpr int kChunk = G::kRowsA <= Cell::kChunk ? G::kRowsA : (G::kRowsA % Cell::kChunk == 0 ? Cell::kChunk : 4);
         constexpr bool kDefer = G::kRowsA == 4;   // more rows keep the epilogue busy by themselves; held back they would spill
+        constexpr bool kAll = Cell::kTotal && ROWS > 4;               // a cluster of four rows often has one or two: the others are left out
         const typename Cell::Lane mine = c.lane(shared, quarter, unit, real);
-        typename Cell::State state[G::kRowsB];
+        typename Cell::State state[G::kRowsB] = {};
 #pragma unroll
         for (int i = 0; i < G::kRowsB; ++i)
             if (real && rowB + i < p.B) c.begin(shared, state[i], rowB + i, unit);
@@ -215,23 +222,25 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
 #pragma unroll 1
         for (int t = 0; t < p.T; ++t) {
             const size_t at = static_cast<size_t>(t) * p.B;   // first row of the step in the [T][B] arrays
-            // Phase A walks its rows kChunk at a time in a rolled loop (the body of a step has to stay small for the instruction
-            // cache); the operands of the next chunk are asked for before the current ones are used.
-            typename Cell::Fetch in[kChunk];
+            // Phase A walks its rows kChunk at a time.  With kAll the operands of all of them are asked for before the product is
+            // awaited (a chunk is too short to hide a load: a training step of 24 rows took 7.2 us with a chunk's lead); else the loop
+            // is rolled and the operands of the next chunk are asked for before the current ones are used.
+            constexpr int kFetched = kAll ? G::kRowsA : kChunk, kUnroll = kAll ? G::kRowsA / kChunk : 1;
+            typename Cell::Fetch in[kFetched];
             typename Cell::FetchB inB[G::kRowsB];
-            auto fetchA = [&](typename Cell::Fetch (&to)[kChunk], int first) {
+            auto fetchA = [&](auto &to, int first, int count) {
 #pragma unroll
-                for (int r = 0; r < kChunk; ++r)
-                    if (real && rowA + first + r < p.B) c.fetch(to[r], at, rowA + first + r, quarter, unit);
+                for (int r = 0; r < count; ++r)
+                    if (kAll || (real && rowA + first + r < p.B)) c.fetch(to[r], at, rowA + first + r, quarter, unit);
             };
-            fetchA(in, 0);
+            fetchA(in, 0, kFetched);
 #pragma unroll
             for (int i = 0; i < G::kRowsB; ++i)
                 if (real && rowB + i < p.B) c.fetchB(inB[i], at, rowB + i, unit);
             wait(smemAddr(&productBar), t & 1);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             typename Cell::Saved saved[kChunk];
-#pragma unroll 1
+#pragma unroll kUnroll
             for (int first = 0; first < G::kRowsA; first += kChunk) {
                 uint32_t acc[PLANES * kChunk];
 #pragma unroll
@@ -239,20 +248,28 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
 #pragma unroll
                     for (int r = 0; r < kChunk; r += 4) tmemLoad4(column + pl * ROWS + first + r, acc + pl * kChunk + r);
                 typename Cell::Fetch later[kChunk];
-                if (first + kChunk < G::kRowsA) fetchA(later, first + kChunk);
+                if (!kAll && first + kChunk < G::kRowsA) fetchA(later, first + kChunk, kChunk);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (quarter < Cell::kGates) {
+                    if constexpr (kAll) {
+                        c.template totals<kChunk, kChunk>(mine, acc);
+#pragma unroll
+                        for (int r = 0; r < kChunk; ++r)
+                            exchangeTile[(quarter * G::kRowsA + first + r) * 32] = c.linearOfTotal(shared, mine, in[first + r], acc[r], saved[r]);
+                    } else
 #pragma unroll
                     for (int r = 0; r < kChunk; ++r)
                         if (rowA + first + r < p.B)
                             exchangeTile[(quarter * G::kRowsA + first + r) * 32] = c.template linear<kChunk>(shared, mine, in[r], acc + r, saved[r]);
-                    if (Cell::kSaves && !kDefer) {
+                    if constexpr (Cell::kSaves && !kDefer && kAll) {
+                        c.storeLinearRows(mine, saved, at, rowA + first, quarter, unit, real ? p.B - rowA - first : 0);
+                    } else if (Cell::kSaves && !kDefer) {
 #pragma unroll
                         for (int r = 0; r < kChunk; ++r)
                             if (real && rowA + first + r < p.B) c.storeLinear(mine, saved[r], at, rowA + first + r, quarter, unit);
                     }
                 }
-                if (G::kRowsA > kChunk) {
+                if (!kAll && G::kRowsA > kChunk) {
 #pragma unroll
                     for (int r = 0; r < kChunk; ++r) in[r] = later[r];
                 }
@@ -260,7 +277,8 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
             asm volatile("bar.sync %0, 128;" ::"r"(1 + (warp >> 2)) : "memory");   // the four quarters of this tile and row group
 #pragma unroll
             for (int i = 0; i < G::kRowsB; ++i) {
-                if (!real || rowB + i >= p.B) continue;
+                const bool exists = real && rowB + i < p.B;
+                if (!kAll && !exists) continue;
                 uint32_t v[4];
 #pragma unroll
                 for (int g = 0; g < 4; ++g) v[g] = g < Cell::kGates ? exchangeTile[(g * G::kRowsA + quarter * G::kRowsB + i) * 32] : 0u;
@@ -272,12 +290,18 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
                 } else {
                     dst[0] = static_cast<uint8_t>(u);
                 }
-                if (!kDefer) c.store(state[i], inB[i], at, rowB + i, unit, valid && alive && !failed);
+                if (!kDefer && !kAll && exists) c.store(state[i], inB[i], at, rowB + i, unit, valid && alive && !failed);
             }
+            if constexpr (!kDefer && kAll) c.storeRows(state, at, rowB, unit, valid && alive && !failed, real ? p.B - rowB : 0);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncthreads();
-            if (kDefer) {   // what nobody waits for leaves while the codes travel and the next product runs
+            if constexpr (kDefer && kAll) {   // what nobody waits for leaves while the codes travel and the next product runs
+                c.storeRows(state, at, rowB, unit, valid && alive && !failed, real ? p.B - rowB : 0);
+                if constexpr (Cell::kSaves) {
+                    if (quarter < Cell::kGates) c.storeLinearRows(mine, saved, at, rowA, quarter, unit, real ? p.B - rowA : 0);
+                }
+            } else if (kDefer) {
 #pragma unroll
                 for (int i = 0; i < G::kRowsB; ++i)
                     if (real && rowB + i < p.B) c.store(state[i], inB[i], at, rowB + i, unit, valid && alive && !failed);
