@@ -1162,7 +1162,7 @@ void backwardPadded(const BackwardCall &call, void *workspace, size_t workspaceB
     regroup("padBackward", out, 5, st);
 }
 
-size_t tiledWorkspaceBytes(int T, int B, int I, int H) {
+size_t tiledWorkspaceBytes(int T, int B, int I, int H, bool padded) {
     const size_t rows = static_cast<size_t>(T) * B, C = 3 * static_cast<size_t>(H);
     WorkspaceSizer ws;
     ws.take<float>(rows * C);          // dp
@@ -1181,10 +1181,10 @@ size_t tiledWorkspaceBytes(int T, int B, int I, int H) {
     ws.take<float>(2 * kBiasSplits * C);
     // tensor-core path: split-K partials of (I+1) and (H+1) rows and the status word
     // (the slab form of the same kernel, for more than 128 rows or 16-bit codes, asks for fewer splits)
-    ws.take<float>(static_cast<size_t>(std::max(wgrad::slabSplitBound(I, H, static_cast<int>(C)),
-                                                I <= 143 ? wgrad::splitBound(static_cast<int>(rows), I, static_cast<int>(C)) : 1)) * (I + 1) * C);
-    ws.take<float>(static_cast<size_t>(std::max(wgrad::slabSplitBound(I, H, static_cast<int>(C)),
-                                                H <= 143 ? wgrad::splitBound(static_cast<int>(rows), H, static_cast<int>(C)) : 1)) * (H + 1) * C);
+    ws.take<float>(static_cast<size_t>(std::max({padded ? wgrad::chainSplits(static_cast<int>(rows)) : 1, wgrad::slabSplitBound(I, H, static_cast<int>(C)),
+                                                I <= 143 ? wgrad::splitBound(static_cast<int>(rows), I, static_cast<int>(C)) : 1})) * (I + 1) * C);
+    ws.take<float>(static_cast<size_t>(std::max({padded ? wgrad::chainSplits(static_cast<int>(rows)) : 1, wgrad::slabSplitBound(I, H, static_cast<int>(C)),
+                                                H <= 143 ? wgrad::splitBound(static_cast<int>(rows), H, static_cast<int>(C)) : 1})) * (H + 1) * C);
     ws.take<int>(64);
     ws.take<float>(static_cast<size_t>(B) * H);   // gradient carried between time chunks
     ws.take<uint8_t>(igrad::widePackedBytes(static_cast<int>(C), I) + 256);   // weight operand of the streaming input-gradient kernel
@@ -1194,12 +1194,12 @@ size_t tiledWorkspaceBytes(int T, int B, int I, int H) {
 }  // namespace
 
 size_t backwardWorkspaceBytes(int T, int B, int I, int H) {
-    size_t bytes = tiledWorkspaceBytes(T, B, I, H);
+    size_t bytes = tiledWorkspaceBytes(T, B, I, H, false);
     if (H <= 256 && (tiledHidden(H) != H || tiledInput(I) != I)) {
         PaddedSizer sizer;
         layoutPadded(sizer, T, B, I, H);
         sizer.take<int32_t>(6 * static_cast<size_t>(H));
-        bytes = std::max(bytes, sizer.ws.used() + 512 + tiledWorkspaceBytes(T, B, tiledInput(I), tiledHidden(H)));
+        bytes = std::max(bytes, sizer.ws.used() + 512 + tiledWorkspaceBytes(T, B, tiledInput(I), tiledHidden(H), true));
     }
     return bytes;
 }
@@ -1528,7 +1528,10 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         // the two problems share one launch of one CTA per SM: each is planned for half of the SMs, so that the
         // launch is a single wave (RXMET_WGRAD_FULL_SPLIT plans each for all SMs, two waves)
         const int planSms = std::getenv("RXMET_WGRAD_FULL_SPLIT") ? sms : std::max(1, sms / 2);
-        const wgrad::Plan planX = wgrad::plan(K, I, C, planSms), planH = wgrad::plan(K, H, C, planSms);
+        wgrad::Plan planX = wgrad::plan(K, I, C, planSms), planH = wgrad::plan(K, H, C, planSms);
+        if (call.dxColumns)   // backwardPadded: as exact as the FP32 kernels that the caller's widths would take
+            for (wgrad::Plan *pl : {&planX, &planH})
+                if (pl->tensorMemory) wgrad::boundChain(K, &pl->chunkK, &pl->splits);
         WeightGradProblem px{}, ph{};
         px.aCodes = call.x_q; px.aZero = e.gate.zp[RXMET_GRU_X]; px.M = I; px.B = dp;
         px.partial = ws.take<float>(static_cast<size_t>(planX.splits) * (I + 1) * C);
@@ -1552,7 +1555,8 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         const Exec &e = *call.exec;
         const int K = static_cast<int>(rows);
         int chunkK = 0;
-        const int splits = wgrad::slabSplits(K, I, H, C, sms, &chunkK);
+        int splits = wgrad::slabSplits(K, I, H, C, sms, &chunkK);
+        if (call.dxColumns) wgrad::boundChain(K, &chunkK, &splits);   // as above
         WeightGradProblem px{}, ph{};
         px.aCodes = call.x_q; px.aZero = e.gate.zp[RXMET_GRU_X]; px.M = I; px.B = dp;
         px.partial = ws.take<float>(static_cast<size_t>(splits) * (I + 1) * C);

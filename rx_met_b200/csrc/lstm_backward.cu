@@ -593,9 +593,9 @@ constexpr int kMaxTensorSplits = 40;
 
 // Splits of the tensor-core weight-gradient partial arrays: the one-tile plan for at most 128 rows, the slab plan
 // (128-row slabs of both problems in one launch) beyond.
-int tensorSplitBound(int rows, int I, int H, int M, int C) {
+int tensorSplitBound(int rows, int I, int H, int M, int C, bool padded) {
     const int single = M <= 143 ? wgrad::splitBound(rows, M, C) : 1;
-    return std::max(single, wgrad::slabPathTakes(I, H, C) ? wgrad::slabSplitBound(I, H, C) : 1);
+    return std::max({single, padded ? wgrad::chainSplits(rows) : 1, wgrad::slabPathTakes(I, H, C) ? wgrad::slabSplitBound(I, H, C) : 1});
 }
 
 namespace {
@@ -712,7 +712,7 @@ void backwardPadded(const BackwardCall &call, void *workspace, size_t workspaceB
     regroup("lstmPadBackward", out, 6, st);
 }
 
-size_t tiledWorkspaceBytes(int T, int B, int I, int H) {
+size_t tiledWorkspaceBytes(int T, int B, int I, int H, bool padded) {
     const size_t rows = static_cast<size_t>(T) * B, C = 4 * static_cast<size_t>(H);
     WorkspaceSizer ws;
     ws.take<float>(rows * C);  // G_ih
@@ -723,8 +723,8 @@ size_t tiledWorkspaceBytes(int T, int B, int I, int H) {
     ws.take<float>(static_cast<size_t>(splitsFor(static_cast<int>(rows), tilesOf(static_cast<int>(C), H))) * C * H);
     ws.take<float>(2 * kBiasSplits * C);
     ws.take<float>(rows * H);  // h_prev codes for the tensor-core weight gradient (QAT)
-    ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, I, static_cast<int>(C))) * (I + 1) * C);
-    ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, H, static_cast<int>(C))) * (H + 1) * C);
+    ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, I, static_cast<int>(C), padded)) * (I + 1) * C);
+    ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, H, static_cast<int>(C), padded)) * (H + 1) * C);
     ws.take<int>(1);              // status word of the tensor-memory weight-gradient kernel
     ws.take<uint32_t>(rows * H);  // packed per-step clamp flags
     ws.take<uint8_t>(igrad::widePackedBytes(static_cast<int>(C), I) + 256);   // weight operand of the streaming input-gradient kernel
@@ -734,11 +734,11 @@ size_t tiledWorkspaceBytes(int T, int B, int I, int H) {
 }  // namespace
 
 size_t backwardWorkspaceBytes(int T, int B, int I, int H) {
-    size_t bytes = tiledWorkspaceBytes(T, B, I, H);
+    size_t bytes = tiledWorkspaceBytes(T, B, I, H, false);
     if (H <= 512 && (tiledHidden(H) != H || tiledInput(I) != I)) {
         PaddedSizer sizer;
         layoutPadded(sizer, T, B, I, H);
-        bytes = std::max(bytes, sizer.ws.used() + 512 + tiledWorkspaceBytes(T, B, tiledInput(I), tiledHidden(H)));
+        bytes = std::max(bytes, sizer.ws.used() + 512 + tiledWorkspaceBytes(T, B, tiledInput(I), tiledHidden(H), true));
     }
     return bytes;
 }
@@ -760,9 +760,10 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
     float *partHh = ws.take<float>(static_cast<size_t>(splitHh) * C * H);
     float *partBias = ws.take<float>(2 * kBiasSplits * static_cast<size_t>(C));
     const float *channelScales = call.channelScales;   // weight_ih, weight_hh
+    const bool padded = call.dxColumns != 0;   // backwardPadded: as exact as the FP32 kernels that the caller's widths would take
     float *hPrev = ws.take<float>(rows * H);
-    float *tensorIh = ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, I, C)) * (I + 1) * C);
-    float *tensorHh = ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, H, C)) * (H + 1) * C);
+    float *tensorIh = ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, I, C, padded)) * (I + 1) * C);
+    float *tensorHh = ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, H, C, padded)) * (H + 1) * C);
     int *tensorStatus = ws.take<int>(1);
     uint32_t *stepMasks = ws.take<uint32_t>(rows * H);
 
@@ -931,6 +932,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
                 pl.chunkK = ((static_cast<int>(rows) + kMaxTensorSplits - 1) / kMaxTensorSplits + 31) / 32 * 32;
                 pl.splits = (static_cast<int>(rows) + pl.chunkK - 1) / pl.chunkK;
             }
+            if (padded && pl.tensorMemory) wgrad::boundChain(static_cast<int>(rows), &pl.chunkK, &pl.splits);
             return pl;
         };
         const wgrad::Plan planX = planFor(I), planH = planFor(H);
@@ -968,7 +970,8 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
             RXMET_CUDA(cudaMemcpyAsync(hPrev + static_cast<size_t>(B) * H, call.hiddenOutputs, stateBytes * (T - 1),
                                        cudaMemcpyDeviceToDevice, st));
         int chunkK = 0;
-        const int splits = wgrad::slabSplits(static_cast<int>(rows), I, H, C, currentDevice().sms, &chunkK);
+        int splits = wgrad::slabSplits(static_cast<int>(rows), I, H, C, currentDevice().sms, &chunkK);
+        if (padded) wgrad::boundChain(static_cast<int>(rows), &chunkK, &splits);
         wgrad::Problem px{}, ph{};
         px.aFloat = call.x; px.aFloatZero = call.dqX.zeroPoint; px.M = I; px.B = gIh; px.partial = tensorIh;
         ph.aFloat = hPrev; ph.aFloatZero = call.h0 ? call.dqH.zeroPoint : 0.0f; ph.M = H; ph.B = gHh; ph.partial = tensorHh;
