@@ -51,8 +51,8 @@ __device__ __forceinline__ float lookup(const TableView &v, int segShift, float 
 template <bool TRAIN, int WIDTH = 0>
 struct LstmPlaneCell {
     static constexpr int kGates = 4;
-    static constexpr bool kSaves = TRAIN, kFull = WIDTH != 0, kTotal = true;
-    static constexpr int kChunk = TRAIN ? 4 : 16;
+    static constexpr bool kSaves = TRAIN, kFull = WIDTH != 0;
+    static constexpr int kChunk = TRAIN ? 4 : 16, kTotalFrom = 8;
     ScalarExec s;
     int width, kWords;
     __device__ __forceinline__ int hidden() const { return WIDTH ? WIDTH : width; }
@@ -150,7 +150,12 @@ struct LstmPlaneCell {
         st.hidden = st.tanhC = 0.0f;
         st.flags = 0;
     }
-    __device__ __forceinline__ void fetch(Fetch &f, size_t at, int row, int gate, int unit) const {
+    __device__ __forceinline__ void fetch(Fetch &f, size_t at, uint32_t row, int gate, int unit) const {
+        const int H = hidden();
+        f.lhs = __ldg(lhs + at * (4 * static_cast<size_t>(H)) + (row * (4 * H) + gate * H + unit));
+    }
+    // the same for the rows of a thread: 64 bits all along, so that the rows are immediates of one address
+    __device__ __forceinline__ void fetchRow(Fetch &f, size_t at, int row, int gate, int unit) const {
         const int H = hidden();
         f.lhs = __ldg(lhs + (at + static_cast<size_t>(row)) * (4 * static_cast<size_t>(H)) + (gate * H + unit));
     }
@@ -226,7 +231,7 @@ struct LstmPlaneCell {
     }
     // The same for `count` of N consecutive rows: one address and one test per array.
     template <int N>
-    __device__ __forceinline__ void storeRows(const State (&st)[N], size_t at, int row, int unit, bool good, int count) const {
+    __device__ __forceinline__ void storeRows(const State (&st)[N], const FetchB (&)[N], size_t at, int row, int unit, bool good, int count) const {
         const int H = hidden();
         const size_t o = (at + static_cast<size_t>(row)) * H + unit;
         auto put = [&](auto *to, auto value) {
@@ -288,13 +293,7 @@ struct LstmPlaneCell {
     }
 };
 
-// Rows: a step of n rows costs about 1 + n / 5 of the chain of a one-row step.  48 only without a training forward's stores, whose
-// sixteen warps do not divide them.
-template <class Cell, int HP>
-void launchRows(const planerec::Problem &p, const Cell &cell, cudaStream_t st) {
-    if constexpr (Cell::kSaves) planerec::launchBest<Cell, HP, 64, 2, 5, 4, 8, 12, 16, 24, 32>("lstmRecurrentWide", p, cell, st);
-    else planerec::launchBest<Cell, HP, 64, 2, 5, 4, 8, 12, 16, 24, 32, 48>("lstmRecurrentWide", p, cell, st);
-}
+// Rows: a step of n rows costs about 1 + n / 5 of the chain of a one-row step.
 template <bool TRAIN, int HP>
 void launchLstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &cell, cudaStream_t st) {
     if constexpr (HP <= 128)
@@ -305,9 +304,9 @@ void launchLstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &c
         std::memcpy(&full, &cell, sizeof(full));
         if constexpr (HP <= 128)
             if (lanerec::launch<LstmPlaneCell<TRAIN, HP>, HP / 4, 2>("lstmRecurrentWide", p, full, st)) return;
-        launchRows<LstmPlaneCell<TRAIN, HP>, HP>(p, full, st);
+        planerec::launchBest<LstmPlaneCell<TRAIN, HP>, HP, 64, 2, 5, 4, 8, 12, 16, 24, 32, 48>("lstmRecurrentWide", p, full, st);
     } else {
-        launchRows<LstmPlaneCell<TRAIN>, HP>(p, cell, st);
+        planerec::launchBest<LstmPlaneCell<TRAIN>, HP, 64, 2, 5, 4, 8, 12, 16, 24, 32, 48>("lstmRecurrentWide", p, cell, st);
     }
 }
 // 8-bit inference, at most 128 units, rows that one wave of CTAs holds (lanerec::rowsFor): the same cell on one byte plane.

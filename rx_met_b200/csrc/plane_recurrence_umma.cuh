@@ -59,13 +59,12 @@ constexpr uint32_t powerOfTwoFrom(uint32_t n) {
     return p;
 }
 
-template <int HP, int U, int ROWS, int PLANES, bool SAVES>
+template <int HP, int U, int ROWS, int PLANES>
 struct Geometry {
     static constexpr int kCtas = HP / U, kTiles = U / 32;
-    // Warps of the epilogue; one more issues products and copies.  Three row groups instead of two hide more of the table
-    // look-ups (LSTM, H = 512, 24 rows: 4.5 -> 4.1 us per step); with a training forward's stores they lose (7.6 -> 9.5 us), except
-    // that twelve rows need them.
-    static constexpr int kWarps = ROWS * kTiles < 16 ? 8 : kTiles == 2 && (ROWS == 12 || (ROWS % 24 == 0 && !SAVES)) ? 24 : 16;
+    // Warps of the epilogue; one more issues products and copies.  Three row groups where they divide the rows: they hide more of
+    // the table look-ups than two (LSTM inference, H = 512, 24 rows: 4.5 -> 4.1 us per step).
+    static constexpr int kWarps = ROWS * kTiles < 16 ? 8 : kTiles == 2 && ROWS % 12 == 0 ? 24 : 16;
     static constexpr int kThreads = 32 * (kWarps + 1);
     static constexpr int kRowGroups = kWarps / (4 * kTiles);   // warps that share the rows of a tile's quarter
     static constexpr int kRowsA = ROWS / kRowGroups;            // rows of a lane in phase A
@@ -100,20 +99,21 @@ struct Problem {
 //   void begin(shared, State &, row, unit)                  state of one cell of phase B from h0
 //   void fetch(Fetch &, at, row, gate, unit), fetchB(FetchB &, at, row, unit)     operands of a step, asked for before the product is awaited
 //   uint32_t linear<STRIDE>(shared, Lane, Fetch, acc, Saved &)    phase A; plane p of the sum at acc[p STRIDE]
-//   kTotal                                                  whether it comes in two halves, totals<STRIDE, ROWS>(Lane, acc) and linearOfTotal, and
-//                                                           any operand is safe, also what lies up to 64 rows behind the last row: then
-//                                                           rows and units that do not exist are computed on like the others (no branch per
-//                                                           row keeps the rows of a thread interleaved) and only their stores are left out, by
-//                                                           storeRows(State[], at, row, unit, good, count) and storeLinearRows(Lane, Saved[], at, row, gate,
-//                                                           unit, count): the first `count` rows of the array
+//   kTotalFrom                                              rows of a cluster from which a step leaves no row out: the linear stage comes in two
+//                                                           halves then, totals<STRIDE, ROWS>(Lane, acc) and linearOfTotal, with fetchRow for fetch,
+//                                                           and has to be safe with any operand, also with what lies up to 64 rows behind the last row.
+//                                                           Rows and units that do not exist are computed like the others - without a branch per row
+//                                                           the rows of a thread interleave - and only their stores are left out, by
+//                                                           storeRows(State[], FetchB[], at, row, unit, good, count) and storeLinearRows(Lane, Saved[],
+//                                                           at, row, gate, unit, count): the first `count` rows of the array
 //   uint32_t cell(shared, State &, FetchB, v[4])            phase B: new code - grid minimum
 //   void store<LANES>(State, FetchB, at, row, unit, good, part)   outputs of the step; good = false: make them NaN
 //   void storeLinear(Lane, Saved, at, row, gate, unit)      what phase A saves
 //   void finish(State, row, unit, good)                     after the last step
 template <class Cell, int HP, int U, int ROWS, int PLANES>
-__global__ void __launch_bounds__(Geometry<HP, U, ROWS, PLANES, Cell::kSaves>::kThreads, 1)
+__global__ void __launch_bounds__(Geometry<HP, U, ROWS, PLANES>::kThreads, 1)
 planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c) {
-    using G = Geometry<HP, U, ROWS, PLANES, Cell::kSaves>;
+    using G = Geometry<HP, U, ROWS, PLANES>;
     constexpr int MT = G::kTiles, NC = G::kCtas;
     extern __shared__ __align__(128) uint8_t smemR[];
     __shared__ __align__(8) uint64_t productBar, codeBar[2];
@@ -210,7 +210,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
         // rows of phase A in one go: as many as the operator allows and the rows divide into
         constexpr int kChunk = G::kRowsA <= Cell::kChunk ? G::kRowsA : (G::kRowsA % Cell::kChunk == 0 ? Cell::kChunk : 4);
         constexpr bool kDefer = G::kRowsA == 4;   // more rows keep the epilogue busy by themselves; held back they would spill
-        constexpr bool kAll = Cell::kTotal && ROWS > 4;               // a cluster of four rows often has one or two: the others are left out
+        constexpr bool kAll = ROWS >= Cell::kTotalFrom;
         const typename Cell::Lane mine = c.lane(shared, quarter, unit, real);
         typename Cell::State state[G::kRowsB] = {};
 #pragma unroll
@@ -228,10 +228,13 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
             constexpr int kFetched = kAll ? G::kRowsA : kChunk, kUnroll = kAll ? G::kRowsA / kChunk : 1;
             typename Cell::Fetch in[kFetched];
             typename Cell::FetchB inB[G::kRowsB];
+            if constexpr (kAll)
+                for (int i = 0; i < G::kRowsB; ++i) inB[i] = {};
             auto fetchA = [&](auto &to, int first, int count) {
 #pragma unroll
                 for (int r = 0; r < count; ++r)
-                    if (kAll || (real && rowA + first + r < p.B)) c.fetch(to[r], at, rowA + first + r, quarter, unit);
+                    if constexpr (kAll) c.fetchRow(to[r], at, rowA + first + r, quarter, unit);
+                    else if (real && rowA + first + r < p.B) c.fetch(to[r], at, rowA + first + r, quarter, unit);
             };
             fetchA(in, 0, kFetched);
 #pragma unroll
@@ -292,12 +295,12 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
                 }
                 if (!kDefer && !kAll && exists) c.store(state[i], inB[i], at, rowB + i, unit, valid && alive && !failed);
             }
-            if constexpr (!kDefer && kAll) c.storeRows(state, at, rowB, unit, valid && alive && !failed, real ? p.B - rowB : 0);
+            if constexpr (!kDefer && kAll) c.storeRows(state, inB, at, rowB, unit, valid && alive && !failed, real ? p.B - rowB : 0);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncthreads();
             if constexpr (kDefer && kAll) {   // what nobody waits for leaves while the codes travel and the next product runs
-                c.storeRows(state, at, rowB, unit, valid && alive && !failed, real ? p.B - rowB : 0);
+                c.storeRows(state, inB, at, rowB, unit, valid && alive && !failed, real ? p.B - rowB : 0);
                 if constexpr (Cell::kSaves) {
                     if (quarter < Cell::kGates) c.storeLinearRows(mine, saved, at, rowA, quarter, unit, real ? p.B - rowA : 0);
                 }
@@ -325,7 +328,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
 // Launches a variant with its clusters.
 template <class Cell, int HP, int U, int ROWS, int PLANES>
 void launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t st) {
-    using G = Geometry<HP, U, ROWS, PLANES, Cell::kSaves>;
+    using G = Geometry<HP, U, ROWS, PLANES>;
     const auto kernel = planeRecurrence<Cell, HP, U, ROWS, PLANES>;
     const size_t smem = G::kSharedBytes + cell.sharedBytes();
     ensureDynamicSmem(reinterpret_cast<const void *>(kernel), smem);
@@ -356,7 +359,7 @@ void launchBest(const char *name, const Problem &p, const Cell &cell, cudaStream
     int best = 0;
     (
         [&] {
-            using G = Geometry<HP, U, ROWS, PLANES, Cell::kSaves>;
+            using G = Geometry<HP, U, ROWS, PLANES>;
             if (G::kSharedBytes + cell.sharedBytes() > static_cast<size_t>(currentDevice().smemMax)) return;
             const int resident = std::max(1, residentClusters(reinterpret_cast<const void *>(planeRecurrence<Cell, HP, U, ROWS, PLANES>), G::kCtas,
                                                               G::kThreads, G::kSharedBytes + cell.sharedBytes()) / concurrentPasses());
