@@ -374,6 +374,7 @@ void backwardCluster(const BackwardQArgs &q, const int32_t *Rq, cudaStream_t st)
     int best = 4;
     double bestCost = 1e30;
     for (int rows : {4, 8, 16}) {
+        if (1.0 + rows / 32.0 >= bestCost) break;   // not even in a single wave: leave the variant unloaded
         const Variant v = variantFor(q.H, rows);
         const int resident = std::max(1, residentClusters(reinterpret_cast<const void *>(v.kernel), v.ctas, kThreads, v.smem) / concurrentPasses());
         const int clusters = (q.B + rows - 1) / rows, waves = (clusters + resident - 1) / resident;

@@ -44,7 +44,7 @@ bool backwardClusterTakes(const BackwardClusterArgs &a) {
                           static_cast<const void *>(a.dc0), static_cast<const void *>(a.gIh), static_cast<const void *>(a.gHh),
                           static_cast<const void *>(a.channelScale), static_cast<const void *>(a.stepMasks)})
         if (!alignedTo(p, 8)) return false;
-    return a.H % 32 == 0 && a.H >= 32 && a.H <= 512 && a.c0 != nullptr && (a.H <= 256 || resident(variantFor(a.H, 16)) > 0);
+    return a.H % 32 == 0 && a.H >= 32 && a.H <= 512 && a.c0 != nullptr && (a.H <= 256 || resident(variantFor(a.H, 4)) > 0);
 }
 
 void backwardCluster(const BackwardClusterArgs &args, cudaStream_t st) {
@@ -53,7 +53,9 @@ void backwardCluster(const BackwardClusterArgs &args, cudaStream_t st) {
     int best = 4;
     double bestCost = 1e30;
     for (int rows : {4, 8, 16}) {
+        if (1.0 + rows / 32.0 >= bestCost) break;   // not even in a single wave: leave the variant unloaded
         const Variant v = variantFor(args.H, rows);
+        if (rows > 4 && resident(v) == 0) continue;
         const int held = std::max(1, resident(v) / concurrentPasses());
         const int clusters = (args.B + rows - 1) / rows, waves = (clusters + held - 1) / held;
         const double cost = waves * (1.0 + rows / 32.0);

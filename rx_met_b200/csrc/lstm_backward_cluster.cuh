@@ -203,6 +203,19 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
     // role in the product's read-out: a warp carries tiles of 32 units, up to two, and kSpan of the rows of each
     constexpr int kSpan = MT == 1 ? ROWS / 2 : ROWS, kReadouts = (MT + 1) / 2;
     const int quarter = warp & 3, row0 = MT == 1 ? (warp >> 2) * kSpan : 0;
+    uint32_t column[kReadouts], sendTo[kReadouts], sendBar[kReadouts];
+    float *outMine[kReadouts];
+    bool tileReal[kReadouts];
+#pragma unroll
+    for (int i = 0; i < kReadouts; ++i) {
+        const int tile = MT == 1 ? 0 : (warp >> 2) + 2 * i, unit0 = tile * 128 + 32 * quarter;
+        tileReal[i] = unit0 < H;
+        column[i] = tmem + (static_cast<uint32_t>(32 * quarter) << 16) + static_cast<uint32_t>(tile * G::kCols + row0);
+        const uint32_t owner = min(static_cast<uint32_t>(unit0) / U, static_cast<uint32_t>(NC - 1));
+        sendTo[i] = cluster::remote(smemAddr(part), owner) + ((rank * U + static_cast<uint32_t>(unit0) % U) * ROWS + row0 * 32) * 4;
+        sendBar[i] = cluster::remote(smemAddr(&partBar[0]), owner);
+        outMine[i] = outS + (tileReal[i] ? unit0 : 0) * ROWS + row0 * 32 + lane;
+    }
 
     Factors fx[RPT], fy[RPT];
     // the next step's factors from ring slot `slot`
@@ -294,31 +307,24 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
         // partial sums -> the CTAs that own the units
 #pragma unroll
         for (int i = 0; i < kReadouts; ++i) {
-            const int tile = MT == 1 ? 0 : (warp >> 2) + 2 * i, unit0 = tile * 128 + 32 * quarter;
+            if (!tileReal[i]) continue;
             wait(smemAddr(&productBar[i]), n & 1);
-            if (unit0 >= H) continue;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             constexpr int kLoad = kSpan < 8 ? kSpan : 8;
-            const uint32_t column = tmem + (static_cast<uint32_t>(32 * quarter) << 16) + static_cast<uint32_t>(tile * G::kCols + row0);
-            float *out = outS + (n & 1) * (ROWS * H) + unit0 * ROWS + row0 * 32;
+            float *out = outMine[i] + (n & 1) * (ROWS * H);
 #pragma unroll
             for (int r = 0; r < kSpan; r += kLoad) {
                 uint32_t v[3][kLoad];
 #pragma unroll
-                for (int term = 0; term < 3; ++term) tmemLoad<kLoad>(column + term * ROWS + r, v[term]);
+                for (int term = 0; term < 3; ++term) tmemLoad<kLoad>(column[i] + term * ROWS + r, v[term]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                 for (int e = 0; e < kLoad; ++e)
-                    out[(r + e) * 32 + lane] = (__uint_as_float(v[2][e]) + __uint_as_float(v[1][e])) + __uint_as_float(v[0][e]);
+                    out[(r + e) * 32] = (__uint_as_float(v[2][e]) + __uint_as_float(v[1][e])) + __uint_as_float(v[0][e]);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) {
-                const uint32_t owner = static_cast<uint32_t>(unit0) / U;
-                const uint32_t sendTo = cluster::remote(smemAddr(part), owner) + ((rank * U + static_cast<uint32_t>(unit0) % U) * ROWS + row0 * 32) * 4;
-                cluster::copyTo(sendTo + (n & 1) * G::kPartBytes, smemAddr(out), kSpan * 128,
-                                cluster::remote(smemAddr(&partBar[0]), owner) + (n & 1) * 8);
-            }
+            if (lane == 0) cluster::copyTo(sendTo[i] + (n & 1) * G::kPartBytes, smemAddr(out), kSpan * 128, sendBar[i] + (n & 1) * 8);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         if (n + 3 < a.T) fetch(a.T - 1 - (n + 3), slot);   // while the partial sums travel

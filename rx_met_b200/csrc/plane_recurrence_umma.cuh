@@ -360,7 +360,8 @@ void launchBest(const char *name, const Problem &p, const Cell &cell, cudaStream
     (
         [&] {
             using G = Geometry<HP, U, ROWS, PLANES>;
-            if (G::kSharedBytes + cell.sharedBytes() > static_cast<size_t>(currentDevice().smemMax)) return;
+            // a single wave of it would not beat what is found already: do not even load the variant
+            if (1.0 + ROWS / static_cast<double>(PER) >= bestCost || G::kSharedBytes + cell.sharedBytes() > static_cast<size_t>(currentDevice().smemMax)) return;
             const int resident = std::max(1, residentClusters(reinterpret_cast<const void *>(planeRecurrence<Cell, HP, U, ROWS, PLANES>), G::kCtas,
                                                               G::kThreads, G::kSharedBytes + cell.sharedBytes()) / concurrentPasses());
             const int clusters = (p.B + ROWS - 1) / ROWS, waves = (clusters + resident - 1) / resident;
