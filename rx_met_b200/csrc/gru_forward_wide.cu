@@ -298,6 +298,7 @@ recurrentPlanes(const __grid_constant__ RecurrentArgs a, const __grid_constant__
 // Epilogue of the tensor-core input projection: exact 64-bit sum of the two planes and the addend, the
 // rounding rescale onto the linear-output grid, clamp, code and keep flag.
 struct PlaneEpilogue {
+    static constexpr bool kTakesRows = false;
     const int64_t *addend;
     const Rescale *rescale;
     int32_t zpOut, lo, hi;

@@ -823,32 +823,74 @@ struct WideLayout {
 
 // Epilogue of the tensor-core input projection: the exact sum of the planes and the addend rounded once to
 // float, then the reference's float rescale, clamp and gate-grid rescale (the same lines as inputLinearWide).
+//
+// Bound by issue and by the conversion pipe, a quarter as wide as the others: a 64-bit sum to float and two rint took half of it.
+// Where the sums of a warp's channels provably fit 32 bits and the gate-grid values 2^22 (both from the grids alone), a value
+// costs one conversion, rounding adds and subtracts 1.5 * 2^23, multiplier and power of two are one factor (the same value),
+// and sixteen rows share their addresses and tests.  T = 1000, B = 4096, H = 512: the pass 59.4 -> 57.0 ms.
 template <int PLANES>
 struct WidePlaneEpilogue {
+    static constexpr bool kTakesRows = true;
     const int64_t *addend;
     const float *fields;     // the per-channel float block (kChannelFields x 4H)
     ScalarExec s;
-    int H;
+    int H, I;
     float *lhs, *linear;
     uint8_t *linearClamped;
     struct Channel {
         int64_t addend;
         DevRescale out, toGate;
+        bool small;   // warp-uniform
     };
+    __device__ float lowest() const { return static_cast<float>(s.lo[RXMET_LSTM_WEIGHT_IH_LINEAR] - s.zp[RXMET_LSTM_WEIGHT_IH_LINEAR]); }
+    __device__ float highest() const { return static_cast<float>(s.hi[RXMET_LSTM_WEIGHT_IH_LINEAR] - s.zp[RXMET_LSTM_WEIGHT_IH_LINEAR]); }
     __device__ Channel channel(int c) const {
         const size_t C = 4 * static_cast<size_t>(H);
-        return Channel{addend[c], DevRescale{fields[static_cast<size_t>(kIhOutMult) * C + c], fields[static_cast<size_t>(kIhOutPow2) * C + c]},
-                       s.ihToGate[c / H]};
+        Channel ch{addend[c], DevRescale{fields[static_cast<size_t>(kIhOutMult) * C + c], fields[static_cast<size_t>(kIhOutPow2) * C + c]},
+                   s.ihToGate[c / H], false};
+        const int64_t wMax = max(-static_cast<int64_t>(s.lo[RXMET_LSTM_WEIGHT_IH]), static_cast<int64_t>(s.hi[RXMET_LSTM_WEIGHT_IH]));
+        const float most = fmaxf(fabsf(lowest()), fabsf(highest())) + 1.0f;
+        ch.small = __all_sync(0xffffffffu, wMax * (PLANES == 2 ? 65535 : 255) * I + llabs(ch.addend) < (int64_t{1} << 31) && most < 4194304.0f &&
+                                               most * (ch.toGate.mult * ch.toGate.pow2) < 4194304.0f);
+        return ch;
     }
     __device__ void store(const Channel &ch, size_t row, int c, const int32_t (&acc)[PLANES]) const {
         const int op = RXMET_LSTM_WEIGHT_IH_LINEAR;
-        const float cLo = static_cast<float>(s.lo[op] - s.zp[op]), cHi = static_cast<float>(s.hi[op] - s.zp[op]);
         uint8_t m;
-        const float cen = linearCentredF(combine<PLANES>(acc, ch.addend), ch.out, cLo, cHi, m);
+        const float cen = linearCentredF(combine<PLANES>(acc, ch.addend), ch.out, lowest(), highest(), m);
         const size_t o = row * (4 * static_cast<size_t>(H)) + c;
         lhs[o] = rescaleF(cen, ch.toGate);
         if (linear) linear[o] = cen + s.zpF[op];
         if (linearClamped) linearClamped[o] = m;
+    }
+    // `count` rows of N; small channels only
+    template <int N>
+    __device__ void storeRows(const Channel &ch, size_t row, int c, const uint32_t (&acc)[PLANES][N], int count) const {
+        const float lo = lowest(), hi = highest(), scale = __fmul_rn(ch.out.mult, ch.out.pow2), gate = __fmul_rn(ch.toGate.mult, ch.toGate.pow2);
+        const uint32_t plus = static_cast<uint32_t>(ch.addend);
+        auto rounded = [](float v) { return __fadd_rn(__fadd_rn(v, 12582912.0f), -12582912.0f); };
+        float r[N];   // one step beyond the grid where it clamps
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const uint32_t sum = (PLANES == 2 ? acc[0][j] * 256u + acc[PLANES - 1][j] : acc[0][j]) + plus;
+            r[j] = rounded(fminf(fmaxf(__fmul_rn(__int2float_rn(static_cast<int32_t>(sum)), scale), lo - 1.0f), hi + 1.0f));
+        }
+        const size_t C = 4 * static_cast<size_t>(H), o = row * C + c;
+        auto centred = [&](int j) { return fminf(fmaxf(r[j], lo), hi); };
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (j < count) lhs[o + j * C] = rounded(__fmul_rn(centred(j), gate));
+        if (linear) {
+            const float zp = s.zpF[RXMET_LSTM_WEIGHT_IH_LINEAR];
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+                if (j < count) linear[o + j * C] = centred(j) + zp;
+        }
+        if (linearClamped) {
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+                if (j < count) linearClamped[o + j * C] = (r[j] < lo || r[j] > hi) ? 1 : 0;
+        }
     }
 };
 
@@ -1005,7 +1047,7 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
         const int rowTiles = static_cast<int>((rows + rowsPerTile - 1) / rowsPerTile);
         const int grid = std::max(1, std::min(rowTiles, smsPerPass()));
         auto launchTensor = [&](auto kernel, auto epi) {
-            epi.addend = l.addIh; epi.fields = l.channel; epi.s = s; epi.H = H; epi.lhs = l.lhs;
+            epi.addend = l.addIh; epi.fields = l.channel; epi.s = s; epi.H = H; epi.I = I; epi.lhs = l.lhs;
             epi.linear = ck.weight_ih_linear; epi.linearClamped = ck.weight_ih_linear_clamped;
             ensureDynamicSmem(reinterpret_cast<const void *>(kernel), smem);
             KernelTimer timer__("lstmInputLinearWide", st);

@@ -90,6 +90,7 @@ static __global__ void packTiles(const uint32_t *__restrict__ words, int kWords,
 //   struct Channel;                                        per-channel constants
 //   __device__ Channel channel(int c) const;
 //   __device__ void store(const Channel &, size_t row, int c, const int32_t (&acc)[PLANES]) const;
+//   kTakesRows: also storeRows<N>(Channel, row, c, acc[PLANES][N], count), for channels with Channel::small (warp-uniform)
 template <class Epilogue, int PLANES, int NR>
 __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const Problem p, const Epilogue epi) {
     constexpr uint32_t kBufCols = PLANES * NR;
@@ -151,6 +152,12 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const Problem p, co
             }
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             const int row0 = rowTile * NR + 16 * chunk;
+            if constexpr (Epilogue::kTakesRows) {
+                if (ch.small) {
+                    epi.template storeRows<16>(ch, static_cast<size_t>(row0), c, acc, real ? p.rows - row0 : 0);
+                    continue;
+                }
+            }
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 if (row0 + j >= p.rows) break;

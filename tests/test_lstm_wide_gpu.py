@@ -169,3 +169,9 @@ def test_wide_qat_backward_over_clusters_and_padded_widths(T, B, I, H, wb, ab):
 def test_wide_forward_at_the_row_counts_of_a_cluster(B):
     """Twelve, sixteen or 24, 24 and 48 rows of a cluster, two or three groups of warps over them, a partial last tile of units."""
     test_wide_forward_is_bit_exact(2, B, 8, 500, 4, 16, L.PER_CHANNEL, True, True)
+
+
+@pytest.mark.parametrize("T,B,I,H,wb,ab", [(2, 3, 256, 64, 8, 16), (3, 43, 5, 33, 4, 12), (1, 1, 37, 65, 8, 9)])
+def test_wide_projection_beside_32_bit_sums(T, B, I, H, wb, ab):
+    """Sums of the input projection that may leave 32 bits (W8, A16, 256 inputs) and such that cannot, ragged rows and channels."""
+    test_wide_forward_is_bit_exact(T, B, I, H, wb, ab, L.PER_CHANNEL, True, True)
