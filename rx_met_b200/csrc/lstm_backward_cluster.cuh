@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
     uint32_t slot = 0;   // of the current step
 #pragma unroll 1
     for (int n = 0; n < a.T; ++n) {
-        if (n > 0) collect(n - 1);   // this CTA's own sums among them: the product of that step has read the B operand
+        if (n > 0) collect(n - 1);   // the B operand is free as well: every thread has waited for the whole product of step n - 1
         float2 gate[RPT][4];
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
@@ -304,11 +304,12 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
         const uint32_t nextSlot = slot == 2 * G::kSlotBytes ? 0 : slot + G::kSlotBytes;
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         if (n + 1 < a.T) prepare(nextSlot);
-        // partial sums -> the CTAs that own the units
+        // partial sums -> the CTAs that own the units.  A warp without a tile in some pair waits for that pair too: the next step
+        // overwrites the B operand, and the sums that collect() waits for may all come from the first pair.
 #pragma unroll
         for (int i = 0; i < kReadouts; ++i) {
-            if (!tileReal[i]) continue;
             wait(smemAddr(&productBar[i]), n & 1);
+            if (!tileReal[i]) continue;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             constexpr int kLoad = kSpan < 8 ? kSpan : 8;
             float *out = outMine[i] + (n & 1) * (ROWS * H);

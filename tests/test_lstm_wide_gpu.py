@@ -175,3 +175,11 @@ def test_wide_forward_at_the_row_counts_of_a_cluster(B):
 def test_wide_projection_beside_32_bit_sums(T, B, I, H, wb, ab):
     """Sums of the input projection that may leave 32 bits (W8, A16, 256 inputs) and such that cannot, ragged rows and channels."""
     test_wide_forward_is_bit_exact(T, B, I, H, wb, ab, L.PER_CHANNEL, True, True)
+
+
+@pytest.mark.parametrize("H", [288, 320, 352, 416, 480])
+def test_wide_qat_backward_of_many_steps_beyond_256_units(H):
+    """Widths whose last 128 units are partly empty, so that some warps read nothing of the second part of a step's product,
+    over enough steps for the CTAs of a cluster to drift apart: nobody may write the next step's operand before the whole product is
+    through.  60 steps of two roundings of 2^-24 each in the carried gradient stay below 1e-5, half the tolerance."""
+    test_wide_qat_backward(60, 9, 8, H, 8, 16)
