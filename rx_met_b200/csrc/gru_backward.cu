@@ -1101,6 +1101,8 @@ bool paddedTakes(const BackwardCall &call) {
                                  std::getenv("RXMET_GRU_BWD_SIMT") != nullptr;
     if (disabled || call.W_q == nullptr || call.exec == nullptr || call.H > 256 || call.I > 512) return false;
     if (tiledHidden(call.H) == call.H && tiledInput(call.I) == call.I) return false;
+    // dx has the caller's width: only the tensor-core kernel stores fewer columns than its operands have
+    if (!igrad::eligible(3 * tiledHidden(call.H), call.I)) return false;
     return call.exec->weightClass == CodeClass::I8 && call.exec->actClass != CodeClass::I32 && alignedTo(call.dx, 16) &&
            (call.masks == nullptr || alignedTo(call.masks->x, 8));
 }

@@ -642,6 +642,8 @@ bool paddedTakes(const BackwardCall &call) {
         !call.codesFitTwoTerms || call.h0 == nullptr || call.c0 == nullptr)
         return false;
     if (tiledHidden(call.H) == call.H && tiledInput(call.I) == call.I) return false;
+    // dx and weight_ih have the caller's width: only the tensor-core kernel takes them beside operands of the padded one
+    if (!igrad::eligible(4 * tiledHidden(call.H), call.I)) return false;
     return alignedTo(call.grads.input, 16) && (call.masks == nullptr || alignedTo(call.masks->input, 8));
 }
 

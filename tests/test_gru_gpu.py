@@ -686,3 +686,18 @@ def test_backward_quant_on_padded_widths(gl, cfg_name, shape):
 def test_forward_quant_planes_in_lanes(gl, shape):
     """16-bit grids of at most 128 units: one, two and four rows per CTA with a partly empty last CTA, odd and even step counts."""
     test_forward_quant_matches_restatement(gl, "a16", shape)
+
+
+def test_padded_widths_without_the_tensor_core_input_gradient():
+    """With the tensor-core input gradient switched off (the switch is read once per process) a call of such widths keeps the kernels
+    of its own width: those store all columns that their operands have, and dx has fewer."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    here = Path(__file__).resolve().parent
+    nodes = [f"{here}/test_gru_gpu.py::test_backward_quant_on_padded_widths",
+             f"{here}/test_lstm_wide_gpu.py::test_wide_qat_backward_over_clusters_and_padded_widths[2-5-37-150-8-16]"]
+    done = subprocess.run([sys.executable, "-m", "pytest", "-q", "-m", "gpu", *nodes], cwd=here.parent, capture_output=True, text=True,
+                          env=dict(os.environ, RXMET_IGRAD_SIMT="1"), timeout=300)
+    assert done.returncode == 0, done.stdout[-2000:]
