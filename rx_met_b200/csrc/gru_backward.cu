@@ -1386,7 +1386,8 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         // gradient GEMMs of chunk i (dx rows, dW / dR partial sums) run on the library's second stream; only the
         // last (short) chunk's GEMMs and the reduction of the partial sums stay behind the recurrence.
         std::vector<int> chunks{T};
-        if (mmaPath && tensorInputGrad && tensorGrads && (static_cast<size_t>(B) * I) % 8 == 0)
+        if (mmaPath && tensorInputGrad && tensorGrads && (static_cast<size_t>(B) * I) % 8 == 0 &&
+            call.dxColumns == 0)   // the chunks' launches know one width of dx and no chunks of rows
             chunks = overlapChunks(T, rows, true);
         std::vector<wgrad::Plan> plans;
         int totalSplits = 0;

@@ -701,3 +701,10 @@ def test_padded_widths_without_the_tensor_core_input_gradient():
     done = subprocess.run([sys.executable, "-m", "pytest", "-q", "-m", "gpu", *nodes], cwd=here.parent, capture_output=True, text=True,
                           env=dict(os.environ, RXMET_IGRAD_SIMT="1"), timeout=300)
     assert done.returncode == 0, done.stdout[-2000:]
+
+
+def test_padded_widths_with_time_chunks_asked_for(gl, monkeypatch):
+    """RXMET_GRU_BWD_CHUNKS cuts the backward in time where its kernels know the widths of all operands; a call on padded copies,
+    whose dx keeps the caller's 29 columns, is not cut."""
+    monkeypatch.setenv("RXMET_GRU_BWD_CHUNKS", "20,30,50")
+    test_backward_quant(gl, "w8a8", (20, 8, 29, 100))
