@@ -1183,9 +1183,9 @@ size_t tiledWorkspaceBytes(int T, int B, int I, int H, bool padded) {
     ws.take<float>(2 * kBiasSplits * C);
     // tensor-core path: split-K partials of (I+1) and (H+1) rows and the status word
     // (the slab form of the same kernel, for more than 128 rows or 16-bit codes, asks for fewer splits)
-    ws.take<float>(static_cast<size_t>(std::max({padded ? wgrad::chainSplits(static_cast<int>(rows)) : 1, wgrad::slabSplitBound(I, H, static_cast<int>(C)),
+    ws.take<float>(static_cast<size_t>(std::max({padded ? wgrad::chainPartials(static_cast<int>(rows)) : 1, wgrad::slabSplitBound(I, H, static_cast<int>(C)),
                                                 I <= 143 ? wgrad::splitBound(static_cast<int>(rows), I, static_cast<int>(C)) : 1})) * (I + 1) * C);
-    ws.take<float>(static_cast<size_t>(std::max({padded ? wgrad::chainSplits(static_cast<int>(rows)) : 1, wgrad::slabSplitBound(I, H, static_cast<int>(C)),
+    ws.take<float>(static_cast<size_t>(std::max({padded ? wgrad::chainPartials(static_cast<int>(rows)) : 1, wgrad::slabSplitBound(I, H, static_cast<int>(C)),
                                                 H <= 143 ? wgrad::splitBound(static_cast<int>(rows), H, static_cast<int>(C)) : 1})) * (H + 1) * C);
     ws.take<int>(64);
     ws.take<float>(static_cast<size_t>(B) * H);   // gradient carried between time chunks
@@ -1235,8 +1235,11 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
     // 8-byte loads); callers' buffers that are not aligned that way take the scalar kernels.
     const bool tensorInputGrad = qat && call.exec->weightClass == CodeClass::I8 && igrad::eligible(C, I) && !simtGrads &&
                                  alignedTo(call.dx, 16) && alignedTo(mk.x, 8) && alignedTo(call.W_q, 16);
+    // backwardPadded: as exact as the FP32 kernels that the caller's widths would take, so the rows go in chunks (wgrad::chained)
+    const bool padded = call.dxColumns != 0;
     const bool tensorGrads = qat && call.exec->actClass == CodeClass::I8 && I + 1 <= 144 && H + 1 <= 144 && I % 4 == 0 &&
-                             H % 4 == 0 && !simtGrads && alignedTo(call.x_q, 16) && alignedTo(call.h, 16);
+                             H % 4 == 0 && !simtGrads && alignedTo(call.x_q, 16) && alignedTo(call.h, 16) &&
+                             (!padded || std::max(I, H) <= 128);   // one kernel for both arrays
     // More than 128 rows or 16-bit activation codes: the same tcgen05 kernel over 128-row slabs, two exact
     // bf16 terms per code when the grid is wider than 8 bits.
     const bool wideCodes = qat && call.exec->actClass != CodeClass::I8;
@@ -1387,7 +1390,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         // last (short) chunk's GEMMs and the reduction of the partial sums stay behind the recurrence.
         std::vector<int> chunks{T};
         if (mmaPath && tensorInputGrad && tensorGrads && (static_cast<size_t>(B) * I) % 8 == 0 &&
-            call.dxColumns == 0)   // the chunks' launches know one width of dx and no chunks of rows
+            !padded)   // the chunks' launches know one width of dx and no chunks of rows
             chunks = overlapChunks(T, rows, true);
         std::vector<wgrad::Plan> plans;
         int totalSplits = 0;
@@ -1531,21 +1534,28 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         // the two problems share one launch of one CTA per SM: each is planned for half of the SMs, so that the
         // launch is a single wave (RXMET_WGRAD_FULL_SPLIT plans each for all SMs, two waves)
         const int planSms = std::getenv("RXMET_WGRAD_FULL_SPLIT") ? sms : std::max(1, sms / 2);
-        wgrad::Plan planX = wgrad::plan(K, I, C, planSms), planH = wgrad::plan(K, H, C, planSms);
-        if (call.dxColumns)   // backwardPadded: as exact as the FP32 kernels that the caller's widths would take
-            for (wgrad::Plan *pl : {&planX, &planH})
-                if (pl->tensorMemory) wgrad::boundChain(K, &pl->chunkK, &pl->splits);
+        const wgrad::Plan planX = wgrad::plan(K, I, C, planSms), planH = wgrad::plan(K, H, C, planSms);
+        const bool chain = padded && planX.tensorMemory && planH.tensorMemory && planX.chunkK > wgrad::kChainRows;
+        int splitsX = planX.splits, splitsH = planH.splits;
         WeightGradProblem px{}, ph{};
         px.aCodes = call.x_q; px.aZero = e.gate.zp[RXMET_GRU_X]; px.M = I; px.B = dp;
-        px.partial = ws.take<float>(static_cast<size_t>(planX.splits) * (I + 1) * C);
+        px.partial = ws.take<float>(static_cast<size_t>(chain ? wgrad::chainPartials(K) : splitsX) * (I + 1) * C);
         ph.aFloat = call.h; ph.aInvScale = 1.0f / e.gate.eff[RXMET_GRU_H]; ph.M = H; ph.B = dq;
-        ph.partial = ws.take<float>(static_cast<size_t>(planH.splits) * (H + 1) * C);
+        ph.partial = ws.take<float>(static_cast<size_t>(chain ? wgrad::chainPartials(K) : splitsH) * (H + 1) * C);
         px.status = ph.status = status;
-        wgrad::launchPair(px, planX, ph, planH, K, C, st);
-        afterLaunch("weightGrad");
+        if (chain) {
+            splitsX = splitsH = wgrad::chained(px, ph, K, C, st, [&](const WeightGradProblem &a, const WeightGradProblem &b, int n, int chunks) {
+                const wgrad::Plan plan{chunks, wgrad::kChainRows, true};
+                wgrad::launchPair(a, plan, b, plan, n, C, st);
+                afterLaunch("weightGrad");
+            });
+        } else {
+            wgrad::launchPair(px, planX, ph, planH, K, C, st);
+            afterLaunch("weightGrad");
+        }
         {
-            const ReduceJob jobX{px.partial, planX.splits, I, e.gate.eff[RXMET_GRU_X], mk.W, mk.bw, call.dW, call.dbw};
-            const ReduceJob jobH{ph.partial, planH.splits, H, e.gate.eff[RXMET_GRU_H], mk.R, mk.br, call.dR, call.dbr};
+            const ReduceJob jobX{px.partial, splitsX, I, e.gate.eff[RXMET_GRU_X], mk.W, mk.bw, call.dW, call.dbw};
+            const ReduceJob jobH{ph.partial, splitsH, H, e.gate.eff[RXMET_GRU_H], mk.R, mk.br, call.dR, call.dbr};
             const size_t largest = static_cast<size_t>(std::max(I, H) + 1) * C;
             KernelTimer timer__("reduceWeightGrad", st);
             reduceWeightGrad<<<dim3(static_cast<unsigned>((largest + kReduceWidth - 1) / kReduceWidth), 2),
@@ -1559,15 +1569,23 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         const int K = static_cast<int>(rows);
         int chunkK = 0;
         int splits = wgrad::slabSplits(K, I, H, C, sms, &chunkK);
-        if (call.dxColumns) wgrad::boundChain(K, &chunkK, &splits);   // as above
+        const bool chain = padded && chunkK > wgrad::kChainRows;
+        const int partials = chain ? wgrad::chainPartials(K) : splits;
         WeightGradProblem px{}, ph{};
         px.aCodes = call.x_q; px.aZero = e.gate.zp[RXMET_GRU_X]; px.M = I; px.B = dp;
-        px.partial = ws.take<float>(static_cast<size_t>(splits) * (I + 1) * C);
+        px.partial = ws.take<float>(static_cast<size_t>(partials) * (I + 1) * C);
         ph.aFloat = call.h; ph.aInvScale = 1.0f / e.gate.eff[RXMET_GRU_H]; ph.M = H; ph.B = dq;
-        ph.partial = ws.take<float>(static_cast<size_t>(splits) * (H + 1) * C);
+        ph.partial = ws.take<float>(static_cast<size_t>(partials) * (H + 1) * C);
         px.status = ph.status = status;
-        wgrad::launchSlabs(px, ph, K, C, chunkK, splits, wideCodes, st);
-        afterLaunch("weightGrad");
+        if (chain) {
+            splits = wgrad::chained(px, ph, K, C, st, [&](const WeightGradProblem &a, const WeightGradProblem &b, int n, int chunks) {
+                wgrad::launchSlabs(a, b, n, C, wgrad::kChainRows, chunks, wideCodes, st);
+                afterLaunch("weightGrad");
+            });
+        } else {
+            wgrad::launchSlabs(px, ph, K, C, chunkK, splits, wideCodes, st);
+            afterLaunch("weightGrad");
+        }
         {
             const ReduceJob jobX{px.partial, splits, I, e.gate.eff[RXMET_GRU_X], mk.W, mk.bw, call.dW, call.dbw};
             const ReduceJob jobH{ph.partial, splits, H, e.gate.eff[RXMET_GRU_H], mk.R, mk.br, call.dR, call.dbr};

@@ -595,7 +595,7 @@ constexpr int kMaxTensorSplits = 40;
 // (128-row slabs of both problems in one launch) beyond.
 int tensorSplitBound(int rows, int I, int H, int M, int C, bool padded) {
     const int single = M <= 143 ? wgrad::splitBound(rows, M, C) : 1;
-    return std::max({single, padded ? wgrad::chainSplits(rows) : 1, wgrad::slabPathTakes(I, H, C) ? wgrad::slabSplitBound(I, H, C) : 1});
+    return std::max({single, padded ? wgrad::chainPartials(rows) : 1, wgrad::slabPathTakes(I, H, C) ? wgrad::slabSplitBound(I, H, C) : 1});
 }
 
 namespace {
@@ -920,6 +920,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
     // QAT on 8-bit activation grids: x and h_prev are integer codes, which the tensor-core GEMM
     // multiplies exactly; its ones row also yields the bias gradients.
     if (call.quantized && call.codesFitTensorPath && I % 4 == 0 && H % 4 == 0 && I <= 140 && H <= 140 &&
+        (!padded || std::max(I, H) <= 128) &&   // chunks of rows: one kernel for both arrays
         alignedTo(call.x, 16)) {
         const size_t stateBytes = sizeof(float) * static_cast<size_t>(B) * H;
         if (call.h0) RXMET_CUDA(cudaMemcpyAsync(hPrev, call.h0, stateBytes, cudaMemcpyDeviceToDevice, st));
@@ -934,7 +935,6 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
                 pl.chunkK = ((static_cast<int>(rows) + kMaxTensorSplits - 1) / kMaxTensorSplits + 31) / 32 * 32;
                 pl.splits = (static_cast<int>(rows) + pl.chunkK - 1) / pl.chunkK;
             }
-            if (padded && pl.tensorMemory) wgrad::boundChain(static_cast<int>(rows), &pl.chunkK, &pl.splits);
             return pl;
         };
         const wgrad::Plan planX = planFor(I), planH = planFor(H);
@@ -946,12 +946,21 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
             fail(RXMET_ERR_INVALID_ARGUMENT, "the QAT backward needs the quantized initial hidden state");
         }
         px.status = ph.status = tensorStatus;
-        wgrad::launchPair(px, planX, ph, planH, static_cast<int>(rows), C, st);
-        afterLaunch("weightGrad");
+        int splitsX = planX.splits, splitsH = planH.splits;
+        if (padded && planX.tensorMemory && planH.tensorMemory && planX.chunkK > wgrad::kChainRows) {
+            splitsX = splitsH = wgrad::chained(px, ph, static_cast<int>(rows), C, st, [&](const wgrad::Problem &a, const wgrad::Problem &b, int n, int chunks) {
+                const wgrad::Plan plan{chunks, wgrad::kChainRows, true};
+                wgrad::launchPair(a, plan, b, plan, n, C, st);
+                afterLaunch("weightGrad");
+            });
+        } else {
+            wgrad::launchPair(px, planX, ph, planH, static_cast<int>(rows), C, st);
+            afterLaunch("weightGrad");
+        }
         {
-            const ReduceJob jobIh{tensorIh, planX.splits, I, call.dqX.scale, static_cast<const uint8_t *>(mk.weight_ih),
+            const ReduceJob jobIh{tensorIh, splitsX, I, call.dqX.scale, static_cast<const uint8_t *>(mk.weight_ih),
                                   static_cast<const uint8_t *>(mk.bias_ih), call.grads.weight_ih, call.grads.bias_ih};
-            const ReduceJob jobHh{tensorHh, planH.splits, H, call.dqH.scale, static_cast<const uint8_t *>(mk.weight_hh),
+            const ReduceJob jobHh{tensorHh, splitsH, H, call.dqH.scale, static_cast<const uint8_t *>(mk.weight_hh),
                                   static_cast<const uint8_t *>(mk.bias_hh), call.grads.weight_hh, call.grads.bias_hh};
             const int rowBlocks = (std::max(I, H) + 1 + kReduceRows - 1) / kReduceRows;
             KernelTimer timer__("lstmReduceWeightGradT", st);
@@ -973,13 +982,19 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
                                        cudaMemcpyDeviceToDevice, st));
         int chunkK = 0;
         int splits = wgrad::slabSplits(static_cast<int>(rows), I, H, C, currentDevice().sms, &chunkK);
-        if (padded) wgrad::boundChain(static_cast<int>(rows), &chunkK, &splits);
         wgrad::Problem px{}, ph{};
         px.aFloat = call.x; px.aFloatZero = call.dqX.zeroPoint; px.M = I; px.B = gIh; px.partial = tensorIh;
         ph.aFloat = hPrev; ph.aFloatZero = call.h0 ? call.dqH.zeroPoint : 0.0f; ph.M = H; ph.B = gHh; ph.partial = tensorHh;
         px.status = ph.status = tensorStatus;
-        wgrad::launchSlabs(px, ph, static_cast<int>(rows), C, chunkK, splits, !call.codesFitTensorPath, st);
-        afterLaunch("weightGrad");
+        if (padded && chunkK > wgrad::kChainRows) {
+            splits = wgrad::chained(px, ph, static_cast<int>(rows), C, st, [&](const wgrad::Problem &a, const wgrad::Problem &b, int n, int chunks) {
+                wgrad::launchSlabs(a, b, n, C, wgrad::kChainRows, chunks, !call.codesFitTensorPath, st);
+                afterLaunch("weightGrad");
+            });
+        } else {
+            wgrad::launchSlabs(px, ph, static_cast<int>(rows), C, chunkK, splits, !call.codesFitTensorPath, st);
+            afterLaunch("weightGrad");
+        }
         {
             const ReduceJob jobIh{tensorIh, splits, I, call.dqX.scale, static_cast<const uint8_t *>(mk.weight_ih),
                                   static_cast<const uint8_t *>(mk.bias_ih), call.grads.weight_ih, call.grads.bias_ih};

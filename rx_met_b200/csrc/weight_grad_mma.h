@@ -11,6 +11,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cstddef>
 #include <cstdint>
 
 namespace rxmet {
@@ -53,19 +55,40 @@ struct Plan {
     bool tensorMemory = false;
 };
 Plan plan(int K, int M, int N, int sms);
-// The tensor core truncates every addition to an accumulator; over a chunk of n rows of 16-bit codes that costs about 5e-9 n of
-// the sum (40000 rows in seven splits: 2.7e-5 beside FP32 FMA), half of it for 8-bit codes.  Calls that would otherwise take
-// the FP32 kernels cut the rows into chunks of at most 512 (longer ones beyond 512 splits, whose partial sums would cost more
-// than they are worth).
-inline int chainRows(int K) {
-    const int rows = (K + 511) / 512;
-    return rows <= 512 ? 512 : (rows + 255) / 256 * 256;
-}
-inline int chainSplits(int K) { return (K + chainRows(K) - 1) / chainRows(K); }
-inline void boundChain(int K, int *chunkK, int *splits) {
-    if (*chunkK <= chainRows(K)) return;
-    *chunkK = chainRows(K);
-    *splits = chainSplits(K);
+// The tensor core truncates every addition to an accumulator; over a chunk of n rows that costs up to 8e-9 n of a sum of terms of one
+// sign with 16-bit codes (512 rows: 4.3e-6, 4096: 3.5e-5), a fifth of it with 8-bit codes.  Calls that would otherwise take
+// the FP32 kernels therefore cut the rows into chunks of kChainRows, however many there are: up to kChainGroup chunks (three
+// waves of the widest layers) leave their partial sums to the reduction that follows, more go in several launches, after each of which
+// addPartials folds the partial sums into one more array of them, so that the arrays do not grow with the rows.
+constexpr int kChainRows = 512, kChainGroup = 32;
+inline int chainChunks(int K) { return (K + kChainRows - 1) / kChainRows; }
+// Arrays of (M + 1) x N partial sums that chained() writes.
+inline int chainPartials(int K) { return chainChunks(K) <= kChainGroup ? chainChunks(K) : kChainGroup + 1; }
+// sums of a and b (sum[i] = or += partial[0][i] + partial[1][i] + ...), `partial` behind the sums
+void addPartials(float *a, size_t countA, float *b, size_t countB, int partials, bool first, cudaStream_t stream);
+// launch(a, b, rows, chunks) runs both problems over `rows` rows; returns the number of partial sums at a.partial and b.partial.
+template <class Launch>
+int chained(const Problem &a, const Problem &b, int K, int N, cudaStream_t stream, Launch &&launch) {
+    const int chunks = chainChunks(K);
+    if (chunks <= kChainGroup) {
+        launch(a, b, K, chunks);
+        return chunks;
+    }
+    const size_t countA = static_cast<size_t>(a.M + 1) * N, countB = static_cast<size_t>(b.M + 1) * N;
+    for (int first = 0; first < chunks; first += kChainGroup) {
+        const size_t row = static_cast<size_t>(first) * kChainRows;
+        const int rows = std::min(K - static_cast<int>(row), kChainGroup * kChainRows);
+        auto part = [&](Problem p, size_t count) {
+            if (p.aCodes) p.aCodes += row * p.M;
+            if (p.aFloat) p.aFloat += row * p.M;
+            p.B += row * N;
+            p.partial += count;
+            return p;
+        };
+        launch(part(a, countA), part(b, countB), rows, chainChunks(rows));
+        addPartials(a.partial, countA, b.partial, countB, chainChunks(rows), first == 0, stream);
+    }
+    return 1;
 }
 // Upper bound of plan(...).splits over every device, for sizing the partial buffers.
 int splitBound(int K, int M, int N);

@@ -395,6 +395,39 @@ void launchSlabs(const Problem &a, const Problem &b, int K, int N, int chunkK, i
     }
 }
 
+namespace {
+
+// blockIdx.y: which of the two.  Bound by memory, 16 bytes a load: the counts are multiples of four (N is).
+__global__ void foldPartials(float4 *a, size_t countA, float4 *b, size_t countB, int partials, bool first) {
+    float4 *sums = blockIdx.y == 0 ? a : b;
+    const size_t count = blockIdx.y == 0 ? countA : countB;
+    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < count; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+        float4 s = sums[count + i];
+#pragma unroll 4
+        for (int p = 2; p <= partials; ++p) {
+            const float4 v = sums[p * count + i];
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+        if (!first) {
+            const float4 v = sums[i];
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+        sums[i] = s;
+    }
+}
+
+}  // namespace
+
+void addPartials(float *a, size_t countA, float *b, size_t countB, int partials, bool first, cudaStream_t st) {
+    const size_t most = std::max(countA, countB) / 4;
+    {
+        KernelTimer timer__("foldPartials", st);
+        foldPartials<<<dim3(static_cast<unsigned>(std::min<size_t>((most + 255) / 256, 148 * 8)), 2), 256, 0, st>>>(
+            reinterpret_cast<float4 *>(a), countA / 4, reinterpret_cast<float4 *>(b), countB / 4, partials, first);
+    }
+    afterLaunch("foldPartials");
+}
+
 }  // namespace wgrad
 
 namespace {

@@ -708,3 +708,40 @@ def test_padded_widths_with_time_chunks_asked_for(gl, monkeypatch):
     whose dx keeps the caller's 29 columns, is not cut."""
     monkeypatch.setenv("RXMET_GRU_BWD_CHUNKS", "20,30,50")
     test_backward_quant(gl, "w8a8", (20, 8, 29, 100))
+
+
+@pytest.mark.parametrize("cfg_name,shape", [("w8a8", (1, 16900, 5, 33)), ("a16", (1, 16900, 5, 33)), ("w8a8", (2, 8300, 37, 150))],
+                         ids=lambda s: s if isinstance(s, str) else "x".join(map(str, s)))
+def test_padded_weight_gradient_of_more_rows_than_one_launch(gl, cfg_name, shape):
+    """Rows beyond the 32 chunks of 512 that one launch takes, the last chunk partly empty: partial sums folded between launches."""
+    test_backward_quant(gl, cfg_name, shape)
+
+
+def test_padded_weight_gradient_of_a_million_rows():
+    """One step of 2^20 rows at widths that no tile divides, gradients of one sign, against 64 bits.  A chunk of 512 rows is 192
+    additions of a product to the accumulator (32 steps of 16 rows, two terms of a code, three of a gradient); each truncates, by half a
+    unit of 2^-23 on average: at most 192 * 6e-8 / 2 = 5.8e-6 of a sum that grows evenly.  More rows must not add to that."""
+    import torch
+    from rx_met_b200 import gru_interface_binding as m
+    T, B, I, H = 1, 1 << 20, 5, 33
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rand = lambda *shape: torch.rand(shape, generator=gen, device="cuda")  # noqa: E731
+    W, R, bw, br = (rand(I, 3 * H) - 0.5, rand(H, 3 * H) * 0.2 - 0.1, rand(3 * H) - 0.5, rand(3 * H) - 0.5)
+    x, dh = rand(T, B, I) + 0.5, rand(T + 1, B, H) + 0.5
+    ranges = m.GRUQuantizationRanges(H)
+    m.forward_calibrate(True, T, B, I, H, W, R, bw, br, x, None, "minmax", None, ranges)
+    cfg = m.OperatorQuantConfig()
+    for name in cabi.OP_NAMES:
+        setattr(cfg, f"{name}_", 8 if name in ("W", "R", "bw", "br") else 16)
+    params = m.calculate_gru_quantitative_parameters(ranges, cfg)
+    h, v, *codes = m.forward_quant_int_storage(True, T, B, I, H, W, R, bw, br, x, None, params)[:7]
+    got = m.backward_quant_int_storage(T, B, I, H, *codes, dh, h, v, params, *[torch.empty(0, dtype=torch.uint8, device="cuda")] * 11)
+    z, r, n, q = v[0].double().split(H, dim=1)
+    d = dh[1].double()
+    new = (1 - n * n) * (1 - z) * d
+    dp = torch.cat([z * (1 - z) * (h[0].double() - n) * d, r * (1 - r) * new * q, new], 1)
+    scale = m.decode_effective_scale(params.scale_x_, False) if hasattr(m, "decode_effective_scale") else params.scale_x_
+    real = (codes[4][0].double() - params.zp_x_) * m.decode_effective_scale(params.scale_x_, False)
+    for name, want, have in (("dW", real.t() @ dp, got[1]), ("dbw", dp.sum(0), got[3])):
+        error = float((have.double() - want).norm() / want.norm())
+        assert error < 6e-6, (name, error)
