@@ -214,7 +214,12 @@ RXMET_API int rxmet_gru_decode_effective_scale(float scale, int use_pot2, float 
 
 /* Bytes of device scratch the entry point named by `op` needs for these
  * sizes.  op: 0 forward_fp / forward_calibrate, 1 forward_quant,
- * 2 backward_quant / backward_fp, 3 forward_calibrate with histograms. */
+ * 2 backward_quant / backward_fp, 3 forward_calibrate with histograms,
+ * 4 what is enough for backward_fp and for backward_quant on grids that the
+ * tensor-core kernels do not take (weights of more than 8 bits, activations of
+ * more than 16).  Op 2 adds copies of the step tensors at widths that the
+ * tensor-core kernels tile; backward_quant does without them, on slower
+ * kernels, where the workspace has no room for them. */
 RXMET_API size_t rxmet_gru_workspace_bytes(int op, int T, int B, int I, int H);
 
 /* Float GRU forward.  Replaces forward_fp -> gru::ForwardPass<float>::Run

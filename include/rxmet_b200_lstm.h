@@ -216,7 +216,10 @@ RXMET_API int rxmet_lstm_derive_execution(const rxmet_lstm_quant_params *params,
 
 /* Workspace bytes of: op 0 float / calibration forward, 1 quantized forward,
  * 2 backward, 3 histogram calibration forward (lstmQuantizedFpCudaWorkspaceBreakdown, forward_quantized_fp_cuda.h:133-135;
- * cudaBackwardWorkspaceElementCount, backward_float_cuda.h:45-46). */
+ * cudaBackwardWorkspaceElementCount, backward_float_cuda.h:45-46), 4 what is enough for the float backward and for the QAT
+ * backward on grids that the tensor-core kernels do not take (weights of more than 8 bits, activations of more than 16).
+ * Op 2 adds copies of the step tensors at widths that the tensor-core kernels tile; the QAT backward does without them, on
+ * slower kernels, where the workspace has no room for them. */
 RXMET_API size_t rxmet_lstm_workspace_bytes(int op, int T, int B, int I, int H);
 
 /* Float forward (lstmForwardFloatCuda, operators/quant-lstm/include/lstm/

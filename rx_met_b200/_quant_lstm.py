@@ -208,7 +208,7 @@ def _backward(p: _Prepared, batch_first, trace4, grad_output, grad_final_hidden,
     gs = L.Gradients()
     for n, t in zip(L.MASTER_VALUES, grads):
         setattr(gs, n, t.data_ptr())
-    ws, n = _workspace(2, T, B, I, H, p.device)
+    ws, n = _workspace(4, T, B, I, H, p.device)
     with torch.cuda.device(p.device):
         rc = lib.rxmet_lstm_backward_float(T, B, I, H, _ptr(p.w_ih), _ptr(p.w_hh), _ptr(p.x), _ptr(p.h0), _ptr(p.c0),
                                            _ptr(gates), _ptr(cells), _ptr(ctanh), _ptr(hidden), _ptr(g_out), _ptr(g_hn),

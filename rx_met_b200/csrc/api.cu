@@ -372,8 +372,9 @@ size_t rxmet_gru_workspace_bytes(int op, int T, int B, int I, int H) {
     switch (op) {
         case 0: return gru::forwardFloatWorkspaceBytes(T, B, I, H);
         case 1: return gru::forwardQuantWorkspaceBytes(T, B, I, H);
-        case 2: return gru::backwardWorkspaceBytes(T, B, I, H);
+        case 2: return gru::backwardWorkspaceBytes(T, B, I, H, true);
         case 3: return gru::histCalibrationWorkspaceBytes(T, B, I, H, 8192);
+        case 4: return gru::backwardWorkspaceBytes(T, B, I, H, false);
         default: return 0;
     }
 }

@@ -159,8 +159,10 @@ std::pair<int, std::vector<Tensor>> gruBackwardQuant(int T, int B, int I, int H,
     }
     const c10::cuda::CUDAGuard guard(h.device());
     std::vector<Tensor> out = carve(h, at::kFloat, {{T, B, I}, {I, C}, {H, C}, {C}, {C}, {B, H}});
-    const Tensor ws = workspace(h.device(), static_cast<int64_t>(rxmet_gru_workspace_bytes(2, T, B, I, H)));
     const auto *params = reinterpret_cast<const rxmet_gru_quant_params *>(paramsAddress);
+    const int8_t *bits = params->config.bits;
+    const bool tensorCores = bits[RXMET_GRU_W] <= 8 && bits[RXMET_GRU_R] <= 8 && bits[RXMET_GRU_X] <= 16 && bits[RXMET_GRU_H] <= 16;
+    const Tensor ws = workspace(h.device(), static_cast<int64_t>(rxmet_gru_workspace_bytes(tensorCores ? 2 : 4, T, B, I, H)));
     const pybind11::gil_scoped_release release;
     const int status = rxmet_gru_backward_quant(
         T, B, I, H, pointer<int32_t>(codes[0]), pointer<int32_t>(codes[1]), pointer<int32_t>(codes[2]), pointer<int32_t>(codes[3]),
@@ -320,7 +322,10 @@ std::pair<int, std::vector<Tensor>> lstmBackwardQat(const std::vector<Tensor> &m
     std::array<void *, kMasters> table;
     for (int k = 0; k < kMasters; ++k) table[k] = grads[k].data_ptr();
     std::memcpy(&out, table.data(), sizeof(out));
-    const Tensor ws = emptyLike(p.x, {static_cast<int64_t>(rxmet_lstm_workspace_bytes(2, p.T, p.B, p.I, p.H))}, at::kByte);
+    const auto *bits = params->config.bitwidth;
+    const bool tensorCores = bits[RXMET_LSTM_WEIGHT_IH] <= 8 && bits[RXMET_LSTM_WEIGHT_HH] <= 8 && bits[RXMET_LSTM_INPUT] <= 16 &&
+                             bits[RXMET_LSTM_OUTPUT] <= 16;
+    const Tensor ws = emptyLike(p.x, {static_cast<int64_t>(rxmet_lstm_workspace_bytes(tensorCores ? 2 : 4, p.T, p.B, p.I, p.H))}, at::kByte);
     int status;
     {
         const pybind11::gil_scoped_release release;

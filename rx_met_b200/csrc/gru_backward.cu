@@ -1193,21 +1193,23 @@ size_t tiledWorkspaceBytes(int T, int B, int I, int H, bool padded) {
     return ws.used() + 4096;
 }
 
+// 0 where the widths are tiled already or beyond the padded route.
+size_t paddedWorkspaceBytes(int T, int B, int I, int H) {
+    if (H > 256 || I > 512 || (tiledHidden(H) == H && tiledInput(I) == I)) return 0;
+    PaddedSizer sizer;
+    layoutPadded(sizer, T, B, I, H);
+    sizer.take<int32_t>(6 * static_cast<size_t>(H));
+    return sizer.ws.used() + 512 + tiledWorkspaceBytes(T, B, tiledInput(I), tiledHidden(H), true);
+}
+
 }  // namespace
 
-size_t backwardWorkspaceBytes(int T, int B, int I, int H) {
-    size_t bytes = tiledWorkspaceBytes(T, B, I, H, false);
-    if (H <= 256 && (tiledHidden(H) != H || tiledInput(I) != I)) {
-        PaddedSizer sizer;
-        layoutPadded(sizer, T, B, I, H);
-        sizer.take<int32_t>(6 * static_cast<size_t>(H));
-        bytes = std::max(bytes, sizer.ws.used() + 512 + tiledWorkspaceBytes(T, B, tiledInput(I), tiledHidden(H), true));
-    }
-    return bytes;
+size_t backwardWorkspaceBytes(int T, int B, int I, int H, bool padded) {
+    return std::max(tiledWorkspaceBytes(T, B, I, H, false), padded ? paddedWorkspaceBytes(T, B, I, H) : 0);
 }
 
 void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, cudaStream_t st) {
-    if (paddedTakes(call)) return backwardPadded(call, workspace, workspaceBytes, st);
+    if (paddedTakes(call) && workspaceBytes >= paddedWorkspaceBytes(call.T, call.B, call.I, call.H)) return backwardPadded(call, workspace, workspaceBytes, st);
     const int T = call.T, B = call.B, I = call.I, H = call.H, C = 3 * H;
     const size_t rows = static_cast<size_t>(T) * B;
     Workspace ws(workspace, workspaceBytes);

@@ -28,7 +28,9 @@ struct BackwardCall {
     float *dx = nullptr, *dW = nullptr, *dR = nullptr, *dbw = nullptr, *dbr = nullptr, *dh0 = nullptr;
 };
 
-size_t backwardWorkspaceBytes(int T, int B, int I, int H);
+// padded: with room for copies at widths that the tensor-core kernels tile (quantized calls on 8-bit weights; without it they
+// run on the kernels of their own width)
+size_t backwardWorkspaceBytes(int T, int B, int I, int H, bool padded);
 void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, cudaStream_t stream);
 
 }  // namespace gru

@@ -87,8 +87,9 @@ size_t rxmet_lstm_workspace_bytes(int op, int T, int B, int I, int H) {
     switch (op) {
         case 0: return lstm::forwardFloatWorkspaceBytes(T, B, I, H);
         case 1: return lstm::forwardQuantWorkspaceBytes(T, B, I, H);
-        case 2: return lstm::backwardWorkspaceBytes(T, B, I, H);
+        case 2: return lstm::backwardWorkspaceBytes(T, B, I, H, true);
         case 3: return lstm::histCalibrationWorkspaceBytes(T, B, I, H);
+        case 4: return lstm::backwardWorkspaceBytes(T, B, I, H, false);
         default: return 0;
     }
 }

@@ -77,7 +77,9 @@ struct BackwardCall {
     bool weightCodesFitBf16 = false;  // weight_hh grid of at most 8 bits: codes are exact in bf16
     bool weightIhCodesFitBf16 = false;  // the same for weight_ih
 };
-size_t backwardWorkspaceBytes(int T, int B, int I, int H);
+// padded: with room for copies at widths that the tensor-core kernels tile (QAT on 8-bit weights; without it such calls run on
+// the kernels of their own width)
+size_t backwardWorkspaceBytes(int T, int B, int I, int H, bool padded);
 void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, cudaStream_t stream);
 
 }  // namespace lstm

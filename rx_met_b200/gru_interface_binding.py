@@ -578,7 +578,7 @@ def backward_fp(time_steps, batch_size, input_size, hidden_size, W, R, bw, br, x
     dev = x.device
     dx, dW, dR, dbw, dbr, dh0 = _carve(dev, torch.float32,
                                        [(T, B, I), (I, 3 * H), (H, 3 * H), (3 * H,), (3 * H,), (B, H)])
-    ws = _workspace(dev, lib.rxmet_gru_workspace_bytes(2, T, B, I, H))
+    ws = _workspace(dev, lib.rxmet_gru_workspace_bytes(4, T, B, I, H))
     with torch.cuda.device(dev):
         cabi.check(lib.rxmet_gru_backward_fp(
             T, B, I, H, _ptr(W), _ptr(R), _ptr(bw), _ptr(br), _ptr(x), _ptr(dh_new), _ptr(h), _ptr(v),

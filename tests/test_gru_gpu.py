@@ -745,3 +745,11 @@ def test_padded_weight_gradient_of_a_million_rows():
     for name, want, have in (("dW", real.t() @ dp, got[1]), ("dbw", dp.sum(0), got[3])):
         error = float((have.double() - want).norm() / want.norm())
         assert error < 6e-6, (name, error)
+
+
+@pytest.mark.parametrize("shape", [(3, 2, 29, 100), (2, 5, 33, 255)], ids=lambda s: "x".join(map(str, s)))
+def test_backward_quant_without_room_for_padded_copies(gl, monkeypatch, shape):
+    """A workspace that has no room for copies at tiled widths: the call takes the kernels of its own width."""
+    given = gl.workspace
+    monkeypatch.setattr(gl, "workspace", lambda op, *sizes, **more: given(4 if op == 2 else op, *sizes, **more))
+    test_backward_quant(gl, "w8a8", shape)

@@ -274,3 +274,19 @@ def test_float_storage_carrier_switch_is_host_state():
     finally:
         assert ops.set_float_storage_carrier("integer") == "fp32"
     assert ops.float_storage_carrier() == "integer"
+
+
+def test_backward_workspace_without_padded_copies():
+    """Op 4 leaves out the copies at tiled widths; beside them op 2 holds at most 33 arrays of weight-gradient sums, whatever the
+    number of rows."""
+    lib = cabi.load_library()
+    lib.rxmet_lstm_workspace_bytes.restype = C.c_size_t
+    for bytes_of, gates, tile, I, H in ((lib.rxmet_gru_workspace_bytes, 3, 64, 61, 250), (lib.rxmet_lstm_workspace_bytes, 4, 32, 61, 500)):
+        wide = (H + tile - 1) // tile * tile
+        assert bytes_of(4, 100, 50, 64, wide) == bytes_of(2, 100, 50, 64, wide) > 0     # tiled already
+        partials = 33 * 4 * gates * wide * (64 + 1 + wide + 1)
+        rows = [50 * 100, 50 * 1000, 50 * 20000]
+        for n in rows:
+            small, large = bytes_of(4, n // 50, 50, I, H), bytes_of(2, n // 50, 50, I, H)
+            copies = 4 * (n + 50) * (7 * wide + gates * wide + 64) * 2   # step tensors and the gate gradients, each at most twice
+            assert small < large < small + copies + 2 * partials + (64 << 20), (I, H, n)
