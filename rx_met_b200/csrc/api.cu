@@ -87,6 +87,44 @@ int residentPerSm(const void *kernel, int block, size_t smem) {
     return n;
 }
 
+namespace {
+
+// Allocating, freeing and waiting for a stream of one's own would end a capture that is under way; in this mode they do not.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+}  // namespace
+
+std::shared_ptr<void> copyToDevice(const void *host, size_t bytes) {
+    const RelaxedCapture relaxed;
+    void *buffer = nullptr;
+    RXMET_CUDA(cudaMalloc(&buffer, bytes));
+    std::shared_ptr<void> block(buffer, [](void *ptr) {
+        const RelaxedCapture whileFreeing;
+        cudaFree(ptr);
+    });
+    // a stream of its own: the legacy stream would wait for streams that are being captured
+    cudaStream_t stream = nullptr;
+    RXMET_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    cudaError_t rc = cudaMemcpyAsync(buffer, host, bytes, cudaMemcpyHostToDevice, stream);
+    if (rc == cudaSuccess) rc = cudaStreamSynchronize(stream);
+    cudaStreamDestroy(stream);
+    RXMET_CUDA(rc);
+    return block;
+}
+
+void keepForCapture(const std::shared_ptr<void> &block, cudaStream_t stream) {
+    static std::mutex mutex;
+    static auto &kept = *new std::vector<std::shared_ptr<void>>;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess || status == cudaStreamCaptureStatusNone) return;
+    std::lock_guard<std::mutex> lock(mutex);
+    if (std::find(kept.begin(), kept.end(), block) == kept.end()) kept.push_back(block);
+}
+
 int residentClusters(const void *kernel, int ctas, int block, size_t smem) {
     static std::mutex guard;
     static std::map<std::tuple<int, const void *, int, int, size_t>, int> known;

@@ -454,8 +454,8 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, 
     uint32_t *wIh, *wHh;
     int32_t *addIh, *addHh;
     layout(ws, T, B, I, H, &xq, &h0q, &c0c, &wIh, &wHh, &addIh, &addHh, &lhs);
-    const float *channel = e.channelOnDevice();
-    const int32_t *tables = e.tablesOnDevice();
+    const float *channel = e.channelOnDevice(st);
+    const int32_t *tables = e.tablesOnDevice(st);
 
     const rxmet_lstm_masters none{};
     const rxmet_lstm_masters &m = call.masters ? *call.masters : none;

@@ -673,39 +673,35 @@ const CompactTables &Exec::compactTables() const {
 namespace {
 
 // Device copy of host bytes, one per device, kept with the Exec.
-template <class T>
-T *deviceCopy(std::mutex &mutex, std::vector<std::pair<int, std::shared_ptr<T>>> &copies, const void *host, size_t bytes) {
+const void *deviceCopy(std::mutex &mutex, Exec::DeviceCopies &copies, const void *host, size_t bytes, cudaStream_t stream) {
     int device = 0;
     RXMET_CUDA(cudaGetDevice(&device));
     std::lock_guard<std::mutex> lock(mutex);
-    for (const auto &entry : copies)
-        if (entry.first == device) return entry.second.get();
-    RXMET_REQUIRE(bytes > 0, "the parameter set has no such table");
-    T *buffer = nullptr;
-    RXMET_CUDA(cudaMalloc(reinterpret_cast<void **>(&buffer), bytes));
-    std::shared_ptr<T> owner(buffer, [](T *ptr) { cudaFree(ptr); });
-    // synchronous on purpose: the bytes are pageable host memory and the buffer is shared by every stream
-    RXMET_CUDA(cudaMemcpy(buffer, host, bytes, cudaMemcpyHostToDevice));
-    copies.emplace_back(device, owner);
-    return buffer;
+    auto at = std::find_if(copies.begin(), copies.end(), [&](const auto &entry) { return entry.first == device; });
+    if (at == copies.end()) {
+        RXMET_REQUIRE(bytes > 0, "the parameter set has no such table");
+        at = copies.emplace(copies.end(), device, copyToDevice(host, bytes));
+    }
+    keepForCapture(at->second, stream);
+    return at->second.get();
 }
 
 }  // namespace
 
-const int32_t *Exec::wideTablesOnDevice() const {
-    return deviceCopy(deviceLock, deviceTables, wide.entries.data(), wide.entries.size() * sizeof(int32_t));
+const int32_t *Exec::wideTablesOnDevice(cudaStream_t stream) const {
+    return static_cast<const int32_t *>(deviceCopy(deviceLock, deviceTables, wide.entries.data(), wide.entries.size() * sizeof(int32_t), stream));
 }
 
-const float *Exec::channelOnDevice() const {
-    return deviceCopy(deviceLock, deviceChannel, channel.data(), channel.size() * sizeof(float));
+const float *Exec::channelOnDevice(cudaStream_t stream) const {
+    return static_cast<const float *>(deviceCopy(deviceLock, deviceChannel, channel.data(), channel.size() * sizeof(float), stream));
 }
 
-const int32_t *Exec::tablesOnDevice() const {
-    return deviceCopy(deviceLock, deviceSmallTables, tables.data(), tables.size() * sizeof(int32_t));
+const int32_t *Exec::tablesOnDevice(cudaStream_t stream) const {
+    return static_cast<const int32_t *>(deviceCopy(deviceLock, deviceSmallTables, tables.data(), tables.size() * sizeof(int32_t), stream));
 }
 
-const uint8_t *Exec::compactTablesOnDevice() const {
-    return deviceCopy(deviceLock, deviceCompact, compactTables().bytes.data(), compactTables().bytes.size());
+const uint8_t *Exec::compactTablesOnDevice(cudaStream_t stream) const {
+    return static_cast<const uint8_t *>(deviceCopy(deviceLock, deviceCompact, compactTables().bytes.data(), compactTables().bytes.size(), stream));
 }
 
 }  // namespace lstm

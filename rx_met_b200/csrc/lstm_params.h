@@ -3,6 +3,8 @@
 // blocks (scalar struct, per-channel array, activation tables) the kernels consume.
 #pragma once
 
+#include <cuda_runtime.h>
+
 #include <cstdint>
 #include <memory>
 #include <mutex>
@@ -109,21 +111,19 @@ struct Exec {
     bool exactAccumulators = false;        // every integer accumulator stays below 2^24
     bool weightsFitBytes = false;          // weight_ih and weight_hh grids of at most 8 bits
     int activationPlanes = 1;              // byte planes that hold an input / hidden code: 1 (<= 8 bit) or 2 (<= 16 bit); 0 = wider
-    // Device copy of wide.entries on the current device (cudaMalloc on first use, freed with the Exec).
-    const int32_t *wideTablesOnDevice() const;
-    // The compact form of the wide tables, built on first use, and its device copy.
+    // The compact form of the wide tables, built on first use.
     const CompactTables &compactTables() const;
-    const uint8_t *compactTablesOnDevice() const;
-    // Device copies of `channel` and of `tables`.
-    const float *channelOnDevice() const;
-    const int32_t *tablesOnDevice() const;
-    mutable std::vector<std::pair<int, std::shared_ptr<float>>> deviceChannel;
-    mutable std::vector<std::pair<int, std::shared_ptr<int32_t>>> deviceSmallTables;
+    // Copies of wide.entries, the compact tables, `channel` and `tables` on the current device: made on first use, also inside a
+    // capture of `stream`, and freed with the Exec, or never once a graph refers to them.
+    const int32_t *wideTablesOnDevice(cudaStream_t stream) const;
+    const uint8_t *compactTablesOnDevice(cudaStream_t stream) const;
+    const float *channelOnDevice(cudaStream_t stream) const;
+    const int32_t *tablesOnDevice(cudaStream_t stream) const;
+    using DeviceCopies = std::vector<std::pair<int, std::shared_ptr<void>>>;   // (device ordinal, buffer)
     mutable std::once_flag compactOnce;
     mutable CompactTables compact;
-    mutable std::vector<std::pair<int, std::shared_ptr<uint8_t>>> deviceCompact;
     mutable std::mutex deviceLock;
-    mutable std::vector<std::pair<int, std::shared_ptr<int32_t>>> deviceTables;  // (device ordinal, buffer)
+    mutable DeviceCopies deviceTables, deviceCompact, deviceChannel, deviceSmallTables;
 };
 
 // Cached on the content of `params`: callers pass the same encodings on every step.
