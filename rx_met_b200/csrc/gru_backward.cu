@@ -1114,8 +1114,7 @@ void backwardPadded(const BackwardCall &call, void *workspace, size_t workspaceB
     const rxmet_gru_masks &mk = call.masks ? *call.masks : none;
     Workspace ws(workspace, workspaceBytes);
     const PaddedOperands o = layoutPadded(ws, T, B, I, H);
-    int32_t *scratch = ws.take<int32_t>(6 * static_cast<size_t>(H));
-    const int32_t *scales = channelBlockOnDevice(*call.exec, scratch, 6 * static_cast<size_t>(H), st);
+    const int32_t *scales = channelBlockOnDevice(*call.exec, st);
     auto copy = [](const void *src, void *dst, int srcRows, int dstRows, int groups, int srcWidth, int dstWidth, uint32_t fill = 0) {
         RegroupJob j;
         j.src = src; j.dst = dst; j.srcRows = srcRows; j.dstRows = dstRows;
@@ -1175,7 +1174,6 @@ size_t tiledWorkspaceBytes(int T, int B, int I, int H, bool padded) {
     ws.take<float>(static_cast<size_t>(I) * C);  // W real-valued
     ws.take<float>(static_cast<size_t>(H) * C);  // R real-valued
     ws.take<float>(rows * I);          // x real-valued
-    ws.take<float>(12 * C);            // per-channel block
     const size_t splitW = splitsFor(static_cast<int>(rows), ((I + kTile - 1) / kTile) * ((static_cast<int>(C) + kTile - 1) / kTile));
     const size_t splitR = splitsFor(static_cast<int>(rows), ((H + kTile - 1) / kTile) * ((static_cast<int>(C) + kTile - 1) / kTile));
     ws.take<float>(splitW * I * C);
@@ -1198,7 +1196,6 @@ size_t paddedWorkspaceBytes(int T, int B, int I, int H) {
     if (H > 256 || I > 512 || (tiledHidden(H) == H && tiledInput(I) == I)) return 0;
     PaddedSizer sizer;
     layoutPadded(sizer, T, B, I, H);
-    sizer.take<int32_t>(6 * static_cast<size_t>(H));
     return sizer.ws.used() + 512 + tiledWorkspaceBytes(T, B, tiledInput(I), tiledHidden(H), true);
 }
 
@@ -1256,10 +1253,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         float *Rf = ws.take<float>(static_cast<size_t>(H) * C);
         float *xf = ws.take<float>(rows * I);
         // effective scales of W then R: the first two arrays of the per-channel block
-        const size_t chanWords = 2 * static_cast<size_t>(C);
-        int32_t *chanScratch = ws.take<int32_t>(chanWords);
-        const float *chan = call.channelScales ? call.channelScales
-                                               : reinterpret_cast<const float *>(channelBlockOnDevice(e, chanScratch, chanWords, st));
+        const float *chan = call.channelScales ? call.channelScales : reinterpret_cast<const float *>(channelBlockOnDevice(e, st));
         if (!tensorInputGrad) {
             KernelTimer timer__("dequantCodes", st);
             dequantCodes<<<gridFor(static_cast<size_t>(I) * C, 256), 256, 0, st>>>(call.W_q, static_cast<size_t>(I) * C, C, chan, 0.f, 0, Wf);

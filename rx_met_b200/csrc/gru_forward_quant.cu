@@ -38,10 +38,9 @@
 namespace rxmet {
 namespace gru {
 
-// The block is page-locked host memory owned by the Exec, and the Exec lives in a small cache that
-// evicts old entries.  A copy recorded into a CUDA graph reads the block again at every replay, long
-// after the call returned, so a block handed out while the stream is being captured is kept for the
-// life of the process (one block per captured parameter set; a few tens of KB each).
+// The Exec that owns the device copy of its block lives in a small cache that evicts old entries.  A CUDA graph
+// reads the block at every replay, long after the call returned, so one handed out while the stream is being
+// captured is kept for the life of the process (one block per captured parameter set; a few tens of KB each).
 namespace {
 
 std::vector<int32_t> channelBlock(const Exec &e) {
@@ -56,38 +55,17 @@ std::vector<int32_t> channelBlock(const Exec &e) {
 
 }  // namespace
 
-const int32_t *channelBlockOnDevice(const Exec &e, int32_t *scratch, size_t words, cudaStream_t st) {
-    const int device = currentDevice().device;
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    const bool capturing = cudaStreamIsCapturing(st, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
+const int32_t *channelBlockOnDevice(const Exec &e, cudaStream_t st) {
     static std::mutex mutex;
-    static std::vector<std::shared_ptr<int32_t>> captured;   // blocks a graph refers to stay for good
-    auto keep = [&](const std::shared_ptr<int32_t> &block) {
-        if (capturing && std::find(captured.begin(), captured.end(), block) == captured.end()) captured.push_back(block);
-    };
+    const int device = currentDevice().device;
     std::lock_guard<std::mutex> lock(mutex);
-    for (const auto &entry : e.deviceChannels)
-        if (entry.first == device) {
-            keep(entry.second);
-            return entry.second.get();
-        }
-    const std::vector<int32_t> host = channelBlock(e);
-    const size_t bytes = host.size() * sizeof(int32_t);
-    int32_t *buffer = nullptr;
-    if (capturing) {   // nothing may be allocated on the device now: the graph copies from page-locked memory
-        RXMET_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&buffer), bytes, cudaHostAllocDefault));
-        const std::shared_ptr<int32_t> block(buffer, [](int32_t *ptr) { cudaFreeHost(ptr); });
-        std::memcpy(buffer, host.data(), bytes);
-        keep(block);
-        RXMET_CUDA(cudaMemcpyAsync(scratch, buffer, words * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-        return scratch;
+    auto at = std::find_if(e.deviceChannels.begin(), e.deviceChannels.end(), [&](const auto &entry) { return entry.first == device; });
+    if (at == e.deviceChannels.end()) {
+        const std::vector<int32_t> host = channelBlock(e);
+        at = e.deviceChannels.emplace(at, device, copyToDevice(host.data(), host.size() * sizeof(int32_t)));
     }
-    RXMET_CUDA(cudaMalloc(reinterpret_cast<void **>(&buffer), bytes));
-    const std::shared_ptr<int32_t> block(buffer, [](int32_t *ptr) { cudaFree(ptr); });
-    // synchronous: the source is pageable and the copy is shared by every stream
-    RXMET_CUDA(cudaMemcpy(buffer, host.data(), bytes, cudaMemcpyHostToDevice));
-    e.deviceChannels.emplace_back(device, block);
-    return buffer;
+    keepForCapture(at->second, st);
+    return static_cast<const int32_t *>(at->second.get());
 }
 
 namespace {
@@ -1395,9 +1373,9 @@ struct ChannelDevice {
     const Rescale *gemmX, *biasX, *gemmH, *biasH;
 };
 
-ChannelDevice uploadChannels(const Exec &e, Workspace &ws, cudaStream_t st) {
+ChannelDevice uploadChannels(const Exec &e, cudaStream_t st) {
     const size_t C = 3 * static_cast<size_t>(e.hidden);
-    const int32_t *block = channelBlockOnDevice(e, ws.take<int32_t>(12 * C), 12 * C, st);
+    const int32_t *block = channelBlockOnDevice(e, st);
     ChannelDevice d;
     d.effW = reinterpret_cast<const float *>(block);
     d.effR = d.effW + C; d.effBw = d.effW + 2 * C; d.effBr = d.effW + 3 * C;
@@ -1461,7 +1439,7 @@ void runWide(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaStr
         RXMET_REQUIRE(mk.gate_input && mk.gate_output && mk.h, "gate_input, gate_output and h masks come together");
     if (call.stepFlags)
         RXMET_REQUIRE(call.isTraining && mk.weight_ih_linear, "packed step flags need a training forward with the weight_ih_linear mask");
-    const ChannelDevice ch = uploadChannels(e, ws, st);
+    const ChannelDevice ch = uploadChannels(e, st);
     const WideOperands o = wideOperands(ws, T, B, I, H);
 
     WidePrepArgs p{};
@@ -1530,7 +1508,7 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
     const rxmet_gru_masks none{};
     const rxmet_gru_masks &mk = (training && call.masks) ? *call.masks : none;
 
-    const ChannelDevice ch = uploadChannels(e, ws, st);
+    const ChannelDevice ch = uploadChannels(e, st);
     auto *wCodes = ws.take<WWord>(static_cast<size_t>(iWords) * C);
     auto *rCodes = ws.take<WWord>(static_cast<size_t>(hWords) * C);
     auto *bwCodes = ws.take<int32_t>(C);
@@ -1859,7 +1837,6 @@ void sizeTyped(WorkspaceSizer &ws, int T, int B, int I, int H) {
     using D = Dot<WT, AT>;
     const size_t C = 3 * static_cast<size_t>(H), rows = static_cast<size_t>(T) * B;
     const int iWords = padTo(I, D::kPack) / D::kPack, hWords = padTo(H, D::kPack) / D::kPack;
-    ws.take<int32_t>(12 * C);
     ws.take<typename D::WWord>(iWords * C);
     ws.take<typename D::WWord>(hWords * C);
     ws.take<int32_t>(C);
@@ -2058,7 +2035,6 @@ __global__ void __launch_bounds__(768) fpRecurrent(const __grid_constant__ FpRec
 size_t fpCarrierBytes(int T, int B, int I, int H) {
     const size_t rows = static_cast<size_t>(T) * B, C = 3 * static_cast<size_t>(H);
     WorkspaceSizer ws;
-    ws.take<float>(12 * C);
     ws.take<int32_t>(static_cast<size_t>(I) * C);
     ws.take<int32_t>(static_cast<size_t>(H) * C);
     ws.take<int32_t>(2 * C);
@@ -2080,7 +2056,7 @@ void forwardFpCarrier(const ForwardQuantCall &call, const Exec &e, Workspace &ws
     const rxmet_gru_masks &mk = (training && call.masks) ? *call.masks : none;
     const FpCarrierParams fp = deriveFpCarrier(*call.fpCarrier);
 
-    const ChannelDevice ch = uploadChannels(e, ws, st);
+    const ChannelDevice ch = uploadChannels(e, st);
     int32_t *wq = ws.take<int32_t>(static_cast<size_t>(I) * C), *rq = ws.take<int32_t>(static_cast<size_t>(H) * C);
     int32_t *biasQ = ws.take<int32_t>(2 * static_cast<size_t>(C));
     int32_t *xq = ws.take<int32_t>(rows * I), *h0q = ws.take<int32_t>(static_cast<size_t>(B) * H);

@@ -34,8 +34,8 @@ struct ForwardQuantCall {
 bool packedFlagsSupported(const Exec &exec, int B, int I, int H);
 
 // The per-channel block (four float arrays, four Rescale arrays of 3 * hidden entries each) on the current device: a copy
-// kept with the Exec, or, inside a stream capture that comes before the first call, `words` words of it copied to `scratch`.
-const int32_t *channelBlockOnDevice(const Exec &exec, int32_t *scratch, size_t words, cudaStream_t stream);
+// kept with the Exec, made on first use, also inside a capture of `stream`.
+const int32_t *channelBlockOnDevice(const Exec &exec, cudaStream_t stream);
 
 size_t forwardQuantWorkspaceBytes(int T, int B, int I, int H);
 void forwardQuant(const ForwardQuantCall &call, const Exec &exec, void *workspace, size_t workspaceBytes,

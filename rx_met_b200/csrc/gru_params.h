@@ -66,7 +66,7 @@ struct Exec {
     CodeClass actClass = CodeClass::I8;     // x and h codes
     CodeClass linearClass = CodeClass::I16; // ih / hh linear codes
     // Device copies of the per-channel block (device ordinal, buffer), made on first use and freed with the Exec.
-    mutable std::vector<std::pair<int, std::shared_ptr<int32_t>>> deviceChannels;
+    mutable std::vector<std::pair<int, std::shared_ptr<void>>> deviceChannels;
 };
 
 // Encodings from ranges (reference: operators/quant-gru/src/gru_host.cc:13-125).

@@ -8,6 +8,7 @@ import torch
 
 import lstm_lib as ll
 from rx_met_b200 import _cabi_lstm as L
+from rx_met_b200 import gru_interface_binding as gru
 from test_lstm_gpu import mod, torch_args
 
 pytestmark = pytest.mark.gpu
@@ -34,7 +35,25 @@ def lstm_step(H, abits, seed):
     return run
 
 
-@pytest.mark.parametrize("step,H,abits", [(lstm_step, 32, 8), (lstm_step, 96, 16), (lstm_step, 200, 8)],
+def gru_step(H, abits, seed):
+    T, B, I = 5, 3, 12
+    gen = torch.Generator().manual_seed(seed)
+    rand = lambda *shape: (torch.rand(shape, generator=gen) - 0.5).cuda()  # noqa: E731
+    W, R, bw, br, x, dh = rand(I, 3 * H), rand(H, 3 * H) * 0.2, rand(3 * H), rand(3 * H), rand(T, B, I), rand(T + 1, B, H)
+    ranges = gru.GRUQuantizationRanges(H)
+    gru.forward_calibrate(True, T, B, I, H, W, R, bw, br, x, None, "minmax", None, ranges)
+    cfg = gru.OperatorQuantConfig()
+    for name in ("x", "h", "weight_ih_linear", "weight_hh_linear"):
+        setattr(cfg, f"{name}_", abits)
+    params = gru.calculate_gru_quantitative_parameters(ranges, cfg)
+
+    def run():
+        out = gru.forward_quant_int_storage(True, T, B, I, H, W, R, bw, br, x, None, params)
+        return [out[0], *gru.backward_quant_int_storage(T, B, I, H, *out[2:7], dh, out[0], out[1], params, *out[7:])]
+    return run
+
+
+@pytest.mark.parametrize("step,H,abits", [(lstm_step, 32, 8), (lstm_step, 96, 16), (lstm_step, 200, 8), (gru_step, 32, 8), (gru_step, 96, 16)],
                          ids=lambda v: v if isinstance(v, int) else v.__name__)
 def test_first_use_of_parameters_inside_a_capture(step, H, abits):
     stream = torch.cuda.Stream()
