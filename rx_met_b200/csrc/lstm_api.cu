@@ -204,8 +204,8 @@ int rxmet_lstm_backward_qat(int T, int B, int I, int H, const rxmet_lstm_quant_p
         call.dqC = gridOfPoint(*params, RXMET_LSTM_CELL_STATE);
         for (int g = 0; g < 4; ++g) call.dqGate[g] = gridOfPoint(*params, RXMET_LSTM_INPUT_GATE_OUTPUT + g);
         call.dqTanh = gridOfPoint(*params, RXMET_LSTM_CELL_TANH_OUTPUT);
-        const auto exec = lstm::deriveExec(*params, false);
-        call.channelScales = exec->channelOnDevice(static_cast<cudaStream_t>(stream));   // its first two fields
+        const auto scales = lstm::weightScalesOnDevice(*params, static_cast<cudaStream_t>(stream));
+        call.channelScales = scales.get();
         call.codesFitTensorPath = params->config.bitwidth[RXMET_LSTM_INPUT] <= 8 && params->config.bitwidth[RXMET_LSTM_OUTPUT] <= 8;
         call.codesFitTwoTerms = params->config.bitwidth[RXMET_LSTM_INPUT] <= 16 && params->config.bitwidth[RXMET_LSTM_OUTPUT] <= 16;
         call.weightCodesFitBf16 = params->config.bitwidth[RXMET_LSTM_WEIGHT_HH] <= 8;

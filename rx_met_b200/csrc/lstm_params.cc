@@ -568,6 +568,22 @@ std::shared_ptr<const Exec> deriveExec(const rxmet_lstm_quant_params &p, bool re
     return e;
 }
 
+std::shared_ptr<const float> weightScalesOnDevice(const rxmet_lstm_quant_params &p, cudaStream_t stream) {
+    static std::mutex mutex;
+    static std::map<std::pair<int, std::vector<float>>, std::shared_ptr<void>> cache;
+    const size_t channels = 4 * static_cast<size_t>(p.hidden_size);
+    int device = 0;
+    RXMET_CUDA(cudaGetDevice(&device));
+    std::pair<int, std::vector<float>> key{device, {p.weight_ih_scale, p.weight_ih_scale + channels}};
+    key.second.insert(key.second.end(), p.weight_hh_scale, p.weight_hh_scale + channels);
+    std::lock_guard<std::mutex> lock(mutex);
+    if (cache.size() > 64) cache.clear();
+    std::shared_ptr<void> &block = cache[key];
+    if (!block) block = copyToDevice(key.second.data(), key.second.size() * sizeof(float));
+    keepForCapture(block, stream);
+    return std::static_pointer_cast<const float>(block);
+}
+
 namespace {
 
 // Line of one segment: codes[i] (centred) for the inputs x0 + i.  Entries at a limit of the output grid bind on one side only

@@ -128,6 +128,9 @@ struct Exec {
 
 // Cached on the content of `params`: callers pass the same encodings on every step.
 std::shared_ptr<const Exec> deriveExec(const rxmet_lstm_quant_params &params, bool requireExact);
+// Scales of weight_ih, then weight_hh (4H each) on the current device, cached on their content.  All that a backward needs of the
+// parameters, where deriveExec builds the tables of a forward.  Hold the block until the kernels that read it are launched.
+std::shared_ptr<const float> weightScalesOnDevice(const rxmet_lstm_quant_params &params, cudaStream_t stream);
 
 }  // namespace lstm
 }  // namespace rxmet

@@ -301,3 +301,28 @@ def test_inference_in_lanes_equals_the_training_forward(T, B, I, H):
     runs = [m.lstm_forward_quantized(*args, False, m._params_to_bundle(box), "pedantic", False, save) for save in (False, True)]
     for a, b in zip(runs[0][:3], runs[1][:3]):
         assert torch.equal(a, b)
+
+
+def test_qat_backward_reads_no_parameters_but_grids_and_weight_scales(monkeypatch):
+    """The backward derives nothing of a forward's execution: it runs on parameters without bias scales and without scales of the
+    linear stages, and gives the gradients of the complete set."""
+    import copy
+    T, B, I, H = 4, 3, 12, 32
+    p = ll.problem(T, B, I, H, seed=2, wscale=0.2)
+    _, box = ll.calibrate("orc", L.default_config(symmetric_activations=True), p, np.stack([p["x"] * 0.8]))
+    m = mod()
+    bundle = m._params_to_bundle(box)
+    _, _, _, ck, _ = m.lstm_forward_quantized(*torch_args(p), False, bundle, "pedantic", False, True)
+    order = ("input", "weight_ih", "weight_hh", "bias_ih", "bias_hh", "h_0", "c_0")
+    g = [torch.ones(shape, device="cuda") for shape in ((T, B, H), (B, H), (B, H))]
+    args = ([ck["quantized_master"][n] for n in order], False, bundle,
+            [ck["values"][n] for n in ("gate_outputs", "cell_states", "cell_tanh_outputs", "hidden_outputs")], *g,
+            [ck["master_clamp_masks"][n] for n in order], [ck["clamp_masks"][n] for n in L.TRACE_VALUES])
+    want = m.lstm_backward_qat(*args)
+    bare = copy.copy(m._bundle_to_params(bundle))
+    bare.struct = L.QuantParams.from_buffer_copy(bare.struct)
+    bare.struct.bias_ih_scale = bare.struct.bias_hh_scale = None
+    bare.struct.scale[L.WEIGHT_IH_LINEAR] = bare.struct.scale[L.WEIGHT_HH_LINEAR] = 0.0
+    monkeypatch.setattr(m, "_bundle_to_params", lambda text: bare)
+    for name, a, b in zip(L.MASTER_VALUES, m.lstm_backward_qat(*args), want):
+        assert torch.equal(a, b), name
