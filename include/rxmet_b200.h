@@ -49,6 +49,10 @@ RXMET_API uint64_t rxmet_kernel_launch_count(void);
  * queueing behind each other.  Default 1; values below 1 are taken as 1.  Results do not depend on
  * it.  No counterpart in the reference. */
 RXMET_API int rxmet_set_concurrent_passes(int passes);
+/* The same for the calls of this thread alone; 0: the process-wide setting holds again.  Returns the thread's setting before. */
+RXMET_API int rxmet_set_thread_concurrent_passes(int passes);
+/* The number of passes that a call of this thread plans for. */
+RXMET_API int rxmet_concurrent_passes(void);
 
 /* Which part of a quantized GRU forward the calls of this thread run: 0 everything, 1 all but the
  * recurrence, 2 only the recurrence (the same arguments and workspace as the call with 1 before it).

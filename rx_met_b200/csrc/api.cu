@@ -9,6 +9,7 @@
 #include <tuple>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "common.h"
@@ -264,7 +265,11 @@ std::atomic<int> &concurrentPassesSetting() {
     static std::atomic<int> passes{1};
     return passes;
 }
-int concurrentPasses() { return concurrentPassesSetting().load(); }
+int &threadConcurrentPasses() {
+    static thread_local int passes = 0;
+    return passes;
+}
+int concurrentPasses() { return threadConcurrentPasses() > 0 ? threadConcurrentPasses() : concurrentPassesSetting().load(); }
 ForwardPhase &forwardPhaseSetting() {
     static thread_local ForwardPhase phase = ForwardPhase::All;
     return phase;
@@ -307,6 +312,8 @@ int rxmet_set_concurrent_passes(int passes) {
     concurrentPassesSetting().store(passes < 1 ? 1 : passes);
     return RXMET_OK;
 }
+int rxmet_set_thread_concurrent_passes(int passes) { return std::exchange(threadConcurrentPasses(), std::max(0, passes)); }
+int rxmet_concurrent_passes(void) { return concurrentPasses(); }
 
 int rxmet_set_kernel_timing(int enabled) {
     return guarded([&] {

@@ -100,7 +100,7 @@ struct DeviceInfo {
     int device = 0, sms = 0, smemMax = 0;
 };
 const DeviceInfo &currentDevice();
-// Recurrent passes the caller runs side by side on one GPU (rxmet_set_concurrent_passes); at least 1.
+// Recurrent passes the caller runs side by side on one GPU (rxmet_set_concurrent_passes, or this thread's own); at least 1.
 int concurrentPasses();
 // Which part of a GRU forward a call of this thread runs (rxmet_set_forward_phase).
 enum class ForwardPhase { All = 0, Projection = 1, Recurrence = 2 };

@@ -95,16 +95,16 @@ class StackedGruQat:
         main = torch.cuda.current_stream(self.device)
         self.side.wait_stream(main)
         # The two directions share the SMs: their CTAs are resident together.  The setting is read where a launch is
-        # planned and holds for the whole process, so it goes back at once: left at 2, every later recurrence of the
-        # program plans for half of the SMs (a wide LSTM forward at batch 4096: 289 ms instead of 143 ms).
-        self._lib.rxmet_set_concurrent_passes(2)
+        # planned; it is this thread's own and goes back at once, so that no other pass of the program plans for half of
+        # the SMs (a wide LSTM forward at batch 4096: 289 ms instead of 143 ms).
+        before = self._lib.rxmet_set_thread_concurrent_passes(2)
         self._lib.rxmet_set_forward_phase(phase)
         try:
             fn_forward()
             with torch.cuda.stream(self.side):
                 fn_reverse()
         finally:
-            self._lib.rxmet_set_concurrent_passes(1)
+            self._lib.rxmet_set_thread_concurrent_passes(before)
             self._lib.rxmet_set_forward_phase(0)
         main.wait_stream(self.side)
 

@@ -290,3 +290,27 @@ def test_backward_workspace_without_padded_copies():
             small, large = bytes_of(4, n // 50, 50, I, H), bytes_of(2, n // 50, 50, I, H)
             copies = 4 * (n + 50) * (7 * wide + gates * wide + 64) * 2   # step tensors and the gate gradients, each at most twice
             assert small < large < small + copies + 2 * partials + (64 << 20), (I, H, n)
+
+
+def test_concurrent_passes_of_a_thread():
+    """A thread's own number of passes holds for its calls alone and gives way to the process-wide one again."""
+    import threading
+    lib = cabi.load_library()
+
+    def elsewhere():
+        seen = []
+        worker = threading.Thread(target=lambda: seen.append(lib.rxmet_concurrent_passes()))
+        worker.start()
+        worker.join()
+        return seen[0]
+
+    assert lib.rxmet_concurrent_passes() == 1
+    assert lib.rxmet_set_thread_concurrent_passes(2) == 0
+    assert (lib.rxmet_concurrent_passes(), elsewhere()) == (2, 1)
+    lib.rxmet_set_concurrent_passes(3)
+    try:
+        assert (lib.rxmet_concurrent_passes(), elsewhere()) == (2, 3)
+        assert lib.rxmet_set_thread_concurrent_passes(0) == 2
+        assert lib.rxmet_concurrent_passes() == 3
+    finally:
+        lib.rxmet_set_concurrent_passes(1)

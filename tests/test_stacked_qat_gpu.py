@@ -140,3 +140,20 @@ def test_captured_step_replays_the_eager_step():
     assert captured.captured_launches > 50
     assert torch.equal(eager.flat_w, captured.flat_w)
     assert torch.equal(loss_e, loss_c)
+
+
+def test_step_leaves_the_planned_passes_as_they_were():
+    """The two directions plan for each other by the calling thread's own setting; a process-wide one stays in force."""
+    from rx_met_b200 import _cabi
+    from rx_met_b200.stacked_qat import StackedGruQat, a16_config
+    lib = _cabi.load_library()
+    model = StackedGruQat(4, 8, 12, 32, 1, 4, torch.device("cuda:0"), a16_config(8, 16), seed=1)
+    x, labels = torch.randn(4, 8, 12, device="cuda"), torch.zeros(8, dtype=torch.int64, device="cuda")
+    model.calibrate([x])
+    lib.rxmet_set_concurrent_passes(3)
+    try:
+        model.step(x, labels, lr=0.1)
+        assert lib.rxmet_concurrent_passes() == 3
+        assert lib.rxmet_set_thread_concurrent_passes(0) == 0
+    finally:
+        lib.rxmet_set_concurrent_passes(1)
