@@ -156,6 +156,7 @@ def backward(grad, tensor, scale, offset, qmin: int, qmax: int, *, reciprocal: b
 
 
 def _apply(tensor, scale, offset, qmin, qmax, reciprocal, block_size):
+    """Forward and autograd node of the binding."""
     if not (tensor.is_cuda and scale.is_cuda and offset.is_cuda):
         raise RuntimeError("affine_qdq runs on CUDA tensors only")
     if tensor.dtype != torch.float32:
@@ -166,12 +167,25 @@ def _apply(tensor, scale, offset, qmin, qmax, reciprocal, block_size):
                                                    *_cached_layout(tensor.shape, scale.shape, block_size))
 
 
-class QuantDequantFunc:
-    """Differentiable quantize-dequantize: the forward and its autograd node live in the binding."""
+class QuantDequantFunc(torch.autograd.Function):
+    """The same node in Python.  A trace records it as one operation; the binding's is invisible to it (the traced function
+    would return the buffer that the forward allocates, unwritten)."""
 
     @staticmethod
-    def apply(tensor, scale, offset, qmin: int, qmax: int, reciprocal: bool = False, block_size=None):
-        return _apply(tensor, scale, offset, qmin, qmax, reciprocal, None if block_size is None else tuple(block_size))
+    def forward(ctx, tensor, scale, offset, qmin: int, qmax: int, reciprocal: bool = False, block_size=None):
+        y, _ = forward(tensor, scale, offset, qmin, qmax, reciprocal=reciprocal, block_size=block_size)
+        ctx.qmin, ctx.qmax, ctx.reciprocal, ctx.block_size = qmin, qmax, reciprocal, block_size
+        ctx.save_for_backward(tensor, scale, offset)
+        return y
+
+    @staticmethod
+    def backward(ctx, grad):
+        tensor, scale, offset = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        dx, ds, do = backward(grad, tensor, scale, offset, ctx.qmin, ctx.qmax, reciprocal=ctx.reciprocal,
+                              want_tensor_grad=need[0], want_scale_grad=need[1], want_offset_grad=need[2],
+                              block_size=ctx.block_size)
+        return dx, ds, do, None, None, None, None
 
 
 def quantize_dequantize(tensor: torch.Tensor, scale: torch.Tensor, offset: torch.Tensor, qmin: int, qmax: int,
@@ -183,4 +197,7 @@ def quantize_dequantize(tensor: torch.Tensor, scale: torch.Tensor, offset: torch
     trained = (scale.requires_grad or offset.requires_grad) and torch.is_grad_enabled()
     # blockwise grids always take the divide form: the reference's fast path does not handle them
     reciprocal = not trained and block_size is None
-    return _apply(tensor, scale, offset, qmin, qmax, reciprocal, None if block_size is None else tuple(block_size))
+    block_size = None if block_size is None else tuple(block_size)
+    if torch.jit.is_tracing():
+        return QuantDequantFunc.apply(tensor, scale, offset, qmin, qmax, reciprocal, block_size)
+    return _apply(tensor, scale, offset, qmin, qmax, reciprocal, block_size)

@@ -210,3 +210,22 @@ def test_backward_of_nan_inputs():
     assert same_bits(dx.cpu().numpy(), want_dx) and not dx.cpu().numpy()[np.isnan(x)].any()
     assert np.isnan(scale_terms).sum() == 3 and np.isnan(ds.cpu().numpy()).all()
     assert np.allclose(do.cpu().numpy().reshape(()), offset_terms.astype(np.float64).sum(), rtol=1e-5)
+
+
+@pytest.mark.parametrize("trained", [False, True])
+def test_traced_quantize_dequantize(trained):
+    """A traced function quantizes the tensors it is called with, not those it was traced with."""
+    import torch
+    from rx_met_b200 import affine_qdq
+    s = (torch.rand(8, 1, device="cuda") * 0.1 + 0.01).requires_grad_(trained)
+    o = torch.zeros(8, 1, device="cuda")
+    x, y = torch.randn(8, 16, device="cuda"), torch.randn(8, 16, device="cuda")
+    traced = torch.jit.trace(lambda t, grid: affine_qdq.quantize_dequantize(t, grid, o, -128, 127), (x, s), check_trace=False)
+    want = affine_qdq.quantize_dequantize(y, s, o, -128, 127)
+    got = traced(y, s)
+    assert torch.equal(got, want)
+    if trained:
+        grads = [torch.autograd.grad(t.sum(), s)[0] for t in (got, want)]
+        assert torch.equal(*grads)
+    out = affine_qdq.QuantDequantFunc.apply(y, s, o, -128, 127, not trained)
+    assert torch.equal(out, want) and isinstance(affine_qdq.QuantDequantFunc, type(torch.autograd.Function))
