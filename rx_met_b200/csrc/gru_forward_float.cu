@@ -445,7 +445,7 @@ void forwardFloat(const ForwardFloatCall &call, void *workspace, size_t workspac
     }
     {
         const int block = std::min((C + 31) / 32 * 32, 512);
-        const size_t smem = sizeof(float) * (kRowsPerBlock * I + 2 * 2 * 32);
+        const size_t smem = sizeof(float) * (kRowsPerBlock * I + 2 * 2 * (block / 32));   // rows, scratch of two statistics
         {
             KernelTimer timer__("inputLinearFloat", st);
             inputLinearFloat<<<static_cast<int>((rows + kRowsPerBlock - 1) / kRowsPerBlock), block, smem, st>>>(

@@ -753,3 +753,8 @@ def test_backward_quant_without_room_for_padded_copies(gl, monkeypatch, shape):
     given = gl.workspace
     monkeypatch.setattr(gl, "workspace", lambda op, *sizes, **more: given(4 if op == 2 else op, *sizes, **more))
     test_backward_quant(gl, "w8a8", shape)
+
+
+def test_float_forward_of_the_widest_input(gl):
+    """1528 inputs: eight rows of them and the reduction scratch of sixteen warps fill the 48 KB that a launch has without asking."""
+    test_calibration_forward(gl, (1, 2, 1528, 176))
