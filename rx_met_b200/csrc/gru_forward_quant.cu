@@ -2134,7 +2134,7 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, 
         fail(RXMET_ERR_UNSUPPORTED, "packed step flags: these grids or sizes take neither the 8-bit register path nor the cluster recurrence");
     Workspace ws(workspace, workspaceBytes);
     if (call.fpCarrier) {
-        forwardFpCarrier(call, e, ws, st);
+        if (forwardPhase() != ForwardPhase::Recurrence) forwardFpCarrier(call, e, ws, st);   // not split: all of it in the call before
         return;
     }
     const CodeClass w = e.weightClass, a = e.actClass, l = e.linearClass;

@@ -758,3 +758,21 @@ def test_backward_quant_without_room_for_padded_copies(gl, monkeypatch, shape):
 def test_float_forward_of_the_widest_input(gl):
     """1528 inputs: eight rows of them and the reduction scratch of sixteen warps fill the 48 KB that a launch has without asking."""
     test_calibration_forward(gl, (1, 2, 1528, 176))
+
+
+@pytest.mark.parametrize("cfg_name,fp_carrier", [("w8a8", False), ("w8a8", True), ("a16", True)])
+def test_forward_paths_that_are_not_split(gl, cfg_name, fp_carrier):
+    """They do all of a forward in phase 1 and launch nothing in phase 2."""
+    lib = cabi.load_library()
+    prob, params = calibrated((4, 3, 12, 64), seed=3, cfg=ol.make_config(**CONFIGS[cfg_name]), with_h0=True)
+    _, want = gl.forward_quant(*prob, params, training=False, fp_carrier=fp_carrier)
+    try:
+        lib.rxmet_set_forward_phase(1)
+        rc, first = gl.forward_quant(*prob, params, training=False, fp_carrier=fp_carrier)
+        assert rc == 0 and np.array_equal(first["h"], want["h"])
+        lib.rxmet_set_forward_phase(2)
+        before = lib.rxmet_kernel_launch_count()
+        assert gl.forward_quant(*prob, params, training=False, fp_carrier=fp_carrier)[0] == 0
+        assert lib.rxmet_kernel_launch_count() == before
+    finally:
+        lib.rxmet_set_forward_phase(0)
