@@ -1284,6 +1284,8 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
     const bool codesPath = qat && !registerPath && call.exec->weightClass == CodeClass::I8 && C % 4 == 0 && hpCodes <= 512 &&
                            codesSmem(1) + 1024 <= static_cast<size_t>(smemMax) && alignedTo(call.R_q, 16) &&
                            std::getenv("RXMET_GRU_BWD_GENERIC") == nullptr;
+    if (call.stepFlags && !registerPath && !codesPath)   // the kernels behind these two read byte masks
+        fail(RXMET_ERR_UNSUPPORTED, "packed step flags beyond 128 units need 16-byte aligned weight codes");
     if (codesPath) {
         BackwardCodesArgs ca{};
         BackwardQArgs &q = ca.q;

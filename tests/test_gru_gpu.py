@@ -776,3 +776,28 @@ def test_forward_paths_that_are_not_split(gl, cfg_name, fp_carrier):
         assert lib.rxmet_kernel_launch_count() == before
     finally:
         lib.rxmet_set_forward_phase(0)
+
+
+def test_packed_flags_are_never_left_out():
+    """Beyond 128 units the packed backward needs 16-byte aligned weight codes: the kernels for other addresses read byte masks, and
+    the call is refused where it would run on them."""
+    import torch
+    from rx_met_b200.qat import GruQatStep
+    from rx_met_b200.stacked_qat import a16_config
+    T, B, I, H = 3, 4, 12, 256
+    eng = GruQatStep(T, B, I, H, torch.device("cuda", 0), a16_config(8, 16), seed=5)
+    x = torch.randn((T, B, I), generator=torch.Generator().manual_seed(1)).cuda()
+    eng.calibrate([x * 0.6])
+    assert eng._packed
+    eng.forward(x)
+    eng.dh_new.fill_(1.0)
+    eng.backward()
+    aligned, want = eng.R_q, eng.flat_g.clone()
+    shifted = torch.empty(aligned.numel() + 1, dtype=torch.int32, device="cuda")[1:].view_as(aligned)
+    eng.R_q = shifted.copy_(aligned)
+    with pytest.raises(RuntimeError, match="aligned"):
+        eng.backward()
+    eng.R_q = aligned
+    eng.flat_g.zero_()
+    eng.backward()
+    assert torch.equal(eng.flat_g, want)
