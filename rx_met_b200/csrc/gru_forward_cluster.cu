@@ -393,9 +393,9 @@ bool prepare(const Exec &e, Prepared &cell) {
 
 }  // namespace
 
-bool forwardWideClusterTakes(const Exec &e, int H) {
+bool forwardWideClusterTakes(const Exec &e, int B, int H) {
     Prepared prepared;
-    return H <= 256 && prepare(e, prepared);
+    return H <= 256 && 4 * static_cast<uint64_t>(H) * B < (uint64_t{1} << 32) && prepare(e, prepared);   // offsets inside a step have 32 bits
 }
 
 void forwardWideCluster(const WideRecurrence &r, const Exec &e, cudaStream_t st) {

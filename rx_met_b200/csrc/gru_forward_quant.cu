@@ -2118,7 +2118,7 @@ void forwardFpCarrier(const ForwardQuantCall &call, const Exec &e, Workspace &ws
 
 bool packedFlagsSupported(const Exec &e, int B, int I, int H) {
     // 16-bit activations: the cluster recurrence packs them, for widths whose backward reads them
-    if (e.actClass == CodeClass::I16 && forwardWideTakes(e, I, H)) return (H <= 128 || H % 32 == 0) && forwardWideClusterTakes(e, H);
+    if (e.actClass == CodeClass::I16 && forwardWideTakes(e, I, H)) return (H <= 128 || H % 32 == 0) && forwardWideClusterTakes(e, B, H);
     if (e.weightClass != CodeClass::I8 || e.actClass != CodeClass::I8 || e.linearClass == CodeClass::I32) return false;
     if (std::getenv("RXMET_GRU_FWD_GENERIC") != nullptr || std::getenv("RXMET_GRU_FWD_BT") != nullptr) return false;
     const int sms = currentDevice().sms, C = 3 * H;
@@ -2141,7 +2141,7 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, 
     // 16-bit codes, and 8-bit ones too wide for the lanes path: the register path below holds R of 256 units in spilled
     // registers (H = 192, B = 500, T = 98: 666 us against 298 us over clusters)
     if (forwardWideTakes(e, call.I, call.H) &&
-        (a == CodeClass::I16 || (call.H > 128 && !call.stepFlags && forwardWideClusterTakes(e, call.H)))) {
+        (a == CodeClass::I16 || (call.H > 128 && !call.stepFlags && forwardWideClusterTakes(e, call.B, call.H)))) {
         runWide(call, e, ws, st);
         return;
     }

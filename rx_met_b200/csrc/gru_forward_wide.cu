@@ -441,7 +441,7 @@ void forwardWide(const WideCall &call, const Exec &e, cudaStream_t st) {
         a.maskHh = call.maskHh; a.maskGateIn = call.maskGateIn; a.maskGateOut = call.maskGateOut; a.maskH = call.maskH;
         a.poison = tensorProjection ? l.projStatus : nullptr;
         a.maskIh = call.maskIh; a.stepBits = call.stepBits;
-        if (forwardWideClusterTakes(e, H)) {
+        if (forwardWideClusterTakes(e, B, H)) {
             forwardWideCluster(a, e, st);
             return;
         }

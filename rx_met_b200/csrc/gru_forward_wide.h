@@ -57,7 +57,7 @@ struct WideRecurrence {
     const int *poison;         // status word of the tensor-core projection: non-zero turns the hidden outputs into NaN
 };
 // The recurrence over thread-block clusters (gru_forward_cluster.cu), and whether it takes the shape and the parameters.
-bool forwardWideClusterTakes(const Exec &exec, int H);
+bool forwardWideClusterTakes(const Exec &exec, int B, int H);
 void forwardWideCluster(const WideRecurrence &r, const Exec &exec, cudaStream_t stream);
 
 }  // namespace gru

@@ -314,3 +314,22 @@ def test_concurrent_passes_of_a_thread():
         assert lib.rxmet_concurrent_passes() == 3
     finally:
         lib.rxmet_set_concurrent_passes(1)
+
+
+def test_cluster_recurrence_keeps_to_32_bit_offsets():
+    """A step of v of 2^32 elements or more is not for the cluster recurrence, the one 16-bit path that packs the flags."""
+    H = 256
+    cfg = ol.make_config()
+    for op in range(len(cabi.OP_NAMES)):
+        cfg.bits[op] = 8 if cabi.OP_NAMES[op] in ("W", "R", "bw", "br") else 16
+    ranges, params = ol.RangesBox(H), ol.ParamsBox(H, cfg)
+    for op in range(len(cabi.OP_NAMES)):
+        ranges.c.min[op], ranges.c.max[op] = -1.0, 1.0
+    for name in ("W", "R", "bw", "br"):
+        for c in range(3 * H):
+            getattr(ranges.c, "min_" + name)[c], getattr(ranges.c, "max_" + name)[c] = -0.5, 0.5
+    lib = cabi.load_library()
+    assert lib.rxmet_gru_params_from_ranges(C.byref(ranges.c), C.byref(cfg), C.byref(params.c)) == 0
+    supported = lambda B: lib.rxmet_gru_packed_flags_supported(C.byref(params.c), B, 40, H)  # noqa: E731
+    assert supported(128) == supported((1 << 22) - 1) == 1
+    assert supported(1 << 22) == 0
