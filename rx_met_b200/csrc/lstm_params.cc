@@ -15,6 +15,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <system_error>
 
 #include "common.h"
 
@@ -340,11 +341,20 @@ void buildTable(const rxmet_lstm_quant_params &p, int inOp, int outOp, bool isTa
     }
 }
 
-// job(table) for all tables, on threads of their own where that pays; whether all returned true.
+// job(table) for all tables, on threads of their own where that pays and the system has them; whether all returned true.
 template <class Job>
 bool forEachTable(bool threads, Job &&job) {
     std::array<std::future<bool>, kTables> running;
-    for (int t = 1; t < kTables; ++t) running[t] = std::async(threads ? std::launch::async : std::launch::deferred, job, t);
+    for (int t = 1; t < kTables; ++t) {
+        if (threads) {
+            try {
+                running[t] = std::async(std::launch::async, job, t);
+                continue;
+            } catch (const std::system_error &) {
+            }
+        }
+        running[t] = std::async(std::launch::deferred, job, t);
+    }
     bool good = job(0);
     for (int t = 1; t < kTables; ++t) good = running[t].get() && good;
     return good;

@@ -302,3 +302,60 @@ def test_library_default_config_and_config_json():
     assert lib.rxmet_lstm_ranges_fold_stats(C.byref(box.struct), stats.ctypes.data_as(C.POINTER(C.c_float)), H, 1) == 0
     assert (box.struct.minimum[L.INPUT], box.struct.maximum[L.INPUT]) == (-2.0, 5.0)
     assert box.struct.minimum[L.OUTPUT] == np.inf  # untouched slots stay empty
+
+
+TABLES_WITHOUT_THREADS = r"""
+#include <atomic>
+#include <cerrno>
+#include <cstdio>
+#include <pthread.h>
+#include <vector>
+#include "common.h"
+#include "lstm_params.h"
+
+// No thread to be had: the program's own definition comes before the C library's.
+static int refused = 0;
+extern "C" int pthread_create(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *) { ++refused; return EAGAIN; }
+
+namespace rxmet {
+std::string &lastError() { static std::string text; return text; }
+std::atomic<uint64_t> &launchCounter() { static std::atomic<uint64_t> n{0}; return n; }
+std::shared_ptr<void> copyToDevice(const void *, size_t) { return nullptr; }
+void keepForCapture(const std::shared_ptr<void> &, cudaStream_t) {}
+}
+extern "C" cudaError_t cudaGetDevice(int *) { return cudaSuccess; }
+extern "C" const char *cudaGetErrorString(cudaError_t) { return ""; }
+
+int main() {
+    using namespace rxmet::lstm;
+    const int H = 4;
+    rxmet_lstm_quant_config cfg;
+    defaultConfig(&cfg);
+    for (int op = 0; op < RXMET_LSTM_NUM_OPS; ++op)
+        if (op < RXMET_LSTM_WEIGHT_IH || op > RXMET_LSTM_BIAS_HH) cfg.bitwidth[op] = 16;
+    rxmet_lstm_ranges ranges{};
+    std::vector<float> low(4 * H, -0.5f), high(4 * H, 0.5f), scales[4];
+    for (int op = 0; op < RXMET_LSTM_NUM_OPS; ++op) { ranges.minimum[op] = -1.0f; ranges.maximum[op] = 1.0f; }
+    for (int s = 0; s < 4; ++s) { ranges.channel_min[s] = low.data(); ranges.channel_max[s] = high.data(); scales[s].resize(4 * H); }
+    rxmet_lstm_quant_params params;
+    paramsFromRanges(cfg, ranges, 3, H, true, scales[0].data(), scales[1].data(), scales[2].data(), scales[3].data(), &params);
+    const auto exec = deriveExec(params, false);
+    std::printf("%d %zu %d\n", refused, exec->wide.entries.size(), exec->compactTables().ok ? 1 : 0);
+    return 0;
+}
+"""
+
+
+def test_activation_tables_without_threads(tmp_path):
+    """The tables of 16-bit grids are built on threads; a process that gets none builds them all the same."""
+    import subprocess
+    root = Path(__file__).resolve().parent.parent
+    source, program = tmp_path / "tables.cc", tmp_path / "tables"
+    source.write_text(TABLES_WITHOUT_THREADS)
+    csrc = root / "rx_met_b200" / "csrc"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", f"-I{root / 'include'}", f"-I{csrc}", "-I/usr/local/cuda/include", str(source),
+                    str(csrc / "lstm_params.cc"), "-o", str(program)], check=True)
+    done = subprocess.run([str(program)], capture_output=True, text=True, timeout=120)
+    assert done.returncode == 0, done.stderr[-500:]
+    refused, entries, compact = map(int, done.stdout.split())
+    assert refused > 0 and entries == 5 << 16 and compact == 1
