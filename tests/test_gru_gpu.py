@@ -188,11 +188,47 @@ def test_backward_quant(gl, cfg_name, shape):
 
 
 @pytest.mark.parametrize("shape", [(1, 1, 8, 96), (2, 5, 8, 128), (3, 9, 8, 160), (4, 17, 8, 192), (5, 3, 12, 224), (3, 300, 8, 256),
-                                   (2, 130, 8, 64), (2, 260, 8, 32)], ids=lambda s: "x".join(map(str, s)))
+                                   (2, 130, 8, 64), (2, 260, 8, 32), (5, 19, 40, 256)], ids=lambda s: "x".join(map(str, s)))
 def test_backward_quant_over_clusters(gl, shape):
-    """Every width the cluster recurrence is built for (32 and 64 units per CTA), 4, 8 and 16 rows per cluster with the
-    last cluster partly empty, and sequences shorter than its three-step operand ring."""
+    """Clusters of one to four CTAs of 64 units, which all widths that 64 does not divide reach through padded copies; 4, 8 and 16 rows
+    per cluster with the last cluster partly empty, and sequences shorter than the three-step operand ring."""
     test_backward_quant(gl, "w8a8" if shape[3] <= 128 else "a16", shape)
+
+
+@pytest.mark.parametrize("shape", [(2, 260, 516, 32), (3, 9, 516, 96), (4, 17, 516, 160), (2, 7, 516, 224)], ids=lambda s: "x".join(map(str, s)))
+def test_backward_quant_over_clusters_of_32_units_a_cta(gl, shape):
+    """Beyond 512 inputs there are no padded copies: odd multiples of 32 units run on clusters of CTAs of 32."""
+    test_backward_quant(gl, "w8a8" if shape[3] <= 128 else "a16", shape)
+
+
+@pytest.mark.parametrize("shape", [(3, 5, 8, 64), (3, 5, 8, 128), (2, 5, 516, 96), (3, 19, 8, 256)], ids=lambda s: "x".join(map(str, s)))
+def test_backward_quant_of_misaligned_tensors(gl, monkeypatch, shape):
+    """h and dh_new four bytes beside the boundary of the cluster kernels' paired accesses: the one-CTA recurrences."""
+    import torch
+    given, T = gl.dev, shape[0]
+
+    def shifted(a):
+        t = given(a)
+        if a is None or a.dtype != np.float32 or a.ndim != 3 or a.shape[0] != T + 1:
+            return t
+        return torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t)
+
+    monkeypatch.setattr(gl, "dev", shifted)
+    test_backward_quant(gl, "w8a8" if shape[3] <= 128 else "a16", shape)
+
+
+@pytest.mark.parametrize("shape", [(3, 4, 9, 300), (2, 150, 8, 512), (3, 5, 7, 257)], ids=lambda s: "x".join(map(str, s)))
+def test_forward_quant_planes_beyond_the_clusters(gl, shape):
+    """W8 / A16 beyond 256 units: one CTA per tile of rows, the product on dp4a."""
+    test_forward_quant_matches_restatement(gl, "a16", shape)
+
+
+@pytest.mark.parametrize("variable,value", [("RXMET_GRU_FWD_MODE", "0"), ("RXMET_GRU_FWD_MODE", "1"), ("RXMET_GRU_FWD_BT", "2")])
+@pytest.mark.parametrize("shape", [(3, 4, 12, 64), (3, 7, 9, 128), (2, 5, 8, 40)], ids=lambda s: "x".join(map(str, s)))
+def test_forward_quant_general_cells(gl, monkeypatch, shape, variable, value):
+    """The one-thread-per-channel recurrence with the cells for grids that the lanes do not take, asked for by their switches."""
+    monkeypatch.setenv(variable, value)
+    test_forward_quant_matches_restatement(gl, "w8a8", shape)
 
 
 @pytest.mark.parametrize("shape", [(80, 256, 40, 128), (80, 256, 72, 64)], ids=lambda s: "x".join(map(str, s)))
@@ -442,23 +478,6 @@ def test_kws_body_layer_shapes(gl, cfg_name, shape):
     dh_new = np.zeros((T + 1, B, H), np.float32)
     dh_new[1:] = np.random.default_rng(I).standard_normal((T, B, H)).astype(np.float32)
     wb = ol.backward_quant(want, dh_new, want["h"], want["v"], params, want["masks"])
-    gb = gl.backward_quant(want, dh_new, want["h"], want["v"], params, want["masks"].arr)
-    for k in wb:
-        close(gb[k], wb[k], what=k)
-
-
-def test_cluster_backward_kernel_agrees(gl, monkeypatch):
-    """The opt-in backward recurrence over clusters of eight CTAs (weights in registers, gate gradients exchanged
-    through distributed shared memory) gives the gradients of the default kernel; a batch that leaves rows of
-    the last cluster empty."""
-    T, B, I, H = 5, 19, 40, 256
-    cfg = ol.make_config(**CONFIGS["a16"])
-    prob, params = calibrated((T, B, I, H), seed=77, cfg=cfg, with_h0=True, x_scale=1.2)
-    want = ol.forward_quant("orc", *prob, params, training=True)
-    dh_new = np.zeros((T + 1, B, H), np.float32)
-    dh_new[1:] = np.random.default_rng(5).standard_normal((T, B, H)).astype(np.float32)
-    wb = ol.backward_quant(want, dh_new, want["h"], want["v"], params, want["masks"])
-    monkeypatch.setenv("RXMET_GRU_BWD_CLUSTER", "1")
     gb = gl.backward_quant(want, dh_new, want["h"], want["v"], params, want["masks"].arr)
     for k in wb:
         close(gb[k], wb[k], what=k)

@@ -183,3 +183,17 @@ def test_wide_qat_backward_of_many_steps_beyond_256_units(H):
     over enough steps for the CTAs of a cluster to drift apart: nobody may write the next step's operand before the whole product is
     through.  60 steps of two roundings of 2^-24 each in the carried gradient stay below 1e-5, half the tolerance."""
     test_wide_qat_backward(60, 9, 8, H, 8, 16)
+
+
+@pytest.mark.parametrize("switch", ["RXMET_LSTM_REC_SIMT", "RXMET_LSTM_REC_UMMA"])
+def test_wide_forward_without_compact_tables(switch):
+    """The recurrences for activation tables that have no compact form or grids of 2^22 and more: dp4a, and the tensor-core kernel over
+    the whole grid.  The switches that ask for them are read once per process."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    here = Path(__file__).resolve()
+    done = subprocess.run([sys.executable, "-m", "pytest", "-q", "-m", "gpu", f"{here}::test_wide_forward_is_bit_exact"], cwd=here.parent.parent,
+                          capture_output=True, text=True, env=dict(os.environ, **{switch: "1"}), timeout=300)
+    assert done.returncode == 0, done.stdout[-2000:]
