@@ -134,8 +134,10 @@ int residentPerSm(const void *kernel, int block, size_t smem);
 // Device copy of host bytes, for constants that outlive a call.  Complete when it returns, and allowed while this or another
 // stream is being captured.
 std::shared_ptr<void> copyToDevice(const void *host, size_t bytes);
-// While `stream` is being captured: keeps `block` for the life of the process, because the graph refers to it at every replay.
-void keepForCapture(const std::shared_ptr<void> &block, cudaStream_t stream);
+// Whether `stream` is being captured: about a microsecond, so once a call.
+bool isCapturing(cudaStream_t stream);
+// Keeps a block that a captured call was given for the life of the process, because the graph refers to it at every replay.
+void keepForGraph(const std::shared_ptr<void> &block);
 // Clusters of `ctas` CTAs of `kernel` that the device holds at the same time (0 when it holds none), asked once per
 // device and configuration.
 int residentClusters(const void *kernel, int ctas, int block, size_t smem);

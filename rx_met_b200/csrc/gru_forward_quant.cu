@@ -64,7 +64,7 @@ const int32_t *channelBlockOnDevice(const Exec &e, cudaStream_t st) {
         const std::vector<int32_t> host = channelBlock(e);
         at = e.deviceChannels.emplace(at, device, copyToDevice(host.data(), host.size() * sizeof(int32_t)));
     }
-    keepForCapture(at->second, st);
+    if (isCapturing(st)) keepForGraph(at->second);
     return static_cast<const int32_t *>(at->second.get());
 }
 

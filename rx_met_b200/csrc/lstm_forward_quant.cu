@@ -454,8 +454,9 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, 
     uint32_t *wIh, *wHh;
     int32_t *addIh, *addHh;
     layout(ws, T, B, I, H, &xq, &h0q, &c0c, &wIh, &wHh, &addIh, &addHh, &lhs);
-    const float *channel = e.channelOnDevice(st);
-    const int32_t *tables = e.tablesOnDevice(st);
+    const bool captured = isCapturing(st);
+    const float *channel = e.channelOnDevice(captured);
+    const int32_t *tables = e.tablesOnDevice(captured);
 
     const rxmet_lstm_masters none{};
     const rxmet_lstm_masters &m = call.masters ? *call.masters : none;

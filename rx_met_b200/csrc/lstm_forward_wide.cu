@@ -983,8 +983,9 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
     const size_t rows = static_cast<size_t>(T) * B;
     Workspace ws(workspace, workspaceBytes);
     WideLayout l = layoutWide(ws, T, B, I, H, planes);
-    const int32_t *tables = e.wideTablesOnDevice(st);
-    l.channel = e.channelOnDevice(st);
+    const bool captured = isCapturing(st);
+    const int32_t *tables = e.wideTablesOnDevice(captured);
+    l.channel = e.channelOnDevice(captured);
 
     const rxmet_lstm_masters none{};
     const rxmet_lstm_masters &m = call.masters ? *call.masters : none;
@@ -1095,7 +1096,7 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
         auto run = [&](auto cell) {
             const CompactTables &t = e.compactTables();
             cell.s = s; cell.width = H; cell.kWords = kHh; cell.B = static_cast<size_t>(B);
-            cell.segShift = t.segShift; cell.tableBytes = static_cast<int>(t.bytes.size()); cell.tables = e.compactTablesOnDevice(st);
+            cell.segShift = t.segShift; cell.tableBytes = static_cast<int>(t.bytes.size()); cell.tables = e.compactTablesOnDevice(captured);
             for (int i = 0; i < kTables; ++i) {
                 cell.segOffset[i] = t.segOffset[i]; cell.bitOffset[i] = t.bitOffset[i]; cell.flagBelow[i] = t.flagBelow[i];
                 cell.flagFrom[i] = t.flagFrom[i]; cell.inLo[i] = t.inLo[i]; cell.outLo[i] = t.outLo[i]; cell.outHi[i] = t.outHi[i];

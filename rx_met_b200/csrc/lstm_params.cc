@@ -590,7 +590,7 @@ std::shared_ptr<const float> weightScalesOnDevice(const rxmet_lstm_quant_params 
     if (cache.size() > 64) cache.clear();
     std::shared_ptr<void> &block = cache[key];
     if (!block) block = copyToDevice(key.second.data(), key.second.size() * sizeof(float));
-    keepForCapture(block, stream);
+    if (isCapturing(stream)) keepForGraph(block);
     return std::static_pointer_cast<const float>(block);
 }
 
@@ -699,7 +699,7 @@ const CompactTables &Exec::compactTables() const {
 namespace {
 
 // Device copy of host bytes, one per device, kept with the Exec.
-const void *deviceCopy(std::mutex &mutex, Exec::DeviceCopies &copies, const void *host, size_t bytes, cudaStream_t stream) {
+const void *deviceCopy(std::mutex &mutex, Exec::DeviceCopies &copies, const void *host, size_t bytes, bool captured) {
     int device = 0;
     RXMET_CUDA(cudaGetDevice(&device));
     std::lock_guard<std::mutex> lock(mutex);
@@ -708,26 +708,26 @@ const void *deviceCopy(std::mutex &mutex, Exec::DeviceCopies &copies, const void
         RXMET_REQUIRE(bytes > 0, "the parameter set has no such table");
         at = copies.emplace(copies.end(), device, copyToDevice(host, bytes));
     }
-    keepForCapture(at->second, stream);
+    if (captured) keepForGraph(at->second);
     return at->second.get();
 }
 
 }  // namespace
 
-const int32_t *Exec::wideTablesOnDevice(cudaStream_t stream) const {
-    return static_cast<const int32_t *>(deviceCopy(deviceLock, deviceTables, wide.entries.data(), wide.entries.size() * sizeof(int32_t), stream));
+const int32_t *Exec::wideTablesOnDevice(bool captured) const {
+    return static_cast<const int32_t *>(deviceCopy(deviceLock, deviceTables, wide.entries.data(), wide.entries.size() * sizeof(int32_t), captured));
 }
 
-const float *Exec::channelOnDevice(cudaStream_t stream) const {
-    return static_cast<const float *>(deviceCopy(deviceLock, deviceChannel, channel.data(), channel.size() * sizeof(float), stream));
+const float *Exec::channelOnDevice(bool captured) const {
+    return static_cast<const float *>(deviceCopy(deviceLock, deviceChannel, channel.data(), channel.size() * sizeof(float), captured));
 }
 
-const int32_t *Exec::tablesOnDevice(cudaStream_t stream) const {
-    return static_cast<const int32_t *>(deviceCopy(deviceLock, deviceSmallTables, tables.data(), tables.size() * sizeof(int32_t), stream));
+const int32_t *Exec::tablesOnDevice(bool captured) const {
+    return static_cast<const int32_t *>(deviceCopy(deviceLock, deviceSmallTables, tables.data(), tables.size() * sizeof(int32_t), captured));
 }
 
-const uint8_t *Exec::compactTablesOnDevice(cudaStream_t stream) const {
-    return static_cast<const uint8_t *>(deviceCopy(deviceLock, deviceCompact, compactTables().bytes.data(), compactTables().bytes.size(), stream));
+const uint8_t *Exec::compactTablesOnDevice(bool captured) const {
+    return static_cast<const uint8_t *>(deviceCopy(deviceLock, deviceCompact, compactTables().bytes.data(), compactTables().bytes.size(), captured));
 }
 
 }  // namespace lstm

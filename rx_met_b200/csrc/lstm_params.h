@@ -114,11 +114,11 @@ struct Exec {
     // The compact form of the wide tables, built on first use.
     const CompactTables &compactTables() const;
     // Copies of wide.entries, the compact tables, `channel` and `tables` on the current device: made on first use, also inside a
-    // capture of `stream`, and freed with the Exec, or never once a graph refers to them.
-    const int32_t *wideTablesOnDevice(cudaStream_t stream) const;
-    const uint8_t *compactTablesOnDevice(cudaStream_t stream) const;
-    const float *channelOnDevice(cudaStream_t stream) const;
-    const int32_t *tablesOnDevice(cudaStream_t stream) const;
+    // capture, and freed with the Exec, or never once a captured call was given them.
+    const int32_t *wideTablesOnDevice(bool captured) const;
+    const uint8_t *compactTablesOnDevice(bool captured) const;
+    const float *channelOnDevice(bool captured) const;
+    const int32_t *tablesOnDevice(bool captured) const;
     using DeviceCopies = std::vector<std::pair<int, std::shared_ptr<void>>>;   // (device ordinal, buffer)
     mutable std::once_flag compactOnce;
     mutable CompactTables compact;

@@ -321,7 +321,8 @@ namespace rxmet {
 std::string &lastError() { static std::string text; return text; }
 std::atomic<uint64_t> &launchCounter() { static std::atomic<uint64_t> n{0}; return n; }
 std::shared_ptr<void> copyToDevice(const void *, size_t) { return nullptr; }
-void keepForCapture(const std::shared_ptr<void> &, cudaStream_t) {}
+bool isCapturing(cudaStream_t) { return false; }
+void keepForGraph(const std::shared_ptr<void> &) {}
 }
 extern "C" cudaError_t cudaGetDevice(int *) { return cudaSuccess; }
 extern "C" const char *cudaGetErrorString(cudaError_t) { return ""; }
