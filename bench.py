@@ -46,7 +46,7 @@ def _algo_bytes_per_st(I, H):
 
 # DRAM traffic per launch of the recurrent kernels at this workload, from the ncu captures
 # summarised under profiles/ (dram__bytes_read.sum + dram__bytes_write.sum, one launch).
-NCU_TRAFFIC_BYTES = {"recurrentForward": 19.80e6 + 42.90e6, "recurrentBackward": 85.42e6 + 40.81e6}
+NCU_TRAFFIC_BYTES = {"recurrentForward": 29.62e6 + 18.50e6, "recurrentBackward": 85.43e6 + 40.17e6}
 
 
 def _peaks():

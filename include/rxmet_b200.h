@@ -489,8 +489,9 @@ RXMET_API int rxmet_gru_forward_quant_fp_carrier(int is_training, int T, int B, 
  * recurrence folds into the word; its other four per-step members may be NULL and are not written then.
  * Results are identical to the byte-mask pair.  For training engines that own their save-for-backward
  * buffers (rx_met_b200.qat.GruQatStep); the reference's binding hands byte masks to Python and has no
- * counterpart.  Supported where rxmet_gru_packed_flags_supported returns 1 (8-bit grids, H <= 128);
- * RXMET_ERR_UNSUPPORTED otherwise. */
+ * counterpart.  Supported where rxmet_gru_packed_flags_supported returns 1 (8-bit grids, H <= 128; 8-bit
+ * weights with activations of 9 to 16 bits, H <= 256 and, beyond 128, a multiple of 32, whose backward wants
+ * R_q_dev on 16 bytes); RXMET_ERR_UNSUPPORTED otherwise. */
 RXMET_API int rxmet_gru_packed_flags_supported(const rxmet_gru_quant_params *params, int B, int I, int H);
 RXMET_API int rxmet_gru_forward_quant_packed(int T, int B, int I, int H,
                                              const float *W_dev, const float *R_dev,

@@ -10,10 +10,11 @@
 // Everything after the sum is the reference's integer arithmetic unchanged (64-bit rounding rescales,
 // piecewise-linear activation tables, clamp flags).
 //
-// Launches (after the shared quantization of weights, x and h0 into one code per element):
-//   packWeightWords  : int8 codes [K][3H] -> words of four along K, per-channel addends
-//   planesFromCodes  : int16 codes -> byte planes (x for all steps, h0)
-//   inputLinearPlanes: all T*B rows of the input projection, persistent CTAs, cp.async staging
+// Launches:
+//   prepareWide      : packed weight words and tiles, addends, x and h0 as byte planes (gru_forward_quant.cu)
+//   planeProjUmma    : all T*B rows of the input projection on the tensor cores (plane_proj_umma.cuh), or
+//   inputLinearPlanes: the same on dp4a where its operands exceed shared memory: persistent CTAs, cp.async staging
+//   the recurrence over clusters or in lanes (gru_forward_cluster.cu) up to 256 units and the usual shifts, else
 //   recurrentPlanes  : ONE launch for all T steps; thread (j, s) owns hidden unit j - all three gates - for
 //                      RB batch rows of row group s, keeps those rows' hidden codes in registers, reads the
 //                      packed recurrent weights from shared memory (3H x H bytes: fits up to H = 256) or

@@ -688,7 +688,7 @@ bool buildCompact(const Exec &e, int segShift, CompactTables &out) {
 const CompactTables &Exec::compactTables() const {
     std::call_once(compactOnce, [&] {
         if (wide.entries.empty()) return;
-        // 8, 16, 32 kB of lines per 16-bit table beside 8 kB of bits; small tables take as many lines as they need
+        // 4, 8, 16 kB of lines per 16-bit table beside 8 kB of bits; small tables take as many lines as they need
         for (int segShift = 7; segShift >= (wide.entries.size() > 8192 ? 5 : 0); --segShift)
             if (buildCompact(*this, segShift, compact)) return;
         compact = CompactTables{};

@@ -204,7 +204,8 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
                                 sendBar + ((t + 1) & 1) * 8);
         }
     } else {
-        // units beyond the layer's width compute on zero weights and store nothing; their operand bytes stay zero
+        // Units beyond the layer's width compute on zero weights and store nothing.  Where a step leaves no row out (kAll) their codes
+        // reach the operand all the same; they meet zero weights there too, those of every k >= H.
         const bool real = Cell::kFull || unit < H;
         const bool valid = c.valid();
         // rows of phase A in one go: as many as the operator allows and the rows divide into
