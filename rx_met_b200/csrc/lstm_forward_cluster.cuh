@@ -20,8 +20,8 @@
 #include "common.h"
 #include "lstm_device.cuh"
 #include "lstm_kernels.h"
-#include "lane_recurrence.cuh"
 #include "plane_recurrence_umma.cuh"
+#include "unit_recurrence_umma.cuh"
 
 namespace rxmet {
 namespace lstm {
@@ -42,9 +42,9 @@ __device__ __forceinline__ float lookup(const TableView &v, int segShift, float 
     asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(slope), "=f"(intercept) : "r"(v.segments + ((index >> segShift) << 3)));
     uint32_t word;
     asm("ld.shared.u32 %0, [%1];" : "=r"(word) : "r"(v.bits + ((index >> 5) << 2)));
-    float y = roundSmall(__fmaf_rn(slope, x, intercept));
-    if ((word >> (index & 31u)) & 1u) y = __fadd_rn(y, 1.0f);
-    return clampF(y, v.outLo, v.outHi);
+    // the bit of an input is bit 31 - (index & 31): shifted to the top it is added to the rounded value's last place, which is 1
+    const uint32_t rounded = __float_as_uint(__fadd_rn(__fmaf_rn(slope, x, intercept), kRoundMagic)) + (__funnelshift_l(0u, word, index) >> 31);
+    return clampF(__fadd_rn(__uint_as_float(rounded), -kRoundMagic), v.outLo, v.outHi);
 }
 
 // WIDTH: the hidden size where it is a compile-time constant, else 0.
@@ -160,17 +160,21 @@ struct LstmPlaneCell {
         f.lhs = __ldg(lhs + (at + static_cast<size_t>(row)) * (4 * static_cast<size_t>(H)) + (gate * H + unit));
     }
     __device__ __forceinline__ void fetchB(FetchB &, size_t, uint32_t, int) const {}
-    // the sums of ROWS rows as floats, in place of the plane sums; one branch for all of them
+    // the sum of the planes as a float; NARROW: it fits 32 bits
+    template <int PLANES, bool NARROW>
+    __device__ __forceinline__ uint32_t total(const Lane &l, uint32_t high, uint32_t low) const {
+        if (NARROW) return __float_as_uint(__int2float_rn(static_cast<int32_t>((PLANES == 2 ? high * 256u : 0u) + low + static_cast<uint32_t>(l.addend))));
+        return __float_as_uint(__ll2float_rn((PLANES == 2 ? static_cast<int64_t>(static_cast<int32_t>(high)) << 8 : 0) + static_cast<int32_t>(low) + l.addend));
+    }
+    // the same for ROWS rows, in place of the plane sums; one branch for all of them
     template <int STRIDE, int ROWS>
     __device__ __forceinline__ void totals(const Lane &l, uint32_t *acc) const {
         if (l.narrow) {
 #pragma unroll
-            for (int r = 0; r < ROWS; ++r)
-                acc[r] = __float_as_uint(__int2float_rn(static_cast<int32_t>(acc[r] * 256u + acc[r + STRIDE] + static_cast<uint32_t>(l.addend))));
+            for (int r = 0; r < ROWS; ++r) acc[r] = total<2, true>(l, acc[r], acc[r + STRIDE]);
         } else {
 #pragma unroll
-            for (int r = 0; r < ROWS; ++r)
-                acc[r] = __float_as_uint(__ll2float_rn((static_cast<int64_t>(static_cast<int32_t>(acc[r])) << 8) + static_cast<int32_t>(acc[r + STRIDE]) + l.addend));
+            for (int r = 0; r < ROWS; ++r) acc[r] = total<2, false>(l, acc[r], acc[r + STRIDE]);
         }
     }
     // gate output (centred code as a float)
@@ -211,15 +215,10 @@ struct LstmPlaneCell {
         const int i = static_cast<int>(index & 0x7fffffu);
         return i < flagBelow[t] || i >= flagFrom[t];
     }
-    // LANES lanes hold the same cell and share its stores, `part` of them is this one's
-    template <int LANES = 1>
-    __device__ __forceinline__ void store(const State &st, const FetchB &, size_t at, uint32_t row, int unit, bool good, int part = 0) const {
+    __device__ __forceinline__ void store(const State &st, const FetchB &, size_t at, uint32_t row, int unit, bool good) const {
         const int H = hidden();
         const size_t o = at * H + (row * H + unit);
-        if (LANES == 1 || part == 0) output[o] = __fmul_rn(st.hidden, scaleH(good));
-        if (TRAIN && LANES > 1) {
-            if (part != LANES - 1) return;
-        }
+        output[o] = __fmul_rn(st.hidden, scaleH(good));
         if (TRAIN) {
             if (ck.cell_states) ck.cell_states[o] = st.cell + s.zpF[RXMET_LSTM_CELL_STATE];
             if (ck.cell_states_clamped) ck.cell_states_clamped[o] = static_cast<uint8_t>(st.flags & 1u);
@@ -293,40 +292,191 @@ struct LstmPlaneCell {
     }
 };
 
-// Rows: a step of n rows costs about 1 + n / 5 of the chain of a one-row step.
+// What a forward saves beside its outputs: nothing, some of the checkpoints, all of them.
+enum class Saves { None, Some, All };
+
+// The same cell with all gates of a unit in one thread (unit_recurrence_umma.cuh), one or two byte planes.  What is the same for all
+// units is prepared on the host and read as constants: registers of a thread decide how many rows an SM has in flight.
+struct LstmUnitConstants {
+    struct Table {
+        float toIndex, outLo, outHi;
+        uint32_t segments, bits;          // offsets, moved by the exponent bits that an index carries
+        uint32_t flagBelow, flagCount;    // clamped: index - flagBelow >= flagCount
+    } table[kTables];
+    float gateScale[4], giLo[4], giHi[4], zpIn[4], zpOut[4];
+    float hhLo, hhHi, cLo, cHi, oLo, oHi, productScale, codePlus;
+    int plain;                            // the cell's ratios are single factors
+};
+template <Saves SAVES, int WIDTH = 0>
+struct LstmUnitCell : LstmPlaneCell<SAVES != Saves::None, WIDTH> {
+    static constexpr bool kTrain = SAVES != Saves::None, kTwoRows = !kTrain;
+    using Base = LstmPlaneCell<kTrain, WIDTH>;
+    LstmUnitConstants k;
+    struct Unit {
+        int64_t addend[4];
+        float outScale[4];
+        bool narrow[4], plain;            // uniform in the warp: the sum fits 32 bits; all of them and k.plain
+        uint32_t shared;
+    };
+    struct State {
+        float cell, hidden;
+    };
+    struct Fetch {
+        float lhs[4];
+    };
+    struct Out {
+        float hh[4], sum[4], gate[4];   // hh before its clamp, gate input before its clamp, gate output
+        uint32_t index[5];
+        float cellRaw, cell, tanhC, hiddenRaw, hidden;   // Raw: before the clamp
+    };
+    // host: everything of k from the fields of the base
+    void prepareConstants() {
+        const auto &s = this->s;
+        auto low = [&](int op) { return static_cast<float>(s.lo[op] - s.zp[op]); };
+        auto high = [&](int op) { return static_cast<float>(s.hi[op] - s.zp[op]); };
+        constexpr uint32_t kExponent = 0x4B000000u;   // of 2^23
+        for (int t = 0; t < kTables; ++t)
+            k.table[t] = {8388608.0f - this->inLo[t], this->outLo[t], this->outHi[t], static_cast<uint32_t>(this->segOffset[t]) - ((kExponent >> this->segShift) << 3),
+                          static_cast<uint32_t>(this->bitOffset[t]) - ((kExponent >> 5) << 2), kExponent + static_cast<uint32_t>(this->flagBelow[t]),
+                          static_cast<uint32_t>(this->flagFrom[t] - this->flagBelow[t])};
+        for (int g = 0; g < 4; ++g) {
+            const int in = RXMET_LSTM_INPUT_GATE_INPUT + g;
+            k.gateScale[g] = s.hhToGate[g].mult * s.hhToGate[g].pow2;
+            k.giLo[g] = low(in); k.giHi[g] = high(in);
+            k.zpIn[g] = s.zpF[in]; k.zpOut[g] = s.zpF[RXMET_LSTM_INPUT_GATE_OUTPUT + g];
+        }
+        k.hhLo = low(RXMET_LSTM_WEIGHT_HH_LINEAR); k.hhHi = high(RXMET_LSTM_WEIGHT_HH_LINEAR);
+        k.cLo = low(RXMET_LSTM_CELL_STATE); k.cHi = high(RXMET_LSTM_CELL_STATE);
+        k.oLo = low(RXMET_LSTM_OUTPUT); k.oHi = high(RXMET_LSTM_OUTPUT);
+        k.productScale = s.productToOutput.mult * s.productToOutput.pow2;
+        k.codePlus = 8388608.0f + static_cast<float>(s.zp[RXMET_LSTM_OUTPUT] - s.lo[RXMET_LSTM_OUTPUT]);
+        k.plain = !s.forgetUsesFp && !s.inputUsesFp;
+    }
+    __device__ __forceinline__ void init(uint8_t *at, uint32_t, int tid, int threads) const { Base::init(at, tid, threads); }
+    __device__ __forceinline__ Unit unitOf(uint32_t shared, int unit) const {
+        Unit u;
+        u.shared = shared;
+        u.plain = k.plain;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const typename Base::Lane l = Base::lane(shared, g, unit, true);
+            u.addend[g] = l.addend;
+            u.outScale[g] = l.outScale;
+            u.narrow[g] = l.narrow;
+            u.plain = u.plain && l.narrow;
+        }
+        return u;
+    }
+    __device__ __forceinline__ void begin(State &st, int row, int unit) const {
+        st.cell = this->c0[static_cast<size_t>(row) * this->hidden() + unit];
+        st.hidden = 0.0f;
+    }
+    __device__ __forceinline__ void fetch(Fetch &f, size_t at, uint32_t row, int unit) const {
+        const uint32_t H = this->hidden(), mine = row * (4 * H) + unit;
+        const float *from = this->lhs + at * (4 * H);
+#pragma unroll
+        for (int g = 0; g < 4; ++g) f.lhs[g] = __ldg(from + g * H + mine);
+    }
+    // as Base::quantized, with the value before the clamp to the grid where flags are asked for
+    __device__ __forceinline__ float rounded(float x, float lo, float hi) const {
+        return kTrain ? roundSmall(clampF(x, lo - 1.0f, hi + 1.0f)) : roundSmall(clampF(x, lo, hi));
+    }
+    __device__ __forceinline__ float activation(const Unit &u, int t, float x, uint32_t &index) const {
+        const LstmUnitConstants::Table &v = k.table[t];
+        return lookup(TableView{u.shared + v.segments, u.shared + v.bits, v.toIndex, v.outLo, v.outHi}, this->segShift, x, index);
+    }
+    template <int PLANES, bool PLAIN>
+    __device__ __forceinline__ uint32_t advance(const Unit &u, State &st, const Fetch &in, const uint32_t (&acc)[4][PLANES], Out &o) const {
+        const auto &s = this->s;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            typename Base::Lane l;
+            l.addend = u.addend[g];
+            const uint32_t bits = PLAIN || u.narrow[g] ? Base::template total<PLANES, true>(l, acc[g][0], acc[g][PLANES - 1])
+                                                       : Base::template total<PLANES, false>(l, acc[g][0], acc[g][PLANES - 1]);
+            o.hh[g] = rounded(__fmul_rn(__uint_as_float(bits), u.outScale[g]), k.hhLo, k.hhHi);
+            const float hh = kTrain ? clampF(o.hh[g], k.hhLo, k.hhHi) : o.hh[g];
+            o.sum[g] = __fadd_rn(in.lhs[g], roundSmall(__fmul_rn(hh, k.gateScale[g])));
+            o.gate[g] = activation(u, g, clampF(o.sum[g], k.giLo[g], k.giHi[g]), o.index[g]);
+        }
+        const float pf = __fmul_rn(o.gate[1], st.cell), pi = __fmul_rn(o.gate[0], o.gate[2]);
+        const float sf = PLAIN ? __fmul_rn(pf, s.forgetRatio) : dev::scaleCell(pf, s.forgetRatio, s.forgetMantissa, s.forgetExponent, s.forgetUsesFp);
+        const float si = PLAIN ? __fmul_rn(pi, s.inputRatio) : dev::scaleCell(pi, s.inputRatio, s.inputMantissa, s.inputExponent, s.inputUsesFp);
+        o.cellRaw = rounded(__fadd_rn(sf, si), k.cLo, k.cHi);
+        o.cell = st.cell = kTrain ? clampF(o.cellRaw, k.cLo, k.cHi) : o.cellRaw;
+        o.tanhC = activation(u, 4, st.cell, o.index[4]);
+        o.hiddenRaw = rounded(__fmul_rn(__fmul_rn(o.gate[3], o.tanhC), k.productScale), k.oLo, k.oHi);
+        o.hidden = st.hidden = kTrain ? clampF(o.hiddenRaw, k.oLo, k.oHi) : o.hiddenRaw;
+        return __float_as_uint(__fadd_rn(st.hidden, k.codePlus)) & 0xffffu;
+    }
+    __device__ __forceinline__ void store(const Unit &, const Out &v, size_t at, uint32_t row, int unit, bool good) const {
+        const uint32_t H = this->hidden(), mine = row * H + unit, mine4 = row * (4 * H) + unit;
+        const auto &s = this->s;
+        const auto &ck = this->ck;
+        (this->output + at * H)[mine] = __fmul_rn(v.hidden, Base::scaleH(good));
+        if (!kTrain) return;
+        auto put = [&](auto *to, auto value) {
+            if (SAVES == Saves::All || to) (to + at * H)[mine] = value();
+        };
+        auto put4 = [&](auto *to, auto value) {
+            if (SAVES != Saves::All && !to) return;
+            auto *step = to + at * (4 * H);
+#pragma unroll
+            for (int g = 0; g < 4; ++g) (step + g * H)[mine4] = value(g);
+        };
+        auto flag = [](bool set) { return static_cast<uint8_t>(set ? 1 : 0); };
+        auto clamped = [&](int t) { return flag(v.index[t] - k.table[t].flagBelow >= k.table[t].flagCount); };
+        put4(ck.weight_hh_linear, [&](int g) { return clampF(v.hh[g], k.hhLo, k.hhHi) + s.zpF[RXMET_LSTM_WEIGHT_HH_LINEAR]; });
+        put4(ck.weight_hh_linear_clamped, [&](int g) { return flag(v.hh[g] < k.hhLo || v.hh[g] > k.hhHi); });
+        put4(ck.gate_inputs, [&](int g) { return clampF(v.sum[g], k.giLo[g], k.giHi[g]) + k.zpIn[g]; });
+        put4(ck.gate_inputs_clamped, [&](int g) { return flag(v.sum[g] < k.giLo[g] || v.sum[g] > k.giHi[g]); });
+        put4(ck.gate_outputs, [&](int g) { return v.gate[g] + k.zpOut[g]; });
+        put4(ck.gate_outputs_clamped, [&](int g) { return clamped(g); });
+        put(ck.cell_states, [&] { return v.cell + s.zpF[RXMET_LSTM_CELL_STATE]; });
+        put(ck.cell_states_clamped, [&] { return flag(v.cellRaw < k.cLo || v.cellRaw > k.cHi); });
+        put(ck.cell_tanh_outputs, [&] { return v.tanhC + s.zpF[RXMET_LSTM_CELL_TANH_OUTPUT]; });
+        put(ck.cell_tanh_outputs_clamped, [&] { return clamped(4); });
+        put(ck.hidden_outputs, [&] { return v.hidden + s.zpF[RXMET_LSTM_OUTPUT]; });
+        put(ck.hidden_outputs_clamped, [&] { return flag(v.hiddenRaw < k.oLo || v.hiddenRaw > k.oHi); });
+    }
+    __device__ __forceinline__ void finish(const State &st, int row, int unit, bool good) const {
+        const size_t o = static_cast<size_t>(row) * this->hidden() + unit;
+        this->finalHidden[o] = __fmul_rn(st.hidden, Base::scaleH(good));
+        this->finalCell[o] = __fmul_rn(st.cell, good ? this->s.scale[RXMET_LSTM_CELL_STATE] : __int_as_float(0x7fc00000));
+    }
+};
+
+// Up to 128 units: inside one CTA, rows as few as let all CTAs run at the same time, up to four (64 units: eight).
+template <Saves SAVES, int HP, int PLANES>
+void launchLstmUnits(const char *name, const planerec::Problem &p, const LstmPlaneCell<SAVES != Saves::None> &cell, cudaStream_t st) {
+    auto run = [&](auto width) {
+        using Cell = LstmUnitCell<SAVES, decltype(width)::value>;
+        static_assert(sizeof(typename Cell::Base) == sizeof(cell), "the variants differ in the width only");
+        Cell c;
+        std::memcpy(static_cast<typename Cell::Base *>(&c), &cell, sizeof(cell));
+        c.prepareConstants();
+        unitrec::launchRows<Cell, HP, PLANES>(name, p, c, st);
+    };
+    if (p.H == HP) run(std::integral_constant<int, HP>{});
+    else run(std::integral_constant<int, 0>{});
+}
+// Wider layers, over clusters.  Rows: a step of n rows costs about 1 + n / 5 of the chain of a one-row step.
 template <bool TRAIN, int HP>
 void launchLstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &cell, cudaStream_t st) {
-    if constexpr (HP <= 128)
-        if (p.H != HP && lanerec::launch<LstmPlaneCell<TRAIN>, HP / 4, 2>("lstmRecurrentWide", p, cell, st)) return;
     if (p.H == HP) {
         LstmPlaneCell<TRAIN, HP> full;
         static_assert(sizeof(full) == sizeof(cell), "the variants differ in the width only");
         std::memcpy(&full, &cell, sizeof(full));
-        if constexpr (HP <= 128)
-            if (lanerec::launch<LstmPlaneCell<TRAIN, HP>, HP / 4, 2>("lstmRecurrentWide", p, full, st)) return;
         planerec::launchBest<LstmPlaneCell<TRAIN, HP>, HP, 64, 2, 5, 4, 8, 12, 16, 24, 32, 48>("lstmRecurrentWide", p, full, st);
     } else {
         planerec::launchBest<LstmPlaneCell<TRAIN>, HP, 64, 2, 5, 4, 8, 12, 16, 24, 32, 48>("lstmRecurrentWide", p, cell, st);
     }
 }
-// 8-bit inference, at most 128 units, rows that one wave of CTAs holds (lanerec::rowsFor): the same cell on one byte plane.
-template <int HP>
-void launchLstmBytes(const planerec::Problem &p, const LstmPlaneCell<false> &cell, cudaStream_t st) {
-    bool done;
-    if (p.H == HP) {
-        LstmPlaneCell<false, HP> full;
-        std::memcpy(&full, &cell, sizeof(full));
-        done = lanerec::launch<LstmPlaneCell<false, HP>, HP / 4, 1>("lstmRecurrent", p, full, st);
-    } else {
-        done = lanerec::launch<LstmPlaneCell<false>, HP / 4, 1>("lstmRecurrent", p, cell, st);
-    }
-    RXMET_REQUIRE(done, "8-bit LSTM recurrence: %d rows", p.B);
-}
-// One padded width each, built in separate files (lstm_forward_cluster_*.cu).
+// One padded width each, built in separate files (lstm_forward_cluster_*.cu, lstm_forward_units_*.cu).
 template <bool TRAIN, int HP>
 void lstmCluster(const planerec::Problem &p, const LstmPlaneCell<TRAIN> &cell, cudaStream_t st);
-template <int HP>
-void lstmBytes(const planerec::Problem &p, const LstmPlaneCell<false> &cell, cudaStream_t st);
+template <Saves SAVES, int HP, int PLANES>
+void lstmUnits(const planerec::Problem &p, const LstmPlaneCell<SAVES != Saves::None> &cell, cudaStream_t st);
 
 }  // namespace lstm
 }  // namespace rxmet

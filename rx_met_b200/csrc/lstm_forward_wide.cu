@@ -943,12 +943,10 @@ bool clusterTakes(const Exec &e) {
 
 }  // namespace
 
-// Inference on 8-bit grids, T = 150, I = 40, against the byte-code kernels (lstm_forward_quant.cu): B = 1, H = 128 153 -> 119 us;
-// B = 128, H = 128 186 -> 148 us; B = 256, H = 64 160 -> 146 us; four rows of 64 units lose (B = 500: 204 -> 219 us), and so
-// does a forward with checkpoints (T = 100, B = 256, H = 128: 160 -> 229 us).
-bool forwardBytesInLanes(const Exec &e, int B, int I, int H) {
-    const int rows = H <= 64 ? lanerec::rowsFor<16, 1>(B) : H <= 128 ? lanerec::rowsFor<32, 1>(B) : 0;
-    return rows != 0 && e.activationPlanes == 1 && forwardQuantWideTakes(e, I, H, nullptr) && clusterTakes(e);
+// Up to 128 units: the recurrence with a thread per unit, on one byte plane or two.
+bool forwardInUnits(const Exec &e, int B, int I, int H) {
+    return H <= 128 && 4 * static_cast<uint64_t>(H) * B < (uint64_t{1} << 32) && e.activationPlanes != 0 &&   // offsets inside a step have 32 bits
+           forwardQuantWideTakes(e, I, H, nullptr) && clusterTakes(e);
 }
 
 bool forwardQuantWideTakes(const Exec &e, int I, int H, const char **why) {
@@ -1087,12 +1085,14 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
         afterLaunch("lstmInputLinearWide");
     }
     // Recurrence over clusters wherever the activation tables have a compact form and the grids are the usual ones.
-    const bool bytes = !call.checkpoints && forwardBytesInLanes(e, B, I, H);
-    if (bytes || (planes == 2 && clusterTakes(e))) {
+    const bool units = forwardInUnits(e, B, I, H);
+    if (units || (planes == 2 && H > 128 && clusterTakes(e))) {
         const planerec::Problem problem{T, B, H, l.h0};
-        const bool saves = ck.weight_hh_linear || ck.weight_hh_linear_clamped || ck.gate_inputs || ck.gate_inputs_clamped || ck.gate_outputs ||
-                           ck.gate_outputs_clamped || ck.cell_states || ck.cell_states_clamped || ck.cell_tanh_outputs ||
-                           ck.cell_tanh_outputs_clamped || ck.hidden_outputs || ck.hidden_outputs_clamped;
+        const void *const kept[] = {ck.weight_hh_linear, ck.weight_hh_linear_clamped, ck.gate_inputs, ck.gate_inputs_clamped, ck.gate_outputs,
+                                    ck.gate_outputs_clamped, ck.cell_states, ck.cell_states_clamped, ck.cell_tanh_outputs,
+                                    ck.cell_tanh_outputs_clamped, ck.hidden_outputs, ck.hidden_outputs_clamped};
+        const bool saves = std::any_of(std::begin(kept), std::end(kept), [](const void *p) { return p != nullptr; });
+        const bool all = std::all_of(std::begin(kept), std::end(kept), [](const void *p) { return p != nullptr; });
         auto run = [&](auto cell) {
             const CompactTables &t = e.compactTables();
             cell.s = s; cell.width = H; cell.kWords = kHh; cell.B = static_cast<size_t>(B);
@@ -1105,12 +1105,17 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
             cell.c0 = l.c0; cell.output = call.output; cell.finalHidden = call.finalHidden; cell.finalCell = call.finalCell; cell.ck = ck;
             cell.poison = tensorProjection ? l.projStatus : nullptr;
             constexpr bool kTrain = decltype(cell)::kSaves;
-            if constexpr (!kTrain) {
-                if (bytes) return H <= 64 ? lstmBytes<64>(problem, cell, st) : lstmBytes<128>(problem, cell, st);
+            auto narrow = [&](auto saved) {
+                constexpr Saves kSaved = decltype(saved)::value;
+                if (planes == 2) return H <= 64 ? lstmUnits<kSaved, 64, 2>(problem, cell, st) : lstmUnits<kSaved, 128, 2>(problem, cell, st);
+                return H <= 64 ? lstmUnits<kSaved, 64, 1>(problem, cell, st) : lstmUnits<kSaved, 128, 1>(problem, cell, st);
+            };
+            if (units) {
+                if constexpr (!kTrain) return narrow(std::integral_constant<Saves, Saves::None>{});
+                else if (all) return narrow(std::integral_constant<Saves, Saves::All>{});
+                else return narrow(std::integral_constant<Saves, Saves::Some>{});
             }
-            if (H <= 64) lstmCluster<kTrain, 64>(problem, cell, st);
-            else if (H <= 128) lstmCluster<kTrain, 128>(problem, cell, st);
-            else if (H <= 256) lstmCluster<kTrain, 256>(problem, cell, st);
+            if (H <= 256) lstmCluster<kTrain, 256>(problem, cell, st);
             else if (H <= 384) lstmCluster<kTrain, 384>(problem, cell, st);
             else lstmCluster<kTrain, 512>(problem, cell, st);
         };

@@ -43,8 +43,8 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &exec, void *workspac
 
 // Activation grids up to 16 bits, weight grids up to 8 bits, H <= 512, I <= 256 (lstm_forward_wide.cu).
 bool forwardQuantWideTakes(const Exec &exec, int I, int H, const char **why);
-// 8-bit grids whose recurrence runs there too (lane_recurrence.cuh), up to 128 units.
-bool forwardBytesInLanes(const Exec &exec, int B, int I, int H);
+// Up to 128 units: the recurrence with a thread per unit (unit_recurrence_umma.cuh), 8-bit grids included.
+bool forwardInUnits(const Exec &exec, int B, int I, int H);
 size_t forwardQuantWideWorkspaceBytes(int T, int B, int I, int H);
 void forwardQuantWide(const ForwardQuantCall &call, const Exec &exec, void *workspace, size_t workspaceBytes,
                       cudaStream_t stream);

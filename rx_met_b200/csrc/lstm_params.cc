@@ -668,7 +668,7 @@ bool buildCompact(const Exec &e, int segShift, CompactTables &out) {
                 auto clamped = [&](float v) { return std::fmin(std::fmax(v, out.outLo[t]), out.outHi[t]); };
                 if (clamped(base) == want) continue;
                 if (clamped(base + 1.0f) != want) return false;
-                bits[i >> 5] |= 1u << (i & 31);
+                bits[i >> 5] |= 0x80000000u >> (i & 31);
             }
         }
         int below = 0, from = entries;

@@ -90,7 +90,7 @@ struct WideTables {
 // The same tables in the form that fits shared memory: per segment of 2^segShift inputs a line, per input one correction
 // bit.  For the centred input code x (a float): t = fmaf(slope, x, intercept), base = round-half-even(t) and the centred
 // output code is clamp(base + bit, outLo, outHi), where (slope, intercept) sit at segOffset + 8 * (index >> segShift) and
-// the bit at bit (index & 31) of the word at bitOffset + 4 * (index >> 5), index = x - inLo.  The clamp flag of an
+// the bit at bit 31 - (index & 31) of the word at bitOffset + 4 * (index >> 5), index = x - inLo.  The clamp flag of an
 // entry is index < flagBelow || index >= flagFrom.  Built from the full tables and checked entry by entry; `ok` is false
 // when some segment has no such line, an output grid is wider than 16 bits or the flags have another shape.
 struct CompactTables {
