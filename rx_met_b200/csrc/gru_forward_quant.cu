@@ -390,8 +390,7 @@ __global__ void __launch_bounds__(32 * kPrepLayers) prepareWide(const __grid_con
                 word |= static_cast<uint32_t>(q & 0xff) << (8 * b);
             }
             if (live && kk < words) packed[static_cast<size_t>(kk) * a.C + c] = word;
-            // canonical tile (packTiles in plane_proj_umma.cuh): 128 channels x tileWords, 16-byte rows of core matrices
-            if (tiles) tiles[static_cast<size_t>(c / 128) * (128 * a.tileWords) + (c % 128 / 8) * (8 * a.tileWords) + (kk / 4) * 32 + (c % 8) * 4 + kk % 4] = word;
+            if (tiles) tiles[4 * planeproj::tilePlace(c, kk / 4, 4 * a.tileWords) + kk % 4] = word;
         }
         return sum;
     };

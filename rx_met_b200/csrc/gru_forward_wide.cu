@@ -297,9 +297,10 @@ recurrentPlanes(const __grid_constant__ RecurrentArgs a, const __grid_constant__
 }
 
 // Epilogue of the tensor-core input projection: exact 64-bit sum of the two planes and the addend, the
-// rounding rescale onto the linear-output grid, clamp, code and keep flag.
+// rounding rescale onto the linear-output grid, clamp, code and keep flag.  Shifts in [1, 31] and multipliers that leave room for a byte
+// (all usual ones) take two widening multiply-adds - one per plane, the addend and half a unit in them -, a funnel shift and, for
+// the exact ties, a cleared lowest bit.
 struct PlaneEpilogue {
-    static constexpr bool kTakesRows = false;
     const int64_t *addend;
     const Rescale *rescale;
     int32_t zpOut, lo, hi;
@@ -309,8 +310,18 @@ struct PlaneEpilogue {
     struct Channel {
         int64_t addend;
         Rescale rs;
+        bool small;
     };
-    __device__ Channel channel(int c) const { return Channel{addend[c], rescale[c]}; }
+    struct Loaded {
+        int64_t addend;
+        Rescale rs;
+    };
+    __device__ Loaded load(int c) const { return Loaded{__ldg(addend + c), rescale[c]}; }
+    __device__ Channel channel(const Loaded &l, int) const {
+        Channel ch{l.addend, l.rs, false};
+        ch.small = __all_sync(0xffffffffu, ch.rs.shift >= 1 && ch.rs.shift <= 31 && ch.rs.mult >= 0 && ch.rs.mult < (1 << 23));
+        return ch;
+    }
     __device__ void store(const Channel &ch, size_t row, int c, const int32_t (&acc)[2]) const {
         uint8_t keep;
         const int32_t q = clampCode(static_cast<int32_t>(applyRescale(combine(acc[0], acc[1], ch.addend), ch.rs)) + zpOut, lo, hi, keep);
@@ -318,16 +329,36 @@ struct PlaneEpilogue {
         out[o] = static_cast<int16_t>(q);
         if (mask) mask[o] = keep;
     }
+    template <int N>
+    __device__ void storeRows(const Channel &ch, size_t row, uint32_t c, const uint32_t (&acc)[2][N], int count) const {
+        const int64_t plus = ch.addend * ch.rs.mult + (int64_t{1} << (ch.rs.shift - 1));
+        const int32_t multHigh = ch.rs.mult << 8;
+        const uint32_t tie = (1u << ch.rs.shift) - 1u;
+        int32_t code[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const int64_t sum = static_cast<int64_t>(static_cast<int32_t>(acc[0][j])) * multHigh +
+                                (static_cast<int64_t>(static_cast<int32_t>(acc[1][j])) * ch.rs.mult + plus);
+            const uint32_t low = static_cast<uint32_t>(sum);
+            const int32_t q = static_cast<int32_t>(__funnelshift_r(low, static_cast<uint32_t>(static_cast<uint64_t>(sum) >> 32), ch.rs.shift));
+            code[j] = ((low & tie) == 0 ? q & ~1 : q) + zpOut;
+        }
+        planeproj::Column<int16_t> to(out, row, c, C);
+        if (mask == nullptr) {
+            planeproj::eachRow<N>(count, [&](int j) { to.put(static_cast<int16_t>(max(lo, min(code[j], hi)))); });
+            return;
+        }
+        planeproj::Column<uint8_t> toMask(mask, row, c, C);
+        planeproj::eachRow<N>(count, [&](int j) {
+            const int32_t q = max(lo, min(code[j], hi));
+            to.put(static_cast<int16_t>(q));
+            toMask.put(static_cast<uint8_t>(q == code[j] ? 1 : 0));
+        });
+    }
 };
 
-// Rows of a tile of the tensor-core projection, 0 where it does not run: operands beyond shared memory, or RXMET_IPROJ_SIMT.
-int projectionRows(int kI) {
-    const int kPad = planeproj::paddedK(kI);
-    if (std::getenv("RXMET_IPROJ_SIMT") != nullptr) return 0;
-    for (int rows : {128, 64})
-        if (planeproj::sharedBytes(kPad, 2, rows) <= 200 * 1024) return rows;
-    return 0;
-}
+// Whether the tensor-core projection runs: not where the operands exceed shared memory, or under RXMET_IPROJ_SIMT.
+bool projects(int kI) { return std::getenv("RXMET_IPROJ_SIMT") == nullptr && planeproj::fits(planeproj::paddedK(kI), 2); }
 
 template <class W>
 WideOperands layoutWide(W &ws, int T, int B, int I, int H) {
@@ -347,7 +378,7 @@ WideOperands layoutWide(W &ws, int T, int B, int I, int H) {
     o.wTiles = ws.template take<uint4>(static_cast<size_t>(planeproj::paddedC(static_cast<int>(C))) * o.tileWords / 4);
     o.projStatus = ws.template take<int>(1);
     o.ihCodes = ws.template take<int16_t>(rows * C);
-    if (projectionRows(o.kI) == 0) o.wTiles = nullptr;
+    if (!projects(o.kI)) o.wTiles = nullptr;
     return o;
 }
 
@@ -388,8 +419,6 @@ void forwardWide(const WideCall &call, const Exec &e, cudaStream_t st) {
     const int sms = currentDevice().sms;
 
     // Input projection: the tcgen05 kind::i8 kernel when the operands fit shared memory, else the dp4a kernel.
-    const int kPadI = planeproj::paddedK(kI);
-    const int rowsPerTile = projectionRows(kI);
     const bool tensorProjection = l.wTiles != nullptr;
     if (forwardPhase() == ForwardPhase::Recurrence) {
         // the call before has projected
@@ -400,17 +429,7 @@ void forwardWide(const WideCall &call, const Exec &e, cudaStream_t st) {
         epi.addend = l.addX; epi.rescale = call.gemmX;
         epi.zpOut = g.zp[RXMET_GRU_WEIGHT_IH_LINEAR]; epi.lo = g.qlo[RXMET_GRU_WEIGHT_IH_LINEAR]; epi.hi = g.qhi[RXMET_GRU_WEIGHT_IH_LINEAR];
         epi.out = l.ihCodes; epi.mask = call.maskIh; epi.C = C;
-        const size_t smem = planeproj::sharedBytes(kPadI, 2, rowsPerTile);
-        const int rowTiles = static_cast<int>((rows + rowsPerTile - 1) / rowsPerTile);
-        const int grid = std::max(1, std::min(rowTiles, smsPerPass()));
-        auto launchTensor = [&](auto kernel) {
-            ensureDynamicSmem(reinterpret_cast<const void *>(kernel), smem);
-            KernelTimer timer__("inputLinear", st);
-            kernel<<<grid, planeproj::kThreads, smem, st>>>(pp, epi);
-        };
-        if (rowsPerTile == 128) launchTensor(planeproj::planeProjUmma<PlaneEpilogue, 2, 128>);
-        else launchTensor(planeproj::planeProjUmma<PlaneEpilogue, 2, 64>);
-        afterLaunch("inputLinear");
+        planeproj::launch<2>("inputLinear", pp, epi, smsPerPass(), st);
     } else {
         InputArgs a{};
         a.rows = static_cast<int>(rows); a.C = C; a.kWords = kI;

@@ -830,7 +830,6 @@ struct WideLayout {
 // and sixteen rows share their addresses and tests.  T = 1000, B = 4096, H = 512: the pass 59.4 -> 57.0 ms.
 template <int PLANES>
 struct WidePlaneEpilogue {
-    static constexpr bool kTakesRows = true;
     const int64_t *addend;
     const float *fields;     // the per-channel float block (kChannelFields x 4H)
     ScalarExec s;
@@ -844,10 +843,16 @@ struct WidePlaneEpilogue {
     };
     __device__ float lowest() const { return static_cast<float>(s.lo[RXMET_LSTM_WEIGHT_IH_LINEAR] - s.zp[RXMET_LSTM_WEIGHT_IH_LINEAR]); }
     __device__ float highest() const { return static_cast<float>(s.hi[RXMET_LSTM_WEIGHT_IH_LINEAR] - s.zp[RXMET_LSTM_WEIGHT_IH_LINEAR]); }
-    __device__ Channel channel(int c) const {
+    struct Loaded {
+        int64_t addend;
+        DevRescale out;
+    };
+    __device__ Loaded load(int c) const {
         const size_t C = 4 * static_cast<size_t>(H);
-        Channel ch{addend[c], DevRescale{fields[static_cast<size_t>(kIhOutMult) * C + c], fields[static_cast<size_t>(kIhOutPow2) * C + c]},
-                   s.ihToGate[c / H], false};
+        return Loaded{__ldg(addend + c), DevRescale{__ldg(fields + kIhOutMult * C + c), __ldg(fields + kIhOutPow2 * C + c)}};
+    }
+    __device__ Channel channel(const Loaded &loaded, int c) const {
+        Channel ch{loaded.addend, loaded.out, s.ihToGate[c / H], false};
         const int64_t wMax = max(-static_cast<int64_t>(s.lo[RXMET_LSTM_WEIGHT_IH]), static_cast<int64_t>(s.hi[RXMET_LSTM_WEIGHT_IH]));
         const float most = fmaxf(fabsf(lowest()), fabsf(highest())) + 1.0f;
         ch.small = __all_sync(0xffffffffu, wMax * (PLANES == 2 ? 65535 : 255) * I + llabs(ch.addend) < (int64_t{1} << 31) && most < 4194304.0f &&
@@ -865,32 +870,33 @@ struct WidePlaneEpilogue {
     }
     // `count` rows of N; small channels only
     template <int N>
-    __device__ void storeRows(const Channel &ch, size_t row, int c, const uint32_t (&acc)[PLANES][N], int count) const {
+    __device__ void storeRows(const Channel &ch, size_t row, uint32_t c, const uint32_t (&acc)[PLANES][N], int count) const {
         const float lo = lowest(), hi = highest(), scale = __fmul_rn(ch.out.mult, ch.out.pow2), gate = __fmul_rn(ch.toGate.mult, ch.toGate.pow2);
         const uint32_t plus = static_cast<uint32_t>(ch.addend);
         auto rounded = [](float v) { return __fadd_rn(__fadd_rn(v, 12582912.0f), -12582912.0f); };
-        float r[N];   // one step beyond the grid where it clamps
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
+        const uint32_t C = 4 * static_cast<uint32_t>(H);
+        planeproj::Column<float> to(lhs, row, c, C);
+        auto value = [&](int j) {
             const uint32_t sum = (PLANES == 2 ? acc[0][j] * 256u + acc[PLANES - 1][j] : acc[0][j]) + plus;
-            r[j] = rounded(fminf(fmaxf(__fmul_rn(__int2float_rn(static_cast<int32_t>(sum)), scale), lo - 1.0f), hi + 1.0f));
+            return __fmul_rn(__int2float_rn(static_cast<int32_t>(sum)), scale);
+        };
+        if (!linear && !linearClamped) {
+            planeproj::eachRow<N>(count, [&](int j) { to.put(rounded(__fmul_rn(rounded(fminf(fmaxf(value(j), lo), hi)), gate))); });
+            return;
         }
-        const size_t C = 4 * static_cast<size_t>(H), o = row * C + c;
-        auto centred = [&](int j) { return fminf(fmaxf(r[j], lo), hi); };
-#pragma unroll
-        for (int j = 0; j < N; ++j)
-            if (j < count) lhs[o + j * C] = rounded(__fmul_rn(centred(j), gate));
-        if (linear) {
-            const float zp = s.zpF[RXMET_LSTM_WEIGHT_IH_LINEAR];
-#pragma unroll
-            for (int j = 0; j < N; ++j)
-                if (j < count) linear[o + j * C] = centred(j) + zp;
-        }
-        if (linearClamped) {
-#pragma unroll
-            for (int j = 0; j < N; ++j)
-                if (j < count) linearClamped[o + j * C] = (r[j] < lo || r[j] > hi) ? 1 : 0;
-        }
+        const float zp = s.zpF[RXMET_LSTM_WEIGHT_IH_LINEAR];
+        auto save = [&](auto both) {
+            planeproj::Column<float> toLinear(linear, row, c, C);
+            planeproj::Column<uint8_t> toFlags(linearClamped, row, c, C);
+            planeproj::eachRow<N>(count, [&](int j) {
+                const float r = rounded(fminf(fmaxf(value(j), lo - 1.0f), hi + 1.0f)), centred = fminf(fmaxf(r, lo), hi);   // r: one step beyond the grid where it clamps
+                to.put(rounded(__fmul_rn(centred, gate)));
+                if (decltype(both)::value || linear) toLinear.put(centred + zp);
+                if (decltype(both)::value || linearClamped) toFlags.put(static_cast<uint8_t>(r != centred ? 1 : 0));
+            });
+        };
+        if (linear && linearClamped) save(std::true_type{});
+        else save(std::false_type{});
     }
 };
 
@@ -1031,8 +1037,7 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
     // Input projection: the tcgen05 kind::i8 kernel when the operands fit shared memory
     // (RXMET_IPROJ_SIMT turns it off), else the dp4a kernel.
     const int kPadIh = planeproj::paddedK(kIh);
-    const int rowsPerTile = planeproj::sharedBytes(kPadIh, planes, 128) <= 200 * 1024 ? 128 : 64;
-    const bool tensorProjection = planeproj::sharedBytes(kPadIh, planes, rowsPerTile) <= 200 * 1024 && std::getenv("RXMET_IPROJ_SIMT") == nullptr;
+    const bool tensorProjection = planeproj::fits(kPadIh, planes) && std::getenv("RXMET_IPROJ_SIMT") == nullptr;
     if (tensorProjection) {
         RXMET_CUDA(cudaMemsetAsync(l.projStatus, 0, sizeof(int), st));
         {
@@ -1042,21 +1047,13 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
         afterLaunch("packTiles");
         planeproj::Problem pp{};
         pp.planes = l.x; pp.rows = static_cast<int>(rows); pp.kWords = kIh; pp.tiles = l.ihTiles; pp.C = C; pp.status = l.projStatus;
-        const size_t smem = planeproj::sharedBytes(kPadIh, planes, rowsPerTile);
-        const int rowTiles = static_cast<int>((rows + rowsPerTile - 1) / rowsPerTile);
-        const int grid = std::max(1, std::min(rowTiles, smsPerPass()));
-        auto launchTensor = [&](auto kernel, auto epi) {
+        auto launchTensor = [&](auto epi, auto planeCount) {
             epi.addend = l.addIh; epi.fields = l.channel; epi.s = s; epi.H = H; epi.I = I; epi.lhs = l.lhs;
             epi.linear = ck.weight_ih_linear; epi.linearClamped = ck.weight_ih_linear_clamped;
-            ensureDynamicSmem(reinterpret_cast<const void *>(kernel), smem);
-            KernelTimer timer__("lstmInputLinearWide", st);
-            kernel<<<grid, planeproj::kThreads, smem, st>>>(pp, epi);
+            planeproj::launch<decltype(planeCount)::value>("lstmInputLinearWide", pp, epi, smsPerPass(), st);
         };
-        if (planes == 2 && rowsPerTile == 128) launchTensor(planeproj::planeProjUmma<WidePlaneEpilogue<2>, 2, 128>, WidePlaneEpilogue<2>{});
-        else if (planes == 2) launchTensor(planeproj::planeProjUmma<WidePlaneEpilogue<2>, 2, 64>, WidePlaneEpilogue<2>{});
-        else if (rowsPerTile == 128) launchTensor(planeproj::planeProjUmma<WidePlaneEpilogue<1>, 1, 128>, WidePlaneEpilogue<1>{});
-        else launchTensor(planeproj::planeProjUmma<WidePlaneEpilogue<1>, 1, 64>, WidePlaneEpilogue<1>{});
-        afterLaunch("lstmInputLinearWide");
+        if (planes == 2) launchTensor(WidePlaneEpilogue<2>{}, std::integral_constant<int, 2>{});
+        else launchTensor(WidePlaneEpilogue<1>{}, std::integral_constant<int, 1>{});
     } else {
         WideInputArgs a{};
         a.rows = static_cast<int>(rows); a.H = H; a.kWords = kIh;

@@ -3,24 +3,34 @@
 // tensor memory, shared by the QuantGRU W8 / A16 forward and the wide QuantLSTM forward:
 //
 //   acc_p[row][c] = sum_k plane_p[row][k] * w[k][c]        (p = high, low byte plane)
-//   out[row][c]   = epilogue(c, acc_high, acc_low)         (the caller's functor: exact 64-bit combine, rescale,
+//   out[row][c]   = epilogue(c, acc_high, acc_low)         (the caller's functor: exact combine, rescale,
 //                                                           clamp, masks - whatever its operator defines)
 //
 // The product is computed transposed, D[channel][row], so that a lane of tensor memory is a channel: the
 // per-channel constants of the epilogue live in registers and, for one row, the lanes of a warp store
-// neighbouring channels.  A CTA walks row tiles of NR rows with a grid stride.  Per row tile the planes are
-// placed once into the canonical un-swizzled K-major B layout (core matrix = 8 rows x 16 k-bytes); per channel
-// tile of 128 the weight tile - packed beforehand into the same canonical layout, contiguous per tile - is
-// copied into one of two A buffers with 16-byte loads, one thread issues PLANES x K/32 MMAs into one of two
-// accumulator buffers (PLANES x NR columns each) and commits them to that buffer's mbarrier, and the epilogue
-// of the previous item runs meanwhile.  Every mbarrier wait is bounded; a wait that gives up sets the status
-// word and the CTA still frees its tensor memory.
+// neighbouring channels.
+//
+// A work item is a tile of NR rows and a tile of 128 channels; a CTA takes the channel tiles of one share of a row tile one after
+// another.  Few row tiles are cut into shares of fewer channel tiles, so that a short call fills the GPU as well.  Warps by role:
+//   weights   one lane copies weight tiles, packed beforehand in the canonical K-major A layout, in slices of at most 256 k-bytes
+//             into a ring (bulk copies)
+//   rows      places the planes of a row tile into one of two B buffers, 16 bytes at a time
+//   products  one thread issues PLANES x K/32 MMAs per item into one of two accumulator buffers
+//   epilogue  sixteen warps: tensor-memory quarter x four groups of rows
+// so that copies, products and the epilogue of different items run at the same time.  Every mbarrier wait is bounded; one
+// that gives up ends all further waiting of its warp, sets the status word, and the CTA still frees its tensor memory.
+//
+// Bound: the stores of the results and the issue of the epilogue.  I = 256, C = 2048, 4.1 M rows (33.5 GB of 32-bit results) 15.0 -> 7.3 ms;
+// I = 512, C = 768, 12,800 rows on half of the SMs 81 -> 54 us; 1000 rows, C = 2048 79 -> 16 us, where eight CTAs had been at work.
+// The form before it fetched every weight tile through registers between two barriers of all warps.
 #pragma once
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
+#include "common.h"
 #include "umma_device.cuh"
 
 namespace rxmet {
@@ -28,8 +38,10 @@ namespace planeproj {
 
 using namespace umma;
 
-constexpr int kThreads = 512;
 constexpr int kChannelTile = 128;
+constexpr int kEpilogueWarps = 16, kProductWarp = 16, kRowWarps = 2, kRowWarp = 17, kWeightWarp = kRowWarp + kRowWarps;
+constexpr int kThreads = 32 * (kWeightWarp + 1);
+constexpr int kSlice = 256;   // k-bytes of a slice of a weight tile
 
 // kind::i8 with a signed A (weights) and an unsigned B (byte planes): 32-bit integer accumulator (bits [4,6)
 // = 2), A format signed 8-bit (bits [7,10) = 1), B format unsigned 8-bit (bits [10,13) = 0), both K-major,
@@ -53,20 +65,35 @@ __device__ __forceinline__ void mmaI8(uint32_t tmemD, uint64_t descA, uint64_t d
 struct Problem {
     const uint32_t *planes = nullptr;   // [rows][PLANES][kWords] words of four unsigned bytes, kWords a multiple of 4
     int rows = 0, kWords = 0;
-    const uint4 *tiles = nullptr;       // [C / 128][kPad / 16][16 channel groups]... = packTiles' output, 128 * kPad bytes per tile
+    const uint4 *tiles = nullptr;       // packed weight tiles (tilePlace), 128 * kPad bytes each
     int C = 0;                          // channels beyond C in the last tile are computed and dropped
+    int ring = 0, shares = 0;           // slices of weight tiles in shared memory, shares of a row tile's channel tiles (launch())
     int *status = nullptr;              // device word, set to 1 when a bounded wait of the kernel gave up
 };
 
 __host__ __device__ inline int paddedK(int kWords) { return (kWords * 4 + 31) / 32 * 32; }
 __host__ __device__ inline int paddedC(int C) { return (C + kChannelTile - 1) / kChannelTile * kChannelTile; }
-inline size_t sharedBytes(int kPad, int planes, int rowsPerTile) {
-    return 2 * static_cast<size_t>(kChannelTile) * kPad + static_cast<size_t>(planes) * rowsPerTile * kPad;
+// Where the 16 bytes from k-group kg of channel c lie among the packed tiles, in units of 16 bytes: tiles of 128 channels, slices of kSlice
+// k-bytes, eight channels, k-groups, channels.
+__host__ __device__ inline size_t tilePlace(int c, int kg, int kPad) {
+    const int slice = kg / (kSlice / 16), groups = min(kPad / 16 - slice * (kSlice / 16), kSlice / 16);
+    return static_cast<size_t>(c / kChannelTile) * (kChannelTile * (kPad / 16)) + slice * (kChannelTile * (kSlice / 16)) +
+           (c % kChannelTile / 8) * (groups * 8) + kg % (kSlice / 16) * 8 + c % 8;
+}
+// Rows of a tile, and slices of weight tiles that fit beside the planes of two row tiles.
+__host__ __device__ constexpr int rowsPerTile(int kPad) { return kPad <= 256 ? 128 : 64; }
+inline int ringSlices(int kPad, int planes) {
+    const int sliceBytes = kChannelTile * (kPad < kSlice ? kPad : kSlice), rows = 2 * planes * rowsPerTile(kPad) * kPad;
+    return std::min(4, (225 * 1024 - rows) / sliceBytes);
+}
+// Whether the operands fit one SM.
+inline bool fits(int kPad, int planes) { return kPad <= 512 && ringSlices(kPad, planes) >= 2; }
+inline size_t sharedBytes(int kPad, int planes) {
+    return static_cast<size_t>(ringSlices(kPad, planes)) * kChannelTile * std::min(kPad, kSlice) + 2 * static_cast<size_t>(planes) * rowsPerTile(kPad) * kPad;
 }
 
-// words [kWords][C] (four signed codes along k per word) -> per channel tile of 128 the canonical K-major A
-// operand: byte (c, k) of tile c / 128 at ((c % 128) / 8) * (kPad / 16) * 128 + (k / 16) * 128 + (c % 8) * 16 + k % 16;
-// k beyond 4 kWords and channels beyond C are zero.  One thread per 16-byte row of a core matrix.
+// words [kWords][C] (four signed codes along k per word) -> packed tiles (tilePlace); k beyond 4 kWords and channels beyond C are zero.
+// One thread per 16-byte row of a core matrix.
 static __global__ void packTiles(const uint32_t *__restrict__ words, int kWords, int C, int kPad, uint4 *__restrict__ tiles) {
     const int groups = kPad / 16, padded = paddedC(C);
     const size_t total = static_cast<size_t>(padded) * groups;
@@ -79,39 +106,68 @@ static __global__ void packTiles(const uint32_t *__restrict__ words, int kWords,
             const int kw = 4 * kg + e;
             v[e] = kw < kWords && c < C ? words[static_cast<size_t>(kw) * C + c] : 0u;
         }
-        const size_t tile = c / kChannelTile, within = c % kChannelTile;
-        const size_t at = tile * (static_cast<size_t>(kChannelTile) * kPad / 16) + (within / 8) * (static_cast<size_t>(groups) * 8) +
-                          static_cast<size_t>(kg) * 8 + within % 8;
-        tiles[at] = make_uint4(v[0], v[1], v[2], v[3]);
+        tiles[tilePlace(c, kg, kPad)] = make_uint4(v[0], v[1], v[2], v[3]);
     }
 }
 
 // Epilogue functor contract:
-//   struct Channel;                                        per-channel constants
-//   __device__ Channel channel(int c) const;
+//   struct Loaded; __device__ Loaded load(int c) const;    what a channel reads from memory, asked for one item ahead
+//   struct Channel;                                        per-channel constants; Channel::small, uniform in the warp: storeRows takes it
+//   __device__ Channel channel(const Loaded &, int c) const;
 //   __device__ void store(const Channel &, size_t row, int c, const int32_t (&acc)[PLANES]) const;
-//   kTakesRows: also storeRows<N>(Channel, row, c, acc[PLANES][N], count), for channels with Channel::small (warp-uniform)
+//   __device__ void storeRows<N>(const Channel &, size_t row, int c, const uint32_t (&acc)[PLANES][N], int count) const;
+//                                                          the first `count` of N rows from `row` on
+// f(j) for the first `count` of N rows; whole groups without a test per row.
+template <int N, class F>
+__device__ __forceinline__ void eachRow(int count, F f) {
+    if (count >= N) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) f(j);
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (j < count) f(j);
+    }
+}
+// One column of an array, walked row by row.  The pointer is hidden from the compiler after every step: unrolled, it computes a 64-bit
+// product per row instead of an addition, and keeps sixteen of them.
+template <class T>
+struct Column {
+    T *at;
+    uint32_t rowBytes;
+    __device__ __forceinline__ Column(T *array, size_t row, uint32_t c, uint32_t C) : at(array + row * C + c), rowBytes(C * sizeof(T)) {}
+    __device__ __forceinline__ void put(T value) {
+        *at = value;
+        at = reinterpret_cast<T *>(reinterpret_cast<char *>(at) + rowBytes);
+        asm volatile("" : "+l"(at));
+    }
+};
+
 template <class Epilogue, int PLANES, int NR>
-__global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const Problem p, const Epilogue epi) {
+__global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const __grid_constant__ Problem p, const __grid_constant__ Epilogue epi) {
     constexpr uint32_t kBufCols = PLANES * NR;
     constexpr uint32_t kTmemCols = 2 * kBufCols;   // a power of two for the sizes instantiated (128 .. 512)
     constexpr uint32_t kIdesc = instructionDescriptor(NR);
+    constexpr int kMaxSlices = 4;
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ __align__(8) uint64_t bars[2];  // one per accumulator buffer
+    __shared__ __align__(8) uint64_t weightFull[kMaxSlices], weightFree[kMaxSlices], rowsFull[2], rowsFree[2], accFull[2], accFree[2];
     __shared__ uint32_t tmemSlot;
     __shared__ int failed;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
-    const int C = p.C, kWords = p.kWords, kPad = paddedK(kWords);
-    const uint32_t groupStride = static_cast<uint32_t>(kPad / 16) * kCore;   // next 8 channels / 8 rows
-    const uint32_t tileBytes = static_cast<uint32_t>(kChannelTile) * kPad;
-    const uint32_t planeBytes = static_cast<uint32_t>(NR) * kPad;
-    uint8_t *aTiles = smem;                       // 2 x [16 channel groups][kPad / 16][8][16]
-    uint8_t *rowPlanes = smem + 2 * tileBytes;    // PLANES x [NR / 8][kPad / 16][8][16]
+    const int C = p.C, kWords = p.kWords, kPad = paddedK(kWords), ring = p.ring;
+    const uint32_t sliceBytes = static_cast<uint32_t>(kChannelTile) * min(kPad, kSlice);
+    const uint32_t planeBytes = static_cast<uint32_t>(NR) * kPad, rowStride = static_cast<uint32_t>(kPad / 16) * kCore;   // next 8 rows
+    uint8_t *weights = smem;                      // [ring][16 channel groups][slice / 16][8][16]
+    uint8_t *rowPlanes = smem + ring * sliceBytes;   // [2][PLANES][NR / 8][kPad / 16][8][16]
 
     if (tid == 0) {
         failed = 0;
-        for (int i = 0; i < 2; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smemAddr(&bars[i])) : "memory");
+        auto init = [](uint64_t *bar, uint32_t count) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smemAddr(bar)), "r"(count) : "memory");
+        };
+        for (int i = 0; i < kMaxSlices; ++i) { init(&weightFull[i], 1); init(&weightFree[i], 1); }
+        for (int i = 0; i < 2; ++i) { init(&rowsFull[i], kRowWarps); init(&rowsFree[i], 1); init(&accFull[i], 1); init(&accFree[i], kEpilogueWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -120,109 +176,171 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const Problem p, co
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     // the k padding of the planes is never written again
-    for (uint32_t i = tid; i < PLANES * planeBytes / 16; i += kThreads) reinterpret_cast<uint4 *>(rowPlanes)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (uint32_t i = tid; i < 2 * PLANES * planeBytes / 16; i += kThreads) reinterpret_cast<uint4 *>(rowPlanes)[i] = make_uint4(0u, 0u, 0u, 0u);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmemSlot;
-    volatile int *failFlag = &failed;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmemSlot, 0);
 
-    const int channelTiles = paddedC(C) / kChannelTile;
-    const int rowTiles = (p.rows + NR - 1) / NR;
-    const int q = warp & 3, group = warp >> 2;   // tensor-memory lane quarter (32 channels) of this warp, row-chunk group
+    const int channelTiles = paddedC(C) / kChannelTile, slices = (kPad + kSlice - 1) / kSlice;
+    const int shares = p.shares, units = (p.rows + NR - 1) / NR * shares;   // a unit: one share of the channel tiles of a row tile
+    auto tilesFrom = [&](int share) { return share * channelTiles / shares; };
 
-    auto epilogue = [&](int rowTile, int ct, int local) {
-        const int buf = local & 1;
-        if (!*failFlag && !waitPhase(smemAddr(&bars[buf]), (local >> 1) & 1)) *failFlag = 1;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int c = ct * kChannelTile + 32 * q + lane;
-        const bool real = c < C;
-        const typename Epilogue::Channel ch = epi.channel(min(c, C - 1));
-        for (int chunk = group; chunk < NR / 16; chunk += kThreads / 128) {
-            uint32_t acc[PLANES][16];
-#pragma unroll
-            for (int pl = 0; pl < PLANES; ++pl) {
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-                    : "=r"(acc[pl][0]), "=r"(acc[pl][1]), "=r"(acc[pl][2]), "=r"(acc[pl][3]), "=r"(acc[pl][4]), "=r"(acc[pl][5]),
-                      "=r"(acc[pl][6]), "=r"(acc[pl][7]), "=r"(acc[pl][8]), "=r"(acc[pl][9]), "=r"(acc[pl][10]), "=r"(acc[pl][11]),
-                      "=r"(acc[pl][12]), "=r"(acc[pl][13]), "=r"(acc[pl][14]), "=r"(acc[pl][15])
-                    : "r"(tmem + (static_cast<uint32_t>(32 * q) << 16) + static_cast<uint32_t>(buf * kBufCols + pl * NR + 16 * chunk)));
-            }
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            const int row0 = rowTile * NR + 16 * chunk;
-            if constexpr (Epilogue::kTakesRows) {
-                if (ch.small) {
-                    epi.template storeRows<16>(ch, static_cast<size_t>(row0), c, acc, real ? p.rows - row0 : 0);
-                    continue;
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                if (row0 + j >= p.rows) break;
-                int32_t a[PLANES];
-#pragma unroll
-                for (int pl = 0; pl < PLANES; ++pl) a[pl] = static_cast<int32_t>(acc[pl][j]);
-                if (real) epi.store(ch, static_cast<size_t>(row0 + j), c, a);
-            }
-        }
-        // the MMAs of the item after next overwrite this buffer: order them behind these loads
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    bool alive = true;   // false once a wait of this warp gave up
+    auto wait = [&](uint64_t *bar, uint32_t parity) {
+        if (alive) alive = __all_sync(0xffffffffu, waitPhase(smemAddr(bar), parity));
     };
+    auto arrive = [&](uint64_t *bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smemAddr(bar)) : "memory"); };
 
-    int local = 0, prevTile = -1, prevCt = -1;
-    for (int rowTile = blockIdx.x; rowTile < rowTiles; rowTile += gridDim.x) {
-        // The planes of the previous row tile may still be read by the MMAs of its last item: finish that item
-        // (its epilogue waits for the commit) before the planes are overwritten.
-        if (prevTile >= 0) {
-            epilogue(prevTile, prevCt, local - 1);
-            prevTile = -1;
-        }
-        {
-            const size_t first = static_cast<size_t>(rowTile) * NR * PLANES * kWords;
-            const size_t limit = static_cast<size_t>(p.rows) * PLANES * kWords;
-            for (int i = tid; i < NR * PLANES * kWords; i += kThreads) {
-                const int r = i / (PLANES * kWords), rest = i - r * (PLANES * kWords);
-                const int pl = rest / kWords, kw = rest - pl * kWords;
-                const uint32_t v = first + i < limit ? p.planes[first + i] : 0u;
-                *reinterpret_cast<uint32_t *>(rowPlanes + pl * planeBytes + (r >> 3) * groupStride + (kw >> 2) * kCore + (r & 7) * 16 +
-                                              (kw & 3) * 4) = v;
-            }
-        }
-        for (int ct = 0; ct < channelTiles; ++ct, ++local) {
-            const int buf = local & 1;
-            // A buffer `buf` was read by the MMAs of item local - 2, whose epilogue has run: free.
-            {
-                const uint4 *src = p.tiles + static_cast<size_t>(ct) * (tileBytes / 16);
-                uint4 *dst = reinterpret_cast<uint4 *>(aTiles + buf * tileBytes);
-                for (uint32_t i = tid; i < tileBytes / 16; i += kThreads) dst[i] = __ldg(src + i);
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncthreads();
-            if (warp == 0 && electOne()) {
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t descA = operandDescriptor(smemAddr(aTiles + buf * tileBytes), kCore, groupStride);
-                constexpr uint64_t kStep = (2 * kCore) >> 4;   // the start-address field counts 16-byte units
-#pragma unroll
-                for (int pl = 0; pl < PLANES; ++pl) {
-                    const uint64_t descB = operandDescriptor(smemAddr(rowPlanes + pl * planeBytes), kCore, groupStride);
-                    for (int ks = 0; ks < kPad / 32; ++ks)
-                        mmaI8(tmem + buf * kBufCols + pl * NR, descA + ks * kStep, descB + ks * kStep, kIdesc, ks > 0 ? 1u : 0u);
+    if (warp == kWeightWarp) {
+        uint32_t n = 0;   // slices so far
+        for (int unit = blockIdx.x; unit < units; unit += gridDim.x)
+            for (int ct = tilesFrom(unit % shares); ct < tilesFrom(unit % shares + 1); ++ct)
+                for (int s = 0; s < slices; ++s, ++n) {
+                    const uint32_t at = n % ring, round = n / ring;
+                    if (round > 0) wait(&weightFree[at], (round - 1) & 1);
+                    const uint32_t bytes = static_cast<uint32_t>(kChannelTile) * min(kPad - s * kSlice, kSlice);
+                    if (electOne()) {
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smemAddr(&weightFull[at])), "r"(bytes) : "memory");
+                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                         smemAddr(weights + at * sliceBytes)),
+                                     "l"(p.tiles + (static_cast<size_t>(ct) * kChannelTile * kPad + static_cast<size_t>(s) * kChannelTile * kSlice) / 16),
+                                     "r"(bytes), "r"(smemAddr(&weightFull[at]))
+                                     : "memory");
+                    }
+                    __syncwarp();
                 }
-                commitTo(smemAddr(&bars[buf]));
+        // nothing is left in flight, whatever the other warps gave up on
+        for (uint32_t i = n > static_cast<uint32_t>(ring) ? n - ring : 0; i < n; ++i)
+            if (!waitPhase(smemAddr(&weightFull[i % ring]), (i / ring) & 1)) alive = false;
+    } else if (warp >= kRowWarp && warp < kRowWarp + kRowWarps) {
+        // eight rows x four k-groups a pass: whole core matrices in shared memory, 64-byte pieces of rows in global memory
+        const int kGroups = kWords / 4, r8 = lane & 7, quad = lane >> 3, passes = (kGroups + 3) / 4;
+        uint32_t n = 0;
+        for (int unit = blockIdx.x; unit < units; unit += gridDim.x, ++n) {
+            const uint32_t buf = n & 1;
+            if (n > 1) wait(&rowsFree[buf], ((n >> 1) - 1) & 1);
+            const int first = unit / shares * NR;
+            for (int pl = 0; pl < PLANES; ++pl)
+                for (int i = warp - kRowWarp; i < NR / 8 * passes; i += kRowWarps) {
+                    const int rows8 = i / passes, kg = (i - rows8 * passes) * 4 + quad, row = first + rows8 * 8 + r8;
+                    if (kg < kGroups)
+                        copyAsync16(rowPlanes + (buf * PLANES + pl) * planeBytes + rows8 * rowStride + kg * kCore + r8 * 16,
+                                    p.planes + (static_cast<size_t>(min(row, p.rows - 1)) * PLANES + pl) * kWords + 4 * kg, row < p.rows);
+                }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) arrive(&rowsFull[buf]);
+        }
+    } else if (warp == kProductWarp) {
+        uint32_t n = 0, item = 0, unitIndex = 0;
+        for (int unit = blockIdx.x; unit < units; unit += gridDim.x, ++unitIndex) {
+            const uint32_t rowBuf = unitIndex & 1;
+            wait(&rowsFull[rowBuf], (unitIndex >> 1) & 1);
+            for (int ct = tilesFrom(unit % shares); ct < tilesFrom(unit % shares + 1); ++ct, ++item) {
+                const uint32_t buf = item & 1;
+                if (item > 1) wait(&accFree[buf], ((item >> 1) - 1) & 1);
+                for (int s = 0; s < slices; ++s, ++n) {
+                    const uint32_t at = n % ring;
+                    wait(&weightFull[at], (n / ring) & 1);
+                    if (electOne()) {
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const int sliceK = min(kPad - s * kSlice, kSlice);
+                        const uint64_t descA = operandDescriptor(smemAddr(weights + at * sliceBytes), kCore, static_cast<uint32_t>(sliceK / 16) * kCore);
+                        constexpr uint64_t kStep = (2 * kCore) >> 4;   // the start-address field counts 16-byte units
+#pragma unroll
+                        for (int pl = 0; pl < PLANES; ++pl) {
+                            const uint64_t descB = operandDescriptor(smemAddr(rowPlanes + (rowBuf * PLANES + pl) * planeBytes + s * (kSlice / 16) * kCore), kCore, rowStride);
+                            for (int ks = 0; ks < sliceK / 32; ++ks)
+                                mmaI8(tmem + buf * kBufCols + pl * NR, descA + ks * kStep, descB + ks * kStep, kIdesc, s + ks > 0 ? 1u : 0u);
+                        }
+                        commitTo(smemAddr(&weightFree[at]));
+                        if (s + 1 == slices) {
+                            commitTo(smemAddr(&accFull[buf]));
+                            if (ct + 1 == tilesFrom(unit % shares + 1)) commitTo(smemAddr(&rowsFree[rowBuf]));
+                        }
+                    }
+                    __syncwarp();
+                }
             }
-            if (prevTile >= 0) epilogue(prevTile, prevCt, local - 1);
-            prevTile = rowTile;
-            prevCt = ct;
+        }
+    } else {
+        const int q = warp & 3, group = warp >> 2;   // tensor-memory lane quarter (32 channels) of this warp, row-chunk group
+        uint32_t item = 0;
+        auto channelOf = [&](int ct) { return min(ct * kChannelTile + 32 * q + lane, C - 1); };
+        typename Epilogue::Loaded loaded = epi.load(channelOf(tilesFrom(blockIdx.x % shares)));
+        for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+            const int tilesEnd = tilesFrom(unit % shares + 1);
+            for (int ct = tilesFrom(unit % shares); ct < tilesEnd; ++ct, ++item) {
+                const uint32_t buf = item & 1;
+                const int c = ct * kChannelTile + 32 * q + lane;
+                const bool real = c < C;
+                const typename Epilogue::Channel ch = epi.channel(loaded, min(c, C - 1));
+                loaded = epi.load(channelOf(ct + 1 < tilesEnd ? ct + 1 : tilesFrom((unit + gridDim.x) % shares)));
+                wait(&accFull[buf], (item >> 1) & 1);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+                for (int chunk = group; chunk < NR / 16; chunk += kEpilogueWarps / 4) {
+                    uint32_t acc[PLANES][16];
+#pragma unroll
+                    for (int pl = 0; pl < PLANES; ++pl) {
+                        asm volatile(
+                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+                            : "=r"(acc[pl][0]), "=r"(acc[pl][1]), "=r"(acc[pl][2]), "=r"(acc[pl][3]), "=r"(acc[pl][4]), "=r"(acc[pl][5]),
+                              "=r"(acc[pl][6]), "=r"(acc[pl][7]), "=r"(acc[pl][8]), "=r"(acc[pl][9]), "=r"(acc[pl][10]), "=r"(acc[pl][11]),
+                              "=r"(acc[pl][12]), "=r"(acc[pl][13]), "=r"(acc[pl][14]), "=r"(acc[pl][15])
+                            : "r"(tmem + (static_cast<uint32_t>(32 * q) << 16) + static_cast<uint32_t>(buf * kBufCols + pl * NR + 16 * chunk)));
+                    }
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (chunk + kEpilogueWarps / 4 >= NR / 16) {   // the products of the item after next may overwrite this buffer
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) arrive(&accFree[buf]);
+                    }
+                    const int row0 = unit / shares * NR + 16 * chunk;
+                    if (ch.small) {
+                        epi.template storeRows<16>(ch, static_cast<size_t>(row0), c, acc, real ? p.rows - row0 : 0);
+                        continue;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        if (row0 + j >= p.rows) break;
+                        int32_t a[PLANES];
+#pragma unroll
+                        for (int pl = 0; pl < PLANES; ++pl) a[pl] = static_cast<int32_t>(acc[pl][j]);
+                        if (real) epi.store(ch, static_cast<size_t>(row0 + j), c, a);
+                    }
+                }
+            }
         }
     }
-    if (prevTile >= 0) epilogue(prevTile, prevCt, local - 1);
-
+    if (!alive && lane == 0) atomicExch(&failed, 1);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
     if (tid == 0 && failed && p.status) atomicExch(p.status, 1);
+}
+
+// Launches the projection on at most `sms` SMs.
+template <int PLANES, class Epilogue>
+void launch(const char *name, Problem p, const Epilogue &epi, int sms, cudaStream_t st) {
+    const int kPad = paddedK(p.kWords), rows = rowsPerTile(kPad), rowTiles = (p.rows + rows - 1) / rows, channelTiles = paddedC(p.C) / kChannelTile;
+    p.ring = ringSlices(kPad, PLANES);
+    p.shares = std::max(1, std::min(channelTiles, sms / std::max(1, rowTiles)));
+    const size_t smem = sharedBytes(kPad, PLANES);
+    auto run = [&](auto kernel) {
+        ensureDynamicSmem(reinterpret_cast<const void *>(kernel), smem);
+        {
+            KernelTimer timer__(name, st);
+            kernel<<<std::max(1, std::min(rowTiles * p.shares, sms)), kThreads, smem, st>>>(p, epi);
+        }
+        afterLaunch(name);
+    };
+    if (rows == 128) run(planeProjUmma<Epilogue, PLANES, 128>);
+    else run(planeProjUmma<Epilogue, PLANES, 64>);
 }
 
 }  // namespace planeproj
