@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdint>
 
 #include "umma_device.cuh"
@@ -43,6 +44,12 @@ __device__ __forceinline__ void arriveExpect(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void barrierAll() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+
+// Dynamic shared memory that a CTA with `tmemCols` columns of tensor memory asks for at the least: its share of an SM's 228 kB (1 kB of
+// which every CTA takes by itself) is that of the tensor memory.  CTAs that fit an SM together then fit its tensor memory as well.  One too many waits in
+// tcgen05.alloc until another ends, which costs a short kernel its overlap and would stop clusters for good that wait crosswise for one
+// another's SMs.
+inline size_t leastShared(uint32_t tmemCols) { return static_cast<size_t>(228 * 1024) * tmemCols / 512 - 1024 - 512; }   // 512: the static part
 
 }  // namespace cluster
 }  // namespace rxmet

@@ -1,23 +1,26 @@
-// One step after another of a recurrence on byte-plane codes (QuantGRU W8 / A16, QuantLSTM W4 / W8 with 8- or 16-bit
-// activations) over a thread-block cluster, the product W_hh h on tcgen05 kind::i8.
+// One step after another of a recurrence on byte-plane codes (QuantLSTM W4 / W8 beyond 128 units, 16-bit activations) over a
+// thread-block cluster, the product W_hh h on tcgen05 kind::i8.
 //
 // The H / U CTAs of a cluster advance ROWS batch rows together; a CTA owns U hidden units.  Their gate channels are the
-// accumulator lanes - tiles of 128 lanes = 4 quarters (gates; a GRU leaves the fourth empty) x 32 units - and their
+// accumulator lanes - tiles of 128 lanes = 4 quarters (gates) x 32 units - and their
 // weights stay in tensor memory for the whole sequence as the A operand (lane = channel, column = four bytes along K).
-// The hidden codes of the rows, split into unsigned byte planes, are the B operand: plane p of row r is accumulator column
-// p ROWS + r, so the weights are read once for both planes.  Per step:
+// The rows of a CTA fall into one to three groups that run on their own (operands, barriers, eight epilogue warps and a control warp
+// each), so that the tensor pipe and the copies of one work under the epilogue of the others; only the weights and the operator's tables are
+// shared.  The hidden codes of a group's rows, split into unsigned byte planes, are the B operand: plane p of row r is accumulator column
+// p rows + r, so the weights are read once for both planes.  Per step and group:
 //   product -> phase A (warp = quarter, lane = unit: the operator's linear stage and, where it likes, its gate) -> exchange
 //   through shared memory inside the four warps of a tile -> phase B (lane = unit, a quarter of the rows per warp: the
 //   cell) -> the new codes of the CTA's units, staged in operand layout, travel as one bulk copy to every CTA.
 //
-// Bound: the chain of one step.  At H = 256 and 8 rows it is about 0.3 k cycles of tcgen05, 0.4 k of copy latency, 0.2 k of
-// barriers and the operator's epilogue; the operand in shared memory instead of tensor memory or an MMA issue loop
-// that is not warp-uniform double the first part.
+// Bound: the chain of one step where rows are few - about 0.3 k cycles of tcgen05, 0.4 k of copy latency, 0.2 k of
+// barriers and the operator's epilogue at H = 256 -, issue and the table look-ups where they are many.  The operand in shared memory
+// instead of tensor memory or an MMA issue loop that is not warp-uniform double the first part.  Row groups that shared product and
+// barriers took turns with them, T = 100, H = 512: 256 rows, inference 377 -> 301 us, training 580 -> 500; 2048 rows 2045 -> 1390 us.
 //
 // Synchronisation: operand and staging buffers by step parity; a CTA sends the codes of step t only after it has those of
 // step t - 1 of every peer, and a peer sends those only after its product of step t - 1 is complete: the operand
-// buffer of step t (= t - 2) and the staging buffer it came from are free by then.  Every wait is bounded; a thread whose
-// wait gave up waits no more and reports it to the operator, which turns its outputs into NaN.
+// buffer of step t (= t - 2) and the staging buffer it came from are free by then.  The epilogue warps only arrive at the barrier behind
+// the codes.  Every wait is bounded; a warp whose wait gave up waits no more and reports it to the operator, which turns its outputs into NaN.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -62,24 +65,24 @@ constexpr uint32_t powerOfTwoFrom(uint32_t n) {
 template <int HP, int U, int ROWS, int PLANES>
 struct Geometry {
     static constexpr int kCtas = HP / U, kTiles = U / 32;
-    // Warps of the epilogue; one more issues products and copies.  Three row groups where they divide the rows: they hide more of
-    // the table look-ups than two (LSTM inference, H = 512, 24 rows: 4.5 -> 4.1 us per step).
+    // Epilogue warps of all row groups; each group has a control warp beside them.  Three row groups where they divide the rows.
     static constexpr int kWarps = ROWS * kTiles < 16 ? 8 : kTiles == 2 && ROWS % 12 == 0 ? 24 : 16;
-    static constexpr int kThreads = 32 * (kWarps + 1);
-    static constexpr int kRowGroups = kWarps / (4 * kTiles);   // warps that share the rows of a tile's quarter
-    static constexpr int kRowsA = ROWS / kRowGroups;            // rows of a lane in phase A
+    static constexpr int kRowGroups = kWarps / (4 * kTiles);
+    static constexpr int kThreads = 32 * (kWarps + kRowGroups), kGroupThreads = 32 * (4 * kTiles + 1);
+    static constexpr int kRowsA = ROWS / kRowGroups;            // rows of a group = of a lane in phase A
     static constexpr int kRowsB = kRowsA / 4;                   // cells of a lane in phase B
     static_assert(kRowsA % 4 == 0 && kRowsA * kRowGroups == ROWS, "rows divide into quads");
     static constexpr int kPadK = (HP + 31) / 32 * 32;
-    static constexpr int kCols = (PLANES * ROWS + 15) / 16 * 16;          // accumulator columns of a tile
+    static constexpr int kCols = (PLANES * kRowsA + 15) / 16 * 16;        // accumulator columns of a tile and row group
     static constexpr uint32_t kColsA = kPadK / 4;                          // tensor-memory columns of its weights
-    static constexpr uint32_t kTmemCols = powerOfTwoFrom(kTiles * (kCols + kColsA));
+    static constexpr uint32_t kTmemCols = powerOfTwoFrom(kTiles * (kRowGroups * kCols + kColsA));
     static_assert(kTmemCols <= 512, "tensor memory has 512 columns");
-    static constexpr uint32_t kGroupStride = kCols * 16;                   // next 16 bytes along K
+    static constexpr uint32_t kGroupStride = kCols * 16 + 16;              // next 16 bytes along K; the odd 16 bytes part the banks of a warp's two groups
     static constexpr uint32_t kOperandBytes = kPadK / 16 * kGroupStride;
     static constexpr uint32_t kSlabBytes = U / 16 * kGroupStride;          // this CTA's units
+    static constexpr uint32_t kBufferBytes = 2 * kOperandBytes + 2 * kSlabBytes;   // of a row group
     static constexpr uint32_t kExchangeBytes = kTiles * 4 * ROWS * 32 * 4;
-    static constexpr size_t kSharedBytes = 2 * kOperandBytes + 2 * kSlabBytes + kExchangeBytes;
+    static constexpr size_t kSharedBytes = kRowGroups * kBufferBytes + kExchangeBytes;
 };
 
 struct Problem {
@@ -114,48 +117,52 @@ template <class Cell, int HP, int U, int ROWS, int PLANES>
 __global__ void __launch_bounds__(Geometry<HP, U, ROWS, PLANES>::kThreads, 1)
 planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c) {
     using G = Geometry<HP, U, ROWS, PLANES>;
-    constexpr int MT = G::kTiles, NC = G::kCtas;
+    constexpr int MT = G::kTiles, NC = G::kCtas, kFirstGroupBarrier = 1 + G::kWarps / 4;   // named barriers: one per tile and row group, one per group
     extern __shared__ __align__(128) uint8_t smemR[];
-    __shared__ __align__(8) uint64_t productBar, codeBar[2];
+    __shared__ __align__(8) uint64_t productBars[G::kRowGroups], codeBars[G::kRowGroups][2];
     __shared__ uint32_t tmemSlot;
-    __shared__ volatile int failed;   // the control warp's wait gave up
-    uint8_t *operand = smemR;                                                // [2][K / 16][kCols][16]
-    uint8_t *staging = operand + 2 * G::kOperandBytes;                       // [2][U / 16][kCols][16]
-    uint32_t *exchange = reinterpret_cast<uint32_t *>(staging + 2 * G::kSlabBytes);   // [tile][row group][4 gates][rowsA][32 units]
-    const uint32_t shared = smemAddr(smemR) + static_cast<uint32_t>(G::kSharedBytes);                    // the operator's own part
-
+    __shared__ volatile int failed[G::kRowGroups];   // the wait of a group's control warp gave up
     const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
-    const int quarter = warp & 3, tile = (warp >> 2) % MT, rowGroup = (warp >> 2) / MT;
+    const bool control = warp >= G::kWarps;
+    const int quarter = warp & 3, tile = (warp >> 2) % MT, rowGroup = control ? warp - G::kWarps : (warp >> 2) / MT;
+    uint8_t *operand = smemR + rowGroup * G::kBufferBytes;                   // [2][K / 16][kCols + 1][16]
+    uint8_t *staging = operand + 2 * G::kOperandBytes;                       // [2][U / 16][kCols + 1][16]
+    uint32_t *exchange = reinterpret_cast<uint32_t *>(smemR + G::kRowGroups * G::kBufferBytes);   // [tile][row group][4 gates][rowsA][32 units]
+    const uint32_t shared = smemAddr(smemR) + static_cast<uint32_t>(G::kSharedBytes);                    // the operator's own part
+    uint64_t &productBar = productBars[rowGroup], (&codeBar)[2] = codeBars[rowGroup];
+
     const uint32_t rank = cluster::rank();
     const int unit = static_cast<int>(rank) * U + tile * 32 + lane;
     const int b0 = static_cast<int>(blockIdx.x) / NC * ROWS;
     const int rowA = b0 + rowGroup * G::kRowsA, rowB = rowA + quarter * G::kRowsB;   // first rows of the two phases
 
     if (tid == 0) {
-        failed = 0;
-        cluster::initBarrier(&productBar, 1);
-        for (int i = 0; i < 2; ++i) cluster::initBarrier(&codeBar[i], 1);
+        for (int g = 0; g < G::kRowGroups; ++g) {
+            failed[g] = 0;
+            cluster::initBarrier(&productBars[g], 1);
+            for (int i = 0; i < 2; ++i) cluster::initBarrier(&codeBars[g][i], 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int i = 0; i < 2; ++i) cluster::arriveExpect(smemAddr(&codeBar[i]), NC * G::kSlabBytes);
+        for (int g = 0; g < G::kRowGroups; ++g)
+            for (int i = 0; i < 2; ++i) cluster::arriveExpect(smemAddr(&codeBars[g][i]), NC * G::kSlabBytes);
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(&tmemSlot)), "n"(G::kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     c.init(smemR + G::kSharedBytes, tid, G::kThreads);
-    for (uint32_t i = tid; i < (2 * G::kOperandBytes + 2 * G::kSlabBytes) / 16; i += G::kThreads)
-        reinterpret_cast<uint4 *>(operand)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (uint32_t i = tid; i < G::kRowGroups * G::kBufferBytes / 16; i += G::kThreads) reinterpret_cast<uint4 *>(smemR)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     const int H = p.H, kWords = (H + 15) / 16 * 4;   // words of a plane row
     for (int i = tid; i < ROWS * PLANES * (kWords / 4); i += G::kThreads) {
-        const int kg = i % (kWords / 4), n = i / (kWords / 4), pl = n / ROWS, r = n - pl * ROWS;
+        const int kg = i % (kWords / 4), n = i / (kWords / 4), pl = n / ROWS, r = n - pl * ROWS, g = r / G::kRowsA;
         if (b0 + r < p.B)
-            *reinterpret_cast<uint4 *>(operand + kg * G::kGroupStride + n * 16) =
+            *reinterpret_cast<uint4 *>(smemR + g * G::kBufferBytes + kg * G::kGroupStride + (pl * G::kRowsA + r - g * G::kRowsA) * 16) =
                 *reinterpret_cast<const uint4 *>(p.h0 + (static_cast<size_t>(b0 + r) * PLANES + pl) * kWords + 4 * kg);
     }
-    const uint32_t tmem = __shfl_sync(0xffffffffu, tmemSlot, 0), tmemWeights = tmem + MT * G::kCols;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmemSlot, 0), tmemWeights = tmem + MT * G::kRowGroups * G::kCols;
     const uint32_t quarterBase = static_cast<uint32_t>(32 * quarter) << 16;
-    if (rowGroup == 0 && warp < G::kWarps)
+    if (rowGroup == 0 && !control)
         for (int kw = 0; kw < G::kPadK / 4; kw += 4) {
             uint32_t w[4];
 #pragma unroll
@@ -170,12 +177,13 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     constexpr uint32_t kIdesc = planeproj::instructionDescriptor(G::kCols);
-    bool alive = true;   // false once one of this thread's waits gave up
+    bool alive = true;   // false once a wait of this warp gave up
     auto wait = [&](uint32_t bar, uint32_t parity) {
-        if (alive) alive = waitPhase(bar, parity);
+        if (alive) alive = __all_sync(0xffffffffu, G::kWarps > 8 ? waitSuspended(bar, parity) : waitPhase(bar, parity));   // polling wakes 2 % of a step earlier
     };
-    if (warp == G::kWarps) {
-        // ---- control warp: products and copies; lane d sends to CTA d
+    const uint32_t tmemGroup = tmem + rowGroup * G::kCols;   // accumulators of this row group, MT tiles of kRowGroups kCols
+    if (control) {
+        // ---- control warp of a row group: products and copies; lane d sends to CTA d
         const uint32_t peer = static_cast<uint32_t>(lane) % NC;
         const uint32_t sendTo = cluster::remote(smemAddr(operand), peer) + rank * G::kSlabBytes;
         const uint32_t sendBar = cluster::remote(smemAddr(&codeBar[0]), peer);
@@ -184,6 +192,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
         for (int t = 0; t < p.T; ++t) {
             const uint32_t bar = smemAddr(&codeBar[0]) + (t & 1) * 8;
             if (t > 0) wait(bar, ((t - 1) >> 1) & 1);
+            if (!alive) failed[rowGroup] = 1;
             if (electOne()) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t descB = descB0 + static_cast<uint64_t>((t & 1) * (G::kOperandBytes >> 4));
@@ -191,14 +200,13 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
                 for (int m = 0; m < MT; ++m)
 #pragma unroll
                     for (int ks = 0; ks < G::kPadK / 32; ++ks)
-                        mmaI8TmemA(tmem + m * G::kCols, tmemWeights + m * G::kColsA + ks * 8,
+                        mmaI8TmemA(tmemGroup + m * (G::kRowGroups * G::kCols), tmemWeights + m * G::kColsA + ks * 8,
                                    descB + static_cast<uint64_t>(ks * ((2 * G::kGroupStride) >> 4)), kIdesc, ks > 0 ? 1u : 0u);
                 commitTo(smemAddr(&productBar));
                 if (t > 0) cluster::arriveExpect(bar, NC * G::kSlabBytes);   // for step t + 2
             }
             __syncwarp();
-            if (!alive) failed = 1;
-            __syncthreads();   // the codes of step t are staged
+            asm volatile("bar.sync %0, %1;" ::"r"(kFirstGroupBarrier + rowGroup), "n"(G::kGroupThreads) : "memory");   // the codes of step t are staged
             if (t + 1 < p.T && lane < NC)
                 cluster::copyTo(sendTo + ((t + 1) & 1) * G::kOperandBytes, smemAddr(staging) + (t & 1) * G::kSlabBytes, G::kSlabBytes,
                                 sendBar + ((t + 1) & 1) * 8);
@@ -217,9 +225,9 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
 #pragma unroll
         for (int i = 0; i < G::kRowsB; ++i)
             if (real && rowB + i < p.B) c.begin(shared, state[i], rowB + i, unit);
-        const uint32_t column = tmem + quarterBase + tile * G::kCols + rowGroup * G::kRowsA;
+        const uint32_t column = tmemGroup + quarterBase + tile * (G::kRowGroups * G::kCols);
         uint32_t *exchangeTile = exchange + (tile * G::kRowGroups + rowGroup) * (4 * G::kRowsA * 32) + lane;
-        uint8_t *stageMine = staging + (tile * 2 + (lane >> 4)) * G::kGroupStride + (rowB - b0) * 16 + (lane & 15);
+        uint8_t *stageMine = staging + (tile * 2 + (lane >> 4)) * G::kGroupStride + (rowB - rowA) * 16 + (lane & 15);
 #pragma unroll 1
         for (int t = 0; t < p.T; ++t) {
             const size_t at = static_cast<size_t>(t) * p.B;   // first row of the step in the [T][B] arrays
@@ -250,7 +258,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
 #pragma unroll
                 for (int pl = 0; pl < PLANES; ++pl)
 #pragma unroll
-                    for (int r = 0; r < kChunk; r += 4) tmemLoad4(column + pl * ROWS + first + r, acc + pl * kChunk + r);
+                    for (int r = 0; r < kChunk; r += 4) tmemLoad4(column + pl * G::kRowsA + first + r, acc + pl * kChunk + r);
                 typename Cell::Fetch later[kChunk];
                 if (!kAll && first + kChunk < G::kRowsA) fetchA(later, first + kChunk, kChunk);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -290,25 +298,27 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
                 uint8_t *dst = stageMine + (t & 1) * G::kSlabBytes + i * 16;
                 if (PLANES == 2) {
                     dst[0] = static_cast<uint8_t>(u >> 8);
-                    dst[ROWS * 16] = static_cast<uint8_t>(u);
+                    dst[G::kRowsA * 16] = static_cast<uint8_t>(u);
                 } else {
                     dst[0] = static_cast<uint8_t>(u);
                 }
-                if (!kDefer && !kAll && exists) c.store(state[i], inB[i], at, rowB + i, unit, valid && alive && !failed);
+                if (!kDefer && !kAll && exists) c.store(state[i], inB[i], at, rowB + i, unit, valid && alive && !failed[rowGroup]);
             }
-            if constexpr (!kDefer && kAll) c.storeRows(state, inB, at, rowB, unit, valid && alive && !failed, real ? p.B - rowB : 0);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncthreads();
+            // the control warp sends the codes; a warp whose wait gave up must not run ahead of the others and waits here
+            if (alive) asm volatile("bar.arrive %0, %1;" ::"r"(kFirstGroupBarrier + rowGroup), "n"(G::kGroupThreads) : "memory");
+            else asm volatile("bar.sync %0, %1;" ::"r"(kFirstGroupBarrier + rowGroup), "n"(G::kGroupThreads) : "memory");
+            if constexpr (!kDefer && kAll) c.storeRows(state, inB, at, rowB, unit, valid && alive && !failed[rowGroup], real ? p.B - rowB : 0);
             if constexpr (kDefer && kAll) {   // what nobody waits for leaves while the codes travel and the next product runs
-                c.storeRows(state, inB, at, rowB, unit, valid && alive && !failed, real ? p.B - rowB : 0);
+                c.storeRows(state, inB, at, rowB, unit, valid && alive && !failed[rowGroup], real ? p.B - rowB : 0);
                 if constexpr (Cell::kSaves) {
                     if (quarter < Cell::kGates) c.storeLinearRows(mine, saved, at, rowA, quarter, unit, real ? p.B - rowA : 0);
                 }
             } else if (kDefer) {
 #pragma unroll
                 for (int i = 0; i < G::kRowsB; ++i)
-                    if (real && rowB + i < p.B) c.store(state[i], inB[i], at, rowB + i, unit, valid && alive && !failed);
+                    if (real && rowB + i < p.B) c.store(state[i], inB[i], at, rowB + i, unit, valid && alive && !failed[rowGroup]);
                 if (Cell::kSaves && quarter < Cell::kGates) {
 #pragma unroll
                     for (int r = 0; r < kChunk; ++r)
@@ -318,7 +328,7 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
         }
 #pragma unroll
         for (int i = 0; i < G::kRowsB; ++i)
-            if (real && rowB + i < p.B) c.finish(state[i], rowB + i, unit, valid && alive && !failed);
+            if (real && rowB + i < p.B) c.finish(state[i], rowB + i, unit, valid && alive && !failed[rowGroup]);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -326,12 +336,18 @@ planeRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell 
     cluster::barrierAll();   // nobody leaves while a peer may still copy into its shared memory
 }
 
+template <class Cell, int HP, int U, int ROWS, int PLANES>
+size_t sharedBytes(const Cell &cell) {
+    using G = Geometry<HP, U, ROWS, PLANES>;
+    return std::max(G::kSharedBytes + cell.sharedBytes(), cluster::leastShared(G::kTmemCols));
+}
+
 // Launches a variant with its clusters.
 template <class Cell, int HP, int U, int ROWS, int PLANES>
 void launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t st) {
     using G = Geometry<HP, U, ROWS, PLANES>;
     const auto kernel = planeRecurrence<Cell, HP, U, ROWS, PLANES>;
-    const size_t smem = G::kSharedBytes + cell.sharedBytes();
+    const size_t smem = sharedBytes<Cell, HP, U, ROWS, PLANES>(cell);
     ensureDynamicSmem(reinterpret_cast<const void *>(kernel), smem);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(static_cast<unsigned>((p.B + ROWS - 1) / ROWS * G::kCtas));
@@ -362,11 +378,11 @@ void launchBest(const char *name, const Problem &p, const Cell &cell, cudaStream
         [&] {
             using G = Geometry<HP, U, ROWS, PLANES>;
             // a single wave of it would not beat what is found already: do not even load the variant
-            if (1.0 + ROWS / static_cast<double>(PER) >= bestCost || G::kSharedBytes + cell.sharedBytes() > static_cast<size_t>(currentDevice().smemMax)) return;
+            if (1.0 + ROWS / static_cast<double>(PER) >= bestCost || sharedBytes<Cell, HP, U, ROWS, PLANES>(cell) > static_cast<size_t>(currentDevice().smemMax)) return;
             const int resident = std::max(1, residentClusters(reinterpret_cast<const void *>(planeRecurrence<Cell, HP, U, ROWS, PLANES>), G::kCtas,
-                                                              G::kThreads, G::kSharedBytes + cell.sharedBytes()) / concurrentPasses());
+                                                              G::kThreads, sharedBytes<Cell, HP, U, ROWS, PLANES>(cell)) / concurrentPasses());
             const int clusters = (p.B + ROWS - 1) / ROWS, waves = (clusters + resident - 1) / resident;
-            if (ROWS == 4 && 2 * clusters > resident) return;
+            if (ROWS == 4 && G::kTmemCols > 256 && 2 * clusters > resident) return;
             const double cost = waves * (1.0 + ROWS / static_cast<double>(PER));
             if (cost < bestCost) { bestCost = cost; best = ROWS; }
         }(),

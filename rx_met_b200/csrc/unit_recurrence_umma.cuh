@@ -261,9 +261,7 @@ unitRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c
 template <class Cell, int HP, int U, int ROWS, int PLANES>
 size_t sharedBytes(const Cell &cell) {
     using G = Geometry<Cell, HP, U, ROWS, PLANES>;
-    // no more CTAs on an SM than its tensor memory holds: one more would wait there for the whole sequence of another
-    const size_t least = static_cast<size_t>(currentDevice().smemMax) / (512 / G::kTmemCols + 1) + 1024;
-    return std::max(G::kSharedBytes + cell.sharedBytes(), least);
+    return std::max(G::kSharedBytes + cell.sharedBytes(), cluster::leastShared(G::kTmemCols));
 }
 
 template <class Cell, int HP, int U, int ROWS, int PLANES>

@@ -1,4 +1,4 @@
-"""The recurrences with a thread per hidden unit (QuantLSTM up to 128 units, QuantGRU W8 / A16 up to 256): the edges of widths, of rows per CTA
+"""The recurrences with a thread per hidden unit (QuantLSTM up to 128 units, QuantGRU W8 / A16 up to 256) and over clusters: the edges of widths, of rows per CTA
 or cluster and of step counts, every form of what a forward saves, against the CPU checkers."""
 from __future__ import annotations
 
@@ -69,3 +69,10 @@ def test_gru_units_save_what_is_asked_for(T, B, I, H):
         assert np.array_equal(out[0], want["h"]) and np.array_equal(out[1], want["v"])
         for name, flags in zip(_cabi.MASK_NAMES, out[7:]):
             assert flags.size == 0 if not training else np.array_equal(flags, want["masks"].arr[name]), name
+
+
+# clusters with one to three row groups that run on their own: every number of rows, groups and clusters partly empty
+@pytest.mark.parametrize("T,B,H", [(3, 5, 512), (2, 67, 512), (2, 130, 512), (3, 201, 500), (2, 257, 512), (1, 390, 410), (2, 701, 512), (4, 9, 129), (2, 131, 256),
+                                   (3, 261, 200), (2, 401, 256)])
+def test_lstm_clusters(T, B, H):
+    lstm_forward_matches(T, B, 6, H, 8, 16, L.PER_CHANNEL, True, True)
