@@ -1369,11 +1369,8 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         const size_t smem = sizeof(float) * (static_cast<size_t>(bt) * 3 * 2 * CW + 3 * static_cast<size_t>(bt) * H);
         const int grid = (B + bt - 1) / bt;
         auto launchMma = [&](const BackwardQArgs &qa) {
-            // Narrow layers keep the one-CTA kernel while its batch tiles fit one wave of small tiles: 0.68 against 0.85 us
-            // per step at H = 32 and 0.83 against 0.88 at H = 64 (B = 64); it loses from B = 512 and 256 on (0.88 / 0.86
-            // and 0.97 / 0.90), and everywhere at H = 96 (1.17 / 0.87) and 128 (1.40 / 0.91).
-            const bool narrow = (H == 32 && B <= 256) || (H == 64 && B <= 128);
-            if (!narrow && backwardClusterTakes(qa, call.R_q)) return backwardCluster(qa, call.R_q, st);
+            // the register kernels below serve misaligned tensors
+            if (backwardClusterTakes(qa, call.R_q)) return backwardCluster(qa, call.R_q, st);
             KernelTimer timer__("recurrentBackward", st);
 #define RXMET_BWD_CASE(HTV, BTV) \
     if (H == 32 * HTV && bt == BTV) recurrentBackwardMma<HTV, BTV><<<grid, 96 * HTV, 0, st>>>(qa, call.R_q);

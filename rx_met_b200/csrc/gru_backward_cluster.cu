@@ -345,10 +345,6 @@ Variant variant() {
 template <int ROWS>
 Variant variantFor(int H) {
     switch (H) {
-        case 32: return variant<32, ROWS>();
-        case 64: return variant<64, ROWS>();
-        case 96: return variant<96, ROWS>();
-        case 128: return variant<128, ROWS>();
         case 160: return variant<160, ROWS>();
         case 192: return variant<192, ROWS>();
         case 224: return variant<224, ROWS>();
@@ -366,6 +362,7 @@ bool backwardClusterTakes(const BackwardQArgs &q, const int32_t *Rq) {
 }
 
 void backwardCluster(const BackwardQArgs &q, const int32_t *Rq, cudaStream_t st) {
+    if (q.H <= 128) return backwardUnits(q, Rq, st);   // inside one CTA
     ClusterArgs args{};
     args.q = q;
     args.Rq = Rq;

@@ -28,6 +28,8 @@ struct BackwardQArgs {
 // paired accesses.  `Rq` = [H][3H] int32 codes of at most 8 bits.
 bool backwardClusterTakes(const BackwardQArgs &q, const int32_t *Rq);
 void backwardCluster(const BackwardQArgs &q, const int32_t *Rq, cudaStream_t stream);
+// Its part up to 128 units, in steps of 32 (gru_backward_units.cu).
+void backwardUnits(const BackwardQArgs &q, const int32_t *Rq, cudaStream_t stream);
 
 }  // namespace gru
 }  // namespace rxmet

@@ -81,7 +81,7 @@ enum class Saves { None, Packed, Any };
 template <Saves SAVES, int WIDTH>
 struct GruUnitCell {
     static constexpr int kGates = 3;
-    static constexpr bool kFlags = SAVES != Saves::None, kTwoRows = true;
+    static constexpr bool kFlags = SAVES != Saves::None, kTwoRows = true, kSignedCodes = false;
     CellScalars s;
     FastLut luts[3];
     int width;
@@ -125,6 +125,7 @@ struct GruUnitCell {
         const int H = hidden();
         return __ldg(words + static_cast<size_t>(kw) * 3 * H + gate * H + unit);
     }
+    __device__ __forceinline__ uint32_t codeWord(const planerec::Problem &p, int row, int plane, int kw) const { return unitrec::planeWord<2>(p, row, plane, kw); }
     __device__ __forceinline__ void init(uint8_t *at, uint32_t shared, int tid, int threads) const {
         for (int i = tid; i < static_cast<int>(sizeof(luts) / 4); i += threads) {
             const int g = i / static_cast<int>(sizeof(FastLut) / 4), within = i % static_cast<int>(sizeof(FastLut) / 4);
@@ -321,7 +322,7 @@ void launchFor(const WideRecurrence &r, const Prepared &prepared, cudaStream_t s
     cell.maskHh = r.maskHh; cell.maskGateIn = r.maskGateIn; cell.maskGateOut = r.maskGateOut; cell.maskH = r.maskH;
     cell.maskIh = r.maskIh; cell.stepBits = r.stepBits;
     cell.poison = r.poison;
-    unitrec::launchRows<Cell, HP, 2>("recurrentForward", planerec::Problem{r.T, r.B, r.H, r.h0Planes}, cell, st);
+    unitrec::launchRows<Cell, HP, 2>("recurrentForward", planerec::Problem{r.T, r.B, r.H, r.h0Planes}, cell, true, st);
 }
 template <int HP>
 void launchFor(const WideRecurrence &r, const Prepared &prepared, cudaStream_t st) {

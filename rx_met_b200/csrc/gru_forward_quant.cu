@@ -30,6 +30,7 @@
 #include "common.h"
 #include "dependent_launch.cuh"
 #include "gru_device.cuh"
+#include "gru_forward_bytes.h"
 #include "gru_forward_quant.h"
 #include "gru_forward_wide.h"
 #include "input_proj_umma.h"
@@ -1796,6 +1797,14 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
                 afterLaunch("recurrentForwardI8");
             };
             if (chunks.size() == 1) {
+                const bool saves = a.hq || a.vq || a.maskHh || a.maskGateIn || a.stepBits;
+                if (mode == 2 && std::getenv("RXMET_GRU_FWD_BT") == nullptr && forwardBytesTakes(B, H, saves)) {
+                    forwardBytes(ByteRecurrence{T, B, H, hWords, reinterpret_cast<const uint32_t *>(rCodes), compH, biasH, ch.gemmH,
+                                                reinterpret_cast<const int16_t *>(ihCodes), reinterpret_cast<const int8_t *>(a.h0), a.h, a.v, a.hq, a.vq, a.maskHh,
+                                                a.maskGateIn, a.maskGateOut, a.maskH, a.maskIh, a.stepBits, a.poison},
+                                 g, st);
+                    return;
+                }
                 launchSteps(a);
                 return;
             }
@@ -2137,10 +2146,13 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, 
         return;
     }
     const CodeClass w = e.weightClass, a = e.actClass, l = e.linearClass;
-    // 16-bit codes, and 8-bit ones too wide for the lanes path: the register path below holds R of 256 units in spilled
-    // registers (H = 192, B = 500, T = 98: 666 us against 298 us over clusters)
+    // 16-bit codes, and 8-bit ones beyond 128 units that the recurrence on bytes does not take: the register path below holds R of 256
+    // units in spilled registers (H = 192, B = 500, T = 98: 666 us against 298 us over clusters)
+    const bool bytes = w == CodeClass::I8 && a == CodeClass::I8 && l == CodeClass::I16 && fastGateMath(e.gate) && forwardBytesTakes(call.B, call.H, true) &&
+                       std::getenv("RXMET_GRU_FWD_MODE") == nullptr && std::getenv("RXMET_GRU_FWD_BT") == nullptr &&
+                       iproj::eligible(3 * call.H, call.H, padTo(call.I, 4) / 4, nullptr, nullptr, nullptr);
     if (forwardWideTakes(e, call.I, call.H) &&
-        (a == CodeClass::I16 || (call.H > 128 && !call.stepFlags && forwardWideClusterTakes(e, call.B, call.H)))) {
+        (a == CodeClass::I16 || (call.H > 128 && !call.stepFlags && !bytes && forwardWideClusterTakes(e, call.B, call.H)))) {
         runWide(call, e, ws, st);
         return;
     }

@@ -19,10 +19,6 @@ Variant variant() {
 template <int ROWS>
 Variant variantFor(int H) {
     switch (H) {
-        case 32: return variant<32, ROWS>();
-        case 64: return variant<64, ROWS>();
-        case 96: return variant<96, ROWS>();
-        case 128: return variant<128, ROWS>();
         case 160: return variant<160, ROWS>();
         case 192: return variant<192, ROWS>();
         case 224: return variant<224, ROWS>();
@@ -48,6 +44,7 @@ bool backwardClusterTakes(const BackwardClusterArgs &a) {
 }
 
 void backwardCluster(const BackwardClusterArgs &args, cudaStream_t st) {
+    if (args.H <= 128) return backwardUnits(args, st);   // inside one CTA
     // Rows of a cluster: as few as let all clusters of the pass run at the same time (a step costs about 1 + rows / 32
     // of the chain of a one-row step, a second wave costs the whole chain again).
     int best = 4;

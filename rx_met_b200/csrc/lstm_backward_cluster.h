@@ -27,6 +27,8 @@ struct BackwardClusterArgs {
 // True when the kernel takes the call: hidden units in tiles of 32, at most 512 of them, pointers aligned for its paired accesses.
 bool backwardClusterTakes(const BackwardClusterArgs &args);
 void backwardCluster(const BackwardClusterArgs &args, cudaStream_t stream);
+// Its part up to 128 units, in steps of 32 (lstm_backward_units.cu).
+void backwardUnits(const BackwardClusterArgs &args, cudaStream_t stream);
 
 }  // namespace lstm
 }  // namespace rxmet

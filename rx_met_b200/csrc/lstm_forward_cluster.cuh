@@ -307,9 +307,9 @@ struct LstmUnitConstants {
     float hhLo, hhHi, cLo, cHi, oLo, oHi, productScale, codePlus;
     int plain;                            // the cell's ratios are single factors
 };
-template <Saves SAVES, int WIDTH = 0>
+template <Saves SAVES, int PLANES, int WIDTH = 0>
 struct LstmUnitCell : LstmPlaneCell<SAVES != Saves::None, WIDTH> {
-    static constexpr bool kTrain = SAVES != Saves::None, kTwoRows = !kTrain;
+    static constexpr bool kTrain = SAVES != Saves::None, kTwoRows = !kTrain, kSignedCodes = false;
     using Base = LstmPlaneCell<kTrain, WIDTH>;
     LstmUnitConstants k;
     struct Unit {
@@ -352,6 +352,7 @@ struct LstmUnitCell : LstmPlaneCell<SAVES != Saves::None, WIDTH> {
         k.codePlus = 8388608.0f + static_cast<float>(s.zp[RXMET_LSTM_OUTPUT] - s.lo[RXMET_LSTM_OUTPUT]);
         k.plain = !s.forgetUsesFp && !s.inputUsesFp;
     }
+    __device__ __forceinline__ uint32_t codeWord(const planerec::Problem &p, int row, int plane, int kw) const { return unitrec::planeWord<PLANES>(p, row, plane, kw); }
     __device__ __forceinline__ void init(uint8_t *at, uint32_t, int tid, int threads) const { Base::init(at, tid, threads); }
     __device__ __forceinline__ Unit unitOf(uint32_t shared, int unit) const {
         Unit u;
@@ -385,7 +386,7 @@ struct LstmUnitCell : LstmPlaneCell<SAVES != Saves::None, WIDTH> {
         const LstmUnitConstants::Table &v = k.table[t];
         return lookup(TableView{u.shared + v.segments, u.shared + v.bits, v.toIndex, v.outLo, v.outHi}, this->segShift, x, index);
     }
-    template <int PLANES, bool PLAIN>
+    template <int, bool PLAIN>
     __device__ __forceinline__ uint32_t advance(const Unit &u, State &st, const Fetch &in, const uint32_t (&acc)[4][PLANES], Out &o) const {
         const auto &s = this->s;
 #pragma unroll
@@ -450,12 +451,12 @@ struct LstmUnitCell : LstmPlaneCell<SAVES != Saves::None, WIDTH> {
 template <Saves SAVES, int HP, int PLANES>
 void launchLstmUnits(const char *name, const planerec::Problem &p, const LstmPlaneCell<SAVES != Saves::None> &cell, cudaStream_t st) {
     auto run = [&](auto width) {
-        using Cell = LstmUnitCell<SAVES, decltype(width)::value>;
+        using Cell = LstmUnitCell<SAVES, PLANES, decltype(width)::value>;
         static_assert(sizeof(typename Cell::Base) == sizeof(cell), "the variants differ in the width only");
         Cell c;
         std::memcpy(static_cast<typename Cell::Base *>(&c), &cell, sizeof(cell));
         c.prepareConstants();
-        unitrec::launchRows<Cell, HP, PLANES>(name, p, c, st);
+        unitrec::launchRows<Cell, HP, PLANES>(name, p, c, true, st);
     };
     if (p.H == HP) run(std::integral_constant<int, HP>{});
     else run(std::integral_constant<int, 0>{});

@@ -25,6 +25,7 @@
 
 #include "cluster_device.cuh"
 #include "common.h"
+#include "dependent_launch.cuh"
 #include "plane_recurrence_umma.cuh"
 
 namespace rxmet {
@@ -42,6 +43,12 @@ __device__ __forceinline__ void tmemLoad(uint32_t addr, uint32_t *r) {
 #pragma unroll
         for (int i = 0; i < N; i += 4) planerec::tmemLoad4(addr + i, r + i);
     }
+}
+
+// A word of the initial codes at Problem::h0.
+template <int PLANES>
+__device__ __forceinline__ uint32_t planeWord(const Problem &p, int row, int plane, int kw) {
+    return __ldg(p.h0 + (static_cast<size_t>(row) * PLANES + plane) * ((p.H + 15) / 16 * 4) + kw);
 }
 
 template <class Cell, int HP, int U, int ROWS, int PLANES>
@@ -67,9 +74,10 @@ struct Geometry {
 
 // Cell contract (device functions unless marked; `at` = first row of the step in the [T][B] arrays, `shared` = address of the
 // operator's part of shared memory):
-//   kGates, kTwoRows                                        accumulator tiles; whether a thread has registers for two rows
+//   kGates, kTwoRows, kSignedCodes                          accumulator tiles; whether a thread has registers for two rows; codes as signed bytes
 //   size_t sharedBytes()                                    host: size of that part
 //   uint32_t weightWord(gate, unit, kw)                     four weight bytes along K
+//   uint32_t codeWord(Problem, row, plane, kw)              four bytes of the initial codes; [B][PLANES][kWords] words at Problem::h0 or its own
 //   void init(uint8_t *, shared, tid, threads)              fills it
 //   bool valid()                                            false: the inputs are not good, outputs become NaN
 //   Unit unitOf(shared, unit)                               constants of a unit (all lanes of the warp call it); Unit::plain, uniform in the
@@ -115,18 +123,22 @@ unitRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c
     }
     c.init(smemU + G::kSharedBytes, shared, tid, G::kThreads);
     for (uint32_t i = tid; i < G::kSharedBytes / 16; i += G::kThreads) reinterpret_cast<uint4 *>(operand)[i] = make_uint4(0u, 0u, 0u, 0u);
+    waitForPredecessor();   // what is above needs nothing from earlier kernels
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int kWords = (p.H + 15) / 16 * 4;   // words of a plane row
     for (int i = tid; i < ROWS * PLANES * (kWords / 4); i += G::kThreads) {
         const int kg = i % (kWords / 4), n = i / (kWords / 4), row = min(b0 + n / PLANES, p.B - 1);
-        *reinterpret_cast<uint4 *>(operand + kg * G::kGroupStride + n * 16) =
-            *reinterpret_cast<const uint4 *>(p.h0 + (static_cast<size_t>(row) * PLANES + n % PLANES) * kWords + 4 * kg);
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[e] = c.codeWord(p, row, n % PLANES, 4 * kg + e);
+        *reinterpret_cast<uint4 *>(operand + kg * G::kGroupStride + n * 16) = make_uint4(w[0], w[1], w[2], w[3]);
     }
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmemSlot, 0), tmemWeights = tmem + kGates * G::kCols;
     const uint32_t quarterBase = static_cast<uint32_t>(32 * quarter) << 16;
     if (warp < G::kWarps)   // the warps of a quarter share its weights
+#pragma unroll 4
         for (int i = group; i < kGates * (HP / 16); i += G::kGroups) {
             const int g = i / (HP / 16), kw = i % (HP / 16) * 4;
             uint32_t w[4];
@@ -152,7 +164,7 @@ unitRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c
     };
     if (warp == G::kWarps) {
         // ---- control warp: products and copies; lane d sends to CTA d
-        constexpr uint32_t kIdesc = planeproj::instructionDescriptor(G::kCols);
+        constexpr uint32_t kIdesc = planeproj::instructionDescriptor(G::kCols) | (Cell::kSignedCodes ? 1u << 10 : 0u);   // B format signed 8-bit
         const uint64_t descB0 = operandDescriptor(smemAddr(operand), G::kGroupStride, kCore);
         const uint32_t peer = static_cast<uint32_t>(lane) % NC;
         const uint32_t sendTo = NC == 1 ? 0u : cluster::remote(smemAddr(operand), peer) + rank * G::kSlabBytes;
@@ -261,11 +273,14 @@ unitRecurrence(const __grid_constant__ Problem p, const __grid_constant__ Cell c
 template <class Cell, int HP, int U, int ROWS, int PLANES>
 size_t sharedBytes(const Cell &cell) {
     using G = Geometry<Cell, HP, U, ROWS, PLANES>;
-    return std::max(G::kSharedBytes + cell.sharedBytes(), cluster::leastShared(G::kTmemCols));
+    // CTAs by themselves need not keep clusters out, only one CTA too many of their own kind, which would wait there for another's whole sequence
+    const size_t least = G::kCtas > 1 ? cluster::leastShared(G::kTmemCols) : static_cast<size_t>(currentDevice().smemMax) / (512 / G::kTmemCols + 1) + 1024;
+    return std::max(G::kSharedBytes + cell.sharedBytes(), least);
 }
 
+// `early`: before the kernel in front of it has ended (its prologue runs beside that one's end).
 template <class Cell, int HP, int U, int ROWS, int PLANES>
-void launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t st) {
+void launch(const char *name, const Problem &p, const Cell &cell, bool early, cudaStream_t st) {
     using G = Geometry<Cell, HP, U, ROWS, PLANES>;
     const auto kernel = unitRecurrence<Cell, HP, U, ROWS, PLANES>;
     const size_t smem = sharedBytes<Cell, HP, U, ROWS, PLANES>(cell);
@@ -275,12 +290,14 @@ void launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t s
     cfg.blockDim = dim3(G::kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = G::kCtas;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = G::kCtas > 1 ? 1 : 0;
+    cudaLaunchAttribute attrs[2] = {};
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = G::kCtas;
+    attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
+    cfg.attrs = attrs;
+    cfg.numAttrs = G::kCtas > 1 ? 2 : 1;
     {
         KernelTimer timer__(name, st);
         RXMET_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, cell));
@@ -293,7 +310,7 @@ void launch(const char *name, const Problem &p, const Cell &cell, cudaStream_t s
 // better than one of twice the rows (W8 / A16 LSTM inference, T = 100, H = 128: one row a CTA 56 us at 128 rows, two 66 at 256 and 94 at 592, where
 // four take 99; four 144 at 1184, where two take 182 in two waves).
 template <class Cell, int HP, int PLANES>
-void launchRows(const char *name, const Problem &p, const Cell &cell, cudaStream_t st) {
+void launchRows(const char *name, const Problem &p, const Cell &cell, bool early, cudaStream_t st) {
     constexpr int U = HP <= 128 ? HP : 64, kLeast = HP > 128 ? 4 : 128 / U;
     auto fits = [&](auto rows) {
         constexpr int R = decltype(rows)::value;
@@ -304,7 +321,7 @@ void launchRows(const char *name, const Problem &p, const Cell &cell, cudaStream
         return groups <= G::kResident * residentClusters(reinterpret_cast<const void *>(unitRecurrence<Cell, HP, U, R, PLANES>), G::kCtas,
                                                          G::kThreads, sharedBytes<Cell, HP, U, R, PLANES>(cell)) / concurrentPasses();
     };
-    auto with = [&](auto rows) { unitrec::launch<Cell, HP, U, decltype(rows)::value, PLANES>(name, p, cell, st); };
+    auto with = [&](auto rows) { unitrec::launch<Cell, HP, U, decltype(rows)::value, PLANES>(name, p, cell, early, st); };
     if (fits(std::integral_constant<int, kLeast>{})) return with(std::integral_constant<int, kLeast>{});
     constexpr int kNext = 2 * kLeast, kMost = HP > 128 ? kNext : 2 * kNext;
     if constexpr (kNext < kMost && Cell::kTwoRows) {
