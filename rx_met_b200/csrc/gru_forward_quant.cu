@@ -1642,9 +1642,10 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
         const int kw4 = (iWords + 3) / 4;
         bool specialised = false;
         if constexpr (kI8) {
-            // channel counts that leave the last tile partly empty: only where the register kernel below does not go
+            // channel counts that leave the last tile partly empty: where the register kernel below does not go, or with many rows
+            // (PARTIALNUMBERS)
             const bool registerProjection = C <= 512 && kw4 <= 4 && block >= kI8Rows * kw4 * 4;
-            if (iproj::eligible(C, H, iWords, xCodes, ihCodes, mk.weight_ih_linear) && (C % 128 == 0 || !registerProjection) &&
+            if (iproj::eligible(C, H, iWords, xCodes, ihCodes, mk.weight_ih_linear) && (C % 128 == 0 || !registerProjection || rows >= 8192) &&
                 std::getenv("RXMET_GRU_FWD_GENERIC") == nullptr) {
                 // tcgen05 kind::i8 GEMM with the fused epilogue
                 specialised = true;

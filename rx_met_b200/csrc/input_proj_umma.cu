@@ -27,6 +27,7 @@
 #include "dependent_launch.cuh"
 #include "gru_device.cuh"
 #include "input_proj_umma.h"
+#include "plane_proj_umma.cuh"
 #include "umma_device.cuh"
 
 namespace rxmet {
@@ -56,7 +57,9 @@ __device__ __forceinline__ void mmaI8(uint32_t tmemD, uint64_t descA, uint64_t d
         : "memory");
 }
 
-constexpr int kRows = 128;  // rows of the batch per work item = accumulator columns
+// Rows of the batch per work item = accumulator columns.  25,600 rows of 384 channels are 1200 items of 64 rows: four to five for each of the 296
+// CTAs, where 600 of 128 rows were two to three.
+constexpr int kRows = 64;
 
 __host__ __device__ inline int paddedC(int C) { return (C + kTileM - 1) / kTileM * kTileM; }
 size_t sharedBytes(int C, int kPad) { return static_cast<size_t>(paddedC(C)) * kPad + 2 * static_cast<size_t>(kRows) * kPad; }
@@ -138,14 +141,20 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
         const int64_t offset = p.biasAcc[c] - p.comp[c];
         const bool narrow = rs.shift >= 1 && rs.shift <= 31 && rs.mult > 0 && static_cast<int64_t>(rs.mult) <= (1ll << rs.shift) &&
                             offset > -(1ll << 30) && offset < (1ll << 30);
-        const int64_t mulAdd = offset * static_cast<int64_t>(rs.mult);
-        const uint32_t remMask = (1u << (rs.shift & 31)) - 1u, half = 1u << ((rs.shift - 1) & 31);
         const Rescale gateRs = p.pre.enabled ? p.pre.toGate[c / p.pre.hidden] : Rescale{1, 0};
-        const int64_t gateAdd = -static_cast<int64_t>(zpOut) * gateRs.mult;
         const bool gateNarrow = gridsSmall && gateRs.shift >= 1 && gateRs.shift <= 31 && gateRs.mult > 0 &&
                                 static_cast<int64_t>(gateRs.mult) <= (1ll << min(gateRs.shift + 9, 31));
-        const uint32_t gateMask = (1u << (gateRs.shift & 31)) - 1u, gateHalf = 1u << ((gateRs.shift - 1) & 31);
         const bool warpNarrow = __all_sync(0xffffffffu, narrow && (!p.pre.enabled || gateNarrow));
+        // Narrow: half a unit rides in the addend, the floor is right then except for an exact tie, where it is the upper neighbour and an
+        // odd one must step down.
+        const int64_t plus = offset * rs.mult + (narrow ? int64_t{1} << (rs.shift - 1) : 0);
+        const int64_t gatePlus = -static_cast<int64_t>(zpOut) * gateRs.mult + (gateNarrow ? int64_t{1} << (gateRs.shift - 1) : 0);
+        const uint32_t tie = (1u << (rs.shift & 31)) - 1u, gateTie = (1u << (gateRs.shift & 31)) - 1u;
+        auto rounded = [](int64_t sum, int shift, uint32_t mask) {
+            const uint32_t low = static_cast<uint32_t>(sum);
+            const int32_t q = static_cast<int32_t>(__funnelshift_r(low, static_cast<uint32_t>(static_cast<uint64_t>(sum) >> 32), shift));
+            return (low & mask) == 0 ? q & ~1 : q;
+        };
         for (int chunk = group; chunk < kRows / 16; chunk += kThreads / 128) {
             uint32_t acc[16];
             asm volatile(
@@ -155,32 +164,37 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
                   "=r"(acc[8]), "=r"(acc[9]), "=r"(acc[10]), "=r"(acc[11]), "=r"(acc[12]), "=r"(acc[13]), "=r"(acc[14]), "=r"(acc[15])
                 : "r"(tmem + (static_cast<uint32_t>(32 * q) << 16) + static_cast<uint32_t>(buf * kRows + 16 * chunk)));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            const int row0 = tile * kRows + 16 * chunk;
-            size_t o = static_cast<size_t>(row0) * C + c;
-            auto rowsLoop = [&](auto narrowTag) {
-                constexpr bool kNarrow = decltype(narrowTag)::value;
+            const int row0 = tile * kRows + 16 * chunk, count = real ? p.rows - row0 : 0;
+            planeproj::Column<int16_t> to(p.out, row0, c, C);
+            planeproj::Column<uint8_t> toMask(p.mask, row0, c, C);
+            if (warpNarrow) {
+                auto rows = [&](auto preTag, auto maskTag) {
+                    planeproj::eachRow<16>(count, [&](int j) {
+                        const int32_t code = rounded(static_cast<int64_t>(static_cast<int32_t>(acc[j])) * rs.mult + plus, rs.shift, tie) + zpOut;
+                        const int32_t inside = max(lo, min(code, hi));
+                        if (decltype(maskTag)::value) toMask.put(static_cast<uint8_t>(inside == code ? 1 : 0));
+                        to.put(static_cast<int16_t>(decltype(preTag)::value ? rounded(static_cast<int64_t>(inside) * gateRs.mult + gatePlus, gateRs.shift, gateTie)
+                                                                            : inside));
+                    });
+                };
+                if (p.pre.enabled && p.mask) rows(std::true_type{}, std::true_type{});
+                else if (p.pre.enabled) rows(std::true_type{}, std::false_type{});
+                else if (p.mask) rows(std::false_type{}, std::true_type{});
+                else rows(std::false_type{}, std::false_type{});
+                continue;
+            }
+            const int64_t mulAdd = offset * rs.mult, gateAdd = -static_cast<int64_t>(zpOut) * gateRs.mult;
+#pragma unroll 1
+            for (int j = 0; j < min(count, 16); ++j) {
+                uint8_t keep;
+                int32_t sum = 0;
 #pragma unroll
-                for (int j = 0; j < 16; ++j, o += C) {
-                    const int64_t prod = static_cast<int64_t>(static_cast<int32_t>(acc[j])) * rs.mult + mulAdd;
-                    int32_t rounded;
-                    if constexpr (kNarrow) rounded = gru::rshiftRoundNarrow(prod, rs.shift, remMask, half);
-                    else rounded = narrow ? gru::rshiftRoundNarrow(prod, rs.shift, remMask, half) : gru::rshiftRoundCalled(prod, rs.shift);
-                    uint8_t keep;
-                    int32_t code = gru::clampCode(rounded + zpOut, lo, hi, keep);
-                    if (p.pre.enabled) {
-                        const int64_t prodGate = static_cast<int64_t>(code) * gateRs.mult + gateAdd;
-                        if constexpr (kNarrow) code = gru::rshiftRoundNarrow(prodGate, gateRs.shift, gateMask, gateHalf);
-                        else code = gateNarrow ? gru::rshiftRoundNarrow(prodGate, gateRs.shift, gateMask, gateHalf)
-                                               : gru::rshiftRoundCalled(prodGate, gateRs.shift);
-                    }
-                    if (real && row0 + j < p.rows) {
-                        p.out[o] = static_cast<int16_t>(code);
-                        if (p.mask) p.mask[o] = keep;
-                    }
-                }
-            };
-            if (warpNarrow) rowsLoop(std::true_type{});
-            else rowsLoop(std::false_type{});
+                for (int e = 0; e < 16; ++e) sum = e == j ? static_cast<int32_t>(acc[e]) : sum;
+                int32_t code = gru::clampCode(gru::rshiftRoundCalled(static_cast<int64_t>(sum) * rs.mult + mulAdd, rs.shift) + zpOut, lo, hi, keep);
+                if (p.pre.enabled) code = gru::rshiftRoundCalled(static_cast<int64_t>(code) * gateRs.mult + gateAdd, gateRs.shift);
+                to.put(static_cast<int16_t>(code));
+                if (p.mask) toMask.put(keep);
+            }
         }
         // the MMAs of the item after next overwrite this buffer: order them behind these loads
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
