@@ -278,6 +278,17 @@ size_t sharedBytes(const Cell &cell) {
     return std::max(G::kSharedBytes + cell.sharedBytes(), least);
 }
 
+// CTAs without a cluster that an SM holds: as many as its tensor memory, unless the operator's tables are large (16-bit LSTM layers whose
+// activations need 32 inputs a line have 120 kB of them; an SM has 228 kB, of which a CTA takes 1 kB by itself and less than 512 bytes statically).
+template <class Cell, int HP, int U, int ROWS, int PLANES>
+int residentCtas(const Cell &cell) {
+    const size_t each = sharedBytes<Cell, HP, U, ROWS, PLANES>(cell) + 1024 + 512, all = static_cast<size_t>(currentDevice().smemMax) + 1024;
+    return std::max(1, std::min(Geometry<Cell, HP, U, ROWS, PLANES>::kResident, static_cast<int>(all / each)));
+}
+
+// Most CTAs that launchRows() takes for `rows` rows.
+inline int mostCtas(int rows, int H) { return H <= 128 ? rows : (rows + 3) / 4 * ((H + 63) / 64); }
+
 // `early`: before the kernel in front of it has ended (its prologue runs beside that one's end).
 template <class Cell, int HP, int U, int ROWS, int PLANES>
 void launch(const char *name, const Problem &p, const Cell &cell, bool early, cudaStream_t st) {
@@ -316,7 +327,7 @@ void launchRows(const char *name, const Problem &p, const Cell &cell, bool early
         constexpr int R = decltype(rows)::value;
         using G = Geometry<Cell, HP, U, R, PLANES>;
         const int groups = (p.B + R - 1) / R;
-        if (HP == U) return groups <= (U == 128 && R == 1 ? 1 : G::kResident) * smsPerPass();
+        if (HP == U) return groups <= (U == 128 && R == 1 ? 1 : residentCtas<Cell, HP, U, R, PLANES>(cell)) * smsPerPass();
         // the query counts one CTA of a cluster per SM (33 clusters of four); 36 clusters of eight rows run at the same time all the same
         return groups <= G::kResident * residentClusters(reinterpret_cast<const void *>(unitRecurrence<Cell, HP, U, R, PLANES>), G::kCtas,
                                                          G::kThreads, sharedBytes<Cell, HP, U, R, PLANES>(cell)) / concurrentPasses();

@@ -1,0 +1,40 @@
+"""Which kernels calls of one operator take: the recurrences by steps, rows, width and what is saved, and the rows of a CTA beside large tables."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+import lstm_lib as ll
+from launch_lib import launches
+from rx_met_b200 import _cabi_lstm as L
+from test_lstm_gpu import mod, torch_args
+
+pytestmark = pytest.mark.gpu
+
+
+def lstm_call(T, B, I, H, training, abits=8, wscale=1.0, times=1):
+    """`times`: the batch repeated, beside parameters of one of it."""
+    cfg = L.mixed_config(8, abits)
+    p = ll.problem(T, B, I, H, seed=1, wscale=float(wscale / np.sqrt(H)))
+    _, box = ll.calibrate("orc", cfg, p, np.stack([p["x"] * 0.8]))
+    p.update(x=np.tile(p["x"], (1, times, 1)), h0=np.tile(p["h0"], (times, 1)), c0=np.tile(p["c0"], (times, 1)))
+    m, args = mod(), torch_args(p)
+    bundle = m._params_to_bundle(box)
+    return lambda: m.lstm_forward_quantized(*args, False, bundle, "pedantic", False, training)
+
+
+def launched(call, *names):
+    """Of the kernels with one of these names in theirs: (name, CTAs, shared memory)."""
+    return [(n, ctas, smem) for name, ctas, smem in launches(call) for n in names if n in name]
+
+
+LANES, UNITS, BYTES = "recurrentLanesI8", "unitRecurrence", "recurrentQ"
+
+
+@pytest.mark.parametrize("wscale,ctas", [(1.0, 200), (8.0, 100)])
+def test_rows_of_a_cta_beside_large_activation_tables(wscale, ctas):
+    """Steep activations need 32 inputs a line: 120 kB of tables leave room for one CTA on an SM, and 400 rows run at the same time only with four a
+    CTA instead of two."""
+    (_, got, smem), = launched(lstm_call(2, 8, 5, 64, False, 16, wscale, times=50), UNITS)
+    assert got == ctas and (smem > 114 * 1024) == (wscale > 1)
