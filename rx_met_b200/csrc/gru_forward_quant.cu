@@ -1495,7 +1495,19 @@ void runWide(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaStr
 }
 
 template <class WT, class AT, class LT>
-void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaStream_t st) {
+void runTyped(const ForwardQuantCall &call, const Exec &e, bool onBytes, Workspace &ws, cudaStream_t st) {
+// Whether the recurrence of an 8-bit call is the one with a thread per unit (gru_forward_bytes.cu): direct tables, no switch that asks for
+// another form, and a shape for which it is the faster kernel.
+bool recurrenceOnBytes(const ForwardQuantCall &call, const Exec &e) {
+    if (e.weightClass != CodeClass::I8 || e.actClass != CodeClass::I8 || e.linearClass != CodeClass::I16 || !fastGateMath(e.gate)) return false;
+    for (const char *other : {"RXMET_GRU_FWD_GENERIC", "RXMET_GRU_FWD_MODE", "RXMET_GRU_FWD_BT"})
+        if (std::getenv(other) != nullptr) return false;
+    if (overlapChunks(call.T, static_cast<size_t>(call.T) * call.B, false).size() > 1) return false;
+    const bool masks = call.isTraining && call.masks && (call.masks->weight_hh_linear || call.masks->gate_input);
+    return forwardBytesTakes(call.B, call.H, call.h_q || call.v_q || call.stepFlags || masks);
+}
+
+// onBytes: recurrenceOnBytes() of the call.
     using D = Dot<WT, AT>;
     using WWord = typename D::WWord;
     using AWord = typename D::AWord;
@@ -1798,8 +1810,7 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaSt
                 afterLaunch("recurrentForwardI8");
             };
             if (chunks.size() == 1) {
-                const bool saves = a.hq || a.vq || a.maskHh || a.maskGateIn || a.stepBits;
-                if (mode == 2 && std::getenv("RXMET_GRU_FWD_BT") == nullptr && forwardBytesTakes(B, H, saves)) {
+                if (onBytes) {
                     forwardBytes(ByteRecurrence{T, B, H, hWords, reinterpret_cast<const uint32_t *>(rCodes), compH, biasH, ch.gemmH,
                                                 reinterpret_cast<const int16_t *>(ihCodes), reinterpret_cast<const int8_t *>(a.h0), a.h, a.v, a.hq, a.vq, a.maskHh,
                                                 a.maskGateIn, a.maskGateOut, a.maskH, a.maskIh, a.stepBits, a.poison},
@@ -2149,9 +2160,8 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, 
     const CodeClass w = e.weightClass, a = e.actClass, l = e.linearClass;
     // 16-bit codes, and 8-bit ones beyond 128 units that the recurrence on bytes does not take: the register path below holds R of 256
     // units in spilled registers (H = 192, B = 500, T = 98: 666 us against 298 us over clusters)
-    const bool bytes = w == CodeClass::I8 && a == CodeClass::I8 && l == CodeClass::I16 && fastGateMath(e.gate) && forwardBytesTakes(call.B, call.H, true) &&
-                       std::getenv("RXMET_GRU_FWD_MODE") == nullptr && std::getenv("RXMET_GRU_FWD_BT") == nullptr &&
-                       iproj::eligible(3 * call.H, call.H, padTo(call.I, 4) / 4, nullptr, nullptr, nullptr);
+    const bool onBytes = recurrenceOnBytes(call, e);
+    const bool bytes = onBytes && iproj::eligible(3 * call.H, call.H, padTo(call.I, 4) / 4, nullptr, nullptr, nullptr);
     if (forwardWideTakes(e, call.I, call.H) &&
         (a == CodeClass::I16 || (call.H > 128 && !call.stepFlags && !bytes && forwardWideClusterTakes(e, call.B, call.H)))) {
         runWide(call, e, ws, st);
@@ -2159,13 +2169,13 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, 
     }
     if (forwardPhase() == ForwardPhase::Recurrence) return;   // not split: done by the call before
     if (l == CodeClass::I32 || w == CodeClass::I32 || a == CodeClass::I32) {
-        runTyped<int32_t, int32_t, int32_t>(call, e, ws, st);
+        runTyped<int32_t, int32_t, int32_t>(call, e, onBytes, ws, st);
     } else if (w == CodeClass::I8 && a == CodeClass::I8) {
-        runTyped<int8_t, int8_t, int16_t>(call, e, ws, st);
+        runTyped<int8_t, int8_t, int16_t>(call, e, onBytes, ws, st);
     } else if (w == CodeClass::I8) {
-        runTyped<int8_t, int16_t, int16_t>(call, e, ws, st);
+        runTyped<int8_t, int16_t, int16_t>(call, e, onBytes, ws, st);
     } else {
-        runTyped<int16_t, int16_t, int16_t>(call, e, ws, st);
+        runTyped<int16_t, int16_t, int16_t>(call, e, onBytes, ws, st);
     }
 }
 

@@ -7,10 +7,26 @@ import torch
 
 import lstm_lib as ll
 from launch_lib import launches
-from rx_met_b200 import _cabi_lstm as L
+from rx_met_b200 import _cabi, _cabi_lstm as L
+from rx_met_b200 import gru_interface_binding as gru
 from test_lstm_gpu import mod, torch_args
 
 pytestmark = pytest.mark.gpu
+
+
+def gru_call(T, B, I, H, training, bits=8):
+    gen = torch.Generator().manual_seed(T + B + H)
+    rand = lambda *shape: (torch.rand(shape, generator=gen) - 0.5).cuda()  # noqa: E731
+    W, R, bw, br, x = rand(I, 3 * H), rand(H, 3 * H) * 0.2, rand(3 * H), rand(3 * H), rand(T, B, I)
+    ranges = gru.GRUQuantizationRanges(H)
+    gru.forward_calibrate(True, T, B, I, H, W, R, bw, br, x, None, "minmax", None, ranges)
+    cfg = gru.OperatorQuantConfig()
+    for name in _cabi.OP_NAMES:
+        if name not in ("W", "R", "bw", "br"):
+            setattr(cfg, f"{name}_", bits)
+            setattr(cfg, f"{name}_symmetric_", False)
+    params = gru.calculate_gru_quantitative_parameters(ranges, cfg)
+    return lambda: gru.forward_quant_int_storage(training, T, B, I, H, W, R, bw, br, x, None, params)
 
 
 def lstm_call(T, B, I, H, training, abits=8, wscale=1.0, times=1):
@@ -30,6 +46,15 @@ def launched(call, *names):
 
 
 LANES, UNITS, BYTES = "recurrentLanesI8", "unitRecurrence", "recurrentQ"
+
+
+@pytest.mark.parametrize("chunks,cell", [(None, "GruByteCell"), ("15,35,50", "GruUnitCell")])
+def test_8bit_gru_beyond_128_units_in_time_chunks(monkeypatch, chunks, cell):
+    """Asked for in time chunks, which the recurrence on bytes does not know: over clusters on byte planes, not in registers that spill."""
+    call = gru_call(20, 16, 16, 192, False)
+    if chunks:
+        monkeypatch.setenv("RXMET_GRU_FWD_CHUNKS", chunks)
+    assert [n for n, _, _ in launched(call, "GruByteCell", "GruUnitCell", "recurrentForwardI8")] == [cell]
 
 
 @pytest.mark.parametrize("wscale,ctas", [(1.0, 200), (8.0, 100)])
