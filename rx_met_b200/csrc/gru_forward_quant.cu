@@ -1494,8 +1494,6 @@ void runWide(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaStr
     forwardWide(wc, e, st);
 }
 
-template <class WT, class AT, class LT>
-void runTyped(const ForwardQuantCall &call, const Exec &e, bool onBytes, Workspace &ws, cudaStream_t st) {
 // Whether the recurrence of an 8-bit call is the one with a thread per unit (gru_forward_bytes.cu): direct tables, no switch that asks for
 // another form, and a shape for which it is the faster kernel.
 bool recurrenceOnBytes(const ForwardQuantCall &call, const Exec &e) {
@@ -1508,6 +1506,8 @@ bool recurrenceOnBytes(const ForwardQuantCall &call, const Exec &e) {
 }
 
 // onBytes: recurrenceOnBytes() of the call.
+template <class WT, class AT, class LT>
+void runTyped(const ForwardQuantCall &call, const Exec &e, bool onBytes, Workspace &ws, cudaStream_t st) {
     using D = Dot<WT, AT>;
     using WWord = typename D::WWord;
     using AWord = typename D::AWord;
