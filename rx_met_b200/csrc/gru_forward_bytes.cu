@@ -230,9 +230,7 @@ void launchFor(const ByteRecurrence &r, const ByteScalars &s, const GateExec &g,
         cell.s = s;
         cell.luts[0] = g.lut_update; cell.luts[1] = g.lut_reset; cell.luts[2] = g.lut_new;
         cell.r = r;
-        // not early: the projection lets its dependents start with its first blocks, and CTAs that find room among those lie unevenly
-        // on the SMs (training step, H = 64, 64 rows: 203 against 171 us)
-        unitrec::launchRows<Cell, HP, 1>("recurrentForward", planerec::Problem{r.T, r.B, r.H, nullptr}, cell, false, st);
+        unitrec::launchRows<Cell, HP, 1>("recurrentForward", planerec::Problem{r.T, r.B, r.H, nullptr}, cell, true, st);
     };
     if (r.H == HP) run(std::integral_constant<int, HP>{});
     else run(std::integral_constant<int, 0>{});

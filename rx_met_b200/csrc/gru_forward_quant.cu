@@ -35,6 +35,7 @@
 #include "gru_forward_wide.h"
 #include "input_proj_umma.h"
 #include "plane_proj_umma.cuh"
+#include "unit_recurrence_umma.cuh"
 
 namespace rxmet {
 namespace gru {
@@ -508,13 +509,13 @@ __global__ void __launch_bounds__(512)
 inputLinearI8(const int32_t *__restrict__ x, int rows, int kWords, int channels, const int32_t *__restrict__ w,
               const int64_t *__restrict__ comp, const int64_t *__restrict__ biasAcc, const Rescale *__restrict__ rescale,
               int32_t zpOut, int32_t lo, int32_t hi, int16_t *__restrict__ out, uint8_t *__restrict__ mask,
-              const PreRescale pre) {
+              const PreRescale pre, bool late) {   // late: iproj::Problem::dependents
     constexpr int kRowWords = KW4 * 4;
     __shared__ __align__(16) int32_t xs[2][kI8Rows][kRowWords];
     const int tid = threadIdx.x, c = tid;
     const bool live = c < channels;
     waitForPredecessor();
-    letDependentsStart();
+    if (!late) letDependentsStart();
     int32_t wreg[kRowWords];
 #pragma unroll
     for (int kk = 0; kk < kRowWords; ++kk) wreg[kk] = (live && kk < kWords) ? w[static_cast<size_t>(kk) * channels + c] : 0;
@@ -595,6 +596,7 @@ inputLinearI8(const int32_t *__restrict__ x, int rows, int kWords, int channels,
         __syncthreads();
         buf ^= 1;
     }
+    if (late) letDependentsStart();
 }
 
 // ---- 4. the recurrence: one launch for all steps ----------------------------
@@ -1648,16 +1650,23 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, bool onBytes, Workspa
 
     // 3. input projection, all steps
     bool tensorProjection = false;
+    // CTAs of the recurrence behind the projection (iproj::Problem::dependents); lanes of short sequences and few rows gain by the early start whatever
+    // SMs they share
+    const int dependents = onBytes ? unitrec::mostCtas(B, H) : lanesPath && T >= 32 && rows >= 6000 ? (B + btI8 - 1) / btI8 : 0;
     std::vector<int> chunks{T};   // time chunks of the overlapped pipeline (one = none)
     {
         const int block = std::min(padTo(C, 32), 512);
         const int kw4 = (iWords + 3) / 4;
         bool specialised = false;
         if constexpr (kI8) {
-            // channel counts that leave the last tile partly empty: where the register kernel below does not go, or with many rows
-            // (PARTIALNUMBERS)
+            // The tensor cores, or the kernel with the weights in registers: the first costs the same for a partly empty channel tile as for a full one and
+            // prepares itself longer, the second grows with the inputs.  With the recurrence behind it, T 10, 64,000 rows, registers -> tensor cores: 40
+            // inputs, C 24 39 -> 43 us, C 48 53 -> 48, C 144 110 -> 97; 16 inputs, C 48 38 -> 42, C 144 83 -> 87, C 192 83 -> 79, C 300 141 -> 135; 8000 rows
+            // of 40 inputs, C 192 27 -> 27, C 360 37 -> 37.
             const bool registerProjection = C <= 512 && kw4 <= 4 && block >= kI8Rows * kw4 * 4;
-            if (iproj::eligible(C, H, iWords, xCodes, ihCodes, mk.weight_ih_linear) && (C % 128 == 0 || !registerProjection || rows >= 8192) &&
+            const bool filled = 8 * C >= 5 * padTo(C, 128) || (kw4 > 2 && C >= 48);
+            if (iproj::eligible(C, H, iWords, xCodes, ihCodes, mk.weight_ih_linear) &&
+                (C % 128 == 0 || !registerProjection || (filled && rows >= 8192)) &&
                 std::getenv("RXMET_GRU_FWD_GENERIC") == nullptr) {
                 // tcgen05 kind::i8 GEMM with the fused epilogue
                 specialised = true;
@@ -1671,7 +1680,7 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, bool onBytes, Workspa
                     pj.zpOut = g.zp[RXMET_GRU_WEIGHT_IH_LINEAR]; pj.lo = g.qlo[RXMET_GRU_WEIGHT_IH_LINEAR];
                     pj.hi = g.qhi[RXMET_GRU_WEIGHT_IH_LINEAR];
                     pj.pre = pre; pj.out = reinterpret_cast<int16_t *>(ihCodes) + r0 * C;
-                    pj.mask = mk.weight_ih_linear ? mk.weight_ih_linear + r0 * C : nullptr; pj.status = projStatus;
+                    pj.mask = mk.weight_ih_linear ? mk.weight_ih_linear + r0 * C : nullptr; pj.status = projStatus; pj.dependents = dependents;
                     iproj::launch(pj, sms, s);
                 };
                 // Cut into time chunks, the projection of chunk i + 1 runs on the library's second stream under the
@@ -1708,7 +1717,7 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, bool onBytes, Workspa
         const int grid = std::max(1, std::min(blocks, sms * std::max(1, perSm)));                                          \
         launchDependent(inputLinearI8<N>, grid, block, 0, st, reinterpret_cast<const int32_t *>(xCodes), static_cast<int>(rows), \
                         iWords, C, reinterpret_cast<const int32_t *>(wCodes), compX, biasX, ch.gemmX, zp, qlo, qhi,        \
-                        reinterpret_cast<int16_t *>(ihCodes), mk.weight_ih_linear, pre);                                    \
+                        reinterpret_cast<int16_t *>(ihCodes), mk.weight_ih_linear, pre, dependents > 0 && grid + dependents > sms); \
     } break;
                 switch (kw4) {
                     RXMET_IL_CASE(1) RXMET_IL_CASE(2) RXMET_IL_CASE(3) RXMET_IL_CASE(4)

@@ -30,6 +30,7 @@
 #include "gru_device.cuh"
 #include "gru_forward_wide.h"
 #include "plane_proj_umma.cuh"
+#include "unit_recurrence_umma.cuh"
 
 namespace rxmet {
 namespace gru {
@@ -417,6 +418,7 @@ void forwardWide(const WideCall &call, const Exec &e, cudaStream_t st) {
     const WideOperands &l = call.operands;
     const int kI = l.kI, kH = l.kH;
     const int sms = currentDevice().sms;
+    const bool units = forwardWideClusterTakes(e, B, H);   // the recurrence with a thread per unit
 
     // Input projection: the tcgen05 kind::i8 kernel when the operands fit shared memory, else the dp4a kernel.
     const bool tensorProjection = l.wTiles != nullptr;
@@ -429,7 +431,7 @@ void forwardWide(const WideCall &call, const Exec &e, cudaStream_t st) {
         epi.addend = l.addX; epi.rescale = call.gemmX;
         epi.zpOut = g.zp[RXMET_GRU_WEIGHT_IH_LINEAR]; epi.lo = g.qlo[RXMET_GRU_WEIGHT_IH_LINEAR]; epi.hi = g.qhi[RXMET_GRU_WEIGHT_IH_LINEAR];
         epi.out = l.ihCodes; epi.mask = call.maskIh; epi.C = C;
-        planeproj::launch<2>("inputLinear", pp, epi, smsPerPass(), st);
+        planeproj::launch<2>("inputLinear", pp, epi, smsPerPass(), unitrec::mostCtas(B, H), st);
     } else {
         InputArgs a{};
         a.rows = static_cast<int>(rows); a.C = C; a.kWords = kI;
@@ -461,7 +463,7 @@ void forwardWide(const WideCall &call, const Exec &e, cudaStream_t st) {
         a.maskHh = call.maskHh; a.maskGateIn = call.maskGateIn; a.maskGateOut = call.maskGateOut; a.maskH = call.maskH;
         a.poison = tensorProjection ? l.projStatus : nullptr;
         a.maskIh = call.maskIh; a.stepBits = call.stepBits;
-        if (forwardWideClusterTakes(e, B, H)) {
+        if (units) {
             forwardWideCluster(a, e, st);
             return;
         }

@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
         reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     waitForPredecessor();
-    letDependentsStart();
+    if (!p.late) letDependentsStart();
     // weight word (kw, c) = codes k = 4 kw .. 4 kw + 3 of channel c -> four consecutive bytes of row c
     for (int i = tid; i < kWords * C; i += kThreads) {
         const int kw = i / C, c = i - kw * C;
@@ -224,6 +224,7 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (p.late) letDependentsStart();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
     if (tid == 0 && failed && p.status) atomicExch(p.status, 1);
 }
@@ -245,8 +246,10 @@ void launch(const Problem &problem, int sms, cudaStream_t st) {
     const size_t smem = sharedBytes(prob.C, prob.kPad);
     ensureDynamicSmem(reinterpret_cast<const void *>(inputProjUmma), smem);
     const int items = ((prob.rows + kRows - 1) / kRows) * (paddedC(prob.C) / kTileM);
+    const int grid = std::max(1, std::min(items, 2 * sms));
+    prob.late = prob.dependents > 0 && grid + prob.dependents > sms;
     KernelTimer timer__("inputLinear", st);
-    launchDependent(inputProjUmma, std::max(1, std::min(items, 2 * sms)), kThreads, smem, st, prob);
+    launchDependent(inputProjUmma, grid, kThreads, smem, st, prob);
 }
 
 }  // namespace iproj

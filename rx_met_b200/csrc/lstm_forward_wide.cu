@@ -1034,6 +1034,7 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
     const rxmet_lstm_trace noTrace{};
     const rxmet_lstm_trace &ck = call.checkpoints ? *call.checkpoints : noTrace;
     const int sms = currentDevice().sms;
+    const bool units = forwardInUnits(e, B, I, H);
     // Input projection: the tcgen05 kind::i8 kernel when the operands fit shared memory
     // (RXMET_IPROJ_SIMT turns it off), else the dp4a kernel.
     const int kPadIh = planeproj::paddedK(kIh);
@@ -1050,7 +1051,7 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
         auto launchTensor = [&](auto epi, auto planeCount) {
             epi.addend = l.addIh; epi.fields = l.channel; epi.s = s; epi.H = H; epi.I = I; epi.lhs = l.lhs;
             epi.linear = ck.weight_ih_linear; epi.linearClamped = ck.weight_ih_linear_clamped;
-            planeproj::launch<decltype(planeCount)::value>("lstmInputLinearWide", pp, epi, smsPerPass(), st);
+            planeproj::launch<decltype(planeCount)::value>("lstmInputLinearWide", pp, epi, smsPerPass(), unitrec::mostCtas(B, H), st);
         };
         if (planes == 2) launchTensor(WidePlaneEpilogue<2>{}, std::integral_constant<int, 2>{});
         else launchTensor(WidePlaneEpilogue<1>{}, std::integral_constant<int, 1>{});
@@ -1082,7 +1083,6 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
         afterLaunch("lstmInputLinearWide");
     }
     // Recurrence over clusters wherever the activation tables have a compact form and the grids are the usual ones.
-    const bool units = forwardInUnits(e, B, I, H);
     if (units || (planes == 2 && H > 128 && clusterTakes(e))) {
         const planerec::Problem problem{T, B, H, l.h0};
         const void *const kept[] = {ck.weight_hh_linear, ck.weight_hh_linear_clamped, ck.gate_inputs, ck.gate_inputs_clamped, ck.gate_outputs,

@@ -57,6 +57,13 @@ def test_8bit_gru_beyond_128_units_in_time_chunks(monkeypatch, chunks, cell):
     assert [n for n, _, _ in launched(call, "GruByteCell", "GruUnitCell", "recurrentForwardI8")] == [cell]
 
 
+# partly empty channel tiles: the tensor cores with many rows that fill them or have many inputs
+@pytest.mark.parametrize("T,B,I,H,expected", [(98, 80, 40, 64, "inputLinearI8"), (98, 128, 40, 64, "inputProjUmma"), (98, 128, 8, 16, "inputLinearI8"),
+                                              (98, 128, 8, 48, "inputLinearI8"), (98, 128, 40, 16, "inputProjUmma"), (2, 3, 8, 128, "inputProjUmma")])
+def test_8bit_gru_projection(T, B, I, H, expected):
+    assert [n for n, _, _ in launched(gru_call(T, B, I, H, False), "inputLinearI8", "inputProjUmma")] == [expected]
+
+
 @pytest.mark.parametrize("wscale,ctas", [(1.0, 200), (8.0, 100)])
 def test_rows_of_a_cta_beside_large_activation_tables(wscale, ctas):
     """Steep activations need 32 inputs a line: 120 kB of tables leave room for one CTA on an SM, and 400 rows run at the same time only with four a

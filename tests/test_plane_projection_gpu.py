@@ -22,3 +22,9 @@ def test_gru_projection(T, B, I, H):
 @pytest.mark.parametrize("T,B,I,H", [(1, 1, 1, 32), (2, 64, 256, 33), (1, 129, 255, 512), (3, 13000, 4, 3)])
 def test_lstm_projection(T, B, I, H, abits):
     lstm_forward_matches(T, B, I, H, 4, abits, L.PER_CHANNEL, True, True)
+
+
+# 8-bit codes (input_proj_umma.cu): many rows on channel counts that leave the last tile partly empty
+@pytest.mark.parametrize("T,B,I,H", [(21, 400, 13, 37), (12, 700, 40, 20), (9, 1000, 5, 85), (3, 2800, 64, 100)])
+def test_8bit_gru_projection_of_partly_empty_tiles(T, B, I, H):
+    gru_forward_matches(gl, "w8a8", (T, B, I, H))
