@@ -245,13 +245,27 @@ void launchFor(const ByteRecurrence &r, const ByteScalars &s, const GateExec &g,
 
 }  // namespace
 
-// Few rows of narrow layers stay in lanes, whose chain is the shorter one there.  Passes of T = 100: inference, H = 64: 1 row 42 against 45 us, 256
-// rows 47 against 50, 700 rows 146 against 133; 40 units, 700 rows 91 against 105; training, H = 64: 16 rows 162 against 176, 45 rows 199
-// against 184; 32 units, 64 rows 180 against 185, 128 rows 209 against 201.
-bool forwardBytesTakes(int B, int H, bool saves) {
+// Against the lanes: a step is shorter here, but there is more to prepare, and a layer of at most 64 units is padded to that.  Passes in us,
+// lanes -> here:
+//   inference beyond 64 units: H 65, 1 row T 40 27 -> 28, T 98 51 -> 47; 64 rows T 40 31 -> 33, T 64 40 -> 41, T 98 56 -> 55; H 128, 1 row T 8 17 -> 19, T 16
+//     21 -> 21, T 40 36 -> 31; 128 rows T 16 23 -> 25, T 24 31 -> 31; 200 rows T 20, H 80 35 -> 27; 600 rows T 10, H 65 35 -> 33, H 128 47 -> 37
+//   inference of 49 to 64 units: 300 rows T 10 19 -> 23, T 20 33 -> 29; 1200 rows T 40 89 -> 84
+//   saving, beyond 64 units: H 65, 64 rows T 4 74 -> 79, T 12 86 -> 86, T 16 88 -> 86; H 128, 300 rows T 10 105 -> 96
+//   saving, up to 64 units: 64, 64 rows T 40 84 -> 86, T 64 117 -> 105, 100 rows T 40 93 -> 87; 32, 128 rows T 40 103 -> 106, T 98 181 -> 161; 16, 300 rows
+//     T 40 133 -> 123, 600 rows T 40 178 -> 169, 1200 rows 326 -> 334; 48, 1200 rows 369 -> 380; 64, 1200 rows 249 -> 232
+bool forwardBytesTakes(int T, int B, int H, bool saves) {
     if (H > 256 || 4 * static_cast<uint64_t>(H) * B >= (uint64_t{1} << 32)) return false;
-    if (H > 64) return true;
-    return saves ? static_cast<int64_t>(B) * H > 2048 : H > 48 && B > 2 * currentDevice().sms;
+    if (H > 128) return true;
+    const int sms = currentDevice().sms;
+    const int64_t rows = static_cast<int64_t>(T) * B;
+    if (saves) {
+        if (H > 64) return T >= 16 || (H > 112 && B > 2 * sms);
+        return static_cast<int64_t>(B) * H > 2048 && rows * H >= (B > 2 * sms ? 2 : 3) << 16 && (H == 64 || B <= 5 * sms);
+    }
+    if (H <= 64) return H > 48 && B > 2 * sms && (T >= 16 || B > 5 * sms);
+    if (B > sms) return T >= 16 || B > 4 * sms;
+    const bool crowded = (rows + 15) / 16 + B > sms;   // no SMs of their own beside the projection: nothing is prepared under it
+    return T >= (H > 96 ? (crowded ? 24 : 16) : (crowded ? 64 : 48));
 }
 
 void forwardBytes(const ByteRecurrence &r, const GateExec &g, cudaStream_t st) {

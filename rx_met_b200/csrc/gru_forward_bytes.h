@@ -26,8 +26,8 @@ struct ByteRecurrence {
     uint16_t *stepBits;        // optional [T][B][H]: the 13 flags of an element packed
     const int *poison;         // status word of the tensor-core projection: non-zero turns the hidden outputs into NaN
 };
-// Whether it is the faster kernel for the shape (offsets inside a step have to fit 32 bits); saves: codes or flags are asked for.
-bool forwardBytesTakes(int B, int H, bool saves);
+// Whether it takes the shape (offsets inside a step have to fit 32 bits) and is the faster kernel for it; saves: codes or flags are asked for.
+bool forwardBytesTakes(int T, int B, int H, bool saves);
 void forwardBytes(const ByteRecurrence &r, const GateExec &g, cudaStream_t stream);
 
 }  // namespace gru

@@ -1504,7 +1504,7 @@ bool recurrenceOnBytes(const ForwardQuantCall &call, const Exec &e) {
         if (std::getenv(other) != nullptr) return false;
     if (overlapChunks(call.T, static_cast<size_t>(call.T) * call.B, false).size() > 1) return false;
     const bool masks = call.isTraining && call.masks && (call.masks->weight_hh_linear || call.masks->gate_input);
-    return forwardBytesTakes(call.B, call.H, call.h_q || call.v_q || call.stepFlags || masks);
+    return forwardBytesTakes(call.T, call.B, call.H, call.h_q || call.v_q || call.stepFlags || masks);
 }
 
 // onBytes: recurrenceOnBytes() of the call.

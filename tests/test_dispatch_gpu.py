@@ -48,6 +48,15 @@ def launched(call, *names):
 LANES, UNITS, BYTES = "recurrentLanesI8", "unitRecurrence", "recurrentQ"
 
 
+# few steps or few rows: lanes, whose kernel has less to prepare
+@pytest.mark.parametrize("T,B,H,training,expected", [
+    (1, 1, 128, False, LANES), (4, 32, 80, False, LANES), (40, 1, 65, False, LANES), (64, 1, 65, False, UNITS), (20, 128, 128, False, LANES),
+    (40, 128, 128, False, UNITS), (20, 200, 70, False, UNITS), (4, 300, 60, False, LANES), (20, 300, 60, False, UNITS), (98, 32, 64, False, LANES),
+    (4, 64, 128, True, LANES), (16, 8, 70, True, UNITS), (4, 128, 64, True, LANES), (40, 128, 64, True, UNITS), (40, 900, 16, True, LANES)])
+def test_8bit_gru_recurrence(T, B, H, training, expected):
+    assert [n for n, _, _ in launched(gru_call(T, B, 8, H, training), LANES, UNITS)] == [expected]
+
+
 @pytest.mark.parametrize("chunks,cell", [(None, "GruByteCell"), ("15,35,50", "GruUnitCell")])
 def test_8bit_gru_beyond_128_units_in_time_chunks(monkeypatch, chunks, cell):
     """Asked for in time chunks, which the recurrence on bytes does not know: over clusters on byte planes, not in registers that spill."""

@@ -1,4 +1,4 @@
-"""The recurrences with a thread per hidden unit (QuantLSTM up to 128 units, QuantGRU W8 / A16 up to 256) and over clusters: the edges of widths, of rows per CTA
+"""The recurrences with a thread per hidden unit (QuantLSTM up to 128 units, QuantGRU up to 256, 8 and 16 bits) and over clusters: the edges of widths, of rows per CTA
 or cluster and of step counts, every form of what a forward saves, against the CPU checkers."""
 from __future__ import annotations
 
@@ -12,7 +12,8 @@ import gpu_lib as gl
 import lstm_lib as ll
 import oracle_lib as ol
 from rx_met_b200 import _cabi, _cabi_lstm as L
-from test_gru_gpu import CONFIGS, calibrated, test_forward_quant_matches_restatement as gru_forward_matches
+from test_gru_gpu import (CONFIGS, calibrated, test_forward_quant_matches_restatement as gru_forward_matches,
+                          test_packed_step_flags_equal_the_byte_masks as packed_flags_match)
 from test_lstm_gpu import dev, mod, torch_args
 from test_lstm_wide_gpu import setup, test_wide_forward_is_bit_exact as lstm_forward_matches
 
@@ -58,10 +59,23 @@ def test_gru_units(T, B, I, H):
     gru_forward_matches(gl, "a16", (T, B, I, H))
 
 
-@pytest.mark.parametrize("T,B,I,H", [(3, 5, 6, 64), (2, 150, 4, 100), (3, 9, 5, 200)])
-def test_gru_units_save_what_is_asked_for(T, B, I, H):
+# one plane of signed codes: 64 units: 2, 4, 8 rows of a CTA; 128: 1, 2, 4; clusters beyond: 4, 8
+@pytest.mark.parametrize("T,B,I,H", [(64, 100, 4, 33), (16, 700, 3, 50), (40, 101, 5, 64), (16, 1185, 3, 64), (64, 1, 6, 65), (16, 149, 6, 65), (16, 593, 4, 128),
+                                     (17, 601, 3, 100), (2, 131, 5, 129), (2, 500, 4, 129), (2, 421, 5, 192), (3, 265, 7, 193), (5, 3, 5, 256), (2, 301, 4, 255)])
+def test_8bit_gru_units(T, B, I, H):
+    gru_forward_matches(gl, "w8a8", (T, B, I, H))
+
+
+@pytest.mark.parametrize("shape", [(17, 9, 40, 128), (16, 601, 8, 64), (40, 130, 8, 64)], ids=lambda s: "x".join(map(str, s)))
+def test_8bit_gru_units_pack_their_flags(monkeypatch, shape):
+    packed_flags_match(monkeypatch, shape)
+
+
+@pytest.mark.parametrize("cfg_name,T,B,I,H", [("a16", 3, 5, 6, 64), ("a16", 2, 150, 4, 100), ("a16", 3, 9, 5, 200), ("w8a8", 40, 130, 6, 64), ("w8a8", 64, 9, 4, 100),
+                                              ("w8a8", 16, 300, 4, 60), ("w8a8", 3, 9, 5, 200)])
+def test_gru_units_save_what_is_asked_for(cfg_name, T, B, I, H):
     from rx_met_b200 import gru_interface_binding as m
-    prob, params = calibrated((T, B, I, H), seed=T + B + H, cfg=ol.make_config(**CONFIGS["a16"]), with_h0=True)
+    prob, params = calibrated((T, B, I, H), seed=T + B + H, cfg=ol.make_config(**CONFIGS[cfg_name]), with_h0=True)
     want = ol.forward_quant("orc", *prob, params, training=True)
     p = m.GRUQuantParams._from_c(params.c, [params.chan["scale_" + n].tolist() for n in ("W", "R", "bw", "br")])
     for training in (False, True):
