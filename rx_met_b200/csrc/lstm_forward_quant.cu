@@ -443,7 +443,7 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, 
     // I, H <= 128 (weight rows live in registers); everything else goes to the wide kernels.
     bool bytePath = e.exactAccumulators && H <= 128 && I <= 128 && !e.tables.empty();
     for (int op = 0; op < kOps; ++op) bytePath = bytePath && (static_cast<int64_t>(s.hi[op]) - s.lo[op] <= 255);
-    if (!bytePath || forwardInUnits(e, B, I, H)) {
+    if (!bytePath || (unitsFasterThanBytes(T, B, H, call.checkpoints != nullptr) && forwardInUnits(e, B, I, H))) {
         forwardQuantWide(call, e, workspace, workspaceBytes, st);
         return;
     }

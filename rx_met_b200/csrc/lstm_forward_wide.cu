@@ -955,6 +955,17 @@ bool forwardInUnits(const Exec &e, int B, int I, int H) {
            forwardQuantWideTakes(e, I, H, nullptr) && clusterTakes(e);
 }
 
+// More is prepared for the units (planes, tiles, six launches), their steps are shorter.  Passes in us, byte codes -> units:
+//   inference: H 128, 1 row T 8 31 -> 39, T 24 46 -> 45, T 40 57 -> 49; H 48, 128 rows T 24 41 -> 41, T 40 52 -> 47; H 32, 8 rows T 40 42 -> 44, T 98
+//     69 -> 65; H 8, 1200 rows T 40 65 -> 66, 2400 83 -> 108; H 16, 1200 rows T 98 138 -> 121, 2400 T 40 93 -> 108; H 24, 2400 111 -> 112
+//   with checkpoints: H 128, 1 row T 12 106 -> 109, T 16 113 -> 114, T 24 127 -> 120; H 65, 128 rows T 16 142 -> 148, T 24 161 -> 158; H 32, 64 rows T 40
+//     109 -> 118, T 98 165 -> 169, T 200 272 -> 264; 256 rows T 40 128 -> 131, T 98 213 -> 202; 1200 rows T 200, H 32 770 -> 880, H 40 2046 -> 2063, H 48 2265 -> 2100
+bool unitsFasterThanBytes(int T, int B, int H, bool saves) {
+    const int sms = currentDevice().sms;
+    if (saves) return T >= (H > 32 ? 24 : B > sms ? 64 : 128) && (H >= 48 || B <= 5 * sms);
+    return T >= (H <= 32 ? 48 : 32) && (H > 16 || B <= 10 * sms);
+}
+
 bool forwardQuantWideTakes(const Exec &e, int I, int H, const char **why) {
     const char *reason = nullptr;
     if (!e.weightsFitBytes) reason = "weight grids wider than 8 bits are not built";

@@ -45,6 +45,8 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &exec, void *workspac
 bool forwardQuantWideTakes(const Exec &exec, int I, int H, const char **why);
 // Up to 128 units: the recurrence with a thread per unit (unit_recurrence_umma.cuh), 8-bit grids included.
 bool forwardInUnits(const Exec &exec, int B, int I, int H);
+// Whether that is also faster than the byte-code kernels (lstm_forward_quant.cu); saves: checkpoints are asked for.
+bool unitsFasterThanBytes(int T, int B, int H, bool saves);
 size_t forwardQuantWideWorkspaceBytes(int T, int B, int I, int H);
 void forwardQuantWide(const ForwardQuantCall &call, const Exec &exec, void *workspace, size_t workspaceBytes,
                       cudaStream_t stream);

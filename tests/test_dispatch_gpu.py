@@ -73,6 +73,13 @@ def test_8bit_gru_projection(T, B, I, H, expected):
     assert [n for n, _, _ in launched(gru_call(T, B, I, H, False), "inputLinearI8", "inputProjUmma")] == [expected]
 
 
+@pytest.mark.parametrize("T,B,H,training,expected", [
+    (1, 1, 128, False, BYTES), (40, 1, 128, False, UNITS), (40, 16, 32, False, BYTES), (64, 16, 32, False, UNITS), (50, 1600, 12, False, BYTES),
+    (8, 16, 100, True, BYTES), (40, 16, 100, True, UNITS), (64, 16, 32, True, BYTES), (130, 16, 32, True, UNITS), (40, 900, 40, True, BYTES)])
+def test_8bit_lstm_recurrence(T, B, H, training, expected):
+    assert [n for n, _, _ in launched(lstm_call(T, B, 5, H, training), BYTES, UNITS)] == [expected]
+
+
 @pytest.mark.parametrize("wscale,ctas", [(1.0, 200), (8.0, 100)])
 def test_rows_of_a_cta_beside_large_activation_tables(wscale, ctas):
     """Steep activations need 32 inputs a line: 120 kB of tables leave room for one CTA on an SM, and 400 rows run at the same time only with four a

@@ -287,10 +287,10 @@ def test_histogram_calibration_session_matches_reference(method, state):
     assert torch.isfinite(out[0]).all()
 
 
-@pytest.mark.parametrize("T,B,I,H", [(1, 1, 8, 1), (3, 149, 5, 65), (4, 297, 12, 128), (2, 150, 40, 64), (5, 3, 9, 63)])
-def test_inference_in_lanes_equals_the_training_forward(T, B, I, H):
-    """8-bit inference runs another recurrence than the forward with checkpoints: the same outputs bit for bit, one, two and
-    four rows per CTA with a partly empty last CTA, widths at the edges of its tiles."""
+@pytest.mark.parametrize("T,B,I,H", [(1, 1, 8, 1), (3, 149, 5, 65), (4, 297, 12, 128), (2, 150, 40, 64), (5, 3, 9, 63), (28, 149, 5, 65), (64, 17, 9, 32), (64, 5, 8, 24)])
+def test_inference_equals_the_training_forward(T, B, I, H):
+    """The same outputs bit for bit with and without checkpoints, which take the byte-code kernels up to other numbers of steps: both on those, inference
+    on those and training in units (28 steps), the other way round (64 steps of at most 32 units).  Against the checkers: test_unit_recurrence_gpu.py."""
     import torch
     from rx_met_b200 import _quant_lstm as m
     cfg = L.default_config()

@@ -27,10 +27,16 @@ def test_lstm_units(T, B, I, H, abits):
     lstm_forward_matches(T, B, I, H, 8, abits, L.PER_CHANNEL, True, True)
 
 
+# the same on one byte plane, which takes its calls from 24 (up to 32 units 128) steps on
+@pytest.mark.parametrize("T,B,I,H", [(32, 149, 5, 65), (33, 148, 7, 128), (32, 297, 6, 100), (32, 593, 6, 127), (32, 1185, 4, 64), (33, 593, 5, 63), (128, 3, 4, 20)])
+def test_lstm_units_on_one_plane(T, B, I, H):
+    lstm_forward_matches(T, B, I, H, 8, 8, L.PER_CHANNEL, True, True)
+
+
 @pytest.mark.parametrize("keep", [("gate_outputs", "cell_states_clamped"), ("weight_hh_linear_clamped", "hidden_outputs"), ("weight_ih_linear",)])
 @pytest.mark.parametrize("abits", [8, 16])
 def test_lstm_units_save_what_is_asked_for(abits, keep):
-    T, B, I, H = 3, 5, 7, 100
+    T, B, I, H = 25, 5, 7, 100
     p, box, _ = setup(T, B, I, H, 8, abits, L.PER_CHANNEL, True, True)
     q = ll.quantize_masters("orc", p, box)
     _, _, _, want, want_mask = ll.forward_quantized_masked(box, T, B, q, exact_sums=True)
