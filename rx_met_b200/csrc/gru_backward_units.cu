@@ -30,11 +30,16 @@ struct GruReverseCell {
     struct Out {
         float p[3], q[3];
     };
-    __device__ __forceinline__ uint4 weights8(int m, int gate, int unit) const {
-        const int4 *src = reinterpret_cast<const int4 *>(Rq + static_cast<size_t>(m) * 3 * a.H + gate * a.H + unit);
-        const int4 x = __ldg(src), y = __ldg(src + 1);
-        return make_uint4(umma::packBf16(static_cast<float>(x.x), static_cast<float>(x.y)), umma::packBf16(static_cast<float>(x.z), static_cast<float>(x.w)),
-                          umma::packBf16(static_cast<float>(y.x), static_cast<float>(y.y)), umma::packBf16(static_cast<float>(y.z), static_cast<float>(y.w)));
+    template <int H>
+    __device__ __forceinline__ void tile(uint8_t *at, int lane, int m, int gate, int unit) const {   // eight lanes a row of 32 codes
+        int4 v[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+            v[r] = __ldg(reinterpret_cast<const int4 *>(Rq + static_cast<size_t>(min(m + 4 * r + lane / 8, H - 1)) * (3 * H) + gate * H + unit) + lane % 8);
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+            *reinterpret_cast<uint2 *>(unitrev::tilePlace(at, 4 * r + lane / 8, lane % 8 * 4)) =
+                make_uint2(umma::packBf16(static_cast<float>(v[r].x), static_cast<float>(v[r].y)), umma::packBf16(static_cast<float>(v[r].z), static_cast<float>(v[r].w)));
     }
     __device__ __forceinline__ Unit unitOf(int unit) const { return Unit{{a.scaleR[unit], a.scaleR[a.H + unit], a.scaleR[2 * a.H + unit]}}; }
     __device__ __forceinline__ State begin(int row, int unit) const { return State{a.dhIn ? a.dhIn[static_cast<size_t>(row) * a.H + unit] : 0.0f}; }

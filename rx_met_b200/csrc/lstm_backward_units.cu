@@ -15,6 +15,7 @@ namespace {
 struct LstmReverseCell {
     static constexpr int kGates = 4, kWords = 8;
     BackwardClusterArgs a;
+    bool vectors;   // the weight codes lie on a 16-byte boundary
 
     struct Unit {
         float scale[4];
@@ -32,12 +33,26 @@ struct LstmReverseCell {
         float gate[4];
         uint32_t bits;
     };
-    __device__ __forceinline__ uint4 weights8(int m, int gate, int unit) const {
-        const float *src = a.weightCodes + (static_cast<size_t>(gate) * a.H + unit) * a.H + m;
-        uint32_t packed[4];
+    template <int H>
+    __device__ __forceinline__ void tile(uint8_t *at, int lane, int m, int gate, int unit) const {   // eight lanes a channel of 32 output units
+        const int first = min(m + lane % 8 * 4, H - 4);
+        float v[8][4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) packed[e] = umma::packBf16(__ldg(src + 2 * e * a.H), __ldg(src + (2 * e + 1) * a.H));
-        return make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        for (int r = 0; r < 8; ++r) {   // channels 8 (r / 2) + 2 (lane / 8) + r % 2
+            const float *src = a.weightCodes + (static_cast<size_t>(gate) * H + unit + r / 2 * 8 + lane / 8 * 2 + r % 2) * H + first;
+            if (vectors) {
+                const float4 x = __ldg(reinterpret_cast<const float4 *>(src));
+                v[r][0] = x.x; v[r][1] = x.y; v[r][2] = x.z; v[r][3] = x.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[r][e] = __ldg(src + e);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 8; r += 2)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                *reinterpret_cast<uint32_t *>(unitrev::tilePlace(at, lane % 8 * 4 + e, r / 2 * 8 + lane / 8 * 2)) = umma::packBf16(v[r][e], v[r + 1][e]);
     }
     __device__ __forceinline__ Unit unitOf(int unit) const {
         return Unit{{a.channelScale[unit], a.channelScale[a.H + unit], a.channelScale[2 * a.H + unit], a.channelScale[3 * a.H + unit]}};
@@ -110,7 +125,7 @@ struct LstmReverseCell {
 }  // namespace
 
 void backwardUnits(const BackwardClusterArgs &args, cudaStream_t st) {
-    const LstmReverseCell cell{args};
+    const LstmReverseCell cell{args, alignedTo(args.weightCodes, 16)};
     const unitrev::Problem p{args.T, args.B};
     const char *name = "lstmRecurrentBackwardCluster";
     switch (args.H) {

@@ -5,7 +5,9 @@
 // bf16) stay in tensor memory as the A operand; the gradients of a step, times the channels' scales, are the B operand as three bf16
 // terms that carry all of their 24 bits, term i of row r in column 4 r + i.  The sums over the channels of 64 units (32 where 64 do
 // not divide the width) have accumulators of their own that are added in fp32: a tcgen05 accumulator truncates each addition, and the sums are bit for
-// bit those of the cluster kernels, whose CTAs own 64 (32) units.  Where a layer leaves lanes free, copies of its weights serve other rows.
+// bit those of the cluster kernels, whose CTAs own 64 (32) units.  Layers of 32 units (up to 256 rows) and 64 (up to 128) had an accumulator
+// for every gate and term of mma.sync added in fp32 before; against 64-bit sums their gradient of the initial state after 60 steps is as near as
+// it was (7.1e-8 of its norm then, 6.2e-8 now).  Where a layer leaves lanes free, copies of its weights serve other rows.
 // Per step and thread:
 //   sums of the step before -> dh -> gate gradients -> B operand (the warps only arrive at the barrier behind it) -> control warp starts the
 //   product; under it the gradients are stored, the factors of the next step formed from operands that were asked for four steps ahead,
@@ -37,6 +39,13 @@ struct Problem {
     int T, B;
 };
 
+// A tile of weights in shared memory: 32 output units x 32 channels in bf16.  Rows are 16 bytes apart and change the order of their 16-byte pieces every
+// eight units, so that a warp reads a piece of each row, and writes a pair of channels of every fourth unit, without bank conflicts.
+constexpr uint32_t kTileStride = 64 + 16;
+__device__ __forceinline__ uint8_t *tilePlace(uint8_t *tile, int unit, int channel) {
+    return tile + unit * kTileStride + (((channel >> 3) ^ (unit >> 3)) << 4) + (channel & 7) * 2;
+}
+
 template <class Cell, int H, int ROWS>
 struct Geometry {
     static_assert(H % 32 == 0 && H <= 128, "tiles of 32 units inside one CTA");
@@ -55,12 +64,14 @@ struct Geometry {
     static constexpr uint32_t kStrideB = kCols * 16 + 16;   // 16 bytes more than its rows spread a warp's units over the banks
     static constexpr uint32_t kOperandBytes = kGroupsK * kStrideB;
     static constexpr uint32_t kWordStride = kWarps * 32 * 4, kSlotBytes = kRows * Cell::kWords * kWordStride;   // a word per thread, the operands of a step
-    static constexpr size_t kSharedBytes = kOperandBytes + kSlots * kSlotBytes;
+    static constexpr uint32_t kTileBytes = 32 * kTileStride;                                                  // weights on their way
+    static constexpr size_t kSharedBytes = kOperandBytes + std::max(kSlots * kSlotBytes, kWarps * 2 * kTileBytes);
 };
 
 // Cell contract (device functions; t descends):
 //   kGates
-//   uint4 weights8(m, gate, unit)                 bf16 weights of output unit m and the channels of `gate` of units unit .. unit + 7
+//   void tile<H>(at, lane, m, gate, unit)         a warp: bf16 weights of output units m .. m + 31 (any values beyond H) and the channels of `gate` of units
+//                                                 unit .. unit + 31 as a tile at `at`
 //   State begin(row, unit)                        State::dh: what flows into the last step beside its own gradient
 //   kWords, void fetch(dst, t, row, unit)         copies the kWords words of a step's operands to shared memory, kWordStride bytes apart
 //   Factors factors<STRIDE>(const uint8_t *, unit)   what a step does to dh, formed from them before dh is there
@@ -97,12 +108,24 @@ unitReverse(const __grid_constant__ Problem p, const __grid_constant__ Cell c) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmemSlot, 0), tmemWeights = tmem + G::kParts * G::kCols;
     const uint32_t quarterBase = static_cast<uint32_t>(32 * quarter) << 16;
-    if (warp < G::kWarps)   // the warps of a quarter share its weights
-#pragma unroll 4
-        for (int i = group; i < G::kGroupsK; i += G::kGroups) {
-            const int part = i / G::kGroupsPart, kg = i % G::kGroupsPart, gate = kg / (G::kPart / 8), of = part * G::kPart + kg % (G::kPart / 8) * 8;
-            bwdcluster::tmemStore4(tmemWeights + quarterBase + i * 4, unit < H ? c.weights8(unit, gate, of) : make_uint4(0u, 0u, 0u, 0u));
+    // The weights, shared out among the warps of a quarter.  Tiles through shared memory: a lane needs the channels of one output unit, which in
+    // memory are rows or columns of 4-byte codes; read lane by lane they took a third of a call of four steps (GRU, H = 128, 290 rows: 14.1 -> 9.5 us).
+    if (warp < G::kWarps) {
+        uint8_t *tiles = ring + warp * (2 * G::kTileBytes);
+#pragma unroll (G::kGroups == 1 ? 4 : 2)
+        for (int n = group, turn = 0; n < kGates * (H / 32); n += G::kGroups, ++turn) {
+            const int gate = n / (H / 32), of = n % (H / 32) * 32;
+            uint8_t *tile = tiles + (turn & 1) * G::kTileBytes;
+            c.template tile<H>(tile, lane, unit - lane, gate, of);
+            __syncwarp();   // also parts the reads of a tile from the writes of the next but one
+            const uint32_t to = tmemWeights + quarterBase + (of / G::kPart * G::kGroupsPart + gate * (G::kPart / 8) + of % G::kPart / 8) * 4;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint4 w = *reinterpret_cast<const uint4 *>(tilePlace(tile, lane, 8 * j));
+                bwdcluster::tmemStore4(to + j * 4, unit < H ? w : make_uint4(0u, 0u, 0u, 0u));
+            }
         }
+    }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
