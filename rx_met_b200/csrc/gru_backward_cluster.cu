@@ -19,7 +19,7 @@
 // barrier by itself costs the receiver one barrier update per lane).  Distributed shared memory carries about 16 bytes
 // per clock and SM, so a CTA takes U = 64 units where it can and a cluster as few rows as fill the GPU.
 // T = 100, B = 128, H = 256, both directions of a layer at a time: 713 -> 130 us per pass (recurrentBackwardCodes on
-// FP32 FMA); T = 100, B = 256, H = 128: 161 -> 95 us (recurrentBackwardMma on mma.sync).
+// FP32 FMA).  Up to 128 units: unit_reverse_umma.cuh.
 //
 // Synchronisation: the receiver's mbarrier counts the bytes, two partial-sum buffers by step parity.  A CTA
 // sends step t only after it has the partial sums of step t + 1 of every peer, and a peer sends those only after it

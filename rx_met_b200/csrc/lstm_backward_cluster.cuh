@@ -12,7 +12,7 @@
 //
 // Up to 256 units a CTA owns 64 (32 where 64 do not divide H) of them and a cluster has at most eight CTAs.  Beyond, nine to
 // sixteen CTAs own 32 units each: the weights of 64 would fill tensor memory.  Seven such clusters are resident at once.
-// T = 100, B = 256, H = 128: 218 -> 87 us (mma.sync, one CTA per tile); T = 100, B = 100, H = 160: about 1 ms -> 91 us (FP32 FMA);
+// Up to 128 units: unit_reverse_umma.cuh.  T = 100, B = 100, H = 160: about 1 ms -> 91 us (FP32 FMA);
 // T = 1000, B = 256, H = 512: 10.2 -> 6.0 ms, T = 100, B = 112: 1067 -> 213 us (partial sums through L2 and a grid-wide counter per step).
 #pragma once
 
