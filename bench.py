@@ -782,7 +782,7 @@ def _kernel_ms(lib, names, per=1):
     return out
 
 
-_LSTM_WIDE_KERNELS = ["lstmQuantizePlanes", "lstmQuantizeCodes", "lstmPrepChannelsWide", "lstmInputLinearWide", "lstmRecurrentWide",
+_LSTM_WIDE_KERNELS = ["lstmPrepare", "lstmInputLinearWide", "lstmRecurrentWide",
                       "lstmRecurrentFloatWide", "lstmRecurrentFloat", "lstmInputLinearFloat", "lstmJobMinMax", "lstmJobHistogram",
                       "lstmRecurrentBackwardCluster", "lstmRecurrentBackwardWide", "lstmRecurrentBackward", "lstmGemmNN", "lstmGemmRowsTN",
                       "lstmReduceSplits", "lstmColumnSums", "lstmDequantWeights", "lstmPackStepMasks", "inputGradUmma", "weightGradUmma",

@@ -416,18 +416,6 @@ struct SizerAdapter {
 
 }  // namespace
 
-void quantizeCellCodes(const float *c0, int B, int H, const ScalarExec &s, float *centred, float *carrier, uint8_t *mask,
-                       cudaStream_t st) {
-    const int op = RXMET_LSTM_CELL_STATE;
-    const size_t total = static_cast<size_t>(B) * H;
-    {
-        KernelTimer timer__("lstmQuantizeCodes", st);
-        quantizeCodes<<<gridFor(total, 256), 256, 0, st>>>(c0, B, H, H, s.scale[op], s.zp[op], s.lo[op], s.hi[op], 0, nullptr,
-                                                         carrier, mask, centred);
-    }
-    afterLaunch("lstmQuantizeCodes");
-}
-
 size_t forwardQuantWorkspaceBytes(int T, int B, int I, int H) {
     SizerAdapter s;
     layout(s, T, B, I, H, static_cast<int8_t **>(nullptr), static_cast<int8_t **>(nullptr), static_cast<float **>(nullptr),

@@ -15,10 +15,9 @@
 // times unsigned code bytes); sum = 256 * sum_hi + sum_lo + (grid minimum - zero point) * row sum.
 //
 // Launch plan for one call:
-//   quantizePlanes x2    : x, h0 -> byte planes (+ optional q-carrier masters and clamp masks)
-//   quantizeCodes        : c0 -> centred cell codes (lstm_forward_quant.cu)
-//   prepChannelsWide     : weights -> packed byte codes, 64-bit addends (zero-point correction + bias)
-//   inputLinearWide      : all T*B rows of the input projection, persistent CTAs, cp.async staging
+//   prepare              : x, h0 -> byte planes, c0 -> centred cell codes, weights -> packed byte codes or tensor-core tiles, 64-bit
+//                          addends (zero-point correction + bias), optional q-carrier masters and clamp masks (lstm_prepare.cu)
+//   planeProjUmma, inputLinearWide : all T*B rows of the input projection, persistent CTAs
 //   recurrentWide        : ONE launch for all T steps.  Thread (j, s) owns hidden unit j - all four
 //                          gates - for RB batch rows of row group s, so the gate math needs no
 //                          exchange between threads; weight_hh streams from L2 (it no longer fits one
@@ -38,6 +37,7 @@
 #include "lstm_forward_cluster.cuh"
 #include "plane_proj_umma.cuh"
 #include "lstm_kernels.h"
+#include "lstm_prepare.h"
 
 namespace rxmet {
 namespace lstm {
@@ -45,108 +45,8 @@ namespace {
 
 using dev::dotSignedUnsigned;
 using dev::linearCentredF;
-using dev::quantizeCode;
 using dev::rescaleF;
 using dev::scaleCell;
-
-// [rows][cols] floats -> [rows][PLANES][kWords] words of four unsigned bytes of (code - lo); columns
-// beyond `cols` are zero.  With PLANES = 2 plane 0 holds the high bytes.  src == null stands for real
-// zeros (the zero-point code).
-template <int PLANES>
-__global__ void quantizePlanes(const float *__restrict__ src, int rows, int cols, int kWords, float scale, int32_t zp,
-                               int32_t lo, int32_t hi, uint32_t *__restrict__ planes, float *__restrict__ carrier,
-                               uint8_t *__restrict__ mask) {
-    const size_t total = static_cast<size_t>(rows) * kWords;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const size_t r = i / kWords;
-        const int kw = static_cast<int>(i % kWords);
-        uint32_t high = 0, low = 0;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int k = kw * 4 + e;
-            if (k >= cols) continue;
-            const size_t o = r * cols + k;
-            uint8_t m = 0;
-            const int32_t q = src ? quantizeCode(src[o], scale, zp, lo, hi, m) : min(max(zp, lo), hi);
-            const uint32_t u = static_cast<uint32_t>(q - lo);
-            low |= (u & 0xffu) << (8 * e);
-            high |= ((u >> 8) & 0xffu) << (8 * e);
-            if (carrier) carrier[o] = static_cast<float>(q);
-            if (mask) mask[o] = m;
-        }
-        uint32_t *row = planes + r * PLANES * kWords;
-        if (PLANES == 2) {
-            row[kw] = high;
-            row[kWords + kw] = low;
-        } else {
-            row[kw] = low;
-        }
-    }
-}
-
-struct WidePrepArgs {
-    int H, I, kWordsIh, kWordsHh;
-    const float *wIh, *wHh, *bIh, *bHh;  // float masters
-    const float *channel;                // kChannelFields x 4H
-    int32_t wLo, wHi, bLo, bHi;
-    int64_t xCorrection, hCorrection;    // (grid minimum - zero point) of the x and h codes
-    uint32_t *wIhWords;                  // [kWordsIh][4H]
-    uint32_t *wHhWords;                  // [2 gate pairs][kWordsHh][H][2]
-    int64_t *ihAddend, *hhAddend;        // correction * row sum + rescaled bias
-    float *mWIh, *mWHh, *mBIh, *mBHh;    // optional q-carrier masters
-    uint8_t *kWIh, *kWHh, *kBIh, *kBHh;  // optional clamp masks
-};
-
-// One warp per output channel and side (blockIdx.y: 0 = weight_ih, 1 = weight_hh).
-__global__ void prepChannelsWide(const WidePrepArgs a) {
-    const int C = 4 * a.H;
-    const int lane = threadIdx.x & 31;
-    const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (c >= C) return;
-    const int side = blockIdx.y;
-    auto field = [&](int f) { return a.channel[static_cast<size_t>(f) * C + c]; };
-    const int K = side ? a.H : a.I, kWords = side ? a.kWordsHh : a.kWordsIh;
-    const float *w = (side ? a.wHh : a.wIh) + static_cast<size_t>(c) * K;
-    const float scale = field(side ? kWHhScale : kWIhScale);
-    float *master = side ? a.mWHh : a.mWIh;
-    uint8_t *keep = side ? a.kWHh : a.kWIh;
-    const int g = c / a.H, j = c % a.H;
-    int32_t sum = 0;
-    for (int kw = lane; kw < kWords; kw += 32) {
-        uint32_t word = 0;
-        for (int i = 0; i < 4; ++i) {
-            const int k = kw * 4 + i;
-            int32_t q = 0;
-            if (k < K) {
-                uint8_t m;
-                q = quantizeCode(w[k], scale, 0, a.wLo, a.wHi, m);
-                if (master) master[static_cast<size_t>(c) * K + k] = static_cast<float>(q);
-                if (keep) keep[static_cast<size_t>(c) * K + k] = m;
-            }
-            sum += q;
-            word |= (static_cast<uint32_t>(q) & 0xffu) << (8 * i);
-        }
-        if (side) a.wHhWords[((static_cast<size_t>(g >> 1) * kWords + kw) * a.H + j) * 2 + (g & 1)] = word;
-        else a.wIhWords[static_cast<size_t>(kw) * C + c] = word;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane != 0) return;
-    int64_t addend = (side ? a.hCorrection : a.xCorrection) * static_cast<int64_t>(sum);
-    const float *b = side ? a.bHh : a.bIh;
-    if (b) {
-        uint8_t m;
-        const int32_t q = quantizeCode(b[c], field(side ? kBHhScale : kBIhScale), 0, a.bLo, a.bHi, m);
-        const DevRescale r{field(side ? kHhBiasMult : kIhBiasMult), field(side ? kHhBiasPow2 : kIhBiasPow2)};
-        addend += static_cast<int64_t>(rescaleF(static_cast<float>(q), r));
-        float *bm = side ? a.mBHh : a.mBIh;
-        uint8_t *bk = side ? a.kBHh : a.kBIh;
-        if (bm) bm[c] = static_cast<float>(q);
-        if (bk) bk[c] = m;
-    }
-    (side ? a.hhAddend : a.ihAddend)[c] = addend;
-}
 
 __device__ __forceinline__ void copyAsync16(void *dst, const void *src, bool valid) {
     const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
@@ -1004,59 +904,37 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
 
     const rxmet_lstm_masters none{};
     const rxmet_lstm_masters &m = call.masters ? *call.masters : none;
-    auto quantize = [&](const float *src, size_t nRows, int cols, int kWords, int op, uint32_t *dst, float *carrier, uint8_t *mask) {
-        const size_t total = nRows * kWords;
-        {
-            KernelTimer timer__("lstmQuantizePlanes", st);
-            if (planes == 2)
-                quantizePlanes<2><<<gridFor(total, 256), 256, 0, st>>>(src, static_cast<int>(nRows), cols, kWords, s.scale[op], s.zp[op],
-                                                                      s.lo[op], s.hi[op], dst, carrier, mask);
-            else
-                quantizePlanes<1><<<gridFor(total, 256), 256, 0, st>>>(src, static_cast<int>(nRows), cols, kWords, s.scale[op], s.zp[op],
-                                                                      s.lo[op], s.hi[op], dst, carrier, mask);
-        }
-        afterLaunch("lstmQuantizePlanes");
+    // Input projection: the tcgen05 kind::i8 kernel when the operands fit shared memory
+    // (RXMET_IPROJ_SIMT turns it off), else the dp4a kernel.
+    const bool tensorProjection = planeproj::fits(planeproj::paddedK(kIh), planes) && std::getenv("RXMET_IPROJ_SIMT") == nullptr;
+    PrepareCall pc{};
+    pc.H = H; pc.planes = planes; pc.channel = l.channel;
+    pc.wLo = s.lo[RXMET_LSTM_WEIGHT_IH]; pc.wHi = s.hi[RXMET_LSTM_WEIGHT_IH];
+    pc.bLo = s.lo[RXMET_LSTM_BIAS_IH]; pc.bHi = s.hi[RXMET_LSTM_BIAS_IH];
+    auto correction = [&](int op) { return static_cast<int64_t>(s.lo[op]) - s.zp[op]; };
+    pc.ih = PrepareWeights{call.weightIh, call.biasIh, I, kIh, kWIhScale, kBIhScale, kIhBiasMult, kIhBiasPow2, correction(RXMET_LSTM_INPUT), l.addIh,
+                           m.weight_ih, m.bias_ih, m.weight_ih_clamped, m.bias_ih_clamped};
+    pc.hh = PrepareWeights{call.weightHh, call.biasHh, H, kHh, kWHhScale, kBHhScale, kHhBiasMult, kHhBiasPow2, correction(RXMET_LSTM_OUTPUT), l.addHh,
+                           m.weight_hh, m.bias_hh, m.weight_hh_clamped, m.bias_hh_clamped};
+    (tensorProjection ? pc.ihTiles : pc.ihWords) = tensorProjection ? reinterpret_cast<uint32_t *>(l.ihTiles) : l.wIh;
+    pc.hhWords = l.wHh;
+    auto tensor = [&](const float *src, size_t nRows, int cols, int words, int op, float *carrier, uint8_t *clamped) {
+        return PrepareRows{src, nRows, cols, words, s.scale[op], s.zp[op], s.lo[op], s.hi[op], nullptr, nullptr, carrier, clamped};
     };
-    quantize(call.x, rows, I, kIh, RXMET_LSTM_INPUT, l.x, m.input, m.input_clamped);
-    quantize(call.h0, static_cast<size_t>(B), H, kHh, RXMET_LSTM_OUTPUT, l.h0, m.initial_hidden, m.initial_hidden_clamped);
-    quantizeCellCodes(call.c0, B, H, s, l.c0, m.initial_cell, m.initial_cell_clamped, st);
-    if (!call.h0) {
-        if (m.initial_hidden_clamped) RXMET_CUDA(cudaMemsetAsync(m.initial_hidden_clamped, 0, static_cast<size_t>(B) * H, st));
-        if (m.initial_cell_clamped) RXMET_CUDA(cudaMemsetAsync(m.initial_cell_clamped, 0, static_cast<size_t>(B) * H, st));
-    }
-
-    WidePrepArgs pa{};
-    pa.H = H; pa.I = I; pa.kWordsIh = kIh; pa.kWordsHh = kHh;
-    pa.wIh = call.weightIh; pa.wHh = call.weightHh; pa.bIh = call.biasIh; pa.bHh = call.biasHh;
-    pa.channel = l.channel;
-    pa.wLo = s.lo[RXMET_LSTM_WEIGHT_IH]; pa.wHi = s.hi[RXMET_LSTM_WEIGHT_IH];
-    pa.bLo = s.lo[RXMET_LSTM_BIAS_IH]; pa.bHi = s.hi[RXMET_LSTM_BIAS_IH];
-    pa.xCorrection = static_cast<int64_t>(s.lo[RXMET_LSTM_INPUT]) - s.zp[RXMET_LSTM_INPUT];
-    pa.hCorrection = static_cast<int64_t>(s.lo[RXMET_LSTM_OUTPUT]) - s.zp[RXMET_LSTM_OUTPUT];
-    pa.wIhWords = l.wIh; pa.wHhWords = l.wHh; pa.ihAddend = l.addIh; pa.hhAddend = l.addHh;
-    pa.mWIh = m.weight_ih; pa.mWHh = m.weight_hh; pa.mBIh = m.bias_ih; pa.mBHh = m.bias_hh;
-    pa.kWIh = m.weight_ih_clamped; pa.kWHh = m.weight_hh_clamped; pa.kBIh = m.bias_ih_clamped; pa.kBHh = m.bias_hh_clamped;
-    {
-        KernelTimer timer__("lstmPrepChannelsWide", st);
-        prepChannelsWide<<<dim3((C + 7) / 8, 2), 256, 0, st>>>(pa);
-    }
-    afterLaunch("lstmPrepChannelsWide");
+    pc.x = tensor(call.x, rows, I, kIh, RXMET_LSTM_INPUT, m.input, m.input_clamped);
+    pc.x.planes = l.x;
+    pc.h0 = tensor(call.h0, static_cast<size_t>(B), H, kHh, RXMET_LSTM_OUTPUT, m.initial_hidden, m.initial_hidden_clamped);
+    pc.h0.planes = l.h0;
+    pc.c0 = tensor(call.c0, static_cast<size_t>(B), H, (H + 3) / 4, RXMET_LSTM_CELL_STATE, m.initial_cell, m.initial_cell_clamped);
+    pc.c0.centred = l.c0;
+    pc.clear = l.projStatus;
+    prepare(pc, st);
 
     const rxmet_lstm_trace noTrace{};
     const rxmet_lstm_trace &ck = call.checkpoints ? *call.checkpoints : noTrace;
     const int sms = currentDevice().sms;
     const bool units = forwardInUnits(e, B, I, H);
-    // Input projection: the tcgen05 kind::i8 kernel when the operands fit shared memory
-    // (RXMET_IPROJ_SIMT turns it off), else the dp4a kernel.
-    const int kPadIh = planeproj::paddedK(kIh);
-    const bool tensorProjection = planeproj::fits(kPadIh, planes) && std::getenv("RXMET_IPROJ_SIMT") == nullptr;
     if (tensorProjection) {
-        RXMET_CUDA(cudaMemsetAsync(l.projStatus, 0, sizeof(int), st));
-        {
-            KernelTimer timer__("lstmPrepChannelsWide", st);
-            planeproj::packTiles<<<gridFor(static_cast<size_t>(planeproj::paddedC(C)) * kPadIh / 16, 256), 256, 0, st>>>(l.wIh, kIh, C, kPadIh, l.ihTiles);
-        }
-        afterLaunch("packTiles");
         planeproj::Problem pp{};
         pp.planes = l.x; pp.rows = static_cast<int>(rows); pp.kWords = kIh; pp.tiles = l.ihTiles; pp.C = C; pp.status = l.projStatus;
         auto launchTensor = [&](auto epi, auto planeCount) {

@@ -50,10 +50,6 @@ bool unitsFasterThanBytes(int T, int B, int H, bool saves);
 size_t forwardQuantWideWorkspaceBytes(int T, int B, int I, int H);
 void forwardQuantWide(const ForwardQuantCall &call, const Exec &exec, void *workspace, size_t workspaceBytes,
                       cudaStream_t stream);
-// c0 [B,H] (null = real zeros) -> centred cell codes, optional q-carrier copy and clamp mask.
-void quantizeCellCodes(const float *c0, int B, int H, const ScalarExec &scalar, float *centred, float *carrier,
-                       uint8_t *mask, cudaStream_t stream);
-
 // How a saved tensor is turned into real values while it is loaded: real = (value - zeroPoint) * scale.
 // The float backward uses {1, 0}; the QAT backward passes the grid of each saved q-carrier tensor.
 struct Dequant {

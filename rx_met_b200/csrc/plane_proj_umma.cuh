@@ -94,24 +94,6 @@ inline size_t sharedBytes(int kPad, int planes) {
     return static_cast<size_t>(ringSlices(kPad, planes)) * kChannelTile * std::min(kPad, kSlice) + 2 * static_cast<size_t>(planes) * rowsPerTile(kPad) * kPad;
 }
 
-// words [kWords][C] (four signed codes along k per word) -> packed tiles (tilePlace); k beyond 4 kWords and channels beyond C are zero.
-// One thread per 16-byte row of a core matrix.
-static __global__ void packTiles(const uint32_t *__restrict__ words, int kWords, int C, int kPad, uint4 *__restrict__ tiles) {
-    const int groups = kPad / 16, padded = paddedC(C);
-    const size_t total = static_cast<size_t>(padded) * groups;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        // consecutive threads -> consecutive channels of one k-group (coalesced reads of the word rows)
-        const int kg = static_cast<int>(i / padded), c = static_cast<int>(i % padded);
-        uint32_t v[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int kw = 4 * kg + e;
-            v[e] = kw < kWords && c < C ? words[static_cast<size_t>(kw) * C + c] : 0u;
-        }
-        tiles[tilePlace(c, kg, kPad)] = make_uint4(v[0], v[1], v[2], v[3]);
-    }
-}
-
 // Epilogue functor contract:
 //   struct Loaded; __device__ Loaded load(int c) const;    what a channel reads from memory, asked for one item ahead
 //   struct Channel;                                        per-channel constants; Channel::small, uniform in the warp: storeRows takes it
@@ -179,6 +161,7 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const __grid_consta
     }
     // the k padding of the planes is never written again
     for (uint32_t i = tid; i < 2 * PLANES * planeBytes / 16; i += kThreads) reinterpret_cast<uint4 *>(rowPlanes)[i] = make_uint4(0u, 0u, 0u, 0u);
+    waitForPredecessor();   // what is above needs nothing from earlier kernels
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -342,7 +325,7 @@ void launch(const char *name, Problem p, const Epilogue &epi, int sms, int depen
         ensureDynamicSmem(reinterpret_cast<const void *>(kernel), smem);
         {
             KernelTimer timer__(name, st);
-            kernel<<<grid, kThreads, smem, st>>>(p, epi);
+            launchDependent(kernel, grid, kThreads, smem, st, p, epi);
         }
         afterLaunch(name);
     };
