@@ -16,9 +16,9 @@ __device__ __forceinline__ void waitForPredecessor() { asm volatile("griddepcont
 __device__ __forceinline__ void letDependentsStart() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 template <class... Params, class... Args>
-void launchDependent(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, Args &&...args) {
+void launchDependent(void (*kernel)(Params...), dim3 grid, int block, size_t smem, cudaStream_t stream, Args &&...args) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(static_cast<unsigned>(block));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;

@@ -1187,7 +1187,7 @@ size_t tiledWorkspaceBytes(int T, int B, int I, int H, bool padded) {
                                                 H <= 143 ? wgrad::splitBound(static_cast<int>(rows), H, static_cast<int>(C)) : 1})) * (H + 1) * C);
     ws.take<int>(64);
     ws.take<float>(static_cast<size_t>(B) * H);   // gradient carried between time chunks
-    ws.take<uint8_t>(igrad::widePackedBytes(static_cast<int>(C), I) + 256);   // weight operand of the streaming input-gradient kernel
+    ws.take<uint8_t>(igrad::packedBytes(static_cast<int>(C), I) + 256);   // weight operand of the input gradient
     return ws.used() + 4096;
 }
 
@@ -1412,7 +1412,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
             float *partialX = ws.take<float>(static_cast<size_t>(totalSplits) * (I + 1) * C);
             float *partialH = ws.take<float>(static_cast<size_t>(totalSplits) * (H + 1) * C);
             uint8_t *packedW = nullptr;
-            if (const size_t bytes = igrad::widePackedBytes(C, I)) packedW = ws.take<uint8_t>(bytes);
+            if (const size_t bytes = igrad::packedBytes(C, I)) packedW = ws.take<uint8_t>(bytes);
             int tEnd = T, splitBase = 0;
             for (size_t i = 0; i < chunks.size(); ++i) {
                 const int n = chunks[i], t0 = tEnd - n;
@@ -1507,13 +1507,13 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
 
     // dx
     int *status = ws.take<int>(1);  // set by a tcgen05 kernel whose bounded wait gave up
-    if (call.W_q) RXMET_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
+    if (call.W_q && !tensorInputGrad) RXMET_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));   // the input gradient clears it itself
     if (tensorInputGrad) {
         // QAT: gradients times the integer weight codes on the tensor cores, scales folded into the gradients
         igrad::Problem pg{};
         pg.G = dp; pg.kScale = chanScaleW; pg.codesNK = call.W_q; pg.rows = static_cast<int>(rows); pg.K = C; pg.N = call.dxColumns ? call.dxColumns : I;
-        pg.mask = mk.x; pg.maskKeeps = 1; pg.out = call.dx; pg.status = status;
-        if (const size_t bytes = igrad::widePackedBytes(C, pg.N)) pg.packed = ws.take<uint8_t>(bytes);
+        pg.mask = mk.x; pg.maskKeeps = 1; pg.out = call.dx; pg.status = pg.clear = status;
+        if (const size_t bytes = igrad::packedBytes(C, pg.N)) pg.packed = ws.take<uint8_t>(bytes);
         igrad::launch(pg, sms, st);
         afterLaunch("inputGradUmma");
     } else {

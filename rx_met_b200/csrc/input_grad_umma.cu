@@ -1,23 +1,31 @@
-// dx = (G * kScale) code on tcgen05.mma with the accumulator tile in tensor memory.
+// dx = (G * kScale) code on tcgen05.mma, the gradients as A operand in tensor memory.
 //
-// One CTA per SM owns a contiguous range of rows and walks it in tiles of 128 rows (= the 128
-// lanes of tensor memory).  For a tile the accumulator D[128][NP] (NP = N padded to 16) sums
-// over K in chunks of 32 channels:
-//   * A = the chunk of G, K-major as it lies in HBM ([row][k]).  Warp w copies rows [8w, 8w + 8)
-//     of the chunk (8 x 128 bytes) into a ring of raw buffers with cp.async, several chunks ahead,
-//     then scales, splits into three bf16 terms and stores 16-byte pieces into the un-swizzled
-//     canonical K-major layout (core matrix = 8 rows x 8 k).
-//   * B = the weight codes as bf16, converted once per CTA into the same canonical layout and
-//     kept in shared memory for all tiles.
-//   * one thread issues the six MMAs of the chunk (2 k-steps x 3 terms) and commits them to the
-//     mbarrier of the operand stage; kStages stages rotate.
-// After the last chunk of a tile the accumulators are read back with tcgen05.ld (lane = row),
-// masked and stored.  Every mbarrier wait is bounded; a wait that gives up poisons the CTA's
-// outputs with NaN and sets the status word, and the CTA still frees its tensor memory.
+// A CTA walks a contiguous range of rows in tiles of 128 rows (= the lanes of tensor memory) and, with more than 256 columns, one slab
+// of columns.  The accumulator D[128][NP] of a tile sums over K in chunks of 32 channels.  Warps by role:
+//   gradients   one lane copies a chunk's rows as TMA boxes of 32 rows x 128 bytes (128-byte swizzle) into a ring
+//   converters  sixteen warps, two groups that take chunks in turn: thread = row and sixteen channels; reads its pieces, scales them,
+//               splits them into three bf16 terms that carry all 24 bits and stores these to its own tensor-memory lane
+//   weights     up to 64 columns the codes, exact in bf16, are converted once per CTA and stay in shared memory; beyond, packWeights lays
+//               them out before and one lane copies them chunk by chunk (bulk copies)
+//   products    one thread issues the six MMAs of a chunk (2 k-steps x 3 terms, in this order) into one of two accumulators (one beyond 128 columns)
+//   epilogue    eight warps: accumulator rows through shared memory, so that a store covers 128 bytes of a row, masked
+// so that a tile leaves under the products of the next one.  Every mbarrier wait is bounded; one that gives up ends all further waiting of
+// the CTA, turns the outputs that follow into NaN and sets the status word; copies and products in flight are awaited and
+// tensor memory is freed all the same.
+//
+// Bound: the hand-overs and the conversion of a chunk (0.35 us a chunk and SM), beyond 128 columns the tensor pipe (0.41 us at 256 columns).  The forms
+// before it wrote the terms to shared memory, where the MMAs read them again: half of its bandwidth beside copies and conversion; they walked
+// whole tiles (two rounds where a CTA has 173 rows) and left the epilogue outside.  In a step, with what surrounds the kernel: 25,600 rows x 384 -> 40
+// columns 26.8 -> 23.7 us, 25,600 x 512 -> 40 31.7 -> 26.1, 12,800 x 768 -> 40 41.4 -> 24.7, 256,000 x 2048 -> 256 943 -> 707; by itself, back to back, 17, 21, 18 us
+// and 12,800 x 768 -> 512 59 -> 40.
+#include <cuda.h>
+
 #include <algorithm>
 #include <cstdlib>
 
+#include "backward_cluster_device.cuh"
 #include "common.h"
+#include "dependent_launch.cuh"
 #include "input_grad_umma.h"
 #include "umma_device.cuh"
 
@@ -27,268 +35,461 @@ namespace {
 
 using namespace umma;
 
-constexpr int kThreads = 512, kWarps = kThreads / 32;
-constexpr int kChunkK = 64;                      // channels per chunk: four MMA k-steps
-constexpr int kSpans = kChunkK / 32;             // 128-byte spans of a row per chunk
-constexpr int kRing = 2;                         // raw chunks in flight
-constexpr int kStages = 2;                       // operand stages: chunks whose MMAs may be pending
-constexpr uint32_t kRawBytes = kTileM * kChunkK * 4;         // 16 x kSpans pieces of 8 rows x 128 bytes
-constexpr uint32_t kTermBytes = kTileM * kChunkK * 2;        // 8 KB: one bf16 term of a chunk
-constexpr uint32_t kStageBytes = 3 * kTermBytes;
-constexpr uint32_t kAKStride = kCore;                        // next k-group of the same 8 rows
-constexpr uint32_t kAMStride = (kChunkK / 8) * kCore;        // next 8 rows
-constexpr int kMaxK = 768;
+constexpr int kChunk = 32;                                     // channels: two k-steps
+constexpr int kConvWarps = 16, kEpilogueWarps = 8, kFillWarps = kConvWarps + kEpilogueWarps;
+constexpr int kGradientWarp = kFillWarps, kWeightWarp = kFillWarps + 1, kProductWarp = kFillWarps + 2;
+constexpr int kThreads = 32 * (kProductWarp + 1);
+constexpr int kBoxRows = 32, kMaxRing = 6, kMaxStages = 8, kWeightRing = 4;
+constexpr uint32_t kBoxBytes = kBoxRows * kChunk * 4, kRawBytes = kTileM / kBoxRows * kBoxBytes;   // 4 KB, 16 KB
+constexpr uint32_t kStageCols = 3 * kChunk / 2;               // tensor-memory columns of a chunk: three terms, two channels a column
+constexpr uint32_t kGroupStride = kChunk / 8 * kCore;          // weights: next eight columns
+constexpr uint32_t kTmemCols = 512;
+constexpr int kResidentColumns = 64, kMaxColumns = 256;        // of a CTA
+constexpr int kMaxK = 8192;
 
-size_t sharedBytes(int K, int NP) {
-    return kStages * kStageBytes + kRing * kRawBytes + static_cast<size_t>(NP) * K * 2 + sizeof(float) * K;
-}
+struct Shape {
+    int NP, slabs;        // padded columns of a slab
+    int accs, stages;     // accumulators and operand stages in tensor memory
+    int ring;             // chunks of gradients in shared memory
+    int rowsPerCta;       // a multiple of kBoxRows
+};
 
-// gridDim.y = column slabs of the output: slab s works on columns [NP s, NP s + NP) with its own copy of the
-// weight operand; every slab walks all rows (the gradient rows are re-read from L2 once per slab).
-template <int NP>
-__global__ void __launch_bounds__(kThreads, 1) inputGradUmma(const Problem whole, int rowsPerCta) {
-    Problem p = whole;
-    {
-        const int n0 = static_cast<int>(blockIdx.y) * NP;
-        if (p.ldN == 0) p.ldN = p.N;
-        if (p.ldCodesKN == 0) p.ldCodesKN = p.N;
-        if (gridDim.y > 1) {
-            p.N = min(NP, whole.N - n0);
-            if (p.codesNK) p.codesNK += static_cast<size_t>(n0) * p.K;
-            if (p.codesKN) p.codesKN += n0;
-            if (p.mask) p.mask += n0;
-            p.out += n0;
+// codes -> bf16: packed[slab][chunk][n / 8][k-group][n % 8][8 k]; one thread per 16-byte row.
+struct WeightRow {
+    float c[8];
+    __device__ __forceinline__ void load(const Problem &p, int n, int k0) {
+        if (n >= p.N) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) c[j] = 0.0f;
+        } else if (p.codesNK) {   // K is a multiple of 32
+            const int32_t *at = p.codesNK + static_cast<size_t>(n) * p.K + k0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                int4 q;
+                if ((reinterpret_cast<uintptr_t>(at) & 15) == 0) q = __ldg(reinterpret_cast<const int4 *>(at) + h);
+                else q = make_int4(__ldg(at + 4 * h), __ldg(at + 4 * h + 1), __ldg(at + 4 * h + 2), __ldg(at + 4 * h + 3));
+                c[4 * h] = static_cast<float>(q.x); c[4 * h + 1] = static_cast<float>(q.y); c[4 * h + 2] = static_cast<float>(q.z); c[4 * h + 3] = static_cast<float>(q.w);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) c[j] = __ldg(p.codesKN + static_cast<size_t>(k0 + j) * p.ldCodesKN + n);
         }
     }
-    constexpr uint32_t kTmemCols = NP <= 32 ? 32 : 64;
-    constexpr uint32_t kIdesc = instructionDescriptor(NP, false, false);
-    extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ __align__(8) uint64_t bars[kStages + 1];  // one per operand stage, the last for "tile complete"
+    __device__ __forceinline__ uint4 packed() const {
+        return make_uint4(packBf16(c[0], c[1]), packBf16(c[2], c[3]), packBf16(c[4], c[5]), packBf16(c[6], c[7]));
+    }
+};
+__device__ __forceinline__ int rowPlace(int n, int k8, int NP) {   // in units of 16 bytes
+    return (k8 / 4 * (NP / 8) + n / 8) * 32 + k8 % 4 * 8 + n % 8;
+}
+__global__ void packWeights(const Problem p, int NP, int slabs, uint4 *packed) {
+    letDependentsStart();
+    const int groups = p.K / 8, item = blockIdx.x * blockDim.x + threadIdx.x;
+    if (item >= groups * NP * slabs) return;
+    const int k8 = item % groups, n = item / groups, slab = n / NP;
+    WeightRow row;
+    row.load(p, n, 8 * k8);
+    packed[static_cast<size_t>(slab) * groups * NP + rowPlace(n - slab * NP, k8, NP)] = row.packed();
+}
+
+__device__ __forceinline__ bool testPhase(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
+template <int N>
+__device__ __forceinline__ void tmemStore(uint32_t addr, const uint32_t (&v)[N]) {
+    static_assert(N == 8, "a k-step of one row");
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+
+// Walks a ring of mbarriers: place and phase parity of the current use.  Counters, not divisions: a division by a value known at run time costs
+// a lone thread more than issuing the products of a chunk.
+struct Turn {
+    int at = 0;
+    uint32_t parity = 0;
+    bool again = false;   // the place was used before
+    __device__ __forceinline__ void step(int size, int by = 1) {
+        at += by;
+        if (at >= size) {
+            at -= size;
+            parity ^= 1u;
+            again = true;
+        }
+    }
+};
+
+template <bool STREAM>   // weights chunk by chunk
+__global__ void __launch_bounds__(kThreads, 1)
+inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s, const __grid_constant__ CUtensorMap gradients) {
+    extern __shared__ __align__(1024) uint8_t smemRaw[];
+    __shared__ __align__(8) uint64_t rawFull[kMaxRing], rawFree[kMaxRing], termsFull[kMaxStages], termsFree[kMaxStages], weightsFull[kWeightRing],
+        weightsFree[kWeightRing], accFull[2], accFree[2];
     __shared__ uint32_t tmemSlot;
-    __shared__ int failed;
+    __shared__ volatile int failed;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
-    const int rm = lane & 7, cq = lane >> 3;
-    const int K = p.K, N = p.N, chunksPerTile = K / kChunkK;
-    const uint32_t kBNStride = static_cast<uint32_t>(K / 8) * kCore;  // next 8 columns of the weight operand
-    uint8_t *stages = smem;
-    uint4 *raw = reinterpret_cast<uint4 *>(smem + kStages * kStageBytes);   // [kRing][16 warps][kSpans][64]
-    uint8_t *weights = smem + kStages * kStageBytes + kRing * kRawBytes;
-    float *scale = reinterpret_cast<float *>(weights + static_cast<size_t>(NP) * K * 2);
-
-    const int rowBegin = min(p.rows, static_cast<int>(blockIdx.x) * rowsPerCta);
-    const int rowEnd = min(p.rows, rowBegin + rowsPerCta);
-    const int tiles = (rowEnd - rowBegin + kTileM - 1) / kTileM;
-    const int totalChunks = tiles * chunksPerTile;
+    const int K = p.K, NP = s.NP, chunks = K / kChunk, n0 = static_cast<int>(blockIdx.y) * NP, columns = min(p.N - n0, NP);
+    const int rowBegin = min(p.rows, static_cast<int>(blockIdx.x) * s.rowsPerCta), rowEnd = min(p.rows, rowBegin + s.rowsPerCta);
+    const int tiles = (rowEnd - rowBegin + kTileM - 1) / kTileM, total = tiles * chunks;
+    const uint32_t weightBytes = static_cast<uint32_t>(NP) * kChunk * 2;   // of a chunk
+    uint8_t *raw = smemRaw + ((1024u - (smemAddr(smemRaw) & 1023u)) & 1023u);   // swizzled boxes start on 1024 bytes
+    uint8_t *turn = raw + s.ring * kRawBytes;                                    // [8 warps][32 rows][128 bytes]
+    uint8_t *weights = turn + kEpilogueWarps * 4096;
+    float *scale = reinterpret_cast<float *>(weights + (STREAM ? kWeightRing : chunks) * weightBytes);
 
     if (tid == 0) {
         failed = 0;
-        for (int i = 0; i <= kStages; ++i)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smemAddr(&bars[i])) : "memory");
+        auto init = [](uint64_t *bar, uint32_t count) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smemAddr(bar)), "r"(count) : "memory");
+        };
+        for (int i = 0; i < kMaxRing; ++i) { init(&rawFull[i], 1); init(&rawFree[i], kConvWarps / 2); }
+        for (int i = 0; i < kMaxStages; ++i) { init(&termsFull[i], kConvWarps / 2); init(&termsFree[i], 1); }
+        for (int i = 0; i < kWeightRing; ++i) { init(&weightsFull[i], STREAM ? 1 : kFillWarps); init(&weightsFree[i], 1); }
+        for (int i = 0; i < 2; ++i) { init(&accFull[i], 1); init(&accFree[i], kEpilogueWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(&tmemSlot)), "r"(kTmemCols)
-                     : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(&tmemSlot)), "n"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-
-    // Warp w copies rows [8w, 8w + 8) of linear chunk `chunk` (tile chunk / chunksPerTile) into
-    // ring entry `slot`.  A copy instruction covers four whole 128-byte rows (lane -> row
-    // lane / 8, 16-byte part lane % 8); part q of row r is kept at r * 8 + (q ^ r), which keeps
-    // these writes and the converting reads free of bank conflicts.
-    auto issueChunk = [&](int chunk, int slot) {
-        const int tile = chunk / chunksPerTile, kc = chunk - tile * chunksPerTile;
-        uint4 *dst = raw + (static_cast<size_t>(slot) * kWarps + warp) * kSpans * 64;
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int wrow = 4 * i + (lane >> 3), part = lane & 7;
-            const int row = rowBegin + tile * kTileM + 8 * warp + wrow;
-            const bool ok = chunk < totalChunks && row < rowEnd;
-            const float *src = ok ? p.G + static_cast<size_t>(row) * K + kc * kChunkK + 4 * part : p.G;
-#pragma unroll
-            for (int sp = 0; sp < kSpans; ++sp) copyAsync16(dst + sp * 64 + wrow * 8 + (part ^ wrow), ok ? src + 32 * sp : src, ok);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-#pragma unroll
-    for (int r = 0; r < kRing; ++r) issueChunk(r, r);
-
-    // the weight operand: column n, channels [8 j, 8 j + 8) -> one 16-byte row of a core matrix
-    // (consecutive threads walk the contiguous index of whichever code layout was given)
-    for (int item = tid; item < NP * (K / 8); item += kThreads) {
-        const int n = p.codesNK ? item / (K / 8) : item % NP, k8 = p.codesNK ? item % (K / 8) : item / NP;
-        float c[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int k = 8 * k8 + j;
-            c[j] = n >= N ? 0.0f
-                          : (p.codesNK ? static_cast<float>(p.codesNK[static_cast<size_t>(n) * K + k])
-                                       : p.codesKN[static_cast<size_t>(k) * p.ldCodesKN + n]);
-        }
-        *reinterpret_cast<uint4 *>(weights + (n / 8) * kBNStride + k8 * kCore + (n % 8) * 16) =
-            make_uint4(packBf16(c[0], c[1]), packBf16(c[2], c[3]), packBf16(c[4], c[5]), packBf16(c[6], c[7]));
-    }
-    for (int k = tid; k < K; k += kThreads) scale[k] = p.kScale ? p.kScale[k] : 1.0f;
-
+    waitForPredecessor();   // what is above needs nothing from earlier kernels
+    if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && p.clear) *p.clear = 0;
+    for (int k = tid; k < K; k += kThreads) scale[k] = p.kScale ? __ldg(p.kScale + k) : 1.0f;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmemSlot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmemSlot, 0), stageBase = tmem + s.accs * NP;
 
-    for (int g = 0; g < totalChunks; ++g) {
-        const int s = g % kStages, slot = g % kRing;
-        const int tile = g / chunksPerTile, kc = g - tile * chunksPerTile;
-        uint8_t *stage = stages + s * kStageBytes;
-        asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 1) : "memory");
-        __syncwarp();  // the lanes of a warp convert what other lanes of it copied
-        // the MMAs that read this stage kStages chunks ago must have finished
-        if (g >= kStages && !waitPhase(smemAddr(&bars[s]), (g / kStages - 1) & 1)) failed = 1;
-#pragma unroll
-        for (int span = 0; span < kSpans; ++span) {
-            const uint4 *src = raw + ((static_cast<size_t>(slot) * kWarps + warp) * kSpans + span) * 64;
-            const uint4 ru = src[rm * 8 + ((2 * cq) ^ rm)], rv = src[rm * 8 + ((2 * cq + 1) ^ rm)];
-            const float4 su = *reinterpret_cast<const float4 *>(scale + kc * kChunkK + 32 * span + 8 * cq);
-            const float4 sv = *reinterpret_cast<const float4 *>(scale + kc * kChunkK + 32 * span + 8 * cq + 4);
-            const float4 u = make_float4(__uint_as_float(ru.x) * su.x, __uint_as_float(ru.y) * su.y,
-                                         __uint_as_float(ru.z) * su.z, __uint_as_float(ru.w) * su.w);
-            const float4 v = make_float4(__uint_as_float(rv.x) * sv.x, __uint_as_float(rv.y) * sv.y,
-                                         __uint_as_float(rv.z) * sv.z, __uint_as_float(rv.w) * sv.w);
-            const Converted c = splitThree(u, v);
-            uint8_t *dst = stage + warp * kAMStride + (4 * span + cq) * kAKStride + rm * 16;
-            *reinterpret_cast<uint4 *>(dst) = c.hi;
-            *reinterpret_cast<uint4 *>(dst + kTermBytes) = c.mid;
-            *reinterpret_cast<uint4 *>(dst + 2 * kTermBytes) = c.lo;
-        }
+    auto wait = [&](uint64_t *bar, uint32_t parity) {   // one that gives up ends all further waiting of the CTA
+        if (testPhase(smemAddr(bar), parity)) return;
+        if (!failed && !waitSuspended(smemAddr(bar), parity)) failed = 1;
+    };
+    auto arrive = [&](uint64_t *bar) {
         __syncwarp();
-        issueChunk(g + kRing, slot);
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smemAddr(bar)) : "memory");
+    };
+    auto expect = [](uint64_t *bar, uint32_t bytes) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smemAddr(bar)), "r"(bytes) : "memory");
+    };
+    auto boxesOf = [&](int tile) { return min(kTileM / kBoxRows, (rowEnd - rowBegin - tile * kTileM + kBoxRows - 1) / kBoxRows); };
+    if (!STREAM && warp < kFillWarps) {
+        // consecutive threads walk whichever index of the codes is contiguous; three rows are asked for before the first is used
+        constexpr int kAhead = 3, kFill = 32 * kFillWarps;
+        const int inner = p.codesNK ? K / 8 : NP, items = NP * (K / 8);
+        for (int first = tid; first < items; first += kAhead * kFill) {
+            WeightRow rows[kAhead];
+            int place[kAhead];
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+                const int item = min(first + i * kFill, items - 1), outer = item / inner, in = item - outer * inner;
+                const int n = p.codesNK ? outer : in, k8 = p.codesNK ? in : outer;
+                place[i] = rowPlace(n, k8, NP);
+                rows[i].load(p, n, 8 * k8);
+            }
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) reinterpret_cast<uint4 *>(weights)[place[i]] = rows[i].packed();
+        }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (warp == 0 && electOne()) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t aBase = smemAddr(stage), bBase = smemAddr(weights) + kc * (kChunkK / 8) * kCore;
-#pragma unroll
-            for (int ks = 0; ks < kChunkK / 16; ++ks) {
-                const uint64_t descB = operandDescriptor(bBase + ks * 2 * kCore, kCore, kBNStride);
-#pragma unroll
-                for (int sp = 0; sp < 3; ++sp) {
-                    const uint64_t descA = operandDescriptor(aBase + sp * kTermBytes + ks * 2 * kAKStride, kAKStride, kAMStride);
-                    mmaBf16(tmem, descA, descB, kIdesc, (kc > 0 || ks > 0 || sp > 0) ? 1u : 0u);
-                }
-            }
-            commitTo(smemAddr(&bars[s]));
-            if (kc + 1 == chunksPerTile) commitTo(smemAddr(&bars[kStages]));
-        }
-        if (kc + 1 < chunksPerTile) continue;
-
-        // the tile is complete: accumulator rows -> out.  Warp w reads lanes [32 (w % 4), + 32) and
-        // the 16 columns [16 (w / 4), + 16).
-        if (!waitPhase(smemAddr(&bars[kStages]), tile & 1)) failed = 1;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int q = warp & 3, col0 = 16 * (warp >> 2);
-        if (col0 < NP) {
-            uint32_t r[16];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                  "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                : "r"(tmem + (static_cast<uint32_t>(32 * q) << 16) + col0));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            const int row = rowBegin + tile * kTileM + 32 * q + lane;
-            const bool poison = *reinterpret_cast<volatile int *>(&failed) != 0;
-            if (row < rowEnd) {
-                const size_t o = static_cast<size_t>(row) * p.ldN + col0;
-                float v[16];
-                uint8_t m[16];
-                const bool wide = (N % 8) == 0 && (p.ldN % 8) == 0 && col0 + 8 <= N;  // whole 8-column groups, aligned
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (p.mask && wide && col0 + 8 * h + 8 <= N) {
-                        const uint2 w = *reinterpret_cast<const uint2 *>(p.mask + o + 8 * h);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            m[8 * h + j] = static_cast<uint8_t>(w.x >> (8 * j));
-                            m[8 * h + 4 + j] = static_cast<uint8_t>(w.y >> (8 * j));
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            m[8 * h + j] = (p.mask && col0 + 8 * h + j < N) ? p.mask[o + 8 * h + j] : static_cast<uint8_t>(p.maskKeeps);
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float keep = p.maskKeeps ? static_cast<float>(m[j]) : (m[j] == 0 ? 1.0f : 0.0f);
-                    v[j] = poison ? __int_as_float(0x7fc00000) : __uint_as_float(r[j]) * keep;
-                }
-#pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    if ((N % 4) == 0 && (p.ldN % 4) == 0 && col0 + 4 * h + 4 <= N) {
-                        *reinterpret_cast<float4 *>(p.out + o + 4 * h) = make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if (col0 + 4 * h + j < N) p.out[o + 4 * h + j] = v[4 * h + j];
-                    }
-                }
-            }
-        }
-        // the next tile's first MMA overwrites the accumulators: order it behind these loads
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        arrive(&weightsFull[0]);
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+
+    if (warp < kConvWarps) {
+        const int quarter = warp & 3, part = (warp >> 2) & 1, group = warp >> 3, sw = lane & 7;
+        const uint32_t lanes = static_cast<uint32_t>(32 * quarter) << 16;
+        Turn slot, stage;
+        slot.step(s.ring, group);
+        stage.step(s.stages, group);
+        int tile = 0, c = group;
+        while (c >= chunks) { c -= chunks; ++tile; }
+        bool real = quarter < boxesOf(tile);   // lanes of absent rows keep what they held
+        for (int g = group; g < total; g += 2) {
+            wait(&rawFull[slot.at], slot.parity);
+            const uint8_t *row = raw + slot.at * kRawBytes + quarter * kBoxBytes + lane * 128;
+            float v[16];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 x = *reinterpret_cast<const float4 *>(row + (((4 * part + i) ^ sw) << 4));
+                v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
+            }
+            arrive(&rawFree[slot.at]);
+            if (stage.again) wait(&termsFree[stage.at], stage.parity ^ 1u);
+            __syncwarp();
+            if (real) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float4 f = *reinterpret_cast<const float4 *>(scale + c * kChunk + 16 * part + 4 * i);
+                    v[4 * i] *= f.x; v[4 * i + 1] *= f.y; v[4 * i + 2] *= f.z; v[4 * i + 3] *= f.w;
+                }
+                const uint32_t to = stageBase + lanes + stage.at * kStageCols + 8 * part;
+#pragma unroll
+                for (int term = 0; term < 3; ++term) {
+                    uint32_t w[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        w[i] = packBf16(v[2 * i], v[2 * i + 1]);
+                        v[2 * i] -= bf16Lo(w[i]);
+                        v[2 * i + 1] -= bf16Hi(w[i]);
+                    }
+                    tmemStore(to + term * (kChunk / 2), w);
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            }
+            arrive(&termsFull[stage.at]);
+            slot.step(s.ring, 2);
+            stage.step(s.stages, 2);
+            for (c += 2; c >= chunks; c -= chunks) real = quarter < boxesOf(++tile);
+        }
+    } else if (warp < kFillWarps) {
+        // the two warps of a quarter take blocks of 32 columns in turn
+        const int quarter = warp & 3, half = (warp - kConvWarps) >> 2, ldN = p.ldN ? p.ldN : p.N;
+        float4 *mine = reinterpret_cast<float4 *>(turn + (warp - kConvWarps) * 4096);
+        const bool vectors = p.N % 4 == 0 && ldN % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.mask) & 3) == 0;
+        Turn acc;
+        for (int tile = 0; tile < tiles; ++tile, acc.step(s.accs)) {
+            wait(&accFull[acc.at], acc.parity);
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int first = rowBegin + tile * kTileM + 32 * quarter, count = min(32, rowEnd - first);
+            const uint32_t from = tmem + (static_cast<uint32_t>(32 * quarter) << 16) + acc.at * NP;
+            const bool poison = failed != 0;
+            for (int c0 = 32 * half; c0 < NP && count > 0; c0 += 64) {
+                uint32_t r[32];
+                if (c0 + 32 <= NP) {
+                    tmemLoad32(from + c0, r);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) bwdcluster::tmemLoad<8>(from + c0 + 8 * i, *reinterpret_cast<uint32_t (*)[8]>(r + 8 * i));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int i = 16; i < 32; ++i) r[i] = 0u;
+                }
+                // lane = row here: turn the 32 x 32 block so that eight lanes hold 128 bytes of a row
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    mine[lane * 8 + (i ^ (lane & 7))] =
+                        make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
+                __syncwarp();
+                const int i = lane & 7, col = c0 + 4 * i, left = columns - col, at = lane >> 3;
+                const size_t o = static_cast<size_t>(first + at) * ldN + n0 + col;
+                if (left > 0) {
+                    float *to = p.out + o;
+                    const uint8_t *m = p.mask + o;
+                    const size_t step = 4 * static_cast<size_t>(ldN);
+                    uint32_t drop[8];   // a byte is 0xff where the mask drops the value
+#pragma unroll
+                    for (int pass = 0; pass < 8; ++pass) {
+                        uint32_t word = p.maskKeeps ? 0x01010101u : 0u;
+                        if (p.mask && 4 * pass + at < count) {
+                            if (vectors) word = __ldg(reinterpret_cast<const uint32_t *>(m));
+                            else
+                                for (int e = 0; e < 4; ++e)
+                                    if (e < left) word = (word & ~(0xffu << (8 * e))) | static_cast<uint32_t>(__ldg(m + e)) << (8 * e);
+                        }
+                        drop[pass] = p.maskKeeps ? __vcmpeq4(word, 0u) : __vcmpne4(word, 0u);
+                        m += step;
+                    }
+                    float4 x[8];
+#pragma unroll
+                    for (int pass = 0; pass < 8; ++pass) x[pass] = mine[(4 * pass + at) * 8 + (i ^ ((4 * pass + at) & 7))];
+#pragma unroll
+                    for (int pass = 0; pass < 8; ++pass, to += step) {
+                        if (drop[pass] != 0u) {   // rare; a product with 0 keeps NaN and signs
+                            auto times = [&](float v, int e) { return drop[pass] >> (8 * e) & 1u ? v * 0.0f : v; };
+                            x[pass] = make_float4(times(x[pass].x, 0), times(x[pass].y, 1), times(x[pass].z, 2), times(x[pass].w, 3));
+                        }
+                        if (poison) x[pass] = make_float4(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000), __int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
+                        if (4 * pass + at >= count) continue;
+                        if (vectors) {
+                            *reinterpret_cast<float4 *>(to) = x[pass];
+                        } else {
+                            const float v[4] = {x[pass].x, x[pass].y, x[pass].z, x[pass].w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e)
+                                if (e < left) to[e] = v[e];
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            arrive(&accFree[acc.at]);   // the products of a later tile may overwrite the accumulator
+        }
+    } else if (warp == kGradientWarp) {
+        if (electOne()) {
+            Turn slot;
+            int issued = 0;
+            for (int tile = 0; tile < tiles && !failed; ++tile) {
+                const int boxes = boxesOf(tile), row = rowBegin + tile * kTileM;
+                for (int c = 0; c < chunks && !failed; ++c) {
+                    if (slot.again) wait(&rawFree[slot.at], slot.parity ^ 1u);
+                    if (failed) break;
+                    expect(&rawFull[slot.at], boxes * kBoxBytes);
+                    for (int b = 0; b < boxes; ++b)
+                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                                         smemAddr(raw + slot.at * kRawBytes + b * kBoxBytes)),
+                                     "l"(&gradients), "r"(c * kChunk), "r"(row + b * kBoxRows), "r"(smemAddr(&rawFull[slot.at]))
+                                     : "memory");
+                    ++issued;
+                    slot.step(s.ring);
+                }
+            }
+            for (int g = max(0, issued - s.ring); g < issued; ++g) waitPhase(smemAddr(&rawFull[g % s.ring]), (g / s.ring) & 1);   // nothing is left in flight
+        }
+    } else if (warp == kWeightWarp) {
+        if (STREAM && electOne()) {
+            Turn slot;
+            int issued = 0;
+            const uint8_t *first = static_cast<const uint8_t *>(p.packed) + static_cast<size_t>(blockIdx.y) * chunks * weightBytes;
+            for (int tile = 0; tile < tiles && !failed; ++tile) {
+                const uint8_t *src = first;
+                for (int c = 0; c < chunks && !failed; ++c, src += weightBytes) {
+                    if (slot.again) wait(&weightsFree[slot.at], slot.parity ^ 1u);
+                    if (failed) break;
+                    expect(&weightsFull[slot.at], weightBytes);
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                     smemAddr(weights + slot.at * weightBytes)),
+                                 "l"(src), "r"(weightBytes), "r"(smemAddr(&weightsFull[slot.at]))
+                                 : "memory");
+                    ++issued;
+                    slot.step(kWeightRing);
+                }
+            }
+            for (int g = max(0, issued - kWeightRing); g < issued; ++g) waitPhase(smemAddr(&weightsFull[g % kWeightRing]), (g / kWeightRing) & 1);
+        }
+    } else if (electOne()) {
+        const uint32_t idesc = instructionDescriptor(NP, false, false);
+        if (!STREAM) wait(&weightsFull[0], 0);
+        Turn stage, slot, acc;
+        for (int tile = 0; tile < tiles; ++tile, acc.step(s.accs)) {
+            if (acc.again) wait(&accFree[acc.at], acc.parity ^ 1u);
+            for (int c = 0; c < chunks; ++c) {
+                wait(&termsFull[stage.at], stage.parity);
+                if (STREAM) wait(&weightsFull[slot.at], slot.parity);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t descB = operandDescriptor(smemAddr(weights + (STREAM ? slot.at : c) * weightBytes), kCore, kGroupStride);
+                const uint32_t terms = stageBase + stage.at * kStageCols;
+#pragma unroll
+                for (int ks = 0; ks < kChunk / 16; ++ks)
+#pragma unroll
+                    for (int term = 0; term < 3; ++term)
+                        bwdcluster::mmaBf16TmemA(tmem + acc.at * NP, terms + term * (kChunk / 2) + 8 * ks, descB + static_cast<uint64_t>(ks * ((2 * kCore) >> 4)), idesc,
+                                                 (c > 0 || ks > 0 || term > 0) ? 1u : 0u);
+                commitTo(smemAddr(&termsFree[stage.at]));
+                if (STREAM) commitTo(smemAddr(&weightsFree[slot.at]));
+                if (c + 1 == chunks) commitTo(smemAddr(&accFull[acc.at]));
+                stage.step(s.stages);
+                if (STREAM) slot.step(kWeightRing);
+            }
+        }
+        // nothing is left in flight when tensor memory is given back
+        if (tiles > 0) waitPhase(smemAddr(&accFull[(tiles - 1) % s.accs]), ((tiles - 1) / s.accs) & 1);
+    }
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
-    }
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTmemCols) : "memory");
     if (tid == 0 && failed && p.status) atomicExch(p.status, 1);
 }
 
-template <int NP>
-void launchPadded(const Problem &prob, int sms, cudaStream_t st) {
-    const size_t smem = sharedBytes(prob.K, NP);
-    ensureDynamicSmem(reinterpret_cast<const void *>(inputGradUmma<NP>), smem);  // per device
-    const int slabs = (prob.N + NP - 1) / NP;
-    const int groups = (prob.rows + 7) / 8;
-    const int grid = std::max(1, std::min(std::max(1, sms / slabs), groups));
-    const int rowsPerCta = (groups + grid - 1) / grid * 8;
-    KernelTimer timer__("inputGradUmma", st);
-    inputGradUmma<NP><<<dim3(grid, slabs), kThreads, smem, st>>>(prob, rowsPerCta);
+// cuTensorMapEncodeTiled through the runtime's driver entry point (no link against the driver library).
+using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                 const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encodeTiled() {
+    static EncodeTiled fn = [] {
+        void *ptr = nullptr;
+        cudaDriverEntryPointQueryResult status = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &status) != cudaSuccess ||
+            status != cudaDriverEntryPointSuccess)
+            ptr = nullptr;
+        return reinterpret_cast<EncodeTiled>(ptr);
+    }();
+    return fn;
 }
+
+// [rows][K] floats in boxes of 32 rows x 32 floats with the 128-byte swizzle; rows beyond the tensor read as zero.
+// The x coordinate of every copy is a multiple of 32 floats.
+CUtensorMap gradientMap(const float *G, int rows, int K) {
+    CUtensorMap map;
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * sizeof(float)};
+    const cuuint32_t box[2] = {kChunk, kBoxRows};
+    const cuuint32_t elementStrides[2] = {1, 1};
+    const CUresult rc = encodeTiled()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(G), dims, strides, box, elementStrides,
+                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (rc != CUDA_SUCCESS) fail(RXMET_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", static_cast<int>(rc));
+    return map;
+}
+
+// Columns of a CTA: all of them up to 256, else even slabs.
+Shape shapeFor(int N) {
+    Shape s{};
+    s.slabs = (N + kMaxColumns - 1) / kMaxColumns;
+    s.NP = ((N + s.slabs - 1) / s.slabs + 15) / 16 * 16;
+    s.accs = s.NP <= 128 ? 2 : 1;
+    s.stages = std::min<int>(kMaxStages, (kTmemCols - s.accs * s.NP) / kStageCols);
+    return s;
+}
+size_t sharedBytes(const Shape &s, int K, bool stream, int ring) {
+    return 1024 + ring * static_cast<size_t>(kRawBytes) + kEpilogueWarps * 4096 + static_cast<size_t>(stream ? kWeightRing : K / kChunk) * s.NP * kChunk * 2 +
+           sizeof(float) * static_cast<size_t>(K);
+}
+// Weights stay in shared memory up to 64 columns where they leave room for a ring of four chunks.
+bool resident(int K, int N) { return N <= kResidentColumns && sharedBytes(shapeFor(N), K, false, 4) <= 225 * 1024; }
 
 }  // namespace
 
-bool wideTakes(int K, int N);
+size_t packedBytes(int K, int N) {
+    if (N < 1 || K < kChunk || K % kChunk != 0 || K > kMaxK || resident(K, N)) return 0;
+    const Shape s = shapeFor(N);
+    return static_cast<size_t>(s.slabs) * s.NP * K * 2;
+}
 
 bool eligible(int K, int N) {
     static const bool disabled = std::getenv("RXMET_IGRAD_SIMT") != nullptr;
-    if (disabled || N < 1) return false;
-    if (K >= kChunkK && K % kChunkK == 0 && K <= kMaxK) return true;
-    return wideTakes(K, N);   // only with Problem::packed
+    return !disabled && N >= 1 && K >= kChunk && K % kChunk == 0 && K <= kMaxK && encodeTiled() != nullptr;
 }
 
-bool wideTakes(int K, int N);
-bool wideEligible(const Problem &p);
-void launchWide(const Problem &prob, cudaStream_t st);
-
 void launch(const Problem &prob, int sms, cudaStream_t st) {
-    if (wideEligible(prob)) {
-        launchWide(prob, st);
-        return;
-    }
-    if (prob.K > kMaxK || prob.K % kChunkK != 0)
-        fail(RXMET_ERR_UNSUPPORTED, "input gradient: %d channels need the streaming kernel (scratch, 16-byte aligned operands)", prob.K);
-    // widest slab whose weight operand fits shared memory beside the stages and the ring
-    const int widest = prob.K <= 512 ? 64 : 32;
-    const int np = prob.N > widest ? widest : (prob.N + 15) / 16 * 16;
-    switch (np) {
-        case 16: launchPadded<16>(prob, sms, st); break;
-        case 32: launchPadded<32>(prob, sms, st); break;
-        case 48: launchPadded<48>(prob, sms, st); break;
-        case 64: launchPadded<64>(prob, sms, st); break;
-        default: fail(RXMET_ERR_UNSUPPORTED, "input gradient: %d columns", prob.N);
+    Problem p = prob;
+    const bool stream = !resident(p.K, p.N);
+    RXMET_REQUIRE(p.rows >= 1 && p.K % kChunk == 0 && p.K <= kMaxK && alignedTo(p.G, 16) && (!stream || (p.packed != nullptr && alignedTo(p.packed, 16))),
+                  "input gradient: %d channels, %d columns", p.K, p.N);
+    if (p.ldCodesKN == 0) p.ldCodesKN = p.N;
+    Shape s = shapeFor(p.N);
+    const size_t most = std::min<size_t>(225 * 1024, currentDevice().smemMax);
+    s.ring = kMaxRing;
+    while (s.ring > 2 && sharedBytes(s, p.K, stream, s.ring) > most) --s.ring;
+    const size_t smem = sharedBytes(s, p.K, stream, s.ring);
+    const int boxes = (p.rows + kBoxRows - 1) / kBoxRows, most1 = std::max(1, sms / s.slabs);
+    s.rowsPerCta = (boxes + most1 - 1) / most1 * kBoxRows;
+    const CUtensorMap map = gradientMap(p.G, p.rows, p.K);
+    const dim3 grid(static_cast<unsigned>((p.rows + s.rowsPerCta - 1) / s.rowsPerCta), static_cast<unsigned>(s.slabs));
+    KernelTimer timer__("inputGradUmma", st);
+    if (stream) {
+        const int items = p.K / 8 * s.NP * s.slabs;
+        packWeights<<<(items + 255) / 256, 256, 0, st>>>(p, s.NP, s.slabs, static_cast<uint4 *>(p.packed));
+        ensureDynamicSmem(reinterpret_cast<const void *>(inputGradUmma<true>), smem);
+        launchDependent(inputGradUmma<true>, grid, kThreads, smem, st, p, s, map);
+    } else {
+        ensureDynamicSmem(reinterpret_cast<const void *>(inputGradUmma<false>), smem);
+        launchDependent(inputGradUmma<false>, grid, kThreads, smem, st, p, s, map);
     }
 }
 

@@ -729,7 +729,7 @@ size_t tiledWorkspaceBytes(int T, int B, int I, int H, bool padded) {
     ws.take<float>(static_cast<size_t>(tensorSplitBound(static_cast<int>(rows), I, H, H, static_cast<int>(C), padded)) * (H + 1) * C);
     ws.take<int>(1);              // status word of the tensor-memory weight-gradient kernel
     ws.take<uint32_t>(rows * H);  // packed per-step clamp flags
-    ws.take<uint8_t>(igrad::widePackedBytes(static_cast<int>(C), I) + 256);   // weight operand of the streaming input-gradient kernel
+    ws.take<uint8_t>(igrad::packedBytes(static_cast<int>(C), I) + 256);   // weight operand of the input gradient
     return ws.used() + 1024;
 }
 
@@ -887,14 +887,14 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         else if (bt == 2) launch(recurrentBackward<2>, 2);
         else launch(recurrentBackward<1>, 1);
     }
-    if (call.quantized) RXMET_CUDA(cudaMemsetAsync(tensorStatus, 0, sizeof(int), st));
+    if (call.quantized && !tensorInputGrad) RXMET_CUDA(cudaMemsetAsync(tensorStatus, 0, sizeof(int), st));   // the input gradient clears it itself
     if (tensorInputGrad) {
         // QAT: gradients times the integer weight codes on the tensor cores, scales folded into the gradients
         const int sms = currentDevice().sms;
         igrad::Problem pg{};
         pg.G = gIh; pg.kScale = channelScales; pg.codesKN = call.weightIh; pg.rows = static_cast<int>(rows); pg.K = C; pg.N = call.dxColumns ? call.dxColumns : I;
-        pg.mask = static_cast<const uint8_t *>(mk.input); pg.maskKeeps = 0; pg.out = call.grads.input; pg.status = tensorStatus;
-        if (const size_t bytes = igrad::widePackedBytes(C, pg.N)) pg.packed = ws.take<uint8_t>(bytes);
+        pg.mask = static_cast<const uint8_t *>(mk.input); pg.maskKeeps = 0; pg.out = call.grads.input; pg.status = pg.clear = tensorStatus;
+        if (const size_t bytes = igrad::packedBytes(C, pg.N)) pg.packed = ws.take<uint8_t>(bytes);
         igrad::launch(pg, sms, st);
         afterLaunch("inputGradUmma");
     } else if (I <= 128 && C % 4 == 0) {

@@ -571,6 +571,15 @@ def test_packed_step_flags_equal_the_byte_masks(monkeypatch, shape):
     assert torch.equal(packed.flat_w, plain.flat_w) and torch.equal(lp, lb)
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 8, 32), (1, 31, 16, 32), (1, 33, 20, 96), (1, 127, 64, 64), (1, 129, 64, 160), (1, 160, 68, 96), (1, 130, 128, 32),
+                                   (2, 65, 132, 32), (1, 40, 256, 64), (1, 40, 260, 32), (1, 19500, 8, 32), (1, 9600, 72, 32), (1, 9600, 260, 32)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_input_gradient_tiles(gl, shape):
+    """Rows at the edges of boxes and tiles, an odd number of chunks over several tiles of a CTA, weights that stay and weights that are copied
+    chunk by chunk, one and two accumulators, two slabs of columns."""
+    test_backward_quant(gl, "w8a8", shape)
+
+
 @pytest.mark.parametrize("byte_masks", [False, True], ids=["packed", "bytes"])
 def test_time_chunked_step_equals_the_single_launch_step(monkeypatch, byte_masks):
     """The overlapped pipeline cuts the sequence into time chunks (projection / gradient GEMMs of one chunk under the
