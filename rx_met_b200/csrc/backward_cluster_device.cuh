@@ -23,6 +23,11 @@ __device__ __forceinline__ void tmemLoad(uint32_t addr, uint32_t (&r)[COUNT]) {
 __device__ __forceinline__ void tmemStore4(uint32_t addr, const uint4 &v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
+__device__ __forceinline__ void tmemStore8(uint32_t addr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
 // D += A B with A in tensor memory: lane = row of A, a 32-bit column holds two consecutive bf16 along K
 __device__ __forceinline__ void mmaBf16TmemA(uint32_t tmemD, uint32_t tmemA, uint64_t descB, uint32_t idesc, uint32_t accumulate) {
     asm volatile(

@@ -16,10 +16,10 @@ __device__ __forceinline__ void waitForPredecessor() { asm volatile("griddepcont
 __device__ __forceinline__ void letDependentsStart() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 template <class... Params, class... Args>
-void launchDependent(void (*kernel)(Params...), dim3 grid, int block, size_t smem, cudaStream_t stream, Args &&...args) {
+void launchDependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(static_cast<unsigned>(block));
+    cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr{};

@@ -20,6 +20,7 @@
 #include <cstdlib>
 
 #include "common.h"
+#include "dependent_launch.cuh"
 #include "gru_backward.h"
 #include "gru_backward_cluster.h"
 #include "regroup.h"
@@ -875,11 +876,12 @@ __global__ void __launch_bounds__(256, 2) weightGradMma(const WeightGradProblem 
 }
 
 // weight[m][n] = scale * mask * sum_s partial[s][m][n] (m < M); bias[n] = biasMask * sum_s partial[s][M][n].
-// A CTA owns 64 outputs; its four thread layers each sum every fourth split and layer 0 adds the
+// A CTA owns 256 outputs, four a thread; its four thread layers each sum every fourth split and layer 0 adds the
 // four sums in layer order, so the result does not depend on the launch.
 // A set status word (a bounded wait of the producing kernel gave up) turns the results into NaN.
 // One launch reduces both problems of a step (blockIdx.y: 0 = input weights, 1 = recurrent weights).
-constexpr int kReduceLayers = 4, kReduceWidth = 64;
+// Bound by memory: 16 bytes a load (8 splits of 768 x 768 outputs, 19 MB: 16.7 -> 11.3 us).
+constexpr int kReduceLayers = 4, kReduceWidth = 256;
 struct ReduceJob {
     const float *partial;
     int splits, M;
@@ -887,33 +889,41 @@ struct ReduceJob {
     const uint8_t *weightMask, *biasMask;
     float *weight, *bias;
 };
-__global__ void __launch_bounds__(kReduceWidth * kReduceLayers)
+__global__ void __launch_bounds__(kReduceWidth / 4 * kReduceLayers)
 reduceWeightGrad(const ReduceJob jobX, const ReduceJob jobH, int N, const int *__restrict__ status) {
-    __shared__ float layer[kReduceLayers][kReduceWidth];
+    __shared__ float4 layer[kReduceLayers][kReduceWidth / 4];
     const ReduceJob &job = blockIdx.y == 0 ? jobX : jobH;
-    const float *__restrict__ partial = job.partial;
     const int splits = job.splits, M = job.M;
-    const float scale = job.scale;
-    const uint8_t *__restrict__ weightMask = job.weightMask, *__restrict__ biasMask = job.biasMask;
-    float *__restrict__ weight = job.weight, *__restrict__ bias = job.bias;
-    const size_t total = static_cast<size_t>(M + 1) * N;
+    const size_t total = static_cast<size_t>(M + 1) * N;   // a multiple of four, as N is
+    waitForPredecessor();
     if (static_cast<size_t>(blockIdx.x) * kReduceWidth >= total) return;  // the other problem is larger
-    const size_t i = static_cast<size_t>(blockIdx.x) * kReduceWidth + threadIdx.x;
-    float s = 0.0f;
+    const size_t i = static_cast<size_t>(blockIdx.x) * kReduceWidth + 4 * threadIdx.x;
+    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto add = [](float4 &a, const float4 &b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
     if (i < total) {
+        const float4 *from = reinterpret_cast<const float4 *>(job.partial + i);
 #pragma unroll 4
-        for (int sp = threadIdx.y; sp < splits; sp += kReduceLayers) s += partial[static_cast<size_t>(sp) * total + i];
+        for (int sp = threadIdx.y; sp < splits; sp += kReduceLayers) add(s, __ldcs(from + static_cast<size_t>(sp) * (total / 4)));
     }
     layer[threadIdx.y][threadIdx.x] = s;
     __syncthreads();
     if (threadIdx.y != 0 || i >= total) return;
     s = layer[0][threadIdx.x];
 #pragma unroll
-    for (int l = 1; l < kReduceLayers; ++l) s += layer[l][threadIdx.x];
-    if (status && *status) s = __int_as_float(0x7fc00000);
-    const size_t m = i / N, n = i % N;
-    if (m < static_cast<size_t>(M)) weight[i] = s * scale * keepOf(weightMask, i);
-    else bias[n] = s * keepOf(biasMask, n);
+    for (int l = 1; l < kReduceLayers; ++l) add(s, layer[l][threadIdx.x]);
+    if (status && *status) s.x = s.y = s.z = s.w = __int_as_float(0x7fc00000);
+    const bool bias = i >= total - N;   // four outputs are of one row
+    const size_t o = bias ? i - (total - N) : i;
+    const uint8_t *mask = bias ? job.biasMask : job.weightMask;
+    const float scale = bias ? 1.0f : job.scale;
+    float *to = (bias ? job.bias : job.weight) + o;
+    const float v[4] = {s.x * scale * keepOf(mask, o), s.y * scale * keepOf(mask, o + 1), s.z * scale * keepOf(mask, o + 2), s.w * scale * keepOf(mask, o + 3)};
+    if ((reinterpret_cast<uintptr_t>(to) & 15) == 0) {
+        *reinterpret_cast<float4 *>(to) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) to[e] = v[e];
+    }
 }
 
 // out[i] = mask[i] * sum_s partial[s][i], s ascending.
@@ -997,16 +1007,10 @@ constexpr int kBiasSplits = 64;
 
 namespace wgrad {
 
-constexpr int kMaxSms = 160;
-
 Plan plan(int K, int M, int N, int sms) {
+    (void)M;
     Plan pl;
     sms = std::min(sms, kMaxSms);
-    pl.tensorMemory = tensorMemoryPath(M, N);
-    if (pl.tensorMemory) {
-        pl.splits = planTensorMemory(K, N, sms, &pl.chunkK);
-        return pl;
-    }
     const int nTiles = (N + gru::kWgCols - 1) / gru::kWgCols;
     const int splits = std::max(1, std::min((2 * sms + 2 * nTiles - 1) / (2 * nTiles), (K + 255) / 256));
     pl.chunkK = ((K + splits - 1) / splits + gru::kWgChunk - 1) / gru::kWgChunk * gru::kWgChunk;
@@ -1015,16 +1019,12 @@ Plan plan(int K, int M, int N, int sms) {
 }
 
 int splitBound(int K, int M, int N) {
-    // both kernels ask for about two CTAs per SM spread over the column tiles
+    // about two CTAs per SM spread over the column tiles
     (void)M;
     return std::max(1, std::min((K + gru::kWgChunk - 1) / gru::kWgChunk, 2 * kMaxSms + 8));
 }
 
 void launch(const Problem &prob, int K, int N, const Plan &pl, cudaStream_t st) {
-    if (pl.tensorMemory) {
-        launchTensorMemory(prob, nullptr, K, N, pl.chunkK, pl.splits, st);
-        return;
-    }
     const int chunkK = pl.chunkK;
     const int mt = (prob.M + 1 + 15) / 16;
     const dim3 grid((N + gru::kWgCols - 1) / gru::kWgCols, pl.splits);
@@ -1036,18 +1036,6 @@ void launch(const Problem &prob, int K, int N, const Plan &pl, cudaStream_t st) 
 #undef RXMET_WG_CASE
         default: fail(RXMET_ERR_UNSUPPORTED, "weight gradient tile count %d", mt);
     }
-}
-
-void launchPair(const Problem &a, const Plan &planA, const Problem &b, const Plan &planB, int K, int N, cudaStream_t st) {
-    if (planA.tensorMemory && planB.tensorMemory && planA.splits == planB.splits && planA.chunkK == planB.chunkK &&
-        a.status == b.status) {
-        if (launchPairStreamed(a, b, K, N, planA.chunkK, planA.splits, st)) return;
-        const bool aFirst = a.M >= b.M;
-        launchTensorMemory(aFirst ? a : b, aFirst ? &b : &a, K, N, planA.chunkK, planA.splits, st);
-        return;
-    }
-    launch(a, K, N, planA, st);
-    launch(b, K, N, planB, st);
 }
 
 }  // namespace wgrad
@@ -1180,11 +1168,12 @@ size_t tiledWorkspaceBytes(int T, int B, int I, int H, bool padded) {
     ws.take<float>(splitR * H * C);
     ws.take<float>(2 * kBiasSplits * C);
     // tensor-core path: split-K partials of (I+1) and (H+1) rows and the status word
-    // (the slab form of the same kernel, for more than 128 rows or 16-bit codes, asks for fewer splits)
-    ws.take<float>(static_cast<size_t>(std::max({padded ? wgrad::chainPartials(static_cast<int>(rows)) : 1, wgrad::slabSplitBound(I, H, static_cast<int>(C)),
-                                                I <= 143 ? wgrad::splitBound(static_cast<int>(rows), I, static_cast<int>(C)) : 1})) * (I + 1) * C);
-    ws.take<float>(static_cast<size_t>(std::max({padded ? wgrad::chainPartials(static_cast<int>(rows)) : 1, wgrad::slabSplitBound(I, H, static_cast<int>(C)),
-                                                H <= 143 ? wgrad::splitBound(static_cast<int>(rows), H, static_cast<int>(C)) : 1})) * (H + 1) * C);
+    auto partials = [&](int M) {
+        const int c = static_cast<int>(C), most = std::max(wgrad::tileSplitBound(M, c), M <= 143 ? wgrad::splitBound(static_cast<int>(rows), M, c) : 1);
+        ws.take<float>(static_cast<size_t>(std::max(padded ? wgrad::chainPartials(static_cast<int>(rows)) : 1, most)) * (M + 1) * C);
+    };
+    partials(I);
+    partials(H);
     ws.take<int>(64);
     ws.take<float>(static_cast<size_t>(B) * H);   // gradient carried between time chunks
     ws.take<uint8_t>(igrad::packedBytes(static_cast<int>(C), I) + 256);   // weight operand of the input gradient
@@ -1239,11 +1228,10 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
     const bool tensorGrads = qat && call.exec->actClass == CodeClass::I8 && I + 1 <= 144 && H + 1 <= 144 && I % 4 == 0 &&
                              H % 4 == 0 && !simtGrads && alignedTo(call.x_q, 16) && alignedTo(call.h, 16) &&
                              (!padded || std::max(I, H) <= 128);   // one kernel for both arrays
-    // More than 128 rows or 16-bit activation codes: the same tcgen05 kernel over 128-row slabs, two exact
-    // bf16 terms per code when the grid is wider than 8 bits.
+    // More than 128 rows or 16-bit activation codes: the tcgen05 kernel only, two exact bf16 terms per code when the grid is wider than 8 bits.
     const bool wideCodes = qat && call.exec->actClass != CodeClass::I8;
     const bool slabGrads = qat && !tensorGrads && !simtGrads && call.exec->actClass != CodeClass::I32 && I % 4 == 0 && H % 4 == 0 &&
-                           alignedTo(call.x_q, 16) && alignedTo(call.h, 16) && wgrad::slabPathTakes(I, H, C);
+                           alignedTo(call.x_q, 16) && alignedTo(call.h, 16) && wgrad::tensorMemoryPath(I, H, C);
 
     const float *W = call.W, *R = call.R, *x = call.x;
     const float *chanScaleR = nullptr, *chanScaleW = nullptr;
@@ -1387,21 +1375,20 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         if (mmaPath && tensorInputGrad && tensorGrads && (static_cast<size_t>(B) * I) % 8 == 0 &&
             !padded)   // the chunks' launches know one width of dx and no chunks of rows
             chunks = overlapChunks(T, rows, true);
-        std::vector<wgrad::Plan> plans;
-        int totalSplits = 0;
+        std::vector<wgrad::PairPlan> plans;
+        int splits[2] = {0, 0};
         if (chunks.size() > 1) {
             int share = 100;
             if (const char *env = std::getenv("RXMET_GRU_CHUNK_SMS")) share = std::max(5, std::min(100, std::atoi(env)));
-            for (size_t i = 0; i < chunks.size(); ++i) {
-                const int K = chunks[i] * B;
-                const int use = (i + 1 == chunks.size()) ? sms : std::max(4, sms * share / 100);
-                const wgrad::Plan px = wgrad::plan(K, I, C, use), ph = wgrad::plan(K, H, C, use);
-                if (!px.tensorMemory || !ph.tensorMemory || px.splits != ph.splits || px.chunkK != ph.chunkK) { plans.clear(); break; }
-                plans.push_back(px);
-                totalSplits += px.splits;
+            WeightGradProblem px{}, ph{};
+            px.M = I; ph.M = H;
+            for (size_t i = 0; i < chunks.size() && wgrad::tensorMemoryPath(I, H, C); ++i) {
+                plans.push_back(wgrad::planPair(px, ph, chunks[i] * B, C, false, i + 1 == chunks.size() ? sms : std::max(4, sms * share / 100)));
+                for (int k = 0; k < 2; ++k) splits[k] += plans.back().splits[k];
             }
-            const int bound = std::min(wgrad::splitBound(static_cast<int>(rows), I, C), wgrad::splitBound(static_cast<int>(rows), H, C));
-            if (plans.size() != chunks.size() || totalSplits > bound) chunks.assign(1, T);
+            const bool room = splits[0] <= std::max(wgrad::tileSplitBound(I, C), wgrad::splitBound(static_cast<int>(rows), I, C)) &&
+                              splits[1] <= std::max(wgrad::tileSplitBound(H, C), wgrad::splitBound(static_cast<int>(rows), H, C));
+            if (plans.size() != chunks.size() || !room) chunks.assign(1, T);
         }
         if (chunks.size() > 1) {
             const Exec &e = *call.exec;
@@ -1409,11 +1396,11 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
             float *carry = ws.take<float>(static_cast<size_t>(B) * H);
             int *status = ws.take<int>(1);
             RXMET_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
-            float *partialX = ws.take<float>(static_cast<size_t>(totalSplits) * (I + 1) * C);
-            float *partialH = ws.take<float>(static_cast<size_t>(totalSplits) * (H + 1) * C);
+            float *partialX = ws.take<float>(static_cast<size_t>(splits[0]) * (I + 1) * C);
+            float *partialH = ws.take<float>(static_cast<size_t>(splits[1]) * (H + 1) * C);
             uint8_t *packedW = nullptr;
             if (const size_t bytes = igrad::packedBytes(C, I)) packedW = ws.take<uint8_t>(bytes);
-            int tEnd = T, splitBase = 0;
+            int tEnd = T;
             for (size_t i = 0; i < chunks.size(); ++i) {
                 const int n = chunks[i], t0 = tEnd - n;
                 const size_t r0 = static_cast<size_t>(t0) * B;
@@ -1439,24 +1426,25 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
                 afterLaunch("inputGradUmma");
                 WeightGradProblem px{}, ph{};
                 px.aCodes = call.x_q + r0 * I; px.aZero = e.gate.zp[RXMET_GRU_X]; px.M = I; px.B = dp + r0 * C;
-                px.partial = partialX + static_cast<size_t>(splitBase) * (I + 1) * C;
+                px.partial = partialX;
                 ph.aFloat = call.h + r0 * H; ph.aInvScale = 1.0f / e.gate.eff[RXMET_GRU_H]; ph.M = H; ph.B = dq + r0 * C;
-                ph.partial = partialH + static_cast<size_t>(splitBase) * (H + 1) * C;
+                ph.partial = partialH;
                 px.status = ph.status = status;
-                wgrad::launchPair(px, plans[i], ph, plans[i], K, C, lane.stream);
+                wgrad::launchPair(px, ph, K, C, plans[i], false, lane.stream);
                 afterLaunch("weightGrad");
-                splitBase += plans[i].splits;
+                partialX += static_cast<size_t>(plans[i].splits[0]) * (I + 1) * C;
+                partialH += static_cast<size_t>(plans[i].splits[1]) * (H + 1) * C;
                 tEnd = t0;
             }
             RXMET_CUDA(cudaEventRecord(lane.done[0], lane.stream));
             RXMET_CUDA(cudaStreamWaitEvent(st, lane.done[0], 0));
             {
-                const ReduceJob jobX{partialX, totalSplits, I, e.gate.eff[RXMET_GRU_X], mk.W, mk.bw, call.dW, call.dbw};
-                const ReduceJob jobH{partialH, totalSplits, H, e.gate.eff[RXMET_GRU_H], mk.R, mk.br, call.dR, call.dbr};
+                const ReduceJob jobX{partialX - static_cast<size_t>(splits[0]) * (I + 1) * C, splits[0], I, e.gate.eff[RXMET_GRU_X], mk.W, mk.bw, call.dW, call.dbw};
+                const ReduceJob jobH{partialH - static_cast<size_t>(splits[1]) * (H + 1) * C, splits[1], H, e.gate.eff[RXMET_GRU_H], mk.R, mk.br, call.dR, call.dbr};
                 const size_t largest = static_cast<size_t>(std::max(I, H) + 1) * C;
                 KernelTimer timer__("reduceWeightGrad", st);
-                reduceWeightGrad<<<dim3(static_cast<unsigned>((largest + kReduceWidth - 1) / kReduceWidth), 2),
-                                   dim3(kReduceWidth, kReduceLayers), 0, st>>>(jobX, jobH, C, status);
+                launchDependent(reduceWeightGrad, dim3(static_cast<unsigned>((largest + kReduceWidth - 1) / kReduceWidth), 2), dim3(kReduceWidth / 4, kReduceLayers), 0, st,
+                                jobX, jobH, C, status);
             }
             afterLaunch("reduceWeightGrad");
             return;
@@ -1523,71 +1511,43 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         afterLaunch("gemmNT");
     }
     // dW, dR, dbw, dbr
-    if (tensorGrads) {
+    if (tensorGrads || slabGrads) {
         const Exec &e = *call.exec;
         const int K = static_cast<int>(rows);
-        // the two problems share one launch of one CTA per SM: each is planned for half of the SMs, so that the
-        // launch is a single wave (RXMET_WGRAD_FULL_SPLIT plans each for all SMs, two waves)
-        const int planSms = std::getenv("RXMET_WGRAD_FULL_SPLIT") ? sms : std::max(1, sms / 2);
-        const wgrad::Plan planX = wgrad::plan(K, I, C, planSms), planH = wgrad::plan(K, H, C, planSms);
-        const bool chain = padded && planX.tensorMemory && planH.tensorMemory && planX.chunkK > wgrad::kChainRows;
-        int splitsX = planX.splits, splitsH = planH.splits;
         WeightGradProblem px{}, ph{};
         px.aCodes = call.x_q; px.aZero = e.gate.zp[RXMET_GRU_X]; px.M = I; px.B = dp;
-        px.partial = ws.take<float>(static_cast<size_t>(chain ? wgrad::chainPartials(K) : splitsX) * (I + 1) * C);
         ph.aFloat = call.h; ph.aInvScale = 1.0f / e.gate.eff[RXMET_GRU_H]; ph.M = H; ph.B = dq;
-        ph.partial = ws.take<float>(static_cast<size_t>(chain ? wgrad::chainPartials(K) : splitsH) * (H + 1) * C);
         px.status = ph.status = status;
-        if (chain) {
-            splitsX = splitsH = wgrad::chained(px, ph, K, C, st, [&](const WeightGradProblem &a, const WeightGradProblem &b, int n, int chunks) {
-                const wgrad::Plan plan{chunks, wgrad::kChainRows, true};
-                wgrad::launchPair(a, plan, b, plan, n, C, st);
-                afterLaunch("weightGrad");
-            });
-        } else {
-            wgrad::launchPair(px, planX, ph, planH, K, C, st);
-            afterLaunch("weightGrad");
+        int splitsX, splitsH;
+        auto room = [&](int nx, int nh) {
+            splitsX = nx;
+            splitsH = nh;
+            px.partial = ws.take<float>(static_cast<size_t>(nx) * (I + 1) * C);
+            ph.partial = ws.take<float>(static_cast<size_t>(nh) * (H + 1) * C);
+        };
+        if (wgrad::tensorMemoryPath(I, H, C)) {
+            const wgrad::PairPlan plan = wgrad::planPair(px, ph, K, C, wideCodes, sms);
+            if (padded && wgrad::planRows(plan) > wgrad::kChainRows) {
+                room(wgrad::chainPartials(K), wgrad::chainPartials(K));
+                splitsX = splitsH = wgrad::launchChained(px, ph, K, C, wideCodes, st);
+            } else {
+                room(plan.splits[0], plan.splits[1]);
+                wgrad::launchPair(px, ph, K, C, plan, wideCodes, st);
+            }
+        } else {   // tensorGrads: both at most 143
+            const wgrad::Plan planX = wgrad::plan(K, I, C, std::max(1, sms / 2)), planH = wgrad::plan(K, H, C, std::max(1, sms / 2));
+            room(planX.splits, planH.splits);
+            wgrad::launch(px, K, C, planX, st);
+            wgrad::launch(ph, K, C, planH, st);
         }
+        afterLaunch("weightGrad");
         {
             const ReduceJob jobX{px.partial, splitsX, I, e.gate.eff[RXMET_GRU_X], mk.W, mk.bw, call.dW, call.dbw};
             const ReduceJob jobH{ph.partial, splitsH, H, e.gate.eff[RXMET_GRU_H], mk.R, mk.br, call.dR, call.dbr};
             const size_t largest = static_cast<size_t>(std::max(I, H) + 1) * C;
             KernelTimer timer__("reduceWeightGrad", st);
-            reduceWeightGrad<<<dim3(static_cast<unsigned>((largest + kReduceWidth - 1) / kReduceWidth), 2),
-                               dim3(kReduceWidth, kReduceLayers), 0, st>>>(jobX, jobH, C, status);
-        }
-        afterLaunch("reduceWeightGrad");
-        return;
-    }
-    if (slabGrads) {
-        const Exec &e = *call.exec;
-        const int K = static_cast<int>(rows);
-        int chunkK = 0;
-        int splits = wgrad::slabSplits(K, I, H, C, sms, &chunkK);
-        const bool chain = padded && chunkK > wgrad::kChainRows;
-        const int partials = chain ? wgrad::chainPartials(K) : splits;
-        WeightGradProblem px{}, ph{};
-        px.aCodes = call.x_q; px.aZero = e.gate.zp[RXMET_GRU_X]; px.M = I; px.B = dp;
-        px.partial = ws.take<float>(static_cast<size_t>(partials) * (I + 1) * C);
-        ph.aFloat = call.h; ph.aInvScale = 1.0f / e.gate.eff[RXMET_GRU_H]; ph.M = H; ph.B = dq;
-        ph.partial = ws.take<float>(static_cast<size_t>(partials) * (H + 1) * C);
-        px.status = ph.status = status;
-        if (chain) {
-            splits = wgrad::chained(px, ph, K, C, st, [&](const WeightGradProblem &a, const WeightGradProblem &b, int n, int chunks) {
-                wgrad::launchSlabs(a, b, n, C, wgrad::kChainRows, chunks, wideCodes, st);
-                afterLaunch("weightGrad");
-            });
-        } else {
-            wgrad::launchSlabs(px, ph, K, C, chunkK, splits, wideCodes, st);
-            afterLaunch("weightGrad");
-        }
-        {
-            const ReduceJob jobX{px.partial, splits, I, e.gate.eff[RXMET_GRU_X], mk.W, mk.bw, call.dW, call.dbw};
-            const ReduceJob jobH{ph.partial, splits, H, e.gate.eff[RXMET_GRU_H], mk.R, mk.br, call.dR, call.dbr};
-            const size_t largest = static_cast<size_t>(std::max(I, H) + 1) * C;
-            KernelTimer timer__("reduceWeightGrad", st);
-            reduceWeightGrad<<<dim3(static_cast<unsigned>((largest + kReduceWidth - 1) / kReduceWidth), 2),
-                               dim3(kReduceWidth, kReduceLayers), 0, st>>>(jobX, jobH, C, status);
+            launchDependent(reduceWeightGrad, dim3(static_cast<unsigned>((largest + kReduceWidth - 1) / kReduceWidth), 2), dim3(kReduceWidth / 4, kReduceLayers), 0, st,
+                            jobX, jobH, C, status);
         }
         afterLaunch("reduceWeightGrad");
         return;

@@ -2,7 +2,7 @@
 //
 // A CTA walks a contiguous range of rows in tiles of 128 rows (= the lanes of tensor memory) and, with more than 256 columns, one slab
 // of columns.  The accumulator D[128][NP] of a tile sums over K in chunks of 32 channels.  Warps by role:
-//   gradients   one lane copies a chunk's rows as TMA boxes of 32 rows x 128 bytes (128-byte swizzle) into a ring
+//   gradients   copies a chunk's rows as TMA boxes of 32 rows x 128 bytes (128-byte swizzle), one a lane, into a ring
 //   converters  sixteen warps, two groups that take chunks in turn: thread = row and sixteen channels; reads its pieces, scales them,
 //               splits them into three bf16 terms that carry all 24 bits and stores these to its own tensor-memory lane
 //   weights     up to 64 columns the codes, exact in bf16, are converted once per CTA and stay in shared memory; beyond, packWeights lays
@@ -18,8 +18,6 @@
 // whole tiles (two rounds where a CTA has 173 rows) and left the epilogue outside.  In a step, with what surrounds the kernel: 25,600 rows x 384 -> 40
 // columns 26.8 -> 23.7 us, 25,600 x 512 -> 40 31.7 -> 26.1, 12,800 x 768 -> 40 41.4 -> 24.7, 256,000 x 2048 -> 256 943 -> 707; by itself, back to back, 17, 21, 18 us
 // and 12,800 x 768 -> 512 59 -> 40.
-#include <cuda.h>
-
 #include <algorithm>
 #include <cstdlib>
 
@@ -27,6 +25,7 @@
 #include "common.h"
 #include "dependent_launch.cuh"
 #include "input_grad_umma.h"
+#include "tensor_map.cuh"
 #include "umma_device.cuh"
 
 namespace rxmet {
@@ -35,12 +34,12 @@ namespace {
 
 using namespace umma;
 
-constexpr int kChunk = 32;                                     // channels: two k-steps
+constexpr int kChunk = kBoxCols;                               // channels: two k-steps
 constexpr int kConvWarps = 16, kEpilogueWarps = 8, kFillWarps = kConvWarps + kEpilogueWarps;
 constexpr int kGradientWarp = kFillWarps, kWeightWarp = kFillWarps + 1, kProductWarp = kFillWarps + 2;
 constexpr int kThreads = 32 * (kProductWarp + 1);
-constexpr int kBoxRows = 32, kMaxRing = 6, kMaxStages = 8, kWeightRing = 4;
-constexpr uint32_t kBoxBytes = kBoxRows * kChunk * 4, kRawBytes = kTileM / kBoxRows * kBoxBytes;   // 4 KB, 16 KB
+constexpr int kMaxRing = 6, kMaxStages = 8, kWeightRing = 4;
+constexpr uint32_t kRawBytes = kTileM / kBoxRows * kBoxBytes;   // 16 KB
 constexpr uint32_t kStageCols = 3 * kChunk / 2;               // tensor-memory columns of a chunk: three terms, two channels a column
 constexpr uint32_t kGroupStride = kChunk / 8 * kCore;          // weights: next eight columns
 constexpr uint32_t kTmemCols = 512;
@@ -91,44 +90,6 @@ __global__ void packWeights(const Problem p, int NP, int slabs, uint4 *packed) {
     row.load(p, n, 8 * k8);
     packed[static_cast<size_t>(slab) * groups * NP + rowPlace(n - slab * NP, k8, NP)] = row.packed();
 }
-
-__device__ __forceinline__ bool testPhase(uint32_t bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return done != 0;
-}
-
-template <int N>
-__device__ __forceinline__ void tmemStore(uint32_t addr, const uint32_t (&v)[N]) {
-    static_assert(N == 8, "a k-step of one row");
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]),
-                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-                 : "memory");
-}
-
-// Walks a ring of mbarriers: place and phase parity of the current use.  Counters, not divisions: a division by a value known at run time costs
-// a lone thread more than issuing the products of a chunk.
-struct Turn {
-    int at = 0;
-    uint32_t parity = 0;
-    bool again = false;   // the place was used before
-    __device__ __forceinline__ void step(int size, int by = 1) {
-        at += by;
-        if (at >= size) {
-            at -= size;
-            parity ^= 1u;
-            again = true;
-        }
-    }
-};
 
 template <bool STREAM>   // weights chunk by chunk
 __global__ void __launch_bounds__(kThreads, 1)
@@ -244,7 +205,7 @@ inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s
                         v[2 * i] -= bf16Lo(w[i]);
                         v[2 * i + 1] -= bf16Hi(w[i]);
                     }
-                    tmemStore(to + term * (kChunk / 2), w);
+                    bwdcluster::tmemStore8(to + term * (kChunk / 2), w);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -330,26 +291,21 @@ inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s
             arrive(&accFree[acc.at]);   // the products of a later tile may overwrite the accumulator
         }
     } else if (warp == kGradientWarp) {
-        if (electOne()) {
-            Turn slot;
-            int issued = 0;
-            for (int tile = 0; tile < tiles && !failed; ++tile) {
-                const int boxes = boxesOf(tile), row = rowBegin + tile * kTileM;
-                for (int c = 0; c < chunks && !failed; ++c) {
-                    if (slot.again) wait(&rawFree[slot.at], slot.parity ^ 1u);
-                    if (failed) break;
-                    expect(&rawFull[slot.at], boxes * kBoxBytes);
-                    for (int b = 0; b < boxes; ++b)
-                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                                         smemAddr(raw + slot.at * kRawBytes + b * kBoxBytes)),
-                                     "l"(&gradients), "r"(c * kChunk), "r"(row + b * kBoxRows), "r"(smemAddr(&rawFull[slot.at]))
-                                     : "memory");
-                    ++issued;
-                    slot.step(s.ring);
-                }
+        Turn slot;
+        int issued = 0;
+        for (int tile = 0; tile < tiles && !failed; ++tile) {
+            const int boxes = boxesOf(tile), row = rowBegin + tile * kTileM + lane * kBoxRows;
+            for (int c = 0; c < chunks && !failed; ++c) {
+                if (slot.again) wait(&rawFree[slot.at], slot.parity ^ 1u);
+                if (__any_sync(0xffffffffu, failed)) break;
+                if (lane == 0) expect(&rawFull[slot.at], boxes * kBoxBytes);
+                __syncwarp();
+                if (lane < boxes) copyBox(smemAddr(raw + slot.at * kRawBytes + lane * kBoxBytes), &gradients, c * kChunk, row, smemAddr(&rawFull[slot.at]));
+                ++issued;
+                slot.step(s.ring);
             }
-            for (int g = max(0, issued - s.ring); g < issued; ++g) waitPhase(smemAddr(&rawFull[g % s.ring]), (g / s.ring) & 1);   // nothing is left in flight
         }
+        for (int g = max(0, issued - s.ring); g < issued; ++g) waitPhase(smemAddr(&rawFull[g % s.ring]), (g / s.ring) & 1);   // nothing is left in flight
     } else if (warp == kWeightWarp) {
         if (STREAM && electOne()) {
             Turn slot;
@@ -396,6 +352,7 @@ inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s
                 if (STREAM) slot.step(kWeightRing);
             }
         }
+        letDependentsStart();   // the kernel behind this one is launched under the last products and the epilogue
         // nothing is left in flight when tensor memory is given back
         if (tiles > 0) waitPhase(smemAddr(&accFull[(tiles - 1) % s.accs]), ((tiles - 1) / s.accs) & 1);
     }
@@ -404,37 +361,6 @@ inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTmemCols) : "memory");
     if (tid == 0 && failed && p.status) atomicExch(p.status, 1);
-}
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link against the driver library).
-using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                 const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiled encodeTiled() {
-    static EncodeTiled fn = [] {
-        void *ptr = nullptr;
-        cudaDriverEntryPointQueryResult status = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &status) != cudaSuccess ||
-            status != cudaDriverEntryPointSuccess)
-            ptr = nullptr;
-        return reinterpret_cast<EncodeTiled>(ptr);
-    }();
-    return fn;
-}
-
-// [rows][K] floats in boxes of 32 rows x 32 floats with the 128-byte swizzle; rows beyond the tensor read as zero.
-// The x coordinate of every copy is a multiple of 32 floats.
-CUtensorMap gradientMap(const float *G, int rows, int K) {
-    CUtensorMap map;
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * sizeof(float)};
-    const cuuint32_t box[2] = {kChunk, kBoxRows};
-    const cuuint32_t elementStrides[2] = {1, 1};
-    const CUresult rc = encodeTiled()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(G), dims, strides, box, elementStrides,
-                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (rc != CUDA_SUCCESS) fail(RXMET_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", static_cast<int>(rc));
-    return map;
 }
 
 // Columns of a CTA: all of them up to 256, else even slabs.
@@ -479,7 +405,7 @@ void launch(const Problem &prob, int sms, cudaStream_t st) {
     const size_t smem = sharedBytes(s, p.K, stream, s.ring);
     const int boxes = (p.rows + kBoxRows - 1) / kBoxRows, most1 = std::max(1, sms / s.slabs);
     s.rowsPerCta = (boxes + most1 - 1) / most1 * kBoxRows;
-    const CUtensorMap map = gradientMap(p.G, p.rows, p.K);
+    const CUtensorMap map = boxMap(p.G, p.rows, p.K, CU_TENSOR_MAP_SWIZZLE_128B);
     const dim3 grid(static_cast<unsigned>((p.rows + s.rowsPerCta - 1) / s.rowsPerCta), static_cast<unsigned>(s.slabs));
     KernelTimer timer__("inputGradUmma", st);
     if (stream) {

@@ -20,6 +20,7 @@
 #include <cstring>
 
 #include "common.h"
+#include "dependent_launch.cuh"
 #include "input_grad_umma.h"
 #include "lstm_backward_cluster.h"
 #include "lstm_kernels.h"
@@ -487,6 +488,7 @@ reduceWeightGradT(const ReduceJob jobIh, const ReduceJob jobHh, int C, const int
     const float scale = job.scale;
     const uint8_t *__restrict__ weightMask = job.weightMask, *__restrict__ biasMask = job.biasMask;
     float *__restrict__ weight = job.weight, *__restrict__ bias = job.bias;
+    waitForPredecessor();
     if (static_cast<int>(blockIdx.y) * kReduceRows > M) return;  // the other problem has more rows
     const size_t slab = static_cast<size_t>(M + 1) * C;
     const int c = blockIdx.x * 32 + threadIdx.x, m = blockIdx.y * kReduceRows + threadIdx.y;
@@ -591,11 +593,10 @@ constexpr int kMaxTensorSplits = 40;
 
 }  // namespace
 
-// Splits of the tensor-core weight-gradient partial arrays: the one-tile plan for at most 128 rows, the slab plan
-// (128-row slabs of both problems in one launch) beyond.
+// Splits of the tensor-core weight-gradient partial arrays.
 int tensorSplitBound(int rows, int I, int H, int M, int C, bool padded) {
     const int single = M <= 143 ? wgrad::splitBound(rows, M, C) : 1;
-    return std::max({single, padded ? wgrad::chainPartials(rows) : 1, wgrad::slabPathTakes(I, H, C) ? wgrad::slabSplitBound(I, H, C) : 1});
+    return std::max({single, padded ? wgrad::chainPartials(rows) : 1, wgrad::tensorMemoryPath(I, H, C) ? wgrad::tileSplitBound(M, C) : 1});
 }
 
 namespace {
@@ -919,46 +920,66 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         }
         afterLaunch("lstmGemmNN");
     }
-    // QAT on 8-bit activation grids: x and h_prev are integer codes, which the tensor-core GEMM
-    // multiplies exactly; its ones row also yields the bias gradients.
-    if (call.quantized && call.codesFitTensorPath && I % 4 == 0 && H % 4 == 0 && I <= 140 && H <= 140 &&
-        (!padded || std::max(I, H) <= 128) &&   // chunks of rows: one kernel for both arrays
-        alignedTo(call.x, 16)) {
-        const size_t stateBytes = sizeof(float) * static_cast<size_t>(B) * H;
-        if (call.h0) RXMET_CUDA(cudaMemcpyAsync(hPrev, call.h0, stateBytes, cudaMemcpyDeviceToDevice, st));
-        else RXMET_CUDA(cudaMemsetAsync(hPrev, 0, stateBytes, st));
-        if (T > 1)
-            RXMET_CUDA(cudaMemcpyAsync(hPrev + static_cast<size_t>(B) * H, call.hiddenOutputs, stateBytes * (T - 1),
-                                       cudaMemcpyDeviceToDevice, st));
-        const int sms = currentDevice().sms;
-        auto planFor = [&](int M) {
-            wgrad::Plan pl = wgrad::plan(static_cast<int>(rows), M, C, sms);
-            if (!pl.tensorMemory && pl.splits > kMaxTensorSplits) {
-                pl.chunkK = ((static_cast<int>(rows) + kMaxTensorSplits - 1) / kMaxTensorSplits + 31) / 32 * 32;
-                pl.splits = (static_cast<int>(rows) + pl.chunkK - 1) / pl.chunkK;
-            }
-            return pl;
-        };
-        const wgrad::Plan planX = planFor(I), planH = planFor(H);
+    // QAT: x and h_prev are integer codes, which the tensor-core GEMM multiplies exactly; its ones row also yields the bias gradients.
+    // A code is two exact bf16 terms when its grid is wider than 8 bits.
+    const bool tensorMemory = wgrad::tensorMemoryPath(I, H, C);
+    const bool aligned = call.quantized && I % 4 == 0 && H % 4 == 0 && alignedTo(call.x, 16);
+    const bool oneTerm = aligned && call.codesFitTensorPath && I <= 140 && H <= 140 && (!padded || std::max(I, H) <= 128);   // chunks of rows: one kernel for both arrays
+    const bool anyTerms = aligned && call.codesFitTwoTerms && (call.h0 || call.dqH.zeroPoint == 0.0f) && tensorMemory && std::getenv("RXMET_LSTM_WGRAD_SIMT") == nullptr;
+    if (oneTerm || anyTerms) {
+        // a missing h0 means real zeros, i.e. the zero-point code
+        if (!call.h0 && call.dqH.zeroPoint != 0.0f) fail(RXMET_ERR_INVALID_ARGUMENT, "the QAT backward needs the quantized initial hidden state");
+        const int K = static_cast<int>(rows);
+        const bool wideCodes = !call.codesFitTensorPath;
         wgrad::Problem px{}, ph{};
         px.aFloat = call.x; px.aFloatZero = call.dqX.zeroPoint; px.M = I; px.B = gIh; px.partial = tensorIh;
-        ph.aFloat = hPrev; ph.aFloatZero = call.h0 ? call.dqH.zeroPoint : 0.0f; ph.M = H; ph.B = gHh; ph.partial = tensorHh;
-        if (!call.h0 && call.dqH.zeroPoint != 0.0f) {
-            // a missing h0 means real zeros, i.e. the zero-point code: fill instead of zeroing
-            fail(RXMET_ERR_INVALID_ARGUMENT, "the QAT backward needs the quantized initial hidden state");
-        }
+        ph.aFloatZero = call.h0 ? call.dqH.zeroPoint : 0.0f; ph.M = H; ph.B = gHh; ph.partial = tensorHh;
         px.status = ph.status = tensorStatus;
-        int splitsX = planX.splits, splitsH = planH.splits;
-        if (padded && planX.tensorMemory && planH.tensorMemory && planX.chunkK > wgrad::kChainRows) {
-            splitsX = splitsH = wgrad::chained(px, ph, static_cast<int>(rows), C, st, [&](const wgrad::Problem &a, const wgrad::Problem &b, int n, int chunks) {
-                const wgrad::Plan plan{chunks, wgrad::kChainRows, true};
-                wgrad::launchPair(a, plan, b, plan, n, C, st);
-                afterLaunch("weightGrad");
-            });
+        auto previous = [&] {   // hidden states of the step before as one array
+            const size_t stateBytes = sizeof(float) * static_cast<size_t>(B) * H;
+            if (call.h0) RXMET_CUDA(cudaMemcpyAsync(hPrev, call.h0, stateBytes, cudaMemcpyDeviceToDevice, st));
+            else RXMET_CUDA(cudaMemsetAsync(hPrev, 0, stateBytes, st));
+            if (T > 1)
+                RXMET_CUDA(cudaMemcpyAsync(hPrev + static_cast<size_t>(B) * H, call.hiddenOutputs, stateBytes * (T - 1), cudaMemcpyDeviceToDevice, st));
+            ph.aFloat = hPrev;
+            ph.aFirst = nullptr;
+            ph.firstRows = 0;
+        };
+        int splitsX, splitsH;
+        if (tensorMemory) {
+            if (call.h0 && alignedTo(call.h0, 16) && alignedTo(call.hiddenOutputs, 16)) {   // read where they are
+                ph.aFirst = call.h0;   // a copy of all hidden states cost 12 us of a step of T = 100, B = 256, H = 128
+                ph.firstRows = B;
+                ph.aFloat = call.hiddenOutputs;
+            } else {
+                previous();
+            }
+            const wgrad::PairPlan plan = wgrad::planPair(px, ph, K, C, wideCodes, currentDevice().sms);
+            splitsX = plan.splits[0];
+            splitsH = plan.splits[1];
+            if (padded && wgrad::planRows(plan) > wgrad::kChainRows) {
+                if (ph.aFirst) previous();
+                splitsX = splitsH = wgrad::launchChained(px, ph, K, C, wideCodes, st);
+            } else {
+                wgrad::launchPair(px, ph, K, C, plan, wideCodes, st);
+            }
         } else {
-            wgrad::launchPair(px, planX, ph, planH, static_cast<int>(rows), C, st);
-            afterLaunch("weightGrad");
+            previous();
+            auto planFor = [&](int M) {
+                wgrad::Plan pl = wgrad::plan(K, M, C, currentDevice().sms);
+                if (pl.splits > kMaxTensorSplits) {
+                    pl.chunkK = ((K + kMaxTensorSplits - 1) / kMaxTensorSplits + 31) / 32 * 32;
+                    pl.splits = (K + pl.chunkK - 1) / pl.chunkK;
+                }
+                return pl;
+            };
+            const wgrad::Plan planX = planFor(I), planH = planFor(H);
+            splitsX = planX.splits;
+            splitsH = planH.splits;
+            wgrad::launch(px, K, C, planX, st);
+            wgrad::launch(ph, K, C, planH, st);
         }
+        afterLaunch("weightGrad");
         {
             const ReduceJob jobIh{tensorIh, splitsX, I, call.dqX.scale, static_cast<const uint8_t *>(mk.weight_ih),
                                   static_cast<const uint8_t *>(mk.bias_ih), call.grads.weight_ih, call.grads.bias_ih};
@@ -966,46 +987,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
                                   static_cast<const uint8_t *>(mk.bias_hh), call.grads.weight_hh, call.grads.bias_hh};
             const int rowBlocks = (std::max(I, H) + 1 + kReduceRows - 1) / kReduceRows;
             KernelTimer timer__("lstmReduceWeightGradT", st);
-            reduceWeightGradT<<<dim3((C + 31) / 32, rowBlocks, 2), dim3(32, kReduceRows, kReduceLayers), 0, st>>>(jobIh, jobHh, C,
-                                                                                                                  tensorStatus);
-        }
-        afterLaunch("lstmReduceWeightGradT");
-        return;
-    }
-    // Larger layers or 16-bit activation grids: the same tcgen05 kernel over 128-row slabs of both problems in one
-    // launch, a code as two exact bf16 terms when its grid is wider than 8 bits.
-    if (call.quantized && call.codesFitTwoTerms && I % 4 == 0 && H % 4 == 0 && alignedTo(call.x, 16) && (call.h0 || call.dqH.zeroPoint == 0.0f) &&
-        wgrad::slabPathTakes(I, H, C) && std::getenv("RXMET_LSTM_WGRAD_SIMT") == nullptr) {
-        const size_t stateBytes = sizeof(float) * static_cast<size_t>(B) * H;
-        if (call.h0) RXMET_CUDA(cudaMemcpyAsync(hPrev, call.h0, stateBytes, cudaMemcpyDeviceToDevice, st));
-        else RXMET_CUDA(cudaMemsetAsync(hPrev, 0, stateBytes, st));
-        if (T > 1)
-            RXMET_CUDA(cudaMemcpyAsync(hPrev + static_cast<size_t>(B) * H, call.hiddenOutputs, stateBytes * (T - 1),
-                                       cudaMemcpyDeviceToDevice, st));
-        int chunkK = 0;
-        int splits = wgrad::slabSplits(static_cast<int>(rows), I, H, C, currentDevice().sms, &chunkK);
-        wgrad::Problem px{}, ph{};
-        px.aFloat = call.x; px.aFloatZero = call.dqX.zeroPoint; px.M = I; px.B = gIh; px.partial = tensorIh;
-        ph.aFloat = hPrev; ph.aFloatZero = call.h0 ? call.dqH.zeroPoint : 0.0f; ph.M = H; ph.B = gHh; ph.partial = tensorHh;
-        px.status = ph.status = tensorStatus;
-        if (padded && chunkK > wgrad::kChainRows) {
-            splits = wgrad::chained(px, ph, static_cast<int>(rows), C, st, [&](const wgrad::Problem &a, const wgrad::Problem &b, int n, int chunks) {
-                wgrad::launchSlabs(a, b, n, C, wgrad::kChainRows, chunks, !call.codesFitTensorPath, st);
-                afterLaunch("weightGrad");
-            });
-        } else {
-            wgrad::launchSlabs(px, ph, static_cast<int>(rows), C, chunkK, splits, !call.codesFitTensorPath, st);
-            afterLaunch("weightGrad");
-        }
-        {
-            const ReduceJob jobIh{tensorIh, splits, I, call.dqX.scale, static_cast<const uint8_t *>(mk.weight_ih),
-                                  static_cast<const uint8_t *>(mk.bias_ih), call.grads.weight_ih, call.grads.bias_ih};
-            const ReduceJob jobHh{tensorHh, splits, H, call.dqH.scale, static_cast<const uint8_t *>(mk.weight_hh),
-                                  static_cast<const uint8_t *>(mk.bias_hh), call.grads.weight_hh, call.grads.bias_hh};
-            const int rowBlocks = (std::max(I, H) + 1 + kReduceRows - 1) / kReduceRows;
-            KernelTimer timer__("lstmReduceWeightGradT", st);
-            reduceWeightGradT<<<dim3((C + 31) / 32, rowBlocks, 2), dim3(32, kReduceRows, kReduceLayers), 0, st>>>(jobIh, jobHh, C,
-                                                                                                                  tensorStatus);
+            launchDependent(reduceWeightGradT, dim3((C + 31) / 32, rowBlocks, 2), dim3(32, kReduceRows, kReduceLayers), 0, st, jobIh, jobHh, C, tensorStatus);
         }
         afterLaunch("lstmReduceWeightGradT");
         return;

@@ -78,21 +78,25 @@ __device__ __forceinline__ void commitTo(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// Whether the barrier's phase of the given parity is over.
+__device__ __forceinline__ bool testPhase(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
 // Polls the barrier phase of the given parity; false when the limit ran out.  `polls`
 // (optional) receives the number of polls made.
 __device__ __forceinline__ bool waitPhase(uint32_t bar, uint32_t parity, uint32_t *polls = nullptr) {
     for (uint32_t i = 0; i < kSpinLimit; ++i) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t"
-            ".reg .pred p;\n\t"
-            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t"
-            "}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) {
+        if (testPhase(bar, parity)) {
             if (polls) *polls = i + 1;
             return true;
         }
@@ -121,6 +125,22 @@ __device__ __forceinline__ bool waitSuspended(uint32_t bar, uint32_t parity) {
     }
     return false;
 }
+
+// Walks a ring of mbarriers: place and phase parity of the current use.  Counters, not divisions: a division by a value known at run time costs
+// a lone thread more than issuing the products of a chunk.
+struct Turn {
+    int at = 0;
+    uint32_t parity = 0;
+    bool again = false;   // the place was used before
+    __device__ __forceinline__ void step(int size, int by = 1) {
+        at += by;
+        if (at >= size) {
+            at -= size;
+            parity ^= 1u;
+            again = true;
+        }
+    }
+};
 
 __device__ __forceinline__ void tmemLoad32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(

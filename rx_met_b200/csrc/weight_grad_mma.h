@@ -3,10 +3,9 @@
 // partial[s][m][n] = sum over the s-th chunk of the K rows of A[k][m] * B[k][n], for m < M, and
 // partial[s][M][n] = the column sums of B over the same rows, i.e. the bias gradient.
 // A holds small integers (activation codes minus their zero point), which bf16 represents exactly:
-// magnitude at most 256 as one term, or - for 16-bit activation grids - up to 2^17 as the two terms
+// magnitude at most 256 as one term, or - for 16-bit activation grids - below 2^16 as the two terms
 // 256 * floor(a / 256) and a mod 256; B (fp32 gradients) is split into three bf16 terms that together
 // carry all 24 significand bits, so every product is exact and only the fp32 accumulation rounds.
-// Problems with more than 128 rows are cut into slabs of 128 rows that share one launch.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -28,33 +27,35 @@ struct Problem {
     const float *B = nullptr;         // [K][N] gradients, N a multiple of 4
     float *partial = nullptr;         // [splits][M+1][N]
     int *status = nullptr;            // device word, set to 1 when a bounded wait of the kernel gave up
-    // Slabs (tcgen05 kernel only; the defaults describe a whole problem of at most 128 rows).  A slab covers
-    // rows [rowBase, rowBase + M) of a problem of totalRows - 1 real rows: aCodes / aFloat point at its first
-    // column, consecutive K rows lie `lda` elements apart, and its accumulator rows land at row rowBase of the
-    // [splits][totalRows][N] partial array; the slab with writeBias set also writes row totalRows - 1.
-    int lda = 0;                      // 0 = M
-    int rowBase = 0;
-    int totalRows = 0;                // 0 = M + 1
-    int writeBias = 1;
-    int wideCodes = 0;                // 1: |code - zero point| may exceed 256 (two A terms)
+    // tcgen05 kernel only: the codes of the first rows, where they are an array of their own; the others' lie at aFloat then
+    const float *aFirst = nullptr;    // [firstRows][M]
+    int firstRows = 0;
 };
 
-constexpr int kMaxSlabs = 12;
-struct ProblemSet {
-    Problem slab[kMaxSlabs];
-    int count = 0;
-};
-
-// How a problem is cut: K splits of chunkK rows each (a multiple of the kernel's K tile), and
-// which kernel runs it.  The tcgen05 kernel (accumulators in tensor memory) takes problems with
-// at most 128 rows whose column count is a multiple of 128, 192 or 256; the others run on the
-// mma.sync kernel.  Setting RXMET_WGRAD_MMA_SYNC in the environment forces the latter.
+// The mma.sync kernel: one problem cut into K splits of chunkK rows each (a multiple of its K tile).
 struct Plan {
     int splits = 0;
     int chunkK = 0;
-    bool tensorMemory = false;
 };
 Plan plan(int K, int M, int N, int sms);
+void launch(const Problem &problem, int K, int N, const Plan &plan, cudaStream_t stream);
+// Upper bound of plan(...).splits over every device, for sizing the partial buffers.
+int splitBound(int K, int M, int N);
+
+// The tcgen05 kernel (weight_grad_umma.cu): two problems over the same K rows and N columns (the input and the recurrent weights of a step) in
+// one launch.  M a multiple of 4, N of 128 or 192; operands 16-byte aligned.  RXMET_WGRAD_MMA_SYNC in the environment turns it off.
+constexpr int kMaxSms = 160;
+struct PairPlan {
+    int splits[2], chunks[2];   // of a and b: K splits, chunks of 32 rows in a split
+};
+bool tensorMemoryPath(int Ma, int Mb, int N);
+// wide: |code - zero point| may exceed 256 (two terms a code)
+PairPlan planPair(const Problem &a, const Problem &b, int K, int N, bool wide, int sms);
+int planRows(const PairPlan &plan);   // most rows of a split
+void launchPair(const Problem &a, const Problem &b, int K, int N, const PairPlan &plan, bool wide, cudaStream_t stream);
+// Upper bound of a problem's splits over every device, for sizing its partial sums.
+int tileSplitBound(int M, int N);
+
 // The tensor core truncates every addition to an accumulator; over a chunk of n rows that costs up to 8e-9 n of a sum of terms of one
 // sign with 16-bit codes (512 rows: 4.3e-6, 4096: 3.5e-5), a fifth of it with 8-bit codes.  Calls that would otherwise take
 // the FP32 kernels therefore cut the rows into chunks of kChainRows, however many there are: up to kChainGroup chunks (three
@@ -66,12 +67,12 @@ inline int chainChunks(int K) { return (K + kChainRows - 1) / kChainRows; }
 inline int chainPartials(int K) { return chainChunks(K) <= kChainGroup ? chainChunks(K) : kChainGroup + 1; }
 // sums of a and b (sum[i] = or += partial[0][i] + partial[1][i] + ...), `partial` behind the sums
 void addPartials(float *a, size_t countA, float *b, size_t countB, int partials, bool first, cudaStream_t stream);
-// launch(a, b, rows, chunks) runs both problems over `rows` rows; returns the number of partial sums at a.partial and b.partial.
-template <class Launch>
-int chained(const Problem &a, const Problem &b, int K, int N, cudaStream_t stream, Launch &&launch) {
+PairPlan chainPlan(int K);   // kChainRows a split
+// Both problems in chunks of kChainRows; returns the number of partial sums at a.partial and b.partial.
+inline int launchChained(const Problem &a, const Problem &b, int K, int N, bool wide, cudaStream_t stream) {
     const int chunks = chainChunks(K);
     if (chunks <= kChainGroup) {
-        launch(a, b, K, chunks);
+        launchPair(a, b, K, N, chainPlan(K), wide, stream);
         return chunks;
     }
     const size_t countA = static_cast<size_t>(a.M + 1) * N, countB = static_cast<size_t>(b.M + 1) * N;
@@ -85,37 +86,10 @@ int chained(const Problem &a, const Problem &b, int K, int N, cudaStream_t strea
             p.partial += count;
             return p;
         };
-        launch(part(a, countA), part(b, countB), rows, chainChunks(rows));
+        launchPair(part(a, countA), part(b, countB), rows, N, chainPlan(rows), wide, stream);
         addPartials(a.partial, countA, b.partial, countB, chainChunks(rows), first == 0, stream);
     }
     return 1;
 }
-// Upper bound of plan(...).splits over every device, for sizing the partial buffers.
-int splitBound(int K, int M, int N);
-void launch(const Problem &problem, int K, int N, const Plan &plan, cudaStream_t stream);
-// Two problems over the same K rows and N columns (the input and the recurrent weights of a step).
-// When both take the tcgen05 kernel with the same split they share ONE launch, the larger problem's
-// CTAs scheduled first; otherwise two launches.
-void launchPair(const Problem &a, const Plan &planA, const Problem &b, const Plan &planB, int K, int N, cudaStream_t stream);
-
-// The warp-specialised tcgen05 kernel (weight_grad_stream_umma.cu): both problems of a pair with at most 128 rows
-// (a multiple of 8) each, whole arrays (no slabs), 8-bit codes, N a multiple of 128 or 192 but not of 256.  Returns
-// false without launching when it does not take the pair.
-bool launchPairStreamed(const Problem &a, const Problem &b, int K, int N, int chunkK, int splits, cudaStream_t stream);
-
-// The tcgen05 kernel (weight_grad_umma.cu).
-bool tensorMemoryPath(int M, int N);
-int planTensorMemory(int K, int N, int sms, int *chunkK, int slabs = 1);
-void launchTensorMemory(const Problem &problem, const Problem *other, int K, int N, int chunkK, int splits,
-                        cudaStream_t stream);
-// Any number of rows: cuts `a` and `b` (either may have M = 0) into 128-row slabs, plans one K split for
-// all of them and runs them in ONE launch.  wide = two-term A operands for 16-bit codes.  Returns the
-// number of splits (the partial arrays hold [splits][M + 1][N]); slabsOf(M) slabs per problem.
-bool slabPathTakes(int Ma, int Mb, int N);
-int slabSplits(int K, int Ma, int Mb, int N, int sms, int *chunkK);
-// Upper bound of slabSplits over every device, for sizing the partial arrays.
-int slabSplitBound(int Ma, int Mb, int N);
-void launchSlabs(const Problem &a, const Problem &b, int K, int N, int chunkK, int splits, bool wide, cudaStream_t stream);
-
 }  // namespace wgrad
 }  // namespace rxmet

@@ -1,34 +1,40 @@
-// Weight-gradient GEMM on the fifth-generation tensor cores (tcgen05.mma, accumulators in
-// tensor memory).
+// Weight gradients on tcgen05.mma, the gradients as A operand in tensor memory.
 //
-//   partial[s][m][n] = sum over the K rows of split s of A[k][m] * B[k][n]      (m < M)
-//   partial[s][M][n] = sum over the same rows of B[k][n]                        (bias gradient)
+//   partial[s][m][n] = sum over the rows k of split s of code[k][m] * B[k][n]      (m < M)
+//   partial[s][M][n] = sum over the same rows of B[k][n]                            (bias gradient)
 //
-// A holds small integers (activation codes minus their zero point), exact in bf16.  B (fp32
-// gradients) is split into three bf16 terms that together carry all 24 significand bits, and the
-// three products accumulate into the same fp32 accumulator, so every product is exact and only
-// the accumulation rounds, as in an fp32 GEMM.
+// Codes are small integers (activation codes minus their zero point), exact in bf16 as one term, or as 256 floor(a / 256) and a mod 256 on
+// grids of more than 8 bits.  B (fp32 gradients) is split into three bf16 terms that together carry all 24 bits, so that every product is exact
+// and only the accumulation rounds.
 //
-// One CTA owns a 128 x NT accumulator tile (NT columns of tensor memory) over one K split.
-// Both operands arrive from HBM with the contraction index outermost ([k][m], [k][n]), which is
-// the "MN-major" operand form of the instruction: no transposition anywhere.  The producer
-// threads load fp32 / int32 rows, convert, and store 16-byte pieces straight into the
-// un-swizzled canonical operand layout (8 k-rows x 8 mn-elements per 128-byte core matrix);
-// one thread then issues the MMAs for the stage and commits them to an mbarrier.  Two operand
-// stages alternate, so the conversion of one 32-row chunk overlaps the tensor work of the
-// previous one.  One CTA per SM: the raw rows reach shared memory through a ring of cp.async
-// copies issued several chunks ahead, which keeps enough bytes in flight to cover the HBM
-// latency from a single CTA and halves the number of K splits (and partial tiles) against two
-// CTAs per SM.
+// The product is computed transposed: a lane of tensor memory is a gate channel n, an accumulator column an element m.  A CTA owns 128
+// channels, up to 256 elements of one of the two problems of a layer, and a range of rows.  A chunk of 32 rows is two MMA k-steps.  Warps by role:
+//   copies      fetches the raw rows of a chunk as TMA boxes of 32 rows x 128 bytes into a ring
+//   gradients   sixteen warps, two groups that take chunks in turn: thread = channel and sixteen rows; reads its column (neighbouring lanes,
+//               neighbouring words), adds it to the bias gradient, stores the three terms to its own tensor-memory lane
+//   codes       eight warps: raw codes -> bf16 in the canonical MN-major B layout in shared memory, 8 x 16-byte rows of a core matrix at a time
+//   products    one thread issues the MMAs of a chunk (k-steps, code terms, gradient terms, in this order)
+// Accumulators leave without a turn: neighbouring lanes are neighbouring channels of a row of `partial`.
 //
-// Every mbarrier wait is bounded: when a wait gives up the CTA records it in the status word and
-// carries on with the same control flow (the results are then wrong, and the reduction that
-// follows turns them into NaN), so the kernel always reaches the point where it gives its tensor
-// memory back.
+// The tensor core truncates each addition to an accumulator.  Up to 128 elements the first terms, which carry the sum's size, have accumulators
+// of their own, one for each k-step of a chunk, that are added to the others' at the end: a sixth of the additions that truncate at that size.
+//
+// Bound: reading the operands where codes have one term, the tensor pipe where they have two.  With both operands in shared
+// memory (the form before) the MMAs alone took 3/4 of its bandwidth beside the copies and the conversion.  In a step: 256,000 rows, 256 + 512 elements,
+// 2048 channels, two terms 4.25 -> 3.29 ms (its products at the measured burst rate: 2.9); 12,800 rows, 512 + 256, 768 channels by itself 94 -> 61 us; 25,600 rows,
+// 40 + 128, one term, 512 channels 41.7 -> 39.4 us, 384 channels 28.5 (another kernel, deleted) -> 30.5.
+// Error against 64 bits, 2-norm, normal gradients: 25,600 rows, one term 1.0e-6 -> 1.7e-7 (512 channels), 1.9e-6 -> 1.5e-7 (384); 12,800 rows, two terms 8.0e-6, as before.
+//
+// Every mbarrier wait is bounded; one that gives up ends all further waiting of the CTA and sets the status word (the reduction that follows turns
+// its outputs into NaN); copies and products in flight are awaited and tensor memory is freed all the same.
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
+#include "backward_cluster_device.cuh"
 #include "common.h"
+#include "dependent_launch.cuh"
+#include "tensor_map.cuh"
 #include "umma_device.cuh"
 #include "weight_grad_mma.h"
 
@@ -38,361 +44,388 @@ namespace {
 
 using namespace umma;
 
-constexpr int kStageRows = 32;          // K rows per stage: two MMA k-steps of 16
+constexpr int kRows = kBoxRows;                       // of a chunk
+constexpr int kGradientWarps = 16, kCodeWarps = 8, kConvWarps = kGradientWarps + kCodeWarps;
+constexpr int kCopyWarp = kConvWarps, kProductWarp = kConvWarps + 1, kThreads = 32 * (kProductWarp + 1);
+constexpr int kMaxElements = 256, kMaxBoxes = kMaxElements / kBoxCols;   // of a CTA
+constexpr int kMaxRing = 4, kMaxStages = 4;
+constexpr uint32_t kStageCols = 3 * kRows / 2;        // tensor-memory columns of a chunk: three terms, two rows a column
+constexpr uint32_t kTmemCols = 512;
+constexpr int kMaxTiles = 16;                          // element tiles of both problems
 
-// Depth of the ring of raw (unconverted) chunks, chosen so that ring + operand stages fill the
-// shared memory of an SM.
-template <int NT, int ATERMS = 1>
-struct Geometry {
-    static constexpr int kThreads = 2 * NT;                      // two thread halves, two k-groups of B each
-    static constexpr int kWarps = kThreads / 32;
-    static constexpr int kAPieces = (16 + kWarps - 1) / kWarps;  // A pieces (k-group x 32 rows of m) per warp
-    static constexpr uint32_t kAKStride = (kTileM / 8) * kCore;  // bytes between k-groups of the A tile
-    static constexpr uint32_t kBKStride = (NT / 8) * kCore;
-    static constexpr uint32_t kABytes = (kStageRows / 8) * kAKStride;
-    static constexpr uint32_t kBBytes = (kStageRows / 8) * kBKStride;
-    static constexpr uint32_t kStageBytes = ATERMS * kABytes + 3 * kBBytes;
-    static constexpr uint32_t kRawPieces = 2 * kWarps + 16;      // 1 KB pieces of a raw chunk: B per warp, then A
-    static constexpr uint32_t kRawBytes = kRawPieces * 1024;
-    static constexpr int kRing = NT <= 128 ? 4 : (NT <= 192 ? (ATERMS == 1 ? 3 : 2) : 2);
-    static_assert(2 * kStageBytes + kRing * kRawBytes <= 227 * 1024, "shared memory of one SM");
-    static constexpr size_t kSmem = 2 * kStageBytes + static_cast<size_t>(kRing) * kRawBytes;
+// An element tile of a problem, all splits and channel tiles of it.
+struct Tile {
+    int problem, m0, elements;      // elements: of this tile
+    int NP, boxes;                  // elements padded to 16, boxes of 32
+    int accs, stages, ring;
+    int firstBlock, splits, chunks;   // chunks of a split
+};
+struct Pair {
+    Problem of[2];
+    CUtensorMap gradients[2], codes[2], first[2];
+    Tile tile[kMaxTiles];
+    int tiles, channelTiles, N;
+    int firstChunks[2], totalChunks[2];   // chunks that Problem::aFirst gives the codes of; all chunks
+    int K;
 };
 
-// blockDim.x == 2 NT, one CTA per SM.  Warp w produces the B columns [32 (w % (NT/32)), + 32) of
-// the tile for two of the four k-groups of a chunk (which two: w / (NT/32)): lane -> k-row
-// (lane % 8) of a k-group and 8-column piece (lane / 8), so a warp's 16-byte operand stores cover
-// four whole core matrices (512 contiguous bytes) and its loads cover 8 rows x 128 contiguous bytes.  Each thread copies its own pieces of the next chunks into a
-// ring of raw buffers with cp.async, kRing chunks ahead; a warp later converts exactly the pieces
-// it copied, so the ring needs no CTA-wide barrier of its own.
-template <int NT, int ATERMS>
-__global__ void __launch_bounds__(2 * NT, 1)
-weightGradUmma(const __grid_constant__ ProblemSet set, int K, int N, int chunkK, int *status) {
-    const Problem &p = set.slab[blockIdx.z];  // gridDim.z problems / slabs share one launch
-    using G = Geometry<NT, ATERMS>;
-    constexpr int NW = G::kWarps, CW = NT / 32, AT = G::kAPieces, R = G::kRing, TH = G::kThreads;
-    constexpr uint32_t kAKStride = G::kAKStride, kBKStride = G::kBKStride, kABytes = G::kABytes, kBBytes = G::kBBytes;
-    constexpr uint32_t kStageBytes = G::kStageBytes;
-    constexpr uint32_t kTmemCols = NT > 128 ? 256 : 128;
-    constexpr uint32_t kIdesc = instructionDescriptor(NT, true, true);
-
-    extern __shared__ __align__(128) uint8_t stages[];
-    __shared__ __align__(8) uint64_t bars[3];
+// Codes of one term: two groups of warps take chunks in turn, which hides their hand-overs (T = 100, B = 256, H = 128, four gates 42.4 -> 38.9 us); of two
+// terms: all take every chunk (a layer of 512 inputs, 256 units, 12,800 rows 62 -> 59 us).
+template <int TERMS>   // of a code
+__global__ void __launch_bounds__(kThreads, 1) weightGradUmma(const __grid_constant__ Pair set) {
+    constexpr int kCodeGroups = TERMS == 1 ? 2 : 1, kChunkWarps = kGradientWarps / 2 + kCodeWarps / kCodeGroups;   // of a chunk
+    extern __shared__ __align__(1024) uint8_t smemRaw[];
+    __shared__ __align__(8) uint64_t rawFull[kMaxRing], rawFree[kMaxRing], termsFull[kMaxStages], termsFree[kMaxStages], accFull;
     __shared__ uint32_t tmemSlot;
-    __shared__ int failed;
+    __shared__ volatile int failed;
+    __shared__ float biasParts[4][kTileM];
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int rk = lane & 7, cq = lane >> 3;
-    const int cw = warp % CW, half = warp / CW;  // column warp and k-group half of the B pieces
-    const int n0 = blockIdx.x * NT;
-    const int kBegin = blockIdx.y * chunkK, kEnd = min(K, kBegin + chunkK);
-    const int chunks = (kEnd - kBegin + kStageRows - 1) / kStageRows;
-    const int M = p.M, quads = (M + 31) / 32;
-    uint4 *raw = reinterpret_cast<uint4 *>(stages + 2 * kStageBytes);  // [R][kRawPieces][64]
+    const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
+    int t = 0;
+    while (t + 1 < set.tiles && static_cast<int>(blockIdx.x) >= set.tile[t + 1].firstBlock) ++t;
+    const Tile &tile = set.tile[t];
+    const Problem &p = set.of[tile.problem];
+    const int local = static_cast<int>(blockIdx.x) - tile.firstBlock, split = local / set.channelTiles, n0 = (local - split * set.channelTiles) * kTileM, N = set.N;
+    const int chunkBegin = split * tile.chunks, chunks = min(tile.chunks, set.totalChunks[tile.problem] - chunkBegin);
+    const int NP = tile.NP, boxes = tile.boxes, gradientBoxes = min(kTileM / kBoxCols, (N - n0 + kBoxCols - 1) / kBoxCols);
+    const uint32_t slotBytes = static_cast<uint32_t>(kTileM / kBoxCols + boxes) * kBoxBytes;
+    const uint32_t kStride = static_cast<uint32_t>(boxes) * (kBoxCols / 8) * kCore;   // codes: next eight rows
+    const uint32_t termBytes = (kRows / 8) * kStride, stageBytes = TERMS * termBytes;
+    uint8_t *raw = smemRaw + ((1024u - (smemAddr(smemRaw) & 1023u)) & 1023u);   // swizzled boxes start on 1024 bytes
+    uint8_t *stages = raw + tile.ring * slotBytes;
 
     if (tid == 0) {
         failed = 0;
-        for (int i = 0; i < 3; ++i)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smemAddr(&bars[i])) : "memory");
+        auto init = [](uint64_t *bar, uint32_t count) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smemAddr(bar)), "r"(count) : "memory");
+        };
+        for (int i = 0; i < kMaxRing; ++i) { init(&rawFull[i], 1); init(&rawFree[i], kChunkWarps); }
+        for (int i = 0; i < kMaxStages; ++i) { init(&termsFull[i], kChunkWarps); init(&termsFree[i], 1); }
+        init(&accFull, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    // rows of A beyond M stay zero for the whole kernel
-    for (uint32_t i = tid; i < 2 * ATERMS * kABytes / 16; i += TH) {
-        const uint32_t stage = i / (ATERMS * kABytes / 16), off = i % (ATERMS * kABytes / 16);
-        *reinterpret_cast<uint4 *>(stages + stage * kStageBytes + off * 16) = make_uint4(0u, 0u, 0u, 0u);
-    }
-    const int lda = p.lda ? p.lda : M;
-    const int totalRows = p.totalRows ? p.totalRows : M + 1;
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(&tmemSlot)), "r"(kTmemCols)
-                     : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(&tmemSlot)), "n"(kTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-
-    const void *aBase = p.aCodes ? static_cast<const void *>(p.aCodes) : static_cast<const void *>(p.aFloat);
-    // Copies this warp's pieces of chunk `chunk` into ring entry `slot` and closes the group.  A
-    // piece is 8 k-rows x 128 bytes; one copy instruction of the warp covers four whole rows of
-    // it (lane -> row lane / 8, 16-byte part lane % 8), so every request is a full 128-byte line.
-    // Part p of row r is kept at position r * 8 + (p ^ r) of the piece, which makes both these
-    // writes and the converting reads (lane -> row lane % 8, parts 2 (lane / 8) and + 1) free of
-    // bank conflicts.
-    auto issueChunk = [&](int chunk, int slot) {
-        const int k0 = kBegin + chunk * kStageRows;
-        uint4 *dstB = raw + (static_cast<size_t>(slot) * G::kRawPieces + 2 * warp) * 64;
-        uint4 *dstA = raw + (static_cast<size_t>(slot) * G::kRawPieces + 2 * NW) * 64;
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int wrow = 4 * i + (lane >> 3), part = lane & 7, pos = wrow * 8 + (part ^ wrow);
-#pragma unroll
-            for (int gi = 0; gi < 2; ++gi) {
-                const int k = k0 + 8 * (2 * half + gi) + wrow;
-                const bool ok = k < kEnd;
-                copyAsync16(dstB + gi * 64 + pos, ok ? p.B + static_cast<size_t>(k) * N + n0 + 32 * cw + 4 * part : p.B, ok);
-            }
-#pragma unroll
-            for (int t = 0; t < AT; ++t) {
-                const int task = warp + t * NW, m = 32 * (task >> 2) + 4 * part;
-                const int k = k0 + 8 * (task & 3) + wrow;
-                if (task >= 16) continue;
-                const bool ok = task < 4 * quads && k < kEnd && m < M;
-                const size_t at = ok ? static_cast<size_t>(k) * lda + m : 0;
-                copyAsync16(dstA + task * 64 + pos, static_cast<const uint32_t *>(aBase) + at, ok);
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-#pragma unroll
-    for (int r = 0; r < R; ++r) issueChunk(r, r);
-
+    waitForPredecessor();   // what is above needs nothing from earlier kernels
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmemSlot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmemSlot, 0), stageBase = tmem + tile.accs * NP;
 
-    float csum[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) csum[j] = 0.0f;
-
-    // converts ring entry `slot` into the operand stage
-    auto convertChunk = [&](int slot, uint8_t *stage) {
-        const uint4 *srcB = raw + (static_cast<size_t>(slot) * G::kRawPieces + 2 * warp) * 64;
-        const uint4 *srcA = raw + (static_cast<size_t>(slot) * G::kRawPieces + 2 * NW) * 64;
-        const int posU = rk * 8 + ((2 * cq) ^ rk), posV = rk * 8 + ((2 * cq + 1) ^ rk);
-#pragma unroll
-        for (int gi = 0; gi < 2; ++gi) {
-            const int g = 2 * half + gi;
-            const uint4 ru = srcB[gi * 64 + posU], rv = srcB[gi * 64 + posV];
-            const float4 u = make_float4(__uint_as_float(ru.x), __uint_as_float(ru.y), __uint_as_float(ru.z), __uint_as_float(ru.w));
-            const float4 v = make_float4(__uint_as_float(rv.x), __uint_as_float(rv.y), __uint_as_float(rv.z), __uint_as_float(rv.w));
-            csum[0] += u.x; csum[1] += u.y; csum[2] += u.z; csum[3] += u.w;
-            csum[4] += v.x; csum[5] += v.y; csum[6] += v.z; csum[7] += v.w;
-            const Converted c = splitThree(u, v);
-            uint8_t *dst = stage + ATERMS * kABytes + (4 * cw + cq) * kCore + rk * 16 + g * kBKStride;
-            *reinterpret_cast<uint4 *>(dst) = c.hi;
-            *reinterpret_cast<uint4 *>(dst + kBBytes) = c.mid;
-            *reinterpret_cast<uint4 *>(dst + 2 * kBBytes) = c.lo;
-        }
-#pragma unroll
-        for (int t = 0; t < AT; ++t) {
-            const int task = warp + t * NW, g = task & 3, quad = task >> 2;
-            if (task >= 4 * quads) continue;
-            const uint4 ru = srcA[task * 64 + posU], rv = srcA[task * 64 + posV];
-            float x[8];
-            // zero-filled pieces decode to some finite value: they only meet zero rows of B or
-            // accumulator rows that are never stored
-            if (p.aCodes) {
-                const uint32_t q[8] = {ru.x, ru.y, ru.z, ru.w, rv.x, rv.y, rv.z, rv.w};
-#pragma unroll
-                for (int i = 0; i < 8; ++i) x[i] = static_cast<float>(static_cast<int32_t>(q[i]) - p.aZero);
-            } else {  // recover the integer code difference from the dequantized value
-                const uint32_t q[8] = {ru.x, ru.y, ru.z, ru.w, rv.x, rv.y, rv.z, rv.w};
-#pragma unroll
-                for (int i = 0; i < 8; ++i) x[i] = rintf(__uint_as_float(q[i]) * p.aInvScale) - p.aFloatZero;
-            }
-            uint8_t *dstA = stage + (4 * quad + cq) * kCore + rk * 16 + g * kAKStride;
-            if (ATERMS == 2) {
-                // a = 256 * floor(a / 256) + (a mod 256): both terms are exact in bf16 for |a| < 2^17
-                float hi[8], lo[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    hi[i] = floorf(x[i] * (1.0f / 256.0f)) * 256.0f;
-                    lo[i] = x[i] - hi[i];
-                }
-                *reinterpret_cast<uint4 *>(dstA) =
-                    make_uint4(packBf16(hi[0], hi[1]), packBf16(hi[2], hi[3]), packBf16(hi[4], hi[5]), packBf16(hi[6], hi[7]));
-                *reinterpret_cast<uint4 *>(dstA + kABytes) =
-                    make_uint4(packBf16(lo[0], lo[1]), packBf16(lo[2], lo[3]), packBf16(lo[4], lo[5]), packBf16(lo[6], lo[7]));
-            } else {
-                *reinterpret_cast<uint4 *>(dstA) =
-                    make_uint4(packBf16(x[0], x[1]), packBf16(x[2], x[3]), packBf16(x[4], x[5]), packBf16(x[6], x[7]));
-            }
-        }
+    auto wait = [&](uint64_t *bar, uint32_t parity) {   // one that gives up ends all further waiting of the CTA
+        if (testPhase(smemAddr(bar), parity)) return;
+        if (!failed && !waitSuspended(smemAddr(bar), parity)) failed = 1;
     };
-
-    for (int c = 0; c < chunks; ++c) {
-        const int s = c & 1, slot = c % R;
-        uint8_t *stage = stages + s * kStageBytes;
-        asm volatile("cp.async.wait_group %0;" ::"n"(R - 1) : "memory");
-        __syncwarp();  // the lanes of a warp convert what other lanes of it copied
-        // the MMAs that read this stage two chunks ago must have finished
-        if (c >= 2 && !waitPhase(smemAddr(&bars[s]), ((c >> 1) - 1) & 1)) failed = 1;
-        convertChunk(slot, stage);
+    auto arrive = [&](uint64_t *bar) {
         __syncwarp();
-        issueChunk(c + R, slot);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t base = smemAddr(stage);
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smemAddr(bar)) : "memory");
+    };
+    // Rows of a chunk: those of Problem::aFirst come first, in chunks of their own, then the others.
+    const int firstChunks = set.firstChunks[tile.problem];
+    auto rowOf = [&](int chunk) { return chunk < firstChunks ? chunk * kRows : p.firstRows + (chunk - firstChunks) * kRows; };
+    // ... of which the first this many are the chunk's own; rows beyond the last one are read as zeros
+    auto validOf = [&](int chunk) { return chunk < firstChunks ? min(kRows, p.firstRows - chunk * kRows) : kRows; };
+
+    if (warp < kGradientWarps) {
+        const int quarter = warp & 3, half = (warp >> 2) & 1, group = warp >> 3;
+        const uint32_t lanes = static_cast<uint32_t>(32 * quarter) << 16;
+        const bool real = quarter < gradientBoxes;   // lanes of absent channels keep what they held
+        Turn slot, stage;
+        slot.step(tile.ring, group);
+        stage.step(tile.stages, group);
+        float bias = 0.0f;
+        for (int c = group; c < chunks; c += 2, slot.step(tile.ring, 2), stage.step(tile.stages, 2)) {
+            const int valid = validOf(chunkBegin + c) - 16 * half;
+            wait(&rawFull[slot.at], slot.parity);
+            const float *column = reinterpret_cast<const float *>(raw + slot.at * slotBytes + quarter * kBoxBytes) + 16 * half * kBoxCols + lane;
+            float v[16];
 #pragma unroll
-            for (int ks = 0; ks < kStageRows / 16; ++ks) {
+            for (int i = 0; i < 16; ++i) v[i] = column[i * kBoxCols];
+            if (valid < 16) {
 #pragma unroll
-                for (int at = 0; at < ATERMS; ++at) {
-                    const uint64_t descA = operandDescriptor(base + at * kABytes + ks * 2 * kAKStride, kAKStride, kCore);
+                for (int i = 0; i < 16; ++i) v[i] = i < valid ? v[i] : 0.0f;
+            }
+            arrive(&rawFree[slot.at]);
+            float sum[8];
 #pragma unroll
-                    for (int sp = 0; sp < 3; ++sp) {
-                        const uint64_t descB =
-                            operandDescriptor(base + ATERMS * kABytes + sp * kBBytes + ks * 2 * kBKStride, kBKStride, kCore);
-                        mmaBf16(tmem, descA, descB, kIdesc, (c > 0 || ks > 0 || sp > 0 || at > 0) ? 1u : 0u);
+            for (int i = 0; i < 8; ++i) sum[i] = v[i] + v[i + 8];
+#pragma unroll
+            for (int n = 4; n > 0; n /= 2)
+#pragma unroll
+                for (int i = 0; i < n; ++i) sum[i] += sum[i + n];
+            bias += sum[0];
+            if (stage.again) wait(&termsFree[stage.at], stage.parity ^ 1u);
+            __syncwarp();
+            if (real) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t to = stageBase + lanes + stage.at * kStageCols + 8 * half;
+#pragma unroll
+                for (int term = 0; term < 3; ++term) {
+                    uint32_t w[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        w[i] = packBf16(v[2 * i], v[2 * i + 1]);
+                        v[2 * i] -= bf16Lo(w[i]);
+                        v[2 * i + 1] -= bf16Hi(w[i]);
                     }
+                    bwdcluster::tmemStore8(to + term * (kRows / 2), w);
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            }
+            arrive(&termsFull[stage.at]);
+        }
+        biasParts[2 * group + half][32 * quarter + lane] = bias;
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kGradientWarps) : "memory");
+        const int at = 32 * quarter + lane;
+        if (warp < 4 && tile.m0 == 0 && n0 + at < N)
+            p.partial[(static_cast<size_t>(split) * (p.M + 1) + p.M) * N + n0 + at] = (biasParts[0][at] + biasParts[1][at]) + (biasParts[2][at] + biasParts[3][at]);
+    } else if (warp < kConvWarps) {
+        // warp -> eight rows of every other chunk, or of every chunk and every other box; lane -> row and eight elements of a box
+        const int second = (warp - kGradientWarps) >> 2, turn = kCodeGroups == 2 ? second : 0, firstBox = kCodeGroups == 2 ? 0 : second, group = warp & 3, row8 = lane & 7, eighth = lane >> 3, row = 8 * group + row8;
+        // 1.5 * 2^23 rounds to integers, which sit in the low bits, 1.5 * 2^31 to multiples of 256
+        constexpr float kMagic = 12582912.0f, kMagic256 = 3221225472.0f;
+        const float inverse = p.aInvScale, offset = kMagic + (p.aCodes ? static_cast<float>(p.aZero) : p.aFloatZero);   // exact: below 2^24
+        auto run = [&](auto integersTag) {
+            constexpr bool kIntegers = decltype(integersTag)::value;
+            Turn slot, stage;
+            slot.step(tile.ring, turn);
+            stage.step(tile.stages, turn);
+            for (int c = turn; c < chunks; c += kCodeGroups, slot.step(tile.ring, kCodeGroups), stage.step(tile.stages, kCodeGroups)) {
+                const bool mine = row < validOf(chunkBegin + c);
+                wait(&rawFull[slot.at], slot.parity);
+                if (stage.again) wait(&termsFree[stage.at], stage.parity ^ 1u);
+                const uint8_t *from = raw + slot.at * slotBytes + kTileM / kBoxCols * kBoxBytes + row * 128;
+                uint8_t *to = stages + stage.at * stageBytes + group * kStride + eighth * kCore + row8 * 16;
+#pragma unroll 2
+                for (int box = firstBox; box < boxes; box += 3 - kCodeGroups) {
+                    const uint4 a = *reinterpret_cast<const uint4 *>(from + box * kBoxBytes + (((2 * eighth) ^ row8) << 4));
+                    const uint4 b = *reinterpret_cast<const uint4 *>(from + box * kBoxBytes + (((2 * eighth + 1) ^ row8) << 4));
+                    const uint32_t q[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                    float x[8];
+                    // boxes beyond the last element decode to some finite value that only reaches accumulator columns nobody reads
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        x[i] = __fadd_rn(kIntegers ? __uint_as_float(0x4b400000u + q[i]) : __fmaf_rn(__uint_as_float(q[i]), inverse, kMagic), -offset);
+                    uint32_t word[4];
+                    uint8_t *at = to + box * (kBoxCols / 8) * kCore;
+                    if (TERMS == 2) {   // 256 floor(x / 256): x - 127.5 is no tie
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float u = __fadd_rn(__fadd_rn(x[2 * i] - 127.5f, kMagic256), -kMagic256), v = __fadd_rn(__fadd_rn(x[2 * i + 1] - 127.5f, kMagic256), -kMagic256);
+                            word[i] = mine ? packBf16(u, v) : 0u;
+                            x[2 * i] -= u;
+                            x[2 * i + 1] -= v;
+                        }
+                        *reinterpret_cast<uint4 *>(at) = make_uint4(word[0], word[1], word[2], word[3]);
+                        at += termBytes;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) word[i] = mine ? packBf16(x[2 * i], x[2 * i + 1]) : 0u;
+                    *reinterpret_cast<uint4 *>(at) = make_uint4(word[0], word[1], word[2], word[3]);
+                }
+                arrive(&rawFree[slot.at]);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                arrive(&termsFull[stage.at]);
+            }
+        };
+        if (p.aCodes) run(std::true_type{});
+        else run(std::false_type{});
+    } else if (warp == kCopyWarp) {
+        // a box per lane: a lone lane takes 90 cycles a box, longer than 128 elements take to multiply
+        const CUtensorMap *gradients = &set.gradients[tile.problem], *codes = &set.codes[tile.problem], *first = &set.first[tile.problem];
+        Turn slot;
+        int issued = 0;
+        for (int c = 0; c < chunks && !failed; ++c, slot.step(tile.ring)) {
+            const int chunk = chunkBegin + c, row = rowOf(chunk);
+            if (slot.again) wait(&rawFree[slot.at], slot.parity ^ 1u);
+            if (__any_sync(0xffffffffu, failed)) break;
+            const uint32_t bar = smemAddr(&rawFull[slot.at]), to = smemAddr(raw + slot.at * slotBytes);
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((gradientBoxes + boxes) * kBoxBytes) : "memory");
+            __syncwarp();
+            if (lane < gradientBoxes) {
+                copyBox(to + lane * kBoxBytes, gradients, n0 + lane * kBoxCols, row, bar);
+            } else if (lane >= kTileM / kBoxCols && lane < kTileM / kBoxCols + boxes) {
+                const int b = lane - kTileM / kBoxCols;
+                copyBox(to + lane * kBoxBytes, chunk < firstChunks ? first : codes, tile.m0 + b * kBoxCols, chunk < firstChunks ? row : row - p.firstRows, bar);
+            }
+            issued = c + 1;
+        }
+        for (int c = max(0, issued - tile.ring); c < issued; ++c) waitPhase(smemAddr(&rawFull[c % tile.ring]), (c / tile.ring) & 1);   // nothing is left in flight
+    } else if (electOne()) {
+        // A: K-major in tensor memory, B: MN-major in shared memory
+        const uint32_t idesc = instructionDescriptor(NP, false, true), others = tmem + (tile.accs - 1) * NP;
+        const uint64_t descB0 = operandDescriptor(smemAddr(stages), kStride, kCore);
+        const bool parted = tile.accs == 3;
+        Turn stage;
+        for (int c = 0; c < chunks; ++c, stage.step(tile.stages)) {
+            wait(&termsFull[stage.at], stage.parity);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t terms = stageBase + stage.at * kStageCols;
+            const uint64_t descB = descB0 + static_cast<uint64_t>((stage.at * stageBytes) >> 4);
+#pragma unroll
+            for (int ks = 0; ks < kRows / 16; ++ks)
+#pragma unroll
+                for (int a = 0; a < TERMS; ++a)
+#pragma unroll
+                    for (int term = 0; term < 3; ++term)
+                        bwdcluster::mmaBf16TmemA(term > 0 ? others : parted ? tmem + ks * NP : tmem, terms + term * (kRows / 2) + 8 * ks,
+                                                 descB + static_cast<uint64_t>((a * termBytes + 2 * ks * kStride) >> 4), idesc,
+                                                 (c > 0 || a > 0 || (parted ? term > 1 || (term == 1 && ks > 0) : ks > 0 || term > 0)) ? 1u : 0u);
+            commitTo(smemAddr(&termsFree[stage.at]));
+            if (c + 1 == chunks) commitTo(smemAddr(&accFull));
+        }
+        letDependentsStart();   // the reduction is launched under the last products and the epilogue
+    }
+    __syncwarp();
+
+    // accumulators -> partial: lane = channel
+    if (chunks > 0) {
+        if (warp == kProductWarp && lane == 0) waitPhase(smemAddr(&accFull), 0);   // nothing is left in flight, whatever was given up
+        if (warp < kGradientWarps) {
+            wait(&accFull, 0);
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int quarter = warp & 3, n = n0 + 32 * quarter + lane;
+            float *out = p.partial + (static_cast<size_t>(split) * (p.M + 1) + tile.m0) * N + n;
+            const uint32_t from = tmem + (static_cast<uint32_t>(32 * quarter) << 16);
+            for (int m = 16 * (warp >> 2); m < tile.elements; m += 16 * (kGradientWarps / 4)) {
+                uint32_t r[3][16];
+#pragma unroll
+                for (int acc = 0; acc < 3; ++acc) {
+                    if (acc > 0 && tile.accs == 1) break;
+                    bwdcluster::tmemLoad<8>(from + acc * NP + m, *reinterpret_cast<uint32_t (*)[8]>(r[acc]));
+                    bwdcluster::tmemLoad<8>(from + acc * NP + m + 8, *reinterpret_cast<uint32_t (*)[8]>(r[acc] + 8));
+                }
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    float v = __uint_as_float(r[0][i]);
+                    if (tile.accs == 3) v = (v + __uint_as_float(r[1][i])) + __uint_as_float(r[2][i]);
+                    if (m + i < tile.elements && n < N) out[static_cast<size_t>(m + i) * N] = v;
                 }
             }
-            commitTo(smemAddr(&bars[s]));
-            if (c + 1 == chunks) commitTo(smemAddr(&bars[2]));
         }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (chunks > 0 && !waitPhase(smemAddr(&bars[2]), 0)) failed = 1;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-
-    float *slice = p.partial + static_cast<size_t>(blockIdx.y) * totalRows * N;
-    float *out = slice + static_cast<size_t>(p.rowBase) * N;
-    // accumulator rows: warp w may read the tensor-memory lanes [32 (w % 4), 32 (w % 4) + 32)
-    {
-        const int q = warp & 3, sharing = (NW - q + 3) / 4;
-        if (32 * q < M && chunks > 0) {
-            float4 *tile = reinterpret_cast<float4 *>(stages + warp * 4096);  // the operand stages are idle now
-            for (int j = warp >> 2; j < CW; j += sharing) {
-                uint32_t r[32];
-                tmemLoad32(tmem + (static_cast<uint32_t>(32 * q) << 16) + 32 * j, r);
-                // lane = accumulator row here; turn the 32 x 32 block through shared memory so that a
-                // store instruction of the warp writes four whole 128-byte row segments
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    tile[lane * 8 + (i ^ (lane & 7))] = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]),
-                                                                    __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
-                __syncwarp();
-#pragma unroll
-                for (int pass = 0; pass < 8; ++pass) {
-                    const int row = 4 * pass + (lane >> 3), i = lane & 7;
-                    const float4 v = tile[row * 8 + (i ^ (row & 7))];
-                    if (32 * q + row < M)
-                        *reinterpret_cast<float4 *>(out + static_cast<size_t>(32 * q + row) * N + n0 + 32 * j + 4 * i) = v;
-                }
-                __syncwarp();
-            }
-        }
-    }
-    // column sums of B: fold the eight k-row lanes, fixed order
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        float v = csum[j];
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        v += __shfl_xor_sync(0xffffffffu, v, 2);
-        v += __shfl_xor_sync(0xffffffffu, v, 4);
-        csum[j] = v;
-    }
-    // ... then the two thread halves, through the (now idle) first operand stage
-    float *scratch = reinterpret_cast<float *>(stages + NW * 4096);  // behind the warps' epilogue tiles
-    if (half == 1 && rk == 0) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) scratch[32 * cw + 8 * cq + j] = csum[j];
-    }
-    __syncthreads();
-    if (half == 0 && rk == 0 && p.writeBias) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) csum[j] += scratch[32 * cw + 8 * cq + j];
-        float4 *dst = reinterpret_cast<float4 *>(slice + static_cast<size_t>(totalRows - 1) * N + n0 + 32 * cw + 8 * cq);
-        dst[0] = make_float4(csum[0], csum[1], csum[2], csum[3]);
-        dst[1] = make_float4(csum[4], csum[5], csum[6], csum[7]);
-    }
-
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
-    }
-    if (tid == 0 && failed && status) atomicExch(status, 1);
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTmemCols) : "memory");
+    if (tid == 0 && failed && p.status) atomicExch(p.status, 1);
 }
 
-template <int NT, int ATERMS>
-void launchSet(const ProblemSet &set, int K, int N, int chunkK, int splits, cudaStream_t st) {
-    constexpr size_t smem = Geometry<NT, ATERMS>::kSmem;
-    ensureDynamicSmem(reinterpret_cast<const void *>(weightGradUmma<NT, ATERMS>), smem);  // per device
-    KernelTimer timer__("weightGradUmma", st);
-    weightGradUmma<NT, ATERMS><<<dim3(N / NT, splits, set.count), Geometry<NT, ATERMS>::kThreads, smem, st>>>(
-        set, K, N, chunkK, set.slab[0].status);
-}
+int elementTiles(int M) { return (M + kMaxElements - 1) / kMaxElements; }
+int channelTiles(int N) { return (N + kTileM - 1) / kTileM; }
+int paddedTile(int M) { return ((M + elementTiles(M) - 1) / elementTiles(M) + 15) / 16 * 16; }   // elements of a tile
+int chunksOf(int K, int firstRows) { return (firstRows + kRows - 1) / kRows + (K - firstRows + kRows - 1) / kRows; }
 
-template <int NT>
-void launchTile(const Problem &prob, const Problem *other, int K, int N, int chunkK, int splits, cudaStream_t st) {
-    ProblemSet set;
-    set.slab[0] = prob;
-    set.count = 1;
-    if (other) set.slab[set.count++] = *other;
-    launchSet<NT, 1>(set, K, N, chunkK, splits, st);
-}
-
-int tileColumns(int N) {
-    for (int nt : {256, 192, 128})
-        if (N % nt == 0) return nt;
-    return 0;
-}
+size_t slotBytes(const Tile &t) { return static_cast<size_t>(kTileM / kBoxCols + t.boxes) * kBoxBytes; }
+size_t stageBytes(const Tile &t, int terms) { return static_cast<size_t>(terms) * kRows * t.boxes * kBoxCols * 2; }
 
 }  // namespace
 
-bool tensorMemoryPath(int M, int N) {
+bool tensorMemoryPath(int Ma, int Mb, int N) {
     static const bool disabled = std::getenv("RXMET_WGRAD_MMA_SYNC") != nullptr;
-    return !disabled && M >= 4 && M <= kTileM && M % 4 == 0 && N % 4 == 0 && tileColumns(N) != 0;
+    return !disabled && Ma >= 4 && Mb >= 4 && Ma % 4 == 0 && Mb % 4 == 0 && (N % 128 == 0 || N % 192 == 0) && elementTiles(Ma) + elementTiles(Mb) <= kMaxTiles &&
+           encodeTiled() != nullptr;
 }
 
-int planTensorMemory(int K, int N, int sms, int *chunkK, int slabs) {
-    const int tiles = (N / tileColumns(N)) * std::max(1, slabs);
-    const int want = std::max(1, sms / tiles);  // one CTA per SM
-    *chunkK = ((K + want - 1) / want + kStageRows - 1) / kStageRows * kStageRows;
-    return (K + *chunkK - 1) / *chunkK;
-}
+int tileSplitBound(int M, int N) { return std::max(1, kMaxSms / (elementTiles(M) * channelTiles(N))); }
 
-void launchTensorMemory(const Problem &prob, const Problem *other, int K, int N, int chunkK, int splits, cudaStream_t st) {
-    switch (tileColumns(N)) {
-        case 256: launchTile<256>(prob, other, K, N, chunkK, splits, st); break;
-        case 192: launchTile<192>(prob, other, K, N, chunkK, splits, st); break;
-        case 128: launchTile<128>(prob, other, K, N, chunkK, splits, st); break;
-        default: fail(RXMET_ERR_UNSUPPORTED, "no tensor-memory tile for %d columns", N);
+// A chunk costs a CTA what it has to read or, with two terms a code, its products; the SMs are shared out so that both problems end together.
+PairPlan planPair(const Problem &a, const Problem &b, int K, int N, bool wide, int sms) {
+    const Problem *of[2] = {&a, &b};
+    int tiles[2], chunks[2];
+    double cost[2];
+    for (int i = 0; i < 2; ++i) {
+        const int NP = paddedTile(of[i]->M);
+        tiles[i] = elementTiles(of[i]->M) * channelTiles(N);
+        chunks[i] = chunksOf(K, of[i]->firstRows);
+        cost[i] = std::max((wide ? 6.0 : 3.0) * NP, 500.0 + 4.0 * NP);
     }
+    sms = std::min(sms, kMaxSms);
+    int best[2] = {1, 1};
+    double least = 1e30;
+    for (int s = 1; s == 1 || (s <= chunks[0] && s * tiles[0] + tiles[1] <= sms); ++s) {
+        const int other = std::max(1, std::min(chunks[1], (sms - s * tiles[0]) / tiles[1]));
+        const double time = std::max(cost[0] * ((chunks[0] + s - 1) / s), cost[1] * ((chunks[1] + other - 1) / other));
+        if (time < least) { least = time; best[0] = s; best[1] = other; }
+    }
+    PairPlan plan;
+    for (int i = 0; i < 2; ++i) {
+        const int each = (chunks[i] + best[i] - 1) / best[i];
+        plan.chunks[i] = each;
+        plan.splits[i] = (chunks[i] + each - 1) / each;
+    }
+    return plan;
 }
 
-int slabsOf(int M) { return (M + kTileM - 1) / kTileM; }
-
-bool slabPathTakes(int Ma, int Mb, int N) {
-    static const bool disabled = std::getenv("RXMET_WGRAD_MMA_SYNC") != nullptr;
-    if (disabled || tileColumns(N) == 0 || Ma % 4 != 0 || Mb % 4 != 0 || Ma < 0 || Mb < 0) return false;
-    return slabsOf(Ma) + slabsOf(Mb) >= 1 && slabsOf(Ma) + slabsOf(Mb) <= kMaxSlabs;
+PairPlan chainPlan(int K) {
+    PairPlan plan;
+    for (int i = 0; i < 2; ++i) {
+        plan.chunks[i] = kChainRows / kRows;
+        plan.splits[i] = chainChunks(K);
+    }
+    return plan;
 }
 
-int slabSplits(int K, int Ma, int Mb, int N, int sms, int *chunkK) {
-    return planTensorMemory(K, N, sms, chunkK, slabsOf(Ma) + slabsOf(Mb));
-}
+int planRows(const PairPlan &plan) { return std::max(plan.chunks[0], plan.chunks[1]) * kRows; }
 
-int slabSplitBound(int Ma, int Mb, int N) {
-    const int nt = tileColumns(N);
-    if (nt == 0) return 1;
-    return std::max(1, 160 / ((N / nt) * std::max(1, slabsOf(Ma) + slabsOf(Mb))));
-}
-
-void launchSlabs(const Problem &a, const Problem &b, int K, int N, int chunkK, int splits, bool wide, cudaStream_t st) {
-    ProblemSet set;
-    for (const Problem *prob : {&a, &b}) {
-        for (int m0 = 0; m0 < prob->M; m0 += kTileM) {
-            Problem s = *prob;
-            s.M = std::min(kTileM, prob->M - m0);
-            s.lda = prob->M;
-            s.rowBase = m0;
-            s.totalRows = prob->M + 1;
-            s.writeBias = m0 == 0 ? 1 : 0;
-            s.wideCodes = wide ? 1 : 0;
-            if (s.aCodes) s.aCodes += m0;
-            if (s.aFloat) s.aFloat += m0;
-            set.slab[set.count++] = s;
+void launchPair(const Problem &a, const Problem &b, int K, int N, const PairPlan &plan, bool wide, cudaStream_t st) {
+    Pair set;
+    set.of[0] = a;
+    set.of[1] = b;
+    set.tiles = 0;
+    set.channelTiles = channelTiles(N);
+    set.N = N;
+    set.K = K;
+    const int terms = wide ? 2 : 1;
+    size_t smem = 0;
+    int blocks = 0;
+    RXMET_REQUIRE(elementTiles(a.M) + elementTiles(b.M) <= kMaxTiles, "weight gradient: %d and %d elements", a.M, b.M);
+    for (int i : {a.M >= b.M ? 0 : 1, a.M >= b.M ? 1 : 0}) {   // the larger problem's CTAs first
+        const Problem &p = set.of[i];
+        RXMET_REQUIRE(alignedTo(p.B, 16) && alignedTo(p.aCodes, 16) && alignedTo(p.aFloat, 16) && alignedTo(p.aFirst, 16) && p.M % 4 == 0 && N % 4 == 0,
+                      "weight gradient: misaligned operands");
+        const void *codes = p.aCodes ? static_cast<const void *>(p.aCodes) : static_cast<const void *>(p.aFloat);
+        set.gradients[i] = boxMap(p.B, K, N, CU_TENSOR_MAP_SWIZZLE_NONE);
+        // a sequence of one step has no rows but the first ones
+        set.codes[i] = boxMap(K > p.firstRows ? codes : p.aFirst, std::max(1, K > p.firstRows ? K - p.firstRows : p.firstRows), p.M, CU_TENSOR_MAP_SWIZZLE_128B);
+        set.first[i] = p.firstRows > 0 ? boxMap(p.aFirst, p.firstRows, p.M, CU_TENSOR_MAP_SWIZZLE_128B) : set.codes[i];
+        set.firstChunks[i] = (p.firstRows + kRows - 1) / kRows;
+        set.totalChunks[i] = chunksOf(K, p.firstRows);
+        const int each = paddedTile(p.M);
+        for (int m0 = 0; m0 < p.M; m0 += each) {
+            Tile &t = set.tile[set.tiles++];
+            t.problem = i;
+            t.m0 = m0;
+            t.elements = std::min(each, p.M - m0);
+            t.NP = each;
+            t.boxes = (each + kBoxCols - 1) / kBoxCols;
+            t.accs = each <= 128 ? 3 : 1;
+            t.stages = std::min<int>(kMaxStages, (kTmemCols - t.accs * each) / kStageCols);
+            t.ring = kMaxRing;
+            const size_t most = 222 * 1024;
+            while (t.stages > 2 && 2 * slotBytes(t) + t.stages * stageBytes(t, terms) > most) --t.stages;
+            while (t.ring > 2 && t.ring * slotBytes(t) + t.stages * stageBytes(t, terms) > most) --t.ring;
+            while (t.stages > 2 && t.ring == 2 && 3 * slotBytes(t) + (t.stages - 1) * stageBytes(t, terms) <= most) { --t.stages; t.ring = 3; }
+            smem = std::max(smem, 1024 + t.ring * slotBytes(t) + t.stages * stageBytes(t, terms));
+            t.firstBlock = blocks;
+            t.splits = plan.splits[i];
+            t.chunks = plan.chunks[i];
+            blocks += t.splits * set.channelTiles;
         }
     }
-    RXMET_REQUIRE(set.count >= 1 && set.count <= kMaxSlabs, "weight gradient: %d slabs", set.count);
-    switch (tileColumns(N)) {
-        case 256: wide ? launchSet<256, 2>(set, K, N, chunkK, splits, st) : launchSet<256, 1>(set, K, N, chunkK, splits, st); break;
-        case 192: wide ? launchSet<192, 2>(set, K, N, chunkK, splits, st) : launchSet<192, 1>(set, K, N, chunkK, splits, st); break;
-        case 128: wide ? launchSet<128, 2>(set, K, N, chunkK, splits, st) : launchSet<128, 1>(set, K, N, chunkK, splits, st); break;
-        default: fail(RXMET_ERR_UNSUPPORTED, "no tensor-memory tile for %d columns", N);
-    }
+    auto run = [&](auto kernel) {
+        ensureDynamicSmem(reinterpret_cast<const void *>(kernel), smem);
+        KernelTimer timer__("weightGradUmma", st);
+        launchDependent(kernel, static_cast<unsigned>(blocks), kThreads, smem, st, set);
+    };
+    if (wide) run(weightGradUmma<2>);
+    else run(weightGradUmma<1>);
 }
 
 namespace {

@@ -580,6 +580,13 @@ def test_input_gradient_tiles(gl, shape):
     test_backward_quant(gl, "w8a8", shape)
 
 
+@pytest.mark.parametrize("cfg_name", ["w8a8", "a16"])
+@pytest.mark.parametrize("shape", [(1, 1, 4, 64), (1, 31, 128, 64), (1, 33, 260, 64), (1, 65, 516, 128), (3, 700, 12, 128)], ids=lambda s: "x".join(map(str, s)))
+def test_weight_gradient_tiles(gl, cfg_name, shape):
+    """Rows at the edge of a chunk, a partly empty tile of channels (192), up to three tiles of elements, splits of unequal problems."""
+    test_backward_quant(gl, cfg_name, shape)
+
+
 @pytest.mark.parametrize("byte_masks", [False, True], ids=["packed", "bytes"])
 def test_time_chunked_step_equals_the_single_launch_step(monkeypatch, byte_masks):
     """The overlapped pipeline cuts the sequence into time chunks (projection / gradient GEMMs of one chunk under the

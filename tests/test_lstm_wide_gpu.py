@@ -165,6 +165,13 @@ def test_wide_qat_backward_over_clusters_and_padded_widths(T, B, I, H, wb, ab):
     test_wide_qat_backward(T, B, I, H, wb, ab)
 
 
+@pytest.mark.parametrize("T,B,I,H,wb,ab", [(1, 5, 8, 64, 8, 16), (2, 33, 40, 64, 8, 16), (3, 31, 132, 128, 8, 16), (2, 64, 256, 160, 4, 16),
+                                           (2, 40, 48, 256, 8, 8), (5, 97, 44, 192, 8, 12)])
+def test_weight_gradient_tiles(T, B, I, H, wb, ab):
+    """Rows of the initial state by themselves, at and beside the edge of a chunk of 32; one and three accumulators; codes of one and two terms."""
+    test_wide_qat_backward(T, B, I, H, wb, ab)
+
+
 @pytest.mark.parametrize("B", [170, 250, 350, 700])
 def test_wide_forward_at_the_row_counts_of_a_cluster(B):
     """Twelve, sixteen or 24, 24 and 48 rows of a cluster, two or three groups of warps over them, a partial last tile of units."""
