@@ -20,9 +20,10 @@
 // so that copies, products and the epilogue of different items run at the same time.  Every mbarrier wait is bounded; one
 // that gives up ends all further waiting of its warp, sets the status word, and the CTA still frees its tensor memory.
 //
-// Bound: the stores of the results and the issue of the epilogue.  I = 256, C = 2048, 4.1 M rows (33.5 GB of 32-bit results) 15.0 -> 7.3 ms;
-// I = 512, C = 768, 12,800 rows on half of the SMs 81 -> 54 us; 1000 rows, C = 2048 79 -> 16 us, where eight CTAs had been at work.
-// The form before it fetched every weight tile through registers between two barriers of all warps.
+// Bound: the stores of the results and the issue of the epilogue.  I = 256, C = 2048, 4.1 M rows (33.5 GB of 32-bit results) 15.0 -> 7.2 ms;
+// I = 512, C = 768, 12,800 rows on half of the SMs 81 -> 44 us; I = 80, C = 512, 25,600 rows 25 -> 20 us, I = 40 30 -> 26 us with checkpoints; 1000 rows, C = 2048
+// 79 -> 16 us, where eight CTAs had been at work.  The form before it fetched every weight tile through registers between two barriers of
+// all warps; two warps that placed the planes 16 bytes at a time took 3 us a row tile, which shares of a row tile made the bound.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -32,6 +33,7 @@
 
 #include "common.h"
 #include "dependent_launch.cuh"
+#include "tensor_map.cuh"
 #include "umma_device.cuh"
 
 namespace rxmet {
@@ -40,7 +42,7 @@ namespace planeproj {
 using namespace umma;
 
 constexpr int kChannelTile = 128;
-constexpr int kEpilogueWarps = 16, kProductWarp = 16, kRowWarps = 2, kRowWarp = 17, kWeightWarp = kRowWarp + kRowWarps;
+constexpr int kEpilogueWarps = 16, kProductWarp = 16, kRowWarp = 17, kWeightWarp = 18;
 constexpr int kThreads = 32 * (kWeightWarp + 1);
 constexpr int kSlice = 256;   // k-bytes of a slice of a weight tile
 
@@ -89,7 +91,7 @@ inline int ringSlices(int kPad, int planes) {
     return std::min(4, (225 * 1024 - rows) / sliceBytes);
 }
 // Whether the operands fit one SM.
-inline bool fits(int kPad, int planes) { return kPad <= 512 && ringSlices(kPad, planes) >= 2; }
+inline bool fits(int kPad, int planes) { return kPad <= 512 && ringSlices(kPad, planes) >= 2 && encodeTiled() != nullptr; }
 inline size_t sharedBytes(int kPad, int planes) {
     return static_cast<size_t>(ringSlices(kPad, planes)) * kChannelTile * std::min(kPad, kSlice) + 2 * static_cast<size_t>(planes) * rowsPerTile(kPad) * kPad;
 }
@@ -128,7 +130,7 @@ struct Column {
 };
 
 template <class Epilogue, int PLANES, int NR>
-__global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const __grid_constant__ Problem p, const __grid_constant__ Epilogue epi) {
+__global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const __grid_constant__ Problem p, const __grid_constant__ Epilogue epi, const __grid_constant__ CUtensorMap rowsMap) {
     constexpr uint32_t kBufCols = PLANES * NR;
     constexpr uint32_t kTmemCols = 2 * kBufCols;   // a power of two for the sizes instantiated (128 .. 512)
     constexpr uint32_t kIdesc = instructionDescriptor(NR);
@@ -141,9 +143,10 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const __grid_consta
     const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
     const int C = p.C, kWords = p.kWords, kPad = paddedK(kWords), ring = p.ring;
     const uint32_t sliceBytes = static_cast<uint32_t>(kChannelTile) * min(kPad, kSlice);
-    const uint32_t planeBytes = static_cast<uint32_t>(NR) * kPad, rowStride = static_cast<uint32_t>(kPad / 16) * kCore;   // next 8 rows
+    const uint32_t planeBytes = static_cast<uint32_t>(NR) * kPad;
+    constexpr uint32_t kGroupBytes = NR * 16;   // rows: next 16 bytes along K
     uint8_t *weights = smem;                      // [ring][16 channel groups][slice / 16][8][16]
-    uint8_t *rowPlanes = smem + ring * sliceBytes;   // [2][PLANES][NR / 8][kPad / 16][8][16]
+    uint8_t *rowPlanes = smem + ring * sliceBytes;   // [2][PLANES][kPad / 16][NR][16]
 
     if (tid == 0) {
         failed = 0;
@@ -151,7 +154,7 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const __grid_consta
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smemAddr(bar)), "r"(count) : "memory");
         };
         for (int i = 0; i < kMaxSlices; ++i) { init(&weightFull[i], 1); init(&weightFree[i], 1); }
-        for (int i = 0; i < 2; ++i) { init(&rowsFull[i], kRowWarps); init(&rowsFree[i], 1); init(&accFull[i], 1); init(&accFree[i], kEpilogueWarps); }
+        for (int i = 0; i < 2; ++i) { init(&rowsFull[i], 1); init(&rowsFree[i], 1); init(&accFull[i], 1); init(&accFree[i], kEpilogueWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -200,26 +203,22 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const __grid_consta
         // nothing is left in flight, whatever the other warps gave up on
         for (uint32_t i = n > static_cast<uint32_t>(ring) ? n - ring : 0; i < n; ++i)
             if (!waitPhase(smemAddr(&weightFull[i % ring]), (i / ring) & 1)) alive = false;
-    } else if (warp >= kRowWarp && warp < kRowWarp + kRowWarps) {
-        // eight rows x four k-groups a pass: whole core matrices in shared memory, 64-byte pieces of rows in global memory
-        const int kGroups = kWords / 4, r8 = lane & 7, quad = lane >> 3, passes = (kGroups + 3) / 4;
+    } else if (warp == kRowWarp) {
+        const int kGroups = kWords / 4;
         uint32_t n = 0;
         for (int unit = blockIdx.x; unit < units; unit += gridDim.x, ++n) {
-            const uint32_t buf = n & 1;
+            const uint32_t buf = n & 1, bar = smemAddr(&rowsFull[buf]);
             if (n > 1) wait(&rowsFree[buf], ((n >> 1) - 1) & 1);
-            const int first = unit / shares * NR;
-            for (int pl = 0; pl < PLANES; ++pl)
-                for (int i = warp - kRowWarp; i < NR / 8 * passes; i += kRowWarps) {
-                    const int rows8 = i / passes, kg = (i - rows8 * passes) * 4 + quad, row = first + rows8 * 8 + r8;
-                    if (kg < kGroups)
-                        copyAsync16(rowPlanes + (buf * PLANES + pl) * planeBytes + rows8 * rowStride + kg * kCore + r8 * 16,
-                                    p.planes + (static_cast<size_t>(min(row, p.rows - 1)) * PLANES + pl) * kWords + 4 * kg, row < p.rows);
-                }
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(PLANES * kGroups * kGroupBytes) : "memory");
             __syncwarp();
-            if (lane == 0) arrive(&rowsFull[buf]);
+            for (int i = lane; i < PLANES * kGroups; i += 32) {
+                const int pl = i / kGroups, kg = i - pl * kGroups;
+                copyBox(smemAddr(rowPlanes + (buf * PLANES + pl) * planeBytes + kg * kGroupBytes), &rowsMap, 4 * i, unit / shares * NR, bar);
+            }
         }
+        // nothing is left in flight, whatever the other warps gave up on
+        for (uint32_t i = n > 2 ? n - 2 : 0; i < n; ++i)
+            if (!waitPhase(smemAddr(&rowsFull[i & 1]), (i >> 1) & 1)) alive = false;
     } else if (warp == kProductWarp) {
         uint32_t n = 0, item = 0, unitIndex = 0;
         for (int unit = blockIdx.x; unit < units; unit += gridDim.x, ++unitIndex) {
@@ -238,9 +237,9 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const __grid_consta
                         constexpr uint64_t kStep = (2 * kCore) >> 4;   // the start-address field counts 16-byte units
 #pragma unroll
                         for (int pl = 0; pl < PLANES; ++pl) {
-                            const uint64_t descB = operandDescriptor(smemAddr(rowPlanes + (rowBuf * PLANES + pl) * planeBytes + s * (kSlice / 16) * kCore), kCore, rowStride);
+                            const uint64_t descB = operandDescriptor(smemAddr(rowPlanes + (rowBuf * PLANES + pl) * planeBytes + s * (kSlice / 16) * kGroupBytes), kGroupBytes, kCore);
                             for (int ks = 0; ks < sliceK / 32; ++ks)
-                                mmaI8(tmem + buf * kBufCols + pl * NR, descA + ks * kStep, descB + ks * kStep, kIdesc, s + ks > 0 ? 1u : 0u);
+                                mmaI8(tmem + buf * kBufCols + pl * NR, descA + ks * kStep, descB + ks * ((2 * kGroupBytes) >> 4), kIdesc, s + ks > 0 ? 1u : 0u);
                         }
                         commitTo(smemAddr(&weightFree[at]));
                         if (s + 1 == slices) {
@@ -317,15 +316,23 @@ template <int PLANES, class Epilogue>
 void launch(const char *name, Problem p, const Epilogue &epi, int sms, int dependents, cudaStream_t st) {
     const int kPad = paddedK(p.kWords), rows = rowsPerTile(kPad), rowTiles = (p.rows + rows - 1) / rows, channelTiles = paddedC(p.C) / kChannelTile;
     p.ring = ringSlices(kPad, PLANES);
-    p.shares = std::max(1, std::min(channelTiles, sms / std::max(1, rowTiles)));
+    // Shares of a row tile that leave the SMs least to wait for: 200 row tiles of 25,600 rows are two rounds of 148 CTAs, 400 halves are three
+    // of half the length.  A share reads the planes of its rows again, so fewer where it makes no difference.
+    p.shares = 1;
+    double least = 1e30;
+    for (int shares = 1; shares <= channelTiles; ++shares) {
+        const double time = static_cast<double>((static_cast<long long>(rowTiles) * shares + sms - 1) / sms) * ((channelTiles + shares - 1) / shares + 0.25);
+        if (time < least * 0.99) { least = time; p.shares = shares; }
+    }
     const size_t smem = sharedBytes(kPad, PLANES);
     const int grid = std::max(1, std::min(rowTiles * p.shares, sms));
     p.early = grid + dependents <= sms;
+    const CUtensorMap map = boxMap(p.planes, p.rows, PLANES * p.kWords, CU_TENSOR_MAP_SWIZZLE_NONE, 4, rows);
     auto run = [&](auto kernel) {
         ensureDynamicSmem(reinterpret_cast<const void *>(kernel), smem);
         {
             KernelTimer timer__(name, st);
-            launchDependent(kernel, grid, kThreads, smem, st, p, epi);
+            launchDependent(kernel, grid, kThreads, smem, st, p, epi, map);
         }
         afterLaunch(name);
     };

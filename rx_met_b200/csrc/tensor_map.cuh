@@ -1,4 +1,4 @@
-// Tensor maps of row-major arrays of four-byte values for boxes of 32 rows x 32 values (128 bytes), the TMA copies of the gradient kernels.
+// Tensor maps of row-major arrays of four-byte values, and the TMA copies of their boxes.
 #pragma once
 
 #include <cuda.h>
@@ -28,12 +28,12 @@ constexpr int kBoxRows = 32, kBoxCols = 32;
 constexpr uint32_t kBoxBytes = kBoxRows * kBoxCols * 4;
 
 // [rows][cols], 16-byte aligned, cols a multiple of 4; what lies beyond the array reads as zero bits.  The x coordinate of every copy is a
-// multiple of 32 values.
-inline CUtensorMap boxMap(const void *data, int rows, int cols, CUtensorMapSwizzle swizzle) {
+// multiple of the box's columns, which are a multiple of 4.
+inline CUtensorMap boxMap(const void *data, int rows, int cols, CUtensorMapSwizzle swizzle, int boxCols = kBoxCols, int boxRows = kBoxRows) {
     CUtensorMap map;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 4};
-    const cuuint32_t box[2] = {kBoxCols, kBoxRows};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(boxCols), static_cast<cuuint32_t>(boxRows)};
     const cuuint32_t elementStrides[2] = {1, 1};
     const CUresult rc = encodeTiled()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(data), dims, strides, box, elementStrides,
                                       CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
