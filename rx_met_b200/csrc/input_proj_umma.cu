@@ -10,13 +10,14 @@
 // epilogue, so the per-channel constants (multiplier, shift, offset, gate rescale) live in registers, and
 // for a given row the 32 lanes of a warp store 32 neighbouring channels: 64 contiguous bytes of codes.
 //
-// Work item = 128 channels x kRows rows; CTAs walk the items with a grid stride.  Per CTA, once: the
-// weight codes of ALL channels as the K-major A operand in the un-swizzled canonical layout (core matrix
-// = 8 channels x 16 k-bytes).  Per item: the code rows (contiguous in HBM) are placed into the canonical
-// K-major B layout by plain 4-byte loads and stores (a row is I bytes, not a multiple of 16, so no bulk
-// copy fits), one thread issues K/32 MMAs into one of two accumulator buffers and commits them to that
-// buffer's mbarrier; the epilogue of the previous item runs meanwhile: tcgen05.ld (lane = channel, 16 rows
-// per load), integer rescale with round-half-even, clamp, optional second rescale onto the gate-input grid.
+// A CTA keeps one tile of 128 channels and walks a contiguous range of rows, 64 at a time.  Once: its channels' weight codes as the K-major
+// A operand in the un-swizzled canonical layout (core matrix = 8 channels x 16 k-bytes) and the constants of the
+// epilogue.  Per item: the code rows (contiguous in HBM) come into the canonical K-major B layout as 4-byte asynchronous copies (a row
+// is I bytes, not a multiple of 16, so no bulk copy fits), asked for two items ahead; one thread issues K/32 MMAs into one of two
+// accumulator buffers and commits them to that buffer's mbarrier; the epilogue of the previous item runs meanwhile: tcgen05.ld (lane =
+// channel, 16 rows per load), integer rescale with round-half-even, clamp, optional second rescale onto the gate-input grid.
+// Bound: issue of the epilogue.  25,600 rows, I = 40, 384 channels 24.0 -> 21.4 us against CTAs that walked items of all channel tiles,
+// fetched each item's constants and waited for its rows.
 // Every mbarrier wait is bounded; a wait that gives up sets the status word (the recurrent kernel that
 // consumes the codes turns its outputs into NaN then) and the CTA still frees its tensor memory.
 #include <algorithm>
@@ -57,14 +58,14 @@ __device__ __forceinline__ void mmaI8(uint32_t tmemD, uint64_t descA, uint64_t d
         : "memory");
 }
 
-// Rows of the batch per work item = accumulator columns.  25,600 rows of 384 channels are 1200 items of 64 rows: four to five for each of the 296
-// CTAs, where 600 of 128 rows were two to three.
-constexpr int kRows = 64;
+// Rows of the batch per item = accumulator columns.  A CTA keeps one tile of 128 channels, whose constants stay in its threads' registers,
+// and walks a contiguous range of rows, cut at multiples of 16.
+constexpr int kRows = 64, kRowStep = 16;
 
 __host__ __device__ inline int paddedC(int C) { return (C + kTileM - 1) / kTileM * kTileM; }
-size_t sharedBytes(int C, int kPad) { return static_cast<size_t>(paddedC(C)) * kPad + 2 * static_cast<size_t>(kRows) * kPad; }
+size_t sharedBytes(int kPad) { return static_cast<size_t>(kTileM + 2 * kRows) * kPad; }
 
-__global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
+__global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p, int rowsPerCta) {
     constexpr uint32_t kTmemCols = 2 * kRows;
     constexpr uint32_t kIdesc = instructionDescriptorI8(kRows);
     extern __shared__ __align__(128) uint8_t smem[];
@@ -73,10 +74,12 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
     __shared__ int failed;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = warpIndex();
-    const int C = p.C, padded = paddedC(C), kWords = p.kWords, kPad = p.kPad;
+    const int C = p.C, kWords = p.kWords, kPad = p.kPad, channelTiles = paddedC(C) / kTileM;
+    const int ct = static_cast<int>(blockIdx.x) % channelTiles, rowBegin = static_cast<int>(blockIdx.x) / channelTiles * rowsPerCta;
+    const int rowEnd = min(p.rows, rowBegin + rowsPerCta), items = (rowEnd - rowBegin + kRows - 1) / kRows;
     const uint32_t groupStride = static_cast<uint32_t>(kPad / 16) * kCore;  // next 8 channels / 8 rows
-    uint8_t *weights = smem;                                               // [padded / 8][kPad / 16][8][16]
-    uint8_t *rowStages = smem + static_cast<size_t>(padded) * kPad;             // 2 x [kRows / 8][kPad / 16][8][16]
+    uint8_t *weights = smem;                                               // [kTileM / 8][kPad / 16][8][16]
+    uint8_t *rowStages = smem + static_cast<size_t>(kTileM) * kPad;             // 2 x [kRows / 8][kPad / 16][8][16]
     const size_t stageBytes = static_cast<size_t>(kRows) * kPad;
 
     if (tid == 0) {
@@ -90,33 +93,33 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     // operands start as zeros: the k padding of both and the channels beyond C are never written again
-    for (size_t i = tid; i < (static_cast<size_t>(padded) * kPad + 2 * stageBytes) / 16; i += kThreads)
+    for (size_t i = tid; i < (static_cast<size_t>(kTileM) * kPad + 2 * stageBytes) / 16; i += kThreads)
         reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     waitForPredecessor();
     if (!p.late) letDependentsStart();
     // weight word (kw, c) = codes k = 4 kw .. 4 kw + 3 of channel c -> four consecutive bytes of row c
-    for (int i = tid; i < kWords * C; i += kThreads) {
-        const int kw = i / C, c = i - kw * C;
-        *reinterpret_cast<int32_t *>(weights + (c >> 3) * groupStride + (kw >> 2) * kCore + (c & 7) * 16 + (kw & 3) * 4) = p.w[i];
+    for (int i = tid; i < kWords * kTileM; i += kThreads) {
+        const int kw = i / kTileM, local = i % kTileM, c = ct * kTileM + local;
+        if (c < C)
+            *reinterpret_cast<int32_t *>(weights + (local >> 3) * groupStride + (kw >> 2) * kCore + (local & 7) * 16 + (kw & 3) * 4) = p.w[static_cast<size_t>(kw) * C + c];
     }
 
-    const int channelTiles = padded / kTileM;
-    const int rowTiles = (p.rows + kRows - 1) / kRows;
-    const int items = rowTiles * channelTiles;
-
-    // the code words of a row tile are one contiguous run of kRows * kWords words
+    // the code words of an item's rows are one contiguous run; rows beyond the range become zeros
     auto loadRows = [&](int item, int stage) {
-        const int tile = item / channelTiles;
-        const size_t first = static_cast<size_t>(tile) * kRows * kWords;
-        const size_t limit = static_cast<size_t>(p.rows) * kWords;
+        const size_t first = static_cast<size_t>(rowBegin + item * kRows) * kWords;
+        const size_t limit = static_cast<size_t>(rowEnd) * kWords;
         uint8_t *dst = rowStages + stage * stageBytes;
         for (int i = tid; i < kRows * kWords; i += kThreads) {
             const int r = i / kWords, kw = i - r * kWords;
-            const int32_t v = first + i < limit ? p.x[first + i] : 0;
-            *reinterpret_cast<int32_t *>(dst + (r >> 3) * groupStride + (kw >> 2) * kCore + (r & 7) * 16 + (kw & 3) * 4) = v;
+            const bool real = first + i < limit;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smemAddr(dst + (r >> 3) * groupStride + (kw >> 2) * kCore + (r & 7) * 16 + (kw & 3) * 4)),
+                         "l"(p.x + (real ? first + i : 0)), "r"(real ? 4u : 0u)
+                         : "memory");
         }
     };
+
+    for (int n = 0; n < min(2, items); ++n) loadRows(n, n);
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -128,33 +131,35 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
     // second rescale: |code| and |zero point| below 2^20 keep the product inside 32-bit pieces
     const bool gridsSmall = lo >= -(1 << 20) && hi <= (1 << 20) && zpOut >= -(1 << 20) && zpOut <= (1 << 20);
 
-    auto epilogue = [&](int item, int local) {
-        const int buf = local & 1;
-        if (!waitPhase(smemAddr(&bars[buf]), (local >> 1) & 1)) failed = 1;
+    const bool real = ct * kTileM + 32 * q + lane < C;
+    const int c = min(ct * kTileM + 32 * q + lane, C - 1);  // this thread's channel
+    // per-channel constants in registers.  Narrow channels (|offset| < 2^30, a multiplier that shrinks,
+    // shift in [1, 31]) round with 32-bit pieces of the product; the others take the 64-bit form.
+    const Rescale rs = p.rescale[c];
+    const int64_t offset = p.biasAcc[c] - p.comp[c];
+    const bool narrow = rs.shift >= 1 && rs.shift <= 31 && rs.mult > 0 && static_cast<int64_t>(rs.mult) <= (1ll << rs.shift) &&
+                        offset > -(1ll << 30) && offset < (1ll << 30);
+    const Rescale gateRs = p.pre.enabled ? p.pre.toGate[c / p.pre.hidden] : Rescale{1, 0};
+    const bool gateNarrow = gridsSmall && gateRs.shift >= 1 && gateRs.shift <= 31 && gateRs.mult > 0 &&
+                            static_cast<int64_t>(gateRs.mult) <= (1ll << min(gateRs.shift + 9, 31));
+    const bool warpNarrow = __all_sync(0xffffffffu, narrow && (!p.pre.enabled || gateNarrow));
+    // Narrow: half a unit rides in the addend, the floor is right then except for an exact tie, where it is the upper neighbour and an
+    // odd one must step down.
+    const int64_t plus = offset * rs.mult + (narrow ? int64_t{1} << (rs.shift - 1) : 0);
+    const int64_t gatePlus = -static_cast<int64_t>(zpOut) * gateRs.mult + (gateNarrow ? int64_t{1} << (gateRs.shift - 1) : 0);
+    const uint32_t tie = (1u << (rs.shift & 31)) - 1u, gateTie = (1u << (gateRs.shift & 31)) - 1u;
+    auto rounded = [](int64_t sum, int shift, uint32_t mask) {
+        const uint32_t low = static_cast<uint32_t>(sum);
+        const int32_t q = static_cast<int32_t>(__funnelshift_r(low, static_cast<uint32_t>(static_cast<uint64_t>(sum) >> 32), shift));
+        return (low & mask) == 0 ? q & ~1 : q;
+    };
+
+    auto epilogue = [&](int item) {
+        const int buf = item & 1;
+        if (!waitPhase(smemAddr(&bars[buf]), (item >> 1) & 1)) failed = 1;
+        // the products have read this stage: the rows of the item after next come in under the epilogue
+        if (item + 2 < items) loadRows(item + 2, buf);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int tile = item / channelTiles, ct = item - tile * channelTiles;
-        const bool real = ct * kTileM + 32 * q + lane < C;
-        const int c = min(ct * kTileM + 32 * q + lane, C - 1);  // this thread's channel
-        // per-channel constants in registers.  Narrow channels (|offset| < 2^30, a multiplier that shrinks,
-        // shift in [1, 31]) round with 32-bit pieces of the product; the others take the 64-bit form.
-        const Rescale rs = p.rescale[c];
-        const int64_t offset = p.biasAcc[c] - p.comp[c];
-        const bool narrow = rs.shift >= 1 && rs.shift <= 31 && rs.mult > 0 && static_cast<int64_t>(rs.mult) <= (1ll << rs.shift) &&
-                            offset > -(1ll << 30) && offset < (1ll << 30);
-        const Rescale gateRs = p.pre.enabled ? p.pre.toGate[c / p.pre.hidden] : Rescale{1, 0};
-        const bool gateNarrow = gridsSmall && gateRs.shift >= 1 && gateRs.shift <= 31 && gateRs.mult > 0 &&
-                                static_cast<int64_t>(gateRs.mult) <= (1ll << min(gateRs.shift + 9, 31));
-        const bool warpNarrow = __all_sync(0xffffffffu, narrow && (!p.pre.enabled || gateNarrow));
-        // Narrow: half a unit rides in the addend, the floor is right then except for an exact tie, where it is the upper neighbour and an
-        // odd one must step down.
-        const int64_t plus = offset * rs.mult + (narrow ? int64_t{1} << (rs.shift - 1) : 0);
-        const int64_t gatePlus = -static_cast<int64_t>(zpOut) * gateRs.mult + (gateNarrow ? int64_t{1} << (gateRs.shift - 1) : 0);
-        const uint32_t tie = (1u << (rs.shift & 31)) - 1u, gateTie = (1u << (gateRs.shift & 31)) - 1u;
-        auto rounded = [](int64_t sum, int shift, uint32_t mask) {
-            const uint32_t low = static_cast<uint32_t>(sum);
-            const int32_t q = static_cast<int32_t>(__funnelshift_r(low, static_cast<uint32_t>(static_cast<uint64_t>(sum) >> 32), shift));
-            return (low & mask) == 0 ? q & ~1 : q;
-        };
         for (int chunk = group; chunk < kRows / 16; chunk += kThreads / 128) {
             uint32_t acc[16];
             asm volatile(
@@ -164,7 +169,7 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
                   "=r"(acc[8]), "=r"(acc[9]), "=r"(acc[10]), "=r"(acc[11]), "=r"(acc[12]), "=r"(acc[13]), "=r"(acc[14]), "=r"(acc[15])
                 : "r"(tmem + (static_cast<uint32_t>(32 * q) << 16) + static_cast<uint32_t>(buf * kRows + 16 * chunk)));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            const int row0 = tile * kRows + 16 * chunk, count = real ? p.rows - row0 : 0;
+            const int row0 = rowBegin + item * kRows + 16 * chunk, count = real ? rowEnd - row0 : 0;
             planeproj::Column<int16_t> to(p.out, row0, c, C);
             planeproj::Column<uint8_t> toMask(p.mask, row0, c, C);
             if (warpNarrow) {
@@ -200,27 +205,22 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p) {
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     };
 
-    int local = 0, previous = -1;
-    for (int item = blockIdx.x; item < items; item += gridDim.x, ++local) {
-        const int stage = local & 1;
-        loadRows(item, stage);
+    for (int item = 0; item < items; ++item) {
+        const int stage = item & 1;
+        asm volatile("cp.async.wait_all;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (warp == 0 && electOne()) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int ct = item % channelTiles;
-            const uint32_t aBase = smemAddr(weights) + static_cast<uint32_t>(ct * (kTileM / 8)) * groupStride;
-            const uint32_t bBase = smemAddr(rowStages + stage * stageBytes);
-            const uint64_t descA = operandDescriptor(aBase, kCore, groupStride), descB = operandDescriptor(bBase, kCore, groupStride);
+            const uint64_t descA = operandDescriptor(smemAddr(weights), kCore, groupStride), descB = operandDescriptor(smemAddr(rowStages + stage * stageBytes), kCore, groupStride);
             constexpr uint64_t kStep = (2 * kCore) >> 4;   // the start-address field counts 16-byte units
             for (int ks = 0; ks < kPad / 32; ++ks)
                 mmaI8(tmem + stage * kRows, descA + ks * kStep, descB + ks * kStep, kIdesc, ks > 0 ? 1u : 0u);
             commitTo(smemAddr(&bars[stage]));
         }
-        if (previous >= 0) epilogue(previous, local - 1);
-        previous = item;
+        if (item > 0) epilogue(item - 1);
     }
-    if (previous >= 0) epilogue(previous, local - 1);
+    if (items > 0) epilogue(items - 1);
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -237,19 +237,20 @@ bool eligible(int C, int H, int kWords, const void *x, const void *out, const vo
     static const bool disabled = std::getenv("RXMET_IPROJ_SIMT") != nullptr;
     (void)H; (void)out; (void)mask;
     if (disabled || kWords < 1 || !alignedTo(x, 4)) return false;
-    return sharedBytes(C, paddedK(kWords)) <= 200 * 1024;  // all weight codes and two row stages in one SM
+    return static_cast<size_t>(paddedC(C) + 2 * kRows) * paddedK(kWords) <= 200 * 1024;
 }
 
 void launch(const Problem &problem, int sms, cudaStream_t st) {
     Problem prob = problem;
     prob.kPad = paddedK(prob.kWords);
-    const size_t smem = sharedBytes(prob.C, prob.kPad);
+    const size_t smem = sharedBytes(prob.kPad);
     ensureDynamicSmem(reinterpret_cast<const void *>(inputProjUmma), smem);
-    const int items = ((prob.rows + kRows - 1) / kRows) * (paddedC(prob.C) / kTileM);
-    const int grid = std::max(1, std::min(items, 2 * sms));
+    const int channelTiles = paddedC(prob.C) / kTileM, most = std::max(1, 2 * sms / channelTiles);   // ranges of rows
+    const int rowsPerCta = ((prob.rows + most - 1) / most + kRowStep - 1) / kRowStep * kRowStep;
+    const int grid = (prob.rows + rowsPerCta - 1) / rowsPerCta * channelTiles;
     prob.late = prob.dependents > 0 && grid + prob.dependents > sms;
     KernelTimer timer__("inputLinear", st);
-    launchDependent(inputProjUmma, grid, kThreads, smem, st, prob);
+    launchDependent(inputProjUmma, grid, kThreads, smem, st, prob, rowsPerCta);
 }
 
 }  // namespace iproj

@@ -223,6 +223,14 @@ def test_forward_quant_planes_beyond_the_clusters(gl, shape):
     test_forward_quant_matches_restatement(gl, "a16", shape)
 
 
+@pytest.mark.parametrize("cfg_name,shape", [("w8a8", (1, 1, 40, 128)), ("w8a8", (1, 17, 40, 128)), ("w8a8", (1, 1590, 29, 128)), ("w8a8", (1, 9500, 16, 128)),
+                                            ("w8a8", (1, 8200, 40, 100)), ("a16", (1, 19100, 8, 40)), ("a16", (1, 9600, 260, 36)), ("a16", (1, 65, 36, 65))],
+                         ids=lambda s: s if isinstance(s, str) else "x".join(map(str, s)))
+def test_forward_quant_projection_ranges(gl, cfg_name, shape):
+    """Rows of a CTA of the projections: one, a step of 16 and one more, several items of 64 with a ragged last one; row tiles in shares, two slices of k."""
+    test_forward_quant_matches_restatement(gl, cfg_name, shape)
+
+
 @pytest.mark.parametrize("variable,value", [("RXMET_GRU_FWD_MODE", "0"), ("RXMET_GRU_FWD_MODE", "1"), ("RXMET_GRU_FWD_BT", "2")])
 @pytest.mark.parametrize("shape", [(3, 4, 12, 64), (3, 7, 9, 128), (2, 5, 8, 40)], ids=lambda s: "x".join(map(str, s)))
 def test_forward_quant_general_cells(gl, monkeypatch, shape, variable, value):
