@@ -9,7 +9,6 @@ namespace rxmet {
 namespace lstm {
 namespace {
 
-using reverse::kThreads;
 using reverse::Variant;
 
 template <int H, int ROWS>
@@ -29,7 +28,7 @@ Variant variantFor(int H, int rows) {
     if (H > 256) return reverse::wideVariant(H, rows);
     return rows == 4 ? variantFor<4>(H) : rows == 8 ? variantFor<8>(H) : variantFor<16>(H);
 }
-int resident(const Variant &v) { return residentClusters(reinterpret_cast<const void *>(v.kernel), v.ctas, kThreads, v.smem); }
+int resident(const Variant &v) { return residentClusters(reinterpret_cast<const void *>(v.kernel), v.ctas, v.threads, v.smem); }
 
 }  // namespace
 
@@ -49,7 +48,8 @@ void backwardCluster(const BackwardClusterArgs &args, cudaStream_t st) {
     // of the chain of a one-row step, a second wave costs the whole chain again).
     int best = 4;
     double bestCost = 1e30;
-    for (int rows : {4, 8, 16}) {
+    for (int rows : {4, 8, 16, 20}) {
+        if (rows > 16 && args.H <= 256) break;
         if (1.0 + rows / 32.0 >= bestCost) break;   // not even in a single wave: leave the variant unloaded
         const Variant v = variantFor(args.H, rows);
         if (rows > 4 && resident(v) == 0) continue;
@@ -62,7 +62,7 @@ void backwardCluster(const BackwardClusterArgs &args, cudaStream_t st) {
     ensureDynamicSmem(reinterpret_cast<const void *>(v.kernel), v.smem);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(static_cast<unsigned>((args.B + best - 1) / best * v.ctas));
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(static_cast<unsigned>(v.threads));
     cfg.dynamicSmemBytes = v.smem;
     cfg.stream = st;
     cudaLaunchAttribute attr{};

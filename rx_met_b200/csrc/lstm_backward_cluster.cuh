@@ -12,6 +12,8 @@
 //
 // Up to 256 units a CTA owns 64 (32 where 64 do not divide H) of them and a cluster has at most eight CTAs.  Beyond, nine to
 // sixteen CTAs own 32 units each: the weights of 64 would fill tensor memory.  Seven such clusters are resident at once.
+// Their shared memory takes twenty rows where sixteen would need another round of clusters: a step of 2.5 instead of 2.0 us (T = 100, H = 512, 256 rows
+// 618 -> 505 us in two rounds instead of three, 128 rows 413 -> 257 in one).
 // Up to 128 units: unit_reverse_umma.cuh.  T = 100, B = 100, H = 160: about 1 ms -> 91 us (FP32 FMA);
 // T = 1000, B = 256, H = 512: 10.2 -> 6.0 ms, T = 100, B = 112: 1067 -> 213 us (partial sums through L2 and a grid-wide counter per step).
 #pragma once
@@ -32,13 +34,14 @@ namespace reverse {
 
 using namespace bwdcluster;
 
-constexpr int kThreads = 256, kWarps = kThreads / 32;
 constexpr int kOperands = 8;   // 8-byte pieces of a pair of cells: four gates, tanh(cell), previous cell, incoming gradient, flags
 
 // Geometry of a cluster of H / U CTAs that advances ROWS batch rows.
 template <int H, int U, int ROWS>
 struct Tile {
     static constexpr int kCtas = H / U, kTiles = (H + 127) / 128, kSliceK = 4 * U, kGroupsK = kSliceK / 8;
+    // Twenty rows of 32 units are 320 pairs of cells: a thread each, two warps without a tile to read out.
+    static constexpr int kThreads = ROWS == 20 ? 320 : 256, kReadWarps = 8;
     static constexpr int kPairs = U / 2, kRowPass = kThreads / kPairs, kRowsPerThread = (ROWS + kRowPass - 1) / kRowPass;
     static constexpr int kCols = (3 * ROWS + 15) / 16 * 16;          // accumulator columns of one tile of 128 units
     static constexpr uint32_t kColsA = kSliceK / 2;                   // tensor-memory columns of one weight tile
@@ -49,21 +52,21 @@ struct Tile {
     static constexpr uint32_t kPartBytes = static_cast<uint32_t>(ROWS) * H * 4;
     static constexpr uint32_t kRowBytes = kOperands * kThreads * 8;
     static constexpr uint32_t kSlotBytes = kRowsPerThread * kRowBytes;   // operands of one step
-    static constexpr size_t kSharedBytes = kOperandBytes + 4 * kPartBytes + 3 * kSlotBytes + 128;
+    static constexpr size_t kSharedBytes = kOperandBytes + 4 * kPartBytes + 2 * kSlotBytes + 128;
 };
 
 template <int H, int U, int ROWS>
-__global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __grid_constant__ BackwardClusterArgs a) {
+__global__ void __launch_bounds__(Tile<H, U, ROWS>::kThreads, 1) recurrentBackwardCluster(const __grid_constant__ BackwardClusterArgs a) {
     using namespace umma;
     using G = Tile<H, U, ROWS>;
-    constexpr int C = 4 * H, NC = G::kCtas, MT = G::kTiles, RPT = G::kRowsPerThread;
+    constexpr int C = 4 * H, NC = G::kCtas, MT = G::kTiles, RPT = G::kRowsPerThread, kThreads = G::kThreads;
     extern __shared__ __align__(128) uint8_t smemC[];
     __shared__ __align__(8) uint64_t productBar[2], partBar[2];
     __shared__ uint32_t tmemSlot;
     uint8_t *bTile = smemC;                                                    // [kGroupsK][kCols (+1)][16 bytes]
     float *part = reinterpret_cast<float *>(bTile + G::kOperandBytes);         // [2][NC sources][U / 32][ROWS][32 units]
     float *outS = part + 2 * ROWS * H;                                         // [2][H / 32 unit tiles][ROWS][32 units], to be sent
-    uint8_t *ring = reinterpret_cast<uint8_t *>(outS + 2 * ROWS * H);          // [3 slots][RPT][kOperands][threads] x 8 bytes
+    uint8_t *ring = reinterpret_cast<uint8_t *>(outS + 2 * ROWS * H);          // [2 slots][RPT][kOperands][threads] x 8 bytes
 
     const int tid = threadIdx.x, lane = tid & 31, warp = umma::warpIndex();
     const uint32_t rank = cluster::rank();
@@ -95,7 +98,8 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
         dhBase[i] = *reinterpret_cast<const float2 *>(a.gradFinalHidden + o);
         dc[i] = *reinterpret_cast<const float2 *>(a.gradFinalCell + o);
     }
-    // Operands of a step travel two steps ahead through shared memory (a thread reads back what it copied itself).
+    // Operands of a step travel two steps ahead through shared memory (a thread reads back what it copied itself): those of step n + 2 replace
+    // the operands of step n, of which only the factors are left then.
     const size_t first = (static_cast<size_t>(a.T - 1) * a.B + b0 + rowOf) * H + j;   // element of the last step
     const size_t stepH = static_cast<size_t>(a.B) * H;
     const float *gateFrom = a.gateOutputs + (first - j) * 4 + j, *tanhFrom = a.cellTanh + first, *gradFrom = a.gradOutput + first;
@@ -123,7 +127,7 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
 #pragma unroll 1
-    for (int n = 0; n < 3; ++n) {
+    for (int n = 0; n < 2; ++n) {
         if (n < a.T) fetch(a.T - 1 - n, n * G::kSlotBytes);
         commit();
     }
@@ -131,7 +135,7 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
     __syncthreads();
     const uint32_t tmem = tmemSlot, tmemWeights = tmem + MT * G::kCols;
     // weights: lane = hidden unit m, column = two of this CTA's 4 U channels
-    for (int tile = warp >> 2; tile < MT; tile += kWarps / 4) {
+    for (int tile = warp >> 2; tile < MT && warp < G::kReadWarps; tile += G::kReadWarps / 4) {
         const int m = tile * 128 + 32 * (warp & 3) + lane;
         for (int kg = 0; kg < G::kGroupsK; ++kg) {
             const int gate = kg / (U / 8), within = kg % (U / 8) * 8;
@@ -202,14 +206,14 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
     };
     // role in the product's read-out: a warp carries tiles of 32 units, up to two, and kSpan of the rows of each
     constexpr int kSpan = MT == 1 ? ROWS / 2 : ROWS, kReadouts = (MT + 1) / 2;
-    const int quarter = warp & 3, row0 = MT == 1 ? (warp >> 2) * kSpan : 0;
+    const int quarter = warp & 3, half = min(warp >> 2, 1), row0 = MT == 1 ? half * kSpan : 0;
     uint32_t column[kReadouts], sendTo[kReadouts], sendBar[kReadouts];
     float *outMine[kReadouts];
     bool tileReal[kReadouts];
 #pragma unroll
     for (int i = 0; i < kReadouts; ++i) {
-        const int tile = MT == 1 ? 0 : (warp >> 2) + 2 * i, unit0 = tile * 128 + 32 * quarter;
-        tileReal[i] = unit0 < H;
+        const int tile = MT == 1 ? 0 : half + 2 * i, unit0 = tile * 128 + 32 * quarter;
+        tileReal[i] = unit0 < H && warp < G::kReadWarps;
         column[i] = tmem + (static_cast<uint32_t>(32 * quarter) << 16) + static_cast<uint32_t>(tile * G::kCols + row0);
         const uint32_t owner = min(static_cast<uint32_t>(unit0) / U, static_cast<uint32_t>(NC - 1));
         sendTo[i] = cluster::remote(smemAddr(part), owner) + ((rank * U + static_cast<uint32_t>(unit0) % U) * ROWS + row0 * 32) * 4;
@@ -231,8 +235,10 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
             fy[i] = factorsOf({g0.y, g1.y, g2.y, g3.y}, ct.y, cell.y, grad.y, bits.y);
         }
     };
-    asm volatile("cp.async.wait_group 2;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
     prepare(0);
+    if (a.T > 2) fetch(a.T - 3, 0);
+    commit();
     uint32_t slot = 0;   // of the current step
 #pragma unroll 1
     for (int n = 0; n < a.T; ++n) {
@@ -301,7 +307,7 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
         }
         ihTo -= 4 * stepH;
         hhTo -= 4 * stepH;
-        const uint32_t nextSlot = slot == 2 * G::kSlotBytes ? 0 : slot + G::kSlotBytes;
+        const uint32_t nextSlot = G::kSlotBytes - slot;
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         if (n + 1 < a.T) prepare(nextSlot);
         // partial sums -> the CTAs that own the units.  A warp without a tile in some pair waits for that pair too: the next step
@@ -311,7 +317,7 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
             wait(smemAddr(&productBar[i]), n & 1);
             if (!tileReal[i]) continue;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            constexpr int kLoad = kSpan < 8 ? kSpan : 8;
+            constexpr int kLoad = kSpan % 8 == 0 ? 8 : kSpan < 4 ? kSpan : 4;
             float *out = outMine[i] + (n & 1) * (ROWS * H);
 #pragma unroll
             for (int r = 0; r < kSpan; r += kLoad) {
@@ -328,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
             if (lane == 0) cluster::copyTo(sendTo[i] + (n & 1) * G::kPartBytes, smemAddr(out), kSpan * 128, sendBar[i] + (n & 1) * 8);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        if (n + 3 < a.T) fetch(a.T - 1 - (n + 3), slot);   // while the partial sums travel
+        if (n + 3 < a.T) fetch(a.T - 1 - (n + 3), nextSlot);   // while the partial sums travel
         commit();
         slot = nextSlot;
     }
@@ -351,11 +357,11 @@ __global__ void __launch_bounds__(kThreads, 1) recurrentBackwardCluster(const __
 struct Variant {
     void (*kernel)(BackwardClusterArgs);
     size_t smem;
-    int ctas;
+    int ctas, threads;
 };
 template <int H, int U, int ROWS>
 Variant variant() {
-    return Variant{recurrentBackwardCluster<H, U, ROWS>, Tile<H, U, ROWS>::kSharedBytes, H / U};
+    return Variant{recurrentBackwardCluster<H, U, ROWS>, Tile<H, U, ROWS>::kSharedBytes, H / U, Tile<H, U, ROWS>::kThreads};
 }
 // The variants beyond 256 hidden units, built in lstm_backward_cluster_wide.cu.
 Variant wideVariant(int H, int rows);

@@ -26,7 +26,7 @@ Variant variantFor(int H) {
 
 }  // namespace
 
-Variant wideVariant(int H, int rows) { return rows == 4 ? variantFor<4>(H) : rows == 8 ? variantFor<8>(H) : variantFor<16>(H); }
+Variant wideVariant(int H, int rows) { return rows == 4 ? variantFor<4>(H) : rows == 8 ? variantFor<8>(H) : rows == 16 ? variantFor<16>(H) : variantFor<20>(H); }
 
 }  // namespace reverse
 }  // namespace lstm

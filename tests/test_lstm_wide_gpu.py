@@ -157,9 +157,10 @@ def test_wide_calibration_session_matches_the_reference():
 
 @pytest.mark.parametrize("T,B,I,H,wb,ab", [(1, 1, 1, 1, 8, 16), (3, 4, 29, 31, 8, 16), (2, 5, 37, 150, 8, 16), (2, 130, 6, 160, 4, 16),
                                            (3, 9, 33, 224, 8, 16), (2, 3, 8, 255, 4, 16), (3, 9, 12, 96, 8, 16),
-                                           (1, 1, 12, 288, 8, 16), (3, 9, 29, 350, 8, 16), (2, 130, 16, 480, 4, 16), (3, 17, 6, 500, 4, 16), (4, 400, 6, 500, 4, 16)])
+                                           (1, 1, 12, 288, 8, 16), (3, 9, 29, 350, 8, 16), (2, 130, 16, 480, 4, 16), (3, 17, 6, 500, 4, 16), (4, 400, 6, 500, 4, 16),
+                                           (2, 150, 8, 512, 8, 16), (5, 256, 8, 512, 4, 16), (1, 139, 8, 288, 8, 16)])
 def test_wide_qat_backward_over_clusters_and_padded_widths(T, B, I, H, wb, ab):
-    """The cluster recurrence at its widths of 32 and 64 units per CTA, one to sixteen CTAs and 4, 8 and 16 rows, and widths beside those that
+    """The cluster recurrence at its widths of 32 and 64 units per CTA, one to sixteen CTAs and 4, 8, 16 and 20 rows, and widths beside those that
     the tensor-core kernels tile, which go through padded copies
     (the last: rows cut into chunks of 512)."""
     test_wide_qat_backward(T, B, I, H, wb, ab)
