@@ -197,6 +197,7 @@ __global__ void packStepMasks(const uint8_t *__restrict__ mIh, const uint8_t *__
             bit(mGateIn, gi + H, 4) | bit(mGateIn, gi + 2 * H, 5) | bit(mHh, gi, 6) | bit(mHh, gi + H, 7) |
             bit(mHh, gi + 2 * H, 8) | bit(mIh, gi, 9) | bit(mIh, gi + H, 10) | bit(mIh, gi + 2 * H, 11) | bit(mH, at, 12));
     }
+    waitForPredecessor();   // launched beside regroupArrays, whose output it does not read: whoever waits for this kernel waits for both
 }
 
 // The same packing, four hidden units per thread (H a multiple of 4, flag bytes 0 or 1, as every
@@ -1134,8 +1135,8 @@ void backwardPadded(const BackwardCall &call, void *workspace, size_t workspaceB
     if (call.stepFlags || mk.weight_ih_linear || mk.weight_hh_linear || mk.gate_input || mk.gate_output || mk.h) {
         {
             KernelTimer timer__("packStepMasks", st);
-            packStepMasks<<<gridFor(rows * Hp, 256), 256, 0, st>>>(mk.weight_ih_linear, mk.weight_hh_linear, mk.gate_input, mk.gate_output,
-                                                                   mk.h, call.stepFlags, rows, H, Hp, o.bits);
+            launchDependent(packStepMasks, static_cast<unsigned>(gridFor(rows * Hp, 256)), 256, 0, st, mk.weight_ih_linear, mk.weight_hh_linear, mk.gate_input,
+                            mk.gate_output, mk.h, call.stepFlags, rows, H, Hp, o.bits);
         }
         afterLaunch("packStepMasks");
         inner.stepFlags = o.bits;
@@ -1233,6 +1234,16 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
     const bool slabGrads = qat && !tensorGrads && !simtGrads && call.exec->actClass != CodeClass::I32 && I % 4 == 0 && H % 4 == 0 &&
                            alignedTo(call.x_q, 16) && alignedTo(call.h, 16) && wgrad::tensorMemoryPath(I, H, C);
 
+    // H > 128 with 8-bit weight codes: the codes stay in shared memory for the whole sequence
+    const int hpCodes = (H + 31) / 32 * 32;
+    const int partsCodes = std::max(1, std::min(4, 512 / hpCodes));
+    auto codesSmem = [&](int rb) {
+        return static_cast<size_t>(C) * H + sizeof(float) * (static_cast<size_t>(rb) * C + static_cast<size_t>(partsCodes) * rb * H);
+    };
+    const bool codesPath = qat && !registerPath && call.exec->weightClass == CodeClass::I8 && C % 4 == 0 && hpCodes <= 512 &&
+                           codesSmem(1) + 1024 <= static_cast<size_t>(smemMax) && alignedTo(call.R_q, 16) &&
+                           std::getenv("RXMET_GRU_BWD_GENERIC") == nullptr;
+
     const float *W = call.W, *R = call.R, *x = call.x;
     const float *chanScaleR = nullptr, *chanScaleW = nullptr;
     if (qat) {  // rebuild the real-valued operands that the remaining float kernels read
@@ -1247,7 +1258,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
             dequantCodes<<<gridFor(static_cast<size_t>(I) * C, 256), 256, 0, st>>>(call.W_q, static_cast<size_t>(I) * C, C, chan, 0.f, 0, Wf);
             afterLaunch("dequantCodes");
         }
-        if (!registerPath) {
+        if (!registerPath && !codesPath) {
             KernelTimer timer__("dequantCodes", st);
             dequantCodes<<<gridFor(static_cast<size_t>(H) * C, 256), 256, 0, st>>>(call.R_q, static_cast<size_t>(H) * C, C, chan + C, 0.f, 0, Rf);
             afterLaunch("dequantCodes");
@@ -1263,15 +1274,6 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
         chanScaleW = chan;
     }
 
-    // H > 128 with 8-bit weight codes: the codes stay in shared memory for the whole sequence
-    const int hpCodes = (H + 31) / 32 * 32;
-    const int partsCodes = std::max(1, std::min(4, 512 / hpCodes));
-    auto codesSmem = [&](int rb) {
-        return static_cast<size_t>(C) * H + sizeof(float) * (static_cast<size_t>(rb) * C + static_cast<size_t>(partsCodes) * rb * H);
-    };
-    const bool codesPath = qat && !registerPath && call.exec->weightClass == CodeClass::I8 && C % 4 == 0 && hpCodes <= 512 &&
-                           codesSmem(1) + 1024 <= static_cast<size_t>(smemMax) && alignedTo(call.R_q, 16) &&
-                           std::getenv("RXMET_GRU_BWD_GENERIC") == nullptr;
     if (call.stepFlags && !registerPath && !codesPath)   // the kernels behind these two read byte masks
         fail(RXMET_ERR_UNSUPPORTED, "packed step flags beyond 128 units need 16-byte aligned weight codes");
     if (codesPath) {

@@ -10,6 +10,7 @@
 #include <cstdint>
 
 #include "common.h"
+#include "dependent_launch.cuh"
 #include "rxmet_b200.h"
 
 namespace rxmet {
@@ -21,6 +22,7 @@ constexpr int kLossCtasPerSm = 8;
 __global__ void __launch_bounds__(kLossThreads) mseLossGrad(const float *__restrict__ out, const float *__restrict__ target,
                                                             uint64_t count, float factor, int vector,
                                                             float *__restrict__ grad, float *__restrict__ partial) {
+    letDependentsStart();
     float acc = 0.0f;
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kLossThreads;
     const uint64_t first = static_cast<uint64_t>(blockIdx.x) * kLossThreads + threadIdx.x;
@@ -59,6 +61,7 @@ __global__ void __launch_bounds__(kLossThreads) mseLossGrad(const float *__restr
 }
 
 __global__ void __launch_bounds__(256) mseLossFinish(const float *__restrict__ partial, int parts, double count, float *loss) {
+    waitForPredecessor();   // and nobody starts early behind it: a recurrence beside the CTAs of mseLossGrad shares out its own CTAs unevenly
     double acc = 0.0;
     for (int i = threadIdx.x; i < parts; i += blockDim.x) acc += static_cast<double>(partial[i]);
     __shared__ double part[8];
@@ -99,7 +102,7 @@ int rxmet_mse_loss_grad(const float *out_dev, const float *target_dev, uint64_t 
         float *partial = static_cast<float *>(workspace_dev);
         mseLossGrad<<<grid, kLossThreads, 0, st>>>(out_dev, target_dev, count, factor, vector ? 1 : 0, grad_dev, partial);
         afterLaunch("mseLossGrad");
-        mseLossFinish<<<1, 256, 0, st>>>(partial, grid, static_cast<double>(count), loss_dev);
+        launchDependent(mseLossFinish, 1, 256, 0, st, partial, grid, static_cast<double>(count), loss_dev);
         afterLaunch("mseLossFinish");
     });
 }

@@ -98,6 +98,30 @@ def test_forward_quant_matches_restatement(gl, cfg_name, shape):
     assert np.array_equal(gl.forward_int_io(*prob[:4], want["x_q"], h0_q, params), want["h_q"])
 
 
+@pytest.mark.parametrize("shape", [(3, 5, 8, 64), (2, 40, 64, 96), (1, 3, 7, 33)], ids=lambda s: "x".join(map(str, s)))
+def test_codes_of_inputs_next_to_a_tie(gl, shape):
+    """16-bit codes of x at ties of the quotient, one and two floats beside them, on the grid, outside it, and of every magnitude."""
+    import ctypes as C
+    cfg = ol.make_config(**CONFIGS["a16"])
+    (W, R, bw, br, x, h0), params = calibrated(shape, seed=3, cfg=cfg, with_h0=False)
+    scale = C.c_float()
+    assert cabi.load_library().rxmet_gru_decode_effective_scale(C.c_float(params.c.scale[0]), 0, C.byref(scale)) == 0
+    rng = np.random.default_rng(11)
+    k = rng.integers(-40000, 40000, x.shape)
+    v = ((k + 0.5) * np.float64(scale.value)).astype(np.float32)
+    for _ in range(2):
+        side = rng.integers(-1, 2, x.shape)
+        v = np.where(side > 0, np.nextafter(v, np.float32(np.inf)), np.where(side < 0, np.nextafter(v, np.float32(-np.inf)), v))
+    some = rng.random(x.shape)
+    v = np.where(some < 0.1, k * np.float64(scale.value), np.where(some < 0.2, np.float32(10.0) ** rng.uniform(-44, 38, x.shape) * rng.choice([-1, 1], x.shape), v))
+    x = v.astype(np.float32)
+    x.flat[:3] = [0.0, np.inf, -np.inf]
+    want = ol.forward_quant("orc", W, R, bw, br, x, h0, params)
+    rc, got = gl.forward_quant(W, R, bw, br, x, h0, params)
+    assert rc == 0, got
+    assert_forward_equal(got, want)
+
+
 def test_forward_quant_saturating_inputs(gl):
     """Inputs far outside the calibrated range exercise every clamp mask."""
     cfg = ol.make_config(bits=8, symmetric=False)
