@@ -383,7 +383,7 @@ struct QuantDequant : torch::autograd::Function<QuantDequant> {
         if (wantOffset) out[2] = emptyLike(x, saved[2].sizes());
         if (wantScale || wantOffset) {
             bytes = rxmet_affine_qdq_backward_workspace_bytes(outer, channels, inner);
-            ws = emptyLike(x, {static_cast<int64_t>(std::max<size_t>(bytes, 4))}, at::kByte);
+            if (bytes > 0) ws = emptyLike(x, {static_cast<int64_t>(bytes)}, at::kByte);
         }
         auto raw = [](const Tensor &t) { return t.defined() ? static_cast<float *>(t.data_ptr()) : nullptr; };
         checkQdq(rxmet_affine_qdq_backward(raw(g), raw(x), outer, channels, inner, raw(s), raw(o), static_cast<int>(plan[0]),

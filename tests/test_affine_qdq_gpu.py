@@ -229,3 +229,12 @@ def test_traced_quantize_dequantize(trained):
         assert torch.equal(*grads)
     out = affine_qdq.QuantDequantFunc.apply(y, s, o, -128, 127, not trained)
     assert torch.equal(out, want) and isinstance(affine_qdq.QuantDequantFunc, type(torch.autograd.Function))
+
+
+@pytest.mark.parametrize("rows,inner", [
+    (3, 8192),       # the longest row that one block sums
+    (3, 8193),       # the next one: two segments and a second launch
+    (2500, 1025),    # blocks that sum several rows one after the other, rows of every alignment
+])
+def test_sums_of_rows_with_a_grid_each(rows, inner):
+    test_cuda_matches_the_restatement_on_larger_tensors((rows, inner), (rows, 1), -128, 127)
