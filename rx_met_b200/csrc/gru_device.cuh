@@ -89,6 +89,30 @@ __device__ __forceinline__ int32_t quantizeValue(float v, float scale, int32_t z
     return static_cast<int32_t>(code < lo ? lo : (code > hi ? hi : code));
 }
 
+// quantizeValue on one grid for many values, without a branch or a conversion.  The quotient comes from the reciprocal and two
+// corrections by the exact remainder: the second gives the correctly rounded quotient, because the first left one within a unit of its last place and the
+// reciprocal is correctly rounded (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990, theorem on division).
+// A quotient below a quarter, whose remainder may lose bits, rounds to zero all the same.
+struct CodeGrid {
+    float scale, inverse, least, most;   // values beyond `least` and `most` are off the grid and stay so when cut off there
+    int32_t lo, first, span;             // first: lo - zp
+    bool plain;                          // the form holds: not for scales near the ends of the float range or wide grids
+    __device__ __forceinline__ CodeGrid(float s, int32_t zp, int32_t l, int32_t h) {
+        constexpr int kLimit = 1 << 20;
+        scale = s; inverse = __frcp_rn(s); lo = l; first = l - zp; span = h - l;
+        least = static_cast<float>(first - 2) * s; most = static_cast<float>(first + span + 2) * s;
+        plain = s > 0x1p-100f && s < 0x1p100f && abs(zp) < kLimit && abs(l) < kLimit && abs(h) < kLimit;
+    }
+    // code - lo; NaN is the lower end and not kept, as in quantizeValue
+    __device__ __forceinline__ int32_t place(float v, uint32_t &keep) const {
+        const float a = fminf(fmaxf(v, least), most), q0 = __fmul_rn(a, inverse);
+        const float q1 = __fmaf_rn(__fmaf_rn(-q0, scale, a), inverse, q0), q2 = __fmaf_rn(__fmaf_rn(-q1, scale, a), inverse, q1);
+        const int32_t u = __float_as_int(__fadd_rn(q2, 12582912.0f)) - (__float_as_int(12582912.0f) + first);   // 1.5 * 2^23: the integer in the low bits
+        keep = static_cast<uint32_t>(u) <= static_cast<uint32_t>(span) ? 1 : 0;
+        return max(0, min(u, span));
+    }
+};
+
 // 16-segment table: first segment whose threshold exceeds q_x, else the last
 // (quantize_ops_helper.h:503-532).
 template <bool Narrow = false>

@@ -35,6 +35,7 @@
 #include "gru_forward_wide.h"
 #include "input_proj_umma.h"
 #include "plane_proj_umma.cuh"
+#include "row_words.cuh"
 #include "unit_recurrence_umma.cuh"
 
 namespace rxmet {
@@ -286,13 +287,20 @@ __global__ void __launch_bounds__(32 * kPrepLayers) prepareWeightsI8(const Weigh
 // as packed words (the input weights also as tensor-core tiles), both addends, and x and h0 as byte planes.  Blocks by job:
 // 32 channels, then words of x, then words of h0.  T = 98, B = 32, I = 40, H = 64: 64 -> 5 us of launches.
 struct WidePrepArgs {
-    const float *W, *R, *bw, *br;
-    int I, H, C, kI, kH, tileWords;                // tileWords: words of a channel's row in a tile, k padding included
-    const float *effW, *effR, *effBw, *effBr;
-    int32_t loW, hiW, loR, hiR, loBw, hiBw, loBr, hiBr;
-    uint32_t *wWords, *rWords, *tiles;
-    int32_t *W_q, *R_q, *bw_q, *br_q;              // optional 32-bit copies of the codes
-    uint8_t *mW, *mR, *mBw, *mBr;                  // optional clamp flags
+    struct Matrix {                                // weights [rows][C]
+        const float *src, *scale;
+        int rows, words, allWords;                 // words of a channel; those of a tile's row, k padding included
+        int32_t lo, hi;
+        uint32_t *packed, *tiles;                  // tiles: optional
+        int32_t *codes32;                          // optional 32-bit copies of the codes
+        uint8_t *mask;                             // optional clamp flags
+    } weights[2];                                  // W, R
+    const float *bw, *br;
+    int C, tileWords;
+    const float *effBw, *effBr;
+    int32_t loBw, hiBw, loBr, hiBr;
+    int32_t *bw_q, *br_q;                          // optional, as above
+    uint8_t *mBw, *mBr;
     int64_t zeroX, zeroH;                          // grid minimum - zero point of x and h
     const Rescale *biasRescaleX, *biasRescaleH;
     int64_t *addX, *addH;
@@ -307,38 +315,50 @@ struct WidePrepArgs {
         uint8_t *mask;                             // optional
         int16_t *codes;                            // optional [rows][colsPadded]
         int colsPadded;
-        int vectors;                               // src, codes32 and mask take 16- and 4-byte accesses of four columns, no codes
+        int vectors;                               // src, codes32 and mask take 16- and 4-byte accesses of four columns, rows that eachRowWord takes, no codes
     } x, h0;
     int prepBlocks, xBlocks, h0Blocks;
     int *clear;                                    // status word of a later kernel, set to 0 here
 };
+// kWideLayers warps share a channel's words.
+constexpr int kWideLayers = 32, kWideWords = 4, kWideThreads = 32 * kWideLayers;
+// Whole words: 16-byte loads, 16-byte and 4-byte stores.
+__device__ __forceinline__ void planesOfVectors(const WidePrepArgs::Rows &t, const CodeGrid &grid, int block, int blocks) {
+    eachRowWord<kWideWords>(static_cast<size_t>(t.rows), t.kWords, block, blocks, [&](const RowWord (&at)[kWideWords]) {
+        float4 in[kWideWords];
+        const int words = t.cols / 4;
+#pragma unroll
+        for (int n = 0; n < kWideWords; ++n)
+            if (at[n].real && at[n].word < words) in[n] = reinterpret_cast<const float4 *>(t.src)[at[n].row * words + at[n].word];
+#pragma unroll
+        for (int n = 0; n < kWideWords; ++n) {
+            if (!at[n].real) continue;
+            uint32_t *planes = t.planes + 2 * at[n].row * t.kWords + at[n].word;
+            if (at[n].word >= words) {
+                planes[0] = planes[t.kWords] = 0;
+                continue;
+            }
+            uint32_t k[4];
+            const uint32_t u0 = grid.place(in[n].x, k[0]), u1 = grid.place(in[n].y, k[1]), u2 = grid.place(in[n].z, k[2]), u3 = grid.place(in[n].w, k[3]);
+            const size_t place = at[n].row * words + at[n].word;
+            if (t.codes32) reinterpret_cast<int4 *>(t.codes32)[place] = make_int4(u0 + t.lo, u1 + t.lo, u2 + t.lo, u3 + t.lo);
+            if (t.mask) reinterpret_cast<uint32_t *>(t.mask)[place] = k[0] | k[1] << 8 | k[2] << 16 | k[3] << 24;
+            const uint32_t front = __byte_perm(u0, u1, 0x5410), back = __byte_perm(u2, u3, 0x5410);   // two 16-bit codes each
+            planes[0] = __byte_perm(front, back, 0x7531);
+            planes[t.kWords] = __byte_perm(front, back, 0x6420);
+        }
+    });
+}
 __device__ __forceinline__ void planesOf(const WidePrepArgs::Rows &t, int block, int blocks) {
+    if (t.vectors) {
+        const CodeGrid grid(t.scale, t.zp, t.lo, t.hi);
+        if (grid.plain) return planesOfVectors(t, grid, block, blocks);
+    }
     const size_t total = static_cast<size_t>(t.rows) * t.kWords, stride = static_cast<size_t>(blocks) * blockDim.x;
     for (size_t i = static_cast<size_t>(block) * blockDim.x + threadIdx.x; i < total; i += stride) {
         const size_t r = i / t.kWords;
         const int kw = static_cast<int>(i - r * t.kWords);
         uint32_t high = 0, low = 0;
-        if (t.vectors && 4 * kw < t.cols) {   // whole words: one 16-byte load, one 16-byte and one 4-byte store
-            const size_t at = r * t.cols + 4 * kw;
-            const float4 v = *reinterpret_cast<const float4 *>(t.src + at);
-            const float in[4] = {v.x, v.y, v.z, v.w};
-            int32_t q[4];
-            uint32_t keeps = 0;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                uint8_t keep;
-                q[e] = quantizeValue(in[e], t.scale, t.zp, t.lo, t.hi, keep);
-                keeps |= static_cast<uint32_t>(keep) << (8 * e);
-                const uint32_t u = static_cast<uint32_t>(q[e] - t.lo);
-                low |= (u & 0xffu) << (8 * e);
-                high |= ((u >> 8) & 0xffu) << (8 * e);
-            }
-            if (t.codes32) *reinterpret_cast<int4 *>(t.codes32 + at) = make_int4(q[0], q[1], q[2], q[3]);
-            if (t.mask) *reinterpret_cast<uint32_t *>(t.mask + at) = keeps;
-            t.planes[(2 * r) * t.kWords + kw] = high;
-            t.planes[(2 * r + 1) * t.kWords + kw] = low;
-            continue;
-        }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int k = 4 * kw + e;
@@ -362,47 +382,66 @@ __device__ __forceinline__ void planesOf(const WidePrepArgs::Rows &t, int block,
         t.planes[(2 * r + 1) * t.kWords + kw] = low;
     }
 }
-__global__ void __launch_bounds__(32 * kPrepLayers) prepareWide(const __grid_constant__ WidePrepArgs a) {
-    __shared__ int32_t sums[2][kPrepLayers][32];
+// quantizeValue behind a call, for grids that CodeGrid does not take
+__device__ __noinline__ int32_t quantizeElsewhere(float v, float scale, int32_t lo, int32_t hi, uint32_t &keep) {
+    uint8_t inside;
+    const int32_t q = quantizeValue(v, scale, 0, lo, hi, inside);
+    keep = inside;
+    return q;
+}
+// Bound: every CTA runs through most of the code once, so that fetching it shows before anything else: both matrices, and x and h0, go
+// through the same instructions, a word at a time with the next one's values asked for.  12,800 rows of 512 inputs and 768 channels, two directions at
+// a time, 42 -> 32 us (72 MB each: 4.5 TB/s); 40 inputs 10.3 -> 8.6.  The same with a copy of the code for each matrix and four words unrolled: 63 and 26.
+__global__ void __launch_bounds__(kWideThreads, 1) prepareWide(const __grid_constant__ WidePrepArgs a) {
+    __shared__ int32_t sums[2][kWideLayers][32];
     letDependentsStart();
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.clear = 0;
     const int block = static_cast<int>(blockIdx.x) - a.prepBlocks;
-    if (block >= a.xBlocks) return planesOf(a.h0, block - a.xBlocks, a.h0Blocks);
-    if (block >= 0) return planesOf(a.x, block, a.xBlocks);
+    if (block >= 0) {
+        const bool ofX = block < a.xBlocks;
+        return planesOf(ofX ? a.x : a.h0, ofX ? block : block - a.xBlocks, ofX ? a.xBlocks : a.h0Blocks);
+    }
     const int cl = threadIdx.x & 31, layer = threadIdx.x >> 5, c = blockIdx.x * 32 + cl;
     const bool live = c < a.C;
-    auto pass = [&](const float *__restrict__ src, int rowsK, int words, int allWords, float scale, int32_t lo, int32_t hi,
-                    uint32_t *__restrict__ packed, uint32_t *__restrict__ tiles, int32_t *__restrict__ codes32, uint8_t *__restrict__ mask) {
-        int32_t sum = 0;
-        for (int kk = layer; kk < allWords; kk += kPrepLayers) {
-            float v[4];
+#pragma unroll 1
+    for (int which = 0; which < 2; ++which) {
+        const WidePrepArgs::Matrix &m = a.weights[which];
+        const CodeGrid grid(live ? m.scale[c] : 1.0f, 0, m.lo, m.hi);
+        const float *src = m.src + c;
+        const int rows = live ? m.rows : 0;
+        auto load = [&](int kk, float (&v)[4]) {
 #pragma unroll
-            for (int b = 0; b < 4; ++b) v[b] = live && 4 * kk + b < rowsK ? src[static_cast<size_t>(4 * kk + b) * a.C + c] : 0.0f;
+            for (int b = 0; b < 4; ++b) v[b] = 4 * kk + b < rows ? src[static_cast<size_t>(4 * kk + b) * a.C] : 0.0f;
+        };
+        float next[4];
+        load(layer, next);
+        int32_t sum = 0;
+#pragma unroll 1
+        for (int kk = layer; kk < m.allWords; kk += kWideLayers) {
+            const float v[4] = {next[0], next[1], next[2], next[3]};
+            load(kk + kWideLayers, next);
             uint32_t word = 0;
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
-                const int k = 4 * kk + b;
-                if (!live || k >= rowsK) continue;
-                const size_t at = static_cast<size_t>(k) * a.C + c;
-                uint8_t keep;
-                const int32_t q = quantizeValue(v[b], scale, 0, lo, hi, keep);
-                if (codes32) codes32[at] = q;
-                if (mask) mask[at] = keep;
+                if (4 * kk + b >= rows) continue;
+                const size_t at = static_cast<size_t>(4 * kk + b) * a.C + c;
+                uint32_t keep;
+                const int32_t q = grid.plain ? grid.place(v[b], keep) + m.lo : quantizeElsewhere(v[b], grid.scale, m.lo, m.hi, keep);
+                if (m.codes32) m.codes32[at] = q;
+                if (m.mask) m.mask[at] = static_cast<uint8_t>(keep);
                 sum += q;
                 word |= static_cast<uint32_t>(q & 0xff) << (8 * b);
             }
-            if (live && kk < words) packed[static_cast<size_t>(kk) * a.C + c] = word;
-            if (tiles) tiles[4 * planeproj::tilePlace(c, kk / 4, 4 * a.tileWords) + kk % 4] = word;
+            if (live && kk < m.words) m.packed[static_cast<size_t>(kk) * a.C + c] = word;
+            if (m.tiles) m.tiles[4 * planeproj::tilePlace(c, kk / 4, 4 * a.tileWords) + kk % 4] = word;
         }
-        return sum;
-    };
-    sums[0][layer][cl] = pass(a.W, a.I, a.kI, a.tiles ? a.tileWords : a.kI, live ? a.effW[c] : 1.0f, a.loW, a.hiW, a.wWords, a.tiles, a.W_q, a.mW);
-    sums[1][layer][cl] = pass(a.R, a.H, a.kH, a.kH, live ? a.effR[c] : 1.0f, a.loR, a.hiR, a.rWords, nullptr, a.R_q, a.mR);
+        sums[which][layer][cl] = sum;
+    }
     __syncthreads();
     if (layer != 0 || !live) return;
     int64_t totalW = 0, totalR = 0;
 #pragma unroll
-    for (int l = 0; l < kPrepLayers; ++l) {
+    for (int l = 0; l < kWideLayers; ++l) {
         totalW += sums[0][l][cl];
         totalR += sums[1][l][cl];
     }
@@ -1445,14 +1484,15 @@ void runWide(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaStr
     const WideOperands o = wideOperands(ws, T, B, I, H);
 
     WidePrepArgs p{};
-    p.W = call.W; p.R = call.R; p.bw = call.bw; p.br = call.br;
-    p.I = I; p.H = H; p.C = C; p.kI = o.kI; p.kH = o.kH; p.tileWords = o.tileWords;
-    p.effW = ch.effW; p.effR = ch.effR; p.effBw = ch.effBw; p.effBr = ch.effBr;
-    p.loW = g.qlo[RXMET_GRU_W]; p.hiW = g.qhi[RXMET_GRU_W]; p.loR = g.qlo[RXMET_GRU_R]; p.hiR = g.qhi[RXMET_GRU_R];
+    p.weights[0] = {call.W, ch.effW, I, o.kI, o.wTiles ? o.tileWords : o.kI, g.qlo[RXMET_GRU_W], g.qhi[RXMET_GRU_W],
+                    o.wWords, reinterpret_cast<uint32_t *>(o.wTiles), call.W_q, mk.W};
+    p.weights[1] = {call.R, ch.effR, H, o.kH, o.kH, g.qlo[RXMET_GRU_R], g.qhi[RXMET_GRU_R], o.rWords, nullptr, call.R_q, mk.R};
+    p.bw = call.bw; p.br = call.br;
+    p.C = C; p.tileWords = o.tileWords;
+    p.effBw = ch.effBw; p.effBr = ch.effBr;
     p.loBw = g.qlo[RXMET_GRU_BW]; p.hiBw = g.qhi[RXMET_GRU_BW]; p.loBr = g.qlo[RXMET_GRU_BR]; p.hiBr = g.qhi[RXMET_GRU_BR];
-    p.wWords = o.wWords; p.rWords = o.rWords; p.tiles = reinterpret_cast<uint32_t *>(o.wTiles);
-    p.W_q = call.W_q; p.R_q = call.R_q; p.bw_q = call.bw_q; p.br_q = call.br_q;
-    p.mW = mk.W; p.mR = mk.R; p.mBw = mk.bw; p.mBr = mk.br;
+    p.bw_q = call.bw_q; p.br_q = call.br_q;
+    p.mBw = mk.bw; p.mBr = mk.br;
     p.zeroX = static_cast<int64_t>(g.qlo[RXMET_GRU_X]) - g.zp[RXMET_GRU_X];
     p.zeroH = static_cast<int64_t>(g.qlo[RXMET_GRU_H]) - g.zp[RXMET_GRU_H];
     p.biasRescaleX = ch.biasX; p.biasRescaleH = ch.biasH;
@@ -1467,12 +1507,14 @@ void runWide(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaStr
     };
     p.x = tensor(RXMET_GRU_X, call.x, call.x_codes_in, rows, I, o.kI, o.xPlanes);
     p.x.codes32 = call.x_codes_in ? nullptr : call.x_q; p.x.mask = mk.x;
-    p.x.vectors = I % 4 == 0 && p.x.src && alignedTo(p.x.src, 16) && alignedTo(p.x.codes32, 16) && alignedTo(p.x.mask, 4);
+    p.x.vectors = I % 4 == 0 && p.x.src && alignedTo(p.x.src, 16) && alignedTo(p.x.codes32, 16) && alignedTo(p.x.mask, 4) &&
+                  p.x.kWords <= (1 << 15) / kWideWords;
     p.h0 = tensor(RXMET_GRU_H, call.h0, call.h0_codes_in, static_cast<size_t>(B), H, o.kH, o.h0Planes);
     p.h0.mask = mk.h0; p.h0.codes = o.h0Codes; p.h0.colsPadded = o.hPad;
-    constexpr int kBlock = 32 * kPrepLayers;
+    const int most = 2 * currentDevice().sms;
     auto blocksFor = [&](const WidePrepArgs::Rows &r) {
-        return static_cast<int>(std::min<size_t>((static_cast<size_t>(r.rows) * r.kWords + kBlock - 1) / kBlock, 4 * 148));
+        return r.vectors ? rowWordBlocks(static_cast<size_t>(r.rows), r.kWords, kWideWords, kWideThreads, most)
+                         : static_cast<int>(std::min<size_t>((static_cast<size_t>(r.rows) * r.kWords + kWideThreads - 1) / kWideThreads, most));
     };
     p.prepBlocks = o.wTiles ? planeproj::paddedC(C) / 32 : (C + 31) / 32;
     p.xBlocks = blocksFor(p.x); p.h0Blocks = blocksFor(p.h0);
@@ -1480,7 +1522,7 @@ void runWide(const ForwardQuantCall &call, const Exec &e, Workspace &ws, cudaStr
     if (forwardPhase() != ForwardPhase::Recurrence) {
         {
             KernelTimer timer__("prepareWeights", st);
-            prepareWide<<<p.prepBlocks + p.xBlocks + p.h0Blocks, kBlock, 0, st>>>(p);
+            prepareWide<<<p.prepBlocks + p.xBlocks + p.h0Blocks, kWideThreads, 0, st>>>(p);
         }
         afterLaunch("prepareWeights");
     }
