@@ -291,21 +291,17 @@ inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s
             arrive(&accFree[acc.at]);   // the products of a later tile may overwrite the accumulator
         }
     } else if (warp == kGradientWarp) {
-        Turn slot;
-        int issued = 0;
-        for (int tile = 0; tile < tiles && !failed; ++tile) {
+        int tile = 0, c = 0;   // of the next chunk
+        fillRing(total, s.ring, rawFull, rawFree, failed, wait, [&](int, int place) {
             const int boxes = boxesOf(tile), row = rowBegin + tile * kTileM + lane * kBoxRows;
-            for (int c = 0; c < chunks && !failed; ++c) {
-                if (slot.again) wait(&rawFree[slot.at], slot.parity ^ 1u);
-                if (__any_sync(0xffffffffu, failed)) break;
-                if (lane == 0) expect(&rawFull[slot.at], boxes * kBoxBytes);
-                __syncwarp();
-                if (lane < boxes) copyBox(smemAddr(raw + slot.at * kRawBytes + lane * kBoxBytes), &gradients, c * kChunk, row, smemAddr(&rawFull[slot.at]));
-                ++issued;
-                slot.step(s.ring);
+            if (lane == 0) expect(&rawFull[place], boxes * kBoxBytes);
+            __syncwarp();
+            if (lane < boxes) copyBox(smemAddr(raw + place * kRawBytes + lane * kBoxBytes), &gradients, c * kChunk, row, smemAddr(&rawFull[place]));
+            if (++c == chunks) {
+                c = 0;
+                ++tile;
             }
-        }
-        for (int g = max(0, issued - s.ring); g < issued; ++g) waitPhase(smemAddr(&rawFull[g % s.ring]), (g / s.ring) & 1);   // nothing is left in flight
+        });
     } else if (warp == kWeightWarp) {
         if (STREAM && electOne()) {
             Turn slot;

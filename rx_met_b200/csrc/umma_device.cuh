@@ -142,6 +142,22 @@ struct Turn {
     }
 };
 
+// The loop of a copy warp: ask(i, place) issues the copies of chunk i, which complete on full[place]; a place is asked for again once its
+// chunk was read (`wait` on freed[place]).  After a wait of the CTA that gave up (`failed`) the warp leaves by vote, all lanes after the same chunk: `failed`
+// may change between the reads of two lanes.  Nothing is left in flight when it returns the number of chunks asked for.
+template <class Wait, class Ask>
+__device__ __forceinline__ int fillRing(int chunks, int ring, uint64_t *full, uint64_t *freed, const volatile int &failed, Wait wait, Ask ask) {
+    Turn slot;
+    int issued = 0;
+    for (; issued < chunks; ++issued, slot.step(ring)) {
+        if (slot.again) wait(&freed[slot.at], slot.parity ^ 1u);
+        if (__any_sync(0xffffffffu, failed)) break;
+        ask(issued, slot.at);
+    }
+    for (int i = max(0, issued - ring); i < issued; ++i) waitPhase(smemAddr(&full[i % ring]), (i / ring) & 1);
+    return issued;
+}
+
 __device__ __forceinline__ void tmemLoad32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "

@@ -237,13 +237,9 @@ __global__ void __launch_bounds__(kThreads, 1) weightGradUmma(const __grid_const
     } else if (warp == kCopyWarp) {
         // a box per lane: a lone lane takes 90 cycles a box, longer than 128 elements take to multiply
         const CUtensorMap *gradients = &set.gradients[tile.problem], *codes = &set.codes[tile.problem], *first = &set.first[tile.problem];
-        Turn slot;
-        int issued = 0;
-        for (int c = 0; c < chunks && !failed; ++c, slot.step(tile.ring)) {
+        fillRing(chunks, tile.ring, rawFull, rawFree, failed, wait, [&](int c, int place) {
             const int chunk = chunkBegin + c, row = rowOf(chunk);
-            if (slot.again) wait(&rawFree[slot.at], slot.parity ^ 1u);
-            if (__any_sync(0xffffffffu, failed)) break;
-            const uint32_t bar = smemAddr(&rawFull[slot.at]), to = smemAddr(raw + slot.at * slotBytes);
+            const uint32_t bar = smemAddr(&rawFull[place]), to = smemAddr(raw + place * slotBytes);
             if (lane == 0)
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((gradientBoxes + boxes) * kBoxBytes) : "memory");
             __syncwarp();
@@ -253,9 +249,7 @@ __global__ void __launch_bounds__(kThreads, 1) weightGradUmma(const __grid_const
                 const int b = lane - kTileM / kBoxCols;
                 copyBox(to + lane * kBoxBytes, chunk < firstChunks ? first : codes, tile.m0 + b * kBoxCols, chunk < firstChunks ? row : row - p.firstRows, bar);
             }
-            issued = c + 1;
-        }
-        for (int c = max(0, issued - tile.ring); c < issued; ++c) waitPhase(smemAddr(&rawFull[c % tile.ring]), (c / tile.ring) & 1);   // nothing is left in flight
+        });
     } else if (electOne()) {
         // A: K-major in tensor memory, B: MN-major in shared memory
         const uint32_t idesc = instructionDescriptor(NP, false, true), others = tmem + (tile.accs - 1) * NP;
@@ -465,19 +459,32 @@ void addPartials(float *a, size_t countA, float *b, size_t countB, int partials,
 
 namespace {
 
-// One warp polls a barrier that nothing completes, with the poll loop of the tcgen05 kernels.
+// One warp polls a barrier that nothing completes, with the poll loop of the tcgen05 kernels, then fills a ring whose places nothing frees, with
+// the loop of their copy warps.  status: 1 where both gave up, the lanes of the second after the same chunk; 2 otherwise.
 __global__ void boundedWaitProbe(int *status, unsigned int *polls) {
-    __shared__ __align__(8) uint64_t bar;
+    constexpr int kRing = 2;
+    __shared__ __align__(8) uint64_t bar, full[kRing], freed[kRing];
+    __shared__ volatile int failed;
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(umma::smemAddr(&bar)) : "memory");
+        failed = 0;
+        for (uint64_t *b : {&bar, &full[0], &full[1], &freed[0], &freed[1]}) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(umma::smemAddr(b)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     uint32_t made = 0;
     const bool completed = umma::waitPhase(umma::smemAddr(&bar), 0, &made);
+    const int issued = umma::fillRing(
+        8, kRing, full, freed, failed,
+        [&](uint64_t *b, uint32_t parity) {
+            if (threadIdx.x == 5 && !umma::waitPhase(umma::smemAddr(b), parity)) failed = 1;   // one lane finds out
+        },
+        [&](int, int place) {
+            if (threadIdx.x == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smemAddr(&full[place])) : "memory");
+        });
+    const bool together = __all_sync(0xffffffffu, issued == kRing);
     if (threadIdx.x == 0) {
         *polls = made;
-        if (!completed) atomicExch(status, 1);
+        atomicExch(status, !completed && failed && together ? 1 : 2);
     }
 }
 
@@ -499,6 +506,7 @@ extern "C" int rxmet_selftest_bounded_wait(int *status_dev, unsigned int *polls_
         RXMET_CUDA(cudaMemcpyAsync(&polls, pollsDev, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
         RXMET_CUDA(cudaStreamSynchronize(st));
         if (polls_out) *polls_out = polls;
-        if (status != 0) fail(RXMET_ERR_DEVICE_TIMEOUT, "a bounded device-side wait ran out after %u polls", polls);
+        if (status != 1) fail(RXMET_ERR_CUDA, "a bounded device-side wait did not give up as it should (%d)", status);
+        fail(RXMET_ERR_DEVICE_TIMEOUT, "a bounded device-side wait ran out after %u polls", polls);
     });
 }

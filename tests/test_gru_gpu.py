@@ -517,7 +517,9 @@ def test_kws_body_layer_shapes(gl, cfg_name, shape):
 
 def test_bounded_device_wait_gives_up_with_a_status(gl):
     """The poll loop of the tcgen05 kernels on a barrier nothing completes: the kernel returns after its
-    limit, the status word is set, the call reports RXMET_ERR_DEVICE_TIMEOUT and the context keeps working."""
+    limit, the status word is set, the call reports RXMET_ERR_DEVICE_TIMEOUT and the context keeps working.  The kernel
+    then fills a ring whose places nothing frees, with the loop of the copy warps: one lane finds out, all leave after the same
+    chunk (the status would be 2 otherwise)."""
     import torch
     lib = cabi.load_library()
     status = torch.zeros(2, dtype=torch.int32, device="cuda")
