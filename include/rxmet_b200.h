@@ -94,7 +94,8 @@ RXMET_API int rxmet_stage_from_pinned_host(void *dst_dev, const void *src_host, 
 /* Self-test of the bounded device-side wait that the tcgen05 kernels use: launches one CTA that
  * polls an mbarrier nothing ever arrives on, with the kernels' own poll loop and limit, and fills a
  * ring whose places nothing frees, with the loop of their copy warps.  The kernel gives up when the
- * limits run out, sets status_dev[0] to 1 and returns (2: one of the two did not give up); the call waits
+ * limits run out, sets status_dev[0] to 1 and returns (2: one of the two did not give up, 3: a
+ * second kernel, whose warps take the chunks of a ring in turn, was let through to a chunk that had not been asked for); the call waits
  * for it and returns RXMET_ERR_DEVICE_TIMEOUT, the context stays usable.  status_dev: two ints of
  * device memory (status, polls made); polls_out (optional, host) receives the number of polls. */
 RXMET_API int rxmet_selftest_bounded_wait(int *status_dev, unsigned int *polls_out, void *stream);

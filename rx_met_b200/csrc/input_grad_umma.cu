@@ -95,7 +95,7 @@ template <bool STREAM>   // weights chunk by chunk
 __global__ void __launch_bounds__(kThreads, 1)
 inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s, const __grid_constant__ CUtensorMap gradients) {
     extern __shared__ __align__(1024) uint8_t smemRaw[];
-    __shared__ __align__(8) uint64_t rawFull[kMaxRing], rawFree[kMaxRing], termsFull[kMaxStages], termsFree[kMaxStages], weightsFull[kWeightRing],
+    __shared__ __align__(8) uint64_t rawFull[2 * kMaxRing], rawFree[kMaxRing], termsFull[kMaxStages], termsFree[kMaxStages], weightsFull[kWeightRing],
         weightsFree[kWeightRing], accFull[2], accFree[2];
     __shared__ uint32_t tmemSlot;
     __shared__ volatile int failed;
@@ -115,7 +115,8 @@ inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s
         auto init = [](uint64_t *bar, uint32_t count) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smemAddr(bar)), "r"(count) : "memory");
         };
-        for (int i = 0; i < kMaxRing; ++i) { init(&rawFull[i], 1); init(&rawFree[i], kConvWarps / 2); }
+        for (int i = 0; i < 2 * kMaxRing; ++i) init(&rawFull[i], 1);
+        for (int i = 0; i < kMaxRing; ++i) init(&rawFree[i], kConvWarps / 2);
         for (int i = 0; i < kMaxStages; ++i) { init(&termsFull[i], kConvWarps / 2); init(&termsFree[i], 1); }
         for (int i = 0; i < kWeightRing; ++i) { init(&weightsFull[i], STREAM ? 1 : kFillWarps); init(&weightsFree[i], 1); }
         for (int i = 0; i < 2; ++i) { init(&accFull[i], 1); init(&accFree[i], kEpilogueWarps); }
@@ -170,22 +171,23 @@ inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s
     if (warp < kConvWarps) {
         const int quarter = warp & 3, part = (warp >> 2) & 1, group = warp >> 3, sw = lane & 7;
         const uint32_t lanes = static_cast<uint32_t>(32 * quarter) << 16;
-        Turn slot, stage;
-        slot.step(s.ring, group);
+        RingTurn slot(s.ring, group);
+        Turn stage;
         stage.step(s.stages, group);
         int tile = 0, c = group;
         while (c >= chunks) { c -= chunks; ++tile; }
         bool real = quarter < boxesOf(tile);   // lanes of absent rows keep what they held
         for (int g = group; g < total; g += 2) {
-            wait(&rawFull[slot.at], slot.parity);
-            const uint8_t *row = raw + slot.at * kRawBytes + quarter * kBoxBytes + lane * 128;
+            const int place = slot.place();
+            wait(&rawFull[slot.full.at], slot.full.parity);
+            const uint8_t *row = raw + place * kRawBytes + quarter * kBoxBytes + lane * 128;
             float v[16];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const float4 x = *reinterpret_cast<const float4 *>(row + (((4 * part + i) ^ sw) << 4));
                 v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
             }
-            arrive(&rawFree[slot.at]);
+            arrive(&rawFree[place]);
             if (stage.again) wait(&termsFree[stage.at], stage.parity ^ 1u);
             __syncwarp();
             if (real) {
@@ -211,7 +213,7 @@ inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             }
             arrive(&termsFull[stage.at]);
-            slot.step(s.ring, 2);
+            slot.step(2);
             stage.step(s.stages, 2);
             for (c += 2; c >= chunks; c -= chunks) real = quarter < boxesOf(++tile);
         }
@@ -292,11 +294,11 @@ inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s
         }
     } else if (warp == kGradientWarp) {
         int tile = 0, c = 0;   // of the next chunk
-        fillRing(total, s.ring, rawFull, rawFree, failed, wait, [&](int, int place) {
+        fillRing(total, s.ring, rawFull, rawFree, failed, wait, [&](int, int place, uint64_t *bar) {
             const int boxes = boxesOf(tile), row = rowBegin + tile * kTileM + lane * kBoxRows;
-            if (lane == 0) expect(&rawFull[place], boxes * kBoxBytes);
+            if (lane == 0) expect(bar, boxes * kBoxBytes);
             __syncwarp();
-            if (lane < boxes) copyBox(smemAddr(raw + place * kRawBytes + lane * kBoxBytes), &gradients, c * kChunk, row, smemAddr(&rawFull[place]));
+            if (lane < boxes) copyBox(smemAddr(raw + place * kRawBytes + lane * kBoxBytes), &gradients, c * kChunk, row, smemAddr(bar));
             if (++c == chunks) {
                 c = 0;
                 ++tile;

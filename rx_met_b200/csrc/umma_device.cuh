@@ -142,19 +142,31 @@ struct Turn {
     }
 };
 
-// The loop of a copy warp: ask(i, place) issues the copies of chunk i, which complete on full[place]; a place is asked for again once its
-// chunk was read (`wait` on freed[place]).  After a wait of the CTA that gave up (`failed`) the warp leaves by vote, all lanes after the same chunk: `failed`
-// may change between the reads of two lanes.  Nothing is left in flight when it returns the number of chunks asked for.
+// Walks a ring whose chunks two groups of warps take in turn.  A place has two "full" barriers, chunk i that of index i mod 2 ring, so that
+// each barrier belongs to one group.  With one a place, a ring of an odd number of places handed it from group to group, and a group that came for
+// chunk i + ring before chunk i had landed was let through by the phase before it, which has the parity that it waits for.
+struct RingTurn {
+    int ring;
+    Turn full;
+    __device__ __forceinline__ RingTurn(int places, int first) : ring(places) { step(first); }
+    __device__ __forceinline__ void step(int by) { full.step(2 * ring, by); }
+    __device__ __forceinline__ int place() const { return full.at < ring ? full.at : full.at - ring; }
+};
+
+// The loop of a copy warp: ask(i, place, bar) issues the copies of chunk i, which complete on `bar`, one of full[2 ring] (RingTurn); a place is asked
+// for again once its chunk was read (`wait` on freed[place]).  After a wait of the CTA that gave up (`failed`) the warp leaves by vote, all lanes after the same
+// chunk: `failed` may change between the reads of two lanes.  Nothing is left in flight when it returns the number of chunks asked for.
 template <class Wait, class Ask>
 __device__ __forceinline__ int fillRing(int chunks, int ring, uint64_t *full, uint64_t *freed, const volatile int &failed, Wait wait, Ask ask) {
+    RingTurn turn(ring, 0);
     Turn slot;
     int issued = 0;
-    for (; issued < chunks; ++issued, slot.step(ring)) {
+    for (; issued < chunks; ++issued, turn.step(1), slot.step(ring)) {
         if (slot.again) wait(&freed[slot.at], slot.parity ^ 1u);
         if (__any_sync(0xffffffffu, failed)) break;
-        ask(issued, slot.at);
+        ask(issued, slot.at, &full[turn.full.at]);
     }
-    for (int i = max(0, issued - ring); i < issued; ++i) waitPhase(smemAddr(&full[i % ring]), (i / ring) & 1);
+    for (int i = max(0, issued - ring); i < issued; ++i) waitPhase(smemAddr(&full[i % (2 * ring)]), (i / (2 * ring)) & 1);
     return issued;
 }
 

@@ -75,7 +75,7 @@ template <int TERMS>   // of a code
 __global__ void __launch_bounds__(kThreads, 1) weightGradUmma(const __grid_constant__ Pair set) {
     constexpr int kCodeGroups = TERMS == 1 ? 2 : 1, kChunkWarps = kGradientWarps / 2 + kCodeWarps / kCodeGroups;   // of a chunk
     extern __shared__ __align__(1024) uint8_t smemRaw[];
-    __shared__ __align__(8) uint64_t rawFull[kMaxRing], rawFree[kMaxRing], termsFull[kMaxStages], termsFree[kMaxStages], accFull;
+    __shared__ __align__(8) uint64_t rawFull[2 * kMaxRing], rawFree[kMaxRing], termsFull[kMaxStages], termsFree[kMaxStages], accFull;
     __shared__ uint32_t tmemSlot;
     __shared__ volatile int failed;
     __shared__ float biasParts[4][kTileM];
@@ -99,7 +99,8 @@ __global__ void __launch_bounds__(kThreads, 1) weightGradUmma(const __grid_const
         auto init = [](uint64_t *bar, uint32_t count) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smemAddr(bar)), "r"(count) : "memory");
         };
-        for (int i = 0; i < kMaxRing; ++i) { init(&rawFull[i], 1); init(&rawFree[i], kChunkWarps); }
+        for (int i = 0; i < 2 * kMaxRing; ++i) init(&rawFull[i], 1);
+        for (int i = 0; i < kMaxRing; ++i) init(&rawFree[i], kChunkWarps);
         for (int i = 0; i < kMaxStages; ++i) { init(&termsFull[i], kChunkWarps); init(&termsFree[i], 1); }
         init(&accFull, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -133,14 +134,14 @@ __global__ void __launch_bounds__(kThreads, 1) weightGradUmma(const __grid_const
         const int quarter = warp & 3, half = (warp >> 2) & 1, group = warp >> 3;
         const uint32_t lanes = static_cast<uint32_t>(32 * quarter) << 16;
         const bool real = quarter < gradientBoxes;   // lanes of absent channels keep what they held
-        Turn slot, stage;
-        slot.step(tile.ring, group);
+        RingTurn slot(tile.ring, group);
+        Turn stage;
         stage.step(tile.stages, group);
         float bias = 0.0f;
-        for (int c = group; c < chunks; c += 2, slot.step(tile.ring, 2), stage.step(tile.stages, 2)) {
-            const int valid = validOf(chunkBegin + c) - 16 * half;
-            wait(&rawFull[slot.at], slot.parity);
-            const float *column = reinterpret_cast<const float *>(raw + slot.at * slotBytes + quarter * kBoxBytes) + 16 * half * kBoxCols + lane;
+        for (int c = group; c < chunks; c += 2, slot.step(2), stage.step(tile.stages, 2)) {
+            const int valid = validOf(chunkBegin + c) - 16 * half, place = slot.place();
+            wait(&rawFull[slot.full.at], slot.full.parity);
+            const float *column = reinterpret_cast<const float *>(raw + place * slotBytes + quarter * kBoxBytes) + 16 * half * kBoxCols + lane;
             float v[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) v[i] = column[i * kBoxCols];
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(kThreads, 1) weightGradUmma(const __grid_const
 #pragma unroll
                 for (int i = 0; i < 16; ++i) v[i] = i < valid ? v[i] : 0.0f;
             }
-            arrive(&rawFree[slot.at]);
+            arrive(&rawFree[place]);
             float sum[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) sum[i] = v[i] + v[i + 8];
@@ -191,14 +192,15 @@ __global__ void __launch_bounds__(kThreads, 1) weightGradUmma(const __grid_const
         const float inverse = p.aInvScale, offset = kMagic + (p.aCodes ? static_cast<float>(p.aZero) : p.aFloatZero);   // exact: below 2^24
         auto run = [&](auto integersTag) {
             constexpr bool kIntegers = decltype(integersTag)::value;
-            Turn slot, stage;
-            slot.step(tile.ring, turn);
+            RingTurn slot(tile.ring, turn);
+            Turn stage;
             stage.step(tile.stages, turn);
-            for (int c = turn; c < chunks; c += kCodeGroups, slot.step(tile.ring, kCodeGroups), stage.step(tile.stages, kCodeGroups)) {
+            for (int c = turn; c < chunks; c += kCodeGroups, slot.step(kCodeGroups), stage.step(tile.stages, kCodeGroups)) {
                 const bool mine = row < validOf(chunkBegin + c);
-                wait(&rawFull[slot.at], slot.parity);
+                const int place = slot.place();
+                wait(&rawFull[slot.full.at], slot.full.parity);
                 if (stage.again) wait(&termsFree[stage.at], stage.parity ^ 1u);
-                const uint8_t *from = raw + slot.at * slotBytes + kTileM / kBoxCols * kBoxBytes + row * 128;
+                const uint8_t *from = raw + place * slotBytes + kTileM / kBoxCols * kBoxBytes + row * 128;
                 uint8_t *to = stages + stage.at * stageBytes + group * kStride + eighth * kCore + row8 * 16;
 #pragma unroll 2
                 for (int box = firstBox; box < boxes; box += 3 - kCodeGroups) {
@@ -227,7 +229,7 @@ __global__ void __launch_bounds__(kThreads, 1) weightGradUmma(const __grid_const
                     for (int i = 0; i < 4; ++i) word[i] = mine ? packBf16(x[2 * i], x[2 * i + 1]) : 0u;
                     *reinterpret_cast<uint4 *>(at) = make_uint4(word[0], word[1], word[2], word[3]);
                 }
-                arrive(&rawFree[slot.at]);
+                arrive(&rawFree[place]);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 arrive(&termsFull[stage.at]);
             }
@@ -237,9 +239,9 @@ __global__ void __launch_bounds__(kThreads, 1) weightGradUmma(const __grid_const
     } else if (warp == kCopyWarp) {
         // a box per lane: a lone lane takes 90 cycles a box, longer than 128 elements take to multiply
         const CUtensorMap *gradients = &set.gradients[tile.problem], *codes = &set.codes[tile.problem], *first = &set.first[tile.problem];
-        fillRing(chunks, tile.ring, rawFull, rawFree, failed, wait, [&](int c, int place) {
+        fillRing(chunks, tile.ring, rawFull, rawFree, failed, wait, [&](int c, int place, uint64_t *full) {
             const int chunk = chunkBegin + c, row = rowOf(chunk);
-            const uint32_t bar = smemAddr(&rawFull[place]), to = smemAddr(raw + place * slotBytes);
+            const uint32_t bar = smemAddr(full), to = smemAddr(raw + place * slotBytes);
             if (lane == 0)
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((gradientBoxes + boxes) * kBoxBytes) : "memory");
             __syncwarp();
@@ -459,15 +461,20 @@ void addPartials(float *a, size_t countA, float *b, size_t countB, int partials,
 
 namespace {
 
+__device__ __forceinline__ void initProbeBarrier(uint64_t &bar) { asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(umma::smemAddr(&bar)) : "memory"); }
+__device__ __forceinline__ void arriveOnProbe(uint64_t *bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smemAddr(bar)) : "memory"); }
+
 // One warp polls a barrier that nothing completes, with the poll loop of the tcgen05 kernels, then fills a ring whose places nothing frees, with
 // the loop of their copy warps.  status: 1 where both gave up, the lanes of the second after the same chunk; 2 otherwise.
 __global__ void boundedWaitProbe(int *status, unsigned int *polls) {
     constexpr int kRing = 2;
-    __shared__ __align__(8) uint64_t bar, full[kRing], freed[kRing];
+    __shared__ __align__(8) uint64_t bar, full[2 * kRing], freed[kRing];
     __shared__ volatile int failed;
     if (threadIdx.x == 0) {
         failed = 0;
-        for (uint64_t *b : {&bar, &full[0], &full[1], &freed[0], &freed[1]}) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(umma::smemAddr(b)) : "memory");
+        initProbeBarrier(bar);
+        for (uint64_t &b : full) initProbeBarrier(b);
+        for (uint64_t &b : freed) initProbeBarrier(b);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -478,14 +485,55 @@ __global__ void boundedWaitProbe(int *status, unsigned int *polls) {
         [&](uint64_t *b, uint32_t parity) {
             if (threadIdx.x == 5 && !umma::waitPhase(umma::smemAddr(b), parity)) failed = 1;   // one lane finds out
         },
-        [&](int, int place) {
-            if (threadIdx.x == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smemAddr(&full[place])) : "memory");
+        [&](int, int, uint64_t *b) {
+            if (threadIdx.x == 0) arriveOnProbe(b);
         });
     const bool together = __all_sync(0xffffffffu, issued == kRing);
     if (threadIdx.x == 0) {
         *polls = made;
         atomicExch(status, !completed && failed && together ? 1 : 2);
     }
+}
+
+// Two warps that take the chunks of a ring of an odd number of places in turn, as the warps of the gradient kernels do; the first chunk lands
+// long after those behind it.  status: 3 where a warp was let through to a chunk that had not been asked for, or a wait gave up.
+__global__ void ringTurnProbe(int *status) {
+    constexpr int kRing = 3, kChunks = 24;
+    __shared__ __align__(8) uint64_t full[2 * kRing], freed[kRing];
+    __shared__ volatile int failed, asked;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (threadIdx.x == 0) {
+        failed = asked = 0;
+        for (uint64_t &b : full) initProbeBarrier(b);
+        for (uint64_t &b : freed) initProbeBarrier(b);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    auto wait = [&](uint64_t *b, uint32_t parity) {
+        if (!failed && !umma::waitPhase(umma::smemAddr(b), parity)) failed = 1;
+    };
+    if (warp == 0) {
+        umma::fillRing(kChunks, kRing, full, freed, failed, wait, [&](int i, int, uint64_t *b) {
+            if (lane == 0) {
+                asked = i + 1;
+                if (i > 0) arriveOnProbe(b);
+            }
+            __syncwarp();
+        });
+    } else if (warp == 1) {   // the first chunk
+        for (int i = 0; i < 1000; ++i) __nanosleep(100);
+        if (lane == 0) arriveOnProbe(&full[0]);
+    } else {
+        umma::RingTurn turn(kRing, warp - 2);
+        for (int c = warp - 2; c < kChunks && !__any_sync(0xffffffffu, failed); c += 2, turn.step(2)) {
+            wait(&full[turn.full.at], turn.full.parity);
+            if (c >= asked) failed = 1;   // let through too early
+            if (__any_sync(0xffffffffu, failed)) break;
+            if (lane == 0) arriveOnProbe(&freed[turn.place()]);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && failed) atomicExch(status, 3);
 }
 
 }  // namespace
@@ -500,6 +548,8 @@ extern "C" int rxmet_selftest_bounded_wait(int *status_dev, unsigned int *polls_
         RXMET_CUDA(cudaMemsetAsync(status_dev, 0, 2 * sizeof(int), st));
         boundedWaitProbe<<<1, 32, 0, st>>>(status_dev, pollsDev);
         afterLaunch("boundedWaitProbe");
+        ringTurnProbe<<<1, 128, 0, st>>>(status_dev);
+        afterLaunch("ringTurnProbe");
         int status = 0;
         unsigned int polls = 0;
         RXMET_CUDA(cudaMemcpyAsync(&status, status_dev, sizeof(int), cudaMemcpyDeviceToHost, st));

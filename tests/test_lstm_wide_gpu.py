@@ -173,6 +173,25 @@ def test_weight_gradient_tiles(T, B, I, H, wb, ab):
     test_wide_qat_backward(T, B, I, H, wb, ab)
 
 
+@pytest.mark.parametrize("I,H", [(32, 384), (48, 320), (64, 256), (256, 512)])
+def test_gradients_of_many_rows_are_the_same_in_every_call(I, H):
+    """Rings of odd and even numbers of places (input gradient: five, four and six; weight gradients of more than 128 elements: three), whose chunks two
+    groups of warps take in turn, over enough rows for them to go around many times.  The sums have a fixed order."""
+    T, B, m = 40, 512, mod()
+    p, _, bundle = setup(3, 4, I, H, 4, 16, L.PER_CHANNEL, True, True)
+    gen = torch.Generator(device="cuda").manual_seed(I)
+    normal = lambda *shape: torch.randn(shape, generator=gen, device="cuda")  # noqa: E731
+    weights = [dev(p[k]) for k in ("w_ih", "w_hh", "b_ih", "b_hh")]
+    ck = m.lstm_forward_quantized(normal(T, B, I), *weights, 0.1 * normal(1, B, H), 0.1 * normal(1, B, H), False, bundle, "pedantic", False, True)[3]
+    order = ("input", "weight_ih", "weight_hh", "bias_ih", "bias_hh", "h_0", "c_0")
+    args = ([ck["quantized_master"][n] for n in order], False, bundle, [ck["values"][n] for n in ("gate_outputs", "cell_states", "cell_tanh_outputs", "hidden_outputs")],
+            normal(T, B, H), normal(B, H), normal(B, H), [ck["master_clamp_masks"][n] for n in order], [ck["clamp_masks"][n] for n in L.TRACE_VALUES])
+    first = [t.clone() for t in m.lstm_backward_qat(*args)]
+    assert all(t.isfinite().all() for t in first)
+    for _ in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(first, m.lstm_backward_qat(*args)))
+
+
 @pytest.mark.parametrize("B", [170, 250, 350, 700])
 def test_wide_forward_at_the_row_counts_of_a_cluster(B):
     """Twelve, sixteen or 24, 24 and 48 rows of a cluster, two or three groups of warps over them, a partial last tile of units."""
