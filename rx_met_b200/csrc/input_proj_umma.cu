@@ -246,7 +246,10 @@ void launch(const Problem &problem, int sms, cudaStream_t st) {
     const size_t smem = sharedBytes(prob.kPad);
     ensureDynamicSmem(reinterpret_cast<const void *>(inputProjUmma), smem);
     const int channelTiles = paddedC(prob.C) / kTileM, most = std::max(1, 2 * sms / channelTiles);   // ranges of rows
-    const int rowsPerCta = ((prob.rows + most - 1) / most + kRowStep - 1) / kRowStep * kRowStep;
+    // Up to two CTAs an SM a range is one item: cut finer, the projection of a few thousand rows sits on all SMs, and a recurrence that is launched
+    // beside it finds room for its CTAs on some of them only (T 100, B 32, I 100, H 64: 3200 rows on 200 CTAs 60 us, on 100 43; a QAT step 142 and 119).
+    const bool whole = (prob.rows + kRows - 1) / kRows * channelTiles <= 2 * sms;
+    const int rowsPerCta = whole ? kRows : ((prob.rows + most - 1) / most + kRowStep - 1) / kRowStep * kRowStep;
     const int grid = (prob.rows + rowsPerCta - 1) / rowsPerCta * channelTiles;
     prob.late = prob.dependents > 0 && grid + prob.dependents > sms;
     KernelTimer timer__("inputLinear", st);
