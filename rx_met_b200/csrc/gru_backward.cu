@@ -1528,8 +1528,13 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
             ph.partial = ws.take<float>(static_cast<size_t>(nh) * (H + 1) * C);
         };
         if (wgrad::tensorMemoryPath(I, H, C)) {
-            const wgrad::PairPlan plan = wgrad::planPair(px, ph, K, C, wideCodes, sms);
-            if (padded && wgrad::planRows(plan) > wgrad::kChainRows) {
+            wgrad::PairPlan plan = wgrad::planPair(px, ph, K, C, wideCodes, sms);
+            bool chain = padded && wgrad::planRows(plan) > wgrad::kChainRows;
+            if (chain && wgrad::chainChunks(K) > wgrad::kChainGroup) {
+                const wgrad::PairPlan fine = wgrad::finePlan(px, ph, K, C, sms);
+                if (fine.splits[0] > 0) { plan = fine; chain = false; }
+            }
+            if (chain) {
                 room(wgrad::chainPartials(K), wgrad::chainPartials(K));
                 splitsX = splitsH = wgrad::launchChained(px, ph, K, C, wideCodes, st);
             } else {

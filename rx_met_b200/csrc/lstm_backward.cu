@@ -954,10 +954,15 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
             } else {
                 previous();
             }
-            const wgrad::PairPlan plan = wgrad::planPair(px, ph, K, C, wideCodes, currentDevice().sms);
+            wgrad::PairPlan plan = wgrad::planPair(px, ph, K, C, wideCodes, currentDevice().sms);
+            bool chain = padded && wgrad::planRows(plan) > wgrad::kChainRows;
+            if (chain && wgrad::chainChunks(K) > wgrad::kChainGroup) {
+                const wgrad::PairPlan fine = wgrad::finePlan(px, ph, K, C, currentDevice().sms);
+                if (fine.splits[0] > 0) { plan = fine; chain = false; }
+            }
             splitsX = plan.splits[0];
             splitsH = plan.splits[1];
-            if (padded && wgrad::planRows(plan) > wgrad::kChainRows) {
+            if (chain) {
                 if (ph.aFirst) previous();
                 splitsX = splitsH = wgrad::launchChained(px, ph, K, C, wideCodes, st);
             } else {

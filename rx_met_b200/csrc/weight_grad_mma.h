@@ -68,6 +68,10 @@ inline int chainPartials(int K) { return chainChunks(K) <= kChainGroup ? chainCh
 // sums of a and b (sum[i] = or += partial[0][i] + partial[1][i] + ...), `partial` behind the sums
 void addPartials(float *a, size_t countA, float *b, size_t countB, int partials, bool first, cudaStream_t stream);
 PairPlan chainPlan(int K);   // kChainRows a split
+// More chunks than kChainGroup in one launch all the same, where the partial sums that tileSplitBound makes room for are enough: as many splits, of at
+// most kChainRows rows, as fill whole waves of CTAs.  No splits: not enough room.  8-bit GRU training, T = 100, B = 256, I = 40, H = 16: two launches and two
+// folds 194 us a pass, one launch 179; LSTM, T = 200, B = 200, H = 30 381 -> 331.
+PairPlan finePlan(const Problem &a, const Problem &b, int K, int N, int sms);
 // Both problems in chunks of kChainRows; returns the number of partial sums at a.partial and b.partial.
 inline int launchChained(const Problem &a, const Problem &b, int K, int N, bool wide, cudaStream_t stream) {
     const int chunks = chainChunks(K);

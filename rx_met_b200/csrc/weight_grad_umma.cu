@@ -368,6 +368,24 @@ PairPlan chainPlan(int K) {
     return plan;
 }
 
+PairPlan finePlan(const Problem &a, const Problem &b, int K, int N, int sms) {
+    const Problem *of[2] = {&a, &b};
+    const int room = std::min(tileSplitBound(a.M, N), tileSplitBound(b.M, N)), tiles = (elementTiles(a.M) + elementTiles(b.M)) * channelTiles(N);
+    int chunks[2], least = 1;
+    for (int i = 0; i < 2; ++i) {
+        chunks[i] = chunksOf(K, of[i]->firstRows);
+        least = std::max(least, (chunks[i] * kRows + kChainRows - 1) / kChainRows);
+    }
+    PairPlan plan{};
+    if (least > room) return plan;
+    const int waves = (least * tiles + sms - 1) / sms, splits = std::min(room, std::max(least, waves * sms / tiles));
+    for (int i = 0; i < 2; ++i) {
+        plan.chunks[i] = (chunks[i] + splits - 1) / splits;
+        plan.splits[i] = (chunks[i] + plan.chunks[i] - 1) / plan.chunks[i];
+    }
+    return plan;
+}
+
 int planRows(const PairPlan &plan) { return std::max(plan.chunks[0], plan.chunks[1]) * kRows; }
 
 void launchPair(const Problem &a, const Problem &b, int K, int N, const PairPlan &plan, bool wide, cudaStream_t st) {

@@ -605,6 +605,12 @@ def test_packed_step_flags_equal_the_byte_masks(monkeypatch, shape):
     assert torch.equal(packed.flat_w, plain.flat_w) and torch.equal(lp, lb)
 
 
+@pytest.mark.parametrize("shape", [(1, 16500, 8, 16), (2, 20480, 3, 20), (1, 41500, 4, 16)], ids=lambda s: "x".join(map(str, s)))
+def test_weight_gradient_of_padded_widths_over_many_rows(gl, shape):
+    """More than 32 chunks of 512 rows: in one launch, up to the last split that the partial sums have room for, and in several launches beyond."""
+    test_backward_quant(gl, "w8a8", shape)
+
+
 @pytest.mark.parametrize("shape", [(1, 1, 8, 32), (1, 31, 16, 32), (1, 33, 20, 96), (1, 127, 64, 64), (1, 129, 64, 160), (1, 160, 68, 96), (1, 130, 128, 32),
                                    (2, 65, 132, 32), (1, 40, 256, 64), (1, 40, 260, 32), (1, 19500, 8, 32), (1, 9600, 72, 32), (1, 9600, 260, 32)],
                          ids=lambda s: "x".join(map(str, s)))

@@ -173,6 +173,12 @@ def test_weight_gradient_tiles(T, B, I, H, wb, ab):
     test_wide_qat_backward(T, B, I, H, wb, ab)
 
 
+@pytest.mark.parametrize("T,B,I,H,wb,ab", [(2, 8300, 6, 20, 8, 8), (2, 20600, 4, 20, 8, 16)])
+def test_weight_gradient_of_padded_widths_over_many_rows(T, B, I, H, wb, ab):
+    """More than 32 chunks of 512 rows in one launch, the rows of the initial state by themselves, and in several launches."""
+    test_wide_qat_backward(T, B, I, H, wb, ab)
+
+
 @pytest.mark.parametrize("I,H", [(32, 384), (48, 320), (64, 256), (256, 512)])
 def test_gradients_of_many_rows_are_the_same_in_every_call(I, H):
     """Rings of odd and even numbers of places (input gradient: five, four and six; weight gradients of more than 128 elements: three), whose chunks two
