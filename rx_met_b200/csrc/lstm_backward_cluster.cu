@@ -30,6 +30,20 @@ Variant variantFor(int H, int rows) {
 }
 int resident(const Variant &v) { return residentClusters(reinterpret_cast<const void *>(v.kernel), v.ctas, v.threads, v.smem); }
 
+// A step of clusters of `rows` rows.  Beyond 256 units in us, as measured at 288 and 512 units and on a line between (384: 1.17, 1.35, 1.87, 2.22).  By 1 + rows / 32,
+// which holds for the narrower ones, twenty rows cost 1.08 times sixteen instead of 1.2: of the calls with more than 560 rows some took 1 to 2.5 % longer
+// (T = 60, H = 512, 1000 rows 3350 -> 3269 us a training pass).
+double stepCost(int H, int rows) {
+    if (H <= 256) return 1.0 + rows / 32.0;
+    const double between = (H - 288) / 224.0;
+    switch (rows) {
+        case 4: return 1.13 + 0.11 * between;
+        case 8: return 1.29 + 0.12 * between;
+        case 16: return 1.66 + 0.56 * between;
+        default: return 2.00 + 0.69 * between;
+    }
+}
+
 }  // namespace
 
 bool backwardClusterTakes(const BackwardClusterArgs &a) {
@@ -44,19 +58,18 @@ bool backwardClusterTakes(const BackwardClusterArgs &a) {
 
 void backwardCluster(const BackwardClusterArgs &args, cudaStream_t st) {
     if (args.H <= 128) return backwardUnits(args, st);   // inside one CTA
-    // Rows of a cluster: as few as let all clusters of the pass run at the same time (a step costs about 1 + rows / 32
-    // of the chain of a one-row step, a second wave costs the whole chain again).
+    // Rows of a cluster: as few as let all clusters of the pass run at the same time; a second wave costs the whole chain again.
     int best = 4;
     double bestCost = 1e30;
     for (int rows : {4, 8, 16, 20}) {
         if (rows > 16 && args.H <= 256) break;
-        if (1.0 + rows / 32.0 >= bestCost) break;   // not even in a single wave: leave the variant unloaded
+        const double step = stepCost(args.H, rows);
+        if (step >= bestCost) break;   // not even in a single wave: leave the variant unloaded
         const Variant v = variantFor(args.H, rows);
         if (rows > 4 && resident(v) == 0) continue;
         const int held = std::max(1, resident(v) / concurrentPasses());
         const int clusters = (args.B + rows - 1) / rows, waves = (clusters + held - 1) / held;
-        const double cost = waves * (1.0 + rows / 32.0);
-        if (cost < bestCost) { bestCost = cost; best = rows; }
+        if (waves * step < bestCost) { bestCost = waves * step; best = rows; }
     }
     const Variant v = variantFor(args.H, best);
     ensureDynamicSmem(reinterpret_cast<const void *>(v.kernel), v.smem);

@@ -12,7 +12,7 @@
 //
 // Up to 256 units a CTA owns 64 (32 where 64 do not divide H) of them and a cluster has at most eight CTAs.  Beyond, nine to
 // sixteen CTAs own 32 units each: the weights of 64 would fill tensor memory.  Seven such clusters are resident at once.
-// Their shared memory takes twenty rows where sixteen would need another round of clusters: a step of 2.5 instead of 2.0 us (T = 100, H = 512, 256 rows
+// Their shared memory takes twenty rows where sixteen would need another round of clusters: a step of 2.7 instead of 2.2 us (T = 100, H = 512, 256 rows
 // 618 -> 505 us in two rounds instead of three, 128 rows 413 -> 257 in one).
 // Up to 128 units: unit_reverse_umma.cuh.  T = 100, B = 100, H = 160: about 1 ms -> 91 us (FP32 FMA);
 // T = 1000, B = 256, H = 512: 10.2 -> 6.0 ms, T = 100, B = 112: 1067 -> 213 us (partial sums through L2 and a grid-wide counter per step).
