@@ -2,6 +2,8 @@
 // stream still runs, and calls waitForPredecessor() before it touches anything an earlier kernel wrote or reads.  A kernel
 // calls letDependentsStart() once its own wait is over: all its CTAs are resident then, so that waiting CTAs of the
 // dependent cannot keep any of them from an SM.  Saves the launch latency between short kernels (1.5 to 3 us each).
+// The one exception: packStepMasks (gru_backward.cu) waits only at its end when it is launched right behind regroupArrays, which lets it start after its
+// own wait and writes nothing that it reads; the launch there makes sure of that.
 #pragma once
 
 #include <cuda_runtime.h>

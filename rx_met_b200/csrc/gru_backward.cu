@@ -197,7 +197,7 @@ __global__ void packStepMasks(const uint8_t *__restrict__ mIh, const uint8_t *__
             bit(mGateIn, gi + H, 4) | bit(mGateIn, gi + 2 * H, 5) | bit(mHh, gi, 6) | bit(mHh, gi + H, 7) |
             bit(mHh, gi + 2 * H, 8) | bit(mIh, gi, 9) | bit(mIh, gi + H, 10) | bit(mIh, gi + 2 * H, 11) | bit(mH, at, 12));
     }
-    waitForPredecessor();   // launched beside regroupArrays, whose output it does not read: whoever waits for this kernel waits for both
+    waitForPredecessor();   // launched beside regroupArrays, whose output it does not read (backwardPadded): whoever waits for this kernel waits for both
 }
 
 // The same packing, four hidden units per thread (H a multiple of 4, flag bytes 0 or 1, as every
@@ -1127,7 +1127,8 @@ void backwardPadded(const BackwardCall &call, void *workspace, size_t workspaceB
         copy(call.R_q, o.R, H, Hp, 3, H, Hp),
         copy(scales, o.scales, 2, 2, 3, H, Hp),
     };
-    regroup("padBackward", in, 7, st);
+    // packStepMasks reads the caller's flags before its wait: only behind a kernel that starts it after a wait of its own and does not write them
+    RXMET_REQUIRE(regroup("padBackward", in, 7, st), "nothing to copy in a padded backward");
     rxmet_gru_masks innerMasks{};
     innerMasks.x = mk.x;
     inner.masks = &innerMasks;

@@ -64,23 +64,25 @@ __global__ void __launch_bounds__(kThreads) regroupArrays(const __grid_constant_
 
 }  // namespace
 
-void regroup(const char *name, const RegroupJob *jobs, int count, cudaStream_t st) {
+bool regroup(const char *name, const RegroupJob *jobs, int count, cudaStream_t st) {
     RXMET_REQUIRE(count <= kMaxRegroupJobs, "too many arrays in one launch");
     Jobs all{};
+    const size_t most = 8 * static_cast<size_t>(currentDevice().sms);
     for (int i = 0; i < count; ++i) {
         if (jobs[i].dst == nullptr) continue;
         const size_t items = static_cast<size_t>(jobs[i].rowGroups) * jobs[i].dstRows * jobs[i].colGroups;
         all.job[all.count] = jobs[i];
-        all.firstBlock[all.count + 1] = all.firstBlock[all.count] + static_cast<int>(std::min<size_t>((items + kWarps * kItems - 1) / (kWarps * kItems), 148 * 8));
+        all.firstBlock[all.count + 1] = all.firstBlock[all.count] + static_cast<int>(std::min<size_t>((items + kWarps * kItems - 1) / (kWarps * kItems), most));
         ++all.count;
     }
     const int blocks = all.firstBlock[all.count];
-    if (blocks == 0) return;
+    if (blocks == 0) return false;
     {
         KernelTimer timer__(name, st);
         launchDependent(regroupArrays, static_cast<unsigned>(blocks), kThreads, 0, st, all);
     }
     afterLaunch(name);
+    return true;
 }
 
 }  // namespace rxmet

@@ -20,6 +20,7 @@ struct RegroupJob {
 };
 
 constexpr int kMaxRegroupJobs = 16;
-void regroup(const char *name, const RegroupJob *jobs, int count, cudaStream_t stream);   // one launch
+// One launch; false where no array has anything to copy and nothing was launched.  Kernels behind it may start early, once everything before it is complete.
+bool regroup(const char *name, const RegroupJob *jobs, int count, cudaStream_t stream);
 
 }  // namespace rxmet
