@@ -122,6 +122,69 @@ def test_codes_of_inputs_next_to_a_tie(gl, shape):
     assert_forward_equal(got, want)
 
 
+def effective_scales(scales):
+    import ctypes as C
+    out = []
+    for v in scales:
+        scale = C.c_float()
+        assert cabi.load_library().rxmet_gru_decode_effective_scale(C.c_float(v), 0, C.byref(scale)) == 0
+        out.append(scale.value)
+    return np.array(out, np.float64)
+
+
+def near_ties(shape, scales, limit, seed):
+    """Ties of the quotient by `scales`, up to two floats beside them, on the grid and outside it; multiples of the scale; values of every magnitude."""
+    rng = np.random.default_rng(seed)
+    k = rng.integers(-limit, limit, shape)
+    v = ((k + 0.5) * scales).astype(np.float32)
+    for _ in range(2):
+        side = rng.integers(-1, 2, shape)
+        v = np.where(side > 0, np.nextafter(v, np.float32(np.inf)), np.where(side < 0, np.nextafter(v, np.float32(-np.inf)), v))
+    some = rng.random(shape)
+    v = np.where(some < 0.1, k * scales, np.where(some < 0.2, np.float32(10.0) ** rng.uniform(-44, 38, shape) * rng.choice([-1, 1], shape), v))
+    v = v.astype(np.float32)
+    v.flat[:3] = [0.0, np.inf, -np.inf]
+    return v
+
+
+@pytest.mark.parametrize("shape", [(3, 5, 8, 64), (2, 40, 64, 96), (1, 3, 7, 33)], ids=lambda s: "x".join(map(str, s)))
+def test_codes_of_weights_next_to_a_tie(gl, shape):
+    """8-bit codes and clamp flags of W and R behind 16-bit activations, as test_codes_of_inputs_next_to_a_tie has them of x."""
+    T, B, I, H = shape
+    (_, _, bw, br, x, h0), params = calibrated(shape, seed=3, cfg=ol.make_config(**CONFIGS["a16"]), with_h0=False)
+    W = near_ties((I, 3 * H), effective_scales(params.chan["scale_W"]), 140, seed=5)
+    R = near_ties((H, 3 * H), effective_scales(params.chan["scale_R"]), 140, seed=6)
+    want = ol.forward_quant("orc", W, R, bw, br, x, h0, params)
+    assert all((want["masks"].arr[k] == 0).any() and (want["masks"].arr[k] == 1).any() for k in ("W", "R"))
+    rc, got = gl.forward_quant(W, R, bw, br, x, h0, params)
+    assert rc == 0, got
+    assert_forward_equal(got, want)
+
+
+@pytest.mark.parametrize("exponent", [-101, 101])
+def test_codes_on_grids_near_the_ends_of_the_float_range(gl, exponent):
+    """A scale of x, or of some channels of W and R, beyond 2^-100 and 2^100: the kernel divides there.  Only the codes and flags are
+    compared: the rescales behind them shift by more than 62 places, which nothing defines."""
+    shape = T, B, I, H = 2, 5, 12, 64
+    (W, R, bw, br, x, h0), params = calibrated(shape, seed=3, cfg=ol.make_config(**CONFIGS["a16"]), with_h0=False)
+    def check(names, *problem):
+        want = ol.forward_quant("orc", *problem, h0, params)
+        rc, got = gl.forward_quant(*problem, h0, params)
+        assert rc == 0, got
+        for k in names:
+            assert len(np.unique(want[k + "_q"])) > 20
+            np.testing.assert_array_equal(got[k + "_q"], want[k + "_q"], err_msg=k)
+            np.testing.assert_array_equal(got["masks"][k], want["masks"].arr[k], err_msg=k)
+    scale = params.c.scale[cabi.OP_NAMES.index("x")]
+    params.c.scale[cabi.OP_NAMES.index("x")] = 2.0 ** exponent
+    check(("x",), W, R, bw, br, near_ties((T, B, I), 2.0 ** exponent, 40000, seed=7))
+    params.c.scale[cabi.OP_NAMES.index("x")] = scale
+    for k in ("scale_W", "scale_R"):
+        params.chan[k][::3] = 2.0 ** exponent
+    check(("W", "R"), near_ties((I, 3 * H), effective_scales(params.chan["scale_W"]), 140, seed=8),
+          near_ties((H, 3 * H), effective_scales(params.chan["scale_R"]), 140, seed=9), bw, br, x)
+
+
 def test_forward_quant_saturating_inputs(gl):
     """Inputs far outside the calibrated range exercise every clamp mask."""
     cfg = ol.make_config(bits=8, symmetric=False)
