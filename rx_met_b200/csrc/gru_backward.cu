@@ -1008,8 +1008,7 @@ constexpr int kBiasSplits = 64;
 
 namespace wgrad {
 
-Plan plan(int K, int M, int N, int sms) {
-    (void)M;
+Plan plan(int K, int N, int sms) {
     Plan pl;
     sms = std::min(sms, kMaxSms);
     const int nTiles = (N + gru::kWgCols - 1) / gru::kWgCols;
@@ -1019,9 +1018,8 @@ Plan plan(int K, int M, int N, int sms) {
     return pl;
 }
 
-int splitBound(int K, int M, int N) {
+int splitBound(int K) {
     // about two CTAs per SM spread over the column tiles
-    (void)M;
     return std::max(1, std::min((K + gru::kWgChunk - 1) / gru::kWgChunk, 2 * kMaxSms + 8));
 }
 
@@ -1171,7 +1169,7 @@ size_t tiledWorkspaceBytes(int T, int B, int I, int H, bool padded) {
     ws.take<float>(2 * kBiasSplits * C);
     // tensor-core path: split-K partials of (I+1) and (H+1) rows and the status word
     auto partials = [&](int M) {
-        const int c = static_cast<int>(C), most = std::max(wgrad::tileSplitBound(M, c), M <= 143 ? wgrad::splitBound(static_cast<int>(rows), M, c) : 1);
+        const int c = static_cast<int>(C), most = std::max(wgrad::tileSplitBound(M, c), M <= 143 ? wgrad::splitBound(static_cast<int>(rows)) : 1);
         ws.take<float>(static_cast<size_t>(std::max(padded ? wgrad::chainPartials(static_cast<int>(rows)) : 1, most)) * (M + 1) * C);
     };
     partials(I);
@@ -1225,7 +1223,7 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
     // 8-byte loads); callers' buffers that are not aligned that way take the scalar kernels.
     const bool tensorInputGrad = qat && call.exec->weightClass == CodeClass::I8 && igrad::eligible(C, I) && !simtGrads &&
                                  alignedTo(call.dx, 16) && alignedTo(mk.x, 8) && alignedTo(call.W_q, 16);
-    // backwardPadded: as exact as the FP32 kernels that the caller's widths would take, so the rows go in chunks (wgrad::chained)
+    // backwardPadded: as exact as the FP32 kernels that the caller's widths would take, so the rows go in chunks (wgrad::launchChained)
     const bool padded = call.dxColumns != 0;
     const bool tensorGrads = qat && call.exec->actClass == CodeClass::I8 && I + 1 <= 144 && H + 1 <= 144 && I % 4 == 0 &&
                              H % 4 == 0 && !simtGrads && alignedTo(call.x_q, 16) && alignedTo(call.h, 16) &&
@@ -1389,8 +1387,8 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
                 plans.push_back(wgrad::planPair(px, ph, chunks[i] * B, C, false, i + 1 == chunks.size() ? sms : std::max(4, sms * share / 100)));
                 for (int k = 0; k < 2; ++k) splits[k] += plans.back().splits[k];
             }
-            const bool room = splits[0] <= std::max(wgrad::tileSplitBound(I, C), wgrad::splitBound(static_cast<int>(rows), I, C)) &&
-                              splits[1] <= std::max(wgrad::tileSplitBound(H, C), wgrad::splitBound(static_cast<int>(rows), H, C));
+            const bool room = splits[0] <= std::max(wgrad::tileSplitBound(I, C), wgrad::splitBound(static_cast<int>(rows))) &&
+                              splits[1] <= std::max(wgrad::tileSplitBound(H, C), wgrad::splitBound(static_cast<int>(rows)));
             if (plans.size() != chunks.size() || !room) chunks.assign(1, T);
         }
         if (chunks.size() > 1) {
@@ -1543,10 +1541,10 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
                 wgrad::launchPair(px, ph, K, C, plan, wideCodes, st);
             }
         } else {   // tensorGrads: both at most 143
-            const wgrad::Plan planX = wgrad::plan(K, I, C, std::max(1, sms / 2)), planH = wgrad::plan(K, H, C, std::max(1, sms / 2));
-            room(planX.splits, planH.splits);
-            wgrad::launch(px, K, C, planX, st);
-            wgrad::launch(ph, K, C, planH, st);
+            const wgrad::Plan each = wgrad::plan(K, C, std::max(1, sms / 2));
+            room(each.splits, each.splits);
+            wgrad::launch(px, K, C, each, st);
+            wgrad::launch(ph, K, C, each, st);
         }
         afterLaunch("weightGrad");
         {

@@ -1707,7 +1707,7 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, bool onBytes, Workspa
             // of 40 inputs, C 192 27 -> 27, C 360 37 -> 37.
             const bool registerProjection = C <= 512 && kw4 <= 4 && block >= kI8Rows * kw4 * 4;
             const bool filled = 8 * C >= 5 * padTo(C, 128) || (kw4 > 2 && C >= 48);
-            if (iproj::eligible(C, H, iWords, xCodes, ihCodes, mk.weight_ih_linear) &&
+            if (iproj::eligible(C, iWords, xCodes) &&
                 (C % 128 == 0 || !registerProjection || (filled && rows >= 8192)) &&
                 std::getenv("RXMET_GRU_FWD_GENERIC") == nullptr) {
                 // tcgen05 kind::i8 GEMM with the fused epilogue
@@ -2212,7 +2212,7 @@ void forwardQuant(const ForwardQuantCall &call, const Exec &e, void *workspace, 
     // 16-bit codes, and 8-bit ones beyond 128 units that the recurrence on bytes does not take: the register path below holds R of 256
     // units in spilled registers (H = 192, B = 500, T = 98: 666 us against 298 us over clusters)
     const bool onBytes = recurrenceOnBytes(call, e);
-    const bool bytes = onBytes && iproj::eligible(3 * call.H, call.H, padTo(call.I, 4) / 4, nullptr, nullptr, nullptr);
+    const bool bytes = onBytes && iproj::eligible(3 * call.H, padTo(call.I, 4) / 4, nullptr);
     if (forwardWideTakes(e, call.I, call.H) &&
         (a == CodeClass::I16 || (call.H > 128 && !call.stepFlags && !bytes && forwardWideClusterTakes(e, call.B, call.H)))) {
         runWide(call, e, ws, st);

@@ -71,7 +71,7 @@ struct WeightRow {
             }
         } else {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) c[j] = __ldg(p.codesKN + static_cast<size_t>(k0 + j) * p.ldCodesKN + n);
+            for (int j = 0; j < 8; ++j) c[j] = __ldg(p.codesKN + static_cast<size_t>(k0 + j) * p.N + n);
         }
     }
     __device__ __forceinline__ uint4 packed() const {
@@ -219,9 +219,9 @@ inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s
         }
     } else if (warp < kFillWarps) {
         // the two warps of a quarter take blocks of 32 columns in turn
-        const int quarter = warp & 3, half = (warp - kConvWarps) >> 2, ldN = p.ldN ? p.ldN : p.N;
+        const int quarter = warp & 3, half = (warp - kConvWarps) >> 2;
         float4 *mine = reinterpret_cast<float4 *>(turn + (warp - kConvWarps) * 4096);
-        const bool vectors = p.N % 4 == 0 && ldN % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.mask) & 3) == 0;
+        const bool vectors = p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.mask) & 3) == 0;
         Turn acc;
         for (int tile = 0; tile < tiles; ++tile, acc.step(s.accs)) {
             wait(&accFull[acc.at], acc.parity);
@@ -248,11 +248,11 @@ inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s
                         make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
                 __syncwarp();
                 const int i = lane & 7, col = c0 + 4 * i, left = columns - col, at = lane >> 3;
-                const size_t o = static_cast<size_t>(first + at) * ldN + n0 + col;
+                const size_t o = static_cast<size_t>(first + at) * p.N + n0 + col;
                 if (left > 0) {
                     float *to = p.out + o;
                     const uint8_t *m = p.mask + o;
-                    const size_t step = 4 * static_cast<size_t>(ldN);
+                    const size_t step = 4 * static_cast<size_t>(p.N);
                     uint32_t drop[8];   // a byte is 0xff where the mask drops the value
 #pragma unroll
                     for (int pass = 0; pass < 8; ++pass) {
@@ -326,7 +326,7 @@ inputGradUmma(const __grid_constant__ Problem p, const __grid_constant__ Shape s
             for (int g = max(0, issued - kWeightRing); g < issued; ++g) waitPhase(smemAddr(&weightsFull[g % kWeightRing]), (g / kWeightRing) & 1);
         }
     } else if (electOne()) {
-        const uint32_t idesc = instructionDescriptor(NP, false, false);
+        const uint32_t idesc = instructionDescriptor(NP, false);
         if (!STREAM) wait(&weightsFull[0], 0);
         Turn stage, slot, acc;
         for (int tile = 0; tile < tiles; ++tile, acc.step(s.accs)) {
@@ -390,12 +390,10 @@ bool eligible(int K, int N) {
     return !disabled && N >= 1 && K >= kChunk && K % kChunk == 0 && K <= kMaxK && encodeTiled() != nullptr;
 }
 
-void launch(const Problem &prob, int sms, cudaStream_t st) {
-    Problem p = prob;
+void launch(const Problem &p, int sms, cudaStream_t st) {
     const bool stream = !resident(p.K, p.N);
     RXMET_REQUIRE(p.rows >= 1 && p.K % kChunk == 0 && p.K <= kMaxK && alignedTo(p.G, 16) && (!stream || (p.packed != nullptr && alignedTo(p.packed, 16))),
                   "input gradient: %d channels, %d columns", p.K, p.N);
-    if (p.ldCodesKN == 0) p.ldCodesKN = p.N;
     Shape s = shapeFor(p.N);
     const size_t most = std::min<size_t>(225 * 1024, currentDevice().smemMax);
     s.ring = kMaxRing;

@@ -25,9 +25,6 @@ struct Problem {
     int maskKeeps = 1;                  // 1: a nonzero byte keeps the gradient; 0: a nonzero byte drops it
     float *out = nullptr;               // [rows][N]
     int *status = nullptr;              // device word, set to 1 when a bounded wait of the kernel gave up
-    int ldN = 0;                        // elements between rows of `out` and `mask` (0 = N); wider than N when the
-                                        // problem is one 64-column slab of a larger output
-    int ldCodesKN = 0;                  // elements between k rows of codesKN (0 = N)
     void *packed = nullptr;             // scratch of packedBytes(K, N) bytes, 16-byte aligned
     int *clear = nullptr;               // word that the launch sets to 0, for kernels behind it; may be `status`
 };

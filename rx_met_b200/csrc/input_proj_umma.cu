@@ -233,9 +233,8 @@ __global__ void __launch_bounds__(kThreads, 2) inputProjUmma(const Problem p, in
 
 int paddedK(int kWords) { return (kWords * 4 + 31) / 32 * 32; }
 
-bool eligible(int C, int H, int kWords, const void *x, const void *out, const void *mask) {
+bool eligible(int C, int kWords, const void *x) {
     static const bool disabled = std::getenv("RXMET_IPROJ_SIMT") != nullptr;
-    (void)H; (void)out; (void)mask;
     if (disabled || kWords < 1 || !alignedTo(x, 4)) return false;
     return static_cast<size_t>(paddedC(C) + 2 * kRows) * paddedK(kWords) <= 200 * 1024;
 }

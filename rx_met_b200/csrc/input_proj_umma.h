@@ -32,8 +32,8 @@ struct Problem {
     bool late = false;
 };
 
-// Operands that fit one SM's shared memory, rows of x on a word boundary.  RXMET_IPROJ_SIMT in the environment turns the path off.
-bool eligible(int C, int H, int kWords, const void *x, const void *out, const void *mask);
+// Codes of all channels and two items of rows within 200 kB, rows of x on a word boundary.  RXMET_IPROJ_SIMT in the environment turns the path off.
+bool eligible(int C, int kWords, const void *x);
 void launch(const Problem &problem, int sms, cudaStream_t stream);
 
 }  // namespace iproj

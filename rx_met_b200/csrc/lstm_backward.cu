@@ -595,7 +595,7 @@ constexpr int kMaxTensorSplits = 40;
 
 // Splits of the tensor-core weight-gradient partial arrays.
 int tensorSplitBound(int rows, int I, int H, int M, int C, bool padded) {
-    const int single = M <= 143 ? wgrad::splitBound(rows, M, C) : 1;
+    const int single = M <= 143 ? wgrad::splitBound(rows) : 1;
     return std::max({single, padded ? wgrad::chainPartials(rows) : 1, wgrad::tensorMemoryPath(I, H, C) ? wgrad::tileSplitBound(M, C) : 1});
 }
 
@@ -970,19 +970,14 @@ void backward(const BackwardCall &call, void *workspace, size_t workspaceBytes, 
             }
         } else {
             previous();
-            auto planFor = [&](int M) {
-                wgrad::Plan pl = wgrad::plan(K, M, C, currentDevice().sms);
-                if (pl.splits > kMaxTensorSplits) {
-                    pl.chunkK = ((K + kMaxTensorSplits - 1) / kMaxTensorSplits + 31) / 32 * 32;
-                    pl.splits = (K + pl.chunkK - 1) / pl.chunkK;
-                }
-                return pl;
-            };
-            const wgrad::Plan planX = planFor(I), planH = planFor(H);
-            splitsX = planX.splits;
-            splitsH = planH.splits;
-            wgrad::launch(px, K, C, planX, st);
-            wgrad::launch(ph, K, C, planH, st);
+            wgrad::Plan each = wgrad::plan(K, C, currentDevice().sms);
+            if (each.splits > kMaxTensorSplits) {
+                each.chunkK = ((K + kMaxTensorSplits - 1) / kMaxTensorSplits + 31) / 32 * 32;
+                each.splits = (K + each.chunkK - 1) / each.chunkK;
+            }
+            splitsX = splitsH = each.splits;
+            wgrad::launch(px, K, C, each, st);
+            wgrad::launch(ph, K, C, each, st);
         }
         afterLaunch("weightGrad");
         {

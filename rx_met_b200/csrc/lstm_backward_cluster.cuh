@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(Tile<H, U, ROWS>::kThreads, 1) recurrentBackwa
     __syncthreads();
     cluster::barrierAll();   // every CTA's barriers are armed before anyone sends
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    constexpr uint32_t kIdesc = instructionDescriptor(G::kCols, false, false);
+    constexpr uint32_t kIdesc = instructionDescriptor(G::kCols, false);
     const uint64_t descB0 = operandDescriptor(smemAddr(bTile), G::kStrideB, kCore);
     bool alive = true;   // false once one of this thread's waits gave up: it waits no more and its values become NaN
     auto wait = [&](uint32_t bar, uint32_t parity) {

@@ -27,8 +27,8 @@ inline EncodeTiled encodeTiled() {
 constexpr int kBoxRows = 32, kBoxCols = 32;
 constexpr uint32_t kBoxBytes = kBoxRows * kBoxCols * 4;
 
-// [rows][cols], 16-byte aligned, cols a multiple of 4; what lies beyond the array reads as zero bits.  The x coordinate of every copy is a
-// multiple of the box's columns, which are a multiple of 4.
+// [rows][cols], 16-byte aligned, cols a multiple of 4; what lies beyond the array reads as zero bits.  The x coordinate of every copy has
+// to be a multiple of 4 (16 bytes): element tiles of weight gradients start at multiples of 16, all other boxes at multiples of their columns.
 inline CUtensorMap boxMap(const void *data, int rows, int cols, CUtensorMapSwizzle swizzle, int boxCols = kBoxCols, int boxRows = kBoxRows) {
     CUtensorMap map;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};

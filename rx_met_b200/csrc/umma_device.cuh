@@ -1,6 +1,5 @@
-// Device helpers shared by the tcgen05 kernels: operand and instruction descriptors, MMA issue
-// and commit, bounded mbarrier waits, tensor-memory loads, the three-way bf16 split of fp32
-// values, and 16-byte asynchronous copies.
+// Device helpers shared by the tcgen05 kernels: operand and instruction descriptors, commits, bounded mbarrier waits, rings of
+// chunks, tensor-memory loads.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -55,23 +54,11 @@ __device__ __forceinline__ uint64_t operandDescriptor(uint32_t addr, uint32_t kG
 }
 
 // Instruction descriptor of kind::f16 for a 128-row accumulator tile: fp32 accumulator (bits
-// [4,6) = 1), bf16 A and B ([7,10) = [10,13) = 1), operand majors in bits 15 (A) and 16 (B),
+// [4,6) = 1), bf16 A and B ([7,10) = [10,13) = 1), A K-major (bit 15 clear), the major of B in bit 16,
 // 1 = MN-major, N >> 3 in [17,23), M >> 4 in [24,29).
-__host__ __device__ constexpr uint32_t instructionDescriptor(int n, bool aMnMajor, bool bMnMajor) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (aMnMajor ? (1u << 15) : 0u) | (bMnMajor ? (1u << 16) : 0u) |
+__host__ __device__ constexpr uint32_t instructionDescriptor(int n, bool bMnMajor) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (bMnMajor ? (1u << 16) : 0u) |
            (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(kTileM >> 4) << 24);
-}
-
-__device__ __forceinline__ void mmaBf16(uint32_t tmemD, uint64_t descA, uint64_t descB, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t"
-        "}\n"
-        :
-        : "r"(tmemD), "l"(descA), "l"(descB), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
 }
 
 __device__ __forceinline__ void commitTo(uint32_t bar) {
@@ -181,34 +168,6 @@ __device__ __forceinline__ void tmemLoad32(uint32_t taddr, uint32_t (&r)[32]) {
           "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-struct Converted {
-    uint4 hi, mid, lo;
-};
-
-// Eight fp32 values -> three bf16x8 vectors whose sum is the input exactly.
-__device__ __forceinline__ Converted splitThree(const float4 &u, const float4 &v) {
-    const float x[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
-    uint32_t h[4], m[4], l[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        h[i] = packBf16(x[2 * i], x[2 * i + 1]);
-        const float r0 = x[2 * i] - bf16Lo(h[i]), r1 = x[2 * i + 1] - bf16Hi(h[i]);
-        m[i] = packBf16(r0, r1);
-        l[i] = packBf16(r0 - bf16Lo(m[i]), r1 - bf16Hi(m[i]));
-    }
-    Converted c;
-    c.hi = make_uint4(h[0], h[1], h[2], h[3]);
-    c.mid = make_uint4(m[0], m[1], m[2], m[3]);
-    c.lo = make_uint4(l[0], l[1], l[2], l[3]);
-    return c;
-}
-
-// 16-byte asynchronous copy global -> shared; `valid` false writes zeros instead.
-__device__ __forceinline__ void copyAsync16(void *dst, const void *src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smemAddr(dst)), "l"(src), "r"(valid ? 16u : 0u)
-                 : "memory");
 }
 
 }  // namespace umma

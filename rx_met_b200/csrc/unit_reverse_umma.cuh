@@ -133,7 +133,7 @@ unitReverse(const __grid_constant__ Problem p, const __grid_constant__ Cell c) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     if (warp == G::kWarps) {
-        constexpr uint32_t kIdesc = instructionDescriptor(G::kCols, false, false);
+        constexpr uint32_t kIdesc = instructionDescriptor(G::kCols, false);
         const uint64_t descB = operandDescriptor(smemAddr(bTile), G::kStrideB, kCore);
 #pragma unroll 1
         for (int n = 0; n < p.T; ++n) {

@@ -23,7 +23,7 @@ struct Problem {
     float aInvScale = 1.0f;
     float aFloatZero = 0.0f;
     int32_t aZero = 0;                // zero point of aCodes
-    int M = 0;                        // real rows (multiple of 4, at most 143); row M is the ones row
+    int M = 0;                        // real rows (multiple of 4; the mma.sync kernel: at most 143); row M is the ones row
     const float *B = nullptr;         // [K][N] gradients, N a multiple of 4
     float *partial = nullptr;         // [splits][M+1][N]
     int *status = nullptr;            // device word, set to 1 when a bounded wait of the kernel gave up
@@ -37,13 +37,13 @@ struct Plan {
     int splits = 0;
     int chunkK = 0;
 };
-Plan plan(int K, int M, int N, int sms);
+Plan plan(int K, int N, int sms);
 void launch(const Problem &problem, int K, int N, const Plan &plan, cudaStream_t stream);
 // Upper bound of plan(...).splits over every device, for sizing the partial buffers.
-int splitBound(int K, int M, int N);
+int splitBound(int K);
 
 // The tcgen05 kernel (weight_grad_umma.cu): two problems over the same K rows and N columns (the input and the recurrent weights of a step) in
-// one launch.  M a multiple of 4, N of 128 or 192; operands 16-byte aligned.  RXMET_WGRAD_MMA_SYNC in the environment turns it off.
+// one launch.  M a multiple of 4 up to sixteen tiles of 256, N a multiple of 128 or 192; operands 16-byte aligned.  RXMET_WGRAD_MMA_SYNC in the environment turns it off.
 constexpr int kMaxSms = 160;
 struct PairPlan {
     int splits[2], chunks[2];   // of a and b: K splits, chunks of 32 rows in a split
@@ -56,14 +56,15 @@ void launchPair(const Problem &a, const Problem &b, int K, int N, const PairPlan
 // Upper bound of a problem's splits over every device, for sizing its partial sums.
 int tileSplitBound(int M, int N);
 
-// The tensor core truncates every addition to an accumulator; over a chunk of n rows that costs up to 8e-9 n of a sum of terms of one
-// sign with 16-bit codes (512 rows: 4.3e-6, 4096: 3.5e-5), a fifth of it with 8-bit codes.  Calls that would otherwise take
+// The tensor core truncates every addition to an accumulator.  Largest error of a sum of n terms of one sign: up to 128 elements (accumulators for the
+// leading terms) 4e-7 with 8-bit codes up to 4096 rows, 6e-9 n with 16-bit codes (512 rows: 3.1e-6, 4096: 2.3e-5); beyond 128 elements (one accumulator)
+// 2e-8 n with 8-bit codes (384 rows: 7.4e-6) and 3.5e-8 n with 16-bit codes (384 rows: 1.3e-5).  Calls that would otherwise take
 // the FP32 kernels therefore cut the rows into chunks of kChainRows, however many there are: up to kChainGroup chunks (three
 // waves of the widest layers) leave their partial sums to the reduction that follows, more go in several launches, after each of which
 // addPartials folds the partial sums into one more array of them, so that the arrays do not grow with the rows.
 constexpr int kChainRows = 512, kChainGroup = 32;
 inline int chainChunks(int K) { return (K + kChainRows - 1) / kChainRows; }
-// Arrays of (M + 1) x N partial sums that chained() writes.
+// Arrays of (M + 1) x N partial sums that launchChained() writes.
 inline int chainPartials(int K) { return chainChunks(K) <= kChainGroup ? chainChunks(K) : kChainGroup + 1; }
 // sums of a and b (sum[i] = or += partial[0][i] + partial[1][i] + ...), `partial` behind the sums
 void addPartials(float *a, size_t countA, float *b, size_t countB, int partials, bool first, cudaStream_t stream);

@@ -66,7 +66,6 @@ struct Pair {
     Tile tile[kMaxTiles];
     int tiles, channelTiles, N;
     int firstChunks[2], totalChunks[2];   // chunks that Problem::aFirst gives the codes of; all chunks
-    int K;
 };
 
 // Codes of one term: two groups of warps take chunks in turn, which hides their hand-overs (T = 100, B = 256, H = 128, four gates 42.4 -> 38.9 us); of two
@@ -254,7 +253,7 @@ __global__ void __launch_bounds__(kThreads, 1) weightGradUmma(const __grid_const
         });
     } else if (electOne()) {
         // A: K-major in tensor memory, B: MN-major in shared memory
-        const uint32_t idesc = instructionDescriptor(NP, false, true), others = tmem + (tile.accs - 1) * NP;
+        const uint32_t idesc = instructionDescriptor(NP, true), others = tmem + (tile.accs - 1) * NP;
         const uint64_t descB0 = operandDescriptor(smemAddr(stages), kStride, kCore);
         const bool parted = tile.accs == 3;
         Turn stage;
@@ -395,7 +394,6 @@ void launchPair(const Problem &a, const Problem &b, int K, int N, const PairPlan
     set.tiles = 0;
     set.channelTiles = channelTiles(N);
     set.N = N;
-    set.K = K;
     const int terms = wide ? 2 : 1;
     size_t smem = 0;
     int blocks = 0;
