@@ -18,8 +18,8 @@
 // per-tensor grid.  HBM-bound: the forward moves 8 bytes per element, the backward 12, and the sums ride
 // along: per-CTA partials land in a small workspace and a second launch adds them in a fixed order, so the
 // result does not change from run to run.  Rows of one segment that are whole grid entries (a weight matrix
-// with a grid per row, up to 8192 elements) need neither, as a CTA has all of a row's sums: 4096 x 4096,
-// forward and backward 75.3 -> 71.2 us.
+// with a grid per row, up to 8192 elements) need neither, as a CTA has all of a row's sums: one launch
+// less, 4096 x 4096, forward and backward 75.9 -> 73.1 us where two runs differ by up to 5 %.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -13,10 +13,11 @@
 // the CTA, turns the outputs that follow into NaN and sets the status word; copies and products in flight are awaited and
 // tensor memory is freed all the same.
 //
-// Bound: the hand-overs and the conversion of a chunk (0.35 us a chunk and SM), beyond 128 columns the tensor pipe (0.41 us at 256 columns).  The forms
-// before it wrote the terms to shared memory, where the MMAs read them again: half of its bandwidth beside copies and conversion; they walked
+// Bound: the hand-overs and the conversion of a chunk (0.50 us a chunk and SM up to 128 columns; issue 39 %, DRAM 40 %, tensor pipe 11 %); beyond 128
+// columns the products of a tile wait for the read-out of the one accumulator (256 columns: 30.7 us a tile of 32 chunks, 47.4 of 64, that is 0.52 a chunk, of
+// which the MMAs take 0.41, and 14 for the read-out; tensor pipe 40 %).  The forms before it wrote the terms to shared memory, where the MMAs read them again: half of its bandwidth beside copies and conversion; they walked
 // whole tiles (two rounds where a CTA has 173 rows) and left the epilogue outside.  In a step, with what surrounds the kernel: 25,600 rows x 384 -> 40
-// columns 26.8 -> 23.7 us, 25,600 x 512 -> 40 31.7 -> 26.1, 12,800 x 768 -> 40 41.4 -> 24.7, 256,000 x 2048 -> 256 943 -> 707; by itself, back to back, 17, 21, 18 us
+// columns 26.8 -> 23.7 us, 25,600 x 512 -> 40 31.7 -> 26.1, 12,800 x 768 -> 40 41.4 -> 24.7, 256,000 x 2048 -> 256 943 -> 664; by itself, back to back, 17, 21, 18 us
 // and 12,800 x 768 -> 512 59 -> 40.
 #include <algorithm>
 #include <cstdlib>

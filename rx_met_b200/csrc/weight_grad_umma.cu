@@ -19,10 +19,14 @@
 // The tensor core truncates each addition to an accumulator.  Up to 128 elements the first terms, which carry the sum's size, have accumulators
 // of their own, one for each k-step of a chunk, that are added to the others' at the end: a sixth of the additions that truncate at that size.
 //
-// Bound: reading the operands where codes have one term, the tensor pipe where they have two.  With both operands in shared
-// memory (the form before) the MMAs alone took 3/4 of its bandwidth beside the copies and the conversion.  In a step: 256,000 rows, 256 + 512 elements,
-// 2048 channels, two terms 4.25 -> 3.29 ms (its products at the measured burst rate: 2.9); 12,800 rows, 512 + 256, 768 channels by itself 94 -> 61 us; 25,600 rows,
-// 40 + 128, one term, 512 channels 41.7 -> 39.4 us, 384 channels 28.5 (another kernel, deleted) -> 30.5.
+// Bound: codes of one term hand-overs and reading (102,400 more rows of 40 + 128 elements and 384 channels 92 us = 4.2 TB/s; DRAM 47 %, issue 48 %, tensor pipe
+// 18 %), of two terms the tensor pipe (77 %; 51,200 more rows, 256 + 256 elements, 1024 channels 209 us = 1.54 PFLOP/s).  With both operands in shared
+// memory (the form before) the MMAs alone took 3/4 of its bandwidth beside the copies and the conversion.  256,000 rows, 256 + 512 elements,
+// 2048 channels, two terms 4.25 -> 3.13 ms; 12,800 rows, 512 + 256, 768 channels 94 -> 61 us; 25,600 rows, 40 + 128, one term, 512 channels 41.7 -> 39.4 us.  384
+// channels by itself 28.5 (another kernel, of 192 channels a CTA) -> 30.5 us, in a step from the end of the input gradient on 28.4 -> 27.1, because it prepares
+// itself under that one's tail: one kernel for all widths, with a sixth of the other's error.
+// A last tile of 64 channels (192, 576) is half empty; passes of 25,600 rows, I 40, against that form all the same: 64 units 162 -> 157 us (16-bit codes 201 -> 186),
+// 192 units 422 -> 372 (485 -> 413).
 // Error against 64 bits, 2-norm, normal gradients: 25,600 rows, one term 1.0e-6 -> 1.7e-7 (512 channels), 1.9e-6 -> 1.5e-7 (384); 12,800 rows, two terms 8.0e-6, as before.
 //
 // Every mbarrier wait is bounded; one that gives up ends all further waiting of the CTA and sets the status word (the reduction that follows turns
