@@ -1694,7 +1694,7 @@ void runTyped(const ForwardQuantCall &call, const Exec &e, bool onBytes, Workspa
     bool tensorProjection = false;
     // CTAs of the recurrence behind the projection (iproj::Problem::dependents); lanes of short sequences and few rows gain by the early start whatever
     // SMs they share
-    const int dependents = onBytes ? unitrec::mostCtas(B, H) : lanesPath && T >= 32 && rows >= 6000 ? (B + btI8 - 1) / btI8 : 0;
+    const int dependents = onBytes ? unitrec::smsFor(B, H) : lanesPath && T >= 32 && rows >= 6000 ? (B + btI8 - 1) / btI8 : 0;
     std::vector<int> chunks{T};   // time chunks of the overlapped pipeline (one = none)
     {
         const int block = std::min(padTo(C, 32), 512);

@@ -431,7 +431,7 @@ void forwardWide(const WideCall &call, const Exec &e, cudaStream_t st) {
         epi.addend = l.addX; epi.rescale = call.gemmX;
         epi.zpOut = g.zp[RXMET_GRU_WEIGHT_IH_LINEAR]; epi.lo = g.qlo[RXMET_GRU_WEIGHT_IH_LINEAR]; epi.hi = g.qhi[RXMET_GRU_WEIGHT_IH_LINEAR];
         epi.out = l.ihCodes; epi.mask = call.maskIh; epi.C = C;
-        planeproj::launch<2>("inputLinear", pp, epi, smsPerPass(), unitrec::mostCtas(B, H), st);
+        planeproj::launch<2>("inputLinear", pp, epi, smsPerPass(), unitrec::smsFor(B, H), st);
     } else {
         InputArgs a{};
         a.rows = static_cast<int>(rows); a.C = C; a.kWords = kI;

@@ -940,7 +940,7 @@ void forwardQuantWide(const ForwardQuantCall &call, const Exec &e, void *workspa
         auto launchTensor = [&](auto epi, auto planeCount) {
             epi.addend = l.addIh; epi.fields = l.channel; epi.s = s; epi.H = H; epi.I = I; epi.lhs = l.lhs;
             epi.linear = ck.weight_ih_linear; epi.linearClamped = ck.weight_ih_linear_clamped;
-            planeproj::launch<decltype(planeCount)::value>("lstmInputLinearWide", pp, epi, smsPerPass(), unitrec::mostCtas(B, H), st);
+            planeproj::launch<decltype(planeCount)::value>("lstmInputLinearWide", pp, epi, smsPerPass(), unitrec::smsFor(B, H), st);
         };
         if (planes == 2) launchTensor(WidePlaneEpilogue<2>{}, std::integral_constant<int, 2>{});
         else launchTensor(WidePlaneEpilogue<1>{}, std::integral_constant<int, 1>{});

@@ -286,8 +286,14 @@ int residentCtas(const Cell &cell) {
     return std::max(1, std::min(Geometry<Cell, HP, U, ROWS, PLANES>::kResident, static_cast<int>(all / each)));
 }
 
-// Most CTAs that launchRows() takes for `rows` rows.
-inline int mostCtas(int rows, int H) { return H <= 128 ? rows : (rows + 3) / 4 * ((H + 63) / 64); }
+// SMs that the most CTAs launchRows() takes for `rows` rows need beside a kernel that holds the others: clusters lie within one of about eight groups of
+// SMs, each of which may have up to a cluster less one too many.  Launched beside a projection that leaves them no more than their number, clusters of
+// three came to lie two on an SM: 16-bit GRU, T = 98, B = 64, H = 160 141 us, behind the projection's end 113; T = 98, B = 40,
+// H = 256 142 and 121.
+inline int smsFor(int rows, int H) {
+    const int ctas = (H + 63) / 64;
+    return H <= 128 ? rows : (rows + 3) / 4 * ctas + 8 * (ctas - 1);
+}
 
 // `early`: before the kernel in front of it has ended (its prologue runs beside that one's end).
 template <class Cell, int HP, int U, int ROWS, int PLANES>
