@@ -24,7 +24,7 @@ struct Problem {
     int16_t *out = nullptr;            // [rows][C]
     uint8_t *mask = nullptr;           // [rows][C] keep flags, optional
     int *status = nullptr;             // device word, set to 1 when a bounded wait of the kernel gave up
-    // CTAs of the recurrence behind the projection.  Where both find SMs of their own it starts with the projection's first CTAs and prepares
+    // SMs that the recurrence behind the projection needs, one a CTA or as unitrec::smsFor counts them.  Where both find SMs of their own it starts with the projection's first CTAs and prepares
     // itself beside them; where they do not, with the last (late, filled in by launch()): CTAs that take the room left among those of a
     // projection lie unevenly on the SMs for the whole sequence (inference in lanes: 16 units, T 200, 200 rows 141 -> 75 us, T 98, 300 rows 88 -> 48; 64 units,
     // 80 inputs, T 200, 128 rows 122 -> 89).

@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kThreads, 1) planeProjUmma(const __grid_consta
     if (tid == 0 && failed && p.status) atomicExch(p.status, 1);
 }
 
-// Launches the projection on at most `sms` SMs.  `dependents`: CTAs of the recurrence behind it, which starts with the first CTAs of the
+// Launches the projection on at most `sms` SMs.  `dependents`: SMs that the recurrence behind it needs (unitrec::smsFor), which starts with the first CTAs of the
 // projection where both find SMs of their own, and prepares itself beside them, else when the last of them has gone (16-bit GRU inference, 1 row: T = 1, H = 128
 // 27 -> 21 us, T = 40, H = 100 45 -> 41 us; before it had to wait for the projection's end to be launched at all).
 template <int PLANES, class Epilogue>
